@@ -177,6 +177,24 @@ SO3LR_B200_API int so3lr_b200_system_graph_eval_kspace(so3lr_b200_system* sys, v
                                         float* e_atom_dev, float* g_edges_dev, float* g_edges_lr_dev, float* g_positions_dev,
                                         float* strain6_dev, float* charges_dev, float* hirshfeld_dev);
 
+/* Displacements d_e = R[j_e] - R[i_e] (minimum image when `cell_dev` is given: 3 x 3, rows = lattice vectors, on the device) of
+ * the entries of a list, and the transpose: acc4[j_e] += sign g_e, acc4[i_e] -= sign g_e.  Positions, cell, acc4 and
+ * g_positions are float32 (is_double = 0) or float64; the displacements / their cotangents are float32, or float64 when
+ * positions are and out_double / g_double is set.  Indices are clamped to [0, n_atoms), as a gather under JAX does, so padding
+ * entries (index n_atoms) give d = 0.  acc4_dev holds 4 values per atom (16-byte aligned; zeroed first when `clear` is set, so that several
+ * lists can be added up); g_positions_dev (may be NULL) receives its first three columns.  The calls only enqueue work on the
+ * current device.
+ * Replaces: the endpoint gathers of so3lr/jaxmd_utils.py:57-66 and their transpose under jax.grad. */
+SO3LR_B200_API int so3lr_b200_displacements(void* stream, int is_double, int n_atoms, const void* positions_dev, const void* cell_dev,
+                                            int64_t n_entries, const int32_t* idx_i_dev, const int32_t* idx_j_dev, void* out_dev,
+                                            int out_double);
+SO3LR_B200_API int so3lr_b200_displacements_vjp(void* stream, int is_double, int n_atoms, int64_t n_entries, const int32_t* idx_i_dev,
+                                                const int32_t* idx_j_dev, const void* g_dev, int g_double, double sign, void* acc4_dev,
+                                                int clear, void* g_positions_dev);
+/* flags2_dev[k] = 1 when list k is not grouped by ascending centre index, else 0 (so3lr_b200_system_graph_eval wants grouped lists). */
+SO3LR_B200_API int so3lr_b200_lists_unsorted(void* stream, int64_t n_edges, const int32_t* idx_i_dev, int64_t n_pairs,
+                                             const int32_t* idx_i_lr_dev, int32_t* flags2_dev);
+
 /* A velocity-Verlet (NVE) step driven by the library: positions/velocities/forces stay on the device.
  * masses_dev in amu, dt in fs, velocities in Angstrom/fs.  Runs `n_steps` steps; forces_dev must hold the forces
  * of positions_dev on entry (call so3lr_b200_system_compute first) and holds the final forces on return.

@@ -52,6 +52,9 @@ def _load():
         "so3lr_b200_system_graph_eval": (i32, [p, p, i64, p, p, p, i64, p, p, p, p, p, p, p, p, p]),
         "so3lr_b200_system_set_kspace": (i32, [p, i32, f32, i32, i32, i32]),
         "so3lr_b200_system_graph_eval_kspace": (i32, [p, p, i64, p, p, p, i64, p, p, p, p, p, p, p, p, p, p, p]),
+        "so3lr_b200_displacements": (i32, [p, i32, i32, p, p, i64, p, p, p, i32]),
+        "so3lr_b200_displacements_vjp": (i32, [p, i32, i32, i64, p, p, p, i32, f64, p, i32, p]),
+        "so3lr_b200_lists_unsorted": (i32, [p, i64, p, i64, p, p]),
         "so3lr_b200_system_nve": (i32, [p, p, i32, f32, p, p, p, p, p]),
         "so3lr_b200_system_enable_virial": (i32, [p, i32]),
         "so3lr_b200_system_virial": (i32, [p, p, p]),

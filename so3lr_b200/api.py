@@ -22,7 +22,7 @@ from typing import Optional
 import numpy as np
 import torch
 
-from .engine import Model, System
+from .engine import Model, System, displacements, displacements_vjp, lists_unsorted
 
 CUTOFF_SR = 4.5
 
@@ -76,11 +76,13 @@ class _GraphEnergy(torch.autograd.Function):
     def backward(ctx, g):
         edges, edges_lr, ge, gel, gp, gc = ctx.saved_tensors
         g = g.contiguous()
-        lo, hi = torch.aminmax(g)
-        if bool(lo == hi):
-            c = lo.to(ge.dtype)
+        lo, hi = torch.stack(torch.aminmax(g)).tolist()
+        if lo == hi == 1.0:         # the plain sum, as under quantity.force: nothing to scale
+            return (ge, gel, None, None, None, None, None, None, gp if ctx.has_positions else None, gc if gc.numel() else None)
+        if lo == hi:
+            c = lo
             return (ge * c, gel * c, None, None, None, None, None, None, (gp * c if ctx.has_positions else None),
-                    (gc * c.to(gc.dtype) if gc.numel() else None))
+                    (gc * c if gc.numel() else None))
         if ctx.has_positions:
             raise NotImplementedError("the reciprocal-space energy is differentiated for a uniform cotangent (its sum) only")
         out = ctx.system.graph_eval(ctx.lists[0], ctx.lists[1], edges, ctx.lists[2], ctx.lists[3], edges_lr, g_e_atom=g)
@@ -157,11 +159,12 @@ class So3lrPotentialB200:
         edges, edges_lr = graph.edges, graph.edges_lr
         idx_i, idx_j, idx_i_lr, idx_j_lr = graph.centers, graph.others, graph.idx_i_lr, graph.idx_j_lr
         # the kernels want lists grouped by centre; jax-md style lists already are
-        perm = perm_lr = None
-        if idx_i.numel() > 1 and bool((idx_i[1:] < idx_i[:-1]).any()):
+        idx_i, idx_i_lr = idx_i.to(self.device, torch.int32), idx_i_lr.to(self.device, torch.int32)
+        unsorted, unsorted_lr = lists_unsorted(idx_i, idx_i_lr)
+        if unsorted:
             perm = torch.sort(idx_i, stable=True).indices
             idx_i, idx_j, edges = idx_i[perm], idx_j[perm], edges[perm]
-        if idx_i_lr.numel() > 1 and bool((idx_i_lr[1:] < idx_i_lr[:-1]).any()):
+        if unsorted_lr:
             perm_lr = torch.sort(idx_i_lr, stable=True).indices
             idx_i_lr, idx_j_lr, edges_lr = idx_i_lr[perm_lr], idx_j_lr[perm_lr], edges_lr[perm_lr]
         aux = {}
@@ -318,6 +321,24 @@ def _min_image(dR, cell_t):
     return dR - torch.round(s) @ cell_t
 
 
+class _PairDisplacements(torch.autograd.Function):
+    """(d, d_lr) of both lists from Cartesian positions, minimum image under `cell_t`; `wide` keeps the dtype of the positions,
+    else the displacements come out in float32.  One kernel per list and direction (csrc/displacements.cu)."""
+
+    @staticmethod
+    def forward(ctx, Rc, cell_t, wide, idx_i, idx_j, idx_i_lr, idx_j_lr):
+        ctx.lists, ctx.like = ((idx_i, idx_j), (idx_i_lr, idx_j_lr)), (Rc.shape[0], Rc.dtype, Rc.device)
+        ctx.set_materialize_grads(False)
+        dt = Rc.dtype if wide else torch.float32
+        return tuple(displacements(Rc, cell_t, i, j, dt) for i, j in ctx.lists)
+
+    @staticmethod
+    def backward(ctx, g, g_lr):
+        n, dt, dev = ctx.like
+        parts = [(i, j, gg.contiguous()) for (i, j), gg in zip(ctx.lists, (g, g_lr)) if gg is not None]
+        return (displacements_vjp(n, dt, dev, parts), None, None, None, None, None, None)
+
+
 class _Transform(torch.autograd.Function):
     """Fractional -> Cartesian positions with jax-md's convention for the derivative (jax_md.space.transform has a custom
     JVP whose tangent is dR + transform(dbox, R)): the gradient with respect to fractional positions is the real-space one,
@@ -365,12 +386,13 @@ def neighbor_list_featurizer(displacement_fn, species, fractional_coordinates=Tr
             raise ValueError("k-space electrostatics needs `box`")
         Rc = _Transform.apply(R, cell_t) if (cell_t is not None and fractional_coordinates) else R
         neighbor, neighbor_lr = torch.as_tensor(neighbor, device=dev), torch.as_tensor(neighbor_lr, device=dev)
-        idx_i, idx_j = neighbor[0].long(), neighbor[1].long()
-        idx_i_lr, idx_j_lr = neighbor_lr[0].long(), neighbor_lr[1].long()
-        cl = lambda a: a.clamp(max=n - 1)   # JAX gathers clamp the padding index N to N-1
-        # the kernels take dR = R_j - R_i; the energy does not depend on the sign convention
-        dR = _min_image(Rc[cl(idx_j)] - Rc[cl(idx_i)], cell_t)
-        dR_lr = _min_image(Rc[cl(idx_j_lr)] - Rc[cl(idx_i_lr)], cell_t)
+        # the kernels take dR = R_j - R_i; the energy does not depend on the sign convention.  JAX gathers clamp the padding index N
+        if cell_t is not None and cell_t.requires_grad:      # the caller differentiates with respect to the box itself
+            idx = [a.long().clamp(max=n - 1) for a in (*neighbor[:2], *neighbor_lr[:2])]
+            dR, dR_lr = _min_image(Rc[idx[1]] - Rc[idx[0]], cell_t), _min_image(Rc[idx[3]] - Rc[idx[2]], cell_t)
+        else:
+            idx = [a.to(torch.int32).contiguous() for a in (*neighbor[:2], *neighbor_lr[:2])]
+            dR, dR_lr = _PairDisplacements.apply(Rc.contiguous(), cell_t, pert is not None, *idx)
         positions = Rc if k_grid is not None else None
         if pert is not None:
             p = pert if torch.is_tensor(pert) else torch.as_tensor(pert)
@@ -473,25 +495,20 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
                 c = c[0]
             if bool(c.abs().sum() > 0):
                 cell_t = c
-        ii, jj = torch.as_tensor(inputs["idx_i"], device=dev).long(), torch.as_tensor(inputs["idx_j"], device=dev).long()
-        il, jl = torch.as_tensor(inputs["idx_i_lr"], device=dev).long(), torch.as_tensor(inputs["idx_j_lr"], device=dev).long()
-        cl = lambda a: a.clamp(max=n - 1)
-
-        def sort_by_centre(a, b):
-            if a.numel() > 1 and bool((a[1:] < a[:-1]).any()):
-                p = torch.sort(a, stable=True).indices
-                return a[p], b[p]
-            return a, b
-
-        ii, jj = sort_by_centre(ii, jj)
-        il, jl = sort_by_centre(il, jl)
-        dR = _min_image(R[cl(jj)] - R[cl(ii)], cell_t)
-        dRl = _min_image(R[cl(jl)] - R[cl(il)], cell_t)
+        ii, jj, il, jl = (torch.as_tensor(inputs[k]).to(dev, torch.int32).contiguous() for k in ("idx_i", "idx_j", "idx_i_lr", "idx_j_lr"))
+        for which, unsorted in enumerate(lists_unsorted(ii, il)):
+            if unsorted:
+                p = torch.sort((ii, il)[which], stable=True).indices
+                if which == 0:
+                    ii, jj = ii[p], jj[p]
+                else:
+                    il, jl = il[p], jl[p]
+        dR, dRl = displacements(R, cell_t, ii, jj), displacements(R, cell_t, il, jl)
         nm = inputs.get("node_mask")
         node_mask = torch.ones(n, dtype=torch.bool, device=dev) if nm is None else torch.as_tensor(nm, device=dev).bool()
         # cotangent of the masked energy sum (base_calculator.py:91)
         ge = gm_t[torch.as_tensor(bs_np, device=dev)].float() * node_mask.float()
-        out = s.graph_eval(ii.int(), jj.int(), dR, il.int(), jl.int(), dRl, g_e_atom=ge)
+        out = s.graph_eval(ii, jj, dR, il, jl, dRl, g_e_atom=ge)
         bs_t = torch.as_tensor(bs_np, device=dev)
         e_atom = out["e_atom"] * node_mask
         energy = torch.zeros(n_graphs, device=dev).index_add_(0, bs_t, e_atom) * gm_t
@@ -500,10 +517,8 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
         dip = torch.zeros(n_graphs, 3, device=dev).index_add_(0, bs_t, q[:, None] * R) * gm_t[:, None]
         res = dict(energy=energy, dipole_vec=dip, hirshfeld_ratios=h, partial_charges=q)
         if calculate_forces:
-            F = torch.zeros(n, 3, device=dev)
-            vi, vl = (ii < n) & (jj < n), (il < n) & (jl < n)
-            F.index_add_(0, cl(ii), out["g_edges"] * vi[:, None]); F.index_add_(0, cl(jj), -out["g_edges"] * vi[:, None])
-            F.index_add_(0, cl(il), out["g_edges_lr"] * vl[:, None]); F.index_add_(0, cl(jl), -out["g_edges_lr"] * vl[:, None])
+            # dE/dd is zero for entries with an end outside the structure (padding): only real pairs contribute
+            F = displacements_vjp(n, torch.float32, dev, [(ii, jj, out["g_edges"]), (il, jl, out["g_edges_lr"])], sign=-1.0)
             res["forces"] = F
         return res
 

@@ -1357,6 +1357,29 @@ SO3LR_B200_API int so3lr_b200_system_graph_eval_kspace(so3lr_b200_system* S, voi
                          charges, hirshfeld, positions, g_positions, strain6);
 }
 
+SO3LR_B200_API int so3lr_b200_displacements(void* stream, int is_double, int n_atoms, const void* R, const void* cell, int64_t n_entries,
+                                            const int32_t* idx_i, const int32_t* idx_j, void* out, int out_double) {
+  if (n_atoms <= 0 || n_entries < 0 || !R || (n_entries > 0 && (!idx_i || !idx_j || !out)) || (out_double && !is_double)) return kInvalidArgument;
+  tl_launch_counter = nullptr;
+  return displacements((cudaStream_t)stream, is_double != 0, n_atoms, R, cell, n_entries, idx_i, idx_j, out, out_double != 0);
+}
+
+SO3LR_B200_API int so3lr_b200_displacements_vjp(void* stream, int is_double, int n_atoms, int64_t n_entries, const int32_t* idx_i,
+                                                const int32_t* idx_j, const void* g, int g_double, double sign, void* acc4, int clear,
+                                                void* g_positions) {
+  if (n_atoms <= 0 || n_entries < 0 || !acc4 || (n_entries > 0 && (!idx_i || !idx_j || !g)) || (g_double && !is_double)) return kInvalidArgument;
+  tl_launch_counter = nullptr;
+  return displacements_vjp((cudaStream_t)stream, is_double != 0, n_atoms, n_entries, idx_i, idx_j, g, g_double != 0, sign, acc4, clear != 0,
+                           g_positions);
+}
+
+SO3LR_B200_API int so3lr_b200_lists_unsorted(void* stream, int64_t n_edges, const int32_t* idx_i, int64_t n_pairs, const int32_t* idx_i_lr,
+                                             int32_t* flags2) {
+  if (n_edges < 0 || n_pairs < 0 || (n_edges > 0 && !idx_i) || (n_pairs > 0 && !idx_i_lr) || !flags2) return kInvalidArgument;
+  tl_launch_counter = nullptr;
+  return lists_unsorted((cudaStream_t)stream, n_edges, idx_i, n_pairs, idx_i_lr, flags2);
+}
+
 SO3LR_B200_API int so3lr_b200_system_nve(so3lr_b200_system* S, void* stream, int n_steps, float dt, const float* masses, float* R, float* V,
                           float* F, double* energy) {
   if (!S || !masses || !R || !V || !F || n_steps < 0) return kInvalidArgument;

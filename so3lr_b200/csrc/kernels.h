@@ -82,6 +82,16 @@ int launch_ewald(cudaStream_t st, const KSpaceDev& K, const Cell& cell, int n, c
 // ---- halo.cu: rows idx[r] of up to four row-major float arrays <-> one packed buffer [n_rows][sum of widths] ----
 int pack_rows(void* stream, int n_arrays, float* const* arrays, const int* widths, const int64_t* idx, int64_t n_rows, float* buf, bool unpack);
 
+// ---- displacements.cu: d_e = R[j_e] - R[i_e] (minimum image) of caller-supplied lists, and the transpose ----
+// R, cell (rows = lattice vectors, nullptr: free space) and out are float or double device arrays; indices are clamped to [0, n)
+int displacements(cudaStream_t s, bool dbl, int n, const void* R, const void* cell, long long n_entries, const int* idx_i, const int* idx_j,
+                  void* out, bool out_dbl);
+// acc4[j_e] += sign g_e, acc4[i_e] -= sign g_e (four values per atom); `clear` zeroes acc4 first, `out` (optional) receives [n][3]
+int displacements_vjp(cudaStream_t s, bool dbl, int n, long long n_entries, const int* idx_i, const int* idx_j, const void* g, bool g_dbl,
+                      double sign, void* acc4, bool clear, void* out);
+// flags2[k] = 1 when list k is not grouped by ascending receiver
+int lists_unsorted(cudaStream_t s, long long n0, const int* i0, long long n1, const int* i1, int* flags2);
+
 // ---- attention.cu ----
 // Short-range edges are grouped by receiver: edges row_ptr[i] .. row_ptr[i+1]-1 belong to centre i and hold the
 // neighbour index nbr_j[e] and the displacement dR[e] (3 floats).  Edges with |dR| >= 4.5, |dR| == 0 or

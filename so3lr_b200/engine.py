@@ -294,6 +294,44 @@ class System:
         return E, self._cell.copy()
 
 
+def displacements(R, cell, idx_i, idx_j, dtype=torch.float32):
+    """(E, 3) displacements R[j] - R[i] (minimum image under `cell`, rows = lattice vectors, same dtype as R) of int32 index arrays;
+    indices are clamped to the structure, so padding entries give zero.  R float32 or float64, contiguous, on the GPU."""
+    cell = None if cell is None else cell.to(R.device, R.dtype).contiguous()
+    with torch.cuda.device(R.device):
+        out = torch.empty(idx_i.numel(), 3, dtype=dtype, device=R.device)
+        s = torch.cuda.current_stream(R.device)
+        check(lib.so3lr_b200_displacements(C.c_void_p(s.cuda_stream), int(R.dtype == torch.float64), R.shape[0], _ptr(R), _ptr(cell),
+                                           idx_i.numel(), _ptr(idx_i), _ptr(idx_j), _ptr(out), int(dtype == torch.float64)), "displacements")
+    return out
+
+
+def displacements_vjp(n, dtype, device, parts, sign=1.0):
+    """sum over the lists (idx_i, idx_j, g) in `parts` of the transpose of `displacements`: out[j] += sign g, out[i] -= sign g."""
+    with torch.cuda.device(device):
+        out = torch.empty(n, 3, dtype=dtype, device=device)
+        acc = torch.empty(n, 4, dtype=dtype, device=device)
+        s = torch.cuda.current_stream(device)
+        parts = parts or [(None, None, None)]
+        for k, (i, j, g) in enumerate(parts):
+            check(lib.so3lr_b200_displacements_vjp(C.c_void_p(s.cuda_stream), int(dtype == torch.float64), n, 0 if i is None else i.numel(),
+                                                   _ptr(i), _ptr(j), _ptr(g), int(g is not None and g.dtype == torch.float64), float(sign),
+                                                   _ptr(acc), int(k == 0), _ptr(out) if k == len(parts) - 1 else None), "displacements_vjp")
+    return out
+
+
+def lists_unsorted(idx_i, idx_i_lr):
+    """Two host booleans: whether each index array (int32, on the GPU) is NOT ascending.  Waits for the device."""
+    with torch.cuda.device(idx_i.device):
+        flags = torch.empty(2, dtype=torch.int32, device=idx_i.device)
+        idx_i, idx_i_lr = idx_i.contiguous(), idx_i_lr.contiguous()
+        s = torch.cuda.current_stream(idx_i.device)
+        check(lib.so3lr_b200_lists_unsorted(C.c_void_p(s.cuda_stream), idx_i.numel(), _ptr(idx_i), idx_i_lr.numel(), _ptr(idx_i_lr),
+                                            _ptr(flags)), "lists_unsorted")
+        a, b = flags.tolist()
+    return bool(a), bool(b)
+
+
 NHC_STATE_DOUBLES = 18
 NHC_MAX_CHAIN = 8
 NPT_STATE_DOUBLES = 44
