@@ -1180,37 +1180,37 @@ int configure_attention_tc_kernels() {
 
 int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity) {
   if (n_rows + 1 > V->row_cap) {
-    if (V->row_ptr) cudaFree(V->row_ptr);
-    if (V->count) cudaFree(V->count);
+    if (V->row_ptr) dev_free(V->row_ptr);
+    if (V->count) dev_free(V->count);
     V->row_ptr = nullptr; V->count = nullptr;
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&V->row_ptr, ((size_t)n_rows + 1) * sizeof(int)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&V->count, ((size_t)n_rows + 1) * sizeof(int)));
+    SO3LR_CUDA_CHECK(dev_alloc(&V->row_ptr, ((size_t)n_rows + 1)));
+    SO3LR_CUDA_CHECK(dev_alloc(&V->count, ((size_t)n_rows + 1)));
     V->row_cap = n_rows + 1;
     size_t need = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, need, V->count, V->row_ptr, n_rows);
     if (need > V->cub_bytes) {
-      if (V->cub_tmp) cudaFree(V->cub_tmp);
+      if (V->cub_tmp) dev_free(V->cub_tmp);
       V->cub_tmp = nullptr;
-      SO3LR_CUDA_CHECK(cudaMalloc(&V->cub_tmp, need));
+      SO3LR_CUDA_CHECK(dev_alloc_bytes(&V->cub_tmp, need));
       V->cub_bytes = need;
     }
   }
   if (capacity > V->capacity) {
-    if (V->i) cudaFree(V->i);
-    if (V->j) cudaFree(V->j);
-    if (V->d) cudaFree(V->d);
+    if (V->i) dev_free(V->i);
+    if (V->j) dev_free(V->j);
+    if (V->d) dev_free(V->d);
     V->i = V->j = nullptr; V->d = nullptr;
     if (capacity < 1) capacity = 1;
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&V->i, (size_t)capacity * sizeof(int)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&V->j, (size_t)capacity * sizeof(int)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&V->d, (size_t)capacity * sizeof(float4)));
+    SO3LR_CUDA_CHECK(dev_alloc(&V->i, (size_t)capacity));
+    SO3LR_CUDA_CHECK(dev_alloc(&V->j, (size_t)capacity));
+    SO3LR_CUDA_CHECK(dev_alloc(&V->d, (size_t)capacity));
     V->capacity = capacity;
   }
   return kOk;
 }
 
 void valid_edges_free(ValidEdges* V) {
-  cudaFree(V->row_ptr); cudaFree(V->count); cudaFree(V->i); cudaFree(V->j); cudaFree(V->d); cudaFree(V->orig); cudaFree(V->cub_tmp);
+  dev_free(V->row_ptr); dev_free(V->count); dev_free(V->i); dev_free(V->j); dev_free(V->d); dev_free(V->orig); dev_free(V->cub_tmp);
   *V = ValidEdges{};
 }
 
@@ -1218,9 +1218,9 @@ int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const in
   if (n_rows <= 0) return kOk;
   if (n_rows + 1 > V->row_cap) return kInvalidArgument;
   if (want_orig && V->orig_cap < V->capacity) {
-    if (V->orig) cudaFree(V->orig);
+    if (V->orig) dev_free(V->orig);
     V->orig = nullptr;
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&V->orig, (size_t)V->capacity * sizeof(int)));
+    SO3LR_CUDA_CHECK(dev_alloc(&V->orig, (size_t)V->capacity));
     V->orig_cap = V->capacity;
   }
   const int blocks = (n_rows + 7) / 8;

@@ -16,6 +16,8 @@ struct so3lr_b200_model {
   int device = 0;
   ModelDev M{};
   std::vector<void*> owned;
+  // host copies of the charge / spin embeddings' query rows [element][128] and keys [2][128]
+  std::vector<float> cs_q[2], cs_k[2];
 };
 
 namespace {
@@ -36,23 +38,42 @@ int first_unsupported_element(const int32_t* Z, int n) {
   return 0;
 }
 
-// tracked device allocation
+// Device arrays of one context.  `plan` sizes the arrays of a lambda's get() calls and takes one zeroed block for all of them (rows that
+// a domain-decomposed evaluation never writes -- outer ghost shells -- are still read and multiplied by zero cotangents: they must
+// hold finite numbers); later get() calls take a block each.
 struct Pool {
   std::vector<void*> ptrs;
   int status = kOk;
+  bool counting = false;
+  char* base = nullptr;
+  size_t used = 0, size = 0;
   template <typename T>
   T* get(size_t n) {
+    const size_t bytes = ((n ? n : 1) * sizeof(T) + 255) / 256 * 256;
+    if (counting) { used += bytes; return nullptr; }
+    if (base && used + bytes <= size) { T* p = reinterpret_cast<T*>(base + used); used += bytes; return p; }
+    void* p = block(bytes);
+    cudaStreamSynchronize(nullptr);      // the zeros are there before any stream touches the array
+    return reinterpret_cast<T*>(p);
+  }
+  void* block(size_t bytes) {
     void* p = nullptr;
-    if (n == 0) n = 1;
-    if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) { status = kCudaError; return nullptr; }
-    // rows that a domain-decomposed evaluation never writes (outer ghost shells) are still read and multiplied by zero
-    // cotangents: they must hold finite numbers
-    if (cudaMemset(p, 0, n * sizeof(T)) != cudaSuccess) status = kCudaError;
+    if (dev_alloc_bytes(&p, bytes) != cudaSuccess) { status = kCudaError; return nullptr; }
+    if (cudaMemset(p, 0, bytes) != cudaSuccess) status = kCudaError;
     ptrs.push_back(p);
-    return (T*)p;
+    return p;
+  }
+  template <typename F>
+  void plan(F&& arrays) {
+    counting = true; used = 0;
+    arrays();
+    counting = false; size = used; used = 0;
+    base = static_cast<char*>(block(size));
+    if (base) arrays();
+    base = nullptr; used = size = 0;
   }
   void release() {
-    for (void* p : ptrs) cudaFree(p);
+    for (void* p : ptrs) dev_free(p);
     ptrs.clear();
   }
 };
@@ -253,7 +274,8 @@ struct so3lr_b200_system {
   int n = 0, n_graphs = 1;
   int n_cap = 0;                 // atoms the per-atom arrays were allocated for
   int shells[4] = {0, 0, 0, 0};  // domain-decomposed evaluation: owned | + short-range ghosts | (unused) | all local atoms
-  SpeciesTables sp{};            // per-element-pair tables of the first layer
+  SpeciesTables sp{};            // per-element-pair tables of the first layer (built by the first evaluation that reads them)
+  std::vector<int> elements;     // the structure's elements while the tables are still to be built
   float* GV = nullptr;           // n_cap x 32 scratch of the tabulated first-layer reverse pass
   float *dd_gev2 = nullptr, *dd_gev_in = nullptr;   // ping-pong cotangents of ev between the layers of the reverse pass
   so3lr_b200_options opt{};
@@ -323,6 +345,7 @@ struct so3lr_b200_system {
   // host staging
   float *h_R = nullptr, *h_F = nullptr, *h_q = nullptr, *h_h = nullptr, *h_dip = nullptr;
   double* h_E = nullptr;
+  void* h_stage = nullptr;         // the pinned block that holds them
   float* d_Rstage = nullptr;
   cudaStream_t own_stream = nullptr;
   int64_t n_rebuilds = 0, n_launches = 0;
@@ -356,9 +379,9 @@ void fill(cudaStream_t s, float* p, size_t n, float v) {
 int ensure_edge_buffers(so3lr_b200_system* S, long long n_edges) {
   if (n_edges <= S->edge_cap) return valid_edges_reserve(&S->ve, S->n_cap, S->edge_cap);   // row arrays exist even without edges
   long long cap = n_edges + n_edges / 4 + 1024;
-  if (S->dR) cudaFree(S->dR);
+  if (S->dR) dev_free(S->dR);
   S->dR = nullptr;
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&S->dR, (size_t)cap * 3 * sizeof(float)));
+  SO3LR_CUDA_CHECK(dev_alloc(&S->dR, (size_t)cap * 3));
   S->edge_cap = cap;
   return valid_edges_reserve(&S->ve, S->n_cap, cap);
 }
@@ -768,68 +791,105 @@ int evaluate_fused(so3lr_b200_system* S, cudaStream_t st, const float* R, float*
 // so3lr/base_calculator.py:57-86).  Per graph and embedding: y_i = softplus(<query[Z_i], key[psi < 0]> / sqrt(128)),
 // a_i = psi * y_i / sum_graph y, e_i = a_i * value[psi < 0], output e + W1^T silu(W0^T silu(e)) (bias-free residual block).
 // They depend on the element, the graph's composition and psi only -- not on positions -- so they are evaluated once per
-// context, on the host in double precision, and folded into the initial features: x0 = (embed[Z] + charge + spin) / sqrt(3).
-// `out` receives per (graph, element) rows [n_graphs][119][128], already divided by sqrt(3); returns false when every psi is 0.
-bool charge_spin_rows(const ModelDev& M, int n, const int32_t* Z, int n_graphs, const std::vector<int>& gs, const float* total_charge,
-                      const float* num_unpaired, std::vector<float>* out, int* status) {
+// context, in double precision, and folded into the initial features: x0 = (embed[Z] + charge + spin) / sqrt(3).
+// The scalars a_i are formed on the host; a row (graph, element) of the output is one CTA of 128 threads (two 128 x 128 products,
+// 33 k multiply-adds: about 10 us for the dozen rows of a batch, where the same loops on the host took 0.3 ms a row).
+struct ChargeSpinRow {
+  double a[2];
+  int idx[2], z;
+};
+__global__ void __launch_bounds__(128) charge_spin_rows_kernel(ModelDev M, const ChargeSpinRow* __restrict__ rows, float* __restrict__ out) {
+  __shared__ double sh[kF];
+  const int o = threadIdx.x;
+  const ChargeSpinRow R = rows[blockIdx.x];
+  auto silu = [](double x) { return x / (1.0 + exp(-x)); };
+  float acc = 0.f;
+  for (int e = 0; e < 2; ++e) {
+    if (R.a[e] == 0.0) continue;
+    const double ev = R.a[e] * (double)M.cs_embed_v[e][R.idx[e] * kF + o];
+    double t = ev;
+    for (int w = 0; w < 2; ++w) {
+      const float* W = w == 0 ? M.cs_res0[e] : M.cs_res1[e];
+      sh[o] = silu(t);
+      __syncthreads();
+      double d = 0.0;
+      for (int c = 0; c < kF; ++c) d += sh[c] * (double)W[(size_t)c * kF + o];
+      __syncthreads();
+      t = d;
+    }
+    acc += (float)((ev + t) / sqrt(3.0));
+  }
+  out[(size_t)blockIdx.x * kF + o] = acc;
+}
+// initial features with the rows added: per atom (Z, row_of given: one structure of a batch after the other) or per element (Z = nullptr:
+// row r belongs to element rows[r].z)
+__global__ void __launch_bounds__(128) charge_spin_atoms_kernel(const float* __restrict__ embed, const int* __restrict__ Z, const int* __restrict__ row_of,
+                                                                const float* __restrict__ rows, float* __restrict__ x0) {
+  const int a = blockIdx.x, c = threadIdx.x, r = row_of[a];
+  x0[(size_t)a * kF + c] = embed[(size_t)Z[a] * kF + c] + (r >= 0 ? rows[(size_t)r * kF + c] : 0.f);
+}
+__global__ void __launch_bounds__(128) charge_spin_table_kernel(const ChargeSpinRow* __restrict__ list, const float* __restrict__ rows, float* __restrict__ embed) {
+  embed[(size_t)list[blockIdx.x].z * kF + threadIdx.x] += rows[(size_t)blockIdx.x * kF + threadIdx.x];
+}
+// rows of the charged / open-shell graphs, and per atom the row it takes (-1: none); false when every psi is 0
+bool charge_spin_scalars(const so3lr_b200_model& m, int n, const int32_t* Z, int n_graphs, const std::vector<int>& gs, const float* total_charge,
+                         const float* num_unpaired, std::vector<ChargeSpinRow>* rows, std::vector<int>* row_of) {
   bool any = false;
   for (int g = 0; g < n_graphs; ++g) any |= (total_charge && total_charge[g] != 0.f) || (num_unpaired && num_unpaired[g] != 0.f);
-  *status = kOk;
   if (!any) return false;
-  out->assign((size_t)n_graphs * kZEmbed * kF, 0.f);
-  std::vector<float> q((size_t)kZEmbed * kF), k(2 * kF), v(2 * kF), r0((size_t)kF * kF), r1((size_t)kF * kF);
-  auto silu = [](double x) { return x / (1.0 + std::exp(-x)); };
-  for (int e = 0; e < 2; ++e) {
-    const float* psi_all = e == 0 ? total_charge : num_unpaired;
-    if (!psi_all) continue;
-    bool used = false;
-    for (int g = 0; g < n_graphs; ++g) used |= psi_all[g] != 0.f;
-    if (!used) continue;
-    if (cudaMemcpy(q.data(), M.cs_embed_q[e], q.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(k.data(), M.cs_embed_k[e], k.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(v.data(), M.cs_embed_v[e], v.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(r0.data(), M.cs_res0[e], r0.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(r1.data(), M.cs_res1[e], r1.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) {
-      *status = kCudaError;
-      return false;
+  row_of->assign(n, -1);
+  for (int g = 0; g < n_graphs; ++g) {
+    const double psi[2] = {total_charge ? total_charge[g] : 0.0, num_unpaired ? num_unpaired[g] : 0.0};
+    if (psi[0] == 0.0 && psi[1] == 0.0) continue;
+    int row[kZEmbed];
+    for (int z = 0; z < kZEmbed; ++z) row[z] = -1;
+    const size_t first = rows->size();
+    for (int a = gs[g]; a < gs[g + 1]; ++a) {
+      int& r = row[Z[a]];
+      if (r < 0) { r = (int)rows->size(); rows->push_back(ChargeSpinRow{{0.0, 0.0}, {0, 0}, Z[a]}); }
+      (*row_of)[a] = r;
     }
-    for (int g = 0; g < n_graphs; ++g) {
-      const double psi = psi_all[g];
-      if (psi == 0.0) continue;
-      const int idx = psi < 0.0 ? 1 : 0;
-      double y[kZEmbed];
-      bool present[kZEmbed] = {};
-      for (int a = gs[g]; a < gs[g + 1]; ++a) present[Z[a]] = true;
-      for (int z = 0; z < kZEmbed; ++z) {
-        if (!present[z]) continue;
+    for (int e = 0; e < 2; ++e) {
+      if (psi[e] == 0.0) continue;
+      const int idx = psi[e] < 0.0 ? 1 : 0;
+      double y[kZEmbed], den = 0.0;
+      for (size_t r = first; r < rows->size(); ++r) {
+        const int z = (*rows)[r].z;
         double d = 0.0;
-        for (int c = 0; c < kF; ++c) d += (double)q[(size_t)z * kF + c] * (double)k[idx * kF + c];
+        for (int c = 0; c < kF; ++c) d += (double)m.cs_q[e][(size_t)z * kF + c] * (double)m.cs_k[e][idx * kF + c];
         d /= std::sqrt((double)kF);
         y[z] = d > 30.0 ? d : std::log1p(std::exp(d));
       }
-      double den = 0.0;
       for (int a = gs[g]; a < gs[g + 1]; ++a) den += y[Z[a]];
-      for (int z = 0; z < kZEmbed; ++z) {
-        if (!present[z]) continue;
-        const double a = psi * y[z] / den;
-        double ev[kF], t0[kF], t1[kF];
-        for (int c = 0; c < kF; ++c) ev[c] = a * (double)v[idx * kF + c];
-        for (int o = 0; o < kF; ++o) {
-          double acc = 0.0;
-          for (int c = 0; c < kF; ++c) acc += silu(ev[c]) * (double)r0[(size_t)c * kF + o];
-          t0[o] = acc;
-        }
-        for (int o = 0; o < kF; ++o) {
-          double acc = 0.0;
-          for (int c = 0; c < kF; ++c) acc += silu(t0[c]) * (double)r1[(size_t)c * kF + o];
-          t1[o] = acc;
-        }
-        float* row = out->data() + ((size_t)g * kZEmbed + z) * kF;
-        for (int c = 0; c < kF; ++c) row[c] += (float)((ev[c] + t1[c]) / std::sqrt(3.0));
+      for (size_t r = first; r < rows->size(); ++r) {
+        (*rows)[r].a[e] = psi[e] * y[(*rows)[r].z] / den;
+        (*rows)[r].idx[e] = idx;
       }
     }
   }
   return true;
+}
+
+// tables of the first layer, built when the first evaluation that reads them comes (a graph-level context never does)
+int ensure_species_tables(so3lr_b200_system* S, cudaStream_t st) {
+  if (S->elements.empty()) return kOk;
+  const int rc = species_tables_build(st, S->mctx, S->elements.data(), (int)S->elements.size(), &S->sp);
+  if (rc == kOk) S->elements.clear();
+  return rc;
+}
+
+// pinned buffers of the host-buffer call, taken when it is first used
+int ensure_host_staging(so3lr_b200_system* S) {
+  if (S->h_stage) return kOk;
+  const size_t n = (size_t)S->n_cap, g = (size_t)S->n_graphs;
+  char* p = nullptr;
+  SO3LR_CUDA_CHECK(host_alloc(&p, g * sizeof(double) + (8 * n + 3 * g) * sizeof(float)));
+  S->h_stage = p;
+  S->h_E = reinterpret_cast<double*>(p);
+  S->h_R = reinterpret_cast<float*>(p + g * sizeof(double));
+  S->h_F = S->h_R + 3 * n; S->h_q = S->h_F + 3 * n; S->h_h = S->h_q + n; S->h_dip = S->h_h + n;
+  SO3LR_CUDA_CHECK(cudaStreamCreateWithFlags(&S->own_stream, cudaStreamNonBlocking));
+  return kOk;
 }
 
 }  // namespace
@@ -862,6 +922,13 @@ SO3LR_B200_API int so3lr_b200_model_create(const float* blob_host, size_t n_floa
   so3lr_b200_model* m = new so3lr_b200_model();
   m->device = device;
   int rc = build_model(blob_host, n_floats, &m->M, &m->owned);
+  if (rc == kOk) {
+    const BlobOffsets O = blob_offsets();
+    for (int e = 0; e < 2; ++e) {
+      m->cs_q[e].assign(blob_host + O.cs[e].embed_q, blob_host + O.cs[e].embed_q + (size_t)kZEmbed * kF);
+      m->cs_k[e].assign(blob_host + O.cs[e].embed_k, blob_host + O.cs[e].embed_k + 2 * kF);
+    }
+  }
   if (rc == kOk) rc = configure_atom_kernels();
   if (rc == kOk) rc = configure_attention_kernels();
   if (rc == kOk) rc = configure_attention_sym_kernels();
@@ -878,6 +945,7 @@ SO3LR_B200_API int so3lr_b200_model_destroy(so3lr_b200_model* m) {
   if (!m) return kOk;
   cudaSetDevice(m->device);
   for (void* p : m->owned) cudaFree(p);
+  devmem_flush(m->device);
   delete m;
   return kOk;
 }
@@ -910,92 +978,98 @@ SO3LR_B200_API int so3lr_b200_system_create(so3lr_b200_model* model, int n_atoms
   P.k_alpha = 0.f;
   set_coulomb_shift(P);
   const int n = n_atoms;
-  Pool& A = S->pool;
-  S->d_Z0 = A.get<int>(n); S->d_Zs = A.get<int>(n); S->d_Z = S->d_Z0; S->d_perm = A.get<int>(n);
-  S->d_Rs = A.get<float>((size_t)n * 3); S->F_s = A.get<float>((size_t)n * 3);
-  S->u_e_atom = A.get<float>(n); S->u_q = A.get<float>(n); S->u_h = A.get<float>(n);
-  S->u_zbl = A.get<float>(n); S->u_coul = A.get<float>(n); S->u_disp = A.get<float>(n);
-  S->d_seg = A.get<int>(n); S->d_graph_start = A.get<int>(n_graphs + 1);
-  S->d_total_charge = A.get<float>(n_graphs);
-  std::vector<int> gs(n_graphs + 1), seg(n);
+  // the element of every atom, its graph, the graphs' first atoms, total charges and (charged structures) embedding rows travel in one copy
+  std::vector<int> gs(n_graphs + 1);
   if (graph_start) { for (int g = 0; g <= n_graphs; ++g) gs[g] = graph_start[g]; }
   else { gs[0] = 0; gs[1] = n; }
-  if (gs[0] != 0 || gs[n_graphs] != n) { A.release(); delete S; return kInvalidArgument; }
-  for (int g = 0; g < n_graphs; ++g) {
-    if (gs[g + 1] < gs[g]) { A.release(); delete S; return kInvalidArgument; }
-    for (int a = gs[g]; a < gs[g + 1]; ++a) seg[a] = g;
-  }
-  std::vector<float> tq(n_graphs, 0.f);
-  if (total_charge) for (int g = 0; g < n_graphs; ++g) tq[g] = total_charge[g];
-  S->d_Rref = A.get<float>((size_t)n * 3); S->d_flag = A.get<int>(4);
-  S->d_rowptr_g = A.get<int>((size_t)n + 1); S->d_rowptr_lr_g = A.get<int>((size_t)n + 1);
-  for (int l = 0; l <= kNumLayers; ++l) { S->x[l] = A.get<float>((size_t)n * kF); S->ev[l] = A.get<float>((size_t)n * kMTot); }
-  for (int l = 0; l < kNumLayers; ++l) {
-    S->qkv[l] = A.get<float>((size_t)n * kProj); S->xa[l] = A.get<float>((size_t)n * kF); S->ev1[l] = A.get<float>((size_t)n * kMTot);
-    S->z1[l] = A.get<float>((size_t)n * kF); S->x3[l] = A.get<float>((size_t)n * kF); S->gate[l] = A.get<float>((size_t)n * 4);
-  }
-  S->ze = A.get<float>((size_t)n * kF); S->zq = A.get<float>((size_t)n * kF); S->zh = A.get<float>((size_t)n * 64);
-  S->e_nn = A.get<float>(n); S->q_raw = A.get<float>(n); S->hv = A.get<float>(n); S->q = A.get<float>(n); S->h = A.get<float>(n);
-  S->e_atom = A.get<float>(n); S->e_zbl = A.get<float>(n); S->e_coul = A.get<float>(n); S->e_disp = A.get<float>(n);
-  S->gq = A.get<float>(n); S->gh = A.get<float>(n); S->gq_raw = A.get<float>(n); S->ones = A.get<float>(n);
-  S->pair_pack = A.get<float>((size_t)n * 12);
-  S->g4 = A.get<float>((size_t)n * kF); S->g_xa = A.get<float>((size_t)n * kF);
-  S->gev_a = A.get<float>((size_t)n * kMTot); S->gev_b = A.get<float>((size_t)n * kMTot); S->gev1 = A.get<float>((size_t)n * kMTot);
-  S->g_qkv = A.get<float>((size_t)n * kProj);
-  S->F_int = A.get<float>((size_t)n * 3);
-  S->GV = A.get<float>((size_t)n * 4 * kMaxTabSpecies);
-  S->d_energy = A.get<double>(n_graphs); S->d_dipole = A.get<float>((size_t)n_graphs * 3);
-  S->red_scratch = A.get<double>(4 * 296);
-  S->d_Rstage = A.get<float>((size_t)n * 3);
-  if (A.status != kOk) { A.release(); delete S; return A.status; }
-  bool ok = cudaMemcpy(S->d_Z0, Z, (size_t)n * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-            cudaMemcpy(S->d_seg, seg.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-            cudaMemcpy(S->d_graph_start, gs.data(), (size_t)(n_graphs + 1) * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-            cudaMemcpy(S->d_total_charge, tq.data(), (size_t)n_graphs * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess &&
-            cudaMemset(S->ev[0], 0, (size_t)n * kMTot * sizeof(float)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_flag, 2 * sizeof(int)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_R, (size_t)n * 3 * sizeof(float)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_F, (size_t)n * 3 * sizeof(float)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_q, (size_t)n * sizeof(float)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_h, (size_t)n * sizeof(float)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_dip, (size_t)n_graphs * 3 * sizeof(float)) == cudaSuccess &&
-            cudaMallocHost((void**)&S->h_E, (size_t)n_graphs * sizeof(double)) == cudaSuccess &&
-            cudaStreamCreateWithFlags(&S->own_stream, cudaStreamNonBlocking) == cudaSuccess;
-  if (!ok) { so3lr_b200_system_destroy(S); return kCudaError; }
-  fill(nullptr, S->ones, n, 1.f);
-  {
-    // charge / spin embeddings: per-element table for one structure, per-atom rows for a batch
-    std::vector<float> rows;
-    int cs_status = kOk;
-    const bool charged = charge_spin_rows(model->M, n, Z, n_graphs, gs, total_charge, num_unpaired, &rows, &cs_status);
-    if (cs_status != kOk) { so3lr_b200_system_destroy(S); return cs_status; }
+  if (gs[0] != 0 || gs[n_graphs] != n) { delete S; return kInvalidArgument; }
+  for (int g = 0; g < n_graphs; ++g)
+    if (gs[g + 1] < gs[g]) { delete S; return kInvalidArgument; }
+  std::vector<ChargeSpinRow> cs_rows;
+  std::vector<int> cs_row_of;
+  const bool charged = charge_spin_scalars(*model, n, Z, n_graphs, gs, total_charge, num_unpaired, &cs_rows, &cs_row_of);
+  Pool& A = S->pool;
+  int *d_row_of = nullptr;
+  ChargeSpinRow* d_rows = nullptr;
+  float *d_row_out = nullptr, *d_table = nullptr;
+  A.plan([&] {
+    // first the arrays of the upload, in this order
+    S->d_Z0 = A.get<int>(n); S->d_seg = A.get<int>(n); S->d_graph_start = A.get<int>(n_graphs + 1);
+    S->d_total_charge = A.get<float>(n_graphs);
+    if (charged) { d_rows = A.get<ChargeSpinRow>(cs_rows.size()); if (n_graphs > 1) d_row_of = A.get<int>(n); }
     if (charged) {
-      std::vector<float> base((size_t)kZEmbed * kF);
-      if (cudaMemcpy(base.data(), model->M.embed_z, base.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) {
-        so3lr_b200_system_destroy(S); return kCudaError;
-      }
-      if (n_graphs == 1) {
-        for (size_t k = 0; k < base.size(); ++k) base[k] += rows[k];
-        float* d = S->pool.get<float>(base.size());
-        if (!d || cudaMemcpy(d, base.data(), base.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
-          so3lr_b200_system_destroy(S); return kCudaError;
-        }
-        S->mctx.embed_z = d;
-      } else {
-        std::vector<float> x0((size_t)n * kF);
-        for (int a = 0; a < n; ++a)
-          for (int c = 0; c < kF; ++c)
-            x0[(size_t)a * kF + c] = base[(size_t)Z[a] * kF + c] + rows[((size_t)seg[a] * kZEmbed + Z[a]) * kF + c];
-        S->x0_atom = S->pool.get<float>(x0.size());
-        if (!S->x0_atom || cudaMemcpy(S->x0_atom, x0.data(), x0.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
-          so3lr_b200_system_destroy(S); return kCudaError;
-        }
-      }
+      d_row_out = A.get<float>(cs_rows.size() * kF);
+      if (n_graphs > 1) S->x0_atom = A.get<float>((size_t)n * kF); else d_table = A.get<float>((size_t)kZEmbed * kF);
+    }
+    S->d_Zs = A.get<int>(n); S->d_perm = A.get<int>(n);
+    S->d_Rs = A.get<float>((size_t)n * 3); S->F_s = A.get<float>((size_t)n * 3);
+    S->u_e_atom = A.get<float>(n); S->u_q = A.get<float>(n); S->u_h = A.get<float>(n);
+    S->u_zbl = A.get<float>(n); S->u_coul = A.get<float>(n); S->u_disp = A.get<float>(n);
+    S->d_Rref = A.get<float>((size_t)n * 3); S->d_flag = A.get<int>(4);
+    S->d_rowptr_g = A.get<int>((size_t)n + 1); S->d_rowptr_lr_g = A.get<int>((size_t)n + 1);
+    for (int l = 0; l <= kNumLayers; ++l) { S->x[l] = A.get<float>((size_t)n * kF); S->ev[l] = A.get<float>((size_t)n * kMTot); }
+    for (int l = 0; l < kNumLayers; ++l) {
+      S->qkv[l] = A.get<float>((size_t)n * kProj); S->xa[l] = A.get<float>((size_t)n * kF); S->ev1[l] = A.get<float>((size_t)n * kMTot);
+      S->z1[l] = A.get<float>((size_t)n * kF); S->x3[l] = A.get<float>((size_t)n * kF); S->gate[l] = A.get<float>((size_t)n * 4);
+    }
+    S->ze = A.get<float>((size_t)n * kF); S->zq = A.get<float>((size_t)n * kF); S->zh = A.get<float>((size_t)n * 64);
+    S->e_nn = A.get<float>(n); S->q_raw = A.get<float>(n); S->hv = A.get<float>(n); S->q = A.get<float>(n); S->h = A.get<float>(n);
+    S->e_atom = A.get<float>(n); S->e_zbl = A.get<float>(n); S->e_coul = A.get<float>(n); S->e_disp = A.get<float>(n);
+    S->gq = A.get<float>(n); S->gh = A.get<float>(n); S->gq_raw = A.get<float>(n); S->ones = A.get<float>(n);
+    S->pair_pack = A.get<float>((size_t)n * 12);
+    S->g4 = A.get<float>((size_t)n * kF); S->g_xa = A.get<float>((size_t)n * kF);
+    S->gev_a = A.get<float>((size_t)n * kMTot); S->gev_b = A.get<float>((size_t)n * kMTot); S->gev1 = A.get<float>((size_t)n * kMTot);
+    S->g_qkv = A.get<float>((size_t)n * kProj);
+    S->F_int = A.get<float>((size_t)n * 3);
+    S->GV = A.get<float>((size_t)n * 4 * kMaxTabSpecies);
+    S->d_energy = A.get<double>(n_graphs); S->d_dipole = A.get<float>((size_t)n_graphs * 3);
+    S->red_scratch = A.get<double>(4 * 296);
+    S->d_Rstage = A.get<float>((size_t)n * 3);
+  });
+  if (A.status != kOk) { A.release(); delete S; return A.status; }
+  S->d_Z = S->d_Z0;
+  {
+    std::vector<char> up;
+    auto append = [&](const void* src, size_t bytes) {
+      const size_t at = up.size();
+      up.resize(at + (bytes + 255) / 256 * 256);
+      std::memcpy(up.data() + at, src, bytes);
+    };
+    std::vector<int> seg(n);
+    for (int g = 0; g < n_graphs; ++g)
+      for (int a = gs[g]; a < gs[g + 1]; ++a) seg[a] = g;
+    std::vector<float> tq(n_graphs, 0.f);
+    if (total_charge) for (int g = 0; g < n_graphs; ++g) tq[g] = total_charge[g];
+    append(Z, (size_t)n * sizeof(int)); append(seg.data(), (size_t)n * sizeof(int)); append(gs.data(), gs.size() * sizeof(int));
+    append(tq.data(), tq.size() * sizeof(float));
+    if (charged) { append(cs_rows.data(), cs_rows.size() * sizeof(ChargeSpinRow)); if (n_graphs > 1) append(cs_row_of.data(), (size_t)n * sizeof(int)); }
+    if (cudaMemcpy(S->d_Z0, up.data(), up.size(), cudaMemcpyHostToDevice) != cudaSuccess || host_alloc(&S->h_flag, 2) != cudaSuccess) {
+      so3lr_b200_system_destroy(S);
+      return kCudaError;
     }
   }
+  fill(nullptr, S->ones, n, 1.f);
+  if (charged) {
+    // charge / spin embeddings: per-element table for one structure, per-atom rows for a batch
+    const unsigned nr = (unsigned)cs_rows.size();
+    charge_spin_rows_kernel<<<nr, 128>>>(model->M, d_rows, d_row_out);
+    if (n_graphs == 1) {
+      cudaMemcpyAsync(d_table, model->M.embed_z, (size_t)kZEmbed * kF * sizeof(float), cudaMemcpyDeviceToDevice, nullptr);
+      charge_spin_table_kernel<<<nr, 128>>>(d_rows, d_row_out, d_table);
+      S->mctx.embed_z = d_table;
+    } else {
+      charge_spin_atoms_kernel<<<(unsigned)n, 128>>>(model->M.embed_z, S->d_Z0, d_row_of, d_row_out, S->x0_atom);
+    }
+    count_launch(2);
+  }
   // a batch with per-atom initial features cannot use the per-element-pair tables of the first layer
-  if (!S->x0_atom && species_tables_build(nullptr, S->mctx, Z, n, &S->sp) != kOk) { so3lr_b200_system_destroy(S); return kCudaError; }
-  cudaDeviceSynchronize();
+  if (!S->x0_atom) {
+    bool seen[kMaxZ + 1] = {};
+    for (int a = 0; a < n; ++a) seen[Z[a]] = true;
+    for (int z = 1; z <= kMaxZ; ++z)
+      if (seen[z]) S->elements.push_back(z);
+  }
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) { so3lr_b200_system_destroy(S); return kCudaError; }
   S->nws = nlist_workspace_create();
   *out = S;
   return kOk;
@@ -1005,7 +1079,7 @@ SO3LR_B200_API int so3lr_b200_system_destroy(so3lr_b200_system* S) {
   if (!S) return kOk;
   if (tl_launch_counter == &S->n_launches) tl_launch_counter = nullptr;
   cudaSetDevice(S->model->device);
-  cudaDeviceSynchronize();
+  DevFreeBatch idle;      // the device is idle from here on
   tc_debug_print();
   dense_debug_print();
   drop_step_graph(S);
@@ -1014,19 +1088,11 @@ SO3LR_B200_API int so3lr_b200_system_destroy(so3lr_b200_system* S) {
   species_tables_free(&S->sp);
   S->prof.destroy();
   nlist_workspace_destroy(S->nws);
-  for (NeighborListDev* L : {&S->sr, &S->lrl}) { cudaFree(L->row_ptr); cudaFree(L->nbr_j); cudaFree(L->edge_i); }
-  cudaFree(S->dR);
+  for (NeighborListDev* L : {&S->sr, &S->lrl}) { dev_free(L->row_ptr); dev_free(L->nbr_j); dev_free(L->edge_i); }
+  dev_free(S->dR);
   valid_edges_free(&S->ve);
-  if (S->h_flag) cudaFreeHost(S->h_flag);
-  if (S->h_flag2) cudaFreeHost(S->h_flag2);
   for (int k = 0; k < 2; ++k) if (S->flag_event[k]) cudaEventDestroy(S->flag_event[k]);
-  if (S->h_box) cudaFreeHost(S->h_box);
-  if (S->h_R) cudaFreeHost(S->h_R);
-  if (S->h_F) cudaFreeHost(S->h_F);
-  if (S->h_q) cudaFreeHost(S->h_q);
-  if (S->h_h) cudaFreeHost(S->h_h);
-  if (S->h_dip) cudaFreeHost(S->h_dip);
-  if (S->h_E) cudaFreeHost(S->h_E);
+  host_free(S->h_flag); host_free(S->h_flag2); host_free(S->h_box); host_free(S->h_stage);
   if (S->own_stream) cudaStreamDestroy(S->own_stream);
   delete S;
   return kOk;
@@ -1071,7 +1137,7 @@ SO3LR_B200_API int so3lr_b200_system_defer_skin_test(so3lr_b200_system* S, int e
   if (!S || !(margin >= 0.f)) return kInvalidArgument;
   SO3LR_CUDA_CHECK(cudaSetDevice(S->model->device));
   if (enable && !S->h_flag2) {
-    SO3LR_CUDA_CHECK(cudaMallocHost((void**)&S->h_flag2, 4 * sizeof(int)));
+    SO3LR_CUDA_CHECK(host_alloc(&S->h_flag2, 4));
     for (int k = 0; k < 2; ++k) SO3LR_CUDA_CHECK(cudaEventCreateWithFlags(&S->flag_event[k], cudaEventDisableTiming));
   }
   S->deferred_skin = enable != 0;
@@ -1144,7 +1210,9 @@ SO3LR_B200_API int so3lr_b200_system_compute(so3lr_b200_system* S, void* stream,
   tl_launch_counter = &S->n_launches;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t rebuilds_before = S->n_rebuilds;
-  int rc = prepare_lists(S, st, R);
+  int rc = ensure_species_tables(S, st);
+  if (rc) return rc;
+  rc = prepare_lists(S, st, R);
   if (rc) return rc;
   float* Fout = F ? F : S->F_int;
   const int n = S->n;
@@ -1238,11 +1306,13 @@ SO3LR_B200_API int so3lr_b200_system_compute_host(so3lr_b200_system* S, const fl
   if (!S || !R_host) return kInvalidArgument;
   SO3LR_CUDA_CHECK(cudaSetDevice(S->model->device));
   tl_launch_counter = &S->n_launches;
+  int rc = ensure_host_staging(S);
+  if (rc) return rc;
   cudaStream_t st = S->own_stream;
   const int n = S->n;
   std::memcpy(S->h_R, R_host, (size_t)n * 3 * sizeof(float));
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->d_Rstage, S->h_R, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, st));
-  int rc = so3lr_b200_system_compute(S, st, S->d_Rstage, S->F_int, nullptr, nullptr, nullptr, nullptr, nullptr);
+  rc = so3lr_b200_system_compute(S, st, S->d_Rstage, S->F_int, nullptr, nullptr, nullptr, nullptr, nullptr);
   if (rc) return rc;
   if (F_host) SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->h_F, S->F_int, (size_t)n * 3 * sizeof(float), cudaMemcpyDeviceToHost, st));
   if (E_host) SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->h_E, S->d_energy, (size_t)S->n_graphs * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1541,7 +1611,7 @@ SO3LR_B200_API int so3lr_b200_system_npt(so3lr_b200_system* S, void* stream, int
     S->ke_partials = S->pool.get<double>((size_t)(S->n_cap + 255) / 256);
     if (!S->ke_partials) return kCudaError;
   }
-  if (!S->h_box && cudaMallocHost((void**)&S->h_box, sizeof(double)) != cudaSuccess) return kCudaError;
+  if (!S->h_box && host_alloc(&S->h_box, 1) != cudaSuccess) return kCudaError;
   double h0[9];
   for (int k = 0; k < 9; ++k) h0[k] = cell0_9[k];
   const double V0 = std::fabs(h0[0] * (h0[4] * h0[8] - h0[5] * h0[7]) - h0[1] * (h0[3] * h0[8] - h0[5] * h0[6]) +
@@ -1616,6 +1686,7 @@ SO3LR_B200_API int so3lr_b200_dd_set_atoms(so3lr_b200_system* S, int n_local, co
       std::fprintf(stderr, "so3lr_b200: atomic number %d is outside the supported range 1..%d\n", bad == -1 ? 0 : bad, kMaxZ);
       return kInvalidArgument;
     }
+    S->elements.clear();
     rc = species_tables_build(nullptr, S->mctx, zh.data(), n_local, &S->sp);
     if (rc) return rc;
     SO3LR_CUDA_CHECK(cudaDeviceSynchronize());

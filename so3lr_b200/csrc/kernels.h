@@ -4,6 +4,21 @@
 
 namespace so3lr {
 
+// ---- devmem.cu: cached device / pinned host blocks of evaluation contexts (not cleared; safe with several threads) ----
+cudaError_t dev_alloc_bytes(void** p, size_t bytes);
+void dev_free(void* p);            // waits for the device first, like cudaFree, unless a DevFreeBatch is alive on this thread
+cudaError_t host_alloc_bytes(void** p, size_t bytes);
+void host_free(void* p);
+void devmem_flush(int device);     // gives the idle blocks back
+template <typename T>
+cudaError_t dev_alloc(T** p, size_t n) { return dev_alloc_bytes(reinterpret_cast<void**>(p), (n ? n : 1) * sizeof(T)); }
+template <typename T>
+cudaError_t host_alloc(T** p, size_t n) { return host_alloc_bytes(reinterpret_cast<void**>(p), (n ? n : 1) * sizeof(T)); }
+struct DevFreeBatch {              // one wait for all the frees of a scope
+  DevFreeBatch();
+  ~DevFreeBatch();
+};
+
 // ---- atom_kernels.cu ----
 int configure_atom_kernels();
 void launch_embed(cudaStream_t s, const ModelDev& M, const int* Z, int n, float* x);

@@ -432,7 +432,7 @@ void kspace_free(KSpaceDev* K) {
   if (K->plans) {
     if (CufftApi* f = cufft_api()) { f->destroy(K->plan_r2c); f->destroy(K->plan_c2r); }
   }
-  cudaFree(K->tiles); cudaFree(K->groups); cudaFree(K->wgt); cudaFree(K->Sk); cudaFree(K->acc); cudaFree(K->mesh); cudaFree(K->fq);
+  dev_free(K->tiles); dev_free(K->groups); dev_free(K->wgt); dev_free(K->Sk); dev_free(K->acc); dev_free(K->mesh); dev_free(K->fq);
   *K = KSpaceDev{};
 }
 
@@ -442,9 +442,9 @@ static int kspace_setup_mesh(KSpaceDev* K, int n_atoms, float smearing, int n1, 
   if (!f) return kCudaError;
   K->smearing = smearing;
   K->shape[0] = n1; K->shape[1] = n2; K->shape[2] = n3;
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->mesh, (size_t)n1 * n2 * n3 * sizeof(float)));
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->fq, (size_t)n1 * n2 * (n3 / 2 + 1) * sizeof(float2)));
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->acc, (size_t)n_atoms * 4 * sizeof(float)));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->mesh, (size_t)n1 * n2 * n3));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->fq, (size_t)n1 * n2 * (n3 / 2 + 1)));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->acc, (size_t)n_atoms * 4));
   if (f->plan3d(&K->plan_r2c, n1, n2, n3, CUFFT_R2C) != CUFFT_SUCCESS) return kCudaError;
   if (f->plan3d(&K->plan_c2r, n1, n2, n3, CUFFT_C2R) != CUFFT_SUCCESS) { f->destroy(K->plan_r2c); return kCudaError; }
   K->plans = true;
@@ -505,11 +505,11 @@ int kspace_setup(KSpaceDev* K, int n_atoms, int mode, float smearing, int n1, in
   K->n_groups = (int)groups.size();
   K->smearing = smearing;
   K->shape[0] = n1; K->shape[1] = n2; K->shape[2] = n3;
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->tiles, tiles.size() * sizeof(int4)));
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->wgt, wgt.size() * sizeof(float)));
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->Sk, wgt.size() * sizeof(float2)));
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->acc, (size_t)n_atoms * 4 * sizeof(float)));
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&K->groups, groups.size() * sizeof(int2)));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->tiles, tiles.size()));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->wgt, wgt.size()));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->Sk, wgt.size()));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->acc, (size_t)n_atoms * 4));
+  SO3LR_CUDA_CHECK(dev_alloc(&K->groups, groups.size()));
   SO3LR_CUDA_CHECK(cudaMemcpy(K->groups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice));
   SO3LR_CUDA_CHECK(cudaMemcpy(K->tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
   SO3LR_CUDA_CHECK(cudaMemcpy(K->wgt, wgt.data(), wgt.size() * sizeof(float), cudaMemcpyHostToDevice));

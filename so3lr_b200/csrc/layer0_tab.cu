@@ -65,13 +65,15 @@ __device__ __forceinline__ float warp_transpose_reduce32(float (&v)[32], int lan
 }
 
 // table[(a * SP + b)][interval][32]: the four interval rows of the radial table (value, slope, value difference, far
-// slope) contracted with q_a * k_b per head: entry 8 * row + 4 * filter + head.  Sums are formed in double precision.
+// slope) contracted with q_a * k_b per head: entry 8 * row + 4 * filter + head.  Sums are formed in double precision.  The intervals
+// are spread over kTableSplit CTAs per element pair: with one CTA a water box (4 pairs) used 4 SMs and took 0.81 ms.
+constexpr int kTableSplit = 32;
 __global__ void build_pair_table_kernel(const float* __restrict__ radial, const float* __restrict__ qkv_sp, int n_sp,
                                         float* __restrict__ table) {
-  const int a = blockIdx.x / n_sp, b = blockIdx.x % n_sp;
+  const int a = blockIdx.y / n_sp, b = blockIdx.y % n_sp;
   const float* qa = qkv_sp + (size_t)a * kProj;
   const float* kb = qkv_sp + (size_t)b * kProj;
-  for (int idx = threadIdx.x; idx < (kTableGrid - 1) * 32; idx += blockDim.x) {
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < (kTableGrid - 1) * 32; idx += gridDim.x * blockDim.x) {
     const int iv = idx >> 5, o = idx & 31;
     const int grp = o & 3, filt = (o >> 2) & 1, row = o >> 3;
     const float* w = radial + ((size_t)iv * 4 + row) * 256 + filt * kF + 32 * grp;
@@ -288,12 +290,12 @@ int species_tables_build(cudaStream_t st, const ModelDev& M, const int* Z_host, 
   for (int k = 0; same && k < (int)sp.size(); ++k) same = T->species[k] == sp[k];
   if (same && T->table) return kOk;
   if (!T->table) {
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&T->table, (size_t)SP * SP * (kTableGrid - 1) * 32 * sizeof(float)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&T->v_sp, (size_t)SP * kF * sizeof(float)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&T->slot, 119 * sizeof(int)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&T->qkv_sp, (size_t)SP * kProj * sizeof(float)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&T->x_sp, (size_t)SP * kF * sizeof(float)));
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&T->z_sp, SP * sizeof(int)));
+    SO3LR_CUDA_CHECK(dev_alloc(&T->table, (size_t)SP * SP * (kTableGrid - 1) * 32));
+    SO3LR_CUDA_CHECK(dev_alloc(&T->v_sp, (size_t)SP * kF));
+    SO3LR_CUDA_CHECK(dev_alloc(&T->slot, 119));
+    SO3LR_CUDA_CHECK(dev_alloc(&T->qkv_sp, (size_t)SP * kProj));
+    SO3LR_CUDA_CHECK(dev_alloc(&T->x_sp, (size_t)SP * kF));
+    SO3LR_CUDA_CHECK(dev_alloc(&T->z_sp, SP));
   }
   const int ns = (int)sp.size();
   int slot[119];
@@ -307,13 +309,13 @@ int species_tables_build(cudaStream_t st, const ModelDev& M, const int* Z_host, 
   launch_proj_fwd(st, M.layer[0], T->x_sp, ns, T->qkv_sp);
   SO3LR_CUDA_CHECK(cudaMemcpy2DAsync(T->v_sp, kF * sizeof(float), T->qkv_sp + 2 * kF, kProj * sizeof(float), kF * sizeof(float), ns,
                                      cudaMemcpyDeviceToDevice, st));
-  { build_pair_table_kernel<<<ns * ns, 256, 0, st>>>(M.layer[0].table, T->qkv_sp, ns, T->table); count_launch(); }
+  { build_pair_table_kernel<<<dim3(kTableSplit, ns * ns), 256, 0, st>>>(M.layer[0].table, T->qkv_sp, ns, T->table); count_launch(); }
   SO3LR_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
 
 void species_tables_free(SpeciesTables* T) {
-  cudaFree(T->table); cudaFree(T->v_sp); cudaFree(T->slot); cudaFree(T->qkv_sp); cudaFree(T->x_sp); cudaFree(T->z_sp);
+  dev_free(T->table); dev_free(T->v_sp); dev_free(T->slot); dev_free(T->qkv_sp); dev_free(T->x_sp); dev_free(T->z_sp);
   *T = SpeciesTables{};
 }
 

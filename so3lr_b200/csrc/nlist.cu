@@ -35,10 +35,10 @@ struct NlistWorkspace {
 NlistWorkspace* nlist_workspace_create() { return new NlistWorkspace(); }
 void nlist_workspace_destroy(NlistWorkspace* w) {
   if (!w) return;
-  cudaFree(w->cell_of); cudaFree(w->cell_sorted); cudaFree(w->atom_sorted); cudaFree(w->atom_iota);
-  cudaFree(w->cell_start); cudaFree(w->row_count); cudaFree(w->cub_tmp); cudaFree(w->d_total);
-  cudaFree(w->key); cudaFree(w->key_sorted); cudaFree(w->sort_tmp); cudaFree(w->pos_sorted);
-  if (w->h_total) cudaFreeHost(w->h_total);
+  dev_free(w->cell_of); dev_free(w->cell_sorted); dev_free(w->atom_sorted); dev_free(w->atom_iota);
+  dev_free(w->cell_start); dev_free(w->row_count); dev_free(w->cub_tmp); dev_free(w->d_total);
+  dev_free(w->key); dev_free(w->key_sorted); dev_free(w->sort_tmp); dev_free(w->pos_sorted);
+  if (w->h_total) host_free(w->h_total);
   delete w;
 }
 
@@ -231,9 +231,9 @@ __global__ void morton_keys_kernel(Cell cell, Grid G, int n, const float* __rest
 
 template <typename T>
 int ensure(T** p, size_t n) {
-  if (*p) cudaFree(*p);
+  if (*p) dev_free(*p);
   *p = nullptr;
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)p, n * sizeof(T)));
+  SO3LR_CUDA_CHECK(dev_alloc(p, n));
   return kOk;
 }
 
@@ -241,7 +241,7 @@ int ensure(T** p, size_t n) {
 
 int nlist_row_total(cudaStream_t s, int n, const int* row_count_dev, long long* total_host) {
   unsigned long long* d = nullptr;
-  SO3LR_CUDA_CHECK(cudaMalloc((void**)&d, sizeof(unsigned long long)));
+  SO3LR_CUDA_CHECK(dev_alloc(&d, 1));
   SO3LR_CUDA_CHECK(cudaMemsetAsync(d, 0, sizeof(unsigned long long), s));
   int tb = (n + 255) / 256;
   if (tb > 1024) tb = 1024;
@@ -249,7 +249,7 @@ int nlist_row_total(cudaStream_t s, int n, const int* row_count_dev, long long* 
   unsigned long long t = 0;
   cudaError_t e = cudaMemcpyAsync(&t, d, sizeof(t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(d);
+  dev_free(d);
   if (e != cudaSuccess) return kCudaError;
   *total_host = (long long)t;
   return t > 2147483000ULL ? kTooLarge : kOk;
@@ -286,9 +286,9 @@ int spatial_order(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, co
   size_t need = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, need, w->key, w->key_sorted, w->atom_iota, perm, n, 0, 30, s);
   if (need > w->sort_bytes) {
-    if (w->sort_tmp) cudaFree(w->sort_tmp);
+    if (w->sort_tmp) dev_free(w->sort_tmp);
     w->sort_tmp = nullptr;
-    SO3LR_CUDA_CHECK(cudaMalloc(&w->sort_tmp, need));
+    SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->sort_tmp, need));
     w->sort_bytes = need;
   }
   size_t tmp = w->sort_bytes;
@@ -313,13 +313,13 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     w->n_cap = n;
   }
   if (!w->d_total) {
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&w->d_total, sizeof(long long)));
-    SO3LR_CUDA_CHECK(cudaMallocHost((void**)&w->h_total, sizeof(long long)));
+    SO3LR_CUDA_CHECK(dev_alloc(&w->d_total, 1));
+    SO3LR_CUDA_CHECK(host_alloc(&w->h_total, 1));
   }
   if (n + 1 > out->row_cap) {
-    if (out->row_ptr) cudaFree(out->row_ptr);
+    if (out->row_ptr) dev_free(out->row_ptr);
     out->row_ptr = nullptr;
-    SO3LR_CUDA_CHECK(cudaMalloc((void**)&out->row_ptr, ((size_t)n + 1) * sizeof(int)));
+    SO3LR_CUDA_CHECK(dev_alloc(&out->row_ptr, ((size_t)n + 1)));
     out->row_cap = n + 1;
   }
   const float r2max = r_list * r_list;
@@ -371,8 +371,8 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     cub::DeviceScan::ExclusiveSum(nullptr, need2, w->row_count, out->row_ptr, n, s);   // sized for the largest row count
     if (need2 > need) need = need2;
     if (need > w->cub_bytes) {
-      if (w->cub_tmp) cudaFree(w->cub_tmp);
-      SO3LR_CUDA_CHECK(cudaMalloc(&w->cub_tmp, need));
+      if (w->cub_tmp) dev_free(w->cub_tmp);
+      SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->cub_tmp, need));
       w->cub_bytes = need;
     }
     size_t tmp = w->cub_bytes;
@@ -384,8 +384,8 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     size_t need = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, need, w->row_count, out->row_ptr, n, s);
     if (need > w->cub_bytes) {
-      if (w->cub_tmp) cudaFree(w->cub_tmp);
-      SO3LR_CUDA_CHECK(cudaMalloc(&w->cub_tmp, need));
+      if (w->cub_tmp) dev_free(w->cub_tmp);
+      SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->cub_tmp, need));
       w->cub_bytes = need;
     }
   }
@@ -412,11 +412,11 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
       out->count = out->capacity;   // rows are truncated; the overflow flag is set on the device
     } else {
       long long cap = total + total / 4 + 1024;
-      if (out->nbr_j) cudaFree(out->nbr_j);
-      if (out->edge_i) cudaFree(out->edge_i);
+      if (out->nbr_j) dev_free(out->nbr_j);
+      if (out->edge_i) dev_free(out->edge_i);
       out->nbr_j = nullptr; out->edge_i = nullptr;
-      SO3LR_CUDA_CHECK(cudaMalloc((void**)&out->nbr_j, (size_t)cap * sizeof(int)));
-      SO3LR_CUDA_CHECK(cudaMalloc((void**)&out->edge_i, (size_t)cap * sizeof(int)));
+      SO3LR_CUDA_CHECK(dev_alloc(&out->nbr_j, (size_t)cap));
+      SO3LR_CUDA_CHECK(dev_alloc(&out->edge_i, (size_t)cap));
       out->capacity = cap;
     }
   }
