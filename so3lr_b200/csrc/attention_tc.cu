@@ -1,8 +1,9 @@
 // Attention kernels of layers 1 and 2 as CTA-tiled tcgen05 kernels.
 //
-// A tile is 128 consecutive entries of the compacted short-range edge list (entries inside the 4.5 A cutoff only, grouped
-// by receiver).  Per tile and layer, both filters of all 128 edges come out of ONE chain of tcgen05.mma instructions with
-// the accumulators in tensor memory:
+// A tile is up to 128 consecutive entries of the compacted list of undirected pairs inside the 4.5 A cutoff, grouped by the end with
+// the smaller index (the "receiver" i; j is the partner).  Both filters depend on the pair only -- on its length and on the
+// invariants of the difference of the two `ev` rows -- so one evaluation serves (i <- j) and (j <- i), forward and reverse.  Per
+// tile and layer, both filters of all pairs come out of ONE chain of tcgen05.mma instructions with the accumulators in tensor memory:
 //
 //     w[e, 0:256] = Phi[e, 0:64] * C[0:64, 0:256]  +  hs_f[e, 0:32] * K2_f[0:32, 0:128]   (f = 0, 1)
 //
@@ -16,8 +17,11 @@
 //
 // After the MMA the filter tile is moved from tensor memory to shared memory (row = edge) and the edge loop runs in the
 // "lane = 4 features" layout of the other attention kernels: sender rows are read with coalesced 512-byte loads, logits are
-// 8-lane reductions.  A warp owns a run of consecutive edges and adds its partial sums to the receiver's row with vector
-// reductions in global memory (a receiver's edges can span warps, tiles and CTAs).
+// 8-lane reductions.  A warp owns a run of consecutive pairs and adds its partial sums to the receiver's row with vector
+// reductions in global memory (a receiver's pairs can span warps, tiles and CTAs); the partner's share of a pair goes out as one
+// reduction per row.  Those cost less than the second evaluation they replace: the L2 takes 5.4 TB/s of 512-byte row reductions
+// (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.  With every pair evaluated at
+// both ends instead, 98,304 atoms took 1.99 / 5.12 ms a launch (forward / reverse), with one evaluation 1.23 / 3.12 ms.
 //
 // The reverse kernel forms dw in the same loop, writes it straight into shared memory as the (FP16-split) A operand of a
 // second MMA chain against the SAME weight image read with the other major-ness,
@@ -28,6 +32,7 @@
 #include <cuda_fp16.h>
 #include <cub/cub.cuh>
 #include <cstdlib>
+#include <type_traits>
 
 #include "kernels.h"
 
@@ -82,6 +87,11 @@ __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); 
 __device__ __forceinline__ float4 f4_fma(float a, float4 b, float4 c) {
   const float2 a2 = make_float2(a, a);
   const float2 l = __ffma2_rn(a2, lo2(b), lo2(c)), h = __ffma2_rn(a2, hi2(b), hi2(c));
+  return make_float4(l.x, l.y, h.x, h.y);
+}
+__device__ __forceinline__ float4 f4_scale(float a, float4 b) {
+  const float2 a2 = make_float2(a, a);
+  const float2 l = __fmul2_rn(a2, lo2(b)), h = __fmul2_rn(a2, hi2(b));
   return make_float4(l.x, l.y, h.x, h.y);
 }
 __device__ __forceinline__ float4 f4_zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
@@ -154,20 +164,6 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-        "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
-}
 // main + cross / 2048 of 32 columns (cross accumulators sit 256 columns above the main ones)
 __device__ __forceinline__ void tmem_ld32_combined(uint32_t taddr, float* v) {
   uint32_t a[32], b[32];      // both loads in flight before the one wait
@@ -182,6 +178,26 @@ __device__ __forceinline__ void tmem_ld32_combined(uint32_t taddr, float* v) {
   const float2 s2 = make_float2(kLoInv, kLoInv);
 #pragma unroll
   for (int k = 0; k < 32; k += 2) {
+    const float2 r = __ffma2_rn(make_float2(__uint_as_float(b[k]), __uint_as_float(b[k + 1])), s2,
+                                make_float2(__uint_as_float(a[k]), __uint_as_float(a[k + 1])));
+    v[k] = r.x; v[k + 1] = r.y;
+  }
+}
+
+// the same for 16 columns (half the registers: for places with much else live)
+__device__ __forceinline__ void tmem_ld16_combined(uint32_t taddr, float* v) {
+  uint32_t a[16], b[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]), "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]),
+        "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]), "=r"(b[8]), "=r"(b[9]), "=r"(b[10]), "=r"(b[11]), "=r"(b[12]), "=r"(b[13]), "=r"(b[14]), "=r"(b[15])
+      : "r"(taddr), "r"(taddr + 256)
+      : "memory");
+  const float2 s2 = make_float2(kLoInv, kLoInv);
+#pragma unroll
+  for (int k = 0; k < 16; k += 2) {
     const float2 r = __ffma2_rn(make_float2(__uint_as_float(b[k]), __uint_as_float(b[k + 1])), s2,
                                 make_float2(__uint_as_float(a[k]), __uint_as_float(a[k + 1])));
     v[k] = r.x; v[k + 1] = r.y;
@@ -320,11 +336,14 @@ __device__ __noinline__ void issue_filter_mma(uint32_t tmem, uint32_t a_hi, uint
 // 16-warp version: warps w, w + 4, w + 8, w + 12 share a quadrant and take 32 columns each; all 128 rows
 __device__ __forceinline__ void tmem_to_tile(uint32_t tmem, int f, int warp, int lane, float* wt) {
   const int q = warp & 3, col = 32 * (warp >> 2);
-  float v[32];
-  tmem_ld32_combined(tmem + ((uint32_t)(32 * q) << 16) + 128 * f + col, v);
   float* p = wt + (32 * q + lane) * kWStride + col;
 #pragma unroll
-  for (int k = 0; k < 32; k += 4) st4(p + k, make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+  for (int c = 0; c < 32; c += 16) {      // 16 columns at a time: the sender rows in flight hold most of the registers
+    float v[16];
+    tmem_ld16_combined(tmem + ((uint32_t)(32 * q) << 16) + 128 * f + col + c, v);
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) st4(p + c + k, make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+  }
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -334,59 +353,113 @@ __device__ __forceinline__ bool edge_valid(int j, int n, float dx, float dy, flo
   r2 = dx * dx + dy * dy + dz * dz;
   return j >= 0 && j < n && r2 < kRc2 && r2 > 0.f;
 }
+// One entry per undirected pair: of (i <- j) and (j <- i) the list keeps the one in the row of the smaller index, so rows [0, m)
+// hold every pair with at least one end below m exactly once.  Caller-supplied lists keep the entry that comes before its partner
+// (`partner`, see match_pairs_kernel), or all of them when *asym is set.
 template <bool FILL>
 __global__ void __launch_bounds__(256) compact_rows_kernel(int n_rows, int n, const int* __restrict__ row_ptr, const int* __restrict__ nbr_j,
-                                                           const float* __restrict__ dR, int* __restrict__ vcount,
+                                                           const float* __restrict__ dR, const int* __restrict__ partner,
+                                                           const int* __restrict__ asym, int* __restrict__ vcount,
                                                            const int* __restrict__ vrow_ptr, int* __restrict__ ve_i, int* __restrict__ ve_j,
-                                                           float4* __restrict__ ve_d, int* __restrict__ ve_orig) {
+                                                           float4* __restrict__ ve_d, int2* __restrict__ ve_orig) {
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= n_rows) return;
   const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
+  const bool all = asym && *asym != 0;
   int count = 0;
   const int base = FILL ? vrow_ptr[i] : 0;
   for (int eb = e0; eb < e1; eb += 32) {
     const int e = eb + lane;
     bool valid = false;
-    int j = -1;
+    int j = -1, pe = -1;
     float dx = 0.f, dy = 0.f, dz = 0.f, r2 = 0.f;
     if (e < e1) {
       j = nbr_j[e];
-      dx = dR[3 * (size_t)e]; dy = dR[3 * (size_t)e + 1]; dz = dR[3 * (size_t)e + 2];
-      valid = edge_valid(j, n, dx, dy, dz, r2);
+      if (partner || j > i) {
+        dx = dR[3 * (size_t)e]; dy = dR[3 * (size_t)e + 1]; dz = dR[3 * (size_t)e + 2];
+        valid = edge_valid(j, n, dx, dy, dz, r2);
+      }
+      if (valid && partner && !all) { pe = partner[e]; valid = e < pe; }
     }
     const unsigned m = __ballot_sync(0xffffffffu, valid);
     if (FILL && valid) {
       const int p = base + count + __popc(m & ((1u << lane) - 1u));
       ve_i[p] = i; ve_j[p] = j;
       ve_d[p] = make_float4(dx, dy, dz, sqrtf(r2));
-      if (ve_orig) ve_orig[p] = e;
+      if (ve_orig) ve_orig[p] = make_int2(e, pe);
     }
     count += __popc(m);
   }
   if (!FILL && lane == 0) vcount[i] = count;
 }
-// every compacted entry (i <- j, d) looks for (j <- i, -d) in row j; a miss sets *asym
-__global__ void __launch_bounds__(256) check_symmetric_kernel(int n_rows, const int* __restrict__ vrow_ptr, const int* __restrict__ ve_i,
-                                                              const int* __restrict__ ve_j, const float4* __restrict__ ve_d, int* asym) {
-  const long long n_entries = vrow_ptr[n_rows];
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += (long long)gridDim.x * blockDim.x) {
-    const int i = ve_i[e], j = ve_j[e];
-    const float4 d = ve_d[e];
-    const float tol = 1e-5f * d.w + 1e-6f;
-    bool found = false;
-    if (j >= 0 && j < n_rows) {
-      for (int p = vrow_ptr[j]; p < vrow_ptr[j + 1] && !found; ++p) {
-        if (ve_j[p] != i) continue;
-        const float4 q = ve_d[p];
-        found = fabsf(q.x + d.x) <= tol && fabsf(q.y + d.y) <= tol && fabsf(q.z + d.z) <= tol;
-      }
+// Every entry (i <- j, d) inside the cutoff of a caller-supplied list finds its reversed entry (j <- i, -d): the k-th of several equal
+// entries of a row takes the k-th match.  *asym is set when an entry has none or the numbers of equal entries differ.  One warp per row.
+__global__ void __launch_bounds__(256) match_pairs_kernel(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ nbr_j,
+                                                          const float* __restrict__ dR, int* __restrict__ partner, int* __restrict__ asym) {
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= n_rows) return;
+  const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
+  for (int e = e0 + (threadIdx.x & 31); e < e1; e += 32) {
+    const int j = nbr_j[e];
+    float r2, q2;
+    const float dx = dR[3 * (size_t)e], dy = dR[3 * (size_t)e + 1], dz = dR[3 * (size_t)e + 2];
+    if (!edge_valid(j, n_rows, dx, dy, dz, r2)) { partner[e] = -1; continue; }
+    const float tol = 1e-5f * sqrtf(r2) + 1e-6f;
+    int rank = 0, mult = 0, match = 0, pe = -1;
+    for (int p = e0; p < e1; ++p) {
+      if (nbr_j[p] != j) continue;
+      const float x = dR[3 * (size_t)p], y = dR[3 * (size_t)p + 1], z = dR[3 * (size_t)p + 2];
+      if (!edge_valid(j, n_rows, x, y, z, q2) || fabsf(x - dx) > tol || fabsf(y - dy) > tol || fabsf(z - dz) > tol) continue;
+      ++mult;
+      rank += p < e;
     }
-    if (!found) { atomicExch(asym, 1); return; }
+    for (int p = row_ptr[j]; p < row_ptr[j + 1]; ++p) {
+      if (nbr_j[p] != i) continue;
+      const float x = dR[3 * (size_t)p], y = dR[3 * (size_t)p + 1], z = dR[3 * (size_t)p + 2];
+      if (!edge_valid(i, n_rows, x, y, z, q2) || fabsf(x + dx) > tol || fabsf(y + dy) > tol || fabsf(z + dz) > tol) continue;
+      if (match == rank) pe = p;
+      ++match;
+    }
+    partner[e] = pe;
+    if (match != mult) atomicExch(asym, 1);
   }
+}
+// the matches have to be mutual (displacements that agree within the tolerance only pairwise could break that)
+__global__ void __launch_bounds__(256) check_mutual_kernel(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ partner, int* asym) {
+  const int total = row_ptr[n_rows];
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+    const int p = partner[e];
+    if (p >= 0 && (p == e || partner[p] != e)) { atomicExch(asym, 1); return; }
+  }
+}
+// entries of the directed list: a pair whose ends both own a row stands for two of them
+__global__ void __launch_bounds__(256) count_directed_kernel(int n_rows, const int* __restrict__ vrow_ptr, const int* __restrict__ ve_j,
+                                                             const int* __restrict__ asym, unsigned long long* total) {
+  const int n_entries = vrow_ptr[n_rows];
+  const bool both = !(asym && *asym != 0);
+  unsigned long long c = 0;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += (long long)gridDim.x * blockDim.x)
+    c += both && ve_j[e] < n_rows ? 2 : 1;
+  if (c) atomicAdd(total, c);
 }
 __global__ void close_scan_kernel(int n_rows, const int* __restrict__ vcount, int* __restrict__ vrow_ptr) {
   if (threadIdx.x == 0 && blockIdx.x == 0) vrow_ptr[n_rows] = n_rows > 0 ? vrow_ptr[n_rows - 1] + vcount[n_rows - 1] : 0;
+}
+
+// Entries per warp of a tile (8 fill the 128 rows): the same number of rounds over the grid, with the entries spread evenly.  A tile's
+// time is its chain of phases plus the edge loops, which are as long as a warp's share: a short list runs one thin tile per CTA
+// instead of full tiles on a few of them, and the last round of a longer one is not half empty.
+__device__ __forceinline__ int entries_per_warp(long long n_edges, int grid) {
+  const long long rounds = (n_edges + (long long)TE * grid - 1) / ((long long)TE * grid);
+  return (int)((n_edges + 16 * rounds * grid - 1) / (16 * rounds * grid));
+}
+// `body(full)` with full = true_type where a warp's share is the whole run its loops are unrolled for (the run of a long list: branches
+// on the share inside the loops cost 4 % there), false_type where it is shorter
+template <class Body>
+__device__ __forceinline__ void edge_loops(int share, Body&& body, int run = 8) {
+  if (share == run) body(std::true_type{});
+  else body(std::false_type{});
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -402,7 +475,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
                                                                     const int* __restrict__ ve_j, const float4* __restrict__ ve_d,
                                                                     const float* __restrict__ qkv, const float* __restrict__ ev_in,
                                                                     float* __restrict__ xa, float* __restrict__ ev1, int* __restrict__ err,
-                                                                    long long* __restrict__ dbg) {
+                                                                    long long* __restrict__ dbg, const int* __restrict__ asym) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* rec = reinterpret_cast<float*>(smem + kOffFwRec);
@@ -414,17 +487,21 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffFwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffFwMisc + 16);
   const long long n_edges = vrow_ptr[n_recv];
-  const long long n_tiles = (n_edges + TE - 1) / TE;
+  if (n_edges <= 0) return;
+  const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
+  const long long n_tiles = (n_edges + tr - 1) / tr;
   const long long tile0 = n_tiles * blockIdx.x / gridDim.x, tile1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
   if (tile0 >= tile1) return;
   const int pad_i = ve_i[n_edges - 1];
+  // partners below n_scat receive the pair's other direction (j <- i)
+  const int n_scat = asym && *asym != 0 ? 0 : n_recv;
   // inputs of one tile into the staging buffers: receiver / sender, displacement, both atoms' ev rows (threads 256..383)
   auto stage_tile = [&](long long tile) {
     if (tid < 256 || tid >= 384 || tile >= tile1) return;
     const int row = tid - 256;
-    const long long e = tile * TE + row;
+    const long long e = tile * tr + row;
     int i = pad_i, j = pad_i;
-    if (e < n_edges) {
+    if (row < tr && e < n_edges) {
       i = ve_i[e]; j = ve_j[e];
       cp_async16(st_d + row, ve_d + e);
     } else {
@@ -464,7 +541,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   const uint32_t a_hi = smem_u32(smem + kOffA), img = smem_u32(smem + kOffImg);
   const int col = 4 * lane;
   const int deg = degree_of(lane < kMTot ? lane : 0);
-  const int k0 = 8 * warp;               // this warp's rows of the tile in the edge loop
+  const int k0 = rpw * warp;             // this warp's rows of the tile in the edge loop
   uint32_t parity = 0;
 #ifdef SO3LR_TC_TIMING
   long long tph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -477,7 +554,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     // ---- per-edge preparation from the staged inputs ----
     {
       const int row = tid & 127, role = tid >> 7;
-      const bool valid = tile * TE + row < n_edges;
+      const bool valid = row < tr && tile * tr + row < n_edges;
       if (role < 2) {
         const float4 d = st_d[row];
         const float r = d.w;
@@ -508,19 +585,22 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
       }
     }
     TC_MARK(0);
-    // sender rows of filter 0 for this warp's edges and the first receiver's query row, requested before the barrier (the indices
-    // are in the staging buffer since the previous tile): the warps with the shorter preparation start their gathers while the
-    // others still work, and all of them are in flight while the tensor cores run
-    float4 kf[8], vj[8], qf;
+    // the partners' q / k rows of filter 0 for this warp's pairs and the first receiver's rows, requested before the barrier (the
+    // indices are in the staging buffer since the previous tile): the warps with the shorter preparation start their gathers while
+    // the others still work, and all of them are in flight while the tensor cores run
+    float4 qj[8], kj[8], qi, ki, vi;
     int cur_i;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const float* kj = qkv + (size_t)st_ij[2 * (k0 + u) + 1] * kProj;
-      kf[u] = ld4(kj + kF + col);
-      vj[u] = ld4(kj + 2 * kF + col);
+      const float* pj = qkv + (size_t)st_ij[2 * ((k0 + u) & (TE - 1)) + 1] * kProj + col;      // past this warp's share: not used
+      qj[u] = ld4(pj);
+      kj[u] = ld4(pj + kF);
     }
     cur_i = st_ij[2 * k0];
-    qf = ld4(qkv + (size_t)cur_i * kProj + col);
+    {
+      const float* pi = qkv + (size_t)cur_i * kProj + col;
+      qi = ld4(pi); ki = ld4(pi + kF); vi = ld4(pi + 2 * kF);
+    }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -553,37 +633,51 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     TC_MARK(3);
-    {
-      float4 accx = f4_zero();
-      if (cur_i == __float_as_int(rec[(k0 + 7) * kFwRec + 1])) {      // all eight edges belong to one receiver: no flush inside
-        float a[8];
+    edge_loops(rpw, [&](auto full) {
+      // logits x cutoff of both directions: a of (i <- j), b of (j <- i); b's message goes out at once, a's are summed per receiver.
+      // The value rows are requested as the q / k registers of a pair come free.
+      float a[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          a[u] = group8_sum(dot3(qf, ld4(wt + (k0 + u) * kWStride + col), kf[u])) * rec[(k0 + u) * kFwRec + 2];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) accx = f4_fma(a[u], vj[u], accx);
-      } else {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
-          const int iu = __float_as_int(r0.y);
-          if (iu != cur_i) {
-            if (f4_nonzero(accx)) red_add_v4(xa + (size_t)cur_i * kF + col, accx);
-            cur_i = iu;
-            accx = f4_zero();
-            qf = ld4(qkv + (size_t)cur_i * kProj + col);
-          }
-          const float a = group8_sum(dot3(qf, ld4(wt + (k0 + u) * kWStride + col), kf[u])) * r0.z;
-          accx = f4_fma(a, vj[u], accx);
+      for (int u = 0; u < 8; ++u) {
+        if (!full && u >= rpw) break;
+        const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
+        const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
+        if (i != cur_i) {
+          cur_i = i;
+          const float* pi = qkv + (size_t)cur_i * kProj + col;
+          qi = ld4(pi); ki = ld4(pi + kF); vi = ld4(pi + 2 * kF);
         }
+        const float4 w = ld4(wt + (k0 + u) * kWStride + col);
+        a[u] = group8_sum(dot3(qi, w, kj[u])) * r0.z;
+        const float b = group8_sum(dot3(qj[u], w, ki)) * r0.z;
+        if (j < n_scat && r0.z != 0.f) red_add_v4(xa + (size_t)j * kF + col, f4_scale(b, vi));
+        qj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
+      }
+      float4 accx = f4_zero();
+      cur_i = __float_as_int(rec[k0 * kFwRec + 1]);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (!full && u >= rpw) break;
+        const int i = __float_as_int(rec[(k0 + u) * kFwRec + 1]);
+        if (i != cur_i) {
+          if (f4_nonzero(accx)) red_add_v4(xa + (size_t)cur_i * kF + col, accx);
+          cur_i = i;
+          accx = f4_zero();
+        }
+        accx = f4_fma(a[u], qj[u], accx);
       }
       if (f4_nonzero(accx)) red_add_v4(xa + (size_t)cur_i * kF + col, accx);
-    }
-    // sender rows of filter 1: in flight across the barrier and the second tile copy
+    });
+    // rows of filter 1: in flight across the barrier and the second tile copy
 #pragma unroll
-    for (int u = 0; u < 8; ++u) kf[u] = ld4(qkv + (size_t)__float_as_int(rec[(k0 + u) * kFwRec]) * kProj + 4 * kF + col);
+    for (int u = 0; u < 8; ++u) {
+      const float* pj = qkv + (size_t)__float_as_int(rec[((k0 + u) & (TE - 1)) * kFwRec]) * kProj + 3 * kF + col;
+      qj[u] = ld4(pj);
+      kj[u] = ld4(pj + kF);
+    }
     cur_i = __float_as_int(rec[k0 * kFwRec + 1]);
-    qf = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
+    qi = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
+    ki = ld4(qkv + (size_t)cur_i * kProj + 4 * kF + col);
     TC_MARK(4);
     parity ^= 1;
     __syncthreads();
@@ -593,36 +687,31 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     TC_MARK(6);
-    {
+    edge_loops(rpw, [&](auto full) {
       float accev = 0.f;
-      if (cur_i == __float_as_int(rec[(k0 + 7) * kFwRec + 1])) {
-        float a[8];
+      const float sgn = deg == 0 || deg == 2 ? -1.f : 1.f;      // Y_lm(-u) = (-1)^l Y_lm(u)
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          a[u] = group8_sum(dot3(qf, ld4(wt + (k0 + u) * kWStride + col), kf[u])) * rec[(k0 + u) * kFwRec + 2];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float ym = lane < kMTot ? rec[(k0 + u) * kFwRec + 4 + lane] : 0.f;
-          accev = fmaf(__shfl_sync(0xffffffffu, a[u], 8 * deg), ym, accev);
+      for (int u = 0; u < 8; ++u) {
+        if (!full && u >= rpw) break;
+        const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
+        const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
+        if (i != cur_i) {
+          if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
+          cur_i = i;
+          accev = 0.f;
+          qi = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
+          ki = ld4(qkv + (size_t)cur_i * kProj + 4 * kF + col);
         }
-      } else {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
-          const int iu = __float_as_int(r0.y);
-          if (iu != cur_i) {
-            if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
-            cur_i = iu;
-            accev = 0.f;
-            qf = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
-          }
-          const float a = group8_sum(dot3(qf, ld4(wt + (k0 + u) * kWStride + col), kf[u])) * r0.z;
-          const float ym = lane < kMTot ? rec[(k0 + u) * kFwRec + 4 + lane] : 0.f;
-          accev = fmaf(__shfl_sync(0xffffffffu, a, 8 * deg), ym, accev);
-        }
+        const float4 w = ld4(wt + (k0 + u) * kWStride + col);
+        const float a = group8_sum(dot3(qi, w, kj[u])) * r0.z;
+        const float b = group8_sum(dot3(qj[u], w, ki)) * r0.z;
+        const float ym = lane < kMTot ? rec[(k0 + u) * kFwRec + 4 + lane] : 0.f;
+        accev = fmaf(__shfl_sync(0xffffffffu, a, 8 * deg), ym, accev);
+        const float bd = __shfl_sync(0xffffffffu, b, 8 * deg);
+        if (lane < kMTot && j < n_scat && r0.z != 0.f) atomicAdd(ev1 + (size_t)j * kMTot + lane, sgn * bd * ym);
       }
       if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
-    }
+    });
     cp_async_wait_all();
     __syncthreads();
     TC_MARK(7);
@@ -665,6 +754,7 @@ __device__ __noinline__ void issue_reverse_mma(uint32_t tmem, uint32_t a_hi, uin
 }
 
 // Sender-side q / k rows of four consecutive tile rows for the reverse edge loop of filter F (lane = 4 features)
+// (for every row of the four: past a warp's share these are rows of other warps, whose values are not used)
 struct RevLoads {
   float4 qj[4], kj[4], qa, ka;     // senders' rows; q / k of the first row's receiver
 };
@@ -683,9 +773,10 @@ __device__ __forceinline__ void reverse_prefetch(RevLoads& L, const float* rec, 
 }
 
 // Value path of the invariant filter, split off the edge loop so that it runs while the tensor cores are busy.
-// Before the loop (rows [row0, row0 + 8) of one warp): cotangents of the invariant logits of both directions of every edge,
+// Before the loop (rows [row0, row0 + nu), nu <= 8, of one warp): cotangents of the invariant logits of both directions of every edge,
 // daA_h = <g_xa[i], v[j]>_h and daB_h = <g_xa[j], v[i]>_h, into record fields 36..39 and 40..43.
-__device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int lane, const float* __restrict__ qkv,
+template <bool FULL>
+__device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int nu, int lane, const float* __restrict__ qkv,
                                                        const float* __restrict__ g_xa) {
   const int col = 4 * lane, grp = lane >> 3, cg = lane & 7;
   int cur_i = -1;
@@ -696,7 +787,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
     int ii[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const float* rp = rec + (row0 + k0 + u) * kBwRec;
+      const float* rp = rec + ((row0 + k0 + u) & (TE - 1)) * kBwRec;
       const int j = __float_as_int(rp[0]);
       ii[u] = __float_as_int(rp[1]);
       vj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
@@ -704,6 +795,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
+      if (!FULL && k0 + u >= nu) break;
       if (ii[u] != cur_i) {
         cur_i = ii[u];
         v_i = ld4(qkv + (size_t)cur_i * kProj + 2 * kF + col);
@@ -718,45 +810,53 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
     }
   }
 }
-// After the loop: cotangent of this receiver's value row, gv_i = sum_edges (cutoff x logit of edge j<-i)_h g_xa[j] (fields 44..47)
-__device__ __forceinline__ void value_cotangent(const float* rec, int row0, int lane, const float* __restrict__ g_xa, float* __restrict__ g_qkv) {
+// After the loop: cotangents of the value rows, gv_i = sum over its pairs (cutoff x logit of edge j<-i)_h g_xa[j] (fields 44..47) and,
+// pair by pair, gv_j += (cutoff x logit of edge i<-j)_h g_xa[i] (fields 48..51)
+template <bool FULL>
+__device__ __forceinline__ void value_cotangent(const float* rec, int row0, int nu, int lane, const float* __restrict__ g_xa,
+                                                float* __restrict__ g_qkv, int n_scat) {
   const int col = 4 * lane, grp = lane >> 3;
   float4 gxj[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) gxj[u] = ld4(g_xa + (size_t)__float_as_int(rec[(row0 + u) * kBwRec]) * kF + col);
+  for (int u = 0; u < 8; ++u) gxj[u] = ld4(g_xa + (size_t)__float_as_int(rec[((row0 + u) & (TE - 1)) * kBwRec]) * kF + col);
   int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
-  float4 gv = f4_zero();
+  float4 gv = f4_zero(), gxi = ld4(g_xa + (size_t)cur_i * kF + col);
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
+    if (!FULL && u >= nu) break;
     const float* rp = rec + (row0 + u) * kBwRec;
-    const int i = __float_as_int(rp[1]);
+    const float4 r0 = ld4(rp);
+    const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
     if (i != cur_i) {
       if (f4_nonzero(gv)) red_add_v4(g_qkv + (size_t)cur_i * kProj + 2 * kF + col, gv);
       cur_i = i;
       gv = f4_zero();
+      gxi = ld4(g_xa + (size_t)cur_i * kF + col);
     }
     gv = f4_fma(rp[44 + grp], gxj[u], gv);
+    if (j < n_scat && r0.z != 0.f) red_add_v4(g_qkv + (size_t)j * kProj + 2 * kF + col, f4_scale(rp[48 + grp], gxi));
   }
   if (f4_nonzero(gv)) red_add_v4(g_qkv + (size_t)cur_i * kProj + 2 * kF + col, gv);
 }
 
-// Reverse edge loop of filter F over four tile rows [row0, row0 + 4) of one warp: logits of both directions of every edge,
+// Reverse edge loop of filter F over nu <= 4 tile rows [row0, row0 + nu) of one warp: logits of both directions of every edge,
 // cotangents of this receiver's q / k rows (added to g_qkv with vector reductions when the receiver changes), dw into the
 // A operand of the second MMA chain, the cutoff part of d/dr into the records.  The cotangents of the logits come from the
 // records (fields 36.. for the invariant filter, 12.. for the equivariant one); cutoff x logit goes back (44.. / 20.., 24..).
-template <int F>
-__device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, const float* wt, int wrow0, int row0, unsigned char* a_hi,
-                                               int lane, const float* __restrict__ qkv, float* __restrict__ g_qkv) {
+template <int F, bool FULL>
+__device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, const float* wt, int wrow0, int row0, int nu, unsigned char* a_hi,
+                                               int lane, const float* __restrict__ qkv, float* __restrict__ g_qkv, int n_scat) {
   const int col = 4 * lane, grp = lane >> 3, cg = lane & 7;
   int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
   float4 qa = L.qa, ka = L.ka;
   float4 gq = f4_zero(), gk = f4_zero();
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
+    if (!FULL && u >= nu) break;
     const int row = row0 + u;
     float* rp = rec + row * kBwRec;
     const float4 r0 = ld4(rp);
-    const int i = __float_as_int(r0.y);
+    const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
     const float sc = r0.z, dcn = r0.w;
     if (i != cur_i) {      // rare: a run of four rows mostly stays with one receiver
       {
@@ -782,7 +882,7 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
     const float daA = rp[(F ? 12 : 36) + grp], daB = rp[(F ? 16 : 40) + grp];
     if (cg == 0) {
       if (F) { rp[20 + grp] = sc * DA; rp[24 + grp] = sc * DB; }
-      else rp[44 + grp] = sc * DB;
+      else { rp[44 + grp] = sc * DB; rp[48 + grp] = sc * DA; }
     }
     const float dDA = sc * daA, dDB = sc * daB;
     const float2 a2 = make_float2(dDA, dDA), b2 = make_float2(dDB, dDB);
@@ -793,6 +893,14 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
       const float2 h01 = __ffma2_rn(b2, __fmul2_rn(w01, make_float2(qj.x, qj.y)), make_float2(gk.x, gk.y));
       const float2 h23 = __ffma2_rn(b2, __fmul2_rn(w23, make_float2(qj.z, qj.w)), make_float2(gk.z, gk.w));
       gk = make_float4(h01.x, h01.y, h23.x, h23.y);
+    }
+    if (j < n_scat && sc != 0.f) {      // the partner's shares: gq_j = dDB w k_i, gk_j = dDA w q_i
+      float* gj = g_qkv + (size_t)j * kProj + F * 3 * kF + col;
+      const float2 m01 = __fmul2_rn(b2, w01), m23 = __fmul2_rn(b2, w23), n01 = __fmul2_rn(a2, w01), n23 = __fmul2_rn(a2, w23);
+      const float2 q01 = __fmul2_rn(m01, lo2(ka)), q23 = __fmul2_rn(m23, hi2(ka));
+      const float2 k01 = __fmul2_rn(n01, lo2(qa)), k23 = __fmul2_rn(n23, hi2(qa));
+      red_add_v4(gj, make_float4(q01.x, q01.y, q23.x, q23.y));
+      red_add_v4(gj + kF, make_float4(k01.x, k01.y, k23.x, k23.y));
     }
     const float2 d01 = __ffma2_rn(a2, pA01, __fmul2_rn(b2, pB01)), d23 = __ffma2_rn(a2, pA23, __fmul2_rn(b2, pB23));
     const float dw0 = d01.x, dw1 = d01.y, dw2 = d23.x, dw3 = d23.y;
@@ -838,7 +946,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
                                                                     float* __restrict__ g_qkv, float* __restrict__ gev_in,
                                                                     float* __restrict__ F, float* __restrict__ virial,
                                                                     int* __restrict__ err, long long* __restrict__ dbg,
-                                                                    const int* __restrict__ ve_orig, const int* __restrict__ gate) {
+                                                                    const int2* __restrict__ ve_orig, const int* __restrict__ gate,
+                                                                    int n_own) {
   if (PER_ENTRY && gate && *gate != 0) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -848,7 +957,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffBwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 16);
   const long long n_edges = vrow_ptr[n_recv];
-  const long long n_tiles = (n_edges + TE - 1) / TE;
+  if (n_edges <= 0) return;
+  const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
+  const long long n_tiles = (n_edges + tr - 1) / tr;
   const long long tile0 = n_tiles * blockIdx.x / gridDim.x, tile1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
   if (tile0 >= tile1) return;
   for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
@@ -875,7 +986,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const int pad_i = ve_i[n_edges - 1];
   const int deg = degree_of(lane < kMTot ? lane : 0);
   const int quad = warp & 3;                    // TMEM lane quadrant of this warp
-  const int wrow = 4 * warp;                    // this warp's 4 rows inside a 64-row half of the tile
+  const int n_scat = n_recv;                    // partners below it own a row: they receive their share of a pair here
+  const int nu0 = rpw < 4 ? rpw : 4, nu1 = rpw - nu0;      // this warp's rows inside the two 64-row halves of the tile
+  const int wrow0 = nu0 * warp, wrow1 = nu1 * warp;
   uint32_t parity = 0;
   bool failed = false;
 #ifdef SO3LR_TC_TIMING
@@ -890,8 +1003,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     // ---- per-edge preparation ----
     {
       const int row = tid & 127, role = tid >> 7;
-      const long long e = tile * TE + row;
-      const bool valid = e < n_edges;
+      const long long e = tile * tr + row;
+      const bool valid = row < tr && e < n_edges;
       int i = pad_i, j = pad_i;
       if (valid) { i = ve_i[e]; j = ve_j[e]; }
       float* rp = rec + row * kBwRec;
@@ -960,9 +1073,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     }
     __syncwarp();
     // while the tensor cores run: the value path's logit cotangents (8 rows per warp), then the sender rows of the first edge run
-    value_logit_cotangents(rec, 8 * warp, lane, qkv, g_xa);
+    edge_loops(rpw, [&](auto full) { value_logit_cotangents<full>(rec, rpw * warp, rpw, lane, qkv, g_xa); });
     RevLoads L;
-    reverse_prefetch<0>(L, rec, wrow, lane, qkv);
+    reverse_prefetch<0>(L, rec, wrow0, lane, qkv);
     bool done = true;
     if (tid == 0) done = mbar_wait(mbar, parity);     // one thread polls; the others park at the barrier below
     parity ^= 1;
@@ -973,6 +1086,11 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     for (int f = 0; f < 2 && !failed; ++f) {
 #pragma unroll 1
       for (int hh = 0; hh < 2; ++hh) {
+        if (hh == 1 && nu1 == 0) {      // no rows in the second half
+          if (f == 0) reverse_prefetch<1>(L, rec, wrow0, lane, qkv);
+          break;
+        }
+        const int wrow = hh ? wrow1 : wrow0, nu = hh ? nu1 : nu0;
         if ((quad >> 1) == hh) {          // the 8 warps whose TMEM lanes hold this half: 32 columns each
           float v[32];
           const int col = 32 * (warp >> 2);
@@ -985,12 +1103,12 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         __syncthreads();
         BW_MARK(3);
         if (f == 0) {
-          reverse_edges4<0>(L, rec, wt, wrow, 64 * hh + wrow, a_ptr, lane, qkv, g_qkv);
-          if (hh == 0) reverse_prefetch<0>(L, rec, 64 + wrow, lane, qkv);      // next run: second half of filter 0
-          else reverse_prefetch<1>(L, rec, wrow, lane, qkv);                   // next run: first half of filter 1
+          edge_loops(nu, [&](auto full) { reverse_edges4<0, full>(L, rec, wt, wrow, 64 * hh + wrow, nu, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+          if (hh == 0) reverse_prefetch<0>(L, rec, 64 + wrow1, lane, qkv);      // next run: second half of filter 0
+          else reverse_prefetch<1>(L, rec, wrow0, lane, qkv);                   // next run: first half of filter 1
         } else {
-          reverse_edges4<1>(L, rec, wt, wrow, 64 * hh + wrow, a_ptr, lane, qkv, g_qkv);
-          if (hh == 0) reverse_prefetch<1>(L, rec, 64 + wrow, lane, qkv);
+          edge_loops(nu, [&](auto full) { reverse_edges4<1, full>(L, rec, wt, wrow, 64 * hh + wrow, nu, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+          if (hh == 0) reverse_prefetch<1>(L, rec, 64 + wrow1, lane, qkv);
         }
         BW_MARK(4);
         __syncthreads();
@@ -1007,13 +1125,13 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       if (f == 1 && lane < kMTot) {      // ev differences of this warp's 8 rows of the final flush: requested now, used after the last MMA
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const float* rp = rec + (8 * warp + k) * kBwRec;
+          const float* rp = rec + ((rpw * warp + k) & (TE - 1)) * kBwRec;
           const int j = __float_as_int(rp[0]), i = __float_as_int(rp[1]);
           dev8[k] = ev_in[(size_t)j * kMTot + lane] - ev_in[(size_t)i * kMTot + lane];
         }
       }
       if (f == 0) {
-        value_cotangent(rec, 8 * warp, lane, g_xa, g_qkv);      // while the tensor cores run
+        edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, rpw * warp, rpw, lane, g_xa, g_qkv, n_scat); });      // while the tensor cores run
       } else if (tid < 128) {
         // angular part of the force on the receiver (independent of the radial derivative that the running MMA yields); it
         // takes the record fields 44..46, which the value path has released
@@ -1108,7 +1226,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       const float g_r = rp[32] + rp[35];
       float fsx = on ? fmaf(g_r, uu.x, ang.x) : 0.f, fsy = on ? fmaf(g_r, uu.y, ang.y) : 0.f, fsz = on ? fmaf(g_r, uu.z, ang.z) : 0.f;
       if (virial && on) {
-        const float hr = 0.5f * rp[33];
+        // both ends' halves on the receiver's row, unless the partner's is not summed here (rows below n_own are)
+        const float hr = (__float_as_int(rp[0]) < n_own ? 1.f : 0.5f) * rp[33];
         const float wx = hr * uu.x, wy = hr * uu.y, wz = hr * uu.z;
         float* w = virial + 6 * (size_t)i;
         atomicAdd(w, wx * fsx); atomicAdd(w + 1, wy * fsy); atomicAdd(w + 2, wz * fsz);
@@ -1116,16 +1235,21 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         atomicAdd(w + 5, 0.5f * (wx * fsy + wy * fsx));
       }
       if (PER_ENTRY) {
-        // half of the pair's force on the receiver goes to this entry of the source list; the reversed entry, processed at the
-        // other atom, receives the other half with the opposite sign
+        // half of the pair's force on the receiver goes to this entry of the source list, the other half with the opposite sign to the
+        // reversed entry
         if (on) {
-          const long long e = tile * TE + tid;
-          float* g = F + 3 * (size_t)ve_orig[e];
+          const int2 eo = ve_orig[tile * tr + tid];
+          float *g = F + 3 * (size_t)eo.x, *h = F + 3 * (size_t)eo.y;
           g[0] += 0.5f * fsx; g[1] += 0.5f * fsy; g[2] += 0.5f * fsz;
+          h[0] -= 0.5f * fsx; h[1] -= 0.5f * fsy; h[2] -= 0.5f * fsz;
         }
       } else {
       // the rows of a tile are sorted by receiver: sum each run of equal receivers inside the warp (segmented scan) and let its
-      // last lane add the total, instead of up to 32 additions to one address
+      // last lane add the total, instead of up to 32 additions to one address; the partners differ and get theirs one by one
+      const int jp = __float_as_int(rp[0]);
+      if (on && jp < n_scat) {
+        atomicAdd(F + 3 * (size_t)jp, -fsx); atomicAdd(F + 3 * (size_t)jp + 1, -fsy); atomicAdd(F + 3 * (size_t)jp + 2, -fsz);
+      }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const float tx = __shfl_up_sync(0xffffffffu, fsx, o), ty = __shfl_up_sync(0xffffffffu, fsy, o), tz = __shfl_up_sync(0xffffffffu, fsz, o);
@@ -1138,21 +1262,27 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       }
       }
     }
-    {
+    edge_loops(rpw, [&](auto full) {
       int cur_i = -1;
       float acc = 0.f;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float* rp = rec + (8 * warp + k) * kBwRec;
+        if (!full && k >= rpw) break;
+        const float* rp = rec + (rpw * warp + k) * kBwRec;
         const int i = __float_as_int(rp[1]);
         if (i != cur_i) {
           if (cur_i >= 0 && lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
           cur_i = i; acc = 0.f;
         }
-        if (lane < kMTot) acc = fmaf(-2.f * invw(deg) * rp[8 + deg], dev8[k], acc);
+        if (lane < kMTot) {
+          const float t = -2.f * invw(deg) * rp[8 + deg] * dev8[k];
+          const int j = __float_as_int(rp[0]);
+          acc += t;
+          if (j < n_scat && rp[34] != 0.f) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
+        }
       }
       if (cur_i >= 0 && lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
-    }
+    });
     __syncthreads();
     BW_MARK(7);
   }
@@ -1210,28 +1340,56 @@ int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity) {
 }
 
 void valid_edges_free(ValidEdges* V) {
-  dev_free(V->row_ptr); dev_free(V->count); dev_free(V->i); dev_free(V->j); dev_free(V->d); dev_free(V->orig); dev_free(V->cub_tmp);
+  dev_free(V->row_ptr); dev_free(V->count); dev_free(V->i); dev_free(V->j); dev_free(V->d); dev_free(V->orig); dev_free(V->partner); dev_free(V->cub_tmp);
   *V = ValidEdges{};
 }
 
-int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const int* row_ptr, const int* nbr_j, const float* dR, bool want_orig) {
+int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const int* row_ptr, const int* nbr_j, const float* dR, int* asym,
+                      long long n_source) {
+  V->asym = nullptr;
   if (n_rows <= 0) return kOk;
   if (n_rows + 1 > V->row_cap) return kInvalidArgument;
-  if (want_orig && V->orig_cap < V->capacity) {
-    if (V->orig) dev_free(V->orig);
-    V->orig = nullptr;
-    SO3LR_CUDA_CHECK(dev_alloc(&V->orig, (size_t)V->capacity));
-    V->orig_cap = V->capacity;
-  }
   const int blocks = (n_rows + 7) / 8;
-  { compact_rows_kernel<false><<<blocks, 256, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, V->count, nullptr, nullptr, nullptr, nullptr, nullptr); count_launch(); }
+  if (asym) {
+    if (n_source > V->capacity) return kInvalidArgument;
+    if (V->orig_cap < V->capacity) {
+      dev_free(V->orig); dev_free(V->partner);
+      V->orig = nullptr; V->partner = nullptr; V->orig_cap = 0;
+      SO3LR_CUDA_CHECK(dev_alloc(&V->orig, (size_t)V->capacity));
+      SO3LR_CUDA_CHECK(dev_alloc(&V->partner, (size_t)V->capacity));
+      V->orig_cap = V->capacity;
+    }
+    V->asym = asym;
+    { match_pairs_kernel<<<blocks, 256, 0, s>>>(n_rows, row_ptr, nbr_j, dR, V->partner, asym); count_launch(); }
+    { check_mutual_kernel<<<sm_count() * 8, 256, 0, s>>>(n_rows, row_ptr, V->partner, asym); count_launch(); }
+  }
+  const int* partner = asym ? V->partner : nullptr;
+  { compact_rows_kernel<false><<<blocks, 256, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, V->count, nullptr, nullptr, nullptr, nullptr, nullptr); count_launch(); }
   size_t tmp = V->cub_bytes;
   cub::DeviceScan::ExclusiveSum(V->cub_tmp, tmp, V->count, V->row_ptr, n_rows, s);
   count_launch(2);
   { close_scan_kernel<<<1, 32, 0, s>>>(n_rows, V->count, V->row_ptr); count_launch(); }
-  { compact_rows_kernel<true><<<blocks, 256, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, nullptr, V->row_ptr, V->i, V->j, V->d, want_orig ? V->orig : nullptr); count_launch(); }
+  { compact_rows_kernel<true><<<blocks, 256, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->row_ptr, V->i, V->j, V->d, asym ? V->orig : nullptr); count_launch(); }
   SO3LR_CUDA_CHECK(cudaGetLastError());
   V->n_rows = n_rows;
+  return kOk;
+}
+
+int valid_edges_count_directed(const ValidEdges& V, long long* n_host) {
+  *n_host = 0;
+  if (!V.row_ptr || V.n_rows <= 0) return kOk;
+  SO3LR_CUDA_CHECK(cudaDeviceSynchronize());
+  unsigned long long* t = nullptr;
+  SO3LR_CUDA_CHECK(dev_alloc(&t, 1));
+  unsigned long long h = 0;
+  cudaError_t e = cudaMemset(t, 0, sizeof(h));
+  if (e == cudaSuccess) {
+    { count_directed_kernel<<<sm_count(), 256>>>(V.n_rows, V.row_ptr, V.j, V.asym, t); count_launch(); }
+    e = cudaMemcpy(&h, t, sizeof(h), cudaMemcpyDeviceToHost);
+  }
+  dev_free(t);
+  SO3LR_CUDA_CHECK(e);
+  *n_host = (long long)h;
   return kOk;
 }
 
@@ -1278,19 +1436,19 @@ int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, i
   // the kernel adds the attention sums onto the skip connection
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(xa, x_in, (size_t)n_recv * kF * sizeof(float), cudaMemcpyDeviceToDevice, s));
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(ev1, ev_in, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  { attn_fwd_tc_kernel<<<sm_count(), kFwThreads, kSmemFwd, s>>>(L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer()); count_launch(); }
+  { attn_fwd_tc_kernel<<<sm_count(), kFwThreads, kSmemFwd, s>>>(L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym); count_launch(); }
   return kOk;
 }
 
 int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
-                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int* err) {
+                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err) {
   if (n_recv <= 0) return kOk;
   if (n_recv > V.n_rows) return kInvalidArgument;
   // the kernel adds into the receivers' rows: cotangents of q/k/v start at zero, that of ev at the skip term
   SO3LR_CUDA_CHECK(cudaMemsetAsync(g_qkv, 0, (size_t)n_recv * kProj * sizeof(float), s));
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, gev1, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
   { attn_bwd_tc_kernel<false><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
-                                                              g_qkv, gev_in, F, virial, err, tc_debug_buffer(), nullptr, nullptr); count_launch(); }
+                                                              g_qkv, gev_in, F, virial, err, tc_debug_buffer(), nullptr, nullptr, n_own); count_launch(); }
   return kOk;
 }
 
@@ -1299,13 +1457,8 @@ int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges
   if (n_recv <= 0) return kOk;
   if (n_recv > V.n_rows || !V.orig) return kInvalidArgument;
   { attn_bwd_tc_kernel<true><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
-                                                             g_qkv, gev_in, g_dR, nullptr, err, nullptr, V.orig, asym); count_launch(); }
+                                                             g_qkv, gev_in, g_dR, nullptr, err, nullptr, V.orig, asym, 0); count_launch(); }
   return kOk;
-}
-
-void valid_edges_check_symmetric(const ValidEdges& V, cudaStream_t s, int* asym) {
-  if (V.n_rows <= 0) return;
-  { check_symmetric_kernel<<<sm_count() * 8, 256, 0, s>>>(V.n_rows, V.row_ptr, V.i, V.j, V.d, asym); count_launch(); }
 }
 
 }  // namespace so3lr

@@ -512,9 +512,9 @@ void attn_fwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L,
 }
 void attn_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
                        const float* qkv, const float* ev_in, const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F,
-                       int first_layer, float* virial) {
+                       int first_layer, float* virial, int n_own) {
   if (!first_layer && L.has_spherical && attention_mode() == kAttnTc)
-    launch_attn_bwd_tc(st, L, S->ve, n_recv, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial, S->d_flag + 1);
+    launch_attn_bwd_tc(st, L, S->ve, n_recv, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial, n_own, S->d_flag + 1);
   else if (!first_layer && L.has_spherical && use_mma_attention())
     launch_attn_bwd_mma(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial);
   else launch_attn_bwd_sym(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, first_layer, virial);
@@ -552,9 +552,8 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
     int rcv = valid_edges_reserve(&S->ve, S->n_cap, n_edges);
     if (rcv) return rcv;
     SO3LR_CUDA_CHECK(cudaMemsetAsync(asym, 0, sizeof(int), st));
-    rcv = valid_edges_build(&S->ve, st, n, n, row_ptr, nbr_j, dR, true);
+    rcv = valid_edges_build(&S->ve, st, n, n, row_ptr, nbr_j, dR, asym, n_edges);
     if (rcv) return rcv;
-    valid_edges_check_symmetric(S->ve, st, asym);
   }
   fill(st, S->e_zbl, n, 0.f); fill(st, S->e_coul, n, 0.f); fill(st, S->e_disp, n, 0.f);
   fill(st, S->gq, n, 0.f); fill(st, S->gh, n, 0.f);
@@ -748,7 +747,7 @@ int fused_backward(so3lr_b200_system* S, cudaStream_t st, const Shells& c, float
       launch_layer0_bwd_tab(st, S->sp, nattn[0], c.n3, c.n3, row_ptr, nbr_j, S->dR, S->d_Z, S->g_xa, S->gev1, S->GV, F, S->vir());
     else
       attn_bwd_dispatch(S, st, L, nattn[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, F, l == 0 ? 1 : 0,
-                        S->vir());
+                        S->vir(), c.n0);
     S->prof.end(st);
     if (l > 0) {
       if (!use_mma_dense()) {
@@ -1358,12 +1357,10 @@ SO3LR_B200_API int so3lr_b200_system_valid_edges(so3lr_b200_system* S, int64_t* 
   if (!S || !n_valid) return kInvalidArgument;
   SO3LR_CUDA_CHECK(cudaSetDevice(S->model->device));
   *n_valid = 0;
-  if (!S->ve.row_ptr || S->ve.n_rows <= 0) return kOk;
-  int v = 0;
-  SO3LR_CUDA_CHECK(cudaDeviceSynchronize());
-  SO3LR_CUDA_CHECK(cudaMemcpy(&v, S->ve.row_ptr + S->ve.n_rows, sizeof(int), cudaMemcpyDeviceToHost));
+  long long v = 0;
+  int rc = valid_edges_count_directed(S->ve, &v);
   *n_valid = v;
-  return kOk;
+  return rc;
 }
 
 SO3LR_B200_API int so3lr_b200_system_export_list(so3lr_b200_system* S, void* stream, const float* R, int which, int32_t* idx, int64_t capacity,
@@ -1889,7 +1886,7 @@ SO3LR_B200_API int so3lr_b200_dd_layer_backward_attn(so3lr_b200_system* S, void*
     launch_layer0_bwd_tab(st, S->sp, n0, S->shells[1], S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->d_Z, S->g_xa, S->gev1, S->GV, S->F_s, S->vir());
   else
     attn_bwd_dispatch(S, st, L, n0, S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, S->dd_gev_in, S->F_s,
-                      l == 0 ? 1 : 0, S->vir());
+                      l == 0 ? 1 : 0, S->vir(), n0);
   S->prof.end(st);
   if (l == 0 && S->vir()) reduce_virial(S, st, n0);
   if (l > 0) {

@@ -144,15 +144,18 @@ void launch_attn_bwd_mma(cudaStream_t s, const LayerDev& L, int n_recv, int n, c
                          float* F, float* virial = nullptr);
 
 // ---- attention_tc.cu: layers with a spherical filter as CTA-tiled tcgen05 kernels ----
-// Short-range list entries inside the cutoff, compacted once per evaluation and grouped by receiver: entry p of row i
-// (row_ptr[i] <= p < row_ptr[i + 1]) holds the receiver i[p], the sender j[p] and d[p] = (dx, dy, dz, |dR|).
+// Short-range pairs inside the cutoff, compacted once per evaluation, one entry per undirected pair, grouped by its end with the
+// smaller index: entry p of row i (row_ptr[i] <= p < row_ptr[i + 1]) holds i[p], the partner j[p] and d[p] = (dx, dy, dz, |dR|) from i
+// to j.  Caller-supplied lists whose entries do not come in reversed pairs (*asym != 0) keep every entry i <- j.
 struct ValidEdges {
   int* row_ptr = nullptr;   // n_rows + 1
   int* count = nullptr;     // per-row counts (scratch of the build)
   int* i = nullptr;
   int* j = nullptr;
   float4* d = nullptr;
-  int* orig = nullptr;      // position of each entry in the list it was compacted from (only when asked for)
+  int2* orig = nullptr;     // caller-supplied lists: positions of each entry and of its reversed entry in that list
+  int* partner = nullptr;   // caller-supplied lists: position of each source entry's reversed entry
+  const int* asym = nullptr;
   long long orig_cap = 0;
   void* cub_tmp = nullptr;
   size_t cub_bytes = 0;
@@ -166,10 +169,12 @@ void tc_debug_print();
 int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity);
 void valid_edges_free(ValidEdges* V);
 // no host synchronisation: counts stay on the device
+// `asym` (caller-supplied lists of n_source entries; zeroed by the caller): set to 1 when the entries inside the cutoff do not pair up
+// as (i <- j, d), (j <- i, -d); without it the list has to be symmetric with one entry per pair and direction
 int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const int* row_ptr, const int* nbr_j, const float* dR,
-                      bool want_orig = false);
-// *asym = 1 when some entry (i <- j, d) has no partner (j <- i, -d) in the compacted list (the word must be zero beforehand)
-void valid_edges_check_symmetric(const ValidEdges& V, cudaStream_t s, int* asym);
+                      int* asym = nullptr, long long n_source = 0);
+// entries i <- j of the latest build counted per direction (synchronises)
+int valid_edges_count_directed(const ValidEdges& V, long long* n_host);
 // The reverse kernel for caller-supplied lists: runs only while *asym == 0 and, instead of summing forces, adds to every source
 // entry e (V.orig) half of the force that the pair exerts on its receiver, g[e] += (dE/d dR_e - dE/d dR_e') / 2 with e' the
 // reversed entry.  For any motion of atoms or cell (dR_e' = -dR_e) that is equivalent to the per-entry gradient.  The caller
@@ -180,9 +185,10 @@ int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges
 // tensor-core pipeline ran out; the outputs are then incomplete.
 int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* x_in,
                        const float* ev_in, float* xa, float* ev1, int* err);
-// Same results as launch_attn_bwd_sym (first_layer = 0) for rows [0, n_recv): writes g_qkv and gev_in rows, adds to F (and virial).
+// Same results as launch_attn_bwd_sym (first_layer = 0) for rows [0, n_recv): writes g_qkv and gev_in rows, adds to F (and to virial
+// rows, of which those below n_own add up to the total).
 int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
-                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int* err);
+                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err);
 
 // ---- layer0_tab.cu: first layer through per-element-pair tables (its inputs depend on the elements only) ----
 constexpr int kMaxTabSpecies = 8;

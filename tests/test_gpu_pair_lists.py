@@ -1,0 +1,77 @@
+"""Short-range attention on one entry per undirected pair (csrc/attention_tc.cu): caller-supplied lists of every form that decides how the
+entries pair up, and pair counts around the edges of a warp's share and of a tile, against the float64 oracle on the same lists.
+
+Tolerances are those of the parity tests: energies 1e-5 relative, gradients 1e-4 eV/A."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _structure(name):
+    from so3lr_b200 import workloads as W
+    if name.startswith("water"):
+        n = int(name[5:])
+        return W.water_box(n, (n * 29.9) ** (1 / 3), 3)
+    Z, R = W.molecule(np.random.default_rng(7), int(name[3:]))
+    return Z, R, None
+
+
+def _lists(name, form):
+    from oracle import so3lr_oracle as O
+    Z, R, cell = _structure(name)
+    R = np.asarray(R, np.float32).astype(np.float64)
+    cell = None if cell is None else np.asarray(cell, np.float32).astype(np.float64)
+    i, j = O.neighbor_list(R, cell, 4.5, ordered=False)
+    il, jl = O.neighbor_list(R, cell, 6.0 if cell is not None else 100.0, ordered=False)
+    mi = lambda d: d if cell is None else d - np.round(d @ np.linalg.inv(cell)) @ cell
+    d, dl = mi(R[j] - R[i]), mi(R[jl] - R[il])
+    if form == "twice":                       # every entry two times: still paired
+        i, j, d = np.repeat(i, 2), np.repeat(j, 2), np.repeat(d, 2, axis=0)
+    elif form == "twice_one_way":             # one entry two times, its partner once
+        k = len(i) // 3
+        i, j, d = (np.insert(a, k, a[k], axis=0) for a in (i, j, d))
+    elif form == "one_way":                   # no entry has a partner
+        m = j > i
+        i, j, d = i[m], j[m], d[m]
+    elif form == "images":                    # an atom beside its own periodic images
+        i, j = np.append(i, [0, 0, 1, 1]), np.append(j, [0, 0, 1, 1])
+        d = np.concatenate([d, [[0.0, 0.0, 4.1], [0.0, 0.0, -4.1], [-4.2, 0.3, 0.0], [4.2, -0.3, 0.0]]])
+        o = np.argsort(i, kind="stable")
+        i, j, d = i[o], j[o], d[o]
+    elif form == "padded":                    # entries beyond the cutoff and a tail of padding
+        m = len(Z)
+        far = np.nonzero(i == m - 1)[0][:1]
+        i, j, d = np.append(np.append(i, i[far]), [m] * 5), np.append(np.append(j, j[far]), [m] * 5), np.concatenate([d, d[far] * 9.0, np.zeros((5, 3))])
+    return Z, cell, (i, j, d.astype(np.float32)), (il, jl, dl.astype(np.float32))
+
+
+@pytest.mark.parametrize("name,form", [(n, "plain") for n in ("mol8", "mol11", "mol23", "mol40", "water64", "water192")] +
+                         [("mol23", f) for f in ("twice", "twice_one_way", "one_way", "images", "padded")] + [("water64", f) for f in ("twice", "one_way")])
+def test_list_forms_against_the_oracle(name, form):
+    from oracle import so3lr_oracle as O
+    from so3lr_b200.engine import System
+    Z, cell, (i, j, d), (il, jl, dl) = _lists(name, form)
+    n = len(Z)
+    s = System(Z, cell, cutoff_lr=6.0 if cell is not None else 100.0, damping=2.0, lr_format="sparse")
+    t = lambda a: torch.tensor(a, device="cuda")
+    o = s.graph_eval(t(i), t(j), t(d), t(il), t(jl), t(dl))
+    D, DL = torch.tensor(d, dtype=torch.float64, requires_grad=True), torch.tensor(dl, dtype=torch.float64, requires_grad=True)
+    e, _ = O.energy_from_graph(O.load_params(), Z, D, i, j, DL, il, jl, lr_format="sparse", cutoff_lr=6.0 if cell is not None else 100.0, damping=2.0)
+    g, = torch.autograd.grad(e.sum(), D)
+    got = o["g_edges"].double().cpu()
+    e = e.detach()
+    assert float((o["e_atom"].double().cpu() - e).abs().sum()) <= 1e-5 * float(e.abs().sum())
+    if form in ("one_way", "twice_one_way"):      # lists without partners: the gradient of every entry
+        assert float((got - g).abs().max()) <= 1e-4
+        return
+    # paired lists: what any motion of atoms or cell sees of it
+    m = torch.tensor(i < n)
+    ti, tj = torch.tensor(i)[m], torch.tensor(j)[m]
+    f = lambda x: torch.zeros(n, 3, dtype=torch.float64).index_add(0, ti, x[m]).index_add(0, tj, -x[m])
+    assert float((f(got) - f(g)).abs().max()) <= 1e-4
+    Dd = D.detach()
+    w, wr = Dd.T @ got, Dd.T @ g
+    assert float((w - wr).abs().max()) <= 1e-4 * max(1.0, float(wr.abs().max()))
+    assert float(got[~m].abs().sum()) == 0.0
