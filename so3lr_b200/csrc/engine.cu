@@ -476,31 +476,41 @@ bool use_tc_dense() {
   }();
   return v;
 }
+// Lists that fill only a few 128-atom tiles take the kernels of atom_kernels_small.cu instead (16 atoms per SM at most); SO3LR_B200_DENSE=tc
+// keeps them on dense_tc.cu.
+bool use_small_dense(int n) {
+  static const bool on = std::getenv("SO3LR_B200_DENSE") == nullptr;
+  return on && dense_small_applies(n);
+}
 // With the tensor-core dense blocks the q/k/v projections ride along: the forward block also emits the next layer's
 // q/k/v rows, the reverse block forms its input cotangent from the upper layer's g_xa and g_qkv.  `next` / `up` = that
 // neighbouring layer (nullptr: no fusion at this end of the network).
 void post_fwd_dispatch(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
                        float* x4, float* ev2, const LayerDev* next, float* qkv_next, int* err) {
-  if (use_tc_dense()) launch_atom_post_fwd_tc(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->proj_u : nullptr, qkv_next, err);
+  if (use_small_dense(n)) launch_atom_post_fwd_small(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->projT : nullptr, qkv_next);
+  else if (use_tc_dense()) launch_atom_post_fwd_tc(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->proj_u : nullptr, qkv_next, err);
   else if (use_mma_dense()) launch_atom_post_fwd_mma(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->proj_f : nullptr, qkv_next);
   else launch_atom_post_fwd(s, L, n, xa, ev1, z1, x3, gate, x4, ev2);
 }
 void post_bwd_dispatch(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                        const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const LayerDev* up,
                        const float* g_qkv_up, int* err) {
-  if (use_tc_dense()) launch_atom_post_bwd_tc(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->projT_u : nullptr, g_qkv_up, err);
+  if (use_small_dense(n)) launch_atom_post_bwd_small(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->proj : nullptr, g_qkv_up);
+  else if (use_tc_dense()) launch_atom_post_bwd_tc(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->projT_u : nullptr, g_qkv_up, err);
   else if (use_mma_dense()) launch_atom_post_bwd_mma(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->projT_f : nullptr, g_qkv_up);
   else launch_atom_post_bwd(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1);
 }
 void heads_fwd_dispatch(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* x, float* ze, float* zq, float* zh,
                         float* e_nn, float* q_raw, float* hv, int* err) {
-  if (use_tc_dense()) launch_heads_fwd_tc(s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv, err);
+  if (use_small_dense(n)) launch_heads_fwd_small(s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv);
+  else if (use_tc_dense()) launch_heads_fwd_tc(s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv, err);
   else if (use_mma_dense()) launch_heads_fwd_mma(s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv);
   else launch_heads_fwd(s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv);
 }
 void heads_bwd_dispatch(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* ze, const float* zq, const float* zh,
                         const float* hv, const float* ge, const float* gq, const float* gh, float* gx, int* err) {
-  if (use_tc_dense()) launch_heads_bwd_tc(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx, err);
+  if (use_small_dense(n)) launch_heads_bwd_small(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx);
+  else if (use_tc_dense()) launch_heads_bwd_tc(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx, err);
   else if (use_mma_dense()) launch_heads_bwd_mma(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx);
   else launch_heads_bwd(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx);
 }
@@ -935,6 +945,7 @@ SO3LR_B200_API int so3lr_b200_model_create(const float* blob_host, size_t n_floa
   if (rc == kOk) rc = configure_attention_tc_kernels();
   if (rc == kOk) rc = configure_atom_mma_kernels();
   if (rc == kOk) rc = configure_dense_tc_kernels();
+  if (rc == kOk) rc = configure_dense_small_kernels();
   if (rc != kOk) { so3lr_b200_model_destroy(m); return rc; }
   *out = m;
   return kOk;

@@ -63,6 +63,19 @@ void launch_heads_fwd_tc(cudaStream_t s, const ModelDev& M, int n, const int* Z,
 void launch_heads_bwd_tc(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* ze, const float* zq, const float* zh,
                          const float* hv, const float* ge, const float* gq, const float* gh, float* gx, int* err);
 
+// ---- atom_kernels_small.cu: the same blocks and heads (FP32 throughout) for lists of at most 16 atoms per SM ----
+bool dense_small_applies(int n);
+int configure_dense_small_kernels();
+void launch_atom_post_fwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
+                                float* x4, float* ev2, const float* projT, float* qkv_next);
+void launch_atom_post_bwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
+                                const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const float* proj,
+                                const float* g_qkv_up);
+void launch_heads_fwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* x, float* ze, float* zq, float* zh, float* e_nn,
+                            float* q_raw, float* hv);
+void launch_heads_bwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* ze, const float* zq, const float* zh,
+                            const float* hv, const float* ge, const float* gq, const float* gh, float* gx);
+
 // ---- kspace.cu: reciprocal-space (Ewald) part of the electrostatic energy of one periodic structure ----
 struct KSpaceDev {
   int mode = 0;            // 0 off, 1 Ewald sum over the index grid, 2 particle-mesh Ewald on a mesh of that shape

@@ -1,7 +1,8 @@
 """Short-range attention on one entry per undirected pair (csrc/attention_tc.cu): caller-supplied lists of every form that decides how the
 entries pair up, and pair counts around the edges of a warp's share and of a tile, against the float64 oracle on the same lists.
 
-Tolerances are those of the parity tests: energies 1e-5 relative, gradients 1e-4 eV/A."""
+Tolerances are those of the parity tests: energies 1e-5 relative, gradients 1e-4 eV/A; with every entry two times in the list every pair
+term and its rounding error count twice: 2e-4 eV/A."""
 import numpy as np
 import pytest
 import torch
@@ -70,7 +71,7 @@ def test_list_forms_against_the_oracle(name, form):
     m = torch.tensor(i < n)
     ti, tj = torch.tensor(i)[m], torch.tensor(j)[m]
     f = lambda x: torch.zeros(n, 3, dtype=torch.float64).index_add(0, ti, x[m]).index_add(0, tj, -x[m])
-    assert float((f(got) - f(g)).abs().max()) <= 1e-4
+    assert float((f(got) - f(g)).abs().max()) <= (2e-4 if form == "twice" else 1e-4)
     Dd = D.detach()
     w, wr = Dd.T @ got, Dd.T @ g
     assert float((w - wr).abs().max()) <= 1e-4 * max(1.0, float(wr.abs().max()))
