@@ -21,7 +21,8 @@
 // reductions in global memory (a receiver's pairs can span warps, tiles and CTAs); the partner's share of a pair goes out as one
 // reduction per row.  Those cost less than the second evaluation they replace: the L2 takes 5.4 TB/s of 512-byte row reductions
 // (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.  With every pair evaluated at
-// both ends instead, 98,304 atoms took 1.99 / 5.12 ms a launch (forward / reverse), with one evaluation 1.23 / 3.12 ms.
+// both ends instead, 98,304 atoms took 1.99 / 5.12 ms a launch (forward / reverse), with one evaluation 1.23 / 3.12 ms, and with the
+// logits of four pairs of a receiver summed together, no branches between them, 1.16 / 2.97 ms.
 //
 // The reverse kernel forms dw in the same loop, writes it straight into shared memory as the (FP16-split) A operand of a
 // second MMA chain against the SAME weight image read with the other major-ness,
@@ -94,6 +95,14 @@ __device__ __forceinline__ float4 f4_scale(float a, float4 b) {
   const float2 l = __fmul2_rn(a2, lo2(b)), h = __fmul2_rn(a2, hi2(b));
   return make_float4(l.x, l.y, h.x, h.y);
 }
+__device__ __forceinline__ float4 f4_mul(float4 a, float4 b) {
+  const float2 l = __fmul2_rn(lo2(a), lo2(b)), h = __fmul2_rn(hi2(a), hi2(b));
+  return make_float4(l.x, l.y, h.x, h.y);
+}
+__device__ __forceinline__ float4 f4_mad(float4 a, float4 b, float4 c) {
+  const float2 l = __ffma2_rn(lo2(a), lo2(b), lo2(c)), h = __ffma2_rn(hi2(a), hi2(b), hi2(c));
+  return make_float4(l.x, l.y, h.x, h.y);
+}
 __device__ __forceinline__ float4 f4_zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ float dot3(float4 a, float4 b, float4 c) {
   const float2 s = __ffma2_rn(__fmul2_rn(hi2(a), hi2(b)), hi2(c), __fmul2_rn(__fmul2_rn(lo2(a), lo2(b)), lo2(c)));
@@ -102,6 +111,16 @@ __device__ __forceinline__ float dot3(float4 a, float4 b, float4 c) {
 __device__ __forceinline__ float dot2(float4 a, float4 b) {
   const float2 s = __ffma2_rn(hi2(a), hi2(b), __fmul2_rn(lo2(a), lo2(b)));
   return s.x + s.y;
+}
+// Eight sums over the eight lanes of a group at once: lane cg of the group gets the sum of v[cg].  Seven exchanges, in three dependent
+// steps, where eight separate butterfly sums take 24.
+__device__ __forceinline__ float transpose_sum8(const float (&v)[8], int cg) {
+  float s[4], t[2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k] = ((cg & 4) ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, (cg & 4) ? v[k] : v[k + 4], 4);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) t[k] = ((cg & 2) ? s[k + 2] : s[k]) + __shfl_xor_sync(0xffffffffu, (cg & 2) ? s[k] : s[k + 2], 2);
+  return ((cg & 1) ? t[1] : t[0]) + __shfl_xor_sync(0xffffffffu, (cg & 1) ? t[0] : t[1], 1);
 }
 __device__ __forceinline__ bool f4_nonzero(float4 a) { return a.x != 0.f || a.y != 0.f || a.z != 0.f || a.w != 0.f; }
 
@@ -202,6 +221,19 @@ __device__ __forceinline__ void tmem_ld16_combined(uint32_t taddr, float* v) {
                                 make_float2(__uint_as_float(a[k]), __uint_as_float(a[k + 1])));
     v[k] = r.x; v[k + 1] = r.y;
   }
+}
+__device__ __forceinline__ void tmem_ld8_combined(uint32_t taddr, float* v) {
+  uint32_t a[8], b[8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]),
+        "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7])
+      : "r"(taddr), "r"(taddr + 256)
+      : "memory");
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = fmaf(__uint_as_float(b[k]), kLoInv, __uint_as_float(a[k]));
 }
 
 __device__ __forceinline__ void invariants(const float* __restrict__ evi, const float* __restrict__ evj, float* s) {
@@ -638,33 +670,66 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
       // The value rows are requested as the q / k registers of a pair come free.
       float a[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (!full && u >= rpw) break;
-        const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
-        const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
-        if (i != cur_i) {
-          cur_i = i;
-          const float* pi = qkv + (size_t)cur_i * kProj + col;
-          qi = ld4(pi); ki = ld4(pi + kF); vi = ld4(pi + 2 * kF);
+      for (int h = 0; h < 8; h += 4) {
+        const float* rp = rec + (k0 + h) * kFwRec;
+        if (full && __float_as_int(rp[1]) == __float_as_int(rp[3 * kFwRec + 1])) {      // four pairs of one receiver: their sums together
+          if (__float_as_int(rp[1]) != cur_i) {
+            cur_i = __float_as_int(rp[1]);
+            const float* pi = qkv + (size_t)cur_i * kProj + col;
+            qi = ld4(pi); ki = ld4(pi + kF); vi = ld4(pi + 2 * kF);
+          }
+          float v[8];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float4 w = ld4(wt + (k0 + h + u) * kWStride + col);
+            v[2 * u] = dot3(qi, w, kj[h + u]);
+            v[2 * u + 1] = dot3(qj[h + u], w, ki);
+          }
+          const float d = transpose_sum8(v, lane & 7) * rp[((lane & 7) >> 1) * kFwRec + 2];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = __float_as_int(rp[u * kFwRec]);
+            a[h + u] = __shfl_sync(0xffffffffu, d, (lane & 24) + 2 * u);
+            const float b = __shfl_sync(0xffffffffu, d, (lane & 24) + 2 * u + 1);
+            if (j < n_scat) red_add_v4(xa + (size_t)j * kF + col, f4_scale(b, vi));
+            qj[h + u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
+          }
+          continue;
         }
-        const float4 w = ld4(wt + (k0 + u) * kWStride + col);
-        a[u] = group8_sum(dot3(qi, w, kj[u])) * r0.z;
-        const float b = group8_sum(dot3(qj[u], w, ki)) * r0.z;
-        if (j < n_scat && r0.z != 0.f) red_add_v4(xa + (size_t)j * kF + col, f4_scale(b, vi));
-        qj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
+#pragma unroll
+        for (int u = h; u < h + 4; ++u) {
+          if (!full && u >= rpw) break;
+          const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
+          const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
+          if (i != cur_i) {
+            cur_i = i;
+            const float* pi = qkv + (size_t)cur_i * kProj + col;
+            qi = ld4(pi); ki = ld4(pi + kF); vi = ld4(pi + 2 * kF);
+          }
+          const float4 w = ld4(wt + (k0 + u) * kWStride + col);
+          a[u] = group8_sum(dot3(qi, w, kj[u])) * r0.z;
+          const float b = group8_sum(dot3(qj[u], w, ki)) * r0.z;
+          if (j < n_scat && r0.z != 0.f) red_add_v4(xa + (size_t)j * kF + col, f4_scale(b, vi));
+          qj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
+        }
       }
       float4 accx = f4_zero();
       cur_i = __float_as_int(rec[k0 * kFwRec + 1]);
+      if (full && cur_i == __float_as_int(rec[(k0 + 7) * kFwRec + 1])) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (!full && u >= rpw) break;
-        const int i = __float_as_int(rec[(k0 + u) * kFwRec + 1]);
-        if (i != cur_i) {
-          if (f4_nonzero(accx)) red_add_v4(xa + (size_t)cur_i * kF + col, accx);
-          cur_i = i;
-          accx = f4_zero();
+        for (int u = 0; u < 8; ++u) accx = f4_fma(a[u], qj[u], accx);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (!full && u >= rpw) break;
+          const int i = __float_as_int(rec[(k0 + u) * kFwRec + 1]);
+          if (i != cur_i) {
+            if (f4_nonzero(accx)) red_add_v4(xa + (size_t)cur_i * kF + col, accx);
+            cur_i = i;
+            accx = f4_zero();
+          }
+          accx = f4_fma(a[u], qj[u], accx);
         }
-        accx = f4_fma(a[u], qj[u], accx);
       }
       if (f4_nonzero(accx)) red_add_v4(xa + (size_t)cur_i * kF + col, accx);
     });
@@ -690,25 +755,50 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     edge_loops(rpw, [&](auto full) {
       float accev = 0.f;
       const float sgn = deg == 0 || deg == 2 ? -1.f : 1.f;      // Y_lm(-u) = (-1)^l Y_lm(u)
+      auto new_receiver = [&](int i) {
+        if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
+        cur_i = i;
+        accev = 0.f;
+        qi = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
+        ki = ld4(qkv + (size_t)cur_i * kProj + 4 * kF + col);
+      };
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (!full && u >= rpw) break;
-        const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
-        const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
-        if (i != cur_i) {
-          if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
-          cur_i = i;
-          accev = 0.f;
-          qi = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
-          ki = ld4(qkv + (size_t)cur_i * kProj + 4 * kF + col);
+      for (int h = 0; h < 8; h += 4) {
+        const float* rp = rec + (k0 + h) * kFwRec;
+        if (full && __float_as_int(rp[1]) == __float_as_int(rp[3 * kFwRec + 1])) {
+          if (__float_as_int(rp[1]) != cur_i) new_receiver(__float_as_int(rp[1]));
+          float v[8];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float4 w = ld4(wt + (k0 + h + u) * kWStride + col);
+            v[2 * u] = dot3(qi, w, kj[h + u]);
+            v[2 * u + 1] = dot3(qj[h + u], w, ki);
+          }
+          const float d = transpose_sum8(v, lane & 7) * rp[((lane & 7) >> 1) * kFwRec + 2];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = __float_as_int(rp[u * kFwRec]);
+            const float ym = lane < kMTot ? rp[u * kFwRec + 4 + lane] : 0.f;
+            accev = fmaf(__shfl_sync(0xffffffffu, d, 8 * deg + 2 * u), ym, accev);
+            const float bd = __shfl_sync(0xffffffffu, d, 8 * deg + 2 * u + 1);
+            if (lane < kMTot && j < n_scat) atomicAdd(ev1 + (size_t)j * kMTot + lane, sgn * bd * ym);
+          }
+          continue;
         }
-        const float4 w = ld4(wt + (k0 + u) * kWStride + col);
-        const float a = group8_sum(dot3(qi, w, kj[u])) * r0.z;
-        const float b = group8_sum(dot3(qj[u], w, ki)) * r0.z;
-        const float ym = lane < kMTot ? rec[(k0 + u) * kFwRec + 4 + lane] : 0.f;
-        accev = fmaf(__shfl_sync(0xffffffffu, a, 8 * deg), ym, accev);
-        const float bd = __shfl_sync(0xffffffffu, b, 8 * deg);
-        if (lane < kMTot && j < n_scat && r0.z != 0.f) atomicAdd(ev1 + (size_t)j * kMTot + lane, sgn * bd * ym);
+#pragma unroll
+        for (int u = h; u < h + 4; ++u) {
+          if (!full && u >= rpw) break;
+          const float4 r0 = ld4(rec + (k0 + u) * kFwRec);
+          const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
+          if (i != cur_i) new_receiver(i);
+          const float4 w = ld4(wt + (k0 + u) * kWStride + col);
+          const float a = group8_sum(dot3(qi, w, kj[u])) * r0.z;
+          const float b = group8_sum(dot3(qj[u], w, ki)) * r0.z;
+          const float ym = lane < kMTot ? rec[(k0 + u) * kFwRec + 4 + lane] : 0.f;
+          accev = fmaf(__shfl_sync(0xffffffffu, a, 8 * deg), ym, accev);
+          const float bd = __shfl_sync(0xffffffffu, b, 8 * deg);
+          if (lane < kMTot && j < n_scat && r0.z != 0.f) atomicAdd(ev1 + (size_t)j * kMTot + lane, sgn * bd * ym);
+        }
       }
       if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
     });
@@ -793,6 +883,18 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
       vj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
       gxj[u] = ld4(g_xa + (size_t)j * kF + col);
     }
+    if (FULL && ii[0] == ii[3]) {      // four pairs of one receiver
+      if (ii[0] != cur_i) {
+        cur_i = ii[0];
+        v_i = ld4(qkv + (size_t)cur_i * kProj + 2 * kF + col);
+        gx_i = ld4(g_xa + (size_t)cur_i * kF + col);
+      }
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { v[2 * u] = dot2(gx_i, vj[u]); v[2 * u + 1] = dot2(gxj[u], v_i); }
+      rec[(row0 + k0 + (cg >> 1)) * kBwRec + 36 + 4 * (cg & 1) + grp] = transpose_sum8(v, cg);
+      continue;
+    }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (!FULL && k0 + u >= nu) break;
@@ -821,6 +923,17 @@ __device__ __forceinline__ void value_cotangent(const float* rec, int row0, int 
   for (int u = 0; u < 8; ++u) gxj[u] = ld4(g_xa + (size_t)__float_as_int(rec[((row0 + u) & (TE - 1)) * kBwRec]) * kF + col);
   int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
   float4 gv = f4_zero(), gxi = ld4(g_xa + (size_t)cur_i * kF + col);
+  if (FULL && cur_i == __float_as_int(rec[(row0 + 7) * kBwRec + 1])) {      // eight pairs of one receiver
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float* rp = rec + (row0 + u) * kBwRec;
+      const int j = __float_as_int(rp[0]);
+      gv = f4_fma(rp[44 + grp], gxj[u], gv);
+      if (j < n_scat) red_add_v4(g_qkv + (size_t)j * kProj + 2 * kF + col, f4_scale(rp[48 + grp], gxi));
+    }
+    red_add_v4(g_qkv + (size_t)cur_i * kProj + 2 * kF + col, gv);
+    return;
+  }
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     if (!FULL && u >= nu) break;
@@ -850,6 +963,52 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
   int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
   float4 qa = L.qa, ka = L.ka;
   float4 gq = f4_zero(), gk = f4_zero();
+  if (FULL && cur_i == __float_as_int(rec[(row0 + 3) * kBwRec + 1])) {
+    // four pairs of one receiver (five runs of six): no branches between the rows, the eight logits summed together; lane cg of a head's
+    // group then holds row cg / 2, direction cg & 1
+    float v[8];
+    float4 w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      w[u] = ld4(wt + (wrow0 + u) * kWStride + col);
+      v[2 * u] = dot3(qa, w[u], L.kj[u]);
+      v[2 * u + 1] = dot3(L.qj[u], w[u], ka);
+    }
+    float* mp = rec + (row0 + (cg >> 1)) * kBwRec;
+    const int dir = cg & 1;
+    const float sc = mp[2], dcn = mp[3], da = mp[(F ? 12 : 36) + 4 * dir + grp];
+    const float D = transpose_sum8(v, cg);
+    mp[(F ? 20 + 4 * dir : 48 - 4 * dir) + grp] = sc * D;
+    const float dD = sc * da;
+    float gc = dcn * da * D;      // cutoff part of d/dr, summed over the directions and heads
+    gc += __shfl_xor_sync(0xffffffffu, gc, 1);
+    gc += __shfl_xor_sync(0xffffffffu, gc, 8);
+    gc += __shfl_xor_sync(0xffffffffu, gc, 16);
+    if (grp == 0 && dir == 0) mp[32] += gc;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float dDA = __shfl_sync(0xffffffffu, dD, (lane & 24) + 2 * u), dDB = __shfl_sync(0xffffffffu, dD, (lane & 24) + 2 * u + 1);
+      const float4 aw = f4_scale(dDA, w[u]), bw = f4_scale(dDB, w[u]);
+      gq = f4_mad(aw, L.kj[u], gq);
+      gk = f4_mad(bw, L.qj[u], gk);
+      const int j = __float_as_int(rec[(row0 + u) * kBwRec]);
+      if (j < n_scat) {
+        float* gj = g_qkv + (size_t)j * kProj + F * 3 * kF + col;
+        red_add_v4(gj, f4_mul(bw, ka));
+        red_add_v4(gj + kF, f4_mul(aw, qa));
+      }
+      const float4 dw = f4_fma(dDA, f4_mul(qa, L.kj[u]), f4_scale(dDB, f4_mul(L.qj[u], ka)));
+      uint2 h, l;
+      split2(dw.x, dw.y, h.x, l.x); split2(dw.z, dw.w, h.y, l.y);
+      unsigned char* p = a_hi + (lane >> 1) * kLboA + (row0 + u) * 16 + (lane & 1) * 8;
+      *reinterpret_cast<uint2*>(p) = h;
+      *reinterpret_cast<uint2*>(p + kAHalf) = l;
+    }
+    float* gi = g_qkv + (size_t)cur_i * kProj + F * 3 * kF + col;
+    red_add_v4(gi, gq);
+    red_add_v4(gi + kF, gk);
+    return;
+  }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     if (!FULL && u >= nu) break;
@@ -923,11 +1082,12 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
   if (f4_nonzero(gk)) red_add_v4(gi + kF, gk);
 }
 
-// record fields (floats): 0 j | 1 i | 2 cutoff / nbar | 3 its r-derivative | 4-7 invariants | 8-11 their cotangents |
+// record fields (floats): 0 j | 1 i | 2 cutoff / nbar | 3 its r-derivative | 4-7 invariants |
 // 12-15 dA, 16-19 dB: cotangents of the equivariant logits of edge (i<-j) and (j<-i) | 20-23, 24-27 those logits x cutoff |
-// 28-30 unit vector | 31 1/r | 32 d/dr (cutoff part + even Chebyshev terms) | 33 r | 34 1 for a list entry, 0 for a padding row |
-// 35 d/dr (odd Chebyshev terms) | 36-39, 40-43 cotangents of the invariant logits of edge (i<-j) and (j<-i) |
-// 44-47 invariant logit of edge (j<-i) x cutoff; after the value path has read it: 44-46 angular part of the force on the receiver
+// 28-30 unit vector | 31 1/r | 32 d/dr (cutoff part) | 33 r | 34 1 for a list entry, 0 for a padding row |
+// 36-39, 40-43 cotangents of the invariant logits of edge (i<-j) and (j<-i) |
+// 44-47, 48-51 invariant logits of edges (j<-i) and (i<-j) x cutoff; after the value path has read them: 44-46 angular part of the force
+// on the receiver
 //
 // 16 warps.  Per tile: (1) four threads per edge prepare records and the A operand; (2) MMA chain w = Phi C + hs K2 (both filters);
 // (3) per filter, in two halves of 64 rows: tensor memory -> shared tile, reverse edge loop (4 rows per warp, sender rows
@@ -1028,7 +1188,6 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
           float cut, dcut;
           phys_cutoff(r, cut, dcut);
           st4(rp, make_float4(__int_as_float(j), __int_as_float(i), valid ? cut * kInvNbar : 0.f, valid ? dcut * kInvNbar : 0.f));
-          st4(rp + 8, f4_zero());
           st4(rp + 20, f4_zero());
           st4(rp + 24, f4_zero());
           st4(rp + 28, make_float4(ux, uy, uz, ir));
@@ -1082,6 +1241,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     if (!__syncthreads_and(done)) { failed = true; break; }
     tc_fence_after();
     BW_MARK(2);
+    // this thread's shares of its row's cotangents of the invariants and of the radial derivative, both filters
+    float ds0 = 0.f, ds1 = 0.f, ds2 = 0.f, ds3 = 0.f, drad = 0.f;
 #pragma unroll 1
     for (int f = 0; f < 2 && !failed; ++f) {
 #pragma unroll 1
@@ -1171,33 +1332,41 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         const int row = tid & 127, role = tid >> 7;
         float* rp = rec + row * kBwRec;
         const uint32_t lane_base = tmem + ((uint32_t)(32 * quad) << 16) + 128 * f;
-        if (role < 2) {
+        {
+          // thread (odd, upper) takes the terms m = 2c + odd of c in [16 upper, 16 upper + 16): columns 32 odd + c.  T_m' = m U_{m-1}, and
+          // U_{n+2} = 2 T_2 U_n - U_{n-2} from (U_{-2}, U_0) or (U_{-3}, U_{-1}), in the upper half from (U_30, U_32) or (U_29, U_31),
+          // which follow from t by doubling: T_2n = 2 T_n^2 - 1, U_{2n-1} = 2 T_n U_{n-1}, U_n = t U_{n-1} + T_n, U_{n-2} = t U_{n-1} - T_n
+          const int odd = role & 1, upper = role >> 1;
           const float r = rp[33];
           const float x = expf(-kChebHalfGamma * r);
           const float t = fmaf(kChebA, x, kChebB), t2 = 2.f * t;
           const float dtdr = -kChebA * kChebHalfGamma * x;
-          // T_m' = m U_{m-1}; columns 0..31 hold m = 2c (U of odd index), columns 32..63 hold m = 2c + 1 (U of even index);
-          // both run U_{n+2} = 2 T_2 U_n - U_{n-2}
-          const float T2x2 = 2.f * fmaf(t2, t, -1.f);
-          float v[32];
-          tmem_ld32_combined(lane_base + 32 * role, v);
-          float up = role ? -1.f : -t2, uc = role ? 1.f : 0.f;      // (U_{-2}, U_0) or (U_{-3}, U_{-1})
+          const float T2 = fmaf(t2, t, -1.f), T2x2 = 2.f * T2;
+          float v[16];
+          tmem_ld16_combined(lane_base + 32 * odd + 16 * upper, v);
+          float up = odd ? -1.f : -t2, uc = odd ? 1.f : 0.f;
+          if (upper) {
+            const float T4 = fmaf(T2x2, T2, -1.f), T8 = fmaf(2.f * T4, T4, -1.f), T16 = fmaf(2.f * T8, T8, -1.f), T32 = fmaf(2.f * T16, T16, -1.f);
+            const float U31 = 16.f * (((T16 * T8) * (T4 * T2)) * t2);
+            const float U30 = fmaf(t, U31, -T32), U32 = fmaf(t, U31, T32);
+            up = odd ? U30 : fmaf(t2, U30, -U31);
+            uc = odd ? U32 : U31;
+          }
           float acc = 0.f;
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            acc = fmaf(v[c] * (float)(2 * c + role), uc, acc);
+          for (int c = 0; c < 16; ++c) {
+            const int m = 2 * c + odd + 32 * upper;
+            acc = fmaf(v[c] * (float)m, uc, acc);
             const float un = fmaf(T2x2, uc, -up);
             up = uc; uc = un;
           }
-          rp[role ? 35 : 32] += acc * dtdr;
+          drad = fmaf(acc, dtdr, drad);
         }
-        // spherical hidden layer, reverse: the four threads of a row take eight hidden units each and add their shares of the
-        // invariants' cotangents to the record
+        // spherical hidden layer, reverse: the four threads of a row take eight hidden units each
         {
-          float v[32];
-          tmem_ld32_combined(lane_base + 64, v);
+          float v[8];
+          tmem_ld8_combined(lane_base + 64 + 8 * role, v);
           const float4 s4 = ld4(rp + 4);
-          float ds0 = 0.f, ds1 = 0.f, ds2 = 0.f, ds3 = 0.f;
 #pragma unroll
           for (int c8 = 0; c8 < 8; ++c8) {
             const int c = 8 * role + c8;
@@ -1205,11 +1374,14 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
             const float4 k = ld4(p);
             const float z = fmaf(s4.x, k.x, fmaf(s4.y, k.y, fmaf(s4.z, k.z, fmaf(s4.w, k.w, p[4]))));
             const float sg = __fdividef(1.f, 1.f + __expf(-z));
-            const float vc = role == 0 ? v[c8] : (role == 1 ? v[8 + c8] : (role == 2 ? v[16 + c8] : v[24 + c8]));
-            const float dz = vc * sg * (1.f + z * (1.f - sg));
+            const float dz = v[c8] * sg * (1.f + z * (1.f - sg));
             ds0 = fmaf(dz, k.x, ds0); ds1 = fmaf(dz, k.y, ds1); ds2 = fmaf(dz, k.z, ds2); ds3 = fmaf(dz, k.w, ds3);
           }
-          atomicAdd(rp + 8, ds0); atomicAdd(rp + 9, ds1); atomicAdd(rp + 10, ds2); atomicAdd(rp + 11, ds3);
+          // the filter tile is free after the second filter's edge loops: it takes the four threads' shares
+          if (f == 1) {
+            st4(wt + (role * TE + row) * 4, make_float4(ds0, ds1, ds2, ds3));
+            wt[(4 * 4 + role) * TE + row] = drad;
+          }
         }
       }
       tc_fence_before();
@@ -1223,7 +1395,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       const bool on = rp[34] != 0.f;
       const int i = on ? __float_as_int(rp[1]) : -1;
       const float4 uu = ld4(rp + 28), ang = ld4(rp + 44);
-      const float g_r = rp[32] + rp[35];
+      const float* dr = wt + 4 * 4 * TE + tid;
+      const float g_r = rp[32] + ((dr[0] + dr[TE]) + (dr[2 * TE] + dr[3 * TE]));
       float fsx = on ? fmaf(g_r, uu.x, ang.x) : 0.f, fsy = on ? fmaf(g_r, uu.y, ang.y) : 0.f, fsz = on ? fmaf(g_r, uu.z, ang.z) : 0.f;
       if (virial && on) {
         // both ends' halves on the receiver's row, unless the partner's is not summed here (rows below n_own are)
@@ -1263,25 +1436,40 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       }
     }
     edge_loops(rpw, [&](auto full) {
-      int cur_i = -1;
+      const float sc = -2.f * invw(deg);
+      const float* dp0 = wt + rpw * warp * 4 + deg;
+      auto share = [&](int k) {      // derivative with respect to the receiver's component; the partner's is its negative
+        const float* dp = dp0 + 4 * k;
+        return sc * ((dp[0] + dp[TE * 4]) + (dp[2 * TE * 4] + dp[3 * TE * 4])) * dev8[k];
+      };
+      const float* rp0 = rec + rpw * warp * kBwRec;
+      int cur_i = __float_as_int(rp0[1]);
       float acc = 0.f;
+      if (full && cur_i == __float_as_int(rp0[7 * kBwRec + 1])) {      // eight pairs of one receiver
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (!full && k >= rpw) break;
-        const float* rp = rec + (rpw * warp + k) * kBwRec;
-        const int i = __float_as_int(rp[1]);
-        if (i != cur_i) {
-          if (cur_i >= 0 && lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
-          cur_i = i; acc = 0.f;
+        for (int k = 0; k < 8; ++k) {
+          const float t = share(k);
+          const int j = __float_as_int(rp0[k * kBwRec]);
+          acc += t;
+          if (lane < kMTot && j < n_scat) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
         }
-        if (lane < kMTot) {
-          const float t = -2.f * invw(deg) * rp[8 + deg] * dev8[k];
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (!full && k >= rpw) break;
+          const float* rp = rp0 + k * kBwRec;
+          const int i = __float_as_int(rp[1]);
+          if (i != cur_i) {
+            if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
+            cur_i = i; acc = 0.f;
+          }
+          const float t = share(k);
           const int j = __float_as_int(rp[0]);
           acc += t;
-          if (j < n_scat && rp[34] != 0.f) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
+          if (lane < kMTot && j < n_scat && rp[34] != 0.f) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
         }
       }
-      if (cur_i >= 0 && lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
+      if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
     });
     __syncthreads();
     BW_MARK(7);
