@@ -276,6 +276,7 @@ struct so3lr_b200_system {
   int shells[4] = {0, 0, 0, 0};  // domain-decomposed evaluation: owned | + short-range ghosts | (unused) | all local atoms
   SpeciesTables sp{};            // per-element-pair tables of the first layer (built by the first evaluation that reads them)
   std::vector<int> elements;     // the structure's elements while the tables are still to be built
+  int64_t graph_evals = 0;       // evaluations on caller-supplied lists
   float* GV = nullptr;           // n_cap x 32 scratch of the tabulated first-layer reverse pass
   float *dd_gev2 = nullptr, *dd_gev_in = nullptr;   // ping-pong cotangents of ev between the layers of the reverse pass
   so3lr_b200_options opt{};
@@ -530,6 +531,13 @@ void attn_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L,
   else launch_attn_bwd_sym(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, first_layer, virial);
 }
 
+void layer0_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, int n_recv, int n_gv, int n, float* F, int n_own) {
+  if (attention_mode() >= kAttnTcFwd)      // the compacted pair list is there
+    launch_layer0_bwd_pairs(st, S->sp, n_recv, n_gv, S->ve, S->d_Z, S->g_xa, S->gev1, S->GV, F, S->vir(), n_own);
+  else
+    launch_layer0_bwd_tab(st, S->sp, n_recv, n_gv, n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->d_Z, S->g_xa, S->gev1, S->GV, F, S->vir());
+}
+
 // SO3LR_B200_GRAPH=scatter keeps the graph-level call on the first-generation scatter kernels throughout (exact per-entry
 // gradients also for lists that are symmetric)
 bool graph_fast_path() {
@@ -568,16 +576,21 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
   fill(st, S->e_zbl, n, 0.f); fill(st, S->e_coul, n, 0.f); fill(st, S->e_disp, n, 0.f);
   fill(st, S->gq, n, 0.f); fill(st, S->gh, n, 0.f);
   S->prof.begin(kPGeom, st); launch_sr_geometry_zbl(st, M, S->cell, n, n_edges, edge_i, nbr_j, S->d_Z, nullptr, 1, dR, S->e_zbl, g_dR, ge, nullptr); S->prof.end(st);
-  { int rce = embed_atoms(S, st, n, S->x[0]); if (rce) return rce; }
+  const bool tab0 = tiled && S->sp.n_species > 0 && use_layer0_tables();
+  const bool fuse = use_mma_dense();   // q/k/v rows of layer l + 1 come out of layer l's dense block, their transpose goes into it
+  if (!tab0) { int rce = embed_atoms(S, st, n, S->x[0]); if (rce) return rce; }
   for (int l = 0; l < kNumLayers; ++l) {
     const LayerDev& L = M.layer[l];
-    S->prof.begin(kPProj, st); launch_proj_fwd(st, L, S->x[l], n, S->qkv[l]); S->prof.end(st);
+    if (!(l == 0 ? tab0 : fuse)) { S->prof.begin(kPProj, st); launch_proj_fwd(st, L, S->x[l], n, S->qkv[l]); S->prof.end(st); }
     S->prof.begin(kPAttnFwd, st);
-    if (tiled && L.has_spherical) launch_attn_fwd_tc(st, L, S->ve, n, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], S->d_flag + 1);
+    if (l == 0 && tab0) launch_layer0_fwd_tab(st, S->sp, M, n, n, row_ptr, nbr_j, dR, S->d_Z, S->xa[0], S->ev1[0]);
+    else if (tiled && L.has_spherical) launch_attn_fwd_tc(st, L, S->ve, n, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], S->d_flag + 1);
     else launch_attn_fwd(st, L, n, row_ptr, nbr_j, dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l]);
     S->prof.end(st);
     S->prof.begin(kPPostFwd, st);
-    post_fwd_dispatch(st, L, n, S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->x[l + 1], S->ev[l + 1], nullptr, nullptr, S->d_flag + 1);
+    const bool emit = fuse && l + 1 < kNumLayers;
+    post_fwd_dispatch(st, L, n, S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->x[l + 1], S->ev[l + 1],
+                      emit ? &M.layer[l + 1] : nullptr, emit ? S->qkv[l + 1] : nullptr, S->d_flag + 1);
     S->prof.end(st);
   }
   S->prof.begin(kPHeads, st);
@@ -605,7 +618,8 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
   for (int l = kNumLayers - 1; l >= 0; --l) {
     const LayerDev& L = M.layer[l];
     S->prof.begin(kPPostBwd, st);
-    post_bwd_dispatch(st, L, n, S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->g4, gev2, S->g_xa, S->gev1, nullptr, nullptr, S->d_flag + 1);
+    post_bwd_dispatch(st, L, n, S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->g4, gev2, S->g_xa, S->gev1,
+                      fuse && l + 1 < kNumLayers ? &M.layer[l + 1] : nullptr, S->g_qkv, S->d_flag + 1);
     S->prof.end(st);
     if (l > 0) {
       SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, S->gev1, (size_t)n * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, st));
@@ -619,10 +633,14 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
         launch_attn_bwd(st, L, n, row_ptr, nbr_j, dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, g_dR, 0);
       }
       S->prof.end(st);
-      // dL/dx_in = g_xa (skip connection) + projections^T
-      SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->g4, S->g_xa, (size_t)n * kF * sizeof(float), cudaMemcpyDeviceToDevice, st));
-      S->prof.begin(kPProjBwd, st); launch_proj_bwd(st, L, S->g_qkv, n, S->g4, 1); S->prof.end(st);
+      if (!fuse) {
+        // dL/dx_in = g_xa (skip connection) + projections^T
+        SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->g4, S->g_xa, (size_t)n * kF * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        S->prof.begin(kPProjBwd, st); launch_proj_bwd(st, L, S->g_qkv, n, S->g4, 1); S->prof.end(st);
+      }
       float* t = gev2; gev2 = gev_in; gev_in = t;
+    } else if (tab0) {
+      S->prof.begin(kPAttnBwd, st); launch_layer0_bwd_entries(st, S->sp, n, n_edges, edge_i, nbr_j, dR, S->d_Z, S->g_xa, S->gev1, S->GV, g_dR); S->prof.end(st);
     } else {
       S->prof.begin(kPAttnBwd, st); launch_attn_bwd(st, L, n, row_ptr, nbr_j, dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, nullptr, nullptr, g_dR, 1); S->prof.end(st);
     }
@@ -754,7 +772,7 @@ int fused_backward(so3lr_b200_system* S, cudaStream_t st, const Shells& c, float
     }
     S->prof.begin(l == 0 ? kPLayer0Bwd : kPAttnBwd, st);
     if (l == 0 && S->sp.n_species > 0 && use_layer0_tables())
-      launch_layer0_bwd_tab(st, S->sp, nattn[0], c.n3, c.n3, row_ptr, nbr_j, S->dR, S->d_Z, S->g_xa, S->gev1, S->GV, F, S->vir());
+      layer0_bwd_dispatch(S, st, nattn[0], c.n3, c.n3, F, c.n0);
     else
       attn_bwd_dispatch(S, st, L, nattn[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, F, l == 0 ? 1 : 0,
                         S->vir(), c.n0);
@@ -1408,7 +1426,18 @@ static int graph_eval_impl(so3lr_b200_system* S, void* stream, int64_t n_edges, 
   S->o_e_atom = S->e_atom; S->o_q = S->q; S->o_h = S->h; S->o_zbl = S->e_zbl; S->o_coul = S->e_coul; S->o_disp = S->e_disp;
   { row_ptr_from_sorted_kernel<<<(n + 1 + 255) / 256, 256, 0, st>>>(n, n_edges, idx_i, S->d_rowptr_g); count_launch(); }
   { row_ptr_from_sorted_kernel<<<(n + 1 + 255) / 256, 256, 0, st>>>(n, n_pairs, idx_i_lr, S->d_rowptr_lr_g); count_launch(); }
-  int rc = evaluate_graph(S, st, S->d_rowptr_g, idx_j, idx_i, n_edges, S->d_rowptr_lr_g, idx_j_lr, edges, edges_lr, g_edges, g_edges_lr,
+  // The first layer's element-pair tables pay from the second evaluation of a context on (forming them costs about what they save in
+  // one); a stream that is being captured takes them only if they are there.
+  int rc = kOk;
+  if (S->graph_evals++ > 0 && !S->elements.empty()) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
+    if (cap == cudaStreamCaptureStatusNone) {
+      rc = ensure_species_tables(S, st);
+      if (rc) return rc;
+    }
+  }
+  rc = evaluate_graph(S, st, S->d_rowptr_g, idx_j, idx_i, n_edges, S->d_rowptr_lr_g, idx_j_lr, edges, edges_lr, g_edges, g_edges_lr,
                           g_e_atom, positions, g_positions, strain6);
   if (rc) return rc;
   if (e_atom) SO3LR_CUDA_CHECK(cudaMemcpyAsync(e_atom, S->e_atom, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, st));
@@ -1894,7 +1923,7 @@ SO3LR_B200_API int so3lr_b200_dd_layer_backward_attn(so3lr_b200_system* S, void*
   const LayerDev& L = S->mctx.layer[l];
   S->prof.begin(l == 0 ? kPLayer0Bwd : kPAttnBwd, st);
   if (l == 0 && S->sp.n_species > 0 && use_layer0_tables())
-    launch_layer0_bwd_tab(st, S->sp, n0, S->shells[1], S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->d_Z, S->g_xa, S->gev1, S->GV, S->F_s, S->vir());
+    layer0_bwd_dispatch(S, st, n0, S->shells[1], S->n, S->F_s, n0);
   else
     attn_bwd_dispatch(S, st, L, n0, S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, S->dd_gev_in, S->F_s,
                       l == 0 ? 1 : 0, S->vir(), n0);

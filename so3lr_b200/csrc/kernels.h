@@ -223,6 +223,13 @@ void launch_layer0_fwd_tab(cudaStream_t s, const SpeciesTables& T, const ModelDe
 void launch_layer0_bwd_tab(cudaStream_t s, const SpeciesTables& T, int n_recv, int n_gv, int n, const int* row_ptr, const int* nbr_j,
                            const float* dR, const int* Z, const float* g_xa, const float* gev1, float* GV, float* F,
                            float* virial = nullptr);
+// the same from the compacted pair list of the tiled attention kernels (virial: rows below n_own add up to the total)
+void launch_layer0_bwd_pairs(cudaStream_t s, const SpeciesTables& T, int n_recv, int n_gv, const ValidEdges& V, const int* Z, const float* g_xa,
+                             const float* gev1, float* GV, float* F, float* virial, int n_own);
+// gradient with respect to every displacement of a caller-supplied list, added to g_dR
+void launch_layer0_bwd_entries(cudaStream_t s, const SpeciesTables& T, int n, long long n_entries, const int* idx_i, const int* idx_j,
+                               const float* dR, const int* Z, const float* g_xa, const float* gev1, float* GV, float* g_dR);
+
 
 // ---- pair_kernels.cu ----
 // dR for every short-range edge from positions (+ minimum image), ZBL energy into e_atom[centre], ZBL gradient

@@ -174,6 +174,78 @@ __global__ void __launch_bounds__(256) layer0_gv_kernel(SpeciesTables T, int n, 
   GV[(size_t)a * (4 * SP) + lane] = out;
 }
 
+// One direction (receiver of element zr, sender of element zs) of a pair's table entry: adds to the derivative with respect to r and
+// returns the equivariant logits x cutoff.  d1, d2: cotangents of the invariant and of the equivariant coefficients.
+__device__ __forceinline__ void table_reverse(const SpeciesTables& T, int zr, int zs, int g, float4 hv, float4 hd, float sc, float dcn, float4 d1,
+                                              const float (&d2)[4], float& gr, float (&a2)[4]) {
+  const float* row = T.table + ((size_t)(zr * SP + zs) * (kTableGrid - 1) + g) * 32;
+  const float4 v0a = ld4(row), v0b = ld4(row + 4), m0a = ld4(row + 8), m0b = ld4(row + 12);
+  const float4 v1a = ld4(row + 16), v1b = ld4(row + 20), m1a = ld4(row + 24), m1b = ld4(row + 28);
+  const float D1[4] = {hv.x * v0a.x + hv.y * m0a.x + hv.z * v1a.x + hv.w * m1a.x, hv.x * v0a.y + hv.y * m0a.y + hv.z * v1a.y + hv.w * m1a.y,
+                       hv.x * v0a.z + hv.y * m0a.z + hv.z * v1a.z + hv.w * m1a.z, hv.x * v0a.w + hv.y * m0a.w + hv.z * v1a.w + hv.w * m1a.w};
+  const float D2[4] = {hv.x * v0b.x + hv.y * m0b.x + hv.z * v1b.x + hv.w * m1b.x, hv.x * v0b.y + hv.y * m0b.y + hv.z * v1b.y + hv.w * m1b.y,
+                       hv.x * v0b.z + hv.y * m0b.z + hv.z * v1b.z + hv.w * m1b.z, hv.x * v0b.w + hv.y * m0b.w + hv.z * v1b.w + hv.w * m1b.w};
+  const float E1[4] = {hd.x * v0a.x + hd.y * m0a.x + hd.z * v1a.x + hd.w * m1a.x, hd.x * v0a.y + hd.y * m0a.y + hd.z * v1a.y + hd.w * m1a.y,
+                       hd.x * v0a.z + hd.y * m0a.z + hd.z * v1a.z + hd.w * m1a.z, hd.x * v0a.w + hd.y * m0a.w + hd.z * v1a.w + hd.w * m1a.w};
+  const float E2[4] = {hd.x * v0b.x + hd.y * m0b.x + hd.z * v1b.x + hd.w * m1b.x, hd.x * v0b.y + hd.y * m0b.y + hd.z * v1b.y + hd.w * m1b.y,
+                       hd.x * v0b.z + hd.y * m0b.z + hd.z * v1b.z + hd.w * m1b.z, hd.x * v0b.w + hd.y * m0b.w + hd.z * v1b.w + hd.w * m1b.w};
+  const float d1v[4] = {d1.x, d1.y, d1.z, d1.w};
+  float dsc = 0.f, dder = 0.f;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    dsc = fmaf(d1v[h], D1[h], fmaf(d2[h], D2[h], dsc));
+    dder = fmaf(d1v[h], E1[h], fmaf(d2[h], E2[h], dder));
+    a2[h] = sc * D2[h];
+  }
+  gr += dcn * dsc + sc * dder;
+}
+__device__ __forceinline__ int element_slot(const SpeciesTables& T, int z) { return T.slot[z < 0 ? 0 : (z > 118 ? 118 : z)]; }
+__device__ __forceinline__ void load_ev(const float* __restrict__ p, float (&v)[kMTot]) {
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const float4 q = ld4(p + 4 * c);
+    v[4 * c] = q.x; v[4 * c + 1] = q.y; v[4 * c + 2] = q.z; v[4 * c + 3] = q.w;
+  }
+}
+// Force on atom i of the pair (i, j), d = (dx, dy, dz) from i to j: both directions (BOTH), or the derivative of the direction (i <- j)
+// with respect to d alone.
+template <bool BOTH>
+__device__ __forceinline__ float3 pair_reverse(const SpeciesTables& T, int i, int j, float dx, float dy, float dz, float r, const int* __restrict__ Z,
+                                               const float* __restrict__ GV, const float* __restrict__ gev1) {
+  const float ir = 1.f / r, ux = dx * ir, uy = dy * ir, uz = dz * ir;
+  float cut, dcut;
+  phys_cutoff(r, cut, dcut);
+  const float sc = cut * kInvNbar, dcn = dcut * kInvNbar;
+  int g; float4 hv, hd;
+  hermite_weights(r, g, hv, hd);
+  const int zi = element_slot(T, Z[i]), zj = element_slot(T, Z[j]);
+  float Y[kMTot], gi[kMTot], gj[kMTot];
+  sph_harm_24(ux, uy, uz, Y);
+  load_ev(gev1 + (size_t)i * kMTot, gi);
+  if (BOTH) load_ev(gev1 + (size_t)j * kMTot, gj);
+  float dA2[4] = {0.f, 0.f, 0.f, 0.f}, dB2[4] = {0.f, 0.f, 0.f, 0.f}, a2A[4], a2B[4], gr = 0.f;
+#pragma unroll
+  for (int m = 0; m < kMTot; ++m) {
+    dA2[degree_of(m)] = fmaf(gi[m], Y[m], dA2[degree_of(m)]);
+    if (BOTH) dB2[degree_of(m)] = fmaf(gj[m], Y[m], dB2[degree_of(m)]);
+  }
+  dB2[0] = -dB2[0]; dB2[2] = -dB2[2];       // Y_lm(-u) = (-1)^l Y_lm(u)
+  table_reverse(T, zi, zj, g, hv, hd, sc, dcn, ld4(GV + (size_t)i * (4 * SP) + 4 * zj), dA2, gr, a2A);
+  if (BOTH) table_reverse(T, zj, zi, g, hv, hd, sc, dcn, ld4(GV + (size_t)j * (4 * SP) + 4 * zi), dB2, gr, a2B);
+  float gY[kMTot];
+#pragma unroll
+  for (int m = 0; m < kMTot; ++m) {
+    const int l = degree_of(m);
+    const float sgn = (l == 0 || l == 2) ? -1.f : 1.f;
+    gY[m] = BOTH ? a2A[l] * gi[m] + sgn * a2B[l] * gj[m] : a2A[l] * gi[m];
+  }
+  float gux, guy, guz;
+  sph_harm_24_vjp(ux, uy, uz, gY, gux, guy, guz);
+  const float gd = gux * ux + guy * uy + guz * uz;
+  return make_float3(gr * ux + (gux - gd * ux) * ir, gr * uy + (guy - gd * uy) * ir, gr * uz + (guz - gd * uz) * ir);
+}
+
+// Forces from the full list, a warp per receiver (with the attention kernels that do not build the compacted pair list).
 __global__ void __launch_bounds__(256) layer0_bwd_tab_kernel(SpeciesTables T, int n_recv, int n, const int* __restrict__ row_ptr,
                                                              const int* __restrict__ nbr_j, const float* __restrict__ dR,
                                                              const int* __restrict__ Z, const float* __restrict__ GV,
@@ -182,15 +254,6 @@ __global__ void __launch_bounds__(256) layer0_bwd_tab_kernel(SpeciesTables T, in
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= n_recv) return;
-  const int Zi = Z[i];
-  const int zi = T.slot[Zi < 0 ? 0 : (Zi > 118 ? 118 : Zi)];
-  const float* GVi = GV + (size_t)i * (4 * SP);
-  float gevi[kMTot];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    const float4 v = ld4(gev1 + (size_t)i * kMTot + 4 * c);
-    gevi[4 * c] = v.x; gevi[4 * c + 1] = v.y; gevi[4 * c + 2] = v.z; gevi[4 * c + 3] = v.w;
-  }
   float fx = 0.f, fy = 0.f, fz = 0.f;
   VirialAcc va;
   const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
@@ -199,77 +262,72 @@ __global__ void __launch_bounds__(256) layer0_bwd_tab_kernel(SpeciesTables T, in
     const float dx = dR[3 * (size_t)e], dy = dR[3 * (size_t)e + 1], dz = dR[3 * (size_t)e + 2];
     const float r2 = dx * dx + dy * dy + dz * dz;
     if (j < 0 || j >= n || !(r2 < kRc2) || !(r2 > 0.f)) continue;
-    const float r = sqrtf(r2), ir = 1.f / r;
-    const float ux = dx * ir, uy = dy * ir, uz = dz * ir;
-    float cut, dcut;
-    phys_cutoff(r, cut, dcut);
-    const float sc = cut * kInvNbar, dcn = dcut * kInvNbar;
-    int g; float4 hv, hd;
-    hermite_weights(r, g, hv, hd);
-    const int Zj = Z[j];
-    const int zj = T.slot[Zj < 0 ? 0 : (Zj > 118 ? 118 : Zj)];
-    float Y[kMTot];
-    sph_harm_24(ux, uy, uz, Y);
-    const float* gevj = gev1 + (size_t)j * kMTot;
-    float dA2[4] = {0.f, 0.f, 0.f, 0.f}, dB2[4] = {0.f, 0.f, 0.f, 0.f}, gj[kMTot];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      const float4 v = ld4(gevj + 4 * c);
-      gj[4 * c] = v.x; gj[4 * c + 1] = v.y; gj[4 * c + 2] = v.z; gj[4 * c + 3] = v.w;
-    }
-#pragma unroll
-    for (int m = 0; m < kMTot; ++m) {
-      dA2[degree_of(m)] = fmaf(gevi[m], Y[m], dA2[degree_of(m)]);
-      dB2[degree_of(m)] = fmaf(gj[m], Y[m], dB2[degree_of(m)]);
-    }
-    dB2[0] = -dB2[0]; dB2[2] = -dB2[2];       // Y_lm(-u) = (-1)^l Y_lm(u)
-    const float4 dA1 = ld4(GVi + 4 * zj);                          // cotangents of the invariant coefficients, edge (i<-j)
-    const float4 dB1 = ld4(GV + (size_t)j * (4 * SP) + 4 * zi);    // and edge (j<-i)
-    float gr = 0.f, a2A[4], a2B[4];
-#pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
-      const float* row = T.table + ((size_t)((dir ? zj : zi) * SP + (dir ? zi : zj)) * (kTableGrid - 1) + g) * 32;
-      const float4 v0a = ld4(row), v0b = ld4(row + 4), m0a = ld4(row + 8), m0b = ld4(row + 12);
-      const float4 v1a = ld4(row + 16), v1b = ld4(row + 20), m1a = ld4(row + 24), m1b = ld4(row + 28);
-      const float4 d1 = dir ? dB1 : dA1;
-      const float* d2 = dir ? dB2 : dA2;
-      const float D1[4] = {hv.x * v0a.x + hv.y * m0a.x + hv.z * v1a.x + hv.w * m1a.x, hv.x * v0a.y + hv.y * m0a.y + hv.z * v1a.y + hv.w * m1a.y,
-                           hv.x * v0a.z + hv.y * m0a.z + hv.z * v1a.z + hv.w * m1a.z, hv.x * v0a.w + hv.y * m0a.w + hv.z * v1a.w + hv.w * m1a.w};
-      const float D2[4] = {hv.x * v0b.x + hv.y * m0b.x + hv.z * v1b.x + hv.w * m1b.x, hv.x * v0b.y + hv.y * m0b.y + hv.z * v1b.y + hv.w * m1b.y,
-                           hv.x * v0b.z + hv.y * m0b.z + hv.z * v1b.z + hv.w * m1b.z, hv.x * v0b.w + hv.y * m0b.w + hv.z * v1b.w + hv.w * m1b.w};
-      const float E1[4] = {hd.x * v0a.x + hd.y * m0a.x + hd.z * v1a.x + hd.w * m1a.x, hd.x * v0a.y + hd.y * m0a.y + hd.z * v1a.y + hd.w * m1a.y,
-                           hd.x * v0a.z + hd.y * m0a.z + hd.z * v1a.z + hd.w * m1a.z, hd.x * v0a.w + hd.y * m0a.w + hd.z * v1a.w + hd.w * m1a.w};
-      const float E2[4] = {hd.x * v0b.x + hd.y * m0b.x + hd.z * v1b.x + hd.w * m1b.x, hd.x * v0b.y + hd.y * m0b.y + hd.z * v1b.y + hd.w * m1b.y,
-                           hd.x * v0b.z + hd.y * m0b.z + hd.z * v1b.z + hd.w * m1b.z, hd.x * v0b.w + hd.y * m0b.w + hd.z * v1b.w + hd.w * m1b.w};
-      const float d1v[4] = {d1.x, d1.y, d1.z, d1.w};
-      float dsc = 0.f, dder = 0.f;
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        dsc = fmaf(d1v[h], D1[h], fmaf(d2[h], D2[h], dsc));
-        dder = fmaf(d1v[h], E1[h], fmaf(d2[h], E2[h], dder));
-        if (dir == 0) a2A[h] = sc * D2[h]; else a2B[h] = sc * D2[h];
-      }
-      gr += dcn * dsc + sc * dder;
-    }
-    float gY[kMTot];
-#pragma unroll
-    for (int m = 0; m < kMTot; ++m) {
-      const int l = degree_of(m);
-      const float sgn = (l == 0 || l == 2) ? -1.f : 1.f;
-      gY[m] = a2A[l] * gevi[m] + sgn * a2B[l] * gj[m];
-    }
-    float gux, guy, guz;
-    sph_harm_24_vjp(ux, uy, uz, gY, gux, guy, guz);
-    const float gd = gux * ux + guy * uy + guz * uz;
-    const float fsx = gr * ux + (gux - gd * ux) * ir;
-    const float fsy = gr * uy + (guy - gd * uy) * ir;
-    const float fsz = gr * uz + (guz - gd * uz) * ir;
-    fx += fsx; fy += fsy; fz += fsz;
-    if (virial) va.add(0.5f, dx, dy, dz, fsx, fsy, fsz);
+    const float3 f = pair_reverse<true>(T, i, j, dx, dy, dz, sqrtf(r2), Z, GV, gev1);
+    fx += f.x; fy += f.y; fz += f.z;
+    if (virial) va.add(0.5f, dx, dy, dz, f.x, f.y, f.z);
   }
   fx = warp_sum(fx); fy = warp_sum(fy); fz = warp_sum(fz);
   if (lane == 0) { F[3 * (size_t)i] += fx; F[3 * (size_t)i + 1] += fy; F[3 * (size_t)i + 2] += fz; }
   if (virial) va.flush_warp(virial, (size_t)i, lane);
+}
+
+// Forces from the compacted pair list (one entry per undirected pair, sorted by its receiver): a thread per pair, so that every lane
+// has one (the full list's rows hold the skin too and leave 45 % of the lanes without work, and every pair was evaluated at both ends).
+// Equal receivers inside a warp are summed before they go out; the partner gets its share if it owns a row.  Rows of `virial` below
+// n_own add up to the total, in any distribution: every warp adds its sum to one of them.
+__global__ void __launch_bounds__(128) layer0_bwd_pairs_kernel(SpeciesTables T, int n_recv, const int* __restrict__ vrow_ptr,
+                                                               const int* __restrict__ ve_i, const int* __restrict__ ve_j,
+                                                               const float4* __restrict__ ve_d, const int* __restrict__ Z,
+                                                               const float* __restrict__ GV, const float* __restrict__ gev1,
+                                                               float* __restrict__ F, float* __restrict__ virial, int n_own) {
+  const int lane = threadIdx.x & 31;
+  const long long n_pairs = vrow_ptr[n_recv];
+  const long long warp0 = (long long)blockIdx.x * 4 + (threadIdx.x >> 5), step = (long long)gridDim.x * 128;
+  VirialAcc va;
+  for (long long e0 = 32 * warp0; e0 < n_pairs; e0 += step) {
+    const long long e = e0 + lane;
+    int i = -1, j = -1;
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    if (e < n_pairs) {
+      i = ve_i[e]; j = ve_j[e];
+      const float4 d = ve_d[e];
+      f = pair_reverse<true>(T, i, j, d.x, d.y, d.z, d.w, Z, GV, gev1);
+      if (virial) va.add(0.5f * ((i < n_own ? 1.f : 0.f) + (j < n_own ? 1.f : 0.f)), d.x, d.y, d.z, f.x, f.y, f.z);
+      if (j < n_recv) { atomicAdd(F + 3 * (size_t)j, -f.x); atomicAdd(F + 3 * (size_t)j + 1, -f.y); atomicAdd(F + 3 * (size_t)j + 2, -f.z); }
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float tx = __shfl_up_sync(0xffffffffu, f.x, o), ty = __shfl_up_sync(0xffffffffu, f.y, o), tz = __shfl_up_sync(0xffffffffu, f.z, o);
+      const int ti = __shfl_up_sync(0xffffffffu, i, o);
+      if (lane >= o && ti == i) { f.x += tx; f.y += ty; f.z += tz; }
+    }
+    const int inext = __shfl_down_sync(0xffffffffu, i, 1);
+    if (i >= 0 && (lane == 31 || inext != i)) {
+      atomicAdd(F + 3 * (size_t)i, f.x); atomicAdd(F + 3 * (size_t)i + 1, f.y); atomicAdd(F + 3 * (size_t)i + 2, f.z);
+    }
+  }
+  if (virial && n_own > 0 && 32 * warp0 < n_pairs) {
+    const float a = warp_sum(va.xx), b = warp_sum(va.yy), c = warp_sum(va.zz), d = warp_sum(va.yz), e = warp_sum(va.xz), h = warp_sum(va.xy);
+    if (lane == 0) {
+      float* w = virial + 6 * (size_t)(warp0 % n_own);
+      atomicAdd(w, a); atomicAdd(w + 1, b); atomicAdd(w + 2, c); atomicAdd(w + 3, d); atomicAdd(w + 4, e); atomicAdd(w + 5, h);
+    }
+  }
+}
+
+// Gradient with respect to every displacement of a caller-supplied list (added to g_dR); the list may be of any form.
+__global__ void __launch_bounds__(128) layer0_bwd_entries_kernel(SpeciesTables T, int n, long long n_entries, const int* __restrict__ idx_i,
+                                                                 const int* __restrict__ idx_j, const float* __restrict__ dR,
+                                                                 const int* __restrict__ Z, const float* __restrict__ GV,
+                                                                 const float* __restrict__ gev1, float* __restrict__ g_dR) {
+  const long long e = (long long)blockIdx.x * 128 + threadIdx.x;
+  if (e >= n_entries) return;
+  const int i = idx_i[e], j = idx_j[e];
+  const float dx = dR[3 * e], dy = dR[3 * e + 1], dz = dR[3 * e + 2];
+  const float r2 = dx * dx + dy * dy + dz * dz;
+  if (i < 0 || i >= n || j < 0 || j >= n || !(r2 < kRc2) || !(r2 > 0.f)) return;
+  const float3 f = pair_reverse<false>(T, i, j, dx, dy, dz, sqrtf(r2), Z, GV, gev1);
+  g_dR[3 * e] += f.x; g_dR[3 * e + 1] += f.y; g_dR[3 * e + 2] += f.z;
 }
 
 }  // namespace
@@ -330,6 +388,23 @@ void launch_layer0_bwd_tab(cudaStream_t s, const SpeciesTables& T, int n_recv, i
   if (n_recv <= 0) return;
   { layer0_gv_kernel<<<(n_gv + 7) / 8, 256, 0, s>>>(T, n_gv, g_xa, GV); count_launch(); }
   { layer0_bwd_tab_kernel<<<(n_recv + 7) / 8, 256, 0, s>>>(T, n_recv, n, row_ptr, nbr_j, dR, Z, GV, gev1, F, virial); count_launch(); }
+}
+
+void launch_layer0_bwd_pairs(cudaStream_t s, const SpeciesTables& T, int n_recv, int n_gv, const ValidEdges& V, const int* Z, const float* g_xa,
+                             const float* gev1, float* GV, float* F, float* virial, int n_own) {
+  if (n_recv <= 0) return;
+  { layer0_gv_kernel<<<(n_gv + 7) / 8, 256, 0, s>>>(T, n_gv, g_xa, GV); count_launch(); }
+  // the number of pairs stays on the device: four CTAs per SM walk over the list, fewer where the rows cannot fill them
+  int blocks = (int)(((long long)n_recv * 24 + 127) / 128);
+  if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
+  { layer0_bwd_pairs_kernel<<<blocks, 128, 0, s>>>(T, n_recv, V.row_ptr, V.i, V.j, V.d, Z, GV, gev1, F, virial, n_own); count_launch(); }
+}
+
+void launch_layer0_bwd_entries(cudaStream_t s, const SpeciesTables& T, int n, long long n_entries, const int* idx_i, const int* idx_j,
+                               const float* dR, const int* Z, const float* g_xa, const float* gev1, float* GV, float* g_dR) {
+  if (n <= 0 || n_entries <= 0) return;
+  { layer0_gv_kernel<<<(n + 7) / 8, 256, 0, s>>>(T, n, g_xa, GV); count_launch(); }
+  { layer0_bwd_entries_kernel<<<(unsigned)((n_entries + 127) / 128), 128, 0, s>>>(T, n, n_entries, idx_i, idx_j, dR, Z, GV, gev1, g_dR); count_launch(); }
 }
 
 }  // namespace so3lr

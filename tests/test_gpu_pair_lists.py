@@ -57,12 +57,18 @@ def test_list_forms_against_the_oracle(name, form):
     n = len(Z)
     s = System(Z, cell, cutoff_lr=6.0 if cell is not None else 100.0, damping=2.0, lr_format="sparse")
     t = lambda a: torch.tensor(a, device="cuda")
-    o = s.graph_eval(t(i), t(j), t(d), t(il), t(jl), t(dl))
+    # the first evaluation of a context runs the generic first layer, later ones its tables
+    results = [s.graph_eval(t(i), t(j), t(d), t(il), t(jl), t(dl)) for _ in range(2)]
     D, DL = torch.tensor(d, dtype=torch.float64, requires_grad=True), torch.tensor(dl, dtype=torch.float64, requires_grad=True)
     e, _ = O.energy_from_graph(O.load_params(), Z, D, i, j, DL, il, jl, lr_format="sparse", cutoff_lr=6.0 if cell is not None else 100.0, damping=2.0)
     g, = torch.autograd.grad(e.sum(), D)
-    got = o["g_edges"].double().cpu()
     e = e.detach()
+    for o in results:
+        _check(o, e, g, i, j, D.detach(), n, form)
+
+
+def _check(o, e, g, i, j, D, n, form):
+    got = o["g_edges"].double().cpu()
     assert float((o["e_atom"].double().cpu() - e).abs().sum()) <= 1e-5 * float(e.abs().sum())
     if form in ("one_way", "twice_one_way"):      # lists without partners: the gradient of every entry
         assert float((got - g).abs().max()) <= 1e-4
@@ -72,7 +78,6 @@ def test_list_forms_against_the_oracle(name, form):
     ti, tj = torch.tensor(i)[m], torch.tensor(j)[m]
     f = lambda x: torch.zeros(n, 3, dtype=torch.float64).index_add(0, ti, x[m]).index_add(0, tj, -x[m])
     assert float((f(got) - f(g)).abs().max()) <= (2e-4 if form == "twice" else 1e-4)
-    Dd = D.detach()
-    w, wr = Dd.T @ got, Dd.T @ g
+    w, wr = D.T @ got, D.T @ g
     assert float((w - wr).abs().max()) <= 1e-4 * max(1.0, float(wr.abs().max()))
     assert float(got[~m].abs().sum()) == 0.0
