@@ -197,6 +197,7 @@ struct Cell {
   float h[9];     // rows = lattice vectors
   float hinv[9];  // inverse, so that s = dR @ hinv
   int periodic;   // 0: free space
+  int ortho;      // 1: every off-diagonal element of h and hinv is zero
 };
 
 // minimum-image displacement: dR - round(dR h^-1) h, the operation order of oracle.min_image.  The lattice translation is
@@ -206,6 +207,12 @@ struct Cell {
 SO3LR_HD void min_image(const Cell& c, float& dx, float& dy, float& dz) {
   if (!c.periodic) return;
 #ifdef __CUDA_ARCH__
+  if (c.ortho) {      // the same operations without those on zeros: bit for bit the same result with a quarter of the instructions
+    dx = __fsub_rn(dx, __fmul_rn(rintf(__fmul_rn(dx, c.hinv[0])), c.h[0]));
+    dy = __fsub_rn(dy, __fmul_rn(rintf(__fmul_rn(dy, c.hinv[4])), c.h[4]));
+    dz = __fsub_rn(dz, __fmul_rn(rintf(__fmul_rn(dz, c.hinv[8])), c.h[8]));
+    return;
+  }
   const float k0 = rintf(__fadd_rn(__fadd_rn(__fmul_rn(dx, c.hinv[0]), __fmul_rn(dy, c.hinv[3])), __fmul_rn(dz, c.hinv[6])));
   const float k1 = rintf(__fadd_rn(__fadd_rn(__fmul_rn(dx, c.hinv[1]), __fmul_rn(dy, c.hinv[4])), __fmul_rn(dz, c.hinv[7])));
   const float k2 = rintf(__fadd_rn(__fadd_rn(__fmul_rn(dx, c.hinv[2]), __fmul_rn(dy, c.hinv[5])), __fmul_rn(dz, c.hinv[8])));

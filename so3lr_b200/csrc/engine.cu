@@ -223,6 +223,9 @@ int make_cell(const float* cell9, Cell* c) {
   inv[6] = (h[3] * h[7] - h[4] * h[6]) / det; inv[7] = (h[1] * h[6] - h[0] * h[7]) / det; inv[8] = (h[0] * h[4] - h[1] * h[3]) / det;
   for (int k = 0; k < 9; ++k) { c->h[k] = (float)h[k]; c->hinv[k] = (float)inv[k]; }
   c->periodic = 1;
+  c->ortho = 1;
+  for (int k = 0; k < 9; ++k)
+    if (k % 4 != 0 && (c->h[k] != 0.f || c->hinv[k] != 0.f)) c->ortho = 0;
   return kOk;
 }
 

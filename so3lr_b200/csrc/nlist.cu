@@ -30,6 +30,8 @@ struct NlistWorkspace {
   void* sort_tmp = nullptr;
   size_t sort_bytes = 0;
   int key_cap = 0;
+  unsigned* masks = nullptr;   // votes of the row count for the fill
+  size_t mask_cap = 0;
 };
 
 NlistWorkspace* nlist_workspace_create() { return new NlistWorkspace(); }
@@ -37,7 +39,7 @@ void nlist_workspace_destroy(NlistWorkspace* w) {
   if (!w) return;
   dev_free(w->cell_of); dev_free(w->cell_sorted); dev_free(w->atom_sorted); dev_free(w->atom_iota);
   dev_free(w->cell_start); dev_free(w->row_count); dev_free(w->cub_tmp); dev_free(w->d_total);
-  dev_free(w->key); dev_free(w->key_sorted); dev_free(w->sort_tmp); dev_free(w->pos_sorted);
+  dev_free(w->key); dev_free(w->key_sorted); dev_free(w->sort_tmp); dev_free(w->pos_sorted); dev_free(w->masks);
   if (w->h_total) host_free(w->h_total);
   delete w;
 }
@@ -95,12 +97,18 @@ __global__ void gather_sorted_positions_kernel(int n, const float* __restrict__ 
 }
 
 // FILL = false: row_count[i] = number of neighbours.  FILL = true: write rows at row_ptr[i].
+// The candidates of a row come in cell order.  Cells that are neighbours along the first axis are neighbours in the sorted array: up to
+// three of them are walked as one range (the 5.5 A cells of the short-range list hold half a warp of atoms each).  In an orthorhombic
+// box a cell further from the atom than the list's radius is left out: of the 27 cells of edge r, 20.6 remain on average.  The count
+// leaves the warps' votes in `masks` (optional, mask_stride words per row), and the fill takes them instead of testing every candidate
+// a second time; a row that needs more words is tested again.
 template <bool FILL>
-__global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int n, const float* __restrict__ R, float r2max,
+__global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int n, const float* __restrict__ R, float r_list, float r2max,
                                                          int ordered, const int* __restrict__ seg,
                                                          const float4* __restrict__ pos_sorted, const int* __restrict__ cell_start,
                                                          int* __restrict__ row_count, const int* __restrict__ row_ptr,
-                                                         int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity) {
+                                                         int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
+                                                         unsigned* __restrict__ masks, int mask_stride) {
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= n) return;
@@ -108,8 +116,54 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
   const int segi = seg ? seg[i] : 0;
   int ci[3];
   cell_coords(cell, G, xi, yi, zi, ci);
+  // squared distances from the atom to the neighbouring cells along each axis (lower bounds; 0 where they are not known)
+  float gap2[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+  const bool prune = cell.periodic && cell.ortho;
+  if (prune) {
+    const float x[3] = {xi, yi, zi};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (G.nc[k] < 3) continue;
+      float s = x[k] * cell.hinv[4 * k];
+      s -= floorf(s);
+      const float t = s * G.nc[k] - (float)ci[k], w = fabsf(cell.h[4 * k]) / (float)G.nc[k];      // position inside the cell, its width
+      const float margin = 1e-5f * fabsf(cell.h[4 * k]) + 1e-6f * fabsf(x[k]) + 1e-3f;                                   // roundings of positions and cells
+      const float below = fmaxf(t * w - margin, 0.f), above = fmaxf((1.f - t) * w - margin, 0.f);
+      gap2[k][0] = below * below; gap2[k][2] = above * above;
+    }
+  }
+  const float reach2 = r_list * r_list;
   long long base = FILL ? row_ptr[i] : 0;
-  int count = 0;
+  int count = 0, word = 0;
+  unsigned* mine = masks ? masks + (size_t)i * mask_stride : nullptr;
+  auto range = [&](int s0, int s1) {
+    for (int k0 = s0; k0 < s1; k0 += 32, ++word) {
+      const int k = k0 + lane;
+      unsigned m;
+      int j = -1;
+      if (FILL && mine && word < mask_stride) {
+        m = mine[word];
+        if ((m >> lane) & 1u) j = __float_as_int(pos_sorted[k].w);
+      } else {
+        bool hit = false;
+        if (k < s1) {
+          const float4 pj = pos_sorted[k];
+          j = __float_as_int(pj.w);
+          float dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
+          min_image(cell, dx, dy, dz);
+          const float dd = dist2_rn(dx, dy, dz);
+          hit = dd < r2max && (ordered ? j > i : j != i) && (!seg || seg[j] == segi);
+        }
+        m = __ballot_sync(0xffffffffu, hit);
+        if (!FILL && mine && word < mask_stride && lane == 0) mine[word] = m;
+      }
+      if (FILL && ((m >> lane) & 1u)) {
+        long long pos = base + count + __popc(m & ((1u << lane) - 1u));
+        if (pos < capacity) { nbr_j[pos] = j; edge_i[pos] = i; }
+      }
+      count += __popc(m);
+    }
+  };
   const int lo0 = G.nc[0] > 1 ? -1 : 0, hi0 = G.nc[0] > 1 ? 1 : 0;
   const int lo1 = G.nc[1] > 1 ? -1 : 0, hi1 = G.nc[1] > 1 ? 1 : 0;
   const int lo2 = G.nc[2] > 1 ? -1 : 0, hi2 = G.nc[2] > 1 ? 1 : 0;
@@ -119,31 +173,20 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
     for (int d1 = lo1; d1 <= hi1; ++d1) {
       int c1 = ci[1] + d1;
       if (G.wrap[1]) c1 = (c1 + G.nc[1]) % G.nc[1]; else if (c1 < 0 || c1 >= G.nc[1]) continue;
+      const float g12 = (d1 < 0 ? gap2[1][0] : (d1 > 0 ? gap2[1][2] : 0.f)) + (d2 < 0 ? gap2[2][0] : (d2 > 0 ? gap2[2][2] : 0.f));
+      if (g12 > reach2) continue;
+      const int row = (c2 * G.nc[1] + c1) * G.nc[0];
+      int open0 = -1, open1 = -1;      // range under way
       for (int d0 = lo0; d0 <= hi0; ++d0) {
         int c0 = ci[0] + d0;
         if (G.wrap[0]) c0 = (c0 + G.nc[0]) % G.nc[0]; else if (c0 < 0 || c0 >= G.nc[0]) continue;
-        const int c = (c2 * G.nc[1] + c1) * G.nc[0] + c0;
-        const int s0 = cell_start[c], s1 = cell_start[c + 1];
-        for (int k0 = s0; k0 < s1; k0 += 32) {
-          const int k = k0 + lane;
-          bool hit = false;
-          int j = -1;
-          if (k < s1) {
-            const float4 pj = pos_sorted[k];
-            j = __float_as_int(pj.w);
-            float dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
-            min_image(cell, dx, dy, dz);
-            const float dd = dist2_rn(dx, dy, dz);
-            hit = dd < r2max && (ordered ? j > i : j != i) && (!seg || seg[j] == segi);
-          }
-          const unsigned m = __ballot_sync(0xffffffffu, hit);
-          if (FILL && hit) {
-            long long pos = base + count + __popc(m & ((1u << lane) - 1u));
-            if (pos < capacity) { nbr_j[pos] = j; edge_i[pos] = i; }
-          }
-          count += __popc(m);
-        }
+        if (d0 != 0 && g12 + (d0 < 0 ? gap2[0][0] : gap2[0][2]) > reach2) continue;
+        const int s0 = cell_start[row + c0], s1 = cell_start[row + c0 + 1];
+        if (s0 == open1) { open1 = s1; continue; }
+        if (open1 > open0) range(open0, open1);
+        open0 = s0; open1 = s1;
       }
+      if (open1 > open0) range(open0, open1);
     }
   }
   if (!FILL && lane == 0) row_count[i] = count;
@@ -391,11 +434,29 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   }
   const int blocks = (n_rows + 7) / 8;
   if (n_rows == 0) { out->count = 0; return kOk; }
+  // votes of the count for the fill: room for 1.25 times the mean number of candidates of a row (and one partial word per range); 0.8 KB
+  // per atom for the 12 A list of water.  Short of memory the fill tests the candidates again.
+  unsigned* masks = nullptr;
+  int mask_stride = 0;
+  if (!by_graph) {
+    double cells = 1.0;
+    for (int k = 0; k < 3; ++k) cells *= G.nc[k] > 1 ? 3.0 : 1.0;
+    const double mean = cells * (double)n / (double)n_cells;
+    mask_stride = (int)std::min(mean * 1.25 / 32.0 + 12.0, 1024.0);
+    const size_t words = (size_t)n_rows * mask_stride;
+    if (words > w->mask_cap) {
+      if (w->masks) dev_free(w->masks);
+      w->masks = nullptr; w->mask_cap = 0;
+      if (dev_alloc(&w->masks, words) == cudaSuccess) w->mask_cap = words;
+      else { w->masks = nullptr; cudaGetLastError(); }
+    }
+    masks = w->masks;
+  }
   if (by_graph)
     { build_rows_graph_kernel<false><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, w->row_count, nullptr, nullptr, nullptr, 0); count_launch(); }
   else
-    { build_rows_kernel<false><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r2max, ordered, seg, w->pos_sorted, w->cell_start,
-                                                    w->row_count, nullptr, nullptr, nullptr, 0); count_launch(); }
+    { build_rows_kernel<false><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r_list, r2max, ordered, seg, w->pos_sorted, w->cell_start,
+                                                    w->row_count, nullptr, nullptr, nullptr, 0, masks, mask_stride); count_launch(); }
   SO3LR_CUDA_CHECK(cudaMemsetAsync(w->d_total, 0, sizeof(long long), s));
   { int tb = (n_rows + 255) / 256; if (tb > 1024) tb = 1024;
     row_total_kernel<<<tb, 256, 0, s>>>(n_rows, w->row_count, reinterpret_cast<unsigned long long*>(w->d_total)); count_launch(); }
@@ -426,8 +487,8 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     { build_rows_graph_kernel<true><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, nullptr, out->row_ptr,
                                                          out->nbr_j, out->edge_i, out->capacity); count_launch(); }
   else
-    { build_rows_kernel<true><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r2max, ordered, seg, w->pos_sorted, w->cell_start, nullptr,
-                                                   out->row_ptr, out->nbr_j, out->edge_i, out->capacity); count_launch(); }
+    { build_rows_kernel<true><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r_list, r2max, ordered, seg, w->pos_sorted, w->cell_start, nullptr,
+                                                   out->row_ptr, out->nbr_j, out->edge_i, out->capacity, masks, mask_stride); count_launch(); }
   if (truncated) { clamp_rows_kernel<<<(n_rows + 1 + 255) / 256, 256, 0, s>>>(n_rows, out->row_ptr, out->capacity); count_launch(); }
   SO3LR_CUDA_CHECK(cudaGetLastError());
   return truncated ? kOverflow : kOk;

@@ -1,0 +1,39 @@
+"""Neighbor lists of the cell builder (csrc/nlist.cu) against a float64 search over all pairs: boxes of 1, 3, 4 and more cells per axis,
+orthorhombic (cells beyond the radius are left out) and skew, atoms far outside the box, counts around a warp's width.  Pairs
+within 1e-4 A of the radius may fall on either side."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,edge,skew,spread", [(2, 14.0, 0.0, 0), (33, 13.0, 0.0, 0), (600, 16.6, 0.0, 0), (600, 16.6, 0.0, 3), (700, 23.0, 0.0, 0),
+                                                (700, 23.0, 3.0, 2), (1500, (14.1, 31.0, 20.5), 0.0, 2), (2600, 38.0, 0.0, 1), (2600, 38.0, 5.0, 0)])
+@pytest.mark.parametrize("ordered", [False, True])
+def test_rows_are_exact(n, edge, skew, spread, ordered):
+    from so3lr_b200.engine import System
+    rng = np.random.default_rng(n)
+    L = np.broadcast_to(np.asarray(edge, float), 3)
+    cell = np.diag(L).astype(np.float32).astype(np.float64)
+    cell[1, 0], cell[2, 1] = skew, -skew
+    f = rng.random((n, 3))
+    f[: n // 4] = np.round(f[: n // 4] * 4) / 4 + rng.normal(scale=1e-6, size=(n // 4, 3))      # on the borders of cells
+    R = ((f + rng.integers(-spread, spread + 1, (n, 3))) @ cell).astype(np.float32)
+    s = System(np.full(n, 8), cell, cutoff_lr=6.0, damping=2.0, lr_format="ordered_sparse" if ordered else "sparse")
+    Rt = torch.tensor(R, device="cuda")
+    for which, rc in ((0, 4.5), (1, 6.0)):
+        _, count, _ = s.neighbor_list(Rt, which, 1)
+        idx, count, over = s.neighbor_list(Rt, which, max(int(count), 1))
+        i, j = idx[:, : int(count)].cpu().numpy().astype(np.int64)
+        d = R[None].astype(np.float64) - R[:, None]
+        d -= np.round(d @ np.linalg.inv(cell)) @ cell
+        r = np.sqrt((d ** 2).sum(-1))
+        np.fill_diagonal(r, 1e9)
+        if which == 1 and ordered:
+            r[np.tril_indices(n)] = 1e9
+        got = np.zeros((n, n), dtype=np.int64)
+        np.add.at(got, (i, j), 1)
+        assert got.max(initial=0) <= 1 and (np.diff(i) >= 0).all()
+        sure, never = r < rc - 1e-4, r > rc + 1e-4
+        assert got[sure].all() and not got[never].any()
