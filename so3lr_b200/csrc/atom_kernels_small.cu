@@ -120,7 +120,8 @@ template <int AT>
 __global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int n, const float* __restrict__ xa, const float* __restrict__ ev1,
                                                                  float* __restrict__ z1_out, float* __restrict__ x3_out, float* __restrict__ gate_out,
                                                                  float* __restrict__ x4_out, float* __restrict__ ev2_out,
-                                                                 const float* __restrict__ projT, float* __restrict__ qkv_next) {
+                                                                 const float* __restrict__ projT, float* __restrict__ qkv_next,
+                                                                 float* __restrict__ x4_copy, float* __restrict__ ev2_copy) {
   extern __shared__ __align__(16) float sm[];
   float* act = sm;                // [AT][128]
   float* red = sm + AT * kF;      // [4][AT][128]
@@ -166,7 +167,11 @@ __global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int
     g = fma4(inv.x, ldg4(L.ex_ig), fma4(inv.y, ldg4(L.ex_ig + 4), fma4(inv.z, ldg4(L.ex_ig + 8), fma4(inv.w, ldg4(L.ex_ig + 12), g))));
     if (own) {
       if (lane == 0) st4(gate_out + (size_t)atom * 4, g);
-      if (lane < kMTot) ev2_out[(size_t)atom * kMTot + lane] = e * (1.f + pick(g, deg));
+      if (lane < kMTot) {
+        const float ev2 = e * (1.f + pick(g, deg));
+        ev2_out[(size_t)atom * kMTot + lane] = ev2;
+        if (ev2_copy) ev2_copy[(size_t)atom * kMTot + lane] = ev2;
+      }
     }
   }
   __syncthreads();
@@ -180,7 +185,10 @@ __global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int
     float rstd;
     const float4 xh = normalise(x3, rstd);
     const float4 x4 = add4(mul4(xh, ldg4(L.ln2_s + col)), ldg4(L.ln2_b + col));
-    if (own) { st4(x3_out + ra, x3); st4(x4_out + ra, x4); }
+    if (own) {
+      st4(x3_out + ra, x3); st4(x4_out + ra, x4);
+      if (x4_copy) st4(x4_copy + ra, x4);
+    }
     st4(act + warp * kF + col, x4);
   }
   if (!projT) return;
@@ -201,7 +209,8 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
                                                                  const float* __restrict__ z1, const float* __restrict__ x3,
                                                                  const float* __restrict__ gate, const float* __restrict__ g4,
                                                                  const float* __restrict__ gev2, float* g_xa, float* __restrict__ gev1,
-                                                                 const float* __restrict__ proj, const float* __restrict__ g_qkv_up) {
+                                                                 const float* __restrict__ proj, float* g_qkv_up,
+                                                                 float* __restrict__ gev1_copy) {
   extern __shared__ __align__(16) float sm[];
   float* act = sm;                        // [AT][128]
   float* red = act + AT * kF;             // [5][AT][128]
@@ -218,7 +227,9 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
     load_w<32>(w, proj + (size_t)((tid >> 7) * 4 + ((tid >> 5) & 3)) * 1024 + lane, 32);
     for (int k = tid; k < AT * (kProj / 4); k += NTHR) {
       const int a = k / (kProj / 4);
-      st4(gq + 4 * k, row0 + a < n ? ldg4(g_qkv_up + (size_t)row0 * kProj + 4 * k) : zero4());
+      float* p = g_qkv_up + (size_t)row0 * kProj + 4 * k;
+      st4(gq + 4 * k, row0 + a < n ? ld4(p) : zero4());
+      if (row0 + a < n) st4(p, zero4());      // the next attention layer adds into zeros
     }
   } else {
     load_w128(w, L.ex_xxT);
@@ -251,7 +262,11 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
     float4 gi = make_float4(wsum(dot4(g3, ldg4(L.ex_ix + col))), wsum(dot4(g3, ldg4(L.ex_ix + kF + col))),
                             wsum(dot4(g3, ldg4(L.ex_ix + 2 * kF + col))), wsum(dot4(g3, ldg4(L.ex_ix + 3 * kF + col))));
     gi = add4(gi, make_float4(dot4(gg, ldg4(L.ex_ig)), dot4(gg, ldg4(L.ex_ig + 4)), dot4(gg, ldg4(L.ex_ig + 8)), dot4(gg, ldg4(L.ex_ig + 12))));
-    if (own && lane < kMTot) gev1[(size_t)atom * kMTot + lane] = ge2 * (1.f + gt) + pick(gi, deg) * 2.f * e * inv_weight(deg);
+    if (own && lane < kMTot) {
+      const float v = ge2 * (1.f + gt) + pick(gi, deg) * 2.f * e * inv_weight(deg);
+      gev1[(size_t)atom * kMTot + lane] = v;
+      if (gev1_copy) gev1_copy[(size_t)atom * kMTot + lane] = v;
+    }
   }
   __syncthreads();
   contract<AT>(red, w, act);
@@ -458,15 +473,15 @@ int configure_dense_small_kernels() {
   } while (0)
 
 void launch_atom_post_fwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
-                                float* x4, float* ev2, const float* projT, float* qkv_next) {
+                                float* x4, float* ev2, const float* projT, float* qkv_next, float* x4_copy, float* ev2_copy) {
   if (n <= 0) return;
-  SO3LR_SMALL_DISPATCH(n, (post_fwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_post_fwd<AT>(), s>>>(L, n, xa, ev1, z1, x3, gate, x4, ev2, projT, qkv_next)));
+  SO3LR_SMALL_DISPATCH(n, (post_fwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_post_fwd<AT>(), s>>>(L, n, xa, ev1, z1, x3, gate, x4, ev2, projT, qkv_next, x4_copy, ev2_copy)));
 }
 void launch_atom_post_bwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                                 const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const float* proj,
-                                const float* g_qkv_up) {
+                                float* g_qkv_up, float* gev1_copy) {
   if (n <= 0) return;
-  SO3LR_SMALL_DISPATCH(n, (post_bwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_post_bwd<AT>(), s>>>(L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, proj, g_qkv_up)));
+  SO3LR_SMALL_DISPATCH(n, (post_bwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_post_bwd<AT>(), s>>>(L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, proj, g_qkv_up, gev1_copy)));
 }
 void launch_heads_fwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* x, float* ze, float* zq, float* zh, float* e_nn,
                             float* q_raw, float* hv) {

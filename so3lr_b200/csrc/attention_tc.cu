@@ -31,7 +31,6 @@
 //
 // and finishes the radial derivative (sum_m dPhi[e,m] T_m'(t) dt/dr) and the spherical hidden layer per edge.
 #include <cuda_fp16.h>
-#include <cub/cub.cuh>
 #include <cstdlib>
 #include <type_traits>
 
@@ -385,45 +384,88 @@ __device__ __forceinline__ bool edge_valid(int j, int n, float dx, float dy, flo
   r2 = dx * dx + dy * dy + dz * dz;
   return j >= 0 && j < n && r2 < kRc2 && r2 > 0.f;
 }
-// One entry per undirected pair: of (i <- j) and (j <- i) the list keeps the one in the row of the smaller index, so rows [0, m)
-// hold every pair with at least one end below m exactly once.  Caller-supplied lists keep the entry that comes before its partner
+// One entry per undirected pair: of (i <- j) and (j <- i) the list keeps the one in the row of the smaller index (rows [0, n_rows) hold
+// every pair with at least one end below n_rows).  Caller-supplied lists keep the entry that comes before its partner
 // (`partner`, see match_pairs_kernel), or all of them when *asym is set.
-template <bool FILL>
-__global__ void __launch_bounds__(256) compact_rows_kernel(int n_rows, int n, const int* __restrict__ row_ptr, const int* __restrict__ nbr_j,
-                                                           const float* __restrict__ dR, const int* __restrict__ partner,
-                                                           const int* __restrict__ asym, int* __restrict__ vcount,
-                                                           const int* __restrict__ vrow_ptr, int* __restrict__ ve_i, int* __restrict__ ve_j,
-                                                           float4* __restrict__ ve_d, int2* __restrict__ ve_orig) {
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (i >= n_rows) return;
-  const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
+// One pass (kReserve): the rows of a CTA are counted, the CTA reserves its stretch of the list with one addition to *total (zero
+// beforehand), and the rows are written from a second look at them in the L1.  A row's entries stay together and so do the rows of a CTA;
+// the order of the stretches is the order in which the CTAs got there.  No result depends on it, but the gathers of neighbouring tiles
+// do once the rows exceed the L2: at 98,304 atoms the attention kernels lose 8 % / 3 % (forward / reverse).  Long lists therefore take
+// two passes (kCount, kFill) around a scan of the CTAs' counts, which keep the rows in order.
+constexpr int kCompactRows = 16;
+constexpr int kOrderedRows = 8192;      // from here on: 0.1 GB of q / k / v and cotangent rows
+enum CompactPass { kReserve, kCount, kFill };
+template <int PASS>
+__global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_rows, int n, const int* __restrict__ row_ptr,
+                                                                         const int* __restrict__ nbr_j, const float* __restrict__ dR,
+                                                                         const int* __restrict__ partner, const int* __restrict__ asym,
+                                                                         int* __restrict__ total, int* __restrict__ blocks, int* __restrict__ ve_i,
+                                                                         int* __restrict__ ve_j, float4* __restrict__ ve_d, int2* __restrict__ ve_orig) {
+  __shared__ int start[kCompactRows + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * kCompactRows + warp;
+  const int e0 = i < n_rows ? row_ptr[i] : 0, e1 = i < n_rows ? row_ptr[i + 1] : 0;
   const bool all = asym && *asym != 0;
-  int count = 0;
-  const int base = FILL ? vrow_ptr[i] : 0;
+  auto look = [&](int e, int& j, int& pe, float4& d) -> bool {
+    if (e >= e1) return false;
+    j = nbr_j[e];
+    if (!partner && j <= i) return false;
+    float r2;
+    d.x = dR[3 * (size_t)e]; d.y = dR[3 * (size_t)e + 1]; d.z = dR[3 * (size_t)e + 2];
+    if (!edge_valid(j, n, d.x, d.y, d.z, r2)) return false;
+    d.w = sqrtf(r2);
+    if (partner && !all) { pe = partner[e]; return e < pe; }
+    return true;
+  };
+  int count = 0, j = -1, pe = -1;
+  float4 d = f4_zero();
+  for (int eb = e0; eb < e1; eb += 32) count += __popc(__ballot_sync(0xffffffffu, look(eb + lane, j, pe, d)));
+  if (lane == 0) start[warp + 1] = count;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < kCompactRows; ++w) { const int c = start[w + 1]; start[w + 1] = sum; sum += c; }
+    if (PASS == kCount) blocks[blockIdx.x] = sum;
+    else start[0] = PASS == kFill ? blocks[blockIdx.x] : (sum ? atomicAdd(total, sum) : 0);
+  }
+  if (PASS == kCount) return;
+  __syncthreads();
+  int base = start[0] + start[warp + 1];
   for (int eb = e0; eb < e1; eb += 32) {
     const int e = eb + lane;
-    bool valid = false;
-    int j = -1, pe = -1;
-    float dx = 0.f, dy = 0.f, dz = 0.f, r2 = 0.f;
-    if (e < e1) {
-      j = nbr_j[e];
-      if (partner || j > i) {
-        dx = dR[3 * (size_t)e]; dy = dR[3 * (size_t)e + 1]; dz = dR[3 * (size_t)e + 2];
-        valid = edge_valid(j, n, dx, dy, dz, r2);
-      }
-      if (valid && partner && !all) { pe = partner[e]; valid = e < pe; }
-    }
+    const bool valid = look(e, j, pe, d);
     const unsigned m = __ballot_sync(0xffffffffu, valid);
-    if (FILL && valid) {
-      const int p = base + count + __popc(m & ((1u << lane) - 1u));
-      ve_i[p] = i; ve_j[p] = j;
-      ve_d[p] = make_float4(dx, dy, dz, sqrtf(r2));
-      if (ve_orig) ve_orig[p] = make_int2(e, pe);
+    if (valid) {
+      const int q = base + __popc(m & ((1u << lane) - 1u));
+      ve_i[q] = i; ve_j[q] = j;
+      ve_d[q] = d;
+      if (ve_orig) ve_orig[q] = make_int2(e, pe);
     }
-    count += __popc(m);
+    base += __popc(m);
   }
-  if (!FILL && lane == 0) vcount[i] = count;
+}
+// counts -> exclusive offsets, and their sum; one CTA (an eighth of a million atoms per 8 counts of a thread)
+__global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* __restrict__ blocks, int* __restrict__ total) {
+  __shared__ int warp_sum_[32];
+  const int tid = threadIdx.x, lane = tid & 31, per = (n + 1023) / 1024;
+  const int b0 = min(tid * per, n), b1 = min(b0 + per, n);
+  int sum = 0;
+  for (int b = b0; b < b1; ++b) sum += blocks[b];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+  if (lane == 31) warp_sum_[tid >> 5] = incl;
+  __syncthreads();
+  if (tid < 32) {
+    int v = warp_sum_[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += t; }
+    warp_sum_[lane] = v;
+  }
+  __syncthreads();
+  int at = incl - sum + (tid >= 32 ? warp_sum_[(tid >> 5) - 1] : 0);
+  for (int b = b0; b < b1; ++b) { const int c = blocks[b]; blocks[b] = at; at += c; }
+  if (tid == 1023) *total = at;
 }
 // Every entry (i <- j, d) inside the cutoff of a caller-supplied list finds its reversed entry (j <- i, -d): the k-th of several equal
 // entries of a row takes the k-th match.  *asym is set when an entry has none or the numbers of equal entries differ.  One warp per row.
@@ -466,19 +508,15 @@ __global__ void __launch_bounds__(256) check_mutual_kernel(int n_rows, const int
   }
 }
 // entries of the directed list: a pair whose ends both own a row stands for two of them
-__global__ void __launch_bounds__(256) count_directed_kernel(int n_rows, const int* __restrict__ vrow_ptr, const int* __restrict__ ve_j,
+__global__ void __launch_bounds__(256) count_directed_kernel(int n_rows, const int* __restrict__ n_listed, const int* __restrict__ ve_j,
                                                              const int* __restrict__ asym, unsigned long long* total) {
-  const int n_entries = vrow_ptr[n_rows];
+  const int n_entries = *n_listed;
   const bool both = !(asym && *asym != 0);
   unsigned long long c = 0;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += (long long)gridDim.x * blockDim.x)
     c += both && ve_j[e] < n_rows ? 2 : 1;
   if (c) atomicAdd(total, c);
 }
-__global__ void close_scan_kernel(int n_rows, const int* __restrict__ vcount, int* __restrict__ vrow_ptr) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) vrow_ptr[n_rows] = n_rows > 0 ? vrow_ptr[n_rows - 1] + vcount[n_rows - 1] : 0;
-}
-
 // Entries per warp of a tile (8 fill the 128 rows): the same number of rounds over the grid, with the entries spread evenly.  A tile's
 // time is its chain of phases plus the edge loops, which are as long as a warp's share: a short list runs one thin tile per CTA
 // instead of full tiles on a few of them, and the last round of a longer one is not half empty.
@@ -503,7 +541,7 @@ __device__ __forceinline__ void edge_loops(int share, Body&& body, int run = 8) 
 // its 8 edges in flight and 128 threads stage the next tile; (3) per filter: tensor memory -> shared tile, then the edge loop.
 __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsigned char* __restrict__ img_g, const float* __restrict__ sph1_k,
                                                                     const float* __restrict__ sph1_b, int n_recv,
-                                                                    const int* __restrict__ vrow_ptr, const int* __restrict__ ve_i,
+                                                                    const int* __restrict__ n_listed, const int* __restrict__ ve_i,
                                                                     const int* __restrict__ ve_j, const float4* __restrict__ ve_d,
                                                                     const float* __restrict__ qkv, const float* __restrict__ ev_in,
                                                                     float* __restrict__ xa, float* __restrict__ ev1, int* __restrict__ err,
@@ -518,7 +556,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   float* st_ev = reinterpret_cast<float*>(smem + kOffFwStEv);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffFwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffFwMisc + 16);
-  const long long n_edges = vrow_ptr[n_recv];
+  const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
   const long long n_tiles = (n_edges + tr - 1) / tr;
@@ -1099,7 +1137,7 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
 template <bool PER_ENTRY>
 __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsigned char* __restrict__ img_g, const float* __restrict__ sph1_k,
                                                                     const float* __restrict__ sph1_b, int n_recv,
-                                                                    const int* __restrict__ vrow_ptr, const int* __restrict__ ve_i,
+                                                                    const int* __restrict__ n_listed, const int* __restrict__ ve_i,
                                                                     const int* __restrict__ ve_j, const float4* __restrict__ ve_d,
                                                                     const float* __restrict__ qkv, const float* __restrict__ ev_in,
                                                                     const float* __restrict__ g_xa, const float* __restrict__ gev1,
@@ -1116,7 +1154,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   float* wt = reinterpret_cast<float*>(smem + kOffBwW);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffBwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 16);
-  const long long n_edges = vrow_ptr[n_recv];
+  const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
   const long long n_tiles = (n_edges + tr - 1) / tr;
@@ -1497,21 +1535,13 @@ int configure_attention_tc_kernels() {
 }
 
 int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity) {
-  if (n_rows + 1 > V->row_cap) {
-    if (V->row_ptr) dev_free(V->row_ptr);
-    if (V->count) dev_free(V->count);
-    V->row_ptr = nullptr; V->count = nullptr;
-    SO3LR_CUDA_CHECK(dev_alloc(&V->row_ptr, ((size_t)n_rows + 1)));
-    SO3LR_CUDA_CHECK(dev_alloc(&V->count, ((size_t)n_rows + 1)));
-    V->row_cap = n_rows + 1;
-    size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, V->count, V->row_ptr, n_rows);
-    if (need > V->cub_bytes) {
-      if (V->cub_tmp) dev_free(V->cub_tmp);
-      V->cub_tmp = nullptr;
-      SO3LR_CUDA_CHECK(dev_alloc_bytes(&V->cub_tmp, need));
-      V->cub_bytes = need;
-    }
+  if (!V->total) SO3LR_CUDA_CHECK(dev_alloc(&V->total, 1));
+  const int n_blocks = (n_rows + kCompactRows - 1) / kCompactRows;
+  if (n_blocks > V->block_cap) {
+    dev_free(V->blocks);
+    V->blocks = nullptr; V->block_cap = 0;
+    SO3LR_CUDA_CHECK(dev_alloc(&V->blocks, (size_t)n_blocks));
+    V->block_cap = n_blocks;
   }
   if (capacity > V->capacity) {
     if (V->i) dev_free(V->i);
@@ -1528,15 +1558,17 @@ int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity) {
 }
 
 void valid_edges_free(ValidEdges* V) {
-  dev_free(V->row_ptr); dev_free(V->count); dev_free(V->i); dev_free(V->j); dev_free(V->d); dev_free(V->orig); dev_free(V->partner); dev_free(V->cub_tmp);
+  dev_free(V->total); dev_free(V->blocks); dev_free(V->i); dev_free(V->j); dev_free(V->d); dev_free(V->orig); dev_free(V->partner);
   *V = ValidEdges{};
 }
 
 int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const int* row_ptr, const int* nbr_j, const float* dR, int* asym,
-                      long long n_source) {
+                      long long n_source, bool total_cleared) {
   V->asym = nullptr;
+  V->n_rows = n_rows;
   if (n_rows <= 0) return kOk;
-  if (n_rows + 1 > V->row_cap) return kInvalidArgument;
+  if (!V->total) return kInvalidArgument;
+  if (!total_cleared) SO3LR_CUDA_CHECK(cudaMemsetAsync(V->total, 0, sizeof(int), s));
   const int blocks = (n_rows + 7) / 8;
   if (asym) {
     if (n_source > V->capacity) return kInvalidArgument;
@@ -1552,27 +1584,30 @@ int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const in
     { check_mutual_kernel<<<sm_count() * 8, 256, 0, s>>>(n_rows, row_ptr, V->partner, asym); count_launch(); }
   }
   const int* partner = asym ? V->partner : nullptr;
-  { compact_rows_kernel<false><<<blocks, 256, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, V->count, nullptr, nullptr, nullptr, nullptr, nullptr); count_launch(); }
-  size_t tmp = V->cub_bytes;
-  cub::DeviceScan::ExclusiveSum(V->cub_tmp, tmp, V->count, V->row_ptr, n_rows, s);
-  count_launch(2);
-  { close_scan_kernel<<<1, 32, 0, s>>>(n_rows, V->count, V->row_ptr); count_launch(); }
-  { compact_rows_kernel<true><<<blocks, 256, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->row_ptr, V->i, V->j, V->d, asym ? V->orig : nullptr); count_launch(); }
+  int2* orig = asym ? V->orig : nullptr;
+  const int n_blocks = (n_rows + kCompactRows - 1) / kCompactRows, threads = 32 * kCompactRows;
+  if (n_blocks > V->block_cap) return kInvalidArgument;
+  if (n_rows < kOrderedRows) {
+    { compact_rows_kernel<kReserve><<<n_blocks, threads, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, V->total, nullptr, V->i, V->j, V->d, orig); count_launch(); }
+  } else {
+    { compact_rows_kernel<kCount><<<n_blocks, threads, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->blocks, nullptr, nullptr, nullptr, nullptr); count_launch(); }
+    { scan_blocks_kernel<<<1, 1024, 0, s>>>(n_blocks, V->blocks, V->total); count_launch(); }
+    { compact_rows_kernel<kFill><<<n_blocks, threads, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->blocks, V->i, V->j, V->d, orig); count_launch(); }
+  }
   SO3LR_CUDA_CHECK(cudaGetLastError());
-  V->n_rows = n_rows;
   return kOk;
 }
 
 int valid_edges_count_directed(const ValidEdges& V, long long* n_host) {
   *n_host = 0;
-  if (!V.row_ptr || V.n_rows <= 0) return kOk;
+  if (!V.total || V.n_rows <= 0) return kOk;
   SO3LR_CUDA_CHECK(cudaDeviceSynchronize());
   unsigned long long* t = nullptr;
   SO3LR_CUDA_CHECK(dev_alloc(&t, 1));
   unsigned long long h = 0;
   cudaError_t e = cudaMemset(t, 0, sizeof(h));
   if (e == cudaSuccess) {
-    { count_directed_kernel<<<sm_count(), 256>>>(V.n_rows, V.row_ptr, V.j, V.asym, t); count_launch(); }
+    { count_directed_kernel<<<sm_count(), 256>>>(V.n_rows, V.total, V.j, V.asym, t); count_launch(); }
     e = cudaMemcpy(&h, t, sizeof(h), cudaMemcpyDeviceToHost);
   }
   dev_free(t);
@@ -1618,24 +1653,27 @@ void tc_debug_print() {
                h[5] / (h[8] ? h[8] : 1), h[6] / (h[8] ? h[8] : 1), h[7] / (h[8] ? h[8] : 1));
 }
 int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* x_in,
-                       const float* ev_in, float* xa, float* ev1, int* err) {
+                       const float* ev_in, float* xa, float* ev1, int* err, bool preset) {
   if (n_recv <= 0) return kOk;
-  if (n_recv > V.n_rows) return kInvalidArgument;
+  if (n_recv != V.n_rows) return kInvalidArgument;
   // the kernel adds the attention sums onto the skip connection
-  SO3LR_CUDA_CHECK(cudaMemcpyAsync(xa, x_in, (size_t)n_recv * kF * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  SO3LR_CUDA_CHECK(cudaMemcpyAsync(ev1, ev_in, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  { attn_fwd_tc_kernel<<<sm_count(), kFwThreads, kSmemFwd, s>>>(L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym); count_launch(); }
+  if (!preset) {
+    SO3LR_CUDA_CHECK(cudaMemcpyAsync(xa, x_in, (size_t)n_recv * kF * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    SO3LR_CUDA_CHECK(cudaMemcpyAsync(ev1, ev_in, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
+  }
+  { attn_fwd_tc_kernel<<<sm_count(), kFwThreads, kSmemFwd, s>>>(L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym); count_launch(); }
   return kOk;
 }
 
 int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
-                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err) {
+                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err,
+                       bool gev_preset, bool gq_preset) {
   if (n_recv <= 0) return kOk;
-  if (n_recv > V.n_rows) return kInvalidArgument;
+  if (n_recv != V.n_rows) return kInvalidArgument;
   // the kernel adds into the receivers' rows: cotangents of q/k/v start at zero, that of ev at the skip term
-  SO3LR_CUDA_CHECK(cudaMemsetAsync(g_qkv, 0, (size_t)n_recv * kProj * sizeof(float), s));
-  SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, gev1, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  { attn_bwd_tc_kernel<false><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
+  if (!gq_preset) SO3LR_CUDA_CHECK(cudaMemsetAsync(g_qkv, 0, (size_t)n_recv * kProj * sizeof(float), s));
+  if (!gev_preset) SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, gev1, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
+  { attn_bwd_tc_kernel<false><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
                                                               g_qkv, gev_in, F, virial, err, tc_debug_buffer(), nullptr, nullptr, n_own); count_launch(); }
   return kOk;
 }
@@ -1643,8 +1681,8 @@ int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, i
 int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
                              const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* g_dR, int* err, const int* asym) {
   if (n_recv <= 0) return kOk;
-  if (n_recv > V.n_rows || !V.orig) return kInvalidArgument;
-  { attn_bwd_tc_kernel<true><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.row_ptr, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
+  if (n_recv != V.n_rows || !V.orig) return kInvalidArgument;
+  { attn_bwd_tc_kernel<true><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
                                                              g_qkv, gev_in, g_dR, nullptr, err, nullptr, V.orig, asym, 0); count_launch(); }
   return kOk;
 }

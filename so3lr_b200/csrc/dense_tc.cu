@@ -348,7 +348,8 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
                                                                    float* __restrict__ z1_out, float* __restrict__ x3_out,
                                                                    float* __restrict__ gate_out, float* __restrict__ x4_out,
                                                                    float* __restrict__ ev2_out, const unsigned char* __restrict__ proj_u,
-                                                                   float* __restrict__ qkv_next, int* err) {
+                                                                   float* __restrict__ qkv_next, int* err, float* __restrict__ x4_copy,
+                                                                   float* __restrict__ ev2_copy) {
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
   T.init(smem);
@@ -479,6 +480,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
           e.x *= 1.f + g[degree_of(4 * m4)]; e.y *= 1.f + g[degree_of(4 * m4 + 1)];
           e.z *= 1.f + g[degree_of(4 * m4 + 2)]; e.w *= 1.f + g[degree_of(4 * m4 + 3)];
           st4(ev2_out + (size_t)a * kMTot + 4 * m4, e);
+          if (ev2_copy) st4(ev2_copy + (size_t)a * kMTot + 4 * m4, e);
         }
       }
     }
@@ -555,6 +557,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
       }
       DN_MARK(14);
       T.flush_rows(x4_out, kF, row0, n, kF);
+      if (x4_copy) T.flush_rows(x4_copy, kF, row0, n, kF);
       DN_MARK(15);
 #pragma unroll 1
       for (int r = 0; r < 5; ++r) {
@@ -593,6 +596,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
       }
     } else {
       T.flush_rows(x4_out, kF, row0, n, kF);
+      if (x4_copy) T.flush_rows(x4_copy, kF, row0, n, kF);
     }
     __syncthreads();   // staging tile and operand buffers are free for the next tile
     DN_MARK(13);
@@ -637,7 +641,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
                                                                    const float* __restrict__ gate, const float* __restrict__ g4,
                                                                    const float* __restrict__ gev2, float* g_xa, float* __restrict__ gev1,
                                                                    const unsigned char* __restrict__ projT_u, const float* __restrict__ g_qkv_up,
-                                                                   int* err) {
+                                                                   int* err, float* __restrict__ gev1_copy) {
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
   T.init(smem);
@@ -805,7 +809,11 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
         const float gt = 1.f + gate_l, f = 2.f * ginv * inv_weight(ch);
 #pragma unroll
         for (int m = 0; m < 9; ++m)
-          if (m < nm) gev1[(size_t)aw * kMTot + m0 + m] = e2[m] * gt + f * e1[m];
+          if (m < nm) {
+            const float v = e2[m] * gt + f * e1[m];
+            gev1[(size_t)aw * kMTot + m0 + m] = v;
+            if (gev1_copy) gev1_copy[(size_t)aw * kMTot + m0 + m] = v;
+          }
       }
       if (ch == 0) T.red[wr] = make_float4(gg0, gg1, gg2, gg3);
     }
@@ -1273,19 +1281,19 @@ int configure_dense_tc_kernels() {
 }
 
 void launch_atom_post_fwd_tc(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
-                             float* x4, float* ev2, const unsigned char* proj_u, float* qkv_next, int* err) {
+                             float* x4, float* ev2, const unsigned char* proj_u, float* qkv_next, int* err, float* x4_copy, float* ev2_copy) {
   if (n <= 0) return;
   const int tiles = (n + TM - 1) / TM, grid = tiles < sm_count() ? tiles : sm_count();
-  atom_post_fwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(L, n, xa, ev1, z1, x3, gate, x4, ev2, proj_u, qkv_next, err);
+  atom_post_fwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(L, n, xa, ev1, z1, x3, gate, x4, ev2, proj_u, qkv_next, err, x4_copy, ev2_copy);
   count_launch();
 }
 
 void launch_atom_post_bwd_tc(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                              const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const unsigned char* projT_u,
-                             const float* g_qkv_up, int* err) {
+                             const float* g_qkv_up, int* err, float* gev1_copy) {
   if (n <= 0) return;
   const int tiles = (n + TM - 1) / TM, grid = tiles < sm_count() ? tiles : sm_count();
-  atom_post_bwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, projT_u, g_qkv_up, err);
+  atom_post_bwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, projT_u, g_qkv_up, err, gev1_copy);
   count_launch();
 }
 

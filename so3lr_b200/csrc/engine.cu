@@ -82,6 +82,25 @@ __global__ void fill_kernel(float* p, size_t n, float v) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
+// several arrays set to zero in one launch
+struct ClearArgs {
+  static constexpr int kMax = 10;
+  float* p[kMax];
+  long long n[kMax];
+  int count = 0;
+  void add(void* q, long long words) { if (q && words > 0) { p[count] = static_cast<float*>(q); n[count++] = words; } }
+};
+__global__ void __launch_bounds__(256) clear_kernel(ClearArgs A) {
+  for (int k = 0; k < A.count; ++k)
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < A.n[k]; i += (long long)gridDim.x * 256) A.p[k][i] = 0.f;
+}
+void launch_clear(cudaStream_t s, const ClearArgs& A) {
+  long long most = 0;
+  for (int k = 0; k < A.count; ++k) most = std::max(most, A.n[k]);
+  if (most <= 0) return;
+  const int blocks = (int)std::min<long long>(8LL * sm_count(), (most + 255) / 256);
+  { clear_kernel<<<blocks, 256, 0, s>>>(A); count_launch(); }
+}
 __global__ void combine_energy_kernel(int n, const float* e_nn, const float* e_zbl, const float* e_c, const float* e_d, float* e_atom) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) e_atom[i] = ((e_nn[i] + e_zbl[i]) + e_c[i]) + e_d[i];
@@ -486,21 +505,27 @@ bool use_small_dense(int n) {
   static const bool on = std::getenv("SO3LR_B200_DENSE") == nullptr;
   return on && dense_small_applies(n);
 }
+// dense blocks that can leave second copies of their outputs where the attention kernels add onto them
+bool dense_copies() { return use_tc_dense(); }
 // With the tensor-core dense blocks the q/k/v projections ride along: the forward block also emits the next layer's
 // q/k/v rows, the reverse block forms its input cotangent from the upper layer's g_xa and g_qkv.  `next` / `up` = that
 // neighbouring layer (nullptr: no fusion at this end of the network).
 void post_fwd_dispatch(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
-                       float* x4, float* ev2, const LayerDev* next, float* qkv_next, int* err) {
-  if (use_small_dense(n)) launch_atom_post_fwd_small(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->projT : nullptr, qkv_next);
-  else if (use_tc_dense()) launch_atom_post_fwd_tc(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->proj_u : nullptr, qkv_next, err);
+                       float* x4, float* ev2, const LayerDev* next, float* qkv_next, int* err, float* x4_copy = nullptr,
+                       float* ev2_copy = nullptr) {
+  if (use_small_dense(n))
+    launch_atom_post_fwd_small(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->projT : nullptr, qkv_next, x4_copy, ev2_copy);
+  else if (use_tc_dense())
+    launch_atom_post_fwd_tc(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->proj_u : nullptr, qkv_next, err, x4_copy, ev2_copy);
   else if (use_mma_dense()) launch_atom_post_fwd_mma(s, L, n, xa, ev1, z1, x3, gate, x4, ev2, next ? next->proj_f : nullptr, qkv_next);
   else launch_atom_post_fwd(s, L, n, xa, ev1, z1, x3, gate, x4, ev2);
 }
 void post_bwd_dispatch(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                        const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const LayerDev* up,
-                       const float* g_qkv_up, int* err) {
-  if (use_small_dense(n)) launch_atom_post_bwd_small(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->proj : nullptr, g_qkv_up);
-  else if (use_tc_dense()) launch_atom_post_bwd_tc(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->projT_u : nullptr, g_qkv_up, err);
+                       float* g_qkv_up, int* err, float* gev1_copy = nullptr) {
+  if (use_small_dense(n)) launch_atom_post_bwd_small(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->proj : nullptr, g_qkv_up, gev1_copy);
+  else if (use_tc_dense())
+    launch_atom_post_bwd_tc(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->projT_u : nullptr, g_qkv_up, err, gev1_copy);
   else if (use_mma_dense()) launch_atom_post_bwd_mma(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, up ? up->projT_f : nullptr, g_qkv_up);
   else launch_atom_post_bwd(s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1);
 }
@@ -519,16 +544,17 @@ void heads_bwd_dispatch(cudaStream_t s, const ModelDev& M, int n, const int* Z, 
   else launch_heads_bwd(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx);
 }
 void attn_fwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
-                       const float* qkv, const float* x_in, const float* ev_in, float* xa, float* ev1) {
-  if (L.has_spherical && attention_mode() >= kAttnTcFwd) launch_attn_fwd_tc(st, L, S->ve, n_recv, qkv, x_in, ev_in, xa, ev1, S->d_flag + 1);
+                       const float* qkv, const float* x_in, const float* ev_in, float* xa, float* ev1, bool preset = false) {
+  if (L.has_spherical && attention_mode() >= kAttnTcFwd) launch_attn_fwd_tc(st, L, S->ve, n_recv, qkv, x_in, ev_in, xa, ev1, S->d_flag + 1, preset);
   else if (L.has_spherical && use_mma_attention()) launch_attn_fwd_mma(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, x_in, ev_in, xa, ev1);
   else launch_attn_fwd_sym(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, x_in, ev_in, xa, ev1);
 }
 void attn_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
                        const float* qkv, const float* ev_in, const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F,
-                       int first_layer, float* virial, int n_own) {
+                       int first_layer, float* virial, int n_own, bool gev_preset = false, bool gq_preset = false) {
   if (!first_layer && L.has_spherical && attention_mode() == kAttnTc)
-    launch_attn_bwd_tc(st, L, S->ve, n_recv, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial, n_own, S->d_flag + 1);
+    launch_attn_bwd_tc(st, L, S->ve, n_recv, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial, n_own, S->d_flag + 1, gev_preset,
+                       gq_preset);
   else if (!first_layer && L.has_spherical && use_mma_attention())
     launch_attn_bwd_mma(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial);
   else launch_attn_bwd_sym(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, first_layer, virial);
@@ -540,6 +566,9 @@ void layer0_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, int n_recv, int 
   else
     launch_layer0_bwd_tab(st, S->sp, n_recv, n_gv, n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->d_Z, S->g_xa, S->gev1, S->GV, F, S->vir());
 }
+
+// the reverse blocks of short lists leave zeros in the q/k/v cotangents they have read: one clearing at the start serves both layers
+bool small_presets(int n) { return use_small_dense(n) && attention_mode() == kAttnTc; }
 
 // SO3LR_B200_GRAPH=scatter keeps the graph-level call on the first-generation scatter kernels throughout (exact per-entry
 // gradients also for lists that are symmetric)
@@ -572,14 +601,20 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
   if (tiled) {
     int rcv = valid_edges_reserve(&S->ve, S->n_cap, n_edges);
     if (rcv) return rcv;
-    SO3LR_CUDA_CHECK(cudaMemsetAsync(asym, 0, sizeof(int), st));
-    rcv = valid_edges_build(&S->ve, st, n, n, row_ptr, nbr_j, dR, asym, n_edges);
+  }
+  const bool gq_preset = tiled && small_presets(n);
+  ClearArgs A;
+  A.add(S->e_zbl, n); A.add(S->e_coul, n); A.add(S->e_disp, n); A.add(S->gq, n); A.add(S->gh, n); A.add(S->gev_a, (long long)n * kMTot);
+  if (tiled) { A.add(asym, 1); A.add(S->ve.total, 1); }
+  if (gq_preset) A.add(S->g_qkv, (long long)n * kProj);
+  launch_clear(st, A);
+  if (tiled) {
+    int rcv = valid_edges_build(&S->ve, st, n, n, row_ptr, nbr_j, dR, asym, n_edges, true);
     if (rcv) return rcv;
   }
-  fill(st, S->e_zbl, n, 0.f); fill(st, S->e_coul, n, 0.f); fill(st, S->e_disp, n, 0.f);
-  fill(st, S->gq, n, 0.f); fill(st, S->gh, n, 0.f);
   S->prof.begin(kPGeom, st); launch_sr_geometry_zbl(st, M, S->cell, n, n_edges, edge_i, nbr_j, S->d_Z, nullptr, 1, dR, S->e_zbl, g_dR, ge, nullptr); S->prof.end(st);
   const bool tab0 = tiled && S->sp.n_species > 0 && use_layer0_tables();
+  const bool copies = tiled && dense_copies();
   const bool fuse = use_mma_dense();   // q/k/v rows of layer l + 1 come out of layer l's dense block, their transpose goes into it
   if (!tab0) { int rce = embed_atoms(S, st, n, S->x[0]); if (rce) return rce; }
   for (int l = 0; l < kNumLayers; ++l) {
@@ -587,13 +622,14 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
     if (!(l == 0 ? tab0 : fuse)) { S->prof.begin(kPProj, st); launch_proj_fwd(st, L, S->x[l], n, S->qkv[l]); S->prof.end(st); }
     S->prof.begin(kPAttnFwd, st);
     if (l == 0 && tab0) launch_layer0_fwd_tab(st, S->sp, M, n, n, row_ptr, nbr_j, dR, S->d_Z, S->xa[0], S->ev1[0]);
-    else if (tiled && L.has_spherical) launch_attn_fwd_tc(st, L, S->ve, n, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], S->d_flag + 1);
+    else if (tiled && L.has_spherical) launch_attn_fwd_tc(st, L, S->ve, n, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], S->d_flag + 1, l > 0 && copies);
     else launch_attn_fwd(st, L, n, row_ptr, nbr_j, dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l]);
     S->prof.end(st);
     S->prof.begin(kPPostFwd, st);
     const bool emit = fuse && l + 1 < kNumLayers;
     post_fwd_dispatch(st, L, n, S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->x[l + 1], S->ev[l + 1],
-                      emit ? &M.layer[l + 1] : nullptr, emit ? S->qkv[l + 1] : nullptr, S->d_flag + 1);
+                      emit ? &M.layer[l + 1] : nullptr, emit ? S->qkv[l + 1] : nullptr, S->d_flag + 1,
+                      copies && l + 1 < kNumLayers ? S->xa[l + 1] : nullptr, copies && l + 1 < kNumLayers ? S->ev1[l + 1] : nullptr);
     S->prof.end(st);
   }
   S->prof.begin(kPHeads, st);
@@ -615,18 +651,17 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
   S->prof.begin(kPHeads, st);
   heads_bwd_dispatch(st, M, n, S->d_Z, S->ze, S->zq, S->zh, S->hv, ge ? ge : S->ones, S->gq_raw, S->gh, S->g4, S->d_flag + 1);
   S->prof.end(st);
-  float* gev2 = S->gev_a;
+  float* gev2 = S->gev_a;      // zeros since the start
   float* gev_in = S->gev_b;
-  fill(st, gev2, (size_t)n * kMTot, 0.f);
   for (int l = kNumLayers - 1; l >= 0; --l) {
     const LayerDev& L = M.layer[l];
     S->prof.begin(kPPostBwd, st);
     post_bwd_dispatch(st, L, n, S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->g4, gev2, S->g_xa, S->gev1,
-                      fuse && l + 1 < kNumLayers ? &M.layer[l + 1] : nullptr, S->g_qkv, S->d_flag + 1);
+                      fuse && l + 1 < kNumLayers ? &M.layer[l + 1] : nullptr, S->g_qkv, S->d_flag + 1, copies && l > 0 ? gev_in : nullptr);
     S->prof.end(st);
     if (l > 0) {
-      SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, S->gev1, (size_t)n * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, st));
-      fill(st, S->g_qkv, (size_t)n * kProj, 0.f);
+      if (!copies) SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, S->gev1, (size_t)n * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, st));
+      if (!gq_preset) fill(st, S->g_qkv, (size_t)n * kProj, 0.f);
       S->prof.begin(kPAttnBwd, st);
       if (tiled && L.has_spherical) {
         int rcb = launch_attn_bwd_tc_graph(st, L, S->ve, n, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, g_dR, S->d_flag + 1, asym);
@@ -694,6 +729,7 @@ void drop_step_graph(so3lr_b200_system* S) {
 
 struct Shells { int n0, n1, n2, n3; };
 
+
 constexpr int kVirialBlocks = 1024;   // capacity of the block-partials buffer of the virial reduction
 // sum of the per-atom virial rows of the atoms whose energy is evaluated here
 void reduce_virial(so3lr_b200_system* S, cudaStream_t st, int n0) {
@@ -711,19 +747,28 @@ int fused_forward(so3lr_b200_system* S, cudaStream_t st, const float* R, const S
   const int* row_ptr = S->sr.row_ptr; const int* nbr_j = S->sr.nbr_j; const int* edge_i = S->sr.edge_i;
   const int nrecv[kNumLayers] = {c.n2, c.n1, c.n0};   // receivers of layer l
   const int nsend[kNumLayers] = {c.n3, c.n2, c.n1};   // atoms whose q/k/v rows layer l reads
-  fill(st, S->e_zbl, c.n0, 0.f);
-  fill(st, F, (size_t)c.n3 * 3, 0.f);
-  if (S->vir()) fill(st, S->virial, (size_t)c.n3 * 6, 0.f);
+  {
+    // everything the evaluation adds into, in one launch (small arrays: as many fills are as many gaps between launches)
+    ClearArgs A;
+    A.add(S->e_zbl, c.n0); A.add(F, (long long)c.n3 * 3);
+    if (S->vir()) A.add(S->virial, (long long)c.n3 * 6);
+    A.add(S->e_coul, c.n0); A.add(S->e_disp, c.n0); A.add(S->gq, c.n0); A.add(S->gh, c.n0);
+    A.add(S->gev_a, (long long)c.n0 * kMTot);
+    A.add(S->ve.total, 1);
+    if (small_presets(c.n0)) A.add(S->g_qkv, (long long)c.n3 * kProj);
+    launch_clear(st, A);
+  }
   S->prof.begin(kPGeom, st);
   launch_sr_geometry_zbl(st, M, S->cell, c.n3, S->sr.count, edge_i, nbr_j, S->d_Z, R, 0, S->dR, S->e_zbl, nullptr, nullptr, F,
                          owned_side_only ? c.n0 : -1, S->vir());
   if (attention_mode() >= kAttnTcFwd) {
-    int rcv = valid_edges_build(&S->ve, st, S->sr_rows, c.n3, row_ptr, nbr_j, S->dR);
+    int rcv = valid_edges_build(&S->ve, st, S->sr_rows, c.n3, row_ptr, nbr_j, S->dR, nullptr, 0, true);
     if (rcv) return rcv;
   }
   S->prof.end(st);
   const bool tab0 = S->sp.n_species > 0 && use_layer0_tables();
   const bool fuse = use_mma_dense();   // q/k/v rows of layer l+1 come out of layer l's dense block
+  const bool copies = dense_copies() && attention_mode() >= kAttnTcFwd;   // and so do the rows its attention adds onto
   if (!tab0) { int rce = embed_atoms(S, st, c.n3, S->x[0]); if (rce) return rce; }
   for (int l = 0; l < kNumLayers; ++l) {
     const LayerDev& L = M.layer[l];
@@ -734,13 +779,14 @@ int fused_forward(so3lr_b200_system* S, cudaStream_t st, const float* R, const S
     } else {
       if (!(fuse && l > 0)) { S->prof.begin(kPProj, st); launch_proj_fwd(st, L, S->x[l], nsend[l], S->qkv[l]); S->prof.end(st); }
       S->prof.begin(kPAttnFwd, st);
-      attn_fwd_dispatch(S, st, L, nrecv[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l]);
+      attn_fwd_dispatch(S, st, L, nrecv[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], l > 0 && copies);
       S->prof.end(st);
     }
     S->prof.begin(kPPostFwd, st);
     const bool emit = fuse && l + 1 < kNumLayers;
     post_fwd_dispatch(st, L, nrecv[l], S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->x[l + 1], S->ev[l + 1],
-                      emit ? &M.layer[l + 1] : nullptr, emit ? S->qkv[l + 1] : nullptr, S->d_flag + 1);
+                      emit ? &M.layer[l + 1] : nullptr, emit ? S->qkv[l + 1] : nullptr, S->d_flag + 1,
+                      copies && l + 1 < kNumLayers ? S->xa[l + 1] : nullptr, copies && l + 1 < kNumLayers ? S->ev1[l + 1] : nullptr);
     S->prof.end(st);
   }
   S->prof.begin(kPHeads, st);
@@ -759,15 +805,15 @@ int fused_backward(so3lr_b200_system* S, cudaStream_t st, const Shells& c, float
   S->prof.begin(kPHeads, st);
   heads_bwd_dispatch(st, M, c.n0, S->d_Z, S->ze, S->zq, S->zh, S->hv, S->ones, S->gq_raw, S->gh, S->g4, S->d_flag + 1);
   S->prof.end(st);
-  float* gev2 = S->gev_a;
+  float* gev2 = S->gev_a;      // zeros since the start of the evaluation
   float* gev_in = S->gev_b;
-  fill(st, gev2, (size_t)c.n0 * kMTot, 0.f);
+  const bool copies = dense_copies() && attention_mode() == kAttnTc;
   for (int l = kNumLayers - 1; l >= 0; --l) {
     const LayerDev& L = M.layer[l];
     const bool fused_in = use_mma_dense() && l + 1 < kNumLayers;   // cotangent formed from the layer above inside the block
     S->prof.begin(kPPostBwd, st);
     post_bwd_dispatch(st, L, npost[l], S->xa[l], S->ev1[l], S->z1[l], S->x3[l], S->gate[l], S->g4, gev2, S->g_xa, S->gev1,
-                      fused_in ? &M.layer[l + 1] : nullptr, S->g_qkv, S->d_flag + 1);
+                      fused_in ? &M.layer[l + 1] : nullptr, S->g_qkv, S->d_flag + 1, copies && l > 0 ? gev_in : nullptr);
     S->prof.end(st);
     if (c.n3 > npost[l]) {   // atoms beyond the layer's receivers have no cotangent of their own (any of them can be a neighbour)
       fill(st, S->g_xa + (size_t)npost[l] * kF, (size_t)(c.n3 - npost[l]) * kF, 0.f);
@@ -778,7 +824,7 @@ int fused_backward(so3lr_b200_system* S, cudaStream_t st, const Shells& c, float
       layer0_bwd_dispatch(S, st, nattn[0], c.n3, c.n3, F, c.n0);
     else
       attn_bwd_dispatch(S, st, L, nattn[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, F, l == 0 ? 1 : 0,
-                        S->vir(), c.n0);
+                        S->vir(), c.n0, copies, small_presets(c.n0));
     S->prof.end(st);
     if (l > 0) {
       if (!use_mma_dense()) {
@@ -800,19 +846,18 @@ int evaluate_fused(so3lr_b200_system* S, cudaStream_t st, const float* R, float*
   const Shells c{n, n, n, n};
   int rc = fused_forward(S, st, R, c, false, F);
   if (rc) return rc;
-  fill(st, S->e_coul, n, 0.f); fill(st, S->e_disp, n, 0.f); fill(st, S->gq, n, 0.f); fill(st, S->gh, n, 0.f);
   launch_charge_conserve(st, S->n_graphs, S->d_graph_start, S->q_raw, S->d_total_charge, S->hv, S->q, S->h, S->n, S->red_scratch);
   S->prof.begin(kPPairLr, st);
   launch_pair_lr_packed(st, S->lr, S->cell, n, S->lrl.row_ptr, S->lrl.nbr_j, S->d_Z, R, S->q, S->h, S->pair_pack, F, S->gq, S->gh, S->e_coul,
-                        S->e_disp, S->vir());
+                        S->e_disp, S->vir(), S->e_nn, S->e_zbl, S->ks.mode ? nullptr : S->e_atom);
   S->prof.end(st);
   if (S->ks.mode) {
     S->prof.begin(kPKspace, st);
     rc = launch_ewald(st, S->ks, S->cell, n, R, S->q, S->d_total_charge, S->e_coul, S->gq, F, S->vir(), 1.f);
     S->prof.end(st);
     if (rc) return rc;
+    { combine_energy_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, S->e_nn, S->e_zbl, S->e_coul, S->e_disp, S->e_atom); count_launch(); }
   }
-  { combine_energy_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, S->e_nn, S->e_zbl, S->e_coul, S->e_disp, S->e_atom); count_launch(); }
   launch_charge_conserve_bwd(st, S->n_graphs, S->d_graph_start, S->gq, S->gq_raw, S->n, S->red_scratch);
   return fused_backward(S, st, c, F);
 }

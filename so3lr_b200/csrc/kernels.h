@@ -53,10 +53,10 @@ void launch_heads_bwd_mma(cudaStream_t s, const ModelDev& M, int n, const int* Z
 int configure_dense_tc_kernels();
 void dense_debug_print();   // development aid of timing builds; prints nothing otherwise
 void launch_atom_post_fwd_tc(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
-                             float* x4, float* ev2, const unsigned char* proj_u, float* qkv_next, int* err);
+                             float* x4, float* ev2, const unsigned char* proj_u, float* qkv_next, int* err, float* x4_copy, float* ev2_copy);
 void launch_atom_post_bwd_tc(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                              const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const unsigned char* projT_u,
-                             const float* g_qkv_up, int* err);
+                             const float* g_qkv_up, int* err, float* gev1_copy);
 
 void launch_heads_fwd_tc(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* x, float* ze, float* zq, float* zh, float* e_nn,
                          float* q_raw, float* hv, int* err);
@@ -64,13 +64,14 @@ void launch_heads_bwd_tc(cudaStream_t s, const ModelDev& M, int n, const int* Z,
                          const float* hv, const float* ge, const float* gq, const float* gh, float* gx, int* err);
 
 // ---- atom_kernels_small.cu: the same blocks and heads (FP32 throughout) for lists of at most 16 atoms per SM ----
+// x4_copy / ev2_copy / gev1_copy (may be nullptr): second places for x4, ev2, gev1.  With `proj` the reverse block leaves zeros in g_qkv_up.
 bool dense_small_applies(int n);
 int configure_dense_small_kernels();
 void launch_atom_post_fwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
-                                float* x4, float* ev2, const float* projT, float* qkv_next);
+                                float* x4, float* ev2, const float* projT, float* qkv_next, float* x4_copy, float* ev2_copy);
 void launch_atom_post_bwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                                 const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const float* proj,
-                                const float* g_qkv_up);
+                                float* g_qkv_up, float* gev1_copy);
 void launch_heads_fwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* x, float* ze, float* zq, float* zh, float* e_nn,
                             float* q_raw, float* hv);
 void launch_heads_bwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* ze, const float* zq, const float* zh,
@@ -157,12 +158,12 @@ void launch_attn_bwd_mma(cudaStream_t s, const LayerDev& L, int n_recv, int n, c
                          float* F, float* virial = nullptr);
 
 // ---- attention_tc.cu: layers with a spherical filter as CTA-tiled tcgen05 kernels ----
-// Short-range pairs inside the cutoff, compacted once per evaluation, one entry per undirected pair, grouped by its end with the
-// smaller index: entry p of row i (row_ptr[i] <= p < row_ptr[i + 1]) holds i[p], the partner j[p] and d[p] = (dx, dy, dz, |dR|) from i
-// to j.  Caller-supplied lists whose entries do not come in reversed pairs (*asym != 0) keep every entry i <- j.
+// Short-range pairs inside the cutoff, compacted once per evaluation, one entry per undirected pair: i[p] is its end with the smaller
+// index (the entries of one i are consecutive), j[p] the partner and d[p] = (dx, dy, dz, |dR|) from i to j, p < *total.  Caller-supplied lists whose entries do not come in reversed pairs (*asym != 0) keep every entry i <- j.
 struct ValidEdges {
-  int* row_ptr = nullptr;   // n_rows + 1
-  int* count = nullptr;     // per-row counts (scratch of the build)
+  int* total = nullptr;     // number of entries (on the device)
+  int* blocks = nullptr;    // scratch of the build
+  int block_cap = 0;
   int* i = nullptr;
   int* j = nullptr;
   float4* d = nullptr;
@@ -170,22 +171,19 @@ struct ValidEdges {
   int* partner = nullptr;   // caller-supplied lists: position of each source entry's reversed entry
   const int* asym = nullptr;
   long long orig_cap = 0;
-  void* cub_tmp = nullptr;
-  size_t cub_bytes = 0;
-  int row_cap = 0;
   long long capacity = 0;
   int n_rows = 0;           // rows of the latest build
 };
 int configure_attention_tc_kernels();
 void tc_debug_print();
-// (re)allocates for n_rows receivers and `capacity` entries (the capacity of the list they are compacted from)
+// (re)allocates for n_rows rows and `capacity` entries (the capacity of the list they are compacted from)
 int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity);
 void valid_edges_free(ValidEdges* V);
 // no host synchronisation: counts stay on the device
 // `asym` (caller-supplied lists of n_source entries; zeroed by the caller): set to 1 when the entries inside the cutoff do not pair up
 // as (i <- j, d), (j <- i, -d); without it the list has to be symmetric with one entry per pair and direction
 int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const int* row_ptr, const int* nbr_j, const float* dR,
-                      int* asym = nullptr, long long n_source = 0);
+                      int* asym = nullptr, long long n_source = 0, bool total_cleared = false);
 // entries i <- j of the latest build counted per direction (synchronises)
 int valid_edges_count_directed(const ValidEdges& V, long long* n_host);
 // The reverse kernel for caller-supplied lists: runs only while *asym == 0 and, instead of summing forces, adds to every source
@@ -194,14 +192,15 @@ int valid_edges_count_directed(const ValidEdges& V, long long* n_host);
 // zeroes g_qkv and presets gev_in.
 int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
                              const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* g_dR, int* err, const int* asym);
-// Same results as launch_attn_fwd_sym for rows [0, n_recv).  `err` (device int) is set to 1 when a bounded wait on the
+// Same results as launch_attn_fwd_sym for rows [0, n_recv), all rows of the list.  `preset`: xa and ev1 hold x_in and ev_in already.  `err` (device int) is set to 1 when a bounded wait on the
 // tensor-core pipeline ran out; the outputs are then incomplete.
 int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* x_in,
-                       const float* ev_in, float* xa, float* ev1, int* err);
+                       const float* ev_in, float* xa, float* ev1, int* err, bool preset = false);
 // Same results as launch_attn_bwd_sym (first_layer = 0) for rows [0, n_recv): writes g_qkv and gev_in rows, adds to F (and to virial
-// rows, of which those below n_own add up to the total).
+// rows, of which those below n_own add up to the total).  Presets: gev_in holds gev1, g_qkv zeros already.
 int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
-                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err);
+                       const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err,
+                       bool gev_preset = false, bool gq_preset = false);
 
 // ---- layer0_tab.cu: first layer through per-element-pair tables (its inputs depend on the elements only) ----
 constexpr int kMaxTabSpecies = 8;
@@ -251,7 +250,8 @@ void launch_pair_lr(cudaStream_t s, const LrParams& P, const Cell& cell, int n, 
 // F, gq, gh, e_coul, e_disp like launch_pair_lr in mode 0
 void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, int n, const int* row_ptr, const int* nbr_j, const int* Z,
                            const float* R, const float* q, const float* h, float* pack, float* F, float* gq, float* gh, float* e_coul,
-                           float* e_disp, float* virial);
+                           float* e_disp, float* virial,
+                           const float* e_nn = nullptr, const float* e_zbl = nullptr, float* e_atom = nullptr);
 // Domain-decomposed variant: rows 0 .. n_owned-1 of an ordered list (j > i) over owned atoms and ghosts, ghosts carrying
 // the larger indices.  Pairs of two owned atoms are evaluated once and scatter the partner's derivatives (atomics); pairs
 // with a ghost end book half of the energy and the row atom's derivatives.  gq, gh are zeroed here and accumulated, F_add is

@@ -275,13 +275,13 @@ __global__ void __launch_bounds__(256) layer0_bwd_tab_kernel(SpeciesTables T, in
 // has one (the full list's rows hold the skin too and leave 45 % of the lanes without work, and every pair was evaluated at both ends).
 // Equal receivers inside a warp are summed before they go out; the partner gets its share if it owns a row.  Rows of `virial` below
 // n_own add up to the total, in any distribution: every warp adds its sum to one of them.
-__global__ void __launch_bounds__(128) layer0_bwd_pairs_kernel(SpeciesTables T, int n_recv, const int* __restrict__ vrow_ptr,
+__global__ void __launch_bounds__(128) layer0_bwd_pairs_kernel(SpeciesTables T, int n_recv, const int* __restrict__ n_listed,
                                                                const int* __restrict__ ve_i, const int* __restrict__ ve_j,
                                                                const float4* __restrict__ ve_d, const int* __restrict__ Z,
                                                                const float* __restrict__ GV, const float* __restrict__ gev1,
                                                                float* __restrict__ F, float* __restrict__ virial, int n_own) {
   const int lane = threadIdx.x & 31;
-  const long long n_pairs = vrow_ptr[n_recv];
+  const long long n_pairs = *n_listed;
   const long long warp0 = (long long)blockIdx.x * 4 + (threadIdx.x >> 5), step = (long long)gridDim.x * 128;
   VirialAcc va;
   for (long long e0 = 32 * warp0; e0 < n_pairs; e0 += step) {
@@ -397,7 +397,7 @@ void launch_layer0_bwd_pairs(cudaStream_t s, const SpeciesTables& T, int n_recv,
   // the number of pairs stays on the device: four CTAs per SM walk over the list, fewer where the rows cannot fill them
   int blocks = (int)(((long long)n_recv * 24 + 127) / 128);
   if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-  { layer0_bwd_pairs_kernel<<<blocks, 128, 0, s>>>(T, n_recv, V.row_ptr, V.i, V.j, V.d, Z, GV, gev1, F, virial, n_own); count_launch(); }
+  { layer0_bwd_pairs_kernel<<<blocks, 128, 0, s>>>(T, n_recv, V.total, V.i, V.j, V.d, Z, GV, gev1, F, virial, n_own); count_launch(); }
 }
 
 void launch_layer0_bwd_entries(cudaStream_t s, const SpeciesTables& T, int n, long long n_entries, const int* idx_i, const int* idx_j,

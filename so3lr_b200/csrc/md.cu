@@ -98,33 +98,34 @@ __global__ void nhc_init_kernel(double* chain) {
   if (t < kNhcStateDoubles) chain[t] = t == 1 ? 1.0 : 0.0;
 }
 
-// One factor of the chain propagator over `delta`; returns the momentum scale.  xi, p: chain positions and momenta.
-__device__ double nhc_substep(int L, double* xi, double* p, const double* Q, double& ke, double delta, double kT, double dof) {
+// One factor of the chain propagator over `delta`; returns the momentum scale.  xi, p: chain positions and momenta, iQ: reciprocal
+// masses (one thread walks a chain of dependent operations: a division costs it as much as an exponential).
+__device__ double nhc_substep(int L, double* xi, double* p, const double* iQ, double& ke, double delta, double kT, double dof) {
   const int M = L - 1;
   const double d2 = 0.5 * delta, d4 = 0.25 * delta, d8 = 0.125 * delta;
   if (L == 1) {
     p[0] += d4 * (2.0 * ke - dof * kT);
   } else {
-    p[M] += d4 * (p[M - 1] * p[M - 1] / Q[M - 1] - kT);
+    p[M] += d4 * (p[M - 1] * p[M - 1] * iQ[M - 1] - kT);
     for (int m = M - 1; m > 0; --m) {
-      double G = p[m - 1] * p[m - 1] / Q[m - 1] - kT;
-      double s = exp(-d8 * p[m + 1] / Q[m + 1]);
+      double G = p[m - 1] * p[m - 1] * iQ[m - 1] - kT;
+      double s = exp(-d8 * p[m + 1] * iQ[m + 1]);
       p[m] = s * (s * p[m] + d4 * G);
     }
-    double s = exp(-d8 * p[1] / Q[1]);
+    double s = exp(-d8 * p[1] * iQ[1]);
     p[0] = s * (s * p[0] + d4 * (2.0 * ke - dof * kT));
   }
-  const double scale = exp(-d2 * p[0] / Q[0]);
+  const double scale = exp(-d2 * p[0] * iQ[0]);
   ke *= scale * scale;
-  for (int m = 0; m < L; ++m) xi[m] += d2 * p[m] / Q[m];
+  for (int m = 0; m < L; ++m) xi[m] += d2 * p[m] * iQ[m];
   double G = 2.0 * ke - dof * kT;
   if (L == 1) {
     p[0] += d4 * G;
   } else {
     for (int m = 0; m < M; ++m) {
-      double s = exp(-d8 * p[m + 1] / Q[m + 1]);
+      double s = exp(-d8 * p[m + 1] * iQ[m + 1]);
       p[m] = s * (s * p[m] + d4 * G);
-      G = p[m] * p[m] / Q[m] - kT;
+      G = p[m] * p[m] * iQ[m] - kT;
     }
     p[M] += d4 * G;
   }
@@ -135,17 +136,17 @@ __device__ double nhc_substep(int L, double* xi, double* p, const double* Q, dou
 // chain[0] (kinetic energy) follows the scaling; chain[1] is left to the caller.
 __device__ double nhc_advance(double* chain, int L, int chain_steps, int sy_steps, double dt, double tau, double kT, double dof,
                               int n_half) {
-  double xi[kNhcMaxChain], p[kNhcMaxChain], Q[kNhcMaxChain];
+  double xi[kNhcMaxChain], p[kNhcMaxChain], iQ[kNhcMaxChain];
   for (int m = 0; m < L; ++m) {
     xi[m] = chain[2 + m];
     p[m] = chain[2 + kNhcMaxChain + m];
-    Q[m] = kT * tau * tau * (m == 0 ? dof : 1.0);
+    iQ[m] = 1.0 / (kT * tau * tau * (m == 0 ? dof : 1.0));
   }
   double ke = chain[0], total = 1.0;
   const double* w = kSyWeights[sy_steps / 2];
   const double delta = dt / chain_steps;
   for (int h = 0; h < n_half; ++h)
-    for (int i = 0; i < chain_steps * sy_steps; ++i) total *= nhc_substep(L, xi, p, Q, ke, delta * w[i % sy_steps], kT, dof);
+    for (int i = 0; i < chain_steps * sy_steps; ++i) total *= nhc_substep(L, xi, p, iQ, ke, delta * w[i % sy_steps], kT, dof);
   for (int m = 0; m < L; ++m) {
     chain[2 + m] = xi[m];
     chain[2 + kNhcMaxChain + m] = p[m];

@@ -231,12 +231,16 @@ __global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* __re
   hz[i] = make_float4(h[i], alpha_free(Z[i]), c6_free(Z[i]), 0.f);
   acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
-__global__ void __launch_bounds__(256) pair_unpack_kernel(int n, const float4* __restrict__ acc, float* __restrict__ F, float* __restrict__ gq) {
+// with e_atom also the per-atom energies: the sum of the network's, the repulsion's and the two pair terms' shares
+__global__ void __launch_bounds__(256) pair_unpack_kernel(int n, const float4* __restrict__ acc, float* __restrict__ F, float* __restrict__ gq,
+                                                          const float* __restrict__ e_nn, const float* __restrict__ e_zbl,
+                                                          const float* __restrict__ e_coul, const float* __restrict__ e_disp, float* __restrict__ e_atom) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 a = acc[i];
   F[3 * (size_t)i] += a.x; F[3 * (size_t)i + 1] += a.y; F[3 * (size_t)i + 2] += a.z;
   gq[i] += a.w;
+  if (e_atom) e_atom[i] = ((e_nn[i] + e_zbl[i]) + e_coul[i]) + e_disp[i];
 }
 __device__ __forceinline__ void red_add_f4(float4* p, float x, float y, float z, float w) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
@@ -538,14 +542,14 @@ void launch_pair_lr(cudaStream_t s, const LrParams& P, const Cell& cell, int n, 
 
 void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, int n, const int* row_ptr, const int* nbr_j, const int* Z,
                            const float* R, const float* q, const float* h, float* pack /* 12 n floats */, float* F, float* gq, float* gh,
-                           float* e_coul, float* e_disp, float* virial) {
+                           float* e_coul, float* e_disp, float* virial, const float* e_nn, const float* e_zbl, float* e_atom) {
   if (n <= 0) return;
   float4* pq = reinterpret_cast<float4*>(pack);
   float4* acc = pq + n;
   float4* hz = acc + n;
   pair_pack_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, R, q, h, Z, pq, hz, acc);
   pair_lr_packed_kernel<<<(n + 7) / 8, 256, 0, s>>>(P, cell, n, row_ptr, nbr_j, pq, hz, acc, gh, e_coul, e_disp, virial);
-  pair_unpack_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, acc, F, gq);
+  pair_unpack_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, acc, F, gq, e_nn, e_zbl, e_coul, e_disp, e_atom);
   count_launch(3);
 }
 
