@@ -73,7 +73,9 @@ constexpr int kOffBwW = kOffA + kARegion;
 constexpr int kOffBwRec = kOffBwW + 64 * kWStride * 4;
 constexpr int kOffBwSph = kOffBwRec + TE * kBwRec * 4;
 constexpr int kOffBwMisc = kOffBwSph + 512 * 4;
-constexpr int kSmemBwd = kOffBwMisc + 64;
+constexpr int kOffBwStIJ = kOffBwMisc + 64;                  // staged inputs of the next tile: (i, j) | displacement
+constexpr int kOffBwStD = kOffBwStIJ + TE * 8;
+constexpr int kSmemBwd = kOffBwStD + TE * 16;
 static_assert(kSmemFwd <= 232448 && kSmemBwd <= 232448, "shared memory budget of one CTA per SM");
 
 __device__ __forceinline__ float invw(int l) {
@@ -172,6 +174,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
 }
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // fire-and-forget vector add in global memory (no value comes back to the warp)
@@ -950,6 +955,29 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
     }
   }
 }
+constexpr int kAngOff = 4 * 4 * TE + 4 * TE;      // floats: behind the invariants' and radial shares of the last phase
+static_assert((kAngOff + 4 * 4 * TE) <= 64 * kWStride, "shares of the last phase fit the filter tile");
+// share of degree L in the angular part of the force on the receiver: logits x cutoff of both directions (record fields 20.. and 24..)
+// times the cotangents of both atoms' ev, through the transpose of the harmonics
+template <int L>
+__device__ __forceinline__ float4 angular_share(const float* rp, const float* __restrict__ gev1) {
+  if (rp[34] == 0.f) return f4_zero();
+  constexpr int m0 = L * L - 1;      // first component of the degree: 0, 3, 8, 15
+  const float* gi = gev1 + (size_t)__float_as_int(rp[1]) * kMTot + m0;
+  const float* gj = gev1 + (size_t)__float_as_int(rp[0]) * kMTot + m0;
+  float a[2 * L + 1], b[2 * L + 1];
+#pragma unroll
+  for (int m = 0; m < 2 * L + 1; ++m) { a[m] = gi[m]; b[m] = gj[m]; }
+  const float aA = rp[19 + L], aB = (L & 1) ? -rp[23 + L] : rp[23 + L];      // Y_lm(-u) = (-1)^l Y_lm(u)
+  const float4 uu = ld4(rp + 28);
+#pragma unroll
+  for (int m = 0; m < 2 * L + 1; ++m) a[m] = aA * a[m] + aB * b[m];
+  float gx = 0.f, gy = 0.f, gz = 0.f;
+  sph_harm_vjp_degree<L>(uu.x, uu.y, uu.z, a, gx, gy, gz);
+  const float gd = gx * uu.x + gy * uu.y + gz * uu.z;
+  return make_float4((gx - gd * uu.x) * uu.w, (gy - gd * uu.y) * uu.w, (gz - gd * uu.z) * uu.w, 0.f);
+}
+
 // After the loop: cotangents of the value rows, gv_i = sum over its pairs (cutoff x logit of edge j<-i)_h g_xa[j] (fields 44..47) and,
 // pair by pair, gv_j += (cutoff x logit of edge i<-j)_h g_xa[i] (fields 48..51)
 template <bool FULL>
@@ -1124,8 +1152,7 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
 // 12-15 dA, 16-19 dB: cotangents of the equivariant logits of edge (i<-j) and (j<-i) | 20-23, 24-27 those logits x cutoff |
 // 28-30 unit vector | 31 1/r | 32 d/dr (cutoff part) | 33 r | 34 1 for a list entry, 0 for a padding row |
 // 36-39, 40-43 cotangents of the invariant logits of edge (i<-j) and (j<-i) |
-// 44-47, 48-51 invariant logits of edges (j<-i) and (i<-j) x cutoff; after the value path has read them: 44-46 angular part of the force
-// on the receiver
+// 44-47, 48-51 invariant logits of edges (j<-i) and (i<-j) x cutoff
 //
 // 16 warps.  Per tile: (1) four threads per edge prepare records and the A operand; (2) MMA chain w = Phi C + hs K2 (both filters);
 // (3) per filter, in two halves of 64 rows: tensor memory -> shared tile, reverse edge loop (4 rows per warp, sender rows
@@ -1160,6 +1187,23 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const long long n_tiles = (n_edges + tr - 1) / tr;
   const long long tile0 = n_tiles * blockIdx.x / gridDim.x, tile1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
   if (tile0 >= tile1) return;
+  const int pad_i = ve_i[n_edges - 1];
+  int* st_ij = reinterpret_cast<int*>(smem + kOffBwStIJ);
+  float4* st_d = reinterpret_cast<float4*>(smem + kOffBwStD);
+  // (i, j) and displacement of one tile's pairs into the staging buffers (threads 384..511): in flight beneath the tile before
+  auto stage_tile = [&](long long t) {
+    if (tid < 384 || t >= tile1) return;
+    const int row = tid - 384;
+    const long long e = t * tr + row;
+    if (row < tr && e < n_edges) {
+      cp_async4(st_ij + 2 * row, ve_i + e); cp_async4(st_ij + 2 * row + 1, ve_j + e);
+      cp_async16(st_d + row, ve_d + e);
+    } else {
+      st_ij[2 * row] = pad_i; st_ij[2 * row + 1] = pad_i;
+      st_d[row] = make_float4(1.f, 0.f, 0.f, 1.f);
+    }
+  };
+  stage_tile(tile0);
   for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kBwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
     const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
@@ -1174,6 +1218,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  cp_async_wait_all();
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -1181,7 +1226,6 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const uint32_t tmem = *tmem_p;
   const uint32_t a_hi = smem_u32(smem + kOffA), img = smem_u32(smem + kOffImg);
   unsigned char* a_ptr = smem + kOffA;
-  const int pad_i = ve_i[n_edges - 1];
   const int deg = degree_of(lane < kMTot ? lane : 0);
   const int quad = warp & 3;                    // TMEM lane quadrant of this warp
   const int n_scat = n_recv;                    // partners below it own a row: they receive their share of a pair here
@@ -1201,14 +1245,11 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     // ---- per-edge preparation ----
     {
       const int row = tid & 127, role = tid >> 7;
-      const long long e = tile * tr + row;
-      const bool valid = row < tr && e < n_edges;
-      int i = pad_i, j = pad_i;
-      if (valid) { i = ve_i[e]; j = ve_j[e]; }
+      const bool valid = row < tr && tile * tr + row < n_edges;
+      const int i = st_ij[2 * row], j = st_ij[2 * row + 1];
       float* rp = rec + row * kBwRec;
       if (role < 2) {
-        float4 d = make_float4(1.f, 0.f, 0.f, 1.f);
-        if (valid) d = ve_d[e];
+        const float4 d = st_d[row];
         const float r = d.w;
         // the Chebyshev chunks first: once these 256 threads are through, the Chebyshev steps of both filters' MMA chains start
         // beneath the rest of the preparation (the gathers of the other two threads of an entry above all)
@@ -1262,6 +1303,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     BW_MARK(1);
+    stage_tile(tile + 1);
     if (tid == 0) {
       tc_fence_after();
       issue_filter_mma(tmem, a_hi, img, 0, 1);
@@ -1331,33 +1373,17 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       }
       if (f == 0) {
         edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, rpw * warp, rpw, lane, g_xa, g_qkv, n_scat); });      // while the tensor cores run
-      } else if (tid < 128) {
-        // angular part of the force on the receiver (independent of the radial derivative that the running MMA yields); it
-        // takes the record fields 44..46, which the value path has released
-        float* rp = rec + tid * kBwRec;
-        if (rp[34] != 0.f) {
-          const int j = __float_as_int(rp[0]), i = __float_as_int(rp[1]);
-          const float4 aA = ld4(rp + 20), aB = ld4(rp + 24), uu = ld4(rp + 28);
-          const float* gevi = gev1 + (size_t)i * kMTot;
-          const float* gevj = gev1 + (size_t)j * kMTot;
-          const float aAv[4] = {aA.x, aA.y, aA.z, aA.w}, aBv[4] = {aB.x, aB.y, aB.z, aB.w};
-          float gY[kMTot];
-#pragma unroll
-          for (int c = 0; c < 6; ++c) {
-            const float4 a = ld4(gevi + 4 * c), b = ld4(gevj + 4 * c);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int m = 4 * c + q, l = degree_of(m);
-              const float sgn = (l == 0 || l == 2) ? -1.f : 1.f;
-              gY[m] = aAv[l] * av[q] + sgn * aBv[l] * bv[q];
-            }
-          }
-          float gux, guy, guz;
-          sph_harm_24_vjp(uu.x, uu.y, uu.z, gY, gux, guy, guz);
-          const float gd = gux * uu.x + guy * uu.y + guz * uu.z;
-          st4(rp + 44, make_float4((gux - gd * uu.x) * uu.w, (guy - gd * uu.y) * uu.w, (guz - gd * uu.z) * uu.w, 0.f));
-        }
+      } else {
+        // angular part of the force on the receiver (independent of the radial derivative that the running MMA yields): each of the four
+        // threads of a row takes one degree; the shares wait in the filter tile, above the ones of the last phase
+        const int row = tid & 127;
+        float4 ang = f4_zero();
+        const int l = tid >> 7;
+        if (l == 0) ang = angular_share<1>(rec + row * kBwRec, gev1);
+        else if (l == 1) ang = angular_share<2>(rec + row * kBwRec, gev1);
+        else if (l == 2) ang = angular_share<3>(rec + row * kBwRec, gev1);
+        else ang = angular_share<4>(rec + row * kBwRec, gev1);
+        st4(wt + kAngOff + (l * TE + row) * 4, ang);
       }
       done = true;
       if (tid == 0) done = mbar_wait(mbar, parity);
@@ -1432,7 +1458,10 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       const float* rp = rec + tid * kBwRec;
       const bool on = rp[34] != 0.f;
       const int i = on ? __float_as_int(rp[1]) : -1;
-      const float4 uu = ld4(rp + 28), ang = ld4(rp + 44);
+      const float4 uu = ld4(rp + 28);
+      const float* ap = wt + kAngOff + tid * 4;
+      const float4 an0 = ld4(ap), an1 = ld4(ap + TE * 4), an2 = ld4(ap + 2 * TE * 4), an3 = ld4(ap + 3 * TE * 4);
+      const float4 ang = make_float4((an0.x + an1.x) + (an2.x + an3.x), (an0.y + an1.y) + (an2.y + an3.y), (an0.z + an1.z) + (an2.z + an3.z), 0.f);
       const float* dr = wt + 4 * 4 * TE + tid;
       const float g_r = rp[32] + ((dr[0] + dr[TE]) + (dr[2 * TE] + dr[3 * TE]));
       float fsx = on ? fmaf(g_r, uu.x, ang.x) : 0.f, fsy = on ? fmaf(g_r, uu.y, ang.y) : 0.f, fsz = on ? fmaf(g_r, uu.z, ang.z) : 0.f;
@@ -1509,6 +1538,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       }
       if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
     });
+    cp_async_wait_all();
     __syncthreads();
     BW_MARK(7);
   }
@@ -1517,6 +1547,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   if (dbg && (tid & 31) == 0 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[32 + 8 * warp + q] = bph[q]; }
 #endif
   if (failed && tid == 0) atomicExch(err, 1);
+  cp_async_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");

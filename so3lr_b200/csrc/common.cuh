@@ -154,43 +154,57 @@ SO3LR_HD void sph_harm_24(float x, float y, float z, float* Y) {
   Y[23] = g4 * (x * x * (x * x - 3.f * y * y) - y * y * (3.f * x * x - y * y));
 }
 
+// transpose of the harmonics of degree L (components g[0 .. 2L] of that degree alone), added to (gx, gy, gz)
+template <int L>
+SO3LR_HD void sph_harm_vjp_degree(float x, float y, float z, const float* g, float& gx, float& gy, float& gz) {
+  const float x2 = x * x, y2 = y * y, z2 = z * z;
+  if (L == 1) {
+    const float c1 = 0.4886025119029199f;
+    gx += c1 * g[2]; gy += c1 * g[0]; gz += c1 * g[1];
+  } else if (L == 2) {
+    const float a2 = 1.0925484305920792f, b2 = 0.31539156525252005f, d2 = 0.5462742152960396f;
+    gx += a2 * y * g[0] + a2 * z * g[3] + 2.f * d2 * x * g[4];
+    gy += a2 * x * g[0] + a2 * z * g[1] - 2.f * d2 * y * g[4];
+    gz += a2 * y * g[1] + 6.f * b2 * z * g[2] + a2 * x * g[3];
+  } else if (L == 3) {
+    const float a3 = 0.5900435899266435f, b3 = 2.890611442640554f, c3 = 0.4570457994644658f, d3 = 0.3731763325901154f,
+                e3 = 1.445305721320277f;
+    gx += a3 * 6.f * x * y * g[0] + b3 * y * z * g[1] + c3 * (5.f * z2 - 1.f) * g[4] + e3 * 2.f * x * z * g[5] +
+          a3 * (3.f * x2 - 3.f * y2) * g[6];
+    gy += a3 * (3.f * x2 - 3.f * y2) * g[0] + b3 * x * z * g[1] + c3 * (5.f * z2 - 1.f) * g[2] - e3 * 2.f * y * z * g[5] -
+          a3 * 6.f * x * y * g[6];
+    gz += b3 * x * y * g[1] + c3 * 10.f * y * z * g[2] + d3 * (15.f * z2 - 3.f) * g[3] + c3 * 10.f * x * z * g[4] +
+          e3 * (x2 - y2) * g[5];
+  } else {
+    const float a4 = 2.5033429417967046f, b4 = 1.7701307697799304f, c4 = 0.9461746957575601f, d4 = 0.6690465435572892f,
+                e4 = 0.10578554691520431f, f4 = 0.47308734787878004f, g4 = 0.6258357354491761f;
+    // a4 (x^3 y - x y^3)
+    gx += a4 * (3.f * x2 * y - y2 * y) * g[0]; gy += a4 * (x2 * x - 3.f * x * y2) * g[0];
+    // b4 (3 x^2 y z - y^3 z)
+    gx += b4 * 6.f * x * y * z * g[1]; gy += b4 * (3.f * x2 - 3.f * y2) * z * g[1]; gz += b4 * (3.f * x2 * y - y2 * y) * g[1];
+    // c4 x y (7 z^2 - 1)
+    gx += c4 * y * (7.f * z2 - 1.f) * g[2]; gy += c4 * x * (7.f * z2 - 1.f) * g[2]; gz += c4 * 14.f * x * y * z * g[2];
+    // d4 y (7 z^3 - 3 z)
+    gy += d4 * (7.f * z2 * z - 3.f * z) * g[3]; gz += d4 * y * (21.f * z2 - 3.f) * g[3];
+    // e4 (35 z^4 - 30 z^2 + 3)
+    gz += e4 * (140.f * z2 * z - 60.f * z) * g[4];
+    // d4 x (7 z^3 - 3 z)
+    gx += d4 * (7.f * z2 * z - 3.f * z) * g[5]; gz += d4 * x * (21.f * z2 - 3.f) * g[5];
+    // f4 (x^2 - y^2)(7 z^2 - 1)
+    gx += f4 * 2.f * x * (7.f * z2 - 1.f) * g[6]; gy -= f4 * 2.f * y * (7.f * z2 - 1.f) * g[6];
+    gz += f4 * (x2 - y2) * 14.f * z * g[6];
+    // b4 z (x^3 - 3 x y^2)
+    gx += b4 * z * (3.f * x2 - 3.f * y2) * g[7]; gy -= b4 * z * 6.f * x * y * g[7]; gz += b4 * (x2 * x - 3.f * x * y2) * g[7];
+    // g4 (x^4 - 6 x^2 y^2 + y^4)
+    gx += g4 * (4.f * x2 * x - 12.f * x * y2) * g[8]; gy += g4 * (4.f * y2 * y - 12.f * x2 * y) * g[8];
+  }
+}
 SO3LR_HD void sph_harm_24_vjp(float x, float y, float z, const float* g, float& gx, float& gy, float& gz) {
-  const float c1 = 0.4886025119029199f;
-  gx = c1 * g[2]; gy = c1 * g[0]; gz = c1 * g[1];
-  const float a2 = 1.0925484305920792f, b2 = 0.31539156525252005f, d2 = 0.5462742152960396f;
-  gx += a2 * y * g[3] + a2 * z * g[6] + 2.f * d2 * x * g[7];
-  gy += a2 * x * g[3] + a2 * z * g[4] - 2.f * d2 * y * g[7];
-  gz += a2 * y * g[4] + 6.f * b2 * z * g[5] + a2 * x * g[6];
-  const float a3 = 0.5900435899266435f, b3 = 2.890611442640554f, c3 = 0.4570457994644658f, d3 = 0.3731763325901154f,
-              e3 = 1.445305721320277f;
-  float x2 = x * x, y2 = y * y, z2 = z * z;
-  gx += a3 * 6.f * x * y * g[8] + b3 * y * z * g[9] + c3 * (5.f * z2 - 1.f) * g[12] + e3 * 2.f * x * z * g[13] +
-        a3 * (3.f * x2 - 3.f * y2) * g[14];
-  gy += a3 * (3.f * x2 - 3.f * y2) * g[8] + b3 * x * z * g[9] + c3 * (5.f * z2 - 1.f) * g[10] - e3 * 2.f * y * z * g[13] -
-        a3 * 6.f * x * y * g[14];
-  gz += b3 * x * y * g[9] + c3 * 10.f * y * z * g[10] + d3 * (15.f * z2 - 3.f) * g[11] + c3 * 10.f * x * z * g[12] +
-        e3 * (x2 - y2) * g[13];
-  const float a4 = 2.5033429417967046f, b4 = 1.7701307697799304f, c4 = 0.9461746957575601f, d4 = 0.6690465435572892f,
-              e4 = 0.10578554691520431f, f4 = 0.47308734787878004f, g4 = 0.6258357354491761f;
-  // Y15 = a4 (x^3 y - x y^3)
-  gx += a4 * (3.f * x2 * y - y2 * y) * g[15]; gy += a4 * (x2 * x - 3.f * x * y2) * g[15];
-  // Y16 = b4 (3 x^2 y z - y^3 z)
-  gx += b4 * 6.f * x * y * z * g[16]; gy += b4 * (3.f * x2 - 3.f * y2) * z * g[16]; gz += b4 * (3.f * x2 * y - y2 * y) * g[16];
-  // Y17 = c4 x y (7 z^2 - 1)
-  gx += c4 * y * (7.f * z2 - 1.f) * g[17]; gy += c4 * x * (7.f * z2 - 1.f) * g[17]; gz += c4 * 14.f * x * y * z * g[17];
-  // Y18 = d4 y (7 z^3 - 3 z)
-  gy += d4 * (7.f * z2 * z - 3.f * z) * g[18]; gz += d4 * y * (21.f * z2 - 3.f) * g[18];
-  // Y19 = e4 (35 z^4 - 30 z^2 + 3)
-  gz += e4 * (140.f * z2 * z - 60.f * z) * g[19];
-  // Y20 = d4 x (7 z^3 - 3 z)
-  gx += d4 * (7.f * z2 * z - 3.f * z) * g[20]; gz += d4 * x * (21.f * z2 - 3.f) * g[20];
-  // Y21 = f4 (x^2 - y^2)(7 z^2 - 1)
-  gx += f4 * 2.f * x * (7.f * z2 - 1.f) * g[21]; gy -= f4 * 2.f * y * (7.f * z2 - 1.f) * g[21];
-  gz += f4 * (x2 - y2) * 14.f * z * g[21];
-  // Y22 = b4 z (x^3 - 3 x y^2)
-  gx += b4 * z * (3.f * x2 - 3.f * y2) * g[22]; gy -= b4 * z * 6.f * x * y * g[22]; gz += b4 * (x2 * x - 3.f * x * y2) * g[22];
-  // Y23 = g4 (x^4 - 6 x^2 y^2 + y^4)
-  gx += g4 * (4.f * x2 * x - 12.f * x * y2) * g[23]; gy += g4 * (4.f * y2 * y - 12.f * x2 * y) * g[23];
+  gx = gy = gz = 0.f;
+  sph_harm_vjp_degree<1>(x, y, z, g, gx, gy, gz);
+  sph_harm_vjp_degree<2>(x, y, z, g + 3, gx, gy, gz);
+  sph_harm_vjp_degree<3>(x, y, z, g + 8, gx, gy, gz);
+  sph_harm_vjp_degree<4>(x, y, z, g + 15, gx, gy, gz);
 }
 
 struct Cell {
