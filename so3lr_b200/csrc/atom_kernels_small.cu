@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int
   const int deg = degree_of(lane < kMTot ? lane : 0);
   float w[32];
   load_w128(w, L.res1_k);
+  grid_dep_sync();
   float4 xr = zero4(), inv = zero4();
   float e = 0.f;
   if (warp < AT) {
@@ -223,16 +224,16 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
   float w[32];
   float4 g3 = zero4(), gg = zero4(), vx3 = zero4(), vz = zero4(), vxa = zero4();
   float e = 0.f, ge2 = 0.f, gt = 0.f;
-  if (proj) {      // thread (projection, column): 32 outputs of that projection's head
-    load_w<32>(w, proj + (size_t)((tid >> 7) * 4 + ((tid >> 5) & 3)) * 1024 + lane, 32);
+  if (proj) load_w<32>(w, proj + (size_t)((tid >> 7) * 4 + ((tid >> 5) & 3)) * 1024 + lane, 32);      // thread (projection, column): 32 outputs of its head
+  else load_w128(w, L.ex_xxT);
+  grid_dep_sync();
+  if (proj) {
     for (int k = tid; k < AT * (kProj / 4); k += NTHR) {
       const int a = k / (kProj / 4);
       float* p = g_qkv_up + (size_t)row0 * kProj + 4 * k;
       st4(gq + 4 * k, row0 + a < n ? ld4(p) : zero4());
       if (row0 + a < n) st4(p, zero4());      // the next attention layer adds into zeros
     }
-  } else {
-    load_w128(w, L.ex_xxT);
   }
   if (own) {
     g3 = proj ? ld4(g_xa + ra) : ldg4(g4 + ra);
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_small_kernel(ModelDev M, in
   const int p8 = tid >> 6, c64 = tid & 63;      // eight parts of a 64-column contraction
   float w[32];
   load_w128(w, M.e_reg_k);
+  grid_dep_sync();
   if (warp < AT) st4(act + warp * kF + col, own ? ldg4(x + (size_t)atom * kF + col) : zero4());
   const int z = own ? Z[atom] : 0;
   const int z_e = z < 0 ? 0 : (z >= kZEmbed ? kZEmbed - 1 : z), z_h = z < 0 ? 0 : (z >= kZHead ? kZHead - 1 : z);
@@ -379,6 +381,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_small_kernel(ModelDev M, in
   float w[32];
   float dh0 = 0.f, dh1 = 0.f;
   if (p8 < 8) load_w<8>(w, M.h_fin_kT + (size_t)8 * p8 * 64 + c64, 64);
+  grid_dep_sync();
   if (warp < AT) {
     float4 ae = zero4(), aq = zero4();
     float k0 = 0.f, k1 = 0.f;
@@ -475,23 +478,23 @@ int configure_dense_small_kernels() {
 void launch_atom_post_fwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, float* z1, float* x3, float* gate,
                                 float* x4, float* ev2, const float* projT, float* qkv_next, float* x4_copy, float* ev2_copy) {
   if (n <= 0) return;
-  SO3LR_SMALL_DISPATCH(n, (post_fwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_post_fwd<AT>(), s>>>(L, n, xa, ev1, z1, x3, gate, x4, ev2, projT, qkv_next, x4_copy, ev2_copy)));
+  SO3LR_SMALL_DISPATCH(n, (launch_chained(post_fwd_small_kernel<AT>, (n + AT - 1) / AT, NTHR, smem_post_fwd<AT>(), s, L, n, xa, ev1, z1, x3, gate, x4, ev2, projT, qkv_next, x4_copy, ev2_copy)));
 }
 void launch_atom_post_bwd_small(cudaStream_t s, const LayerDev& L, int n, const float* xa, const float* ev1, const float* z1, const float* x3,
                                 const float* gate, const float* g4, const float* gev2, float* g_xa, float* gev1, const float* proj,
                                 float* g_qkv_up, float* gev1_copy) {
   if (n <= 0) return;
-  SO3LR_SMALL_DISPATCH(n, (post_bwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_post_bwd<AT>(), s>>>(L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, proj, g_qkv_up, gev1_copy)));
+  SO3LR_SMALL_DISPATCH(n, (launch_chained(post_bwd_small_kernel<AT>, (n + AT - 1) / AT, NTHR, smem_post_bwd<AT>(), s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, proj, g_qkv_up, gev1_copy)));
 }
 void launch_heads_fwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* x, float* ze, float* zq, float* zh, float* e_nn,
                             float* q_raw, float* hv) {
   if (n <= 0) return;
-  SO3LR_SMALL_DISPATCH(n, (heads_fwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_heads_fwd<AT>(), s>>>(M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv)));
+  SO3LR_SMALL_DISPATCH(n, (launch_chained(heads_fwd_small_kernel<AT>, (n + AT - 1) / AT, NTHR, smem_heads_fwd<AT>(), s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv)));
 }
 void launch_heads_bwd_small(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* ze, const float* zq, const float* zh,
                             const float* hv, const float* ge, const float* gq, const float* gh, float* gx) {
   if (n <= 0) return;
-  SO3LR_SMALL_DISPATCH(n, (heads_bwd_small_kernel<AT><<<(n + AT - 1) / AT, NTHR, smem_heads_bwd<AT>(), s>>>(M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx)));
+  SO3LR_SMALL_DISPATCH(n, (launch_chained(heads_bwd_small_kernel<AT>, (n + AT - 1) / AT, NTHR, smem_heads_bwd<AT>(), s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx)));
 }
 
 }  // namespace so3lr

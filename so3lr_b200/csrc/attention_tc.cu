@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_r
                                                                          const int* __restrict__ partner, const int* __restrict__ asym,
                                                                          int* __restrict__ total, int* __restrict__ blocks, int* __restrict__ ve_i,
                                                                          int* __restrict__ ve_j, float4* __restrict__ ve_d, int2* __restrict__ ve_orig) {
+  grid_dep_sync();
   __shared__ int start[kCompactRows + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * kCompactRows + warp;
@@ -451,6 +452,7 @@ __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_r
 }
 // counts -> exclusive offsets, and their sum; one CTA (an eighth of a million atoms per 8 counts of a thread)
 __global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* __restrict__ blocks, int* __restrict__ total) {
+  grid_dep_sync();
   __shared__ int warp_sum_[32];
   const int tid = threadIdx.x, lane = tid & 31, per = (n + 1023) / 1024;
   const int b0 = min(tid * per, n), b1 = min(b0 + per, n);
@@ -561,6 +563,17 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   float* st_ev = reinterpret_cast<float*>(smem + kOffFwStEv);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffFwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffFwMisc + 16);
+  for (int k = tid; k < kTcImageBytes / 16; k += kFwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
+  for (int k = tid; k < 512; k += kFwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
+    const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
+    sph[k] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
+  }
+  const uint32_t mbar0 = smem_u32(mbar_p);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  grid_dep_sync();
   const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
@@ -592,16 +605,6 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
 #pragma unroll
     for (int c = 0; c < 6; ++c) { cp_async16(d + 4 * c, gi + 4 * c); cp_async16(d + TE * kEvStride + 4 * c, gj + 4 * c); }
   };
-  for (int k = tid; k < kTcImageBytes / 16; k += kFwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
-  for (int k = tid; k < 512; k += kFwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
-    const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
-    sph[k] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
-  }
-  const uint32_t mbar0 = smem_u32(mbar_p);
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -1173,7 +1176,6 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
                                                                     int* __restrict__ err, long long* __restrict__ dbg,
                                                                     const int2* __restrict__ ve_orig, const int* __restrict__ gate,
                                                                     int n_own) {
-  if (PER_ENTRY && gate && *gate != 0) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* rec = reinterpret_cast<float*>(smem + kOffBwRec);
@@ -1181,6 +1183,18 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   float* wt = reinterpret_cast<float*>(smem + kOffBwW);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffBwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 16);
+  for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
+  for (int k = tid; k < 512; k += kBwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
+    const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
+    sph[k] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
+  }
+  const uint32_t mbar = smem_u32(mbar_p);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  grid_dep_sync();
+  if (PER_ENTRY && gate && *gate != 0) return;
   const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
@@ -1204,16 +1218,6 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     }
   };
   stage_tile(tile0);
-  for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
-  for (int k = tid; k < 512; k += kBwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
-    const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
-    sph[k] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
-  }
-  const uint32_t mbar = smem_u32(mbar_p);
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -1619,11 +1623,11 @@ int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const in
   const int n_blocks = (n_rows + kCompactRows - 1) / kCompactRows, threads = 32 * kCompactRows;
   if (n_blocks > V->block_cap) return kInvalidArgument;
   if (n_rows < kOrderedRows) {
-    { compact_rows_kernel<kReserve><<<n_blocks, threads, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, V->total, nullptr, V->i, V->j, V->d, orig); count_launch(); }
+    { launch_chained(compact_rows_kernel<kReserve>, n_blocks, threads, 0, s, n_rows, n, row_ptr, nbr_j, dR, partner, asym, V->total, nullptr, V->i, V->j, V->d, orig); count_launch(); }
   } else {
-    { compact_rows_kernel<kCount><<<n_blocks, threads, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->blocks, nullptr, nullptr, nullptr, nullptr); count_launch(); }
-    { scan_blocks_kernel<<<1, 1024, 0, s>>>(n_blocks, V->blocks, V->total); count_launch(); }
-    { compact_rows_kernel<kFill><<<n_blocks, threads, 0, s>>>(n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->blocks, V->i, V->j, V->d, orig); count_launch(); }
+    { launch_chained(compact_rows_kernel<kCount>, n_blocks, threads, 0, s, n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->blocks, nullptr, nullptr, nullptr, nullptr); count_launch(); }
+    { launch_chained(scan_blocks_kernel, 1, 1024, 0, s, n_blocks, V->blocks, V->total); count_launch(); }
+    { launch_chained(compact_rows_kernel<kFill>, n_blocks, threads, 0, s, n_rows, n, row_ptr, nbr_j, dR, partner, asym, nullptr, V->blocks, V->i, V->j, V->d, orig); count_launch(); }
   }
   SO3LR_CUDA_CHECK(cudaGetLastError());
   return kOk;
@@ -1692,7 +1696,7 @@ int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, i
     SO3LR_CUDA_CHECK(cudaMemcpyAsync(xa, x_in, (size_t)n_recv * kF * sizeof(float), cudaMemcpyDeviceToDevice, s));
     SO3LR_CUDA_CHECK(cudaMemcpyAsync(ev1, ev_in, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
   }
-  { attn_fwd_tc_kernel<<<sm_count(), kFwThreads, kSmemFwd, s>>>(L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym); count_launch(); }
+  { launch_chained(attn_fwd_tc_kernel, sm_count(), kFwThreads, kSmemFwd, s, L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym); count_launch(); }
   return kOk;
 }
 
@@ -1704,7 +1708,7 @@ int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, i
   // the kernel adds into the receivers' rows: cotangents of q/k/v start at zero, that of ev at the skip term
   if (!gq_preset) SO3LR_CUDA_CHECK(cudaMemsetAsync(g_qkv, 0, (size_t)n_recv * kProj * sizeof(float), s));
   if (!gev_preset) SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, gev1, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  { attn_bwd_tc_kernel<false><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
+  { launch_chained(attn_bwd_tc_kernel<false>, sm_count(), kBwThreads, kSmemBwd, s, L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
                                                               g_qkv, gev_in, F, virial, err, tc_debug_buffer(), nullptr, nullptr, n_own); count_launch(); }
   return kOk;
 }
@@ -1713,7 +1717,7 @@ int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges
                              const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* g_dR, int* err, const int* asym) {
   if (n_recv <= 0) return kOk;
   if (n_recv != V.n_rows || !V.orig) return kInvalidArgument;
-  { attn_bwd_tc_kernel<true><<<sm_count(), kBwThreads, kSmemBwd, s>>>(L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
+  { launch_chained(attn_bwd_tc_kernel<true>, sm_count(), kBwThreads, kSmemBwd, s, L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
                                                              g_qkv, gev_in, g_dR, nullptr, err, nullptr, V.orig, asym, 0); count_launch(); }
   return kOk;
 }

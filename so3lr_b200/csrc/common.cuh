@@ -72,6 +72,15 @@ SO3LR_D float dsilu_f(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
+// First statement of every kernel that launch_chained starts: lets the next kernel of the stream take its place on the chip early,
+// and waits until everything before this one has completed.  What a kernel does ahead of the call may only touch its own
+// shared memory and the model's constant weights.
+SO3LR_D void grid_dep_sync() {
+#ifdef __CUDA_ARCH__
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
 SO3LR_D float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

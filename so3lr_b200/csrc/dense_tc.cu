@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
   T.init(smem);
+  grid_dep_sync();
   const int tid = T.tid, warp = T.warp, lane = T.lane, row = T.row, quarter = T.quarter, c0 = T.c0;
   const uint32_t a_smem = smem_u32(T.A), w_smem = smem_u32(smem + kOffW);
   float* S = T.S;
@@ -645,6 +646,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
   T.init(smem);
+  grid_dep_sync();
   const int tid = T.tid, warp = T.warp, lane = T.lane, row = T.row, quarter = T.quarter, c0 = T.c0;
   const uint32_t a_smem = smem_u32(T.A), w_smem = smem_u32(smem + kOffW);
   unsigned char* A1 = smem + kOffS;   // second operand buffer inside the staging region (projection rounds only)
@@ -985,6 +987,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
   T.init(smem);
+  grid_dep_sync();
   const int tid = T.tid, warp = T.warp, lane = T.lane, row = T.row, quarter = T.quarter, c0 = T.c0;
   const uint32_t a_smem = smem_u32(T.A), w_smem = smem_u32(smem + kOffW);
   float* S = T.S;
@@ -1134,6 +1137,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
   T.init(smem);
+  grid_dep_sync();
   const int tid = T.tid, warp = T.warp, lane = T.lane, row = T.row, quarter = T.quarter, c0 = T.c0;
   const uint32_t a_smem = smem_u32(T.A), w_smem = smem_u32(smem + kOffW);
   unsigned char* A1 = smem + kOffS;   // second operand buffer inside the staging region
@@ -1284,7 +1288,7 @@ void launch_atom_post_fwd_tc(cudaStream_t s, const LayerDev& L, int n, const flo
                              float* x4, float* ev2, const unsigned char* proj_u, float* qkv_next, int* err, float* x4_copy, float* ev2_copy) {
   if (n <= 0) return;
   const int tiles = (n + TM - 1) / TM, grid = tiles < sm_count() ? tiles : sm_count();
-  atom_post_fwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(L, n, xa, ev1, z1, x3, gate, x4, ev2, proj_u, qkv_next, err, x4_copy, ev2_copy);
+  launch_chained(atom_post_fwd_tc_kernel, grid, NTHR, kSmemDense, s, L, n, xa, ev1, z1, x3, gate, x4, ev2, proj_u, qkv_next, err, x4_copy, ev2_copy);
   count_launch();
 }
 
@@ -1293,7 +1297,7 @@ void launch_atom_post_bwd_tc(cudaStream_t s, const LayerDev& L, int n, const flo
                              const float* g_qkv_up, int* err, float* gev1_copy) {
   if (n <= 0) return;
   const int tiles = (n + TM - 1) / TM, grid = tiles < sm_count() ? tiles : sm_count();
-  atom_post_bwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, projT_u, g_qkv_up, err, gev1_copy);
+  launch_chained(atom_post_bwd_tc_kernel, grid, NTHR, kSmemDense, s, L, n, xa, ev1, z1, x3, gate, g4, gev2, g_xa, gev1, projT_u, g_qkv_up, err, gev1_copy);
   count_launch();
 }
 
@@ -1301,14 +1305,14 @@ void launch_heads_fwd_tc(cudaStream_t s, const ModelDev& M, int n, const int* Z,
                          float* q_raw, float* hv, int* err) {
   if (n <= 0) return;
   const int tiles = (n + TM - 1) / TM, grid = tiles < sm_count() ? tiles : sm_count();
-  heads_fwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv, err);
+  launch_chained(heads_fwd_tc_kernel, grid, NTHR, kSmemDense, s, M, n, Z, x, ze, zq, zh, e_nn, q_raw, hv, err);
   count_launch();
 }
 void launch_heads_bwd_tc(cudaStream_t s, const ModelDev& M, int n, const int* Z, const float* ze, const float* zq, const float* zh,
                          const float* hv, const float* ge, const float* gq, const float* gh, float* gx, int* err) {
   if (n <= 0) return;
   const int tiles = (n + TM - 1) / TM, grid = tiles < sm_count() ? tiles : sm_count();
-  heads_bwd_tc_kernel<<<grid, NTHR, kSmemDense, s>>>(M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx, err);
+  launch_chained(heads_bwd_tc_kernel, grid, NTHR, kSmemDense, s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx, err);
   count_launch();
 }
 

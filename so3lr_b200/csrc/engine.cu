@@ -91,6 +91,7 @@ struct ClearArgs {
   void add(void* q, long long words) { if (q && words > 0) { p[count] = static_cast<float*>(q); n[count++] = words; } }
 };
 __global__ void __launch_bounds__(256) clear_kernel(ClearArgs A) {
+  grid_dep_sync();
   for (int k = 0; k < A.count; ++k)
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < A.n[k]; i += (long long)gridDim.x * 256) A.p[k][i] = 0.f;
 }
@@ -99,7 +100,7 @@ void launch_clear(cudaStream_t s, const ClearArgs& A) {
   for (int k = 0; k < A.count; ++k) most = std::max(most, A.n[k]);
   if (most <= 0) return;
   const int blocks = (int)std::min<long long>(8LL * sm_count(), (most + 255) / 256);
-  { clear_kernel<<<blocks, 256, 0, s>>>(A); count_launch(); }
+  { launch_chained(clear_kernel, blocks, 256, 0, s, A); count_launch(); }
 }
 __global__ void combine_energy_kernel(int n, const float* e_nn, const float* e_zbl, const float* e_c, const float* e_d, float* e_atom) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -133,6 +134,7 @@ __global__ void export_list_kernel(int n, long long count, long long capacity, c
 }
 // atoms are evaluated in a spatially sorted order: slot k holds atom perm[k]
 __global__ void gather_positions_kernel(int n, const int* __restrict__ perm, const float* __restrict__ R, float* __restrict__ Rs) {
+  grid_dep_sync();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const size_t a = (size_t)perm[k];
@@ -147,6 +149,7 @@ struct UnsortArgs {
   float* dst[7];
 };
 __global__ void unsort_kernel(int n, const int* __restrict__ perm, const float* __restrict__ Fs, float* __restrict__ F, UnsortArgs A) {
+  grid_dep_sync();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const size_t a = (size_t)perm[k];
@@ -419,7 +422,7 @@ int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bo
   if (S->sorted) {
     int rc0 = spatial_order(S->nws, st, S->cell, S->n, R_user, r_sr, S->d_perm);
     if (rc0) return rc0;
-    { gather_positions_kernel<<<nb, 256, 0, st>>>(S->n, S->d_perm, R_user, S->d_Rs); count_launch(); }
+    { launch_chained(gather_positions_kernel, nb, 256, 0, st, S->n, S->d_perm, R_user, S->d_Rs); count_launch(); }
     { gather_int_kernel<<<nb, 256, 0, st>>>(S->n, S->d_perm, S->d_Z0, S->d_Zs); count_launch(); }
     R = S->d_Rs;
     S->d_Z = S->d_Zs;
@@ -1296,7 +1299,7 @@ SO3LR_B200_API int so3lr_b200_system_compute(so3lr_b200_system* S, void* stream,
   auto evaluate = [&]() -> int {
     const float* R_eval = R;
     if (S->sorted) {
-      { gather_positions_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, S->d_perm, R, S->d_Rs); count_launch(); }
+      { launch_chained(gather_positions_kernel, (n + 255) / 256, 256, 0, st, n, S->d_perm, R, S->d_Rs); count_launch(); }
       R_eval = S->d_Rs;
     }
     int rce = evaluate_fused(S, st, R_eval, S->sorted ? S->F_s : Fout);
@@ -1305,7 +1308,7 @@ SO3LR_B200_API int so3lr_b200_system_compute(so3lr_b200_system* S, void* stream,
     if (S->sorted) {
       UnsortArgs A{{S->e_atom, S->q, S->h, S->e_zbl, S->e_coul, S->e_disp, nullptr},
                    {S->u_e_atom, S->u_q, S->u_h, S->u_zbl, S->u_coul, S->u_disp, nullptr}};
-      { unsort_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, S->d_perm, S->F_s, Fout, A); count_launch(); }
+      { launch_chained(unsort_kernel, (n + 255) / 256, 256, 0, st, n, S->d_perm, S->F_s, Fout, A); count_launch(); }
     }
     return kOk;
   };

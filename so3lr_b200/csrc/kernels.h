@@ -10,6 +10,18 @@ void dev_free(void* p);            // waits for the device first, like cudaFree,
 cudaError_t host_alloc_bytes(void** p, size_t bytes);
 void host_free(void* p);
 void devmem_flush(int device);     // gives the idle blocks back
+// Launch whose kernel starts with grid_dep_sync(): its CTAs may be placed while the kernel before it in the stream still runs, so that the
+// launch itself (1.5 to 2 us between two dependent kernels) and the kernel's own preparations overlap with that one's end.
+template <typename... P, typename... A>
+void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = s;
+  c.attrs = attr; c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
 template <typename T>
 cudaError_t dev_alloc(T** p, size_t n) { return dev_alloc_bytes(reinterpret_cast<void**>(p), (n ? n : 1) * sizeof(T)); }
 template <typename T>

@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(256) layer0_fwd_tab_kernel(SpeciesTables T, co
                                                              const int* __restrict__ row_ptr, const int* __restrict__ nbr_j,
                                                              const float* __restrict__ dR, const int* __restrict__ Z,
                                                              float* __restrict__ xa, float* __restrict__ ev1) {
+  grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= n_recv) return;
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(256) layer0_fwd_tab_kernel(SpeciesTables T, co
 
 // GV[a][z][h] = sum_{t in head h} g_xa[a][t] * v_z[t]
 __global__ void __launch_bounds__(256) layer0_gv_kernel(SpeciesTables T, int n, const float* __restrict__ g_xa, float* __restrict__ GV) {
+  grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int a = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (a >= n) return;
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(128) layer0_bwd_pairs_kernel(SpeciesTables T, 
                                                                const float4* __restrict__ ve_d, const int* __restrict__ Z,
                                                                const float* __restrict__ GV, const float* __restrict__ gev1,
                                                                float* __restrict__ F, float* __restrict__ virial, int n_own) {
+  grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const long long n_pairs = *n_listed;
   const long long warp0 = (long long)blockIdx.x * 4 + (threadIdx.x >> 5), step = (long long)gridDim.x * 128;
@@ -380,30 +383,30 @@ void species_tables_free(SpeciesTables* T) {
 void launch_layer0_fwd_tab(cudaStream_t s, const SpeciesTables& T, const ModelDev& M, int n_recv, int n, const int* row_ptr,
                            const int* nbr_j, const float* dR, const int* Z, float* xa, float* ev1) {
   if (n_recv <= 0) return;
-  { layer0_fwd_tab_kernel<<<(n_recv + 7) / 8, 256, 0, s>>>(T, M.embed_z, n_recv, n, row_ptr, nbr_j, dR, Z, xa, ev1); count_launch(); }
+  { launch_chained(layer0_fwd_tab_kernel, (n_recv + 7) / 8, 256, 0, s, T, M.embed_z, n_recv, n, row_ptr, nbr_j, dR, Z, xa, ev1); count_launch(); }
 }
 
 void launch_layer0_bwd_tab(cudaStream_t s, const SpeciesTables& T, int n_recv, int n_gv, int n, const int* row_ptr, const int* nbr_j,
                            const float* dR, const int* Z, const float* g_xa, const float* gev1, float* GV, float* F, float* virial) {
   if (n_recv <= 0) return;
-  { layer0_gv_kernel<<<(n_gv + 7) / 8, 256, 0, s>>>(T, n_gv, g_xa, GV); count_launch(); }
+  { launch_chained(layer0_gv_kernel, (n_gv + 7) / 8, 256, 0, s, T, n_gv, g_xa, GV); count_launch(); }
   { layer0_bwd_tab_kernel<<<(n_recv + 7) / 8, 256, 0, s>>>(T, n_recv, n, row_ptr, nbr_j, dR, Z, GV, gev1, F, virial); count_launch(); }
 }
 
 void launch_layer0_bwd_pairs(cudaStream_t s, const SpeciesTables& T, int n_recv, int n_gv, const ValidEdges& V, const int* Z, const float* g_xa,
                              const float* gev1, float* GV, float* F, float* virial, int n_own) {
   if (n_recv <= 0) return;
-  { layer0_gv_kernel<<<(n_gv + 7) / 8, 256, 0, s>>>(T, n_gv, g_xa, GV); count_launch(); }
+  { launch_chained(layer0_gv_kernel, (n_gv + 7) / 8, 256, 0, s, T, n_gv, g_xa, GV); count_launch(); }
   // the number of pairs stays on the device: four CTAs per SM walk over the list, fewer where the rows cannot fill them
   int blocks = (int)(((long long)n_recv * 24 + 127) / 128);
   if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-  { layer0_bwd_pairs_kernel<<<blocks, 128, 0, s>>>(T, n_recv, V.total, V.i, V.j, V.d, Z, GV, gev1, F, virial, n_own); count_launch(); }
+  { launch_chained(layer0_bwd_pairs_kernel, blocks, 128, 0, s, T, n_recv, V.total, V.i, V.j, V.d, Z, GV, gev1, F, virial, n_own); count_launch(); }
 }
 
 void launch_layer0_bwd_entries(cudaStream_t s, const SpeciesTables& T, int n, long long n_entries, const int* idx_i, const int* idx_j,
                                const float* dR, const int* Z, const float* g_xa, const float* gev1, float* GV, float* g_dR) {
   if (n <= 0 || n_entries <= 0) return;
-  { layer0_gv_kernel<<<(n + 7) / 8, 256, 0, s>>>(T, n, g_xa, GV); count_launch(); }
+  { launch_chained(layer0_gv_kernel, (n + 7) / 8, 256, 0, s, T, n, g_xa, GV); count_launch(); }
   { layer0_bwd_entries_kernel<<<(unsigned)((n_entries + 127) / 128), 128, 0, s>>>(T, n, n_entries, idx_i, idx_j, dR, Z, GV, gev1, g_dR); count_launch(); }
 }
 

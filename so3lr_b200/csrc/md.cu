@@ -5,6 +5,7 @@
 // advanced by one thread, so a step costs no host round trip.
 //
 // Units: Angstrom, fs, amu, eV.
+#include "kernels.h"
 #include "md.h"
 
 #include <cuda_runtime.h>
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(256) ke_partial_kernel(int n, const float* __r
 __global__ void __launch_bounds__(256) vv_first_scaled_kernel(int n, float dt, const float* __restrict__ m, float* __restrict__ R,
                                                               float* __restrict__ V, const float* __restrict__ F,
                                                               const double* __restrict__ chain) {
+  grid_dep_sync();
   int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const float scale = chain ? (float)chain[1] : 1.0f;
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(256) vv_first_scaled_kernel(int n, float dt, c
 // second half of velocity Verlet; also leaves each block's share of the new kinetic energy (eV)
 __global__ void __launch_bounds__(256) vv_second_ke_kernel(int n, float dt, const float* __restrict__ m, float* __restrict__ V,
                                                            const float* __restrict__ F, double* __restrict__ partials) {
+  grid_dep_sync();
   __shared__ double sh[256];
   int i = blockIdx.x * 256 + threadIdx.x;
   double ke = 0.0;
@@ -166,6 +169,7 @@ __device__ double sum_partials_256(const double* __restrict__ partials, int n_pa
 __global__ void __launch_bounds__(256) nhc_half_steps_kernel(double* chain, int L, int chain_steps, int sy_steps, double dt, double tau,
                                                              double kT, double dof, int n_half, int fresh_scale,
                                                              const double* __restrict__ partials, int n_partials) {
+  grid_dep_sync();
   __shared__ double sh[256];
   if (partials) {
     const double s = sum_partials_256(partials, n_partials, sh);
@@ -308,7 +312,7 @@ void nhc_init(cudaStream_t st, double* chain) {
 
 void nhc_half_steps(cudaStream_t st, double* chain, int L, int chain_steps, int sy_steps, double dt, double tau, double kT, double dof,
                     int n_half, int fresh_scale, const double* partials, int n_partials) {
-  nhc_half_steps_kernel<<<1, 256, 0, st>>>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half, fresh_scale, partials, n_partials);
+  launch_chained(nhc_half_steps_kernel, 1, 256, 0, st, chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half, fresh_scale, partials, n_partials);
   count_launch();
 }
 
@@ -318,12 +322,12 @@ void md_kinetic_partials(cudaStream_t st, int n, const float* m, const float* V,
 }
 
 void md_first_half(cudaStream_t st, int n, float dt, const float* m, float* R, float* V, const float* F, const double* chain) {
-  vv_first_scaled_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, dt, m, R, V, F, chain);
+  launch_chained(vv_first_scaled_kernel, (n + 255) / 256, 256, 0, st, n, dt, m, R, V, F, chain);
   count_launch();
 }
 
 void md_second_half(cudaStream_t st, int n, float dt, const float* m, float* V, const float* F, double* partials) {
-  vv_second_ke_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, dt, m, V, F, partials);
+  launch_chained(vv_second_ke_kernel, (n + 255) / 256, 256, 0, st, n, dt, m, V, F, partials);
   count_launch();
 }
 

@@ -11,6 +11,7 @@ __global__ void sr_geometry_zbl_kernel(ZblParams zbl, Cell cell, int n, long lon
                                        int dR_given, float* __restrict__ dR, float* __restrict__ e_atom,
                                        float* __restrict__ g_dR, const float* __restrict__ ge, float* __restrict__ F_direct, int n_owned,
                                        float* __restrict__ virial) {
+  grid_dep_sync();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_edges) return;
   const int i = edge_i[e], j = nbr_j[e];
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
 __global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* __restrict__ R, const float* __restrict__ q,
                                                         const float* __restrict__ h, const int* __restrict__ Z,
                                                         float4* __restrict__ pq, float4* __restrict__ hz, float4* __restrict__ acc) {
+  grid_dep_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   pq[i] = make_float4(R[3 * (size_t)i], R[3 * (size_t)i + 1], R[3 * (size_t)i + 2], q[i]);
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* __re
 __global__ void __launch_bounds__(256) pair_unpack_kernel(int n, const float4* __restrict__ acc, float* __restrict__ F, float* __restrict__ gq,
                                                           const float* __restrict__ e_nn, const float* __restrict__ e_zbl,
                                                           const float* __restrict__ e_coul, const float* __restrict__ e_disp, float* __restrict__ e_atom) {
+  grid_dep_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 a = acc[i];
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
                                                              const float4* __restrict__ hz, float4* __restrict__ acc,
                                                              float* __restrict__ gh, float* __restrict__ e_coul,
                                                              float* __restrict__ e_disp, float* __restrict__ virial) {
+  grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= n) return;
@@ -362,6 +366,7 @@ __global__ void __launch_bounds__(256) pair_lr_owned_kernel(LrParams P, Cell cel
 __global__ void charge_conserve_kernel(int n_graphs, const int* __restrict__ graph_start, const float* __restrict__ q_raw,
                                        const float* __restrict__ total_charge, const float* __restrict__ hv,
                                        float* __restrict__ q, float* __restrict__ h) {
+  grid_dep_sync();
   __shared__ float red[32];
   const int g = blockIdx.x;
   const int a0 = graph_start[g], a1 = graph_start[g + 1];
@@ -388,6 +393,7 @@ __global__ void charge_conserve_kernel(int n_graphs, const int* __restrict__ gra
 // gq_raw = gq - mean_graph(gq)
 __global__ void charge_conserve_bwd_kernel(int n_graphs, const int* __restrict__ graph_start, const float* __restrict__ gq,
                                            float* __restrict__ gq_raw) {
+  grid_dep_sync();
   __shared__ float red[32];
   const int g = blockIdx.x;
   const int a0 = graph_start[g], a1 = graph_start[g + 1];
@@ -410,6 +416,7 @@ __global__ void charge_conserve_bwd_kernel(int n_graphs, const int* __restrict__
 __global__ void graph_reduce_kernel(int n_graphs, const int* __restrict__ graph_start, const float* __restrict__ e_atom,
                                     const float* __restrict__ q, const float* __restrict__ R, double* __restrict__ e_graph,
                                     float* __restrict__ dipole) {
+  grid_dep_sync();
   __shared__ double red[4][32];
   const int g = blockIdx.x;
   const int a0 = graph_start[g], a1 = graph_start[g + 1];
@@ -453,6 +460,7 @@ __device__ double block_sum_double_256(double v, double* sh) {
 // partials[b][0] = sum a ; with R: partials[b][1..3] = sum q R
 __global__ void __launch_bounds__(256) wide_partial_kernel(int n, const float* __restrict__ a, const float* __restrict__ q,
                                                            const float* __restrict__ R, double* __restrict__ partials) {
+  grid_dep_sync();
   __shared__ double sh[8];
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
@@ -482,6 +490,7 @@ __device__ double wide_total(const double* __restrict__ partials, int n_blocks, 
 __global__ void __launch_bounds__(256) charge_conserve_wide_kernel(int n, const float* __restrict__ q_raw, const float* __restrict__ total_charge,
                                                                    const float* __restrict__ hv, float* __restrict__ q, float* __restrict__ h,
                                                                    const double* __restrict__ partials, int n_blocks) {
+  grid_dep_sync();
   __shared__ double sh[8];
   const float Q = total_charge ? total_charge[0] : 0.f;
   // in double: a float32 shift carries a relative error of 6e-8, which times a million atoms is a visible net charge
@@ -494,6 +503,7 @@ __global__ void __launch_bounds__(256) charge_conserve_wide_kernel(int n, const 
 
 __global__ void __launch_bounds__(256) charge_conserve_bwd_wide_kernel(int n, const float* __restrict__ gq, float* __restrict__ gq_raw,
                                                                        const double* __restrict__ partials, int n_blocks) {
+  grid_dep_sync();
   __shared__ double sh[8];
   const float mean = (float)wide_total(partials, n_blocks, 0, sh) / (float)n;
   for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) gq_raw[i] = gq[i] - mean;
@@ -501,6 +511,7 @@ __global__ void __launch_bounds__(256) charge_conserve_bwd_wide_kernel(int n, co
 
 __global__ void __launch_bounds__(256) graph_reduce_wide_kernel(const double* __restrict__ partials, int n_blocks, int with_dipole,
                                                                 double* __restrict__ e_graph, float* __restrict__ dipole) {
+  grid_dep_sync();
   __shared__ double sh[8];
   for (int k = 0; k < (with_dipole ? 4 : 1); ++k) {
     const double t = wide_total(partials, n_blocks, k, sh);
@@ -519,7 +530,7 @@ void launch_sr_geometry_zbl(cudaStream_t s, const ModelDev& M, const Cell& cell,
                             float* F_direct, int n_owned, float* virial) {
   if (n_edges <= 0) return;
   unsigned blocks = (unsigned)((n_edges + 255) / 256);
-  { sr_geometry_zbl_kernel<<<blocks, 256, 0, s>>>(M.zbl, cell, n, n_edges, edge_i, nbr_j, Z, R, dR_given, dR, e_atom, g_dR, ge, F_direct, n_owned, virial); count_launch(); }
+  { launch_chained(sr_geometry_zbl_kernel, blocks, 256, 0, s, M.zbl, cell, n, n_edges, edge_i, nbr_j, Z, R, dR_given, dR, e_atom, g_dR, ge, F_direct, n_owned, virial); count_launch(); }
 }
 
 void launch_force_scatter(cudaStream_t s, int n, long long n_edges, const int* edge_i, const int* nbr_j, const float* g_dR, float* F) {
@@ -547,9 +558,9 @@ void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, 
   float4* pq = reinterpret_cast<float4*>(pack);
   float4* acc = pq + n;
   float4* hz = acc + n;
-  pair_pack_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, R, q, h, Z, pq, hz, acc);
-  pair_lr_packed_kernel<<<(n + 7) / 8, 256, 0, s>>>(P, cell, n, row_ptr, nbr_j, pq, hz, acc, gh, e_coul, e_disp, virial);
-  pair_unpack_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, acc, F, gq, e_nn, e_zbl, e_coul, e_disp, e_atom);
+  launch_chained(pair_pack_kernel, (n + 255) / 256, 256, 0, s, n, R, q, h, Z, pq, hz, acc);
+  launch_chained(pair_lr_packed_kernel, (n + 7) / 8, 256, 0, s, P, cell, n, row_ptr, nbr_j, pq, hz, acc, gh, e_coul, e_disp, virial);
+  launch_chained(pair_unpack_kernel, (n + 255) / 256, 256, 0, s, n, acc, F, gq, e_nn, e_zbl, e_coul, e_disp, e_atom);
   count_launch(3);
 }
 
@@ -566,34 +577,34 @@ void launch_charge_conserve(cudaStream_t s, int n_graphs, const int* graph_start
                             const float* total_charge, const float* hv, float* q, float* h, int n_atoms, double* scratch) {
   if (n_graphs <= 0) return;
   if (n_graphs == 1 && scratch && n_atoms >= kWideMinAtoms) {
-    wide_partial_kernel<<<kWideBlocks, 256, 0, s>>>(n_atoms, q_raw, nullptr, nullptr, scratch);
-    charge_conserve_wide_kernel<<<kWideBlocks, 256, 0, s>>>(n_atoms, q_raw, total_charge, hv, q, h, scratch, kWideBlocks);
+    launch_chained(wide_partial_kernel, kWideBlocks, 256, 0, s, n_atoms, q_raw, nullptr, nullptr, scratch);
+    launch_chained(charge_conserve_wide_kernel, kWideBlocks, 256, 0, s, n_atoms, q_raw, total_charge, hv, q, h, scratch, kWideBlocks);
     count_launch(2);
     return;
   }
-  { charge_conserve_kernel<<<n_graphs, 256, 0, s>>>(n_graphs, graph_start, q_raw, total_charge, hv, q, h); count_launch(); }
+  { launch_chained(charge_conserve_kernel, n_graphs, 256, 0, s, n_graphs, graph_start, q_raw, total_charge, hv, q, h); count_launch(); }
 }
 void launch_charge_conserve_bwd(cudaStream_t s, int n_graphs, const int* graph_start, const float* gq, float* gq_raw, int n_atoms,
                                 double* scratch) {
   if (n_graphs <= 0) return;
   if (n_graphs == 1 && scratch && n_atoms >= kWideMinAtoms) {
-    wide_partial_kernel<<<kWideBlocks, 256, 0, s>>>(n_atoms, gq, nullptr, nullptr, scratch);
-    charge_conserve_bwd_wide_kernel<<<kWideBlocks, 256, 0, s>>>(n_atoms, gq, gq_raw, scratch, kWideBlocks);
+    launch_chained(wide_partial_kernel, kWideBlocks, 256, 0, s, n_atoms, gq, nullptr, nullptr, scratch);
+    launch_chained(charge_conserve_bwd_wide_kernel, kWideBlocks, 256, 0, s, n_atoms, gq, gq_raw, scratch, kWideBlocks);
     count_launch(2);
     return;
   }
-  { charge_conserve_bwd_kernel<<<n_graphs, 256, 0, s>>>(n_graphs, graph_start, gq, gq_raw); count_launch(); }
+  { launch_chained(charge_conserve_bwd_kernel, n_graphs, 256, 0, s, n_graphs, graph_start, gq, gq_raw); count_launch(); }
 }
 void launch_graph_reduce(cudaStream_t s, int n_graphs, const int* graph_start, const float* e_atom, const float* q,
                          const float* R, double* e_graph, float* dipole, int n_atoms, double* scratch) {
   if (n_graphs <= 0) return;
   if (n_graphs == 1 && scratch && n_atoms >= kWideMinAtoms) {
-    wide_partial_kernel<<<kWideBlocks, 256, 0, s>>>(n_atoms, e_atom, q, R, scratch);
-    graph_reduce_wide_kernel<<<1, 256, 0, s>>>(scratch, kWideBlocks, R ? 1 : 0, e_graph, dipole);
+    launch_chained(wide_partial_kernel, kWideBlocks, 256, 0, s, n_atoms, e_atom, q, R, scratch);
+    launch_chained(graph_reduce_wide_kernel, 1, 256, 0, s, scratch, kWideBlocks, R ? 1 : 0, e_graph, dipole);
     count_launch(2);
     return;
   }
-  { graph_reduce_kernel<<<n_graphs, 256, 0, s>>>(n_graphs, graph_start, e_atom, q, R, e_graph, dipole); count_launch(); }
+  { launch_chained(graph_reduce_kernel, n_graphs, 256, 0, s, n_graphs, graph_start, e_atom, q, R, e_graph, dipole); count_launch(); }
 }
 
 }  // namespace so3lr
