@@ -22,7 +22,8 @@
 // reduction per row.  Those cost less than the second evaluation they replace: the L2 takes 5.4 TB/s of 512-byte row reductions
 // (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.  With every pair evaluated at
 // both ends instead, 98,304 atoms took 1.99 / 5.12 ms a launch (forward / reverse), with one evaluation 1.23 / 3.12 ms, and with the
-// logits of four pairs of a receiver summed together, no branches between them, 1.16 / 2.97 ms.
+// logits of four pairs of a receiver summed together, no branches between them, and the first filter finished beneath the second
+// filter's chain, 1.16 / 2.79 ms.
 //
 // The reverse kernel forms dw in the same loop, writes it straight into shared memory as the (FP16-split) A operand of a
 // second MMA chain against the SAME weight image read with the other major-ness,
@@ -1159,8 +1160,8 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
 //
 // 16 warps.  Per tile: (1) four threads per edge prepare records and the A operand; (2) MMA chain w = Phi C + hs K2 (both filters);
 // (3) per filter, in two halves of 64 rows: tensor memory -> shared tile, reverse edge loop (4 rows per warp, sender rows
-// prefetched across the barriers), dw into the A operand; (4) per filter: MMA chain [dPhi | dhs] = dw [C^T | K2^T], then per
-// edge the radial derivative and the spherical hidden layer (the angular part of the force is formed beneath the last chain);
+// prefetched across the barriers), dw into the A operand, MMA chain [dPhi | dhs] = dw [C^T | K2^T]; (4) per edge the radial derivative
+// and the spherical hidden layer (the first filter's and the angular part of the force beneath the second filter's chain);
 // (5) force on the receiver, cotangent of ev.
 // PER_ENTRY (caller-supplied lists): `F` is the gradient with respect to the source list's displacement vectors (3 floats per
 // source entry, added to), `ve_orig` maps compacted entries to source entries, and the launch returns at once when *gate != 0.
@@ -1327,135 +1328,165 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     BW_MARK(2);
     // this thread's shares of its row's cotangents of the invariants and of the radial derivative, both filters
     float ds0 = 0.f, ds1 = 0.f, ds2 = 0.f, ds3 = 0.f, drad = 0.f;
-#pragma unroll 1
-    for (int f = 0; f < 2 && !failed; ++f) {
-#pragma unroll 1
-      for (int hh = 0; hh < 2; ++hh) {
-        if (hh == 1 && nu1 == 0) {      // no rows in the second half
-          if (f == 0) reverse_prefetch<1>(L, rec, wrow0, lane, qkv);
-          break;
-        }
-        const int wrow = hh ? wrow1 : wrow0, nu = hh ? nu1 : nu0;
-        if ((quad >> 1) == hh) {          // the 8 warps whose TMEM lanes hold this half: 32 columns each
-          float v[32];
-          const int col = 32 * (warp >> 2);
-          tmem_ld32_combined(tmem + ((uint32_t)(32 * quad) << 16) + 128 * f + col, v);
-          float* p = wt + (32 * (quad & 1) + lane) * kWStride + col;
+    // accumulators of filter f, rows [64 hh, 64 hh + 64) -> filter tile: the 8 warps whose TMEM lanes hold them, 32 columns each
+    auto copy_half = [&](int f, int hh) {
+      if ((quad >> 1) != hh) return;
+      float v[32];
+      const int col = 32 * (warp >> 2);
+      tmem_ld32_combined(tmem + ((uint32_t)(32 * quad) << 16) + 128 * f + col, v);
+      float* p = wt + (32 * (quad & 1) + lane) * kWStride + col;
 #pragma unroll
-          for (int k = 0; k < 32; k += 4) st4(p + k, make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
-        }
-        tc_fence_before();
-        __syncthreads();
-        BW_MARK(3);
-        if (f == 0) {
-          edge_loops(nu, [&](auto full) { reverse_edges4<0, full>(L, rec, wt, wrow, 64 * hh + wrow, nu, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-          if (hh == 0) reverse_prefetch<0>(L, rec, 64 + wrow1, lane, qkv);      // next run: second half of filter 0
-          else reverse_prefetch<1>(L, rec, wrow0, lane, qkv);                   // next run: first half of filter 1
-        } else {
-          edge_loops(nu, [&](auto full) { reverse_edges4<1, full>(L, rec, wt, wrow, 64 * hh + wrow, nu, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-          if (hh == 0) reverse_prefetch<1>(L, rec, 64 + wrow1, lane, qkv);
-        }
-        BW_MARK(4);
-        __syncthreads();
-      }
-      fence_async_smem();
-      tc_fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-        issue_reverse_mma(tmem, a_hi, img, f);
-        umma_commit(mbar);
-      }
-      __syncwarp();
-      if (f == 1 && lane < kMTot) {      // ev differences of this warp's 8 rows of the final flush: requested now, used after the last MMA
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float* rp = rec + ((rpw * warp + k) & (TE - 1)) * kBwRec;
-          const int j = __float_as_int(rp[0]), i = __float_as_int(rp[1]);
-          dev8[k] = ev_in[(size_t)j * kMTot + lane] - ev_in[(size_t)i * kMTot + lane];
-        }
-      }
-      if (f == 0) {
-        edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, rpw * warp, rpw, lane, g_xa, g_qkv, n_scat); });      // while the tensor cores run
-      } else {
-        // angular part of the force on the receiver (independent of the radial derivative that the running MMA yields): each of the four
-        // threads of a row takes one degree; the shares wait in the filter tile, above the ones of the last phase
-        const int row = tid & 127;
-        float4 ang = f4_zero();
-        const int l = tid >> 7;
-        if (l == 0) ang = angular_share<1>(rec + row * kBwRec, gev1);
-        else if (l == 1) ang = angular_share<2>(rec + row * kBwRec, gev1);
-        else if (l == 2) ang = angular_share<3>(rec + row * kBwRec, gev1);
-        else ang = angular_share<4>(rec + row * kBwRec, gev1);
-        st4(wt + kAngOff + (l * TE + row) * 4, ang);
-      }
-      done = true;
-      if (tid == 0) done = mbar_wait(mbar, parity);
-      parity ^= 1;
-      if (!__syncthreads_and(done)) { failed = true; break; }
-      tc_fence_after();
-      BW_MARK(5);
-      // ---- per edge: radial derivative (even terms: threads 0..127, odd terms: 128..255), spherical hidden layer (all four threads of a row) ----
+      for (int k = 0; k < 32; k += 4) st4(p + k, make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+    };
+    // per pair, once the second MMA chain of filter f is through: radial derivative and spherical hidden layer (all four threads of a row)
+    auto finish_filter = [&](int f) {
+      const int row = tid & 127, role = tid >> 7;
+      float* rp = rec + row * kBwRec;
+      const uint32_t lane_base = tmem + ((uint32_t)(32 * quad) << 16) + 128 * f;
       {
-        const int row = tid & 127, role = tid >> 7;
-        float* rp = rec + row * kBwRec;
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * quad) << 16) + 128 * f;
-        {
-          // thread (odd, upper) takes the terms m = 2c + odd of c in [16 upper, 16 upper + 16): columns 32 odd + c.  T_m' = m U_{m-1}, and
-          // U_{n+2} = 2 T_2 U_n - U_{n-2} from (U_{-2}, U_0) or (U_{-3}, U_{-1}), in the upper half from (U_30, U_32) or (U_29, U_31),
-          // which follow from t by doubling: T_2n = 2 T_n^2 - 1, U_{2n-1} = 2 T_n U_{n-1}, U_n = t U_{n-1} + T_n, U_{n-2} = t U_{n-1} - T_n
-          const int odd = role & 1, upper = role >> 1;
-          const float r = rp[33];
-          const float x = expf(-kChebHalfGamma * r);
-          const float t = fmaf(kChebA, x, kChebB), t2 = 2.f * t;
-          const float dtdr = -kChebA * kChebHalfGamma * x;
-          const float T2 = fmaf(t2, t, -1.f), T2x2 = 2.f * T2;
-          float v[16];
-          tmem_ld16_combined(lane_base + 32 * odd + 16 * upper, v);
-          float up = odd ? -1.f : -t2, uc = odd ? 1.f : 0.f;
-          if (upper) {
-            const float T4 = fmaf(T2x2, T2, -1.f), T8 = fmaf(2.f * T4, T4, -1.f), T16 = fmaf(2.f * T8, T8, -1.f), T32 = fmaf(2.f * T16, T16, -1.f);
-            const float U31 = 16.f * (((T16 * T8) * (T4 * T2)) * t2);
-            const float U30 = fmaf(t, U31, -T32), U32 = fmaf(t, U31, T32);
-            up = odd ? U30 : fmaf(t2, U30, -U31);
-            uc = odd ? U32 : U31;
-          }
-          float acc = 0.f;
-#pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            const int m = 2 * c + odd + 32 * upper;
-            acc = fmaf(v[c] * (float)m, uc, acc);
-            const float un = fmaf(T2x2, uc, -up);
-            up = uc; uc = un;
-          }
-          drad = fmaf(acc, dtdr, drad);
+        // thread (odd, upper) takes the terms m = 2c + odd of c in [16 upper, 16 upper + 16): columns 32 odd + c.  T_m' = m U_{m-1}, and
+        // U_{n+2} = 2 T_2 U_n - U_{n-2} from (U_{-2}, U_0) or (U_{-3}, U_{-1}), in the upper half from (U_30, U_32) or (U_29, U_31),
+        // which follow from t by doubling: T_2n = 2 T_n^2 - 1, U_{2n-1} = 2 T_n U_{n-1}, U_n = t U_{n-1} + T_n, U_{n-2} = t U_{n-1} - T_n
+        const int odd = role & 1, upper = role >> 1;
+        const float r = rp[33];
+        const float x = expf(-kChebHalfGamma * r);
+        const float t = fmaf(kChebA, x, kChebB), t2 = 2.f * t;
+        const float dtdr = -kChebA * kChebHalfGamma * x;
+        const float T2 = fmaf(t2, t, -1.f), T2x2 = 2.f * T2;
+        float v[16];
+        tmem_ld16_combined(lane_base + 32 * odd + 16 * upper, v);
+        float up = odd ? -1.f : -t2, uc = odd ? 1.f : 0.f;
+        if (upper) {
+          const float T4 = fmaf(T2x2, T2, -1.f), T8 = fmaf(2.f * T4, T4, -1.f), T16 = fmaf(2.f * T8, T8, -1.f), T32 = fmaf(2.f * T16, T16, -1.f);
+          const float U31 = 16.f * (((T16 * T8) * (T4 * T2)) * t2);
+          const float U30 = fmaf(t, U31, -T32), U32 = fmaf(t, U31, T32);
+          up = odd ? U30 : fmaf(t2, U30, -U31);
+          uc = odd ? U32 : U31;
         }
-        // spherical hidden layer, reverse: the four threads of a row take eight hidden units each
-        {
-          float v[8];
-          tmem_ld8_combined(lane_base + 64 + 8 * role, v);
-          const float4 s4 = ld4(rp + 4);
+        float acc = 0.f;
 #pragma unroll
-          for (int c8 = 0; c8 < 8; ++c8) {
-            const int c = 8 * role + c8;
-            const float* p = sph + (f * 32 + c) * 8;
-            const float4 k = ld4(p);
-            const float z = fmaf(s4.x, k.x, fmaf(s4.y, k.y, fmaf(s4.z, k.z, fmaf(s4.w, k.w, p[4]))));
-            const float sg = __fdividef(1.f, 1.f + __expf(-z));
-            const float dz = v[c8] * sg * (1.f + z * (1.f - sg));
-            ds0 = fmaf(dz, k.x, ds0); ds1 = fmaf(dz, k.y, ds1); ds2 = fmaf(dz, k.z, ds2); ds3 = fmaf(dz, k.w, ds3);
-          }
-          // the filter tile is free after the second filter's edge loops: it takes the four threads' shares
-          if (f == 1) {
-            st4(wt + (role * TE + row) * 4, make_float4(ds0, ds1, ds2, ds3));
-            wt[(4 * 4 + role) * TE + row] = drad;
-          }
+        for (int c = 0; c < 16; ++c) {
+          const int m = 2 * c + odd + 32 * upper;
+          acc = fmaf(v[c] * (float)m, uc, acc);
+          const float un = fmaf(T2x2, uc, -up);
+          up = uc; uc = un;
+        }
+        drad = fmaf(acc, dtdr, drad);
+      }
+      // spherical hidden layer, reverse: the four threads of a row take eight hidden units each
+      {
+        float v[8];
+        tmem_ld8_combined(lane_base + 64 + 8 * role, v);
+        const float4 s4 = ld4(rp + 4);
+#pragma unroll
+        for (int c8 = 0; c8 < 8; ++c8) {
+          const int c = 8 * role + c8;
+          const float* p = sph + (f * 32 + c) * 8;
+          const float4 k = ld4(p);
+          const float z = fmaf(s4.x, k.x, fmaf(s4.y, k.y, fmaf(s4.z, k.z, fmaf(s4.w, k.w, p[4]))));
+          const float sg = __fdividef(1.f, 1.f + __expf(-z));
+          const float dz = v[c8] * sg * (1.f + z * (1.f - sg));
+          ds0 = fmaf(dz, k.x, ds0); ds1 = fmaf(dz, k.y, ds1); ds2 = fmaf(dz, k.z, ds2); ds3 = fmaf(dz, k.w, ds3);
         }
       }
+    };
+    // ---- filter 0 ----
+    copy_half(0, 0);
+    tc_fence_before();
+    __syncthreads();
+    BW_MARK(3);
+    edge_loops(nu0, [&](auto full) { reverse_edges4<0, full>(L, rec, wt, wrow0, wrow0, nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+    if (nu1) {
+      reverse_prefetch<0>(L, rec, 64 + wrow1, lane, qkv);
+      BW_MARK(4);
+      __syncthreads();
+      copy_half(0, 1);
       tc_fence_before();
       __syncthreads();
-      BW_MARK(6);
+      BW_MARK(3);
+      edge_loops(nu1, [&](auto full) { reverse_edges4<0, full>(L, rec, wt, wrow1, 64 + wrow1, nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
     }
+    reverse_prefetch<1>(L, rec, wrow0, lane, qkv);
+    BW_MARK(4);
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      tc_fence_after();
+      issue_reverse_mma(tmem, a_hi, img, 0);
+      umma_commit(mbar);
+    }
+    __syncwarp();
+    // while the tensor cores run: the value path, and the first half of filter 1's accumulators (columns that this chain leaves alone).
+    // What the chain yields is picked up beneath the next one.
+    edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, rpw * warp, rpw, lane, g_xa, g_qkv, n_scat); });
+    copy_half(1, 0);
+    tc_fence_before();
+    done = true;
+    if (tid == 0) done = mbar_wait(mbar, parity);
+    parity ^= 1;
+    if (!__syncthreads_and(done)) { failed = true; break; }
+    tc_fence_after();
+    BW_MARK(5);
+    // ---- filter 1 ----
+    edge_loops(nu0, [&](auto full) { reverse_edges4<1, full>(L, rec, wt, wrow0, wrow0, nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+    if (nu1) {
+      reverse_prefetch<1>(L, rec, 64 + wrow1, lane, qkv);
+      BW_MARK(4);
+      __syncthreads();
+      copy_half(1, 1);
+      tc_fence_before();
+      __syncthreads();
+      BW_MARK(3);
+      edge_loops(nu1, [&](auto full) { reverse_edges4<1, full>(L, rec, wt, wrow1, 64 + wrow1, nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+    }
+    BW_MARK(4);
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      tc_fence_after();
+      issue_reverse_mma(tmem, a_hi, img, 1);
+      umma_commit(mbar);
+    }
+    __syncwarp();
+    if (lane < kMTot) {      // ev differences of this warp's rows of the final flush: requested now, used after the last MMA
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float* rp = rec + ((rpw * warp + k) & (TE - 1)) * kBwRec;
+        const int j = __float_as_int(rp[0]), i = __float_as_int(rp[1]);
+        dev8[k] = ev_in[(size_t)j * kMTot + lane] - ev_in[(size_t)i * kMTot + lane];
+      }
+    }
+    {
+      // angular part of the force on the receiver (independent of the radial derivative that the running MMA yields): each of the four
+      // threads of a row takes one degree; the shares wait in the filter tile, above the ones of the last phase
+      const int row = tid & 127;
+      float4 ang = f4_zero();
+      const int l = tid >> 7;
+      if (l == 0) ang = angular_share<1>(rec + row * kBwRec, gev1);
+      else if (l == 1) ang = angular_share<2>(rec + row * kBwRec, gev1);
+      else if (l == 2) ang = angular_share<3>(rec + row * kBwRec, gev1);
+      else ang = angular_share<4>(rec + row * kBwRec, gev1);
+      st4(wt + kAngOff + (l * TE + row) * 4, ang);
+    }
+    finish_filter(0);
+    done = true;
+    if (tid == 0) done = mbar_wait(mbar, parity);
+    parity ^= 1;
+    if (!__syncthreads_and(done)) { failed = true; break; }
+    tc_fence_after();
+    BW_MARK(5);
+    finish_filter(1);
+    {
+      // the filter tile is free: it takes the four threads' shares
+      const int row = tid & 127, role = tid >> 7;
+      st4(wt + (role * TE + row) * 4, make_float4(ds0, ds1, ds2, ds3));
+      wt[(4 * 4 + role) * TE + row] = drad;
+    }
+    tc_fence_before();
+    __syncthreads();
+    BW_MARK(6);
     if (failed) break;
     // ---- force on the receiver (threads 0..127; the angular part was formed under the last MMA); cotangent of ev (8 rows per warp) ----
     if (tid < 128) {
