@@ -113,11 +113,12 @@ SO3LR_B200_API int so3lr_b200_system_graph_replays(so3lr_b200_system* sys, int64
 SO3LR_B200_API int so3lr_b200_system_aux(so3lr_b200_system* sys, const float** zbl_dev, const float** coulomb_dev,
                           const float** dispersion_dev);
 
-/* Counters: number of list rebuilds, current short-range edges and long-range pairs, kernels launched so far. */
+/* Counters: number of list rebuilds, short-range edges and long-range pairs of the latest build of each list (an export builds the
+ * asked list only), kernels launched so far. */
 SO3LR_B200_API int so3lr_b200_system_stats(so3lr_b200_system* sys, int64_t* n_rebuilds, int64_t* n_edges, int64_t* n_pairs,
                             int64_t* n_launches);
-/* Short-range list entries inside the 4.5 A cutoff at the latest evaluation (the compacted list the tiled attention kernels
- * walk; the list of so3lr_b200_system_stats also holds the skin shell).  Waits for the device. */
+/* Short-range list entries inside the 4.5 A cutoff at the latest evaluation, counted per direction (the tiled attention kernels walk
+ * one entry per pair; the list of so3lr_b200_system_stats also holds the skin shell).  Waits for the device. */
 SO3LR_B200_API int so3lr_b200_system_valid_edges(so3lr_b200_system* sys, int64_t* n_valid);
 
 /* Copy the current neighbor lists out in jax-md layout: idx (2, capacity) int32 on the device, padded with n_atoms
@@ -136,7 +137,8 @@ SO3LR_B200_API int so3lr_b200_system_export_list(so3lr_b200_system* sys, void* s
  * device, no host read), both entries of a pair receive the antisymmetrised cotangent (dE/dd_e - dE/dd_e') / 2, which
  * contracts to the same forces and strain derivative for every motion of atoms or cell; otherwise, or with
  * SO3LR_B200_GRAPH=scatter in the environment, each entry receives dE/dd_e itself.  The call only enqueues work; it
- * allocates when the list is longer than any list the context has seen before.
+ * allocates when the list is longer than any list the context has seen before, and at the context's second evaluation outside
+ * a capture for the first layer's tables (8.4 MB; without that memory it carries on without them).
  * Replaces: potential(graph) and its jax.grad w.r.t. graph.edges / graph.edges_lr
  *           (so3lr/jaxmd_utils.py:130-141, so3lr/graph.py:3-24). */
 SO3LR_B200_API int so3lr_b200_system_graph_eval(so3lr_b200_system* sys, void* stream, int64_t n_edges, const int32_t* idx_i,

@@ -325,7 +325,7 @@ struct so3lr_b200_system {
   NeighborListDev sr, lrl;
   int sr_rows = 0;               // rows of the short-range list (all atoms, or the owned ones of a decomposed evaluation)
   ValidEdges ve;                 // its entries inside the cutoff, compacted at every evaluation
-  NlistWorkspace* nws = nullptr;
+  NlistWorkspace *nws = nullptr, *nws_lr = nullptr;      // one per list (the second one is taken when it is first needed)
   float* d_Rref = nullptr;
   int* d_flag = nullptr;   // [0] skin test of the current step, [1] sticky error word of the tensor-core kernels' bounded waits,
                            // [2] graph-level call: the caller's list is not symmetric
@@ -414,7 +414,8 @@ int ensure_edge_buffers(so3lr_b200_system* S, long long n_edges) {
 
 constexpr int kSortMinAtoms = 512;
 
-int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bool allow_sort) {
+// `which` 0 / 1: the short- / long-range list alone (exported lists), otherwise both
+int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bool allow_sort, int which = -1) {
   const float r_sr = kCutoffSr + S->opt.skin;
   const float* R = R_user;
   const int nb = (S->n + 255) / 256;
@@ -435,8 +436,6 @@ int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bo
   const int* seg = S->n_graphs > 1 ? S->d_seg : nullptr;
   const int* gs = (S->n_graphs > 1 && !S->cell.periodic) ? S->d_graph_start : nullptr;
   (void)many;
-  int rc = nlist_build(S->nws, st, S->cell, S->n, R, r_sr, 0, seg, gs, &S->sr, 1, nullptr);
-  if (rc) return rc;
   float r_lr;
   const int* gs_lr = gs;
   if (S->opt.cutoff_lr > 0.f) r_lr = S->opt.cutoff_lr + S->opt.skin;
@@ -446,8 +445,20 @@ int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bo
     if (S->cell.periodic) return kInvalidArgument;   // all-pairs long range needs free space
     gs_lr = S->d_graph_start;                        // loop over the graph's atoms, no cells
   }
-  rc = nlist_build(S->nws, st, S->cell, S->n, R, r_lr, S->opt.lr_both_directions ? 0 : 1, seg ? seg : (gs_lr ? S->d_seg : nullptr),
-                   gs_lr, &S->lrl, 1, nullptr);
+  // both lists are counted, the host reads both totals in one wait, then both are filled
+  int rc = kOk;
+  if (which != 1) rc = nlist_begin(S->nws, st, S->cell, S->n, R, r_sr, 0, seg, gs, &S->sr, 1, nullptr, -1, allow_sort);
+  if (rc) return rc;
+  if (which != 0) {
+    if (!S->nws_lr && !(S->nws_lr = nlist_workspace_create())) return kCudaError;
+    rc = nlist_begin(S->nws_lr, st, S->cell, S->n, R, r_lr, S->opt.lr_both_directions ? 0 : 1, seg ? seg : (gs_lr ? S->d_seg : nullptr),
+                     gs_lr, &S->lrl, 1, nullptr, -1, allow_sort);
+    if (rc) return rc;
+  }
+  SO3LR_CUDA_CHECK(cudaStreamSynchronize(st));
+  if (which != 1) rc = nlist_end(S->nws, st, S->cell, &S->sr);
+  if (rc) return rc;
+  if (which != 0) rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
   if (rc) return rc;
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->d_Rref, R_user, (size_t)S->n * 3 * sizeof(float), cudaMemcpyDeviceToDevice, st));
   rc = ensure_edge_buffers(S, S->sr.count);
@@ -1167,6 +1178,7 @@ SO3LR_B200_API int so3lr_b200_system_destroy(so3lr_b200_system* S) {
   species_tables_free(&S->sp);
   S->prof.destroy();
   nlist_workspace_destroy(S->nws);
+  if (S->nws_lr) nlist_workspace_destroy(S->nws_lr);
   for (NeighborListDev* L : {&S->sr, &S->lrl}) { dev_free(L->row_ptr); dev_free(L->nbr_j); dev_free(L->edge_i); }
   dev_free(S->dR);
   valid_edges_free(&S->ve);
@@ -1450,7 +1462,9 @@ SO3LR_B200_API int so3lr_b200_system_export_list(so3lr_b200_system* S, void* str
   tl_launch_counter = &S->n_launches;
   cudaStream_t st = (cudaStream_t)stream;
   S->have_lists = false;
-  int rc = prepare_lists(S, st, R, false);   // lists in the caller's atom order
+  S->prof.begin(kPNlist, st);
+  int rc = rebuild_lists(S, st, R, false, which == 0 ? 0 : 1);   // in the caller's atom order
+  S->prof.end(st);
   if (rc) return rc;
   S->have_lists = false;                      // the next evaluation rebuilds them in its own (sorted) order
   const NeighborListDev& L = which == 0 ? S->sr : S->lrl;
@@ -1484,8 +1498,11 @@ static int graph_eval_impl(so3lr_b200_system* S, void* stream, int64_t n_edges, 
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
     if (cap == cudaStreamCaptureStatusNone) {
-      rc = ensure_species_tables(S, st);
-      if (rc) return rc;
+      if (ensure_species_tables(S, st) != kOk) {      // no memory for them: the generic first layer needs none
+        cudaGetLastError();
+        S->sp.n_species = 0;
+        S->elements.clear();
+      }
     }
   }
   rc = evaluate_graph(S, st, S->d_rowptr_g, idx_j, idx_i, n_edges, S->d_rowptr_lr_g, idx_j_lr, edges, edges_lr, g_edges, g_edges_lr,

@@ -303,6 +303,11 @@ int spatial_order(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, c
 // 64-bit sum of per-row pair counts as the builder forms it before its 32-bit scan; kTooLarge when the CSR offsets would
 // leave the int range (the builder returns the same status before it fills a single row)
 int nlist_row_total(cudaStream_t s, int n, const int* row_count_dev, long long* total_host);
+// nlist_build in two halves with a wait for the stream between them: several lists (a workspace each) share one wait.  `any_order`: the
+// entries of a row may come in any order.
+int nlist_begin(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered, const int* seg,
+                const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order);
+int nlist_end(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, NeighborListDev* out);
 int nlist_build(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
                 const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows = -1);
 

@@ -11,6 +11,13 @@
 
 namespace so3lr {
 
+struct Grid {
+  int nc[3];        // cells per dimension
+  int wrap[3];      // periodic wrap in that dimension
+  float lo[3];      // free space: lower corner
+  float inv_w[3];   // free space: 1 / cell width
+  int n_atoms;      // candidates in all
+};
 struct NlistWorkspace {
   int* cell_of = nullptr;      // n
   int* cell_sorted = nullptr;  // n
@@ -32,6 +39,14 @@ struct NlistWorkspace {
   int key_cap = 0;
   unsigned* masks = nullptr;   // votes of the row count for the fill
   size_t mask_cap = 0;
+  int* ticket = nullptr;       // of the scan at the end of the count kernels
+  // list under way between nlist_begin and nlist_end
+  Grid G{};
+  int n = 0, n_rows = 0, ordered = 0, allow_grow = 1, mask_stride = 0;
+  bool by_graph = false, binned = false;
+  float r_list = 0.f;
+  const float* R = nullptr;
+  const int *seg = nullptr, *graph_start = nullptr;
 };
 
 NlistWorkspace* nlist_workspace_create() { return new NlistWorkspace(); }
@@ -39,19 +54,13 @@ void nlist_workspace_destroy(NlistWorkspace* w) {
   if (!w) return;
   dev_free(w->cell_of); dev_free(w->cell_sorted); dev_free(w->atom_sorted); dev_free(w->atom_iota);
   dev_free(w->cell_start); dev_free(w->row_count); dev_free(w->cub_tmp); dev_free(w->d_total);
-  dev_free(w->key); dev_free(w->key_sorted); dev_free(w->sort_tmp); dev_free(w->pos_sorted); dev_free(w->masks);
+  dev_free(w->key); dev_free(w->key_sorted); dev_free(w->sort_tmp); dev_free(w->pos_sorted); dev_free(w->masks); dev_free(w->ticket);
   if (w->h_total) host_free(w->h_total);
   delete w;
 }
 
 namespace {
 
-struct Grid {
-  int nc[3];        // cells per dimension
-  int wrap[3];      // periodic wrap in that dimension
-  float lo[3];      // free space: lower corner
-  float inv_w[3];   // free space: 1 / cell width
-};
 
 __device__ __forceinline__ void cell_coords(const Cell& cell, const Grid& G, float x, float y, float z, int* c) {
   if (cell.periodic) {
@@ -96,6 +105,44 @@ __global__ void gather_sorted_positions_kernel(int n, const float* __restrict__ 
   pos_sorted[k] = make_float4(R[3 * (size_t)a], R[3 * (size_t)a + 1], R[3 * (size_t)a + 2], __int_as_float(a));
 }
 
+// What the count kernels of short lists do at their end in place of four more launches: the CTA that finishes last turns the row counts
+// into offsets (32 bits) and leaves their 64-bit sum in row_ptr[n] (clamped) and in pinned host memory.
+struct TailScan {
+  int* ticket = nullptr;            // two words, zero before and after: CTAs that are through, rows with an infinite position
+  int* row_ptr = nullptr;
+  long long* total_host = nullptr;  // pinned; -1: the extent of the atoms is not finite
+  bool check_finite = false;
+};
+constexpr int kTailScanRows = 32768;      // one CTA reads 128 counts per thread; above, the device-wide scan is the faster one
+__device__ __forceinline__ void tail_scan(const TailScan& T, int n, const int* __restrict__ row_count) {
+  if (!T.ticket) return;
+  __shared__ int last;
+  __shared__ long long part[8];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(T.ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int tid = threadIdx.x, lane = tid & 31, per = (n + 255) / 256;
+  const int b0 = min(tid * per, n), b1 = min(b0 + per, n);
+  long long sum = 0;
+  for (int b = b0; b < b1; ++b) sum += __ldcg(row_count + b);
+  long long incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const long long t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+  if (lane == 31) part[tid >> 5] = incl;
+  __syncthreads();
+  long long at = incl - sum;
+  for (int w = 0; w < (tid >> 5); ++w) at += part[w];
+  for (int b = b0; b < b1; ++b) { T.row_ptr[b] = (int)at; at += __ldcg(row_count + b); }
+  if (tid == 255) {
+    T.row_ptr[n] = at > 2147483647LL ? 2147483647 : (int)at;
+    *T.total_host = __ldcg(T.ticket + 1) != 0 ? -1 : at;
+    T.ticket[0] = 0; T.ticket[1] = 0;
+  }
+}
+
 // FILL = false: row_count[i] = number of neighbours.  FILL = true: write rows at row_ptr[i].
 // The candidates of a row come in cell order.  Cells that are neighbours along the first axis are neighbours in the sorted array: up to
 // three of them are walked as one range (the 5.5 A cells of the short-range list hold half a warp of atoms each).  In an orthorhombic
@@ -103,12 +150,10 @@ __global__ void gather_sorted_positions_kernel(int n, const float* __restrict__ 
 // leaves the warps' votes in `masks` (optional, mask_stride words per row), and the fill takes them instead of testing every candidate
 // a second time; a row that needs more words is tested again.
 template <bool FILL>
-__global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int n, const float* __restrict__ R, float r_list, float r2max,
-                                                         int ordered, const int* __restrict__ seg,
-                                                         const float4* __restrict__ pos_sorted, const int* __restrict__ cell_start,
-                                                         int* __restrict__ row_count, const int* __restrict__ row_ptr,
-                                                         int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
-                                                         unsigned* __restrict__ masks, int mask_stride) {
+__device__ __forceinline__ void build_row(const Cell& cell, const Grid& G, int n, const float* __restrict__ R, float r_list, float r2max, int ordered,
+                                          const int* __restrict__ seg, const float4* __restrict__ pos_sorted, const int* __restrict__ cell_start,
+                                          int* __restrict__ row_count, const int* __restrict__ row_ptr, int* __restrict__ nbr_j,
+                                          int* __restrict__ edge_i, long long capacity, unsigned* __restrict__ masks, int mask_stride) {
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= n) return;
@@ -143,11 +188,11 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
       int j = -1;
       if (FILL && mine && word < mask_stride) {
         m = mine[word];
-        if ((m >> lane) & 1u) j = __float_as_int(pos_sorted[k].w);
+        if ((m >> lane) & 1u) j = pos_sorted ? __float_as_int(pos_sorted[k].w) : k;
       } else {
         bool hit = false;
         if (k < s1) {
-          const float4 pj = pos_sorted[k];
+          const float4 pj = pos_sorted ? pos_sorted[k] : make_float4(R[3 * (size_t)k], R[3 * (size_t)k + 1], R[3 * (size_t)k + 2], __int_as_float(k));
           j = __float_as_int(pj.w);
           float dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
           min_image(cell, dx, dy, dz);
@@ -164,6 +209,11 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
       count += __popc(m);
     }
   };
+  if (!pos_sorted) {      // a single cell that was not binned: all atoms, in their order
+    range(0, G.n_atoms);
+    if (!FILL && lane == 0) row_count[i] = count;
+    return;
+  }
   const int lo0 = G.nc[0] > 1 ? -1 : 0, hi0 = G.nc[0] > 1 ? 1 : 0;
   const int lo1 = G.nc[1] > 1 ? -1 : 0, hi1 = G.nc[1] > 1 ? 1 : 0;
   const int lo2 = G.nc[2] > 1 ? -1 : 0, hi2 = G.nc[2] > 1 ? 1 : 0;
@@ -192,15 +242,34 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
   if (!FILL && lane == 0) row_count[i] = count;
 }
 
+template <bool FILL>
+__global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int n, const float* __restrict__ R, float r_list, float r2max,
+                                                         int ordered, const int* __restrict__ seg,
+                                                         const float4* __restrict__ pos_sorted, const int* __restrict__ cell_start,
+                                                         int* __restrict__ row_count, const int* __restrict__ row_ptr,
+                                                         int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
+                                                         unsigned* __restrict__ masks, int mask_stride, TailScan tail) {
+  build_row<FILL>(cell, G, n, R, r_list, r2max, ordered, seg, pos_sorted, cell_start, row_count, row_ptr, nbr_j, edge_i, capacity, masks, mask_stride);
+  if (!FILL) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (tail.check_finite && i < n && (threadIdx.x & 31) < 3) {
+      const float v = R[3 * (size_t)i + (threadIdx.x & 31)];
+      if (isinf(v) || (n == 1 && isnan(v))) atomicExch(tail.ticket + 1, 1);      // what makes the extent of all atoms not finite
+    }
+    tail_scan(tail, n, row_count);
+  }
+}
+
 // batched free-space graphs: the candidates of atom i are the atoms of its own graph
 template <bool FILL>
 __global__ void __launch_bounds__(256) build_rows_graph_kernel(int n, const float* __restrict__ R, float r2max, int ordered,
                                                                const int* __restrict__ seg, const int* __restrict__ graph_start,
                                                                int* __restrict__ row_count, const int* __restrict__ row_ptr,
-                                                               int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity) {
+                                                               int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
+                                                               TailScan tail) {
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (i >= n) return;
+  if (i < n) {
   const float xi = R[3 * (size_t)i], yi = R[3 * (size_t)i + 1], zi = R[3 * (size_t)i + 2];
   const int g = seg[i];
   const int s0 = graph_start[g], s1 = graph_start[g + 1];
@@ -221,6 +290,8 @@ __global__ void __launch_bounds__(256) build_rows_graph_kernel(int n, const floa
     count += __popc(m);
   }
   if (!FILL && lane == 0) row_count[i] = count;
+  }
+  if (!FILL) tail_scan(tail, n, row_count);
 }
 
 // 64-bit sum of the per-row counts.  The exclusive scan that follows runs in 32 bits (CSR offsets are int): this total, not
@@ -341,8 +412,11 @@ int spatial_order(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, co
   return kOk;
 }
 
-int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
-                const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows) {
+constexpr int kOneCellAtoms = 1024;      // free space: up to here testing all atoms costs less than finding the cells
+
+int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
+                const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order) {
+  w->n_rows = 0;
   if (n <= 0) { out->count = 0; return kOk; }
   if (n_rows < 0 || n_rows > n) n_rows = n;
   if (n > w->n_cap) {
@@ -354,6 +428,10 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     if ((st = ensure(&w->row_count, (size_t)n + 1))) return st;
     if ((st = ensure(&w->pos_sorted, (size_t)n))) return st;
     w->n_cap = n;
+  }
+  if (!w->ticket) {
+    SO3LR_CUDA_CHECK(dev_alloc(&w->ticket, 2));
+    SO3LR_CUDA_CHECK(cudaMemsetAsync(w->ticket, 0, 2 * sizeof(int), s));
   }
   if (!w->d_total) {
     SO3LR_CUDA_CHECK(dev_alloc(&w->d_total, 1));
@@ -368,6 +446,8 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   const float r2max = r_list * r_list;
   const bool by_graph = graph_start != nullptr && !cell.periodic;
   Grid G{};
+  G.n_atoms = n;
+  bool binned = false;
   int n_cells = 1;
   if (!by_graph) {
     if (cell.periodic) {
@@ -380,6 +460,9 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
         if (nc > 1024) nc = 1024;
         G.nc[k] = nc; G.wrap[k] = 1;
       }
+    } else if (any_order && n <= kOneCellAtoms) {
+      // the entries of a row may come in any order: all atoms are candidates, without the bounding box (a read-back) and the cells
+      for (int k = 0; k < 3; ++k) G.nc[k] = 1;
     } else {
       // bounding box on the host side would need a reduction; use a coarse device-free approach: the caller
       // passes free-space systems of moderate size, so read the positions back once per build.
@@ -400,30 +483,34 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
       }
     }
     n_cells = G.nc[0] * G.nc[1] * G.nc[2];
-    if (n_cells + 1 > w->cell_cap) {
-      int st;
-      if ((st = ensure(&w->cell_start, (size_t)n_cells + 1))) return st;
-      w->cell_cap = n_cells + 1;
+    binned = n_cells > 1;      // the atoms of a single cell come in their own order either way
+    if (binned) {
+      if (n_cells + 1 > w->cell_cap) {
+        int st;
+        if ((st = ensure(&w->cell_start, (size_t)n_cells + 1))) return st;
+        w->cell_cap = n_cells + 1;
+      }
+      { assign_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(cell, G, n, R, w->cell_of, w->atom_iota); count_launch(); }
+      int bits = 1;
+      while ((1 << bits) < n_cells && bits < 31) ++bits;
+      size_t need = 0;
+      cub::DeviceRadixSort::SortPairs(nullptr, need, w->cell_of, w->cell_sorted, w->atom_iota, w->atom_sorted, n, 0, bits, s);
+      size_t need2 = 0;
+      cub::DeviceScan::ExclusiveSum(nullptr, need2, w->row_count, out->row_ptr, n, s);   // sized for the largest row count
+      if (need2 > need) need = need2;
+      if (need > w->cub_bytes) {
+        if (w->cub_tmp) dev_free(w->cub_tmp);
+        SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->cub_tmp, need));
+        w->cub_bytes = need;
+      }
+      size_t tmp = w->cub_bytes;
+      cub::DeviceRadixSort::SortPairs(w->cub_tmp, tmp, w->cell_of, w->cell_sorted, w->atom_iota, w->atom_sorted, n, 0, bits, s);
+      count_launch(2 + (bits + 7) / 8);
+      { cell_bounds_kernel<<<(n + 1 + 255) / 256, 256, 0, s>>>(n, n_cells, w->cell_sorted, w->cell_start); count_launch(); }
+      { gather_sorted_positions_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, R, w->atom_sorted, w->pos_sorted); count_launch(); }
     }
-    { assign_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(cell, G, n, R, w->cell_of, w->atom_iota); count_launch(); }
-    int bits = 1;
-    while ((1 << bits) < n_cells && bits < 31) ++bits;
-    size_t need = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, need, w->cell_of, w->cell_sorted, w->atom_iota, w->atom_sorted, n, 0, bits, s);
-    size_t need2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need2, w->row_count, out->row_ptr, n, s);   // sized for the largest row count
-    if (need2 > need) need = need2;
-    if (need > w->cub_bytes) {
-      if (w->cub_tmp) dev_free(w->cub_tmp);
-      SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->cub_tmp, need));
-      w->cub_bytes = need;
-    }
-    size_t tmp = w->cub_bytes;
-    cub::DeviceRadixSort::SortPairs(w->cub_tmp, tmp, w->cell_of, w->cell_sorted, w->atom_iota, w->atom_sorted, n, 0, bits, s);
-    count_launch(2 + (bits + 7) / 8);
-    { cell_bounds_kernel<<<(n + 1 + 255) / 256, 256, 0, s>>>(n, n_cells, w->cell_sorted, w->cell_start); count_launch(); }
-    { gather_sorted_positions_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, R, w->atom_sorted, w->pos_sorted); count_launch(); }
-  } else {
+  }
+  if (!binned) {
     size_t need = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, need, w->row_count, out->row_ptr, n, s);
     if (need > w->cub_bytes) {
@@ -452,21 +539,39 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     }
     masks = w->masks;
   }
+  TailScan tail;
+  if (n_rows <= kTailScanRows && allow_grow) { tail.ticket = w->ticket; tail.row_ptr = out->row_ptr; tail.total_host = w->h_total; }
+  tail.check_finite = tail.ticket && !by_graph && !cell.periodic && !binned;      // what the bounding box would have found
   if (by_graph)
-    { build_rows_graph_kernel<false><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, w->row_count, nullptr, nullptr, nullptr, 0); count_launch(); }
+    { build_rows_graph_kernel<false><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, w->row_count, nullptr, nullptr, nullptr, 0, tail); count_launch(); }
   else
-    { build_rows_kernel<false><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r_list, r2max, ordered, seg, w->pos_sorted, w->cell_start,
-                                                    w->row_count, nullptr, nullptr, nullptr, 0, masks, mask_stride); count_launch(); }
-  SO3LR_CUDA_CHECK(cudaMemsetAsync(w->d_total, 0, sizeof(long long), s));
-  { int tb = (n_rows + 255) / 256; if (tb > 1024) tb = 1024;
-    row_total_kernel<<<tb, 256, 0, s>>>(n_rows, w->row_count, reinterpret_cast<unsigned long long*>(w->d_total)); count_launch(); }
-  size_t tmp = w->cub_bytes;
-  cub::DeviceScan::ExclusiveSum(w->cub_tmp, tmp, w->row_count, out->row_ptr, n_rows, s);
-  count_launch(2);
-  { finish_scan_kernel<<<1, 32, 0, s>>>(n_rows, out->row_ptr, w->d_total, out->capacity, allow_grow ? nullptr : d_overflow); count_launch(); }
-  SO3LR_CUDA_CHECK(cudaMemcpyAsync(w->h_total, w->d_total, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  SO3LR_CUDA_CHECK(cudaStreamSynchronize(s));
+    { build_rows_kernel<false><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r_list, r2max, ordered, seg, binned ? w->pos_sorted : nullptr,
+                                                    w->cell_start, w->row_count, nullptr, nullptr, nullptr, 0, masks, mask_stride, tail); count_launch(); }
+  if (!tail.ticket) {
+    SO3LR_CUDA_CHECK(cudaMemsetAsync(w->d_total, 0, sizeof(long long), s));
+    { int tb = (n_rows + 255) / 256; if (tb > 1024) tb = 1024;
+      row_total_kernel<<<tb, 256, 0, s>>>(n_rows, w->row_count, reinterpret_cast<unsigned long long*>(w->d_total)); count_launch(); }
+    size_t tmp = w->cub_bytes;
+    cub::DeviceScan::ExclusiveSum(w->cub_tmp, tmp, w->row_count, out->row_ptr, n_rows, s);
+    count_launch(2);
+    { finish_scan_kernel<<<1, 32, 0, s>>>(n_rows, out->row_ptr, w->d_total, out->capacity, allow_grow ? nullptr : d_overflow); count_launch(); }
+    SO3LR_CUDA_CHECK(cudaMemcpyAsync(w->h_total, w->d_total, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  }
+  w->G = G; w->n = n; w->n_rows = n_rows; w->ordered = ordered; w->allow_grow = allow_grow; w->mask_stride = mask_stride;
+  w->by_graph = by_graph; w->binned = binned; w->r_list = r_list; w->R = R; w->seg = seg; w->graph_start = graph_start;
+  SO3LR_CUDA_CHECK(cudaGetLastError());
+  return kOk;
+}
+
+// the second half, once the stream has been waited for
+int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListDev* out) {
+  const int n_rows = w->n_rows;
+  if (n_rows <= 0) return kOk;
+  const int blocks = (n_rows + 7) / 8, allow_grow = w->allow_grow;
+  const float r2max = w->r_list * w->r_list;
+  w->n_rows = 0;
   const long long total = *w->h_total;
+  if (total < 0) return kNotFinite;
   if (total > 2147483000LL) return kTooLarge;
   if (total > out->capacity) {
     if (!allow_grow) {
@@ -483,15 +588,24 @@ int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   }
   if (total <= out->capacity) out->count = total;
   const bool truncated = total > out->capacity;
-  if (by_graph)
-    { build_rows_graph_kernel<true><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, nullptr, out->row_ptr,
-                                                         out->nbr_j, out->edge_i, out->capacity); count_launch(); }
+  if (w->by_graph)
+    { build_rows_graph_kernel<true><<<blocks, 256, 0, s>>>(n_rows, w->R, r2max, w->ordered, w->seg, w->graph_start, nullptr, out->row_ptr,
+                                                         out->nbr_j, out->edge_i, out->capacity, TailScan{}); count_launch(); }
   else
-    { build_rows_kernel<true><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r_list, r2max, ordered, seg, w->pos_sorted, w->cell_start, nullptr,
-                                                   out->row_ptr, out->nbr_j, out->edge_i, out->capacity, masks, mask_stride); count_launch(); }
+    { build_rows_kernel<true><<<blocks, 256, 0, s>>>(cell, w->G, n_rows, w->R, w->r_list, r2max, w->ordered, w->seg, w->binned ? w->pos_sorted : nullptr,
+                                                   w->cell_start, nullptr, out->row_ptr, out->nbr_j, out->edge_i, out->capacity, w->masks,
+                                                   w->mask_stride, TailScan{}); count_launch(); }
   if (truncated) { clamp_rows_kernel<<<(n_rows + 1 + 255) / 256, 256, 0, s>>>(n_rows, out->row_ptr, out->capacity); count_launch(); }
   SO3LR_CUDA_CHECK(cudaGetLastError());
   return truncated ? kOverflow : kOk;
+}
+
+int nlist_build(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
+                const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows) {
+  int rc = nlist_begin(w, s, cell, n, R, r_list, ordered, seg, graph_start, out, allow_grow, d_overflow, n_rows, false);
+  if (rc) return rc;
+  SO3LR_CUDA_CHECK(cudaStreamSynchronize(s));
+  return nlist_end(w, s, cell, out);
 }
 
 }  // namespace so3lr

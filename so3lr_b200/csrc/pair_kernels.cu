@@ -444,7 +444,7 @@ __global__ void graph_reduce_kernel(int n_graphs, const int* __restrict__ graph_
 
 // ---- one structure with many atoms: the same three operations spread over many CTAs (sums in double, fixed order) ----
 constexpr int kWideBlocks = 296;      // two CTAs per SM of a 148-SM part; a fixed count keeps the order of the double sums independent of the device
-constexpr int kWideMinAtoms = 16384;
+constexpr int kWideMinAtoms = 4096;      // one CTA takes 23 to 28 us for 12,000 atoms, the two wide launches 6
 
 __device__ double block_sum_double_256(double v, double* sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

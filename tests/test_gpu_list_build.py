@@ -37,3 +37,33 @@ def test_rows_are_exact(n, edge, skew, spread, ordered):
         assert got.max(initial=0) <= 1 and (np.diff(i) >= 0).all()
         sure, never = r < rc - 1e-4, r > rc + 1e-4
         assert got[sure].all() and not got[never].any()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 255, 257, 1024, 1025])
+def test_free_space_lists_of_an_evaluation(n):
+    """Below and above the size up to which all atoms of a free-space structure are candidates: the list sizes of an evaluation equal those
+    of a search over all pairs, and an infinite position is refused."""
+    from so3lr_b200.engine import System
+    rng = np.random.default_rng(n)
+    g = np.stack(np.meshgrid(*[np.arange(11)] * 3), -1).reshape(-1, 3)[:n] * 1.9
+    R = (g + rng.normal(scale=0.1, size=g.shape)).astype(np.float32)
+    s = System(np.full(n, 8), None, cutoff_lr=6.0, damping=2.0)
+    Rt = torch.tensor(R, device="cuda")
+    o = s.compute(Rt)
+    torch.cuda.synchronize()
+    r = np.linalg.norm(R[None].astype(np.float64) - R[:, None], axis=-1)
+    np.fill_diagonal(r, 1e9)
+    st = s.stats()
+    near = lambda rc: ((r < rc - 1e-4).sum(), (r < rc + 1e-4).sum())
+    lo, hi = near(4.5)
+    assert lo <= st["edges"] <= hi
+    lo, hi = near(6.0)
+    assert lo <= 2 * st["pairs"] <= hi or lo <= st["pairs"] <= hi
+    assert torch.isfinite(o["forces"]).all()
+    for bad in (float("inf"), -float("inf")):
+        Rb = Rt.clone()
+        Rb[n - 1, 2] = bad
+        with pytest.raises(Exception):
+            s.compute(Rb)
+    o2 = s.compute(Rt)
+    assert float((o2["forces"] - o["forces"]).abs().max()) <= 1e-4 * max(1.0, float(o["forces"].abs().max()))
