@@ -113,7 +113,7 @@ struct TailScan {
   long long* total_host = nullptr;  // pinned; -1: the extent of the atoms is not finite
   bool check_finite = false;
 };
-constexpr int kTailScanRows = 32768;      // one CTA reads 128 counts per thread; above, the device-wide scan is the faster one
+constexpr int kTailScanRows = 32768;      // 16 rounds of one CTA; above, the device-wide scan is the faster one
 __device__ __forceinline__ void tail_scan(const TailScan& T, int n, const int* __restrict__ row_count) {
   if (!T.ticket) return;
   __shared__ int last;
@@ -124,18 +124,42 @@ __device__ __forceinline__ void tail_scan(const TailScan& T, int n, const int* _
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const int tid = threadIdx.x, lane = tid & 31, per = (n + 255) / 256;
-  const int b0 = min(tid * per, n), b1 = min(b0 + per, n);
-  long long sum = 0;
-  for (int b = b0; b < b1; ++b) sum += __ldcg(row_count + b);
-  long long incl = sum;
+  // 2,048 counts at a time, eight consecutive ones per thread (two 16-byte loads and stores)
+  const int tid = threadIdx.x, lane = tid & 31;
+  long long at = 0;
+  for (int base = 0; base < n; base += 2048) {
+    const int k0 = base + 8 * tid;
+    int c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (k0 + 8 <= n) {
+      const int4 a = __ldcg(reinterpret_cast<const int4*>(row_count + k0)), b = __ldcg(reinterpret_cast<const int4*>(row_count + k0) + 1);
+      c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w; c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+    } else {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) { const long long t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
-  if (lane == 31) part[tid >> 5] = incl;
-  __syncthreads();
-  long long at = incl - sum;
-  for (int w = 0; w < (tid >> 5); ++w) at += part[w];
-  for (int b = b0; b < b1; ++b) { T.row_ptr[b] = (int)at; at += __ldcg(row_count + b); }
+      for (int q = 0; q < 8; ++q) if (k0 + q < n) c[q] = __ldcg(row_count + k0 + q);
+    }
+    long long sum = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) sum += c[q];
+    long long incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const long long t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+    if (lane == 31) part[tid >> 5] = incl;
+    __syncthreads();
+    long long mine = at + incl - sum;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { if (w < (tid >> 5)) mine += part[w]; at += part[w]; }
+    __syncthreads();
+    int o[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { o[q] = (int)mine; mine += c[q]; }
+    if (k0 + 8 <= n) {
+      reinterpret_cast<int4*>(T.row_ptr + k0)[0] = make_int4(o[0], o[1], o[2], o[3]);
+      reinterpret_cast<int4*>(T.row_ptr + k0)[1] = make_int4(o[4], o[5], o[6], o[7]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) if (k0 + q < n) T.row_ptr[k0 + q] = o[q];
+    }
+  }
   if (tid == 255) {
     T.row_ptr[n] = at > 2147483647LL ? 2147483647 : (int)at;
     *T.total_host = __ldcg(T.ticket + 1) != 0 ? -1 : at;
