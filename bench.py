@@ -150,15 +150,15 @@ class ClockSampler:
 
 # ---------------------------------------------------------------------------------------------------------------
 # algorithmic (unique-data) bytes per launch of each kernel group: every array the kernel must read or write is
-# counted once.  N atoms, E short-range list entries inside the cutoff (the compacted list the tiled attention kernels walk:
-# receiver, sender and (dx, dy, dz, r) per entry = 24 bytes), P long-range list entries.
+# counted once.  N atoms, E short-range list entries inside the cutoff counted per direction (the tiled attention kernels walk a
+# list of E / 2 pairs: both ends and (dx, dy, dz, r) per pair = 24 bytes), P long-range list entries.
 # ---------------------------------------------------------------------------------------------------------------
 def algorithmic_bytes(group, N, E, P):
     f = 4
     if group == "attn_fwd":      # q1,q2 (256) + ev_i (24) + sender rows k1,v,k2 (384) + ev_j (24) + x_in (128); out xa, ev1 (152)
-        return N * f * (256 + 24 + 384 + 24 + 128 + 152) + E * 24 + (N + 1) * 4
+        return N * f * (256 + 24 + 384 + 24 + 128 + 152) + E * 12
     if group == "attn_bwd":      # q1,q2, g_xa, gev1, ev (i and j once), sender rows; out g_qkv (640), gev_in (24), forces rmw (6)
-        return N * f * (256 + 128 + 24 + 24 + 384 + 640 + 24 + 6) + E * 24 + (N + 1) * 4
+        return N * f * (256 + 128 + 24 + 24 + 384 + 640 + 24 + 6) + E * 12
     if group == "pair_lr":       # per pair: index; per atom: R, q, h, Z in; F, gq, gh, e_coul, e_disp out
         return P * 4 + N * (12 + 4 + 4 + 4 + 12 + 4 + 4 + 4 + 4) + (N + 1) * 4
     if group == "atom_post_fwd":  # xa, ev1 in; z1, x3, gate, x4, ev2 out (+ the next layer's q/k/v rows, 640, where one follows: 2 of 3 launches)
@@ -172,7 +172,7 @@ def algorithmic_bytes(group, N, E, P):
 # box (attn_bwd_tc_kernel, attn_fwd_tc_kernel; atom_post_*_tc_kernel: the launch with the fused projections).  A full-size
 # capture is not taken (ncu replays each launch about 40 times); lists and per-atom arrays grow with the atom count at fixed
 # density, so the figure is scaled by N / 98304 and the line says so in `traffic_source`.
-NCU_TRAFFIC_98K = {"attn_bwd": 2240.7e6, "attn_fwd": 838.8e6, "atom_post_fwd": 430.1e6, "atom_post_bwd": 557.2e6}
+NCU_TRAFFIC_98K = {"attn_bwd": 2524.0e6, "attn_fwd": 851.4e6, "atom_post_fwd": 487.2e6, "atom_post_bwd": 559.4e6}
 
 
 def ncu_traffic(group, n_atoms):
@@ -182,7 +182,7 @@ def ncu_traffic(group, n_atoms):
 
 TRAFFIC_SOURCE = "ncu capture of the same kernel on water_98k (98,304 atoms), scaled by the atom count"
 
-# FP16 MMA work of the tiled attention kernels per tile of 128 list entries (M = 128, K = 16 per instruction, 2 FLOPs per MAC):
+# FP16 MMA work of the tiled attention kernels per tile of 128 pairs (M = 128, K = 16 per instruction, 2 FLOPs per MAC):
 # forward 8 instructions with N = 256 and 12 with N = 128; reverse 28 with N = 128 and 48 with N = 96
 ATTN_TILE_FLOPS = {"attn_fwd": 2.0 * 128 * 16 * (8 * 256 + 12 * 128), "attn_bwd": 2.0 * 128 * 16 * (28 * 128 + 48 * 96)}
 
@@ -190,7 +190,7 @@ ATTN_TILE_FLOPS = {"attn_fwd": 2.0 * 128 * 16 * (8 * 256 + 12 * 128), "attn_bwd"
 def tensor_flops(group, N, E=0):
     """FP16 tensor-core FLOPs one launch of a group issues: every FP32-accurate product is three FP16 MMAs (hi*hi, hi*lo, lo*hi)."""
     if group in ATTN_TILE_FLOPS:
-        return ATTN_TILE_FLOPS[group] * ((E + 127) // 128) if E else None
+        return ATTN_TILE_FLOPS[group] * ((E // 2 + 127) // 128) if E else None
     mac = {"atom_post_fwd": 3 * 128 * 128 + 5 * 4 * 32 * 32, "atom_post_bwd": 3 * 128 * 128 + 5 * 4 * 32 * 32,
            "heads": 2 * 128 * 128 + 128 * 64 + 64 * 64}.get(group)
     return None if mac is None else 2.0 * 3.0 * mac * N
