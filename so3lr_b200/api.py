@@ -321,6 +321,18 @@ def _min_image(dR, cell_t):
     return dR - torch.round(s) @ cell_t
 
 
+def _check_cell(cell):
+    """Refuses what is no lattice: anything but a 3 x 3 matrix, or one whose volume is zero (the test of so3lr_b200_system_create).  The
+    displacement kernels divide by the determinant without a look at it.  A cell on the GPU is read back here."""
+    if tuple(cell.shape) != (3, 3):
+        raise ValueError(f"Invalid cell shape {tuple(cell.shape)}. Expected (3, 3).")
+    h = cell.detach().to("cpu", torch.float64).numpy()
+    with np.errstate(invalid="ignore"):
+        det = float((h[0] * np.cross(h[1], h[2])).sum())
+    if not (abs(det) > 1e-12 and np.isfinite(det)):
+        raise torch.linalg.LinAlgError(f"the cell is singular (volume {det}): {h.tolist()}")
+
+
 class _PairDisplacements(torch.autograd.Function):
     """(d, d_lr) of both lists from Cartesian positions, minimum image under `cell_t`; `wide` keeps the dtype of the positions,
     else the displacements come out in float32.  One kernel per list and direction (csrc/displacements.cu)."""
@@ -387,6 +399,9 @@ def neighbor_list_featurizer(displacement_fn, species, fractional_coordinates=Tr
         Rc = _Transform.apply(R, cell_t) if (cell_t is not None and fractional_coordinates) else R
         neighbor, neighbor_lr = torch.as_tensor(neighbor, device=dev), torch.as_tensor(neighbor_lr, device=dev)
         # the kernels take dR = R_j - R_i; the energy does not depend on the sign convention.  JAX gathers clamp the padding index N
+        if cell_t is not None and not cell_t.requires_grad:
+            b = torch.as_tensor(box).to(R.dtype)      # where the caller holds it: no wait for a box on the host
+            _check_cell(b if b.shape == (3, 3) else torch.diag(b.reshape(-1).expand(3)))
         if cell_t is not None and cell_t.requires_grad:      # the caller differentiates with respect to the box itself
             idx = [a.long().clamp(max=n - 1) for a in (*neighbor[:2], *neighbor_lr[:2])]
             dR, dR_lr = _min_image(Rc[idx[1]] - Rc[idx[0]], cell_t), _min_image(Rc[idx[3]] - Rc[idx[2]], cell_t)
@@ -494,6 +509,7 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
                     raise NotImplementedError("one cell per batch is supported")
                 c = c[0]
             if bool(c.abs().sum() > 0):
+                _check_cell(c)
                 cell_t = c
         ii, jj, il, jl = (torch.as_tensor(inputs[k]).to(dev, torch.int32).contiguous() for k in ("idx_i", "idx_j", "idx_i_lr", "idx_j_lr"))
         for which, unsorted in enumerate(lists_unsorted(ii, il)):

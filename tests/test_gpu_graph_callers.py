@@ -1,0 +1,54 @@
+"""What the graph-level callers (So3lr, the jax-md adapter) refuse, accept and differentiate around the displacement kernels
+(csrc/displacements.cu)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _water(n=64):
+    from so3lr_b200 import workloads as W
+    Z, R, cell = W.water_box(n, (n * 29.9) ** (1 / 3), 3)
+    return Z, np.asarray(R, np.float32), np.asarray(cell, np.float32)
+
+
+def _inputs(Z, R, cell):
+    from oracle import so3lr_oracle as O
+    i, j = O.neighbor_list(R.astype(np.float64), cell.astype(np.float64), 4.5, ordered=False)
+    il, jl = O.neighbor_list(R.astype(np.float64), cell.astype(np.float64), 6.0, ordered=False)
+    return dict(positions=R, atomic_numbers=Z, idx_i=i, idx_j=j, idx_i_lr=il, idx_j_lr=jl, cell=cell)
+
+
+_SINGULAR = {"zero_edge": np.diag([10.0, 10.0, 0.0]), "two_equal_vectors": np.array([[10.0, 0, 0], [10.0, 0, 0], [0, 0, 10.0]]),
+             "in_a_plane": np.array([[1.0, 2, 3], [4, 5, 6], [7, 8, 9]]), "not_finite": np.diag([10.0, 10.0, np.inf])}
+
+
+@pytest.mark.parametrize("name", list(_SINGULAR))
+@pytest.mark.parametrize("where", ["cpu", "cuda"])
+def test_singular_cells_are_refused(name, where):
+    """Every entry's displacement would be NaN and drop out: the energy of isolated atoms without an error."""
+    from so3lr_b200 import So3lr, So3lrPotential, to_jax_md
+    Z, R, cell = _water()
+    inputs = _inputs(Z, R, cell)
+    bad = torch.tensor(_SINGULAR[name], dtype=torch.float32, device=where)
+    fn = So3lr(lr_cutoff=6.0)
+    with pytest.raises(torch.linalg.LinAlgError):
+        fn({**inputs, "cell": bad})
+    assert np.isfinite(float(fn(inputs)["energy"]))
+    _, _, energy_fn = to_jax_md(So3lrPotential(lr_cutoff=6.0), None, None, species=Z, fractional_coordinates=False)
+    nb = [torch.tensor(np.stack([inputs[a], inputs[b]]), device="cuda") for a, b in (("idx_i", "idx_j"), ("idx_i_lr", "idx_j_lr"))]
+    Rt = torch.tensor(R, device="cuda")
+    boxes = [bad.T] if name != "zero_edge" else [bad, torch.diagonal(bad)]
+    for box in boxes:
+        with pytest.raises(torch.linalg.LinAlgError):
+            energy_fn(Rt, *nb, box=box)
+    assert np.isfinite(float(energy_fn(Rt, *nb, box=torch.diagonal(torch.tensor(cell, device=where)))))
+
+
+@pytest.mark.parametrize("shape", [(3,), (1,), (2, 3), (9,)])
+def test_cells_that_are_no_matrix_are_refused(shape):
+    from so3lr_b200 import So3lr
+    Z, R, cell = _water()
+    with pytest.raises((ValueError, RuntimeError)):
+        So3lr(lr_cutoff=6.0)({**_inputs(Z, R, cell), "cell": np.full(shape, 12.0, np.float32)})
