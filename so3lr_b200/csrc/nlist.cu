@@ -108,9 +108,9 @@ __global__ void gather_sorted_positions_kernel(int n, const float* __restrict__ 
 // What the count kernels of short lists do at their end in place of four more launches: the CTA that finishes last turns the row counts
 // into offsets (32 bits) and leaves their 64-bit sum in row_ptr[n] (clamped) and in pinned host memory.
 struct TailScan {
-  int* ticket = nullptr;            // two words, zero before and after: CTAs that are through, rows with an infinite position
+  int* ticket = nullptr;            // two words, zero before and after: CTAs that are through, whether a position is not finite
   int* row_ptr = nullptr;
-  long long* total_host = nullptr;  // pinned; -1: the extent of the atoms is not finite
+  long long* total_host = nullptr;  // pinned; -1: a position is not finite
   bool check_finite = false;
 };
 constexpr int kTailScanRows = 32768;      // 16 rounds of one CTA; above, the device-wide scan is the faster one
@@ -277,8 +277,8 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
   if (!FILL) {
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (tail.check_finite && i < n && (threadIdx.x & 31) < 3) {
-      const float v = R[3 * (size_t)i + (threadIdx.x & 31)];
-      if (isinf(v) || (n == 1 && isnan(v))) atomicExch(tail.ticket + 1, 1);      // what makes the extent of all atoms not finite
+      // a NaN is nobody's neighbour: without this test a structure of NaNs would be one of isolated atoms, with zero forces
+      if (!isfinite(R[3 * (size_t)i + (threadIdx.x & 31)])) atomicExch(tail.ticket + 1, 1);
     }
     tail_scan(tail, n, row_count);
   }
@@ -565,7 +565,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   }
   TailScan tail;
   if (n_rows <= kTailScanRows && allow_grow) { tail.ticket = w->ticket; tail.row_ptr = out->row_ptr; tail.total_host = w->h_total; }
-  tail.check_finite = tail.ticket && !by_graph && !cell.periodic && !binned;      // what the bounding box would have found
+  tail.check_finite = tail.ticket && !by_graph && !cell.periodic && !binned;      // in place of the bounding box's test of the extent
   if (by_graph)
     { build_rows_graph_kernel<false><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, w->row_count, nullptr, nullptr, nullptr, 0, tail); count_launch(); }
   else

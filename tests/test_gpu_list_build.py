@@ -67,3 +67,18 @@ def test_free_space_lists_of_an_evaluation(n):
             s.compute(Rb)
     o2 = s.compute(Rt)
     assert float((o2["forces"] - o["forces"]).abs().max()) <= 1e-4 * max(1.0, float(o["forces"].abs().max()))
+
+
+@pytest.mark.parametrize("n,atoms", [(n, a) for n in (1, 2, 31, 1024) for a in ("all", "one")] + [(1025, "all")])
+@pytest.mark.parametrize("skin", [0.0, 1.0])
+def test_positions_that_are_no_numbers_are_refused(n, atoms, skin):
+    """A structure that has blown up has no neighbours and no forces: it must not come back as a converged one.  Above 1,024 atoms the
+    bounding box decides, which looks for a finite extent: NaN along a whole axis."""
+    from so3lr_b200.engine import System
+    R = (np.arange(3 * n).reshape(n, 3) * 0.37 % 19.0).astype(np.float32)
+    Rb = R.copy()
+    Rb[slice(None) if atoms == "all" else n // 2, :] = np.nan
+    s = System(np.full(n, 8), None, cutoff_lr=6.0, damping=2.0, skin=skin)
+    with pytest.raises(Exception):
+        s.compute_host(Rb)
+    assert np.isfinite(s.compute_host(R + np.arange(n)[:, None].astype(np.float32))["energy"]).all()
