@@ -161,6 +161,9 @@ class So3lrPotentialB200:
         # the kernels want lists grouped by centre; jax-md style lists already are
         idx_i, idx_i_lr = idx_i.to(self.device, torch.int32), idx_i_lr.to(self.device, torch.int32)
         unsorted, unsorted_lr = lists_unsorted(idx_i, idx_i_lr)
+        for unsrt, *arrays in ((unsorted, idx_i, idx_j, edges), (unsorted_lr, idx_i_lr, idx_j_lr, edges_lr)):
+            if unsrt and len({a.shape[0] for a in arrays}) > 1:
+                raise ValueError(f"centres, others and edges of unequal length: {[a.shape[0] for a in arrays]}")
         if unsorted:
             perm = torch.sort(idx_i, stable=True).indices
             idx_i, idx_j, edges = idx_i[perm], idx_j[perm], edges[perm]
@@ -512,6 +515,8 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
                 _check_cell(c)
                 cell_t = c
         ii, jj, il, jl = (torch.as_tensor(inputs[k]).to(dev, torch.int32).contiguous() for k in ("idx_i", "idx_j", "idx_i_lr", "idx_j_lr"))
+        if ii.shape != jj.shape or il.shape != jl.shape:
+            raise ValueError(f"index arrays of unequal length: {[a.numel() for a in (ii, jj, il, jl)]}")
         for which, unsorted in enumerate(lists_unsorted(ii, il)):
             if unsorted:
                 p = torch.sort((ii, il)[which], stable=True).indices

@@ -229,6 +229,12 @@ class System:
         edges, edges_lr = t(edges, torch.float32), t(edges_lr, torch.float32)
         ge = None if g_e_atom is None else t(g_e_atom, torch.float32)
         n = self.n
+        # the kernels read one index pair and three components per entry, one cotangent per atom
+        for e, lists in ((edges, (idx_i, idx_j)), (edges_lr, (idx_i_lr, idx_j_lr))):
+            if e.numel() != 3 * e.shape[0] or any(a.numel() < e.shape[0] for a in lists):
+                raise ValueError(f"{tuple(e.shape)} displacements with {[a.numel() for a in lists]} indices")
+        if ge is not None and ge.numel() != n:
+            raise ValueError(f"{ge.numel()} cotangents for {n} atoms")
         out = dict(e_atom=torch.empty(n, device=dev), g_edges=torch.zeros_like(edges), g_edges_lr=torch.zeros_like(edges_lr),
                    partial_charges=torch.empty(n, device=dev), hirshfeld_ratios=torch.empty(n, device=dev))
         s = torch.cuda.current_stream(dev)
@@ -294,9 +300,26 @@ class System:
         return E, self._cell.copy()
 
 
+def _check_indices(device, *arrays):
+    """int32 index arrays of one length on `device`, contiguous: the kernels take bare pointers and one length."""
+    if any(a.dtype != torch.int32 or a.device != device or a.ndim != 1 for a in arrays):
+        raise ValueError(f"index arrays must be 1-D int32 on {device}, not {[(a.dtype, str(a.device), tuple(a.shape)) for a in arrays]}")
+    if len({a.numel() for a in arrays}) > 1:
+        raise ValueError(f"index arrays of unequal length: {[a.numel() for a in arrays]}")
+    return tuple(a.contiguous() for a in arrays)
+
+
 def displacements(R, cell, idx_i, idx_j, dtype=torch.float32):
-    """(E, 3) displacements R[j] - R[i] (minimum image under `cell`, rows = lattice vectors, same dtype as R) of int32 index arrays;
-    indices are clamped to the structure, so padding entries give zero.  R float32 or float64, contiguous, on the GPU."""
+    """(E, 3) displacements R[j] - R[i] (minimum image under `cell`, 3 x 3 and regular, rows = lattice vectors) of int32 index arrays;
+    indices are clamped to the structure, so padding entries give zero.  R (n, 3) float32 or float64 on the GPU."""
+    if R.device.type != "cuda" or R.dtype not in (torch.float32, torch.float64) or R.ndim != 2 or R.shape[1] != 3:
+        raise ValueError(f"positions must be (n, 3) float32 or float64 on a GPU, not {tuple(R.shape)} {R.dtype} on {R.device}")
+    if dtype != torch.float32 and dtype != R.dtype:
+        raise ValueError(f"{dtype} displacements of {R.dtype} positions")
+    if cell is not None and tuple(cell.shape) != (3, 3):
+        raise ValueError(f"Invalid cell shape {tuple(cell.shape)}. Expected (3, 3).")
+    idx_i, idx_j = _check_indices(R.device, idx_i, idx_j)
+    R = R.contiguous()
     cell = None if cell is None else cell.to(R.device, R.dtype).contiguous()
     with torch.cuda.device(R.device):
         out = torch.empty(idx_i.numel(), 3, dtype=dtype, device=R.device)
@@ -314,6 +337,11 @@ def displacements_vjp(n, dtype, device, parts, sign=1.0):
         s = torch.cuda.current_stream(device)
         parts = parts or [(None, None, None)]
         for k, (i, j, g) in enumerate(parts):
+            if g is not None:
+                i, j = _check_indices(out.device, i, j)
+                if tuple(g.shape) != (i.numel(), 3) or g.device != out.device or g.dtype not in (torch.float32, dtype):
+                    raise ValueError(f"cotangents {tuple(g.shape)} {g.dtype} on {g.device} of {i.numel()} displacements")
+                g = g.contiguous()
             check(lib.so3lr_b200_displacements_vjp(C.c_void_p(s.cuda_stream), int(dtype == torch.float64), n, 0 if i is None else i.numel(),
                                                    _ptr(i), _ptr(j), _ptr(g), int(g is not None and g.dtype == torch.float64), float(sign),
                                                    _ptr(acc), int(k == 0), _ptr(out) if k == len(parts) - 1 else None), "displacements_vjp")
@@ -324,7 +352,7 @@ def lists_unsorted(idx_i, idx_i_lr):
     """Two host booleans: whether each index array (int32, on the GPU) is NOT ascending.  Waits for the device."""
     with torch.cuda.device(idx_i.device):
         flags = torch.empty(2, dtype=torch.int32, device=idx_i.device)
-        idx_i, idx_i_lr = idx_i.contiguous(), idx_i_lr.contiguous()
+        (idx_i,), (idx_i_lr,) = _check_indices(idx_i.device, idx_i), _check_indices(idx_i.device, idx_i_lr)
         s = torch.cuda.current_stream(idx_i.device)
         check(lib.so3lr_b200_lists_unsorted(C.c_void_p(s.cuda_stream), idx_i.numel(), _ptr(idx_i), idx_i_lr.numel(), _ptr(idx_i_lr),
                                             _ptr(flags)), "lists_unsorted")

@@ -52,3 +52,53 @@ def test_cells_that_are_no_matrix_are_refused(shape):
     Z, R, cell = _water()
     with pytest.raises((ValueError, RuntimeError)):
         So3lr(lr_cutoff=6.0)({**_inputs(Z, R, cell), "cell": np.full(shape, 12.0, np.float32)})
+
+
+@pytest.mark.parametrize("key", ["idx_i", "idx_j", "idx_i_lr", "idx_j_lr"])
+@pytest.mark.parametrize("order", ["sorted", "shuffled"])
+def test_lists_of_unequal_length_are_refused(key, order):
+    """The kernels take one length per list; a shorter partner array would be read past its end."""
+    from so3lr_b200 import Graph, So3lr, So3lrPotential
+    Z, R, cell = _water()
+    inputs = _inputs(Z, R, cell)
+    if order == "shuffled":
+        for a, b in (("idx_i", "idx_j"), ("idx_i_lr", "idx_j_lr")):
+            p = np.random.default_rng(0).permutation(len(inputs[a]))
+            inputs[a], inputs[b] = inputs[a][p], inputs[b][p]
+    short = {**inputs, key: inputs[key][:-3]}
+    with pytest.raises((ValueError, RuntimeError)):
+        So3lr(lr_cutoff=6.0)(short)
+    t = {k: torch.tensor(short[k], device="cuda") for k in ("idx_i", "idx_j", "idx_i_lr", "idx_j_lr")}
+    d, dl = (torch.ones(len(inputs[k]), 3, device="cuda") for k in ("idx_i", "idx_i_lr"))
+    g = Graph(None, d, torch.tensor(Z), t["idx_i"], t["idx_j"], None, None, None, dl, t["idx_i_lr"], t["idx_j_lr"], None)
+    with pytest.raises((ValueError, RuntimeError)):
+        So3lrPotential(lr_cutoff=6.0)(g)
+
+
+def test_arrays_the_kernels_cannot_read_are_refused():
+    from so3lr_b200.engine import displacements, displacements_vjp, lists_unsorted
+    R = torch.zeros(5, 3, device="cuda")
+    i = torch.arange(4, dtype=torch.int32, device="cuda")
+    g = torch.zeros(4, 3, device="cuda")
+    for a in (i[:3], i.long(), i.cpu(), i.reshape(2, 2)):
+        for pair in ((i, a), (a, i)):
+            with pytest.raises(ValueError):
+                displacements(R, None, *pair)
+            with pytest.raises(ValueError):
+                displacements_vjp(5, torch.float32, R.device, [(*pair, g)])
+    for bad in (R.half(), R.cpu(), R.reshape(-1), torch.zeros(5, 4, device="cuda")):
+        with pytest.raises(ValueError):
+            displacements(bad, None, i, i)
+    for bad in (g[:3], g.half(), g.double(), g.cpu(), g.reshape(-1)):
+        with pytest.raises(ValueError):
+            displacements_vjp(5, torch.float32, R.device, [(i, i, bad)])
+    with pytest.raises(ValueError):
+        displacements(R, torch.ones(3, device="cuda"), i, i)
+    with pytest.raises(ValueError):
+        lists_unsorted(i, i.long())
+    # strided arrays are taken as what they show
+    R2, i2, g2 = torch.randn(5, 6, device="cuda")[:, ::2], torch.arange(8, dtype=torch.int32, device="cuda")[::2] % 5, torch.randn(3, 4, device="cuda").T
+    ref = R2[i2.long()] - R2[i.long()]
+    assert torch.equal(displacements(R2, None, i, i2), ref)
+    want = torch.zeros(5, 3, device="cuda").index_add(0, i2.long(), g2).index_add(0, i.long(), -g2)
+    assert torch.allclose(displacements_vjp(5, torch.float32, R.device, [(i, i2, g2)]), want, atol=1e-6)
