@@ -156,10 +156,9 @@ class So3lrPotentialB200:
                 s.set_kspace(shape, sm, method)
         elif s.kspace is not None:
             s.set_kspace(None)
-        edges, edges_lr = graph.edges, graph.edges_lr
-        idx_i, idx_j, idx_i_lr, idx_j_lr = graph.centers, graph.others, graph.idx_i_lr, graph.idx_j_lr
+        edges, edges_lr = graph.edges.to(self.device, torch.float32), graph.edges_lr.to(self.device, torch.float32)
+        idx_i, idx_j, idx_i_lr, idx_j_lr = (a.to(self.device, torch.int32) for a in (graph.centers, graph.others, graph.idx_i_lr, graph.idx_j_lr))
         # the kernels want lists grouped by centre; jax-md style lists already are
-        idx_i, idx_i_lr = idx_i.to(self.device, torch.int32), idx_i_lr.to(self.device, torch.int32)
         unsorted, unsorted_lr = lists_unsorted(idx_i, idx_i_lr)
         for unsrt, *arrays in ((unsorted, idx_i, idx_j, edges), (unsorted_lr, idx_i_lr, idx_j_lr, edges_lr)):
             if unsrt and len({a.shape[0] for a in arrays}) > 1:
@@ -171,8 +170,7 @@ class So3lrPotentialB200:
             perm_lr = torch.sort(idx_i_lr, stable=True).indices
             idx_i_lr, idx_j_lr, edges_lr = idx_i_lr[perm_lr], idx_j_lr[perm_lr], edges_lr[perm_lr]
         aux = {}
-        e = _GraphEnergy.apply(edges.to(self.device, torch.float32), edges_lr.to(self.device, torch.float32), s, idx_i, idx_j,
-                               idx_i_lr, idx_j_lr, aux,
+        e = _GraphEnergy.apply(edges, edges_lr, s, idx_i, idx_j, idx_i_lr, idx_j_lr, aux,
                                graph.positions.to(self.device, torch.float32) if kspace else None,
                                graph.cell.to(self.device) if kspace else None).to(self.dtype)
         if not has_aux:

@@ -102,3 +102,27 @@ def test_arrays_the_kernels_cannot_read_are_refused():
     assert torch.equal(displacements(R2, None, i, i2), ref)
     want = torch.zeros(5, 3, device="cuda").index_add(0, i2.long(), g2).index_add(0, i.long(), -g2)
     assert torch.allclose(displacements_vjp(5, torch.float32, R.device, [(i, i2, g2)]), want, atol=1e-6)
+
+
+@pytest.mark.parametrize("where", ["cpu", "cuda"])
+def test_shuffled_lists_of_a_graph_on_either_side(where):
+    """A Graph whose arrays are on the host, in any order and integer type: same energies and (reordered) gradients as grouped lists."""
+    from so3lr_b200 import Graph, So3lrPotential
+    Z, R, cell = _water()
+    inp = _inputs(Z, R, cell)
+    p, q = (np.random.default_rng(k).permutation(len(inp[a])) for k, a in enumerate(("idx_i", "idx_i_lr")))
+    c = cell.astype(np.float64)
+    mi = lambda d: d - np.round(d @ np.linalg.inv(c)) @ c
+    d, dl = mi(R[inp["idx_j"]] - R[inp["idx_i"]].astype(np.float64)), mi(R[inp["idx_j_lr"]] - R[inp["idx_i_lr"]].astype(np.float64))
+    pot = So3lrPotential(lr_cutoff=6.0)
+
+    def energies(o, ol, dev):
+        e, el = (torch.tensor(a, dtype=torch.float32, device=dev, requires_grad=True) for a in (d[o], dl[ol]))
+        i, j, il, jl = (torch.tensor(inp[k][s], device=dev) for k, s in (("idx_i", o), ("idx_j", o), ("idx_i_lr", ol), ("idx_j_lr", ol)))
+        E = pot(Graph(None, e, torch.tensor(Z), i, j, None, None, None, el, il, jl, None))
+        return E.detach().cpu(), *(g.cpu() for g in torch.autograd.grad(E.sum(), (e, el)))
+
+    ref = energies(np.arange(len(d)), np.arange(len(dl)), "cuda")
+    got = energies(p, q, where)
+    assert float((got[0] - ref[0]).abs().max()) <= 1e-5 * float(ref[0].abs().max())
+    assert float((got[1] - ref[1][torch.tensor(p)]).abs().max()) <= 1e-4 and float((got[2] - ref[2][torch.tensor(q)]).abs().max()) <= 1e-5
