@@ -183,7 +183,7 @@ SO3LR_B200_API int so3lr_b200_system_graph_eval_kspace(so3lr_b200_system* sys, v
  * the entries of a list, and the transpose: acc4[j_e] += sign g_e, acc4[i_e] -= sign g_e.  Positions, cell, acc4 and
  * g_positions are float32 (is_double = 0) or float64; the displacements / their cotangents are float32, or float64 when
  * positions are and out_double / g_double is set.  Indices are clamped to [0, n_atoms), as a gather under JAX does, so padding
- * entries (index n_atoms) give d = 0.  acc4_dev holds 4 values per atom (16-byte aligned; zeroed first when `clear` is set, so that several
+ * entries (index n_atoms) give d = 0; negative ones count from the end.  acc4_dev holds 4 values per atom (16-byte aligned; zeroed first when `clear` is set, so that several
  * lists can be added up); g_positions_dev (may be NULL) receives its first three columns.  The calls only enqueue work on the
  * current device.
  * Replaces: the endpoint gathers of so3lr/jaxmd_utils.py:57-66 and their transpose under jax.grad. */

@@ -36,8 +36,9 @@ __device__ void load_lattice(const T* __restrict__ cell, Lattice<T>& L) {
   __syncthreads();
 }
 
-// padding entries carry index n: like a clamped gather they read the last atom, so both ends coincide and d = 0
-__device__ __forceinline__ int clamp_index(int k, int n) { return min(max(k, 0), n - 1); }
+// padding entries carry index n: like a clamped gather they read the last atom, so both ends coincide and d = 0; a negative index
+// counts from the end
+__device__ __forceinline__ int clamp_index(int k, int n) { return min(max(k < 0 ? k + n : k, 0), n - 1); }
 
 template <typename T, typename O>
 __global__ void __launch_bounds__(256) displacement_kernel(int n, const T* __restrict__ R, const T* __restrict__ cell, long long n_entries,

@@ -311,7 +311,7 @@ def _check_indices(device, *arrays):
 
 def displacements(R, cell, idx_i, idx_j, dtype=torch.float32):
     """(E, 3) displacements R[j] - R[i] (minimum image under `cell`, 3 x 3 and regular, rows = lattice vectors) of int32 index arrays;
-    indices are clamped to the structure, so padding entries give zero.  R (n, 3) float32 or float64 on the GPU."""
+    indices are clamped to the structure, so padding entries give zero, and negative ones count from its end.  R (n, 3) float32 or float64 on the GPU."""
     if R.device.type != "cuda" or R.dtype not in (torch.float32, torch.float64) or R.ndim != 2 or R.shape[1] != 3:
         raise ValueError(f"positions must be (n, 3) float32 or float64 on a GPU, not {tuple(R.shape)} {R.dtype} on {R.device}")
     if dtype != torch.float32 and dtype != R.dtype:

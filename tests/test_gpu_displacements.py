@@ -46,3 +46,15 @@ def test_displacements_and_transpose(n, entries, grouped, cell, dtype):
     terms = 4 * max(1, np.bincount(np.concatenate([ci, cj]), minlength=n).max())
     np.testing.assert_allclose(out.double().cpu().numpy(), want, atol=terms * eps * 2.0 * max(1.0, np.abs(g).max(initial=0.0)) * np.sqrt(terms))
     assert lists_unsorted(ti, tj) == (bool((np.diff(i) < 0).any()), bool((np.diff(j) < 0).any()))
+
+
+def test_negative_indices_count_from_the_end():
+    """As in the gathers of torch (and of JAX): -1 is the last atom.  Below -n there is no atom: clamped to the first."""
+    from so3lr_b200.engine import displacements, displacements_vjp
+    R = torch.randn(6, 3, device="cuda", generator=torch.Generator("cuda").manual_seed(0))
+    i, j = (torch.tensor(a, dtype=torch.int32, device="cuda") for a in ([0, 1, 2, -1, -6, 3, 6], [-1, -2, -6, 4, 5, -99, -3]))
+    ci, cj = (torch.tensor(a, device="cuda") for a in ([0, 1, 2, 5, 0, 3, 5], [5, 4, 0, 4, 5, 0, 3]))
+    assert torch.equal(displacements(R, None, i, j), R[cj] - R[ci])
+    g = torch.randn(7, 3, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    want = torch.zeros(6, 3, device="cuda").index_add(0, cj, g).index_add(0, ci, -g)
+    assert torch.allclose(displacements_vjp(6, torch.float32, R.device, [(i, j, g)]), want, atol=2e-6)      # at most 4 terms of size 3
