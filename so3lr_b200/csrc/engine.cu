@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(128) charge_spin_atoms_kernel(const float* __r
 __global__ void __launch_bounds__(128) charge_spin_table_kernel(const ChargeSpinRow* __restrict__ list, const float* __restrict__ rows, float* __restrict__ embed) {
   embed[(size_t)list[blockIdx.x].z * kF + threadIdx.x] += rows[(size_t)blockIdx.x * kF + threadIdx.x];
 }
-// rows of the charged / open-shell graphs, and per atom the row it takes (-1: none); false when every psi is 0
+// rows of the charged / open-shell graphs, and per atom the row it takes (-1: none); false when no atom has one
 bool charge_spin_scalars(const so3lr_b200_model& m, int n, const int32_t* Z, int n_graphs, const std::vector<int>& gs, const float* total_charge,
                          const float* num_unpaired, std::vector<ChargeSpinRow>* rows, std::vector<int>* row_of) {
   bool any = false;
@@ -956,7 +956,7 @@ bool charge_spin_scalars(const so3lr_b200_model& m, int n, const int32_t* Z, int
       }
     }
   }
-  return true;
+  return !rows->empty();      // a charged graph without atoms has none
 }
 
 // tables of the first layer, built when the first evaluation that reads them comes (a graph-level context never does)

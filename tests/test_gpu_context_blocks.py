@@ -39,3 +39,19 @@ def test_reused_blocks_give_the_same_results():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not errors, errors[0]
+
+
+@pytest.mark.parametrize("charges", [[1.0, 0.0, 0.0], [0.0, 0.0, -1.0], [2.0, 0.0, 1.0], [1.0, -1.0, 1.0]])
+@pytest.mark.parametrize("kind", ["total_charge", "num_unpaired"])
+def test_charged_graphs_without_atoms(charges, kind):
+    """Three graphs of which the first and the last have no atoms: they have no embedding rows, and a charge of theirs changes nothing."""
+    from so3lr_b200 import workloads as W
+    from so3lr_b200.engine import System
+    Z, R = W.molecule(np.random.default_rng(3), 70)
+    R = torch.tensor(R, dtype=torch.float32, device="cuda")
+    gs = [0, 0, len(Z), len(Z)]
+    make = lambda c: System(Z, None, cutoff_lr=12.0, damping=2.0, lr_format="sparse", graph_start=gs, **{kind: c}).compute(R)
+    got, ref = make(charges), make([0.0, charges[1], 0.0])
+    assert abs(float(got["energy"][1] - ref["energy"][1])) <= 2e-6 * abs(float(ref["energy"][1]))
+    assert float((got["forces"] - ref["forces"]).abs().max()) <= 5e-5
+    assert float(got["energy"][0]) == float(got["energy"][2]) == 0.0
