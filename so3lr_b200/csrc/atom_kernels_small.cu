@@ -23,6 +23,7 @@ constexpr int KP = kF / NP;
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+// the model's weights only (see grid_dep_sync)
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
@@ -117,7 +118,7 @@ __device__ __forceinline__ float pick(float4 v, int l) { return l == 0 ? v.x : (
 
 // The blocks' definitions, inputs and outputs are those of dense_tc.cu.
 template <int AT>
-__global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int n, const float* __restrict__ xa, const float* __restrict__ ev1,
+__global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int n, const float* xa, const float* ev1,
                                                                  float* __restrict__ z1_out, float* __restrict__ x3_out, float* __restrict__ gate_out,
                                                                  float* __restrict__ x4_out, float* __restrict__ ev2_out,
                                                                  const float* __restrict__ projT, float* __restrict__ qkv_next,
@@ -136,8 +137,8 @@ __global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int
   float4 xr = zero4(), inv = zero4();
   float e = 0.f;
   if (warp < AT) {
-    const float4 x = own ? ldg4(xa + ra) : zero4();
-    if (own && lane < kMTot) e = __ldg(ev1 + (size_t)atom * kMTot + lane);
+    const float4 x = own ? ld4(xa + ra) : zero4();
+    if (own && lane < kMTot) e = ev1[(size_t)atom * kMTot + lane];
     float rstd;
     const float4 xh = normalise(x, rstd), sc = ldg4(L.ln1_s + col), bi = ldg4(L.ln1_b + col);
     xr = add4(mul4(xh, sc), bi);
@@ -206,10 +207,10 @@ __global__ void __launch_bounds__(NTHR, 1) post_fwd_small_kernel(LayerDev L, int
 }
 
 template <int AT>
-__global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int n, const float* __restrict__ xa, const float* __restrict__ ev1,
-                                                                 const float* __restrict__ z1, const float* __restrict__ x3,
-                                                                 const float* __restrict__ gate, const float* __restrict__ g4,
-                                                                 const float* __restrict__ gev2, float* g_xa, float* __restrict__ gev1,
+__global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int n, const float* xa, const float* ev1,
+                                                                 const float* z1, const float* x3,
+                                                                 const float* gate, const float* g4,
+                                                                 const float* gev2, float* g_xa, float* __restrict__ gev1,
                                                                  const float* __restrict__ proj, float* g_qkv_up,
                                                                  float* __restrict__ gev1_copy) {
   extern __shared__ __align__(16) float sm[];
@@ -236,12 +237,12 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
     }
   }
   if (own) {
-    g3 = proj ? ld4(g_xa + ra) : ldg4(g4 + ra);
-    vx3 = ldg4(x3 + ra); vz = ldg4(z1 + ra); vxa = ldg4(xa + ra);
+    g3 = ld4((proj ? g_xa : g4) + ra);
+    vx3 = ld4(x3 + ra); vz = ld4(z1 + ra); vxa = ld4(xa + ra);
     if (lane < kMTot) {
-      e = __ldg(ev1 + (size_t)atom * kMTot + lane);
-      ge2 = __ldg(gev2 + (size_t)atom * kMTot + lane);
-      gt = __ldg(gate + (size_t)atom * 4 + deg);
+      e = ev1[(size_t)atom * kMTot + lane];
+      ge2 = gev2[(size_t)atom * kMTot + lane];
+      gt = gate[(size_t)atom * 4 + deg];
     }
   }
   if (proj) {
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
 }
 
 template <int AT>
-__global__ void __launch_bounds__(NTHR, 1) heads_fwd_small_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* __restrict__ x,
+__global__ void __launch_bounds__(NTHR, 1) heads_fwd_small_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* x,
                                                                   float* __restrict__ ze, float* __restrict__ zq, float* __restrict__ zh,
                                                                   float* __restrict__ e_nn, float* __restrict__ q_raw, float* __restrict__ hv) {
   extern __shared__ __align__(16) float sm[];
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_small_kernel(ModelDev M, in
   float w[32];
   load_w128(w, M.e_reg_k);
   grid_dep_sync();
-  if (warp < AT) st4(act + warp * kF + col, own ? ldg4(x + (size_t)atom * kF + col) : zero4());
+  if (warp < AT) st4(act + warp * kF + col, own ? ld4(x + (size_t)atom * kF + col) : zero4());
   const int z = own ? Z[atom] : 0;
   const int z_e = z < 0 ? 0 : (z >= kZEmbed ? kZEmbed - 1 : z), z_h = z < 0 ? 0 : (z >= kZHead ? kZHead - 1 : z);
   __syncthreads();
@@ -365,10 +366,10 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_small_kernel(ModelDev M, in
 }
 
 template <int AT>
-__global__ void __launch_bounds__(NTHR, 1) heads_bwd_small_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* __restrict__ ze,
-                                                                  const float* __restrict__ zq, const float* __restrict__ zh,
-                                                                  const float* __restrict__ hv, const float* __restrict__ ge,
-                                                                  const float* __restrict__ gq, const float* __restrict__ gh, float* __restrict__ gx) {
+__global__ void __launch_bounds__(NTHR, 1) heads_bwd_small_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* ze,
+                                                                  const float* zq, const float* zh,
+                                                                  const float* hv, const float* ge,
+                                                                  const float* gq, const float* gh, float* __restrict__ gx) {
   extern __shared__ __align__(16) float sm[];
   float* act_e = sm;                      // [AT][128]
   float* act_q = act_e + AT * kF;         // [AT][128]
@@ -391,8 +392,8 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_small_kernel(ModelDev M, in
       const float ce = ge[atom] * M.e_scale[z_e], cq = gq[atom], ch = gh[atom] * (hv[atom] < 0.f ? -0.125f : 0.125f);
       k0 = ch * M.h_embed1[z_h * 64 + lane]; k1 = ch * M.h_embed1[z_h * 64 + 32 + lane];
       dh0 = dsilu_f(zh[(size_t)atom * 64 + lane]); dh1 = dsilu_f(zh[(size_t)atom * 64 + 32 + lane]);
-      ae = fma4(ce, mul4(ldg4(M.e_fin_k + col), dsilu4(ldg4(ze + (size_t)atom * kF + col))), ae);
-      aq = fma4(cq, mul4(ldg4(M.q_fin_k + col), dsilu4(ldg4(zq + (size_t)atom * kF + col))), aq);
+      ae = fma4(ce, mul4(ldg4(M.e_fin_k + col), dsilu4(ld4(ze + (size_t)atom * kF + col))), ae);
+      aq = fma4(cq, mul4(ldg4(M.q_fin_k + col), dsilu4(ld4(zq + (size_t)atom * kF + col))), aq);
     }
     st4(act_e + warp * kF + col, ae);
     st4(act_q + warp * kF + col, aq);

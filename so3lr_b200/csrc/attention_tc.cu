@@ -403,9 +403,9 @@ constexpr int kOrderedRows = 8192;      // from here on: 0.1 GB of q / k / v and
 enum CompactPass { kReserve, kCount, kFill };
 template <int PASS>
 __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_rows, int n, const int* __restrict__ row_ptr,
-                                                                         const int* __restrict__ nbr_j, const float* __restrict__ dR,
-                                                                         const int* __restrict__ partner, const int* __restrict__ asym,
-                                                                         int* __restrict__ total, int* __restrict__ blocks, int* __restrict__ ve_i,
+                                                                         const int* __restrict__ nbr_j, const float* dR,
+                                                                         const int* partner, const int* asym,
+                                                                         int* __restrict__ total, int* blocks, int* __restrict__ ve_i,
                                                                          int* __restrict__ ve_j, float4* __restrict__ ve_d, int2* __restrict__ ve_orig) {
   grid_dep_sync();
   __shared__ int start[kCompactRows + 1];
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_r
   }
 }
 // counts -> exclusive offsets, and their sum; one CTA (an eighth of a million atoms per 8 counts of a thread)
-__global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* __restrict__ blocks, int* __restrict__ total) {
+__global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* blocks, int* __restrict__ total) {
   grid_dep_sync();
   __shared__ int warp_sum_[32];
   const int tid = threadIdx.x, lane = tid & 31, per = (n + 1023) / 1024;
@@ -549,11 +549,11 @@ __device__ __forceinline__ void edge_loops(int share, Body&& body, int run = 8) 
 // its 8 edges in flight and 128 threads stage the next tile; (3) per filter: tensor memory -> shared tile, then the edge loop.
 __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsigned char* __restrict__ img_g, const float* __restrict__ sph1_k,
                                                                     const float* __restrict__ sph1_b, int n_recv,
-                                                                    const int* __restrict__ n_listed, const int* __restrict__ ve_i,
-                                                                    const int* __restrict__ ve_j, const float4* __restrict__ ve_d,
-                                                                    const float* __restrict__ qkv, const float* __restrict__ ev_in,
+                                                                    const int* n_listed, const int* ve_i,
+                                                                    const int* ve_j, const float4* ve_d,
+                                                                    const float* qkv, const float* ev_in,
                                                                     float* __restrict__ xa, float* __restrict__ ev1, int* __restrict__ err,
-                                                                    long long* __restrict__ dbg, const int* __restrict__ asym) {
+                                                                    long long* __restrict__ dbg, const int* asym) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* rec = reinterpret_cast<float*>(smem + kOffFwRec);
@@ -1168,14 +1168,14 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
 template <bool PER_ENTRY>
 __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsigned char* __restrict__ img_g, const float* __restrict__ sph1_k,
                                                                     const float* __restrict__ sph1_b, int n_recv,
-                                                                    const int* __restrict__ n_listed, const int* __restrict__ ve_i,
-                                                                    const int* __restrict__ ve_j, const float4* __restrict__ ve_d,
-                                                                    const float* __restrict__ qkv, const float* __restrict__ ev_in,
-                                                                    const float* __restrict__ g_xa, const float* __restrict__ gev1,
+                                                                    const int* n_listed, const int* ve_i,
+                                                                    const int* ve_j, const float4* ve_d,
+                                                                    const float* qkv, const float* ev_in,
+                                                                    const float* g_xa, const float* gev1,
                                                                     float* __restrict__ g_qkv, float* __restrict__ gev_in,
-                                                                    float* __restrict__ F, float* __restrict__ virial,
+                                                                    float* F, float* __restrict__ virial,
                                                                     int* __restrict__ err, long long* __restrict__ dbg,
-                                                                    const int2* __restrict__ ve_orig, const int* __restrict__ gate,
+                                                                    const int2* ve_orig, const int* gate,
                                                                     int n_own) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

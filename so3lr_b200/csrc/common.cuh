@@ -75,6 +75,11 @@ SO3LR_D float dsilu_f(float x) {
 // First statement of every kernel that launch_chained starts: lets the next kernel of the stream take its place on the chip early,
 // and waits until everything before this one has completed.  What a kernel does ahead of the call may only touch its own
 // shared memory and the model's constant weights.
+// The kernel's lifetime begins while the kernels before it still write what it reads.  So a pointer parameter to an array that any
+// other kernel writes carries no __restrict__ where this one reads it: the qualifier promises that nobody else changes the array
+// while the kernel runs, which lets the compiler take the non-coherent path, or move a load above the wait (whose "memory"
+// clobber holds back only loads of memory that somebody else may change).  __ldg is for weights.  Write-only outputs, lists and other
+// arrays that are complete before the first chained kernel starts may keep the qualifier; device functions called after the wait too.
 SO3LR_D void grid_dep_sync() {
 #ifdef __CUDA_ARCH__
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -324,7 +324,7 @@ struct Tile {
 #pragma unroll
     for (int i = 0; i < RPW; ++i) {
       const int a = row0 + warp + (NTHR / 32) * i;
-      v[i] = a < n ? __ldg(reinterpret_cast<const float4*>(src + (size_t)a * ld) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[i] = a < n ? ld4(src + (size_t)a * ld + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   __device__ __forceinline__ void put_rows(const float4 (&v)[RPW]) {
@@ -344,7 +344,7 @@ struct Tile {
 //   x3 = x2 + yx; ev2 = ev1 * (1 + gate_l); x4 = LN2(x3); q/k/v rows of the next layer from x4
 // saves z1 (hidden pre-activation), x3 and gate for the reverse pass
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, int n, const float* __restrict__ xa, const float* __restrict__ ev1,
+__global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, int n, const float* xa, const float* ev1,
                                                                    float* __restrict__ z1_out, float* __restrict__ x3_out,
                                                                    float* __restrict__ gate_out, float* __restrict__ x4_out,
                                                                    float* __restrict__ ev2_out, const unsigned char* __restrict__ proj_u,
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
       if (a < n) {
 #pragma unroll
         for (int m4 = 0; m4 < kMTot / 4; ++m4) {
-          const float4 e = __ldg(reinterpret_cast<const float4*>(ev1 + (size_t)a * kMTot) + m4);
+          const float4 e = ld4(ev1 + (size_t)a * kMTot + 4 * m4);
           s[degree_of(4 * m4)] += e.x * e.x; s[degree_of(4 * m4 + 1)] += e.y * e.y;
           s[degree_of(4 * m4 + 2)] += e.z * e.z; s[degree_of(4 * m4 + 3)] += e.w * e.w;
         }
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
         st4(gate_out + (size_t)a * 4, make_float4(g[0], g[1], g[2], g[3]));
 #pragma unroll
         for (int m4 = 0; m4 < kMTot / 4; ++m4) {
-          float4 e = __ldg(reinterpret_cast<const float4*>(ev1 + (size_t)a * kMTot) + m4);
+          float4 e = ld4(ev1 + (size_t)a * kMTot + 4 * m4);
           e.x *= 1.f + g[degree_of(4 * m4)]; e.y *= 1.f + g[degree_of(4 * m4 + 1)];
           e.z *= 1.f + g[degree_of(4 * m4 + 2)]; e.w *= 1.f + g[degree_of(4 * m4 + 3)];
           st4(ev2_out + (size_t)a * kMTot + 4 * m4, e);
@@ -618,7 +618,7 @@ __device__ __forceinline__ void ldg8(const float* __restrict__ p, float* v) {
   const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
-// the same through the coherent path: for rows this kernel overwrites later on
+// the same through the coherent path: for everything that is no weight (see grid_dep_sync)
 __device__ __forceinline__ void ld8(const float* p, float* v) {
   const float4 a = *reinterpret_cast<const float4*>(p), b = *(reinterpret_cast<const float4*>(p) + 1);
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
@@ -637,11 +637,11 @@ __device__ __forceinline__ int degree_start(int l) { return l == 0 ? 0 : (l == 1
 // post-attention block, reverse.  in: g4 = dL/dx4 (or, with projT_u: the rows of g_xa left by the layer above + the transposed
 // q/k/v projections of that layer's g_qkv), gev2 = dL/dev2; out: g_xa = dL/dxa, gev1 = dL/dev1
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, int n, const float* __restrict__ xa, const float* __restrict__ ev1,
-                                                                   const float* __restrict__ z1, const float* __restrict__ x3,
-                                                                   const float* __restrict__ gate, const float* __restrict__ g4,
-                                                                   const float* __restrict__ gev2, float* g_xa, float* __restrict__ gev1,
-                                                                   const unsigned char* __restrict__ projT_u, const float* __restrict__ g_qkv_up,
+__global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, int n, const float* xa, const float* ev1,
+                                                                   const float* z1, const float* x3,
+                                                                   const float* gate, const float* g4,
+                                                                   const float* gev2, float* g_xa, float* __restrict__ gev1,
+                                                                   const unsigned char* __restrict__ projT_u, const float* g_qkv_up,
                                                                    int* err, float* __restrict__ gev1_copy) {
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
       auto fetch_slab = [&](int w) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          if (aw < n) ldg8(g_qkv_up + (size_t)aw * kProj + w * kF + 8 * (4 * i + ch), sl[i]);
+          if (aw < n) ld8(g_qkv_up + (size_t)aw * kProj + w * kF + 8 * (4 * i + ch), sl[i]);
           else {
 #pragma unroll
             for (int k = 0; k < 8; ++k) sl[i][k] = 0.f;
@@ -729,9 +729,8 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
       for (int i = 0; i < 4; ++i) {
         const int c = 8 * (4 * i + ch);
         if (aw < n) {
-          ldg8(x3 + (size_t)aw * kF + c, xh[i]);
-          if (projT_u) ld8(g_xa + (size_t)aw * kF + c, gy[i]);
-          else ldg8(g4 + (size_t)aw * kF + c, gy[i]);
+          ld8(x3 + (size_t)aw * kF + c, xh[i]);
+          ld8((projT_u ? g_xa : g4) + (size_t)aw * kF + c, gy[i]);
         } else {
 #pragma unroll
           for (int k = 0; k < 8; ++k) { xh[i][k] = 0.f; gy[i][k] = 0.f; }
@@ -742,10 +741,10 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
 #pragma unroll
       for (int m = 0; m < 9; ++m) {
         const bool on = aw < n && m < nm;
-        e2[m] = on ? __ldg(gev2 + (size_t)aw * kMTot + m0 + m) : 0.f;
-        e1[m] = on ? __ldg(ev1 + (size_t)aw * kMTot + m0 + m) : 0.f;
+        e2[m] = on ? gev2[(size_t)aw * kMTot + m0 + m] : 0.f;
+        e1[m] = on ? ev1[(size_t)aw * kMTot + m0 + m] : 0.f;
       }
-      const float gate_l = aw < n ? __ldg(gate + (size_t)aw * 4 + ch) : 0.f;
+      const float gate_l = aw < n ? gate[(size_t)aw * 4 + ch] : 0.f;
       DN_MARK(48);
       float s = 0.f;
 #pragma unroll
@@ -886,7 +885,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
       float s = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        if (aw < n) ldg8(xa + (size_t)aw * kF + 8 * (4 * i + ch), x[i]);
+        if (aw < n) ld8(xa + (size_t)aw * kF + 8 * (4 * i + ch), x[i]);
         else {
 #pragma unroll
           for (int k = 0; k < 8; ++k) x[i][k] = 0.f;
@@ -961,7 +960,7 @@ __device__ __forceinline__ void load_rows64(Tile& T, const float* __restrict__ s
 #pragma unroll
   for (int i = 0; i < TM / (2 * (NTHR / 32)); ++i) {
     const int rr = 2 * (T.warp + (NTHR / 32) * i) + sub, a = row0 + rr;
-    const float4 v = a < n ? __ldg(reinterpret_cast<const float4*>(src + (size_t)a * 64 + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 v = a < n ? ld4(src + (size_t)a * 64 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     st4(T.S + rr * SS + c, v);
   }
 }
@@ -980,7 +979,7 @@ __device__ __forceinline__ void flush_rows64(Tile& T, float* __restrict__ dst, i
 //   hv = embed0[Z] + ((silu(x W_h1 + b_h1) W_h2 + b_h2) . embed1[Z]) / 8
 // saves the pre-activations ze, zq, zh for the reverse pass
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* __restrict__ x,
+__global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* x,
                                                                float* __restrict__ ze, float* __restrict__ zq, float* __restrict__ zh,
                                                                float* __restrict__ e_nn, float* __restrict__ q_raw, float* __restrict__ hv,
                                                                int* err) {
@@ -1002,7 +1001,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float v[8];
-        if (aw < n) ldg8(x + (size_t)aw * kF + 8 * (4 * i + ch), v);
+        if (aw < n) ld8(x + (size_t)aw * kF + 8 * (4 * i + ch), v);
         else {
 #pragma unroll
           for (int k = 0; k < 8; ++k) v[k] = 0.f;
@@ -1129,10 +1128,10 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n
 // ------------------------------------------------------------------------------------------------
 // output heads, reverse: gx = dL/dx_final from the cotangents of e_nn (ge), of the raw charge (gq) and of the Hirshfeld ratio (gh)
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* __restrict__ ze,
-                                                               const float* __restrict__ zq, const float* __restrict__ zh,
-                                                               const float* __restrict__ hv, const float* __restrict__ ge,
-                                                               const float* __restrict__ gq, const float* __restrict__ gh,
+__global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n, const int* __restrict__ Z, const float* ze,
+                                                               const float* zq, const float* zh,
+                                                               const float* hv, const float* ge,
+                                                               const float* gq, const float* gh,
                                                                float* __restrict__ gx, int* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   Tile T;
@@ -1203,7 +1202,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n
     for (int i = 0; i < 4; ++i) {
       const int c = 8 * (4 * i + ch);
       float v[8], f[8];
-      if (aw < n) ldg8(ze + (size_t)aw * kF + c, v);
+      if (aw < n) ld8(ze + (size_t)aw * kF + c, v);
       else {
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = 0.f;
@@ -1220,7 +1219,7 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n
     for (int i = 0; i < 4; ++i) {
       const int c = 8 * (4 * i + ch);
       float v[8], f[8];
-      if (aw < n) ldg8(zq + (size_t)aw * kF + c, v);
+      if (aw < n) ld8(zq + (size_t)aw * kF + c, v);
       else {
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = 0.f;

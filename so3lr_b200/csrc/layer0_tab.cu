@@ -87,7 +87,7 @@ __global__ void build_pair_table_kernel(const float* __restrict__ radial, const 
 
 __global__ void __launch_bounds__(256) layer0_fwd_tab_kernel(SpeciesTables T, const float* __restrict__ embed, int n_recv, int n,
                                                              const int* __restrict__ row_ptr, const int* __restrict__ nbr_j,
-                                                             const float* __restrict__ dR, const int* __restrict__ Z,
+                                                             const float* dR, const int* __restrict__ Z,
                                                              float* __restrict__ xa, float* __restrict__ ev1) {
   grid_dep_sync();
   const int lane = threadIdx.x & 31;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) layer0_fwd_tab_kernel(SpeciesTables T, co
 }
 
 // GV[a][z][h] = sum_{t in head h} g_xa[a][t] * v_z[t]
-__global__ void __launch_bounds__(256) layer0_gv_kernel(SpeciesTables T, int n, const float* __restrict__ g_xa, float* __restrict__ GV) {
+__global__ void __launch_bounds__(256) layer0_gv_kernel(SpeciesTables T, int n, const float* g_xa, float* __restrict__ GV) {
   grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int a = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -277,10 +277,10 @@ __global__ void __launch_bounds__(256) layer0_bwd_tab_kernel(SpeciesTables T, in
 // has one (the full list's rows hold the skin too and leave 45 % of the lanes without work, and every pair was evaluated at both ends).
 // Equal receivers inside a warp are summed before they go out; the partner gets its share if it owns a row.  Rows of `virial` below
 // n_own add up to the total, in any distribution: every warp adds its sum to one of them.
-__global__ void __launch_bounds__(128) layer0_bwd_pairs_kernel(SpeciesTables T, int n_recv, const int* __restrict__ n_listed,
-                                                               const int* __restrict__ ve_i, const int* __restrict__ ve_j,
-                                                               const float4* __restrict__ ve_d, const int* __restrict__ Z,
-                                                               const float* __restrict__ GV, const float* __restrict__ gev1,
+__global__ void __launch_bounds__(128) layer0_bwd_pairs_kernel(SpeciesTables T, int n_recv, const int* n_listed,
+                                                               const int* ve_i, const int* ve_j,
+                                                               const float4* ve_d, const int* __restrict__ Z,
+                                                               const float* GV, const float* gev1,
                                                                float* __restrict__ F, float* __restrict__ virial, int n_own) {
   grid_dep_sync();
   const int lane = threadIdx.x & 31;

@@ -52,9 +52,9 @@ __global__ void __launch_bounds__(256) ke_partial_kernel(int n, const float* __r
 }
 
 // first half of velocity Verlet, after the thermostat's momentum scaling that is waiting in chain[1]
-__global__ void __launch_bounds__(256) vv_first_scaled_kernel(int n, float dt, const float* __restrict__ m, float* __restrict__ R,
-                                                              float* __restrict__ V, const float* __restrict__ F,
-                                                              const double* __restrict__ chain) {
+__global__ void __launch_bounds__(256) vv_first_scaled_kernel(int n, float dt, const float* m, float* R,
+                                                              float* V, const float* F,
+                                                              const double* chain) {
   grid_dep_sync();
   int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
@@ -68,8 +68,8 @@ __global__ void __launch_bounds__(256) vv_first_scaled_kernel(int n, float dt, c
 }
 
 // second half of velocity Verlet; also leaves each block's share of the new kinetic energy (eV)
-__global__ void __launch_bounds__(256) vv_second_ke_kernel(int n, float dt, const float* __restrict__ m, float* __restrict__ V,
-                                                           const float* __restrict__ F, double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) vv_second_ke_kernel(int n, float dt, const float* m, float* V,
+                                                           const float* F, double* __restrict__ partials) {
   grid_dep_sync();
   __shared__ double sh[256];
   int i = blockIdx.x * 256 + threadIdx.x;
@@ -177,7 +177,7 @@ __device__ double sum_partials_256(const double* __restrict__ partials, int n_pa
 // momentum scale of those half steps is multiplied into chain[1] for the next velocity kernel to apply.
 __global__ void __launch_bounds__(256) nhc_half_steps_kernel(double* chain, int L, int chain_steps, int sy_steps, double dt, double tau,
                                                              double kT, double dof, int n_half, int fresh_scale,
-                                                             const double* __restrict__ partials, int n_partials) {
+                                                             const double* partials, int n_partials) {
   grid_dep_sync();
   __shared__ double sh[256];
   if (partials) {

@@ -7,9 +7,9 @@ namespace so3lr {
 namespace {
 
 __global__ void sr_geometry_zbl_kernel(ZblParams zbl, Cell cell, int n, long long n_edges, const int* __restrict__ edge_i,
-                                       const int* __restrict__ nbr_j, const int* __restrict__ Z, const float* __restrict__ R,
-                                       int dR_given, float* __restrict__ dR, float* __restrict__ e_atom,
-                                       float* __restrict__ g_dR, const float* __restrict__ ge, float* __restrict__ F_direct, int n_owned,
+                                       const int* __restrict__ nbr_j, const int* __restrict__ Z, const float* R,
+                                       int dR_given, float* dR, float* __restrict__ e_atom,
+                                       float* g_dR, const float* ge, float* __restrict__ F_direct, int n_owned,
                                        float* __restrict__ virial) {
   grid_dep_sync();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -223,9 +223,9 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
 // The single-device long-range kernel with packed operands: per atom (x, y, z, q) and (h, alpha_free, c6_free, -) so that a pair costs two
 // 16-byte gathers, and a packed accumulator (Fx, Fy, Fz, dE/dq) so that the sender's share of a pair is one
 // vector reduction (red.global.add.v4.f32) and one scalar one (dE/dh) instead of five scalar atomics.
-__global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* __restrict__ R, const float* __restrict__ q,
-                                                        const float* __restrict__ h, const int* __restrict__ Z,
-                                                        float4* __restrict__ pq, float4* __restrict__ hz, float4* __restrict__ acc) {
+__global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* R, const float* q,
+                                                        const float* h, const int* __restrict__ Z,
+                                                        float4* __restrict__ pq, float4* __restrict__ hz, float4* acc) {
   grid_dep_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -234,9 +234,9 @@ __global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* __re
   acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 // with e_atom also the per-atom energies: the sum of the network's, the repulsion's and the two pair terms' shares
-__global__ void __launch_bounds__(256) pair_unpack_kernel(int n, const float4* __restrict__ acc, float* __restrict__ F, float* __restrict__ gq,
-                                                          const float* __restrict__ e_nn, const float* __restrict__ e_zbl,
-                                                          const float* __restrict__ e_coul, const float* __restrict__ e_disp, float* __restrict__ e_atom) {
+__global__ void __launch_bounds__(256) pair_unpack_kernel(int n, const float4* acc, float* F, float* gq,
+                                                          const float* e_nn, const float* e_zbl,
+                                                          const float* e_coul, const float* e_disp, float* __restrict__ e_atom) {
   grid_dep_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -249,10 +249,10 @@ __device__ __forceinline__ void red_add_f4(float4* p, float x, float y, float z,
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell cell, int n, const int* __restrict__ row_ptr,
-                                                             const int* __restrict__ nbr_j, const float4* __restrict__ pq,
-                                                             const float4* __restrict__ hz, float4* __restrict__ acc,
-                                                             float* __restrict__ gh, float* __restrict__ e_coul,
-                                                             float* __restrict__ e_disp, float* __restrict__ virial) {
+                                                             const int* __restrict__ nbr_j, const float4* pq,
+                                                             const float4* hz, float4* __restrict__ acc,
+                                                             float* __restrict__ gh, float* e_coul,
+                                                             float* e_disp, float* __restrict__ virial) {
   grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -268,12 +268,12 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
   for (int e = e0 + lane; e < e1; e += 32) {
     const int j = nbr_j[e];
     if (j < 0 || j >= n) continue;
-    const float4 pj = __ldg(pq + j);
+    const float4 pj = pq[j];
     float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
     min_image(cell, dx, dy, dz);
     const float r2 = dx * dx + dy * dy + dz * dz;
     if (!(r2 > 0.f) || (P.has_cutoff && r2 >= rc2)) continue;
-    const float4 hzj = __ldg(hz + j);
+    const float4 hzj = hz[j];
     const float rinv = rsqrtf(r2), r = r2 * rinv;
     float chi, dchi;
     coulomb_chi_dev(P, r, rinv, chi, dchi);
@@ -363,8 +363,8 @@ __global__ void __launch_bounds__(256) pair_lr_owned_kernel(LrParams P, Cell cel
 }
 
 // one CTA per graph: q = q_raw + (Q - sum q_raw) / n_g ; h = |hv|
-__global__ void charge_conserve_kernel(int n_graphs, const int* __restrict__ graph_start, const float* __restrict__ q_raw,
-                                       const float* __restrict__ total_charge, const float* __restrict__ hv,
+__global__ void charge_conserve_kernel(int n_graphs, const int* __restrict__ graph_start, const float* q_raw,
+                                       const float* __restrict__ total_charge, const float* hv,
                                        float* __restrict__ q, float* __restrict__ h) {
   grid_dep_sync();
   __shared__ float red[32];
@@ -391,7 +391,7 @@ __global__ void charge_conserve_kernel(int n_graphs, const int* __restrict__ gra
 }
 
 // gq_raw = gq - mean_graph(gq)
-__global__ void charge_conserve_bwd_kernel(int n_graphs, const int* __restrict__ graph_start, const float* __restrict__ gq,
+__global__ void charge_conserve_bwd_kernel(int n_graphs, const int* __restrict__ graph_start, const float* gq,
                                            float* __restrict__ gq_raw) {
   grid_dep_sync();
   __shared__ float red[32];
@@ -413,8 +413,8 @@ __global__ void charge_conserve_bwd_kernel(int n_graphs, const int* __restrict__
 }
 
 // per-graph energy (double accumulation) and dipole sum_i q_i R_i; one CTA per graph
-__global__ void graph_reduce_kernel(int n_graphs, const int* __restrict__ graph_start, const float* __restrict__ e_atom,
-                                    const float* __restrict__ q, const float* __restrict__ R, double* __restrict__ e_graph,
+__global__ void graph_reduce_kernel(int n_graphs, const int* __restrict__ graph_start, const float* e_atom,
+                                    const float* q, const float* R, double* __restrict__ e_graph,
                                     float* __restrict__ dipole) {
   grid_dep_sync();
   __shared__ double red[4][32];
@@ -458,8 +458,8 @@ __device__ double block_sum_double_256(double v, double* sh) {
 }
 
 // partials[b][0] = sum a ; with R: partials[b][1..3] = sum q R
-__global__ void __launch_bounds__(256) wide_partial_kernel(int n, const float* __restrict__ a, const float* __restrict__ q,
-                                                           const float* __restrict__ R, double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) wide_partial_kernel(int n, const float* a, const float* q,
+                                                           const float* R, double* __restrict__ partials) {
   grid_dep_sync();
   __shared__ double sh[8];
   double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -487,9 +487,9 @@ __device__ double wide_total(const double* __restrict__ partials, int n_blocks, 
   return total;
 }
 
-__global__ void __launch_bounds__(256) charge_conserve_wide_kernel(int n, const float* __restrict__ q_raw, const float* __restrict__ total_charge,
-                                                                   const float* __restrict__ hv, float* __restrict__ q, float* __restrict__ h,
-                                                                   const double* __restrict__ partials, int n_blocks) {
+__global__ void __launch_bounds__(256) charge_conserve_wide_kernel(int n, const float* q_raw, const float* __restrict__ total_charge,
+                                                                   const float* hv, float* __restrict__ q, float* __restrict__ h,
+                                                                   const double* partials, int n_blocks) {
   grid_dep_sync();
   __shared__ double sh[8];
   const float Q = total_charge ? total_charge[0] : 0.f;
@@ -501,15 +501,15 @@ __global__ void __launch_bounds__(256) charge_conserve_wide_kernel(int n, const 
   }
 }
 
-__global__ void __launch_bounds__(256) charge_conserve_bwd_wide_kernel(int n, const float* __restrict__ gq, float* __restrict__ gq_raw,
-                                                                       const double* __restrict__ partials, int n_blocks) {
+__global__ void __launch_bounds__(256) charge_conserve_bwd_wide_kernel(int n, const float* gq, float* __restrict__ gq_raw,
+                                                                       const double* partials, int n_blocks) {
   grid_dep_sync();
   __shared__ double sh[8];
   const float mean = (float)wide_total(partials, n_blocks, 0, sh) / (float)n;
   for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) gq_raw[i] = gq[i] - mean;
 }
 
-__global__ void __launch_bounds__(256) graph_reduce_wide_kernel(const double* __restrict__ partials, int n_blocks, int with_dipole,
+__global__ void __launch_bounds__(256) graph_reduce_wide_kernel(const double* partials, int n_blocks, int with_dipole,
                                                                 double* __restrict__ e_graph, float* __restrict__ dipole) {
   grid_dep_sync();
   __shared__ double sh[8];

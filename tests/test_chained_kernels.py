@@ -1,0 +1,43 @@
+"""The rule beside grid_dep_sync (csrc/common.cuh), checked in the sources: a kernel that launch_chained starts is alive while the kernels
+before it still write its inputs, so it must not promise the compiler that those inputs are constant (const __restrict__, __ldg)."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "so3lr_b200", "csrc")
+# the model's weights, and arrays that are complete before the first chained kernel of an evaluation starts
+CONSTANT = {"projT", "proj", "projT_u", "proj_u", "img_g", "sph1_k", "sph1_b", "embed", "row_ptr", "nbr_j", "edge_i", "Z", "perm", "graph_start",
+            "total_charge"}
+SOURCES = {os.path.basename(f): re.sub(r"//[^\n]*", "", open(f).read()) for f in sorted(glob.glob(os.path.join(CSRC, "*.cu")))}
+CHAINED = sorted({k for s in SOURCES.values() for k in re.findall(r"launch_chained\((\w+)", s)})
+KERNEL = re.compile(r"__global__ void (?:__launch_bounds__\([^)]*(?:\([^)]*\))?[^)]*\) )?(\w+)\(([^{]*?)\)\s*\{", re.S)
+
+
+def _kernels():
+    for name, s in SOURCES.items():
+        heads = list(KERNEL.finditer(s))
+        for m, nxt in zip(heads, heads[1:] + [None]):
+            if m.group(1) in CHAINED:
+                yield name, m.group(1), m.group(2), s[m.end():nxt.start() if nxt else len(s)]
+
+
+def test_every_chained_kernel_is_found():
+    assert len(CHAINED) > 25 and {k for _, k, _, _ in _kernels()} == set(CHAINED)
+
+
+@pytest.mark.parametrize("kernel", CHAINED)
+def test_inputs_of_chained_kernels_are_not_promised_constant(kernel):
+    for _, k, params, body in _kernels():
+        if k == kernel:
+            assert "grid_dep_sync();" in body
+            promised = set(re.findall(r"const [\w ]+\* __restrict__ (\w+)", params))
+            assert promised <= CONSTANT, promised - CONSTANT
+
+
+@pytest.mark.parametrize("source", sorted({f for f, *_ in _kernels()}))
+def test_non_coherent_loads_are_of_weights(source):
+    for arg in re.findall(r"\b(?:__ldg|ldg4|ldg8)\((?:reinterpret_cast<const float4\*>\()?([A-Za-z_][\w.]*)", SOURCES[source]):
+        # members of the weight records, the arguments of the loading helpers themselves, weights passed on under a name
+        assert arg.startswith(("L.", "M.")) or arg in {"const", "W", "p", "bias", "fin"}, arg
