@@ -126,3 +126,17 @@ def test_shuffled_lists_of_a_graph_on_either_side(where):
     got = energies(p, q, where)
     assert float((got[0] - ref[0]).abs().max()) <= 1e-5 * float(ref[0].abs().max())
     assert float((got[1] - ref[1][torch.tensor(p)]).abs().max()) <= 1e-4 and float((got[2] - ref[2][torch.tensor(q)]).abs().max()) <= 1e-5
+
+
+@pytest.mark.parametrize("order", ["columns", "every_second"])
+def test_strided_positions_are_read_as_what_they_show(order):
+    from so3lr_b200 import So3lr
+    Z, R, cell = _water()
+    inputs = _inputs(Z, R, cell)
+    Rt = torch.tensor(R, device="cuda")
+    strided = Rt.T.contiguous().T if order == "columns" else torch.stack([Rt, Rt + 7.0], -1)[..., 0]
+    assert not strided.is_contiguous()
+    fn = So3lr(lr_cutoff=6.0)
+    ref, got = fn({**inputs, "positions": Rt}), fn({**inputs, "positions": strided})
+    assert abs(float(got["energy"] - ref["energy"])) <= 2e-6 * abs(float(ref["energy"]))
+    assert float((got["forces"] - ref["forces"]).abs().max()) <= 5e-5
