@@ -16,13 +16,14 @@ featurizer does in JAX.
 """
 from __future__ import annotations
 
+import math
 from collections import namedtuple
 from typing import Optional
 
 import numpy as np
 import torch
 
-from .engine import Model, System, displacements, displacements_vjp, lists_unsorted
+from .engine import Model, System, _displacements, _displacements_vjp, lists_unsorted
 
 CUTOFF_SR = 4.5
 
@@ -323,15 +324,23 @@ def _min_image(dR, cell_t):
 
 
 def _check_cell(cell):
-    """Refuses what is no lattice: anything but a 3 x 3 matrix, or one whose volume is zero (the test of so3lr_b200_system_create).  The
-    displacement kernels divide by the determinant without a look at it.  A cell on the GPU is read back here."""
-    if tuple(cell.shape) != (3, 3):
-        raise ValueError(f"Invalid cell shape {tuple(cell.shape)}. Expected (3, 3).")
-    h = cell.detach().to("cpu", torch.float64).numpy()
-    with np.errstate(invalid="ignore"):
-        det = float((h[0] * np.cross(h[1], h[2])).sum())
-    if not (abs(det) > 1e-12 and np.isfinite(det)):
-        raise torch.linalg.LinAlgError(f"the cell is singular (volume {det}): {h.tolist()}")
+    """Refuses what is no lattice: anything but a 3 x 3 matrix (or three edges, or one), or one whose volume is zero (the test of
+    so3lr_b200_system_create).  The displacement kernels divide by the determinant without a look at it.  A cell on the GPU is read
+    back here."""
+    h = cell.tolist() if hasattr(cell, "tolist") else np.asarray(cell).tolist()
+    if not isinstance(h, list):
+        det = h * h * h
+    elif len(h) == 1 and not isinstance(h[0], list):
+        det = h[0] ** 3
+    elif len(h) == 3 and not isinstance(h[0], list):
+        det = h[0] * h[1] * h[2]
+    elif len(h) == 3 and isinstance(h[0], list) and len(h[0]) == 3 and not isinstance(h[0][0], list):
+        (a, b, c), (d, e, f), (g, k, l) = h
+        det = a * (e * l - f * k) - b * (d * l - f * g) + c * (d * k - e * g)
+    else:
+        raise ValueError(f"Invalid cell shape {np.shape(h)}. Expected (3, 3).")
+    if not (abs(det) > 1e-12 and math.isfinite(det)):
+        raise torch.linalg.LinAlgError(f"the cell is singular (volume {det}): {h}")
 
 
 class _PairDisplacements(torch.autograd.Function):
@@ -343,13 +352,13 @@ class _PairDisplacements(torch.autograd.Function):
         ctx.lists, ctx.like = ((idx_i, idx_j), (idx_i_lr, idx_j_lr)), (Rc.shape[0], Rc.dtype, Rc.device)
         ctx.set_materialize_grads(False)
         dt = Rc.dtype if wide else torch.float32
-        return tuple(displacements(Rc, cell_t, i, j, dt) for i, j in ctx.lists)
+        return tuple(_displacements(Rc, cell_t, i, j, dt) for i, j in ctx.lists)
 
     @staticmethod
     def backward(ctx, g, g_lr):
         n, dt, dev = ctx.like
         parts = [(i, j, gg.contiguous()) for (i, j), gg in zip(ctx.lists, (g, g_lr)) if gg is not None]
-        return (displacements_vjp(n, dt, dev, parts), None, None, None, None, None, None)
+        return (_displacements_vjp(n, dt, dev, parts), None, None, None, None, None, None)
 
 
 class _Transform(torch.autograd.Function):
@@ -401,8 +410,7 @@ def neighbor_list_featurizer(displacement_fn, species, fractional_coordinates=Tr
         neighbor, neighbor_lr = torch.as_tensor(neighbor, device=dev), torch.as_tensor(neighbor_lr, device=dev)
         # the kernels take dR = R_j - R_i; the energy does not depend on the sign convention.  JAX gathers clamp the padding index N
         if cell_t is not None and not cell_t.requires_grad:
-            b = torch.as_tensor(box).to(R.dtype)      # where the caller holds it: no wait for a box on the host
-            _check_cell(b if b.shape == (3, 3) else torch.diag(b.reshape(-1).expand(3)))
+            _check_cell(box)      # where the caller holds it: no wait for a box on the host
         if cell_t is not None and cell_t.requires_grad:      # the caller differentiates with respect to the box itself
             idx = [a.long().clamp(max=n - 1) for a in (*neighbor[:2], *neighbor_lr[:2])]
             dR, dR_lr = _min_image(Rc[idx[1]] - Rc[idx[0]], cell_t), _min_image(Rc[idx[3]] - Rc[idx[2]], cell_t)
@@ -483,8 +491,10 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
     pot = So3lrPotentialB200(lr_cutoff, dispersion_energy_cutoff_lr_damping, "sparse", np.float32, dev)
 
     def so3lr_fn(inputs):
-        R = torch.as_tensor(inputs["positions"], dtype=torch.float32, device=dev)
+        R = torch.as_tensor(inputs["positions"], dtype=torch.float32, device=dev).contiguous()
         n = R.shape[0]
+        if tuple(R.shape) != (n, 3):
+            raise ValueError(f"positions must be (n, 3), not {tuple(R.shape)}")
         Z = np.asarray(torch.as_tensor(inputs["atomic_numbers"]).cpu(), dtype=np.int32)
         bs = inputs.get("batch_segments")
         gm = inputs.get("graph_mask")
@@ -510,10 +520,12 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
                     raise NotImplementedError("one cell per batch is supported")
                 c = c[0]
             if bool(c.abs().sum() > 0):
+                if tuple(c.shape) != (3, 3):
+                    raise ValueError(f"Invalid cell shape {tuple(c.shape)}. Expected (3, 3).")
                 _check_cell(c)
                 cell_t = c
         ii, jj, il, jl = (torch.as_tensor(inputs[k]).to(dev, torch.int32).contiguous() for k in ("idx_i", "idx_j", "idx_i_lr", "idx_j_lr"))
-        if ii.shape != jj.shape or il.shape != jl.shape:
+        if ii.shape != jj.shape or il.shape != jl.shape or ii.ndim != 1 or il.ndim != 1:
             raise ValueError(f"index arrays of unequal length: {[a.numel() for a in (ii, jj, il, jl)]}")
         for which, unsorted in enumerate(lists_unsorted(ii, il)):
             if unsorted:
@@ -522,7 +534,7 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
                     ii, jj = ii[p], jj[p]
                 else:
                     il, jl = il[p], jl[p]
-        dR, dRl = displacements(R, cell_t, ii, jj), displacements(R, cell_t, il, jl)
+        dR, dRl = _displacements(R, cell_t, ii, jj), _displacements(R, cell_t, il, jl)
         nm = inputs.get("node_mask")
         node_mask = torch.ones(n, dtype=torch.bool, device=dev) if nm is None else torch.as_tensor(nm, device=dev).bool()
         # cotangent of the masked energy sum (base_calculator.py:91)
@@ -537,7 +549,7 @@ def make_so3lr(lr_cutoff=12.0, dispersion_energy_cutoff_lr_damping=2.0, calculat
         res = dict(energy=energy, dipole_vec=dip, hirshfeld_ratios=h, partial_charges=q)
         if calculate_forces:
             # dE/dd is zero for entries with an end outside the structure (padding): only real pairs contribute
-            F = displacements_vjp(n, torch.float32, dev, [(ii, jj, out["g_edges"]), (il, jl, out["g_edges_lr"])], sign=-1.0)
+            F = _displacements_vjp(n, torch.float32, dev, [(ii, jj, out["g_edges"]), (il, jl, out["g_edges_lr"])], sign=-1.0)
             res["forces"] = F
         return res
 

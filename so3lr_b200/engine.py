@@ -230,9 +230,9 @@ class System:
         ge = None if g_e_atom is None else t(g_e_atom, torch.float32)
         n = self.n
         # the kernels read one index pair and three components per entry, one cotangent per atom
-        for e, lists in ((edges, (idx_i, idx_j)), (edges_lr, (idx_i_lr, idx_j_lr))):
-            if e.numel() != 3 * e.shape[0] or any(a.numel() < e.shape[0] for a in lists):
-                raise ValueError(f"{tuple(e.shape)} displacements with {[a.numel() for a in lists]} indices")
+        for e, i, j in ((edges, idx_i, idx_j), (edges_lr, idx_i_lr, idx_j_lr)):
+            if e.numel() != 3 * e.shape[0] or i.numel() < e.shape[0] or j.numel() < e.shape[0]:
+                raise ValueError(f"{tuple(e.shape)} displacements with {i.numel()} and {j.numel()} indices")
         if ge is not None and ge.numel() != n:
             raise ValueError(f"{ge.numel()} cotangents for {n} atoms")
         out = dict(e_atom=torch.empty(n, device=dev), g_edges=torch.zeros_like(edges), g_edges_lr=torch.zeros_like(edges_lr),
@@ -311,15 +311,19 @@ def _check_indices(device, *arrays):
 
 def displacements(R, cell, idx_i, idx_j, dtype=torch.float32):
     """(E, 3) displacements R[j] - R[i] (minimum image under `cell`, 3 x 3 and regular, rows = lattice vectors) of int32 index arrays;
-    indices are clamped to the structure, so padding entries give zero, and negative ones count from its end.  R (n, 3) float32 or float64 on the GPU."""
+    indices are clamped to the structure, so padding entries give zero, and negative ones count from its end.  R (n, 3) float32 or
+    float64 on the GPU."""
     if R.device.type != "cuda" or R.dtype not in (torch.float32, torch.float64) or R.ndim != 2 or R.shape[1] != 3:
         raise ValueError(f"positions must be (n, 3) float32 or float64 on a GPU, not {tuple(R.shape)} {R.dtype} on {R.device}")
     if dtype != torch.float32 and dtype != R.dtype:
         raise ValueError(f"{dtype} displacements of {R.dtype} positions")
     if cell is not None and tuple(cell.shape) != (3, 3):
         raise ValueError(f"Invalid cell shape {tuple(cell.shape)}. Expected (3, 3).")
-    idx_i, idx_j = _check_indices(R.device, idx_i, idx_j)
-    R = R.contiguous()
+    return _displacements(R.contiguous(), cell, *_check_indices(R.device, idx_i, idx_j), dtype)
+
+
+def _displacements(R, cell, idx_i, idx_j, dtype=torch.float32):
+    """`displacements` of arguments that are known to be of the right form, R and the indices contiguous."""
     cell = None if cell is None else cell.to(R.device, R.dtype).contiguous()
     with torch.cuda.device(R.device):
         out = torch.empty(idx_i.numel(), 3, dtype=dtype, device=R.device)
@@ -331,17 +335,22 @@ def displacements(R, cell, idx_i, idx_j, dtype=torch.float32):
 
 def displacements_vjp(n, dtype, device, parts, sign=1.0):
     """sum over the lists (idx_i, idx_j, g) in `parts` of the transpose of `displacements`: out[j] += sign g, out[i] -= sign g."""
+    checked = []
+    for i, j, g in parts:
+        i, j = _check_indices(g.device, i, j)
+        if tuple(g.shape) != (i.numel(), 3) or g.device != torch.empty(0, device=device).device or g.dtype not in (torch.float32, dtype):
+            raise ValueError(f"cotangents {tuple(g.shape)} {g.dtype} on {g.device} of {i.numel()} displacements")
+        checked.append((i, j, g.contiguous()))
+    return _displacements_vjp(n, dtype, device, checked, sign)
+
+
+def _displacements_vjp(n, dtype, device, parts, sign=1.0):
     with torch.cuda.device(device):
         out = torch.empty(n, 3, dtype=dtype, device=device)
         acc = torch.empty(n, 4, dtype=dtype, device=device)
         s = torch.cuda.current_stream(device)
         parts = parts or [(None, None, None)]
         for k, (i, j, g) in enumerate(parts):
-            if g is not None:
-                i, j = _check_indices(out.device, i, j)
-                if tuple(g.shape) != (i.numel(), 3) or g.device != out.device or g.dtype not in (torch.float32, dtype):
-                    raise ValueError(f"cotangents {tuple(g.shape)} {g.dtype} on {g.device} of {i.numel()} displacements")
-                g = g.contiguous()
             check(lib.so3lr_b200_displacements_vjp(C.c_void_p(s.cuda_stream), int(dtype == torch.float64), n, 0 if i is None else i.numel(),
                                                    _ptr(i), _ptr(j), _ptr(g), int(g is not None and g.dtype == torch.float64), float(sign),
                                                    _ptr(acc), int(k == 0), _ptr(out) if k == len(parts) - 1 else None), "displacements_vjp")
@@ -350,9 +359,11 @@ def displacements_vjp(n, dtype, device, parts, sign=1.0):
 
 def lists_unsorted(idx_i, idx_i_lr):
     """Two host booleans: whether each index array (int32, on the GPU) is NOT ascending.  Waits for the device."""
+    if idx_i.dtype != torch.int32 or idx_i_lr.dtype != torch.int32 or not idx_i.is_cuda or idx_i.device != idx_i_lr.device:
+        raise ValueError("index arrays must be int32 on one GPU")
     with torch.cuda.device(idx_i.device):
         flags = torch.empty(2, dtype=torch.int32, device=idx_i.device)
-        (idx_i,), (idx_i_lr,) = _check_indices(idx_i.device, idx_i), _check_indices(idx_i.device, idx_i_lr)
+        idx_i, idx_i_lr = idx_i.contiguous(), idx_i_lr.contiguous()
         s = torch.cuda.current_stream(idx_i.device)
         check(lib.so3lr_b200_lists_unsorted(C.c_void_p(s.cuda_stream), idx_i.numel(), _ptr(idx_i), idx_i_lr.numel(), _ptr(idx_i_lr),
                                             _ptr(flags)), "lists_unsorted")

@@ -19,8 +19,20 @@ def test_regular_cells_pass(cell, ok, dtype):
             _check_cell(t)
 
 
-@pytest.mark.parametrize("shape", [(3,), (9,), (1, 3, 3), (2, 3), (4, 4)])
+@pytest.mark.parametrize("shape", [(9,), (2,), (1, 3, 3), (2, 3), (3, 2), (4, 4)])
 def test_other_shapes_do_not(shape):
     from so3lr_b200.api import _check_cell
     with pytest.raises(ValueError):
         _check_cell(torch.ones(shape))
+
+
+@pytest.mark.parametrize("edges,ok", [(12.0, True), ([12.0], True), ([12.0, 13.0, 14.0], True), ((9, 9, 9), True), (0.0, False), ([0.0], False),
+                                      ([10.0, 10.0, 0.0], False), ([10.0, float("nan"), 10.0], False)])
+@pytest.mark.parametrize("make", [lambda e: e, np.asarray, torch.as_tensor])
+def test_boxes_given_by_their_edges(edges, ok, make):
+    from so3lr_b200.api import _check_cell
+    if ok:
+        _check_cell(make(edges))
+    else:
+        with pytest.raises(torch.linalg.LinAlgError):
+            _check_cell(make(edges))
