@@ -22,6 +22,7 @@ from typing import Optional
 
 import numpy as np
 import torch
+import torch.autograd.forward_ad
 
 from .engine import Model, System, _displacements, _displacements_vjp, lists_unsorted
 
@@ -343,22 +344,65 @@ def _check_cell(cell):
         raise torch.linalg.LinAlgError(f"the cell is singular (volume {det}): {h}")
 
 
+def _pair_displacements(Rc, cell_t, idx_i, idx_j, idx_i_lr, idx_j_lr):
+    """What _PairDisplacements computes, in torch operations: JAX gathers clamp the padding index n."""
+    idx = [a.long().clamp(max=Rc.shape[0] - 1) for a in (idx_i, idx_j, idx_i_lr, idx_j_lr)]
+    return _min_image(Rc[idx[1]] - Rc[idx[0]], cell_t), _min_image(Rc[idx[3]] - Rc[idx[2]], cell_t)
+
+
 class _PairDisplacements(torch.autograd.Function):
     """(d, d_lr) of both lists from Cartesian positions, minimum image under `cell_t`; `wide` keeps the dtype of the positions,
-    else the displacements come out in float32.  One kernel per list and direction (csrc/displacements.cu)."""
+    else the displacements come out in float32.  One kernel per list and direction (csrc/displacements.cu).  Linear in the positions
+    (the image is constant), so every derivative is this map without a cell or its transpose.  (setup_context and a vmap rule, which the
+    transforms of torch.func ask for, cost 80 us a call: under those the caller takes _pair_displacements.)"""
 
     @staticmethod
-    def forward(ctx, Rc, cell_t, wide, idx_i, idx_j, idx_i_lr, idx_j_lr):
-        ctx.lists, ctx.like = ((idx_i, idx_j), (idx_i_lr, idx_j_lr)), (Rc.shape[0], Rc.dtype, Rc.device)
+    def forward(ctx, Rc, cell_t, wide, *lists):
+        ctx.wide, ctx.like = wide, (Rc.shape[0], Rc.dtype)
+        ctx.save_for_backward(*lists)
+        ctx.save_for_forward(*lists)
         ctx.set_materialize_grads(False)
-        dt = Rc.dtype if wide else torch.float32
-        return tuple(_displacements(Rc, cell_t, i, j, dt) for i, j in ctx.lists)
+        R, dt = Rc.contiguous(), Rc.dtype if wide else torch.float32
+        return _displacements(R, cell_t, *lists[:2], dt), _displacements(R, cell_t, *lists[2:], dt)
 
     @staticmethod
     def backward(ctx, g, g_lr):
-        n, dt, dev = ctx.like
-        parts = [(i, j, gg.contiguous()) for (i, j), gg in zip(ctx.lists, (g, g_lr)) if gg is not None]
-        return (_displacements_vjp(n, dt, dev, parts), None, None, None, None, None, None)
+        if g is None and g_lr is None:
+            return None, None, None, None, None, None, None
+        if torch.is_grad_enabled():      # create_graph
+            return _PairTranspose.apply(g, g_lr, *ctx.like, *ctx.saved_tensors), None, None, None, None, None, None
+        return _transpose(g, g_lr, *ctx.like, ctx.saved_tensors), None, None, None, None, None, None
+
+    @staticmethod
+    def jvp(ctx, tR, *_):
+        return (None, None) if tR is None else _PairDisplacements.apply(tR, None, ctx.wide, *ctx.saved_tensors)
+
+
+def _transpose(g, g_lr, n, dtype, lists):
+    parts = [(*ij, gg.contiguous()) for ij, gg in ((lists[:2], g), (lists[2:], g_lr)) if gg is not None]
+    return _displacements_vjp(n, dtype, lists[0].device, parts)
+
+
+class _PairTranspose(torch.autograd.Function):
+    """Transpose of _PairDisplacements: cotangents of the displacements of both lists (either may be None) to one of the positions."""
+
+    @staticmethod
+    def forward(ctx, g, g_lr, n, dtype, *lists):
+        ctx.n, ctx.dtype, ctx.given = n, dtype, (g is not None, g_lr is not None)
+        ctx.wide = (g_lr if g is None else g).dtype == dtype
+        ctx.save_for_backward(*lists)
+        ctx.save_for_forward(*lists)
+        ctx.set_materialize_grads(False)
+        return _transpose(g, g_lr, n, dtype, lists)
+
+    @staticmethod
+    def backward(ctx, gR):
+        d = (None, None) if gR is None else _PairDisplacements.apply(gR, None, ctx.wide, *ctx.saved_tensors)
+        return *(x if given else None for x, given in zip(d, ctx.given)), None, None, None, None, None, None
+
+    @staticmethod
+    def jvp(ctx, t, t_lr, *_):
+        return None if t is None and t_lr is None else _PairTranspose.apply(t, t_lr, ctx.n, ctx.dtype, *ctx.saved_tensors)
 
 
 class _Transform(torch.autograd.Function):
@@ -389,7 +433,6 @@ def neighbor_list_featurizer(displacement_fn, species, fractional_coordinates=Tr
         R = torch.as_tensor(R, device=dev) if not torch.is_tensor(R) else R.to(dev)
         if R.dtype not in (torch.float32, torch.float64):
             R = R.float()
-        n = R.shape[0]
         box = kwargs.get("box")
         cell_t = None
         if box is not None:
@@ -408,15 +451,17 @@ def neighbor_list_featurizer(displacement_fn, species, fractional_coordinates=Tr
             raise ValueError("k-space electrostatics needs `box`")
         Rc = _Transform.apply(R, cell_t) if (cell_t is not None and fractional_coordinates) else R
         neighbor, neighbor_lr = torch.as_tensor(neighbor, device=dev), torch.as_tensor(neighbor_lr, device=dev)
-        # the kernels take dR = R_j - R_i; the energy does not depend on the sign convention.  JAX gathers clamp the padding index N
-        if cell_t is not None and not cell_t.requires_grad:
-            _check_cell(box)      # where the caller holds it: no wait for a box on the host
-        if cell_t is not None and cell_t.requires_grad:      # the caller differentiates with respect to the box itself
-            idx = [a.long().clamp(max=n - 1) for a in (*neighbor[:2], *neighbor_lr[:2])]
-            dR, dR_lr = _min_image(Rc[idx[1]] - Rc[idx[0]], cell_t), _min_image(Rc[idx[3]] - Rc[idx[2]], cell_t)
+        # the kernels take dR = R_j - R_i; the energy does not depend on the sign convention
+        box_moves = cell_t is not None and (cell_t.requires_grad or torch.autograd.forward_ad.unpack_dual(cell_t).tangent is not None)
+        if box_moves or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
+            # the caller differentiates with respect to the box itself, or transforms or records torch operations, which a bare kernel
+            # call is not
+            dR, dR_lr = _pair_displacements(Rc, cell_t, *neighbor[:2], *neighbor_lr[:2])
         else:
+            if cell_t is not None:
+                _check_cell(box)      # where the caller holds it: no wait for a box on the host
             idx = [a.to(torch.int32).contiguous() for a in (*neighbor[:2], *neighbor_lr[:2])]
-            dR, dR_lr = _PairDisplacements.apply(Rc.contiguous(), cell_t, pert is not None, *idx)
+            dR, dR_lr = _PairDisplacements.apply(Rc, cell_t, pert is not None, *idx)
         positions = Rc if k_grid is not None else None
         if pert is not None:
             p = pert if torch.is_tensor(pert) else torch.as_tensor(pert)
