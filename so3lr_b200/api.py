@@ -78,13 +78,13 @@ class _GraphEnergy(torch.autograd.Function):
     def backward(ctx, g):
         edges, edges_lr, ge, gel, gp, gc = ctx.saved_tensors
         g = g.contiguous()
-        lo, hi = torch.stack(torch.aminmax(g)).tolist()
-        if lo == hi == 1.0:         # the plain sum, as under quantity.force: nothing to scale
-            return (ge, gel, None, None, None, None, None, None, gp if ctx.has_positions else None, gc if gc.numel() else None)
+        bounds = torch.stack(torch.aminmax(g))
+        lo, hi = bounds.tolist()
         if lo == hi:
-            c = lo
+            # copies, also where the factor is one: the caller may change what it gets and come back for more
+            c = bounds[0] if g.requires_grad else lo      # create_graph: the factor has no derivative, and asking for it raises
             return (ge * c, gel * c, None, None, None, None, None, None, (gp * c if ctx.has_positions else None),
-                    (gc * c if gc.numel() else None))
+                    ((gc * c).to(gc.dtype) if gc.numel() else None))
         if ctx.has_positions:
             raise NotImplementedError("the reciprocal-space energy is differentiated for a uniform cotangent (its sum) only")
         out = ctx.system.graph_eval(ctx.lists[0], ctx.lists[1], edges, ctx.lists[2], ctx.lists[3], edges_lr, g_e_atom=g)

@@ -140,3 +140,27 @@ def test_strided_positions_are_read_as_what_they_show(order):
     ref, got = fn({**inputs, "positions": Rt}), fn({**inputs, "positions": strided})
     assert abs(float(got["energy"] - ref["energy"])) <= 2e-6 * abs(float(ref["energy"]))
     assert float((got["forces"] - ref["forces"]).abs().max()) <= 5e-5
+
+
+def test_gradients_belong_to_the_caller():
+    """Gradients with respect to a graph's edges may be changed in place between two backward passes."""
+    from so3lr_b200 import Graph, So3lrPotential
+    Z, R, cell = _water()
+    inp = _inputs(Z, R, cell)
+    t = {k: torch.tensor(inp[k], device="cuda") for k in ("idx_i", "idx_j", "idx_i_lr", "idx_j_lr")}
+    c = cell.astype(np.float64)
+    mi = lambda d: torch.tensor(d - np.round(d @ np.linalg.inv(c)) @ c, dtype=torch.float32, device="cuda").requires_grad_(True)
+    d, dl = mi(R[inp["idx_j"]] - R[inp["idx_i"]].astype(np.float64)), mi(R[inp["idx_j_lr"]] - R[inp["idx_i_lr"]].astype(np.float64))
+    E = So3lrPotential(lr_cutoff=6.0)(Graph(None, d, torch.tensor(Z), t["idx_i"], t["idx_j"], None, None, None, dl, t["idx_i_lr"], t["idx_j_lr"], None)).sum()
+    first = torch.autograd.grad(E, (d, dl), retain_graph=True)
+    ref = [g.clone() for g in first]
+    for g in first:
+        g.mul_(-3.0)
+    again = torch.autograd.grad(E, (d, dl), retain_graph=True)
+    assert all(torch.equal(a, b) for a, b in zip(again, ref))
+    # a factor in front of the sum: the gradient's own dependence on it is not available, and that is said
+    w = torch.tensor(2.5, device="cuda", requires_grad=True)
+    g, = torch.autograd.grad(w * E, d, create_graph=True)
+    assert torch.allclose(g.detach(), 2.5 * ref[0])
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(g.sum(), w)
