@@ -557,21 +557,24 @@ void heads_bwd_dispatch(cudaStream_t s, const ModelDev& M, int n, const int* Z, 
   else if (use_mma_dense()) launch_heads_bwd_mma(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx);
   else launch_heads_bwd(s, M, n, Z, ze, zq, zh, hv, ge, gq, gh, gx);
 }
-void attn_fwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
+[[nodiscard]] int attn_fwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
                        const float* qkv, const float* x_in, const float* ev_in, float* xa, float* ev1, bool preset = false) {
-  if (L.has_spherical && attention_mode() >= kAttnTcFwd) launch_attn_fwd_tc(st, L, S->ve, n_recv, qkv, x_in, ev_in, xa, ev1, S->d_flag + 1, preset);
-  else if (L.has_spherical && use_mma_attention()) launch_attn_fwd_mma(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, x_in, ev_in, xa, ev1);
+  if (L.has_spherical && attention_mode() >= kAttnTcFwd)
+    return launch_attn_fwd_tc(st, L, S->ve, n_recv, qkv, x_in, ev_in, xa, ev1, S->d_flag + 1, preset);
+  if (L.has_spherical && use_mma_attention()) launch_attn_fwd_mma(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, x_in, ev_in, xa, ev1);
   else launch_attn_fwd_sym(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, x_in, ev_in, xa, ev1);
+  return kOk;
 }
-void attn_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
+[[nodiscard]] int attn_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, const LayerDev& L, int n_recv, int n, const int* row_ptr, const int* nbr_j, const float* dR,
                        const float* qkv, const float* ev_in, const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F,
                        int first_layer, float* virial, int n_own, bool gev_preset = false, bool gq_preset = false) {
   if (!first_layer && L.has_spherical && attention_mode() == kAttnTc)
-    launch_attn_bwd_tc(st, L, S->ve, n_recv, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial, n_own, S->d_flag + 1, gev_preset,
-                       gq_preset);
-  else if (!first_layer && L.has_spherical && use_mma_attention())
+    return launch_attn_bwd_tc(st, L, S->ve, n_recv, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial, n_own, S->d_flag + 1, gev_preset,
+                              gq_preset);
+  if (!first_layer && L.has_spherical && use_mma_attention())
     launch_attn_bwd_mma(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, virial);
   else launch_attn_bwd_sym(st, L, n_recv, n, row_ptr, nbr_j, dR, qkv, ev_in, g_xa, gev1, g_qkv, gev_in, F, first_layer, virial);
+  return kOk;
 }
 
 void layer0_bwd_dispatch(so3lr_b200_system* S, cudaStream_t st, int n_recv, int n_gv, int n, float* F, int n_own) {
@@ -636,7 +639,10 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
     if (!(l == 0 ? tab0 : fuse)) { S->prof.begin(kPProj, st); launch_proj_fwd(st, L, S->x[l], n, S->qkv[l]); S->prof.end(st); }
     S->prof.begin(kPAttnFwd, st);
     if (l == 0 && tab0) launch_layer0_fwd_tab(st, S->sp, M, n, n, row_ptr, nbr_j, dR, S->d_Z, S->xa[0], S->ev1[0]);
-    else if (tiled && L.has_spherical) launch_attn_fwd_tc(st, L, S->ve, n, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], S->d_flag + 1, l > 0 && copies);
+    else if (tiled && L.has_spherical) {
+      int rcf = launch_attn_fwd_tc(st, L, S->ve, n, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], S->d_flag + 1, l > 0 && copies);
+      if (rcf) return rcf;
+    }
     else launch_attn_fwd(st, L, n, row_ptr, nbr_j, dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l]);
     S->prof.end(st);
     S->prof.begin(kPPostFwd, st);
@@ -793,8 +799,9 @@ int fused_forward(so3lr_b200_system* S, cudaStream_t st, const float* R, const S
     } else {
       if (!(fuse && l > 0)) { S->prof.begin(kPProj, st); launch_proj_fwd(st, L, S->x[l], nsend[l], S->qkv[l]); S->prof.end(st); }
       S->prof.begin(kPAttnFwd, st);
-      attn_fwd_dispatch(S, st, L, nrecv[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], l > 0 && copies);
+      int rcf = attn_fwd_dispatch(S, st, L, nrecv[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l], l > 0 && copies);
       S->prof.end(st);
+      if (rcf) return rcf;
     }
     S->prof.begin(kPPostFwd, st);
     const bool emit = fuse && l + 1 < kNumLayers;
@@ -833,13 +840,15 @@ int fused_backward(so3lr_b200_system* S, cudaStream_t st, const Shells& c, float
       fill(st, S->g_xa + (size_t)npost[l] * kF, (size_t)(c.n3 - npost[l]) * kF, 0.f);
       fill(st, S->gev1 + (size_t)npost[l] * kMTot, (size_t)(c.n3 - npost[l]) * kMTot, 0.f);
     }
+    int rcb = kOk;
     S->prof.begin(l == 0 ? kPLayer0Bwd : kPAttnBwd, st);
     if (l == 0 && S->sp.n_species > 0 && use_layer0_tables())
       layer0_bwd_dispatch(S, st, nattn[0], c.n3, c.n3, F, c.n0);
     else
-      attn_bwd_dispatch(S, st, L, nattn[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, F, l == 0 ? 1 : 0,
-                        S->vir(), c.n0, copies, small_presets(c.n0));
+      rcb = attn_bwd_dispatch(S, st, L, nattn[l], c.n3, row_ptr, nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, gev_in, F,
+                              l == 0 ? 1 : 0, S->vir(), c.n0, copies, small_presets(c.n0));
     S->prof.end(st);
+    if (rcb) return rcb;
     if (l > 0) {
       if (!use_mma_dense()) {
         // dL/dx_in = g_xa (skip connection) + projections^T
@@ -1322,6 +1331,7 @@ SO3LR_B200_API int so3lr_b200_system_compute(so3lr_b200_system* S, void* stream,
                    {S->u_e_atom, S->u_q, S->u_h, S->u_zbl, S->u_coul, S->u_disp, nullptr}};
       { launch_chained(unsort_kernel, (n + 255) / 256, 256, 0, st, n, S->d_perm, S->F_s, Fout, A); count_launch(); }
     }
+    SO3LR_CUDA_CHECK(cudaGetLastError());
     return kOk;
   };
   so3lr_b200_system::StepGraph& G = S->step_graph;
@@ -1861,8 +1871,9 @@ SO3LR_B200_API int so3lr_b200_dd_layer_forward(so3lr_b200_system* S, void* strea
     launch_proj_fwd(st, L, S->x[l] + (size_t)first * kF, n1 - first, S->qkv[l] + (size_t)first * kProj);
     S->prof.end(st);
     S->prof.begin(kPAttnFwd, st);
-    attn_fwd_dispatch(S, st, L, n0, S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l]);
+    int rcf = attn_fwd_dispatch(S, st, L, n0, S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->qkv[l], S->x[l], S->ev[l], S->xa[l], S->ev1[l]);
     S->prof.end(st);
+    if (rcf) return rcf;
   }
   const bool emit = use_mma_dense() && l + 1 < kNumLayers;
   S->prof.begin(kPPostFwd, st);
@@ -1989,13 +2000,15 @@ SO3LR_B200_API int so3lr_b200_dd_layer_backward_attn(so3lr_b200_system* S, void*
   cudaStream_t st = (cudaStream_t)stream;
   const int n0 = S->shells[0], l = layer;
   const LayerDev& L = S->mctx.layer[l];
+  int rcb = kOk;
   S->prof.begin(l == 0 ? kPLayer0Bwd : kPAttnBwd, st);
   if (l == 0 && S->sp.n_species > 0 && use_layer0_tables())
     layer0_bwd_dispatch(S, st, n0, S->shells[1], S->n, S->F_s, n0);
   else
-    attn_bwd_dispatch(S, st, L, n0, S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, S->dd_gev_in, S->F_s,
-                      l == 0 ? 1 : 0, S->vir(), n0);
+    rcb = attn_bwd_dispatch(S, st, L, n0, S->n, S->sr.row_ptr, S->sr.nbr_j, S->dR, S->qkv[l], S->ev[l], S->g_xa, S->gev1, S->g_qkv, S->dd_gev_in,
+                            S->F_s, l == 0 ? 1 : 0, S->vir(), n0);
   S->prof.end(st);
+  if (rcb) return rcb;
   if (l == 0 && S->vir()) reduce_virial(S, st, n0);
   if (l > 0) {
     if (!use_mma_dense()) {

@@ -11,7 +11,8 @@ cudaError_t host_alloc_bytes(void** p, size_t bytes);
 void host_free(void* p);
 void devmem_flush(int device);     // gives the idle blocks back
 // Launch whose kernel starts with grid_dep_sync(): its CTAs may be placed while the kernel before it in the stream still runs, so that the
-// launch itself (1.5 to 2 us between two dependent kernels) and the kernel's own preparations overlap with that one's end.
+// launch itself (1.5 to 2 us between two dependent kernels) and the kernel's own preparations overlap with that one's end.  Like that of
+// <<<>>>, a failure stays with the runtime: every entry point asks for it with cudaGetLastError after its last launch.
 template <typename... P, typename... A>
 void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchAttribute attr[1];
@@ -202,15 +203,15 @@ int valid_edges_count_directed(const ValidEdges& V, long long* n_host);
 // entry e (V.orig) half of the force that the pair exerts on its receiver, g[e] += (dE/d dR_e - dE/d dR_e') / 2 with e' the
 // reversed entry.  For any motion of atoms or cell (dR_e' = -dR_e) that is equivalent to the per-entry gradient.  The caller
 // zeroes g_qkv and presets gev_in.
-int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
+[[nodiscard]] int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
                              const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* g_dR, int* err, const int* asym);
 // Same results as launch_attn_fwd_sym for rows [0, n_recv), all rows of the list.  `preset`: xa and ev1 hold x_in and ev_in already.  `err` (device int) is set to 1 when a bounded wait on the
 // tensor-core pipeline ran out; the outputs are then incomplete.
-int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* x_in,
+[[nodiscard]] int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* x_in,
                        const float* ev_in, float* xa, float* ev1, int* err, bool preset = false);
 // Same results as launch_attn_bwd_sym (first_layer = 0) for rows [0, n_recv): writes g_qkv and gev_in rows, adds to F (and to virial
 // rows, of which those below n_own add up to the total).  Presets: gev_in holds gev1, g_qkv zeros already.
-int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
+[[nodiscard]] int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* ev_in,
                        const float* g_xa, const float* gev1, float* g_qkv, float* gev_in, float* F, float* virial, int n_own, int* err,
                        bool gev_preset = false, bool gq_preset = false);
 

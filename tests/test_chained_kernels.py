@@ -41,3 +41,12 @@ def test_non_coherent_loads_are_of_weights(source):
     for arg in re.findall(r"\b(?:__ldg|ldg4|ldg8)\((?:reinterpret_cast<const float4\*>\()?([A-Za-z_][\w.]*)", SOURCES[source]):
         # members of the weight records, the arguments of the loading helpers themselves, weights passed on under a name
         assert arg.startswith(("L.", "M.")) or arg in {"const", "W", "p", "bias", "fin"}, arg
+
+
+def test_statuses_of_the_attention_launches_are_looked_at():
+    """They refuse a list that was compacted for other rows; an evaluation that went on would hold no attention sums."""
+    calls = re.findall(r"([^;{}]*?)\b((?:launch_attn_\w+_tc\w*|attn_\w+_dispatch)\()", SOURCES["engine.cu"])
+    used = [(before.split("\n")[-1].strip(), name) for before, name in calls]
+    assert len(used) > 8
+    for before, name in used:
+        assert before.endswith(("return", "=", "int")), (before, name)
