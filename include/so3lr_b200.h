@@ -137,8 +137,9 @@ SO3LR_B200_API int so3lr_b200_system_export_list(so3lr_b200_system* sys, void* s
  * device, no host read), both entries of a pair receive the antisymmetrised cotangent (dE/dd_e - dE/dd_e') / 2, which
  * contracts to the same forces and strain derivative for every motion of atoms or cell; otherwise, or with
  * SO3LR_B200_GRAPH=scatter in the environment, each entry receives dE/dd_e itself.  The call only enqueues work; it
- * allocates when the list is longer than any list the context has seen before, and at the context's second evaluation outside
- * a capture for the first layer's tables (8.4 MB; without that memory it carries on without them).
+ * allocates when the list is longer than any list the context has seen before, and at the context's first evaluation for the
+ * first layer's tables (8.4 MB; without that memory, or when the first evaluation is enqueued on a stream that is being captured, all
+ * evaluations of the context carry on without them).
  * Replaces: potential(graph) and its jax.grad w.r.t. graph.edges / graph.edges_lr
  *           (so3lr/jaxmd_utils.py:130-141, so3lr/graph.py:3-24). */
 SO3LR_B200_API int so3lr_b200_system_graph_eval(so3lr_b200_system* sys, void* stream, int64_t n_edges, const int32_t* idx_i,

@@ -301,7 +301,7 @@ struct so3lr_b200_system {
   int shells[4] = {0, 0, 0, 0};  // domain-decomposed evaluation: owned | + short-range ghosts | (unused) | all local atoms
   SpeciesTables sp{};            // per-element-pair tables of the first layer (built by the first evaluation that reads them)
   std::vector<int> elements;     // the structure's elements while the tables are still to be built
-  int64_t graph_evals = 0;       // evaluations on caller-supplied lists
+  int graph_tables = -1;         // whether evaluations on caller-supplied lists take the tables: decided by the first of them
   float* GV = nullptr;           // n_cap x 32 scratch of the tabulated first-layer reverse pass
   float *dd_gev2 = nullptr, *dd_gev_in = nullptr;   // ping-pong cotangents of ev between the layers of the reverse pass
   so3lr_b200_options opt{};
@@ -630,7 +630,7 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
     if (rcv) return rcv;
   }
   S->prof.begin(kPGeom, st); launch_sr_geometry_zbl(st, M, S->cell, n, n_edges, edge_i, nbr_j, S->d_Z, nullptr, 1, dR, S->e_zbl, g_dR, ge, nullptr); S->prof.end(st);
-  const bool tab0 = tiled && S->sp.n_species > 0 && use_layer0_tables();
+  const bool tab0 = tiled && S->graph_tables > 0 && S->sp.n_species > 0 && use_layer0_tables();
   const bool copies = tiled && dense_copies();
   const bool fuse = use_mma_dense();   // q/k/v rows of layer l + 1 come out of layer l's dense block, their transpose goes into it
   if (!tab0) { int rce = embed_atoms(S, st, n, S->x[0]); if (rce) return rce; }
@@ -968,7 +968,7 @@ bool charge_spin_scalars(const so3lr_b200_model& m, int n, const int32_t* Z, int
   return !rows->empty();      // a charged graph without atoms has none
 }
 
-// tables of the first layer, built when the first evaluation that reads them comes (a graph-level context never does)
+// tables of the first layer, built when the first evaluation that reads them comes
 int ensure_species_tables(so3lr_b200_system* S, cudaStream_t st) {
   if (S->elements.empty()) return kOk;
   const int rc = species_tables_build(st, S->mctx, S->elements.data(), (int)S->elements.size(), &S->sp);
@@ -1501,21 +1501,15 @@ static int graph_eval_impl(so3lr_b200_system* S, void* stream, int64_t n_edges, 
   S->o_e_atom = S->e_atom; S->o_q = S->q; S->o_h = S->h; S->o_zbl = S->e_zbl; S->o_coul = S->e_coul; S->o_disp = S->e_disp;
   { row_ptr_from_sorted_kernel<<<(n + 1 + 255) / 256, 256, 0, st>>>(n, n_edges, idx_i, S->d_rowptr_g); count_launch(); }
   { row_ptr_from_sorted_kernel<<<(n + 1 + 255) / 256, 256, 0, st>>>(n, n_pairs, idx_i_lr, S->d_rowptr_lr_g); count_launch(); }
-  // The first layer's element-pair tables pay from the second evaluation of a context on (forming them costs about what they save in
-  // one); a stream that is being captured takes them only if they are there.
-  int rc = kOk;
-  if (S->graph_evals++ > 0 && !S->elements.empty()) {
+  // The first of these evaluations forms the first layer's element-pair tables (the time of one generic first layer), so that all
+  // evaluations of a context run the same kernels.  If its stream is being captured, or memory is short, they all run the generic layer.
+  if (S->graph_tables < 0) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
-    if (cap == cudaStreamCaptureStatusNone) {
-      if (ensure_species_tables(S, st) != kOk) {      // no memory for them: the generic first layer needs none
-        cudaGetLastError();
-        S->sp.n_species = 0;
-        S->elements.clear();
-      }
-    }
+    S->graph_tables = cap == cudaStreamCaptureStatusNone && ensure_species_tables(S, st) == kOk;
+    if (!S->graph_tables) cudaGetLastError();
   }
-  rc = evaluate_graph(S, st, S->d_rowptr_g, idx_j, idx_i, n_edges, S->d_rowptr_lr_g, idx_j_lr, edges, edges_lr, g_edges, g_edges_lr,
+  int rc = evaluate_graph(S, st, S->d_rowptr_g, idx_j, idx_i, n_edges, S->d_rowptr_lr_g, idx_j_lr, edges, edges_lr, g_edges, g_edges_lr,
                           g_e_atom, positions, g_positions, strain6);
   if (rc) return rc;
   if (e_atom) SO3LR_CUDA_CHECK(cudaMemcpyAsync(e_atom, S->e_atom, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, st));

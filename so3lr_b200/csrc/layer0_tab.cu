@@ -333,6 +333,16 @@ __global__ void __launch_bounds__(128) layer0_bwd_entries_kernel(SpeciesTables T
   g_dR[3 * e] += f.x; g_dR[3 * e + 1] += f.y; g_dR[3 * e + 2] += f.z;
 }
 
+// the elements as a kernel argument: a copy from the host's stack would need a wait, and a context of one evaluation (a batch of a
+// dataset) builds its tables in the middle of it
+struct SpeciesList {
+  int slot[119], z[SP];
+};
+__global__ void set_species_kernel(SpeciesList L, int* __restrict__ slot, int* __restrict__ z) {
+  if (threadIdx.x < 119) slot[threadIdx.x] = L.slot[threadIdx.x];
+  if (threadIdx.x < SP) z[threadIdx.x] = L.z[threadIdx.x];
+}
+
 }  // namespace
 
 // (Re)builds the tables for the elements present in Z_host; returns kOk with T->n_species = 0 when more than
@@ -359,13 +369,11 @@ int species_tables_build(cudaStream_t st, const ModelDev& M, const int* Z_host, 
     SO3LR_CUDA_CHECK(dev_alloc(&T->z_sp, SP));
   }
   const int ns = (int)sp.size();
-  int slot[119];
-  for (int z = 0; z < 119; ++z) slot[z] = 0;
-  for (int k = 0; k < ns; ++k) { slot[sp[k]] = k; T->species[k] = sp[k]; }
+  SpeciesList list{};
+  for (int k = 0; k < ns; ++k) { list.slot[sp[k]] = k; list.z[k] = sp[k]; T->species[k] = sp[k]; }
   T->n_species = ns;
-  SO3LR_CUDA_CHECK(cudaMemcpyAsync(T->slot, slot, sizeof(slot), cudaMemcpyHostToDevice, st));
-  SO3LR_CUDA_CHECK(cudaMemcpyAsync(T->z_sp, sp.data(), ns * sizeof(int), cudaMemcpyHostToDevice, st));
-  SO3LR_CUDA_CHECK(cudaStreamSynchronize(st));   // the host arrays above go out of scope
+  set_species_kernel<<<1, 128, 0, st>>>(list, T->slot, T->z_sp);
+  count_launch();
   launch_embed(st, M, T->z_sp, ns, T->x_sp);
   launch_proj_fwd(st, M.layer[0], T->x_sp, ns, T->qkv_sp);
   SO3LR_CUDA_CHECK(cudaMemcpy2DAsync(T->v_sp, kF * sizeof(float), T->qkv_sp + 2 * kF, kProj * sizeof(float), kF * sizeof(float), ns,

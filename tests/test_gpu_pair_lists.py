@@ -57,7 +57,7 @@ def test_list_forms_against_the_oracle(name, form):
     n = len(Z)
     s = System(Z, cell, cutoff_lr=6.0 if cell is not None else 100.0, damping=2.0, lr_format="sparse")
     t = lambda a: torch.tensor(a, device="cuda")
-    # the first evaluation of a context runs the generic first layer, later ones its tables
+    # the first evaluation of a context forms the first layer's tables
     results = [s.graph_eval(t(i), t(j), t(d), t(il), t(jl), t(dl)) for _ in range(2)]
     D, DL = torch.tensor(d, dtype=torch.float64, requires_grad=True), torch.tensor(dl, dtype=torch.float64, requires_grad=True)
     e, _ = O.energy_from_graph(O.load_params(), Z, D, i, j, DL, il, jl, lr_format="sparse", cutoff_lr=6.0 if cell is not None else 100.0, damping=2.0)
@@ -81,3 +81,41 @@ def _check(o, e, g, i, j, D, n, form):
     w, wr = D.T @ got, D.T @ g
     assert float((w - wr).abs().max()) <= 1e-4 * max(1.0, float(wr.abs().max()))
     assert float(got[~m].abs().sum()) == 0.0
+
+
+def test_more_elements_than_the_tables_hold():
+    """Nine elements: every evaluation of the context runs the generic first layer."""
+    from oracle import so3lr_oracle as O
+    from so3lr_b200.engine import System
+    Z, _, (i, j, d), (il, jl, dl) = _lists("mol40", "plain")
+    Z = np.array(Z)
+    heavy = np.nonzero(Z > 1)[0][:8]
+    Z[heavy] = [5, 6, 7, 8, 9, 15, 16, 17]
+    assert len(set(Z.tolist())) == 9
+    s = System(Z, None, cutoff_lr=100.0, damping=2.0, lr_format="sparse")
+    t = lambda a: torch.tensor(a, device="cuda")
+    D, DL = torch.tensor(d, dtype=torch.float64, requires_grad=True), torch.tensor(dl, dtype=torch.float64)
+    e, _ = O.energy_from_graph(O.load_params(), Z, D, i, j, DL, il, jl, lr_format="sparse", cutoff_lr=100.0, damping=2.0)
+    g, = torch.autograd.grad(e.sum(), D)
+    for _ in range(2):
+        o = s.graph_eval(t(i), t(j), t(d), t(il), t(jl), t(dl))
+        # elements were exchanged under the same positions: strained bonds with forces far above 20 eV/A, so relative to the largest
+        scale = max(1.0, float(g.abs().max()) / 20.0)
+        assert float((o["e_atom"].double().cpu() - e.detach()).abs().sum()) <= 1e-5 * float(e.detach().abs().sum())
+        f = lambda x: torch.zeros(len(Z), 3, dtype=torch.float64).index_add(0, torch.tensor(i), x).index_add(0, torch.tensor(j), -x)
+        assert float((f(o["g_edges"].double().cpu()) - f(g)).abs().max()) <= 1e-4 * scale
+
+
+@pytest.mark.parametrize("system", ["neutral", "batch"])
+def test_evaluations_of_a_context_run_the_same_kernels(system):
+    """Two atoms: every sum has one term, so that evaluations of the same inputs agree bit for bit, the context's first one among them, and
+    the re-evaluation for another cotangent has the same energies."""
+    from so3lr_b200.engine import System
+    t = lambda a, **k: torch.tensor(a, device="cuda", **k)
+    kw = {"graph_start": [0, 2, 2], "total_charge": [1.0, 0.0]} if system == "batch" else {}
+    s = System([8, 1], None, cutoff_lr=100.0, damping=2.0, lr_format="sparse", **kw)
+    i, j = t([0, 1], dtype=torch.int32), t([1, 0], dtype=torch.int32)
+    d = t([[0.3, -0.8, 0.9], [-0.3, 0.8, -0.9]])
+    out = [s.graph_eval(i, j, d, i, j, d, g_e_atom=g) for g in (None, None, t([1.0, 0.5]), None)]
+    assert all(torch.equal(o["e_atom"], out[0]["e_atom"]) for o in out)
+    assert all(torch.equal(o[k], out[0][k]) for o in (out[1], out[3]) for k in ("g_edges", "g_edges_lr", "partial_charges"))
