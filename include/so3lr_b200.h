@@ -378,6 +378,10 @@ SO3LR_B200_API int so3lr_b200_neighbor_list_noalloc(void* stream, int n_atoms, c
  * (so3lr/cli/so3lr_md.py:836-877). */
 SO3LR_B200_API int so3lr_b200_list_row_total(void* stream, const int32_t* row_count_dev, int n_rows, int64_t* total_host);
 
+/* The nth device allocation that the library makes on the calling thread from now on finds no memory (0: none does); with `persistent`
+ * neither do those after it, until the next call.  Returns what is left of the count set before (0 when it ran out).  For tests of
+ * what a context does when memory is short. */
+SO3LR_B200_API int64_t so3lr_b200_host_fail_allocation(int64_t nth, int persistent);
 SO3LR_B200_API void so3lr_b200_host_sph_harm(float x, float y, float z, float* y24);
 SO3LR_B200_API void so3lr_b200_host_sph_harm_vjp(float x, float y, float z, const float* g24, float* g3);
 SO3LR_B200_API void so3lr_b200_host_pair_terms(float r, int zi, int zj, float qi, float qj, float hi, float hj, float cutoff_lr,

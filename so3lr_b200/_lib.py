@@ -83,6 +83,7 @@ def _load():
         "so3lr_b200_system_profile_read": (i32, [p, i32, p, p, p]),
         "so3lr_b200_neighbor_list_noalloc": (i32, [p, i32, p, p, f32, i32, p, i64, p, p]),
         "so3lr_b200_list_row_total": (i32, [p, p, i32, C.POINTER(i64)]),
+        "so3lr_b200_host_fail_allocation": (i64, [i64, i32]),
         "so3lr_b200_host_sph_harm": (None, [f32, f32, f32, p]),
         "so3lr_b200_host_sph_harm_vjp": (None, [f32, f32, f32, p, p]),
         "so3lr_b200_host_pair_terms": (None, [f32, i32, i32, f32, f32, f32, f32, f32, f32, p]),

@@ -1613,7 +1613,7 @@ int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity) {
     if (V->i) dev_free(V->i);
     if (V->j) dev_free(V->j);
     if (V->d) dev_free(V->d);
-    V->i = V->j = nullptr; V->d = nullptr;
+    V->i = V->j = nullptr; V->d = nullptr; V->capacity = 0;
     if (capacity < 1) capacity = 1;
     SO3LR_CUDA_CHECK(dev_alloc(&V->i, (size_t)capacity));
     SO3LR_CUDA_CHECK(dev_alloc(&V->j, (size_t)capacity));

@@ -35,6 +35,8 @@ Cache& cache() {
   return *c;
 }
 thread_local int tl_batch = 0;
+thread_local long long tl_fail_in = 0;      // tests: the allocation of this thread that finds no memory, 0 = none
+thread_local bool tl_fail_on = false;       //   ... and all after it
 
 // sizes in steps of an eighth of their power of two (512 bytes at least), so that similar requests share blocks
 size_t round_size(size_t b) {
@@ -81,6 +83,11 @@ cudaError_t dev_alloc_bytes(void** p, size_t bytes) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
+  *p = nullptr;
+  if (tl_fail_in > 0 && (tl_fail_in == 1 || --tl_fail_in == 0)) {
+    if (!tl_fail_on) tl_fail_in = 0;
+    return cudaErrorMemoryAllocation;
+  }
   bytes = round_size(bytes);
   Cache& c = cache();
   std::lock_guard<std::mutex> g(c.lock);
@@ -90,6 +97,7 @@ cudaError_t dev_alloc_bytes(void** p, size_t bytes) {
     cudaGetLastError();
     flush_locked(c, dev);
     e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();      // the caller has the status; it may go on without the array
   }
   if (e != cudaSuccess) { *p = nullptr; return e; }
   c.live[*p] = {bytes, dev};
@@ -128,6 +136,12 @@ DevFreeBatch::DevFreeBatch() {
   ++tl_batch;
 }
 DevFreeBatch::~DevFreeBatch() { --tl_batch; }
+
+long long devmem_fail(long long nth, bool on) {
+  const long long left = tl_fail_in;
+  tl_fail_in = nth; tl_fail_on = on;
+  return left;
+}
 
 void devmem_flush(int device) {
   Cache& c = cache();

@@ -406,7 +406,7 @@ int ensure_edge_buffers(so3lr_b200_system* S, long long n_edges) {
   if (n_edges <= S->edge_cap) return valid_edges_reserve(&S->ve, S->n_cap, S->edge_cap);   // row arrays exist even without edges
   long long cap = n_edges + n_edges / 4 + 1024;
   if (S->dR) dev_free(S->dR);
-  S->dR = nullptr;
+  S->dR = nullptr; S->edge_cap = 0;      // until the new array is there
   SO3LR_CUDA_CHECK(dev_alloc(&S->dR, (size_t)cap * 3));
   S->edge_cap = cap;
   return valid_edges_reserve(&S->ve, S->n_cap, cap);
@@ -418,6 +418,7 @@ constexpr int kSortMinAtoms = 512;
 int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bool allow_sort, int which = -1) {
   const float r_sr = kCutoffSr + S->opt.skin;
   const float* R = R_user;
+  S->have_lists = false;      // what follows overwrites them: a call that fails on the way leaves none
   const int nb = (S->n + 255) / 256;
   S->sorted = allow_sort && S->cell.periodic && S->n_graphs == 1 && S->n >= kSortMinAtoms;
   if (S->sorted) {
@@ -1583,10 +1584,11 @@ SO3LR_B200_API int so3lr_b200_system_enable_virial(so3lr_b200_system* S, int ena
   if (!S) return kInvalidArgument;
   if (S->n_graphs != 1) return kInvalidArgument;
   SO3LR_CUDA_CHECK(cudaSetDevice(S->model->device));
-  if (enable && !S->virial) {
-    S->virial = S->pool.get<float>((size_t)S->n_cap * 6);
-    S->virial_partials = S->pool.get<double>(6 * kVirialBlocks);
-    S->virial_sum = S->pool.get<double>(9);
+  if (enable) {
+    S->pool.status = kOk;
+    if (!S->virial) S->virial = S->pool.get<float>((size_t)S->n_cap * 6);
+    if (!S->virial_partials) S->virial_partials = S->pool.get<double>(6 * kVirialBlocks);
+    if (!S->virial_sum) S->virial_sum = S->pool.get<double>(9);
     if (S->pool.status != kOk) return S->pool.status;
   }
   S->want_virial = enable != 0;
@@ -2138,6 +2140,7 @@ SO3LR_B200_API void so3lr_b200_host_zbl(const float* blob, float r, int zi, int 
 SO3LR_B200_API void so3lr_b200_host_radial_filter(const float* blob, int layer, double r, double* w256, double* dw256) {
   radial_filter_reference(blob, layer, r, w256, dw256);
 }
+SO3LR_B200_API int64_t so3lr_b200_host_fail_allocation(int64_t nth, int persistent) { return devmem_fail(nth > 0 ? nth : 0, persistent != 0); }
 SO3LR_B200_API int so3lr_b200_list_row_total(void* stream, const int32_t* row_count_dev, int n_rows, int64_t* total_host) {
   if (!row_count_dev || !total_host || n_rows < 0) return kInvalidArgument;
   long long t = 0;

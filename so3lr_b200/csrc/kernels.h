@@ -10,6 +10,7 @@ void dev_free(void* p);            // waits for the device first, like cudaFree,
 cudaError_t host_alloc_bytes(void** p, size_t bytes);
 void host_free(void* p);
 void devmem_flush(int device);     // gives the idle blocks back
+long long devmem_fail(long long nth, bool on);      // tests: see so3lr_b200_host_fail_allocation
 // Launch whose kernel starts with grid_dep_sync(): its CTAs may be placed while the kernel before it in the stream still runs, so that the
 // launch itself (1.5 to 2 us between two dependent kernels) and the kernel's own preparations overlap with that one's end.  Like that of
 // <<<>>>, a failure stays with the runtime: every entry point asks for it with cudaGetLastError after its last launch.

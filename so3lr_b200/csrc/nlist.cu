@@ -367,11 +367,31 @@ __global__ void morton_keys_kernel(Cell cell, Grid G, int n, const float* __rest
   iota[a] = a;
 }
 
+// Every capacity is zero while its arrays are replaced: one that is not there after a failed allocation is asked for again.
 template <typename T>
 int ensure(T** p, size_t n) {
   if (*p) dev_free(*p);
   *p = nullptr;
   SO3LR_CUDA_CHECK(dev_alloc(p, n));
+  return kOk;
+}
+// arrays of one element per atom
+int ensure_atoms(NlistWorkspace* w, int n) {
+  if (n <= w->n_cap) return kOk;
+  w->n_cap = 0;
+  int st;
+  if ((st = ensure(&w->cell_of, n)) || (st = ensure(&w->cell_sorted, n)) || (st = ensure(&w->atom_sorted, n)) || (st = ensure(&w->atom_iota, n)) ||
+      (st = ensure(&w->row_count, (size_t)n + 1)) || (st = ensure(&w->pos_sorted, (size_t)n)))
+    return st;
+  w->n_cap = n;
+  return kOk;
+}
+int ensure_bytes(void** p, size_t* have, size_t need) {
+  if (need <= *have) return kOk;
+  if (*p) dev_free(*p);
+  *p = nullptr; *have = 0;
+  SO3LR_CUDA_CHECK(dev_alloc_bytes(p, need));
+  *have = need;
   return kOk;
 }
 
@@ -397,20 +417,12 @@ int spatial_order(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, co
   if (n <= 0 || !cell.periodic) return kInvalidArgument;
   if (n > w->key_cap) {
     int st;
+    w->key_cap = 0;
     if ((st = ensure(&w->key, n))) return st;
     if ((st = ensure(&w->key_sorted, n))) return st;
     w->key_cap = n;
   }
-  if (n > w->n_cap) {
-    int st;
-    if ((st = ensure(&w->cell_of, n))) return st;
-    if ((st = ensure(&w->cell_sorted, n))) return st;
-    if ((st = ensure(&w->atom_sorted, n))) return st;
-    if ((st = ensure(&w->atom_iota, n))) return st;
-    if ((st = ensure(&w->row_count, (size_t)n + 1))) return st;
-    if ((st = ensure(&w->pos_sorted, (size_t)n))) return st;
-    w->n_cap = n;
-  }
+  if (int rca = ensure_atoms(w, n)) return rca;
   Grid G{};
   for (int k = 0; k < 3; ++k) {
     double nx = cell.hinv[0 + k], ny = cell.hinv[3 + k], nz = cell.hinv[6 + k];
@@ -423,12 +435,7 @@ int spatial_order(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, co
   { morton_keys_kernel<<<(n + 255) / 256, 256, 0, s>>>(cell, G, n, R, w->key, w->atom_iota); count_launch(); }
   size_t need = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, need, w->key, w->key_sorted, w->atom_iota, perm, n, 0, 30, s);
-  if (need > w->sort_bytes) {
-    if (w->sort_tmp) dev_free(w->sort_tmp);
-    w->sort_tmp = nullptr;
-    SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->sort_tmp, need));
-    w->sort_bytes = need;
-  }
+  if (int rcb = ensure_bytes(&w->sort_tmp, &w->sort_bytes, need)) return rcb;
   size_t tmp = w->sort_bytes;
   cub::DeviceRadixSort::SortPairs(w->sort_tmp, tmp, w->key, w->key_sorted, w->atom_iota, perm, n, 0, 30, s);
   count_launch(6);   // histogram, prefix, four 8-bit passes
@@ -443,27 +450,16 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   w->n_rows = 0;
   if (n <= 0) { out->count = 0; return kOk; }
   if (n_rows < 0 || n_rows > n) n_rows = n;
-  if (n > w->n_cap) {
-    int st;
-    if ((st = ensure(&w->cell_of, n))) return st;
-    if ((st = ensure(&w->cell_sorted, n))) return st;
-    if ((st = ensure(&w->atom_sorted, n))) return st;
-    if ((st = ensure(&w->atom_iota, n))) return st;
-    if ((st = ensure(&w->row_count, (size_t)n + 1))) return st;
-    if ((st = ensure(&w->pos_sorted, (size_t)n))) return st;
-    w->n_cap = n;
-  }
+  if (int rca = ensure_atoms(w, n)) return rca;
   if (!w->ticket) {
     SO3LR_CUDA_CHECK(dev_alloc(&w->ticket, 2));
     SO3LR_CUDA_CHECK(cudaMemsetAsync(w->ticket, 0, 2 * sizeof(int), s));
   }
-  if (!w->d_total) {
-    SO3LR_CUDA_CHECK(dev_alloc(&w->d_total, 1));
-    SO3LR_CUDA_CHECK(host_alloc(&w->h_total, 1));
-  }
+  if (!w->d_total) SO3LR_CUDA_CHECK(dev_alloc(&w->d_total, 1));
+  if (!w->h_total) SO3LR_CUDA_CHECK(host_alloc(&w->h_total, 1));
   if (n + 1 > out->row_cap) {
     if (out->row_ptr) dev_free(out->row_ptr);
-    out->row_ptr = nullptr;
+    out->row_ptr = nullptr; out->row_cap = 0;
     SO3LR_CUDA_CHECK(dev_alloc(&out->row_ptr, ((size_t)n + 1)));
     out->row_cap = n + 1;
   }
@@ -510,8 +506,8 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     binned = n_cells > 1;      // the atoms of a single cell come in their own order either way
     if (binned) {
       if (n_cells + 1 > w->cell_cap) {
-        int st;
-        if ((st = ensure(&w->cell_start, (size_t)n_cells + 1))) return st;
+        w->cell_cap = 0;
+        if (int rcc = ensure(&w->cell_start, (size_t)n_cells + 1)) return rcc;
         w->cell_cap = n_cells + 1;
       }
       { assign_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(cell, G, n, R, w->cell_of, w->atom_iota); count_launch(); }
@@ -522,11 +518,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
       size_t need2 = 0;
       cub::DeviceScan::ExclusiveSum(nullptr, need2, w->row_count, out->row_ptr, n, s);   // sized for the largest row count
       if (need2 > need) need = need2;
-      if (need > w->cub_bytes) {
-        if (w->cub_tmp) dev_free(w->cub_tmp);
-        SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->cub_tmp, need));
-        w->cub_bytes = need;
-      }
+      if (int rcb = ensure_bytes(&w->cub_tmp, &w->cub_bytes, need)) return rcb;
       size_t tmp = w->cub_bytes;
       cub::DeviceRadixSort::SortPairs(w->cub_tmp, tmp, w->cell_of, w->cell_sorted, w->atom_iota, w->atom_sorted, n, 0, bits, s);
       count_launch(2 + (bits + 7) / 8);
@@ -537,11 +529,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   if (!binned) {
     size_t need = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, need, w->row_count, out->row_ptr, n, s);
-    if (need > w->cub_bytes) {
-      if (w->cub_tmp) dev_free(w->cub_tmp);
-      SO3LR_CUDA_CHECK(dev_alloc_bytes(&w->cub_tmp, need));
-      w->cub_bytes = need;
-    }
+    if (int rcb = ensure_bytes(&w->cub_tmp, &w->cub_bytes, need)) return rcb;
   }
   const int blocks = (n_rows + 7) / 8;
   if (n_rows == 0) { out->count = 0; return kOk; }
@@ -604,7 +592,7 @@ int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListD
       long long cap = total + total / 4 + 1024;
       if (out->nbr_j) dev_free(out->nbr_j);
       if (out->edge_i) dev_free(out->edge_i);
-      out->nbr_j = nullptr; out->edge_i = nullptr;
+      out->nbr_j = nullptr; out->edge_i = nullptr; out->capacity = 0; out->count = 0;
       SO3LR_CUDA_CHECK(dev_alloc(&out->nbr_j, (size_t)cap));
       SO3LR_CUDA_CHECK(dev_alloc(&out->edge_i, (size_t)cap));
       out->capacity = cap;

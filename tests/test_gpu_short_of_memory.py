@@ -1,0 +1,106 @@
+"""Contexts whose device allocations find no memory (so3lr_b200_host_fail_allocation reports one as failed; nothing is exhausted): a call
+either raises or gives the right results, and once memory is there again the next call does, whichever allocation it was."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _fail(nth, persistent=False):
+    from so3lr_b200._lib import lib
+    return lib.so3lr_b200_host_fail_allocation(nth, int(persistent))
+
+
+def _attempts(call, check, persistent, limit=100):
+    """`call` with its 1st, 2nd, ... allocation failing, until it makes no more of them; a plain call follows each."""
+    raised = 0
+    for nth in range(1, limit):
+        _fail(nth, persistent)
+        try:
+            try:
+                check(call(nth))
+            except Exception as e:
+                assert "check" not in str(e)
+                raised += 1
+        finally:
+            left = _fail(0)
+        check(call(nth))
+        if left > int(persistent):
+            return nth - 1, raised
+    raise AssertionError("the call never ran out of allocations")
+
+
+def _close(out, ref):
+    assert abs(float(out["energy"].sum() - ref["energy"].sum())) <= 2e-6 * abs(float(ref["energy"].sum())), "check: energy"
+    assert float((out["forces"] - ref["forces"]).abs().max()) <= 5e-5, "check: forces"
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("skin", [0.0, 1.0])
+def test_lists_that_grow(skin, persistent):
+    """From a thin structure to a dense one: every list and everything sized by them is replaced."""
+    from so3lr_b200 import workloads as W
+    from so3lr_b200.engine import System
+    Z, R, _ = W.water_box(216, 18.7, 5)
+    dense = torch.tensor(R, dtype=torch.float32, device="cuda")
+    mol = torch.arange(len(Z), device="cuda") // 3
+    centre = dense[::3][mol]
+    thin = centre * 4.0 + (dense - centre)
+    cell = np.eye(3) * 18.7 * 4.0
+    make = lambda: System(Z, cell, cutoff_lr=9.0, damping=2.0, skin=skin)
+    ref, ref_thin = make().compute(dense), make().compute(thin)
+    state = {}
+
+    def call(nth):
+        if state.get("nth") != nth:                   # a context of its own for every allocation
+            left = _fail(0)
+            state.update(nth=nth, s=make())
+            _close(state["s"].compute(thin), ref_thin)
+            _fail(left, persistent)
+        return state["s"].compute(dense)
+
+    made, raised = _attempts(call, lambda o: _close(o, ref), persistent)
+    assert made >= 6, made
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+def test_everything_from_the_first_call_on(persistent):
+    """Creation, virial, a host call, a graph-level call: contexts that could not be made leave nothing behind that hinders the next."""
+    from so3lr_b200 import workloads as W
+    from so3lr_b200.engine import System
+    Z, R, cell = W.water_box(64, 12.42, 1000)
+    R = np.asarray(R, np.float32)
+
+    def call(nth):
+        s = System(Z, cell, cutoff_lr=6.0, damping=2.0, skin=0.5)
+        s.enable_virial(True)
+        s.compute_host(R)
+        return s.compute(torch.tensor(R, device="cuda"))
+
+    ref = call(0)
+
+    def check(o):
+        _close(o, ref)
+        assert float((o["virial"] - ref["virial"]).abs().max()) <= 2e-4 * float(ref["virial"].abs().max()), "check: virial"
+
+    made, raised = _attempts(call, check, persistent)
+    assert made >= 20 and raised >= 1, (made, raised)
+
+
+def test_a_context_whose_virial_arrays_came_late():
+    from so3lr_b200 import workloads as W
+    from so3lr_b200.engine import System
+    Z, R, cell = W.water_box(64, 12.42, 1000)
+    R = torch.tensor(np.asarray(R, np.float32), device="cuda")
+    ref = System(Z, cell, cutoff_lr=6.0, damping=2.0)
+    ref.enable_virial(True)
+    ref = ref.compute(R)
+    for nth in (1, 2, 3):
+        s = System(Z, cell, cutoff_lr=6.0, damping=2.0)
+        _fail(nth)
+        with pytest.raises(Exception):
+            s.enable_virial(True)
+        assert _fail(0) == 0
+        s.enable_virial(True)
+        assert float((s.compute(R)["virial"] - ref["virial"]).abs().max()) <= 2e-4 * float(ref["virial"].abs().max())
