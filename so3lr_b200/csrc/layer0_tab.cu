@@ -345,8 +345,29 @@ __global__ void set_species_kernel(SpeciesList L, int* __restrict__ slot, int* _
 
 }  // namespace
 
+static int build_tables(cudaStream_t st, const ModelDev& M, const std::vector<int>& sp, SpeciesTables* T) {
+  if (!T->table) SO3LR_CUDA_CHECK(dev_alloc(&T->table, (size_t)SP * SP * (kTableGrid - 1) * 32));
+  if (!T->v_sp) SO3LR_CUDA_CHECK(dev_alloc(&T->v_sp, (size_t)SP * kF));
+  if (!T->slot) SO3LR_CUDA_CHECK(dev_alloc(&T->slot, 119));
+  if (!T->qkv_sp) SO3LR_CUDA_CHECK(dev_alloc(&T->qkv_sp, (size_t)SP * kProj));
+  if (!T->x_sp) SO3LR_CUDA_CHECK(dev_alloc(&T->x_sp, (size_t)SP * kF));
+  if (!T->z_sp) SO3LR_CUDA_CHECK(dev_alloc(&T->z_sp, SP));
+  const int ns = (int)sp.size();
+  SpeciesList list{};
+  for (int k = 0; k < ns; ++k) { list.slot[sp[k]] = k; list.z[k] = sp[k]; }
+  set_species_kernel<<<1, 128, 0, st>>>(list, T->slot, T->z_sp);
+  count_launch();
+  launch_embed(st, M, T->z_sp, ns, T->x_sp);
+  launch_proj_fwd(st, M.layer[0], T->x_sp, ns, T->qkv_sp);
+  SO3LR_CUDA_CHECK(cudaMemcpy2DAsync(T->v_sp, kF * sizeof(float), T->qkv_sp + 2 * kF, kProj * sizeof(float), kF * sizeof(float), ns,
+                                     cudaMemcpyDeviceToDevice, st));
+  { build_pair_table_kernel<<<dim3(kTableSplit, ns * ns), 256, 0, st>>>(M.layer[0].table, T->qkv_sp, ns, T->table); count_launch(); }
+  SO3LR_CUDA_CHECK(cudaGetLastError());
+  return kOk;
+}
+
 // (Re)builds the tables for the elements present in Z_host; returns kOk with T->n_species = 0 when more than
-// kMaxTabSpecies elements occur (the caller then uses the generic kernels).
+// kMaxTabSpecies elements occur (the caller then uses the generic kernels).  After a failure there are none: nothing is half built.
 int species_tables_build(cudaStream_t st, const ModelDev& M, const int* Z_host, int n, SpeciesTables* T) {
   std::vector<int> sp;
   for (int a = 0; a < n; ++a) {
@@ -359,27 +380,12 @@ int species_tables_build(cudaStream_t st, const ModelDev& M, const int* Z_host, 
   std::sort(sp.begin(), sp.end());
   bool same = T->n_species == (int)sp.size();
   for (int k = 0; same && k < (int)sp.size(); ++k) same = T->species[k] == sp[k];
-  if (same && T->table) return kOk;
-  if (!T->table) {
-    SO3LR_CUDA_CHECK(dev_alloc(&T->table, (size_t)SP * SP * (kTableGrid - 1) * 32));
-    SO3LR_CUDA_CHECK(dev_alloc(&T->v_sp, (size_t)SP * kF));
-    SO3LR_CUDA_CHECK(dev_alloc(&T->slot, 119));
-    SO3LR_CUDA_CHECK(dev_alloc(&T->qkv_sp, (size_t)SP * kProj));
-    SO3LR_CUDA_CHECK(dev_alloc(&T->x_sp, (size_t)SP * kF));
-    SO3LR_CUDA_CHECK(dev_alloc(&T->z_sp, SP));
-  }
-  const int ns = (int)sp.size();
-  SpeciesList list{};
-  for (int k = 0; k < ns; ++k) { list.slot[sp[k]] = k; list.z[k] = sp[k]; T->species[k] = sp[k]; }
-  T->n_species = ns;
-  set_species_kernel<<<1, 128, 0, st>>>(list, T->slot, T->z_sp);
-  count_launch();
-  launch_embed(st, M, T->z_sp, ns, T->x_sp);
-  launch_proj_fwd(st, M.layer[0], T->x_sp, ns, T->qkv_sp);
-  SO3LR_CUDA_CHECK(cudaMemcpy2DAsync(T->v_sp, kF * sizeof(float), T->qkv_sp + 2 * kF, kProj * sizeof(float), kF * sizeof(float), ns,
-                                     cudaMemcpyDeviceToDevice, st));
-  { build_pair_table_kernel<<<dim3(kTableSplit, ns * ns), 256, 0, st>>>(M.layer[0].table, T->qkv_sp, ns, T->table); count_launch(); }
-  SO3LR_CUDA_CHECK(cudaGetLastError());
+  if (same) return kOk;
+  T->n_species = 0;
+  const int rc = build_tables(st, M, sp, T);
+  if (rc) { species_tables_free(T); return rc; }
+  T->n_species = (int)sp.size();
+  for (int k = 0; k < T->n_species; ++k) T->species[k] = sp[k];
   return kOk;
 }
 

@@ -104,3 +104,38 @@ def test_a_context_whose_virial_arrays_came_late():
         assert _fail(0) == 0
         s.enable_virial(True)
         assert float((s.compute(R)["virial"] - ref["virial"]).abs().max()) <= 2e-4 * float(ref["virial"].abs().max())
+
+
+@pytest.mark.parametrize("call", ["compute", "graph"])
+def test_first_layer_tables_of_one_context(call):
+    """The tables are formed in the middle of the first evaluation: whichever of their arrays is missing, a repeated evaluation of the same
+    context has the right results, and a graph-level one carries on without them at once."""
+    from so3lr_b200.engine import System
+    t = lambda a, **k: torch.tensor(a, device="cuda", **k)
+    Z, R = [8, 1, 1], t([[0.0, 0.0, 0.0], [0.96, 0.0, 0.0], [-0.24, 0.93, 0.0]])
+    i, j = (t(a, dtype=torch.int32) for a in ([0, 0, 1, 1, 2, 2], [1, 2, 0, 2, 0, 1]))
+    d = R[j.long()] - R[i.long()]
+
+    def run(s):
+        if call == "compute":
+            o = s.compute(R)
+            return float(o["energy"].sum()), o["forces"]
+        o = s.graph_eval(i, j, d, i, j, d)
+        return float(o["e_atom"].sum()), o["g_edges"]
+
+    make = lambda: System(Z, None, cutoff_lr=50.0, damping=2.0, lr_format="sparse")
+    ref, raised = run(make()), 0
+    for nth in range(1, 40):
+        s = make()
+        _fail(nth)
+        try:
+            got = [run(s)]
+        except Exception:
+            got, raised = [], raised + 1
+        left = _fail(0)
+        for e, f in got + [run(s), run(s)]:
+            assert abs(e - ref[0]) <= 2e-6 * abs(ref[0])
+            assert float((f - ref[1]).abs().max()) <= 5e-5
+        if left:
+            break
+    assert nth > 7 and raised >= (6 if call == "compute" else 1)
