@@ -459,10 +459,18 @@ int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bo
   SO3LR_CUDA_CHECK(cudaStreamSynchronize(st));
   if (which != 1) rc = nlist_end(S->nws, st, S->cell, &S->sr);
   if (rc) return rc;
-  if (which != 0) rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
+  if (which != 0) {
+    rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
+    // the first list is filled: its votes have served (dev_free waits for the device)
+    if (rc == kCudaError && which != 1 && nlist_drop_votes(S->nws)) rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
+  }
   if (rc) return rc;
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->d_Rref, R_user, (size_t)S->n * 3 * sizeof(float), cudaMemcpyDeviceToDevice, st));
   rc = ensure_edge_buffers(S, S->sr.count);
+  if (rc) {
+    const bool a = nlist_drop_votes(S->nws), b = nlist_drop_votes(S->nws_lr);
+    if (a || b) rc = ensure_edge_buffers(S, S->sr.count);
+  }
   if (rc) return rc;
   S->sr_rows = S->n;
   S->have_lists = true;

@@ -309,6 +309,7 @@ int nlist_row_total(cudaStream_t s, int n, const int* row_count_dev, long long* 
 // entries of a row may come in any order.
 int nlist_begin(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered, const int* seg,
                 const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order);
+bool nlist_drop_votes(NlistWorkspace* ws);      // short of memory: the workspace gives up what it can do without
 int nlist_end(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, NeighborListDev* out);
 int nlist_build(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
                 const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows = -1);

@@ -59,6 +59,14 @@ void nlist_workspace_destroy(NlistWorkspace* w) {
   delete w;
 }
 
+// gives the vote buffer back (its next build asks for it again); false when there is none
+bool nlist_drop_votes(NlistWorkspace* w) {
+  if (!w || !w->masks) return false;
+  dev_free(w->masks);
+  w->masks = nullptr; w->mask_cap = 0;
+  return true;
+}
+
 namespace {
 
 
@@ -533,8 +541,9 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   }
   const int blocks = (n_rows + 7) / 8;
   if (n_rows == 0) { out->count = 0; return kOk; }
-  // votes of the count for the fill: room for 1.25 times the mean number of candidates of a row (and one partial word per range); 0.8 KB
-  // per atom for the 12 A list of water.  Short of memory the fill tests the candidates again.
+  // votes of the count for the fill: room for 1.25 times the candidates of 27 cells (an atom in the middle of its cell has all of them
+  // within the radius, also where cells are left out) and one partial word per range; for the 13 A list of water (12 A and the skin)
+  // 269 words, 1.1 KB per atom.  Short of memory they are given back (see nlist_end) and the fill tests the candidates again.
   unsigned* masks = nullptr;
   int mask_stride = 0;
   if (!by_graph) {
@@ -581,7 +590,6 @@ int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListD
   if (n_rows <= 0) return kOk;
   const int blocks = (n_rows + 7) / 8, allow_grow = w->allow_grow;
   const float r2max = w->r_list * w->r_list;
-  w->n_rows = 0;
   const long long total = *w->h_total;
   if (total < 0) return kNotFinite;
   if (total > 2147483000LL) return kTooLarge;
@@ -593,11 +601,16 @@ int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListD
       if (out->nbr_j) dev_free(out->nbr_j);
       if (out->edge_i) dev_free(out->edge_i);
       out->nbr_j = nullptr; out->edge_i = nullptr; out->capacity = 0; out->count = 0;
-      SO3LR_CUDA_CHECK(dev_alloc(&out->nbr_j, (size_t)cap));
-      SO3LR_CUDA_CHECK(dev_alloc(&out->edge_i, (size_t)cap));
+      // the list itself goes before the votes
+      for (int** p : {&out->nbr_j, &out->edge_i})
+        if (dev_alloc(p, (size_t)cap) != cudaSuccess) {
+          if (!nlist_drop_votes(w)) return kCudaError;
+          SO3LR_CUDA_CHECK(dev_alloc(p, (size_t)cap));
+        }
       out->capacity = cap;
     }
   }
+  w->n_rows = 0;      // not before: a call that found no memory may be repeated
   if (total <= out->capacity) out->count = total;
   const bool truncated = total > out->capacity;
   if (w->by_graph)

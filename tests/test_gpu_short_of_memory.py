@@ -62,6 +62,8 @@ def test_lists_that_grow(skin, persistent):
 
     made, raised = _attempts(call, lambda o: _close(o, ref), persistent)
     assert made >= 6, made
+    # one array that finds no memory gets the place of the builder's votes, which the fill can do without
+    assert raised == 0 or persistent
 
 
 @pytest.mark.parametrize("persistent", [False, True])
