@@ -82,25 +82,31 @@ __global__ void fill_kernel(float* p, size_t n, float v) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
-// several arrays set to zero in one launch
+// several arrays set to zero in one launch; more of them than there is room for are refused by launch_clear
 struct ClearArgs {
-  static constexpr int kMax = 10;
+  static constexpr int kMax = 12;
   float* p[kMax];
   long long n[kMax];
-  int count = 0;
-  void add(void* q, long long words) { if (q && words > 0) { p[count] = static_cast<float*>(q); n[count++] = words; } }
+  int count = 0;      // arrays asked for
+  void add(void* q, long long words) {
+    if (!q || words <= 0) return;
+    if (count < kMax) { p[count] = static_cast<float*>(q); n[count] = words; }
+    ++count;
+  }
 };
 __global__ void __launch_bounds__(256) clear_kernel(ClearArgs A) {
   grid_dep_sync();
   for (int k = 0; k < A.count; ++k)
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < A.n[k]; i += (long long)gridDim.x * 256) A.p[k][i] = 0.f;
 }
-void launch_clear(cudaStream_t s, const ClearArgs& A) {
+int launch_clear(cudaStream_t s, const ClearArgs& A) {
+  if (A.count > ClearArgs::kMax) return kInvalidArgument;
   long long most = 0;
   for (int k = 0; k < A.count; ++k) most = std::max(most, A.n[k]);
-  if (most <= 0) return;
+  if (most <= 0) return kOk;
   const int blocks = (int)std::min<long long>(8LL * sm_count(), (most + 255) / 256);
   { launch_chained(clear_kernel, blocks, 256, 0, s, A); count_launch(); }
+  return kOk;
 }
 __global__ void combine_energy_kernel(int n, const float* e_nn, const float* e_zbl, const float* e_c, const float* e_d, float* e_atom) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -633,7 +639,7 @@ int evaluate_graph(so3lr_b200_system* S, cudaStream_t st, const int* row_ptr, co
   A.add(S->e_zbl, n); A.add(S->e_coul, n); A.add(S->e_disp, n); A.add(S->gq, n); A.add(S->gh, n); A.add(S->gev_a, (long long)n * kMTot);
   if (tiled) { A.add(asym, 1); A.add(S->ve.total, 1); }
   if (gq_preset) A.add(S->g_qkv, (long long)n * kProj);
-  launch_clear(st, A);
+  if (int rcc = launch_clear(st, A)) return rcc;
   if (tiled) {
     int rcv = valid_edges_build(&S->ve, st, n, n, row_ptr, nbr_j, dR, asym, n_edges, true);
     if (rcv) return rcv;
@@ -785,7 +791,7 @@ int fused_forward(so3lr_b200_system* S, cudaStream_t st, const float* R, const S
     A.add(S->gev_a, (long long)c.n0 * kMTot);
     A.add(S->ve.total, 1);
     if (small_presets(c.n0)) A.add(S->g_qkv, (long long)c.n3 * kProj);
-    launch_clear(st, A);
+    if (int rcc = launch_clear(st, A)) return rcc;
   }
   S->prof.begin(kPGeom, st);
   launch_sr_geometry_zbl(st, M, S->cell, c.n3, S->sr.count, edge_i, nbr_j, S->d_Z, R, 0, S->dR, S->e_zbl, nullptr, nullptr, F,

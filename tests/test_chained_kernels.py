@@ -43,6 +43,15 @@ def test_non_coherent_loads_are_of_weights(source):
         assert arg.startswith(("L.", "M.")) or arg in {"const", "W", "p", "bias", "fin"}, arg
 
 
+def test_one_clearing_launch_holds_all_its_arrays():
+    """The arrays travel in an object of fixed size that is passed by value: one too many must not be written behind its end."""
+    s = SOURCES["engine.cu"]
+    room = int(re.search(r"struct ClearArgs \{.*?kMax = (\d+);", s, re.S).group(1))
+    assert "if (count < kMax)" in re.search(r"struct ClearArgs \{.*?\n\};", s, re.S).group(0)
+    uses = re.findall(r"ClearArgs A;(.*?)if \(int rcc = launch_clear\(st, A\)\) return rcc;", s, re.S)
+    assert len(uses) == len(re.findall(r"ClearArgs A;", s)) and all(0 < u.count("A.add(") <= room for u in uses)
+
+
 def test_statuses_of_the_attention_launches_are_looked_at():
     """They refuse a list that was compacted for other rows; an evaluation that went on would hold no attention sums."""
     calls = re.findall(r"([^;{}]*?)\b((?:launch_attn_\w+_tc\w*|attn_\w+_dispatch)\()", SOURCES["engine.cu"])
