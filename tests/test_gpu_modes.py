@@ -2,7 +2,8 @@
 the attention kernels, the dense blocks and the first layer gives the same energies and forces as the default build-up.
 
   SO3LR_B200_ATTENTION = tcf | mma | simt  (default: tiled tcgen05 kernels in both directions)
-  SO3LR_B200_DENSE     = mma | simt        (default: tcgen05 post-attention blocks and heads)
+  SO3LR_B200_DENSE     = tc | mma | simt   (default: tcgen05 post-attention blocks and heads; up to 16 atoms per SM the FP32 blocks of
+                                            short lists, for which tc keeps the tcgen05 ones)
   SO3LR_B200_LAYER0    = generic           (default: per-element-pair tables)
 """
 import os
@@ -48,7 +49,7 @@ def _run(tmp_path, name, env):
 def test_kernel_variants_agree(tmp_path):
     ref = _run(tmp_path, "default", {})
     variants = {"attention_tcf": {"SO3LR_B200_ATTENTION": "tcf"}, "attention_mma": {"SO3LR_B200_ATTENTION": "mma"},
-                "attention_simt": {"SO3LR_B200_ATTENTION": "simt"}, "dense_mma": {"SO3LR_B200_DENSE": "mma"},
+                "attention_simt": {"SO3LR_B200_ATTENTION": "simt"}, "dense_tc": {"SO3LR_B200_DENSE": "tc"}, "dense_mma": {"SO3LR_B200_DENSE": "mma"},
                 "dense_simt": {"SO3LR_B200_DENSE": "simt"},
                 "layer0_generic": {"SO3LR_B200_LAYER0": "generic"}}
     for name, env in variants.items():
@@ -58,6 +59,36 @@ def test_kernel_variants_agree(tmp_path):
         for k in ("F_w", "F_m"):
             assert np.abs(got[k] - ref[k]).max() <= 5e-5, (name, k, np.abs(got[k] - ref[k]).max())
         assert np.abs(got["W_w"] - ref["W_w"]).max() <= 2e-4 * np.abs(ref["W_w"]).max(), name
+
+
+def test_tensor_core_blocks_against_the_oracle(tmp_path):
+    """csrc/dense_tc.cu on structures of the oracle's size, which take the blocks of short lists by default.  Tolerances of the parity tests."""
+    from oracle import so3lr_oracle as O
+    from so3lr_b200 import workloads as W
+    got = _run(tmp_path, "tc", {"SO3LR_B200_DENSE": "tc"})
+    g = np.load(ROOT + "/tests/golden/reference_goldens.npz")
+    Z, R, cell = W.water_box(216, 18.7, 5)
+    f32 = lambda a: np.asarray(a, dtype=np.float32).astype(np.float64)
+    for k, z, r, box, cut in (("w", Z, R, f32(cell), 9.0), ("m", g["bb_Z"], g["bb_R"] - g["bb_R"].mean(0), None, 12.0)):
+        ref = O.energy_forces(O.load_params(), f32(r), z, box, cutoff_lr=cut, damping=2.0)
+        assert abs(float(got["E_" + k].astype(np.float64).sum()) - ref["energy"]) <= 1e-5 * abs(ref["energy"]), k
+        assert np.abs(got["F_" + k] - ref["forces"]).max() <= 1e-4, (k, np.abs(got["F_" + k] - ref["forces"]).max())
+
+
+def test_long_lists_against_the_oracle():
+    """2,700 atoms: the tensor-core blocks by default and full attention tiles, in the positions -> forces call with a skin."""
+    import torch
+    from oracle import so3lr_oracle as O
+    from so3lr_b200 import workloads as W
+    from so3lr_b200.engine import System
+    Z, R, cell = W.water_box(900, (900 * 29.9) ** (1 / 3), 3)
+    assert len(Z) > 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    R, cell = np.asarray(R, dtype=np.float32), np.asarray(cell, dtype=np.float32).astype(np.float64)
+    ref = O.energy_forces(O.load_params(), R.astype(np.float64), Z, cell, cutoff_lr=6.0, damping=2.0)
+    o = System(Z, cell, cutoff_lr=6.0, damping=2.0, skin=0.5).compute(torch.tensor(R, device="cuda"))
+    assert abs(float(o["energy"].double().sum()) - ref["energy"]) <= 1e-5 * abs(ref["energy"])
+    dF = np.abs(o["forces"].cpu().numpy() - ref["forces"]).max()
+    assert dF <= 1e-4, dF
 
 
 GRAPH_CHILD = r"""

@@ -67,6 +67,25 @@ def test_list_forms_against_the_oracle(name, form):
         _check(o, e, g, i, j, D.detach(), n, form)
 
 
+@pytest.mark.parametrize("name,rounds", [("water300", 1), ("water600", 2), ("water900", 3)])
+def test_full_tiles_against_the_oracle(name, rounds):
+    """Tiles of 128 pairs, what every long list runs: 16 warps with a share of 8 pairs each, in one round over the SMs and in several.  The
+    lists above have shares of 1 to 5 (16 n pairs fill the share of n on every SM).  2,700 atoms take the tensor-core dense blocks."""
+    from oracle import so3lr_oracle as O
+    from so3lr_b200.engine import System
+    Z, cell, (i, j, d), (il, jl, dl) = _lists(name, "plain")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    pairs = len(i) // 2
+    assert -(-pairs // (128 * sms)) == rounds and -(-pairs // (16 * sms * rounds)) == 8
+    s = System(Z, cell, cutoff_lr=6.0, damping=2.0, lr_format="sparse")
+    t = lambda a: torch.tensor(a, device="cuda")
+    o = s.graph_eval(t(i), t(j), t(d), t(il), t(jl), t(dl))
+    D, DL = torch.tensor(d, dtype=torch.float64, requires_grad=True), torch.tensor(dl, dtype=torch.float64)
+    e, _ = O.energy_from_graph(O.load_params(), Z, D, i, j, DL, il, jl, lr_format="sparse", cutoff_lr=6.0, damping=2.0)
+    g, = torch.autograd.grad(e.sum(), D)
+    _check(o, e.detach(), g, i, j, D.detach(), len(Z), "plain")
+
+
 def _check(o, e, g, i, j, D, n, form):
     got = o["g_edges"].double().cpu()
     assert float((o["e_atom"].double().cpu() - e).abs().sum()) <= 1e-5 * float(e.abs().sum())
