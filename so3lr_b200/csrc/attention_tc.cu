@@ -399,7 +399,10 @@ __device__ __forceinline__ bool edge_valid(int j, int n, float dx, float dy, flo
 // do once the rows exceed the L2: at 98,304 atoms the attention kernels lose 8 % / 3 % (forward / reverse).  Long lists therefore take
 // two passes (kCount, kFill) around a scan of the CTAs' counts, which keep the rows in order.
 constexpr int kCompactRows = 16;
-constexpr int kOrderedRows = 8192;      // from here on: 0.1 GB of q / k / v and cotangent rows
+// The line: a force evaluation of water (6 A long range) in order / in order of arrival takes 404 / 400 us at 1,536 atoms, 964 / 963 at
+// 6,144, 1,125 / 1,125 at 8,193, 1,498 / 1,497 at 12,288, 2,857 / 2,879 at 24,576, 5,275 / 5,363 at 49,152, 10,242 / 10,530 at 98,304: the
+// two launches more cost 4 us where launches bind, nothing from 6,000 atoms on, and the order pays from about 16,000.
+constexpr int kOrderedRows = 8192;
 enum CompactPass { kReserve, kCount, kFill };
 template <int PASS>
 __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_rows, int n, const int* __restrict__ row_ptr,

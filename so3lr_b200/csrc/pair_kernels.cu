@@ -444,7 +444,10 @@ __global__ void graph_reduce_kernel(int n_graphs, const int* __restrict__ graph_
 
 // ---- one structure with many atoms: the same three operations spread over many CTAs (sums in double, fixed order) ----
 constexpr int kWideBlocks = 296;      // two CTAs per SM of a 148-SM part; a fixed count keeps the order of the double sums independent of the device
-constexpr int kWideMinAtoms = 4096;      // one CTA takes 23 to 28 us for 12,000 atoms, the two wide launches 6
+// One CTA takes 23 to 28 us for 12,000 atoms, the two wide launches 6.  The three sums of an evaluation (water, 6 A long range) wide / in
+// one CTA: 216 / 208 us at 192 atoms, 284 / 280 at 768, 401 / 403 at 1,536, 688 / 694 at 3,072, 794 / 801 at 4,095, 967 / 986 at 6,144,
+// 1,485 / 1,546 at 12,288.  They meet near 1,500 atoms; up to the line the one CTA costs 7 us (1 %) and is one launch less.
+constexpr int kWideMinAtoms = 4096;
 
 __device__ double block_sum_double_256(double v, double* sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
