@@ -8,7 +8,7 @@
 // indices -- the padding of a list, a quarter of it, points at one atom -- and took 54 ms per call at 1,536 atoms (0.8 M entries)
 // and 965 ms at 24,000 (12 M): the whole step 56.3 and 1,048 ms.  Here entries with a zero gradient are skipped, the receiver's
 // share is summed over runs of equal indices inside a warp (lists come grouped by receiver) and every other share is one 16-byte
-// vector reduction: the step takes 2.15 and 8.8 ms.
+// vector reduction: the step takes 1.5 and 5.0 ms.
 #include <algorithm>
 
 #include "kernels.h"
