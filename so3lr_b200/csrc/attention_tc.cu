@@ -73,7 +73,8 @@ constexpr int kSmemFwd = kOffFwStEv + TE * 2 * kEvStride * 4;
 constexpr int kOffBwW = kOffA + kARegion;
 constexpr int kOffBwRec = kOffBwW + 64 * kWStride * 4;
 constexpr int kOffBwSph = kOffBwRec + TE * kBwRec * 4;
-constexpr int kOffBwMisc = kOffBwSph + 512 * 4;
+constexpr int kBwSphFloats = 4 * 136;         // reverse kernel: first spherical layer, 8 floats per hidden unit, 8 more after every 16 units (banks)
+constexpr int kOffBwMisc = kOffBwSph + kBwSphFloats * 4;
 constexpr int kOffBwStIJ = kOffBwMisc + 64;                  // staged inputs of the next tile: (i, j) | displacement
 constexpr int kOffBwStD = kOffBwStIJ + TE * 8;
 constexpr int kSmemBwd = kOffBwStD + TE * 16;
@@ -157,6 +158,35 @@ __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t b
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// The same for a whole warp that runs the issue code: `on` is set in one lane, which issues.  Descriptors then are the same in all lanes and
+// stay in uniform registers: 43 cycles from one MMA to the next instead of 53 where a single thread has branched off.
+__device__ __forceinline__ void umma_if(uint32_t on, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t on, uint32_t mbar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(mbar), "r"(on) : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n" : "=r"(on));
+  return on;
+}
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
@@ -187,6 +217,12 @@ __device__ __forceinline__ void red_add_v4(float* p, float4 v) {
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Every thread that goes on to read what the MMAs left waits for itself.  After a wait that ran out the CTA's later ones return at once:
+// the kernel carries on to its end with an error word set.
+__device__ __forceinline__ void wait_mma(uint32_t mbar, uint32_t parity, volatile int* failed, int* err) {
+  if (!*failed && !mbar_wait(mbar, parity)) { *failed = 1; atomicExch(err, 1); }
+  tc_fence_after();
+}
 
 // main + cross / 2048 of 32 columns (cross accumulators sit 256 columns above the main ones)
 __device__ __forceinline__ void tmem_ld32_combined(uint32_t taddr, float* v) {
@@ -297,6 +333,25 @@ __device__ __forceinline__ void store_spherical_hidden_f(unsigned char* a_hi, in
   }
 }
 
+// first-layer weights of hidden unit u of filter f in the reverse kernel's shared memory
+__device__ __forceinline__ int sph_at(int f, int u) { return (f * 32 + u) * 8 + (2 * f + (u >> 4)) * 8; }
+// One of four neighbouring threads of a pair: two of the eight chunks of both hidden layers
+__device__ __forceinline__ void store_spherical_hidden_quarter(unsigned char* a_hi, int row, const float* s, const float* sph, int quarter) {
+  const float* base = sph + sph_at(quarter >> 1, 16 * (quarter & 1));
+#pragma unroll
+  for (int c8 = 0; c8 < 2; ++c8) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float* p = base + (8 * c8 + q) * 8;
+      const float4 k = ld4(p);
+      const float z = fmaf(s[0], k.x, fmaf(s[1], k.y, fmaf(s[2], k.z, fmaf(s[3], k.w, p[4]))));
+      v[q] = __fdividef(z, 1.f + __expf(-z));
+    }
+    store_chunk(a_hi, 8 + 2 * quarter + c8, row, v);
+  }
+}
+
 // Descriptors differ only in their start-address field (bits 0..13, in units of 16 bytes): desc(addr) = base + (addr >> 4).
 // The issuing thread keeps everything in registers -- shared-memory loads inside the issue loop wait behind the operand
 // traffic of the MMAs already running and throttle the chain.
@@ -351,22 +406,25 @@ __device__ __noinline__ void issue_forward_mma(uint32_t tmem, uint32_t a_hi, uin
 // Forward product (B read MN-major: N = features, K = rows): w_f = [Phi | hs_f] * [C_f ; K2_f], main accumulators in TMEM
 // columns [128 f, 128 f + 128), cross 256 columns above.
 constexpr int kRevImgFilter = 16 * 1536;
-// part 0: the four Chebyshev steps, part 1: the two steps of the filter's hidden layer (see issue_forward_mma)
-__device__ __noinline__ void issue_filter_mma(uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int part) {
+// part 0: the four Chebyshev steps, part 1: the two steps of the filter's hidden layer (see issue_forward_mma).  Four warps share the work, one
+// per filter and accumulator (`cross`: hi * lo + lo * hi): the issue of a chain waits behind the load / store queue of its scheduler.
+__device__ __forceinline__ void issue_filter_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int cross, int part) {
   const uint64_t da = desc_base(kLboA, 128) + (a_hi >> 4), dal = da + (kAHalf >> 4);
   const uint64_t db = desc_base(128, 1536) + ((img + f * kRevImgFilter) >> 4), dbl = db + (2 * kRevImgFilter >> 4);
   const uint32_t id128 = make_idesc(128, 1);
-  const uint32_t d_main = tmem + 128 * f, d_cross = d_main + 256;
+  const uint32_t d = tmem + 128 * f + 256 * cross;
 #pragma unroll
   for (int ks = 0; ks < 6; ++ks) {      // K = 16 rows per step: Chebyshev chunks 0..7 of A, then the two chunks pairs of hs_f
     if ((ks >= 4) != (part == 1)) continue;
     const int chunk = ks < 4 ? 2 * ks : 8 + 4 * f + 2 * (ks - 4);
     const uint64_t ah = da + chunk * (kLboA >> 4), al = dal + chunk * (kLboA >> 4);
     const uint64_t bh = db + ks * (2 * 128 >> 4), bl = dbl + ks * (2 * 128 >> 4);
-    umma(d_main, ah, bh, id128, ks > 0);
-    if (ks == 1 || ks == 3) continue;      // Chebyshev terms of order >= 32: no cross terms (see issue_forward_mma)
-    umma(d_cross, ah, bl, id128, ks > 0);
-    umma(d_cross, al, bh, id128, 1);
+    if (!cross) {
+      umma_if(on, d, ah, bh, id128, ks > 0);
+    } else if (ks != 1 && ks != 3) {      // Chebyshev terms of order >= 32: no cross terms (see issue_forward_mma)
+      umma_if(on, d, ah, bl, id128, ks > 0);
+      umma_if(on, d, al, bh, id128, 1);
+    }
   }
 }
 
@@ -878,21 +936,30 @@ namespace {
 // 28-30 unit vector | 31 1/r | 32 d/dr | 33 r | 34 1 for a list entry, 0 for a padding row
 // [dPhi | dhs_f] = dw_f * [C_f^T | K2_f^T] (the same image read K-major: N = 96 rows, K = features): main accumulators in TMEM
 // columns [128 f, 128 f + 96), cross 256 columns above
-__device__ __noinline__ void issue_reverse_mma(uint32_t tmem, uint32_t a_hi, uint32_t img, int f) {
+__device__ __forceinline__ void issue_reverse_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int cross) {
   const uint64_t da = desc_base(kLboA, 128) + (a_hi >> 4), dal = da + (kAHalf >> 4);
   const uint64_t db = desc_base(1536, 128) + ((img + f * kRevImgFilter) >> 4), dbl = db + (2 * kRevImgFilter >> 4);
   const uint32_t id96 = make_idesc(96, 0);
-  const uint32_t d_main = tmem + 128 * f, d_cross = d_main + 256;
+  const uint32_t d = tmem + 128 * f + 256 * cross;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {      // K = 16 features per step
     const uint64_t ah = da + ks * (2 * kLboA >> 4), al = dal + ks * (2 * kLboA >> 4);
     const uint64_t bh = db + ks * (2 * 1536 >> 4), bl = dbl + ks * (2 * 1536 >> 4);
-    umma(d_main, ah, bh, id96, ks > 0);
-    umma(d_cross, ah, bl, id96, ks > 0);
-    umma(d_cross, al, bh, id96, 1);
+    if (!cross) {
+      umma_if(on, d, ah, bh, id96, ks > 0);
+    } else {
+      umma_if(on, d, ah, bl, id96, ks > 0);
+      umma_if(on, d, al, bh, id96, 1);
+    }
   }
 }
 
+// A warp owns up to eight consecutive pairs of a tile: the first nu0 <= 4 sit in rows [nu0 warp, nu0 warp + nu0), the others in rows
+// [64 + nu1 warp, 64 + nu1 warp + nu1): the filter tile holds 64 rows at a time.
+struct WarpRows {
+  int nu0, nu1, row0, row1;
+  __device__ __forceinline__ int row(int k) const { return k < nu0 ? row0 + k : row1 + (k - nu0); }
+};
 // Sender-side q / k rows of four consecutive tile rows for the reverse edge loop of filter F (lane = 4 features)
 // (for every row of the four: past a warp's share these are rows of other warps, whose values are not used)
 struct RevLoads {
@@ -903,7 +970,7 @@ __device__ __forceinline__ void reverse_prefetch(RevLoads& L, const float* rec, 
   const int col = 4 * lane;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const float* pj = qkv + (size_t)__float_as_int(rec[(row0 + u) * kBwRec]) * kProj + F * 3 * kF;
+    const float* pj = qkv + (size_t)__float_as_int(rec[((row0 + u) & (TE - 1)) * kBwRec]) * kProj + F * 3 * kF;
     L.qj[u] = ld4(pj + col);
     L.kj[u] = ld4(pj + kF + col);
   }
@@ -913,10 +980,10 @@ __device__ __forceinline__ void reverse_prefetch(RevLoads& L, const float* rec, 
 }
 
 // Value path of the invariant filter, split off the edge loop so that it runs while the tensor cores are busy.
-// Before the loop (rows [row0, row0 + nu), nu <= 8, of one warp): cotangents of the invariant logits of both directions of every edge,
-// daA_h = <g_xa[i], v[j]>_h and daB_h = <g_xa[j], v[i]>_h, into record fields 36..39 and 40..43.
+// Before the loop (the nu = nu0 + nu1 pairs of one warp): cotangents of the invariant logits of both directions of every edge,
+// daA_h = <g_xa[i], v[j]>_h and daB_h = <g_xa[j], v[i]>_h, into record fields 24..27 and 28..31.
 template <bool FULL>
-__device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int nu, int lane, const float* __restrict__ qkv,
+__device__ __forceinline__ void value_logit_cotangents(float* rec, const WarpRows& R, int nu, int lane, const float* __restrict__ qkv,
                                                        const float* __restrict__ g_xa) {
   const int col = 4 * lane, grp = lane >> 3, cg = lane & 7;
   int cur_i = -1;
@@ -927,7 +994,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
     int ii[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const float* rp = rec + ((row0 + k0 + u) & (TE - 1)) * kBwRec;
+      const float* rp = rec + ((FULL ? (k0 ? R.row1 : R.row0) + u : R.row(k0 + u)) & (TE - 1)) * kBwRec;
       const int j = __float_as_int(rp[0]);
       ii[u] = __float_as_int(rp[1]);
       vj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
@@ -942,7 +1009,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
       float v[8];
 #pragma unroll
       for (int u = 0; u < 4; ++u) { v[2 * u] = dot2(gx_i, vj[u]); v[2 * u + 1] = dot2(gxj[u], v_i); }
-      rec[(row0 + k0 + (cg >> 1)) * kBwRec + 36 + 4 * (cg & 1) + grp] = transpose_sum8(v, cg);
+      rec[((k0 ? R.row1 : R.row0) + (cg >> 1)) * kBwRec + 24 + 4 * (cg & 1) + grp] = transpose_sum8(v, cg);
       continue;
     }
 #pragma unroll
@@ -955,54 +1022,73 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int
       }
       const float daA = group8_sum(dot2(gx_i, vj[u])), daB = group8_sum(dot2(gxj[u], v_i));
       if (cg == 0) {
-        float* rp = rec + (row0 + k0 + u) * kBwRec;
-        rp[36 + grp] = daA;
-        rp[40 + grp] = daB;
+        float* rp = rec + R.row(k0 + u) * kBwRec;
+        rp[24 + grp] = daA;
+        rp[28 + grp] = daB;
       }
     }
   }
 }
-constexpr int kAngOff = 4 * 4 * TE + 4 * TE;      // floats: behind the invariants' and radial shares of the last phase
-static_assert((kAngOff + 4 * 4 * TE) <= 64 * kWStride, "shares of the last phase fit the filter tile");
-// share of degree L in the angular part of the force on the receiver: logits x cutoff of both directions (record fields 20.. and 24..)
-// times the cotangents of both atoms' ev, through the transpose of the harmonics
+
+// two unit vectors that span the plane across u, without a branch at either pole (Duff et al., J. Comput. Graph. Tech. 6, 2017)
+__device__ __forceinline__ void tangent_frame(float ux, float uy, float uz, float* e1, float* e2) {
+  const float s = copysignf(1.f, uz), a = -1.f / (s + uz), b = ux * uy * a;
+  e1[0] = fmaf(s * ux * ux, a, 1.f); e1[1] = s * b; e1[2] = -s * ux;
+  e2[0] = b; e2[1] = fmaf(uy * uy, a, s); e2[2] = -uy;
+}
+// What one end's cotangent of ev contributes to a pair, ahead of the logits: dl[l] = sum_m g_lm Y_lm (cotangent of the equivariant logit)
+// and, per degree, the two components across the pair of the transposed harmonics (field + 2 l of the record): the angular force is
+// their sum weighted with the logits.
 template <int L>
-__device__ __forceinline__ float4 angular_share(const float* rp, const float* __restrict__ gev1) {
-  if (rp[34] == 0.f) return f4_zero();
-  constexpr int m0 = L * L - 1;      // first component of the degree: 0, 3, 8, 15
-  const float* gi = gev1 + (size_t)__float_as_int(rp[1]) * kMTot + m0;
-  const float* gj = gev1 + (size_t)__float_as_int(rp[0]) * kMTot + m0;
-  float a[2 * L + 1], b[2 * L + 1];
+__device__ __forceinline__ void angular_degree(const float* g, const float* Y, const float* u, const float* e1, const float* e2, float sign,
+                                               float* dl, float* t) {
+  constexpr int m0 = L * L - 1;
+  float d = 0.f;
 #pragma unroll
-  for (int m = 0; m < 2 * L + 1; ++m) { a[m] = gi[m]; b[m] = gj[m]; }
-  const float aA = rp[19 + L], aB = (L & 1) ? -rp[23 + L] : rp[23 + L];      // Y_lm(-u) = (-1)^l Y_lm(u)
-  const float4 uu = ld4(rp + 28);
-#pragma unroll
-  for (int m = 0; m < 2 * L + 1; ++m) a[m] = aA * a[m] + aB * b[m];
+  for (int m = 0; m < 2 * L + 1; ++m) d = fmaf(g[m0 + m], Y[m0 + m], d);
   float gx = 0.f, gy = 0.f, gz = 0.f;
-  sph_harm_vjp_degree<L>(uu.x, uu.y, uu.z, a, gx, gy, gz);
-  const float gd = gx * uu.x + gy * uu.y + gz * uu.z;
-  return make_float4((gx - gd * uu.x) * uu.w, (gy - gd * uu.y) * uu.w, (gz - gd * uu.z) * uu.w, 0.f);
+  sph_harm_vjp_degree<L>(u[0], u[1], u[2], g + m0, gx, gy, gz);
+  dl[L - 1] = sign * d;
+  t[2 * (L - 1)] = sign * fmaf(gx, e1[0], fmaf(gy, e1[1], gz * e1[2]));
+  t[2 * (L - 1) + 1] = sign * fmaf(gx, e2[0], fmaf(gy, e2[1], gz * e2[2]));
+}
+// `odd`: sign of the odd degrees, Y_lm(-u) = (-1)^l Y_lm(u)
+__device__ __forceinline__ void angular_end(const float* __restrict__ gev, float ux, float uy, float uz, float odd, float* rp_dl, float* rp_t) {
+  float g[kMTot];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) st4(g + 4 * c, ld4(gev + 4 * c));
+  const float u[3] = {ux, uy, uz};
+  float Y[kMTot], e1[3], e2[3], dl[4], t[8];
+  sph_harm_24(ux, uy, uz, Y);
+  tangent_frame(ux, uy, uz, e1, e2);
+  angular_degree<1>(g, Y, u, e1, e2, odd, dl, t);
+  angular_degree<2>(g, Y, u, e1, e2, 1.f, dl, t);
+  angular_degree<3>(g, Y, u, e1, e2, odd, dl, t);
+  angular_degree<4>(g, Y, u, e1, e2, 1.f, dl, t);
+  st4(rp_dl, make_float4(dl[0], dl[1], dl[2], dl[3]));
+  st4(rp_t, make_float4(t[0], t[1], t[2], t[3]));
+  st4(rp_t + 4, make_float4(t[4], t[5], t[6], t[7]));
 }
 
-// After the loop: cotangents of the value rows, gv_i = sum over its pairs (cutoff x logit of edge j<-i)_h g_xa[j] (fields 44..47) and,
-// pair by pair, gv_j += (cutoff x logit of edge i<-j)_h g_xa[i] (fields 48..51)
+// After the loop: cotangents of the value rows, gv_i = sum over its pairs (cutoff x logit of edge j<-i)_h g_xa[j] (fields 28..31) and,
+// pair by pair, gv_j += (cutoff x logit of edge i<-j)_h g_xa[i] (fields 24..27)
 template <bool FULL>
-__device__ __forceinline__ void value_cotangent(const float* rec, int row0, int nu, int lane, const float* __restrict__ g_xa,
+__device__ __forceinline__ void value_cotangent(const float* rec, const WarpRows& R, int nu, int lane, const float* __restrict__ g_xa,
                                                 float* __restrict__ g_qkv, int n_scat) {
   const int col = 4 * lane, grp = lane >> 3;
+  auto record = [&](int k) { return rec + ((FULL ? (k < 4 ? R.row0 + k : R.row1 + k - 4) : R.row(k)) & (TE - 1)) * kBwRec; };
   float4 gxj[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) gxj[u] = ld4(g_xa + (size_t)__float_as_int(rec[((row0 + u) & (TE - 1)) * kBwRec]) * kF + col);
-  int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
+  for (int u = 0; u < 8; ++u) gxj[u] = ld4(g_xa + (size_t)__float_as_int(record(u)[0]) * kF + col);
+  int cur_i = __float_as_int(record(0)[1]);
   float4 gv = f4_zero(), gxi = ld4(g_xa + (size_t)cur_i * kF + col);
-  if (FULL && cur_i == __float_as_int(rec[(row0 + 7) * kBwRec + 1])) {      // eight pairs of one receiver
+  if (FULL && cur_i == __float_as_int(record(7)[1])) {      // eight pairs of one receiver
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const float* rp = rec + (row0 + u) * kBwRec;
+      const float* rp = record(u);
       const int j = __float_as_int(rp[0]);
-      gv = f4_fma(rp[44 + grp], gxj[u], gv);
-      if (j < n_scat) red_add_v4(g_qkv + (size_t)j * kProj + 2 * kF + col, f4_scale(rp[48 + grp], gxi));
+      gv = f4_fma(rp[28 + grp], gxj[u], gv);
+      if (j < n_scat) red_add_v4(g_qkv + (size_t)j * kProj + 2 * kF + col, f4_scale(rp[24 + grp], gxi));
     }
     red_add_v4(g_qkv + (size_t)cur_i * kProj + 2 * kF + col, gv);
     return;
@@ -1010,7 +1096,7 @@ __device__ __forceinline__ void value_cotangent(const float* rec, int row0, int 
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     if (!FULL && u >= nu) break;
-    const float* rp = rec + (row0 + u) * kBwRec;
+    const float* rp = record(u);
     const float4 r0 = ld4(rp);
     const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
     if (i != cur_i) {
@@ -1019,24 +1105,48 @@ __device__ __forceinline__ void value_cotangent(const float* rec, int row0, int 
       gv = f4_zero();
       gxi = ld4(g_xa + (size_t)cur_i * kF + col);
     }
-    gv = f4_fma(rp[44 + grp], gxj[u], gv);
-    if (j < n_scat && r0.z != 0.f) red_add_v4(g_qkv + (size_t)j * kProj + 2 * kF + col, f4_scale(rp[48 + grp], gxi));
+    gv = f4_fma(rp[28 + grp], gxj[u], gv);
+    if (j < n_scat && r0.z != 0.f) red_add_v4(g_qkv + (size_t)j * kProj + 2 * kF + col, f4_scale(rp[24 + grp], gxi));
   }
   if (f4_nonzero(gv)) red_add_v4(g_qkv + (size_t)cur_i * kProj + 2 * kF + col, gv);
 }
 
+// dw of one pair as A operand of the second MMA chain: row = pair, columns 4 lane .. 4 lane + 3 of the hi and the lo matrix
+__device__ __forceinline__ void store_dw(unsigned char* a_hi, int row, int lane, float4 dw) {
+  uint2 h, l;
+  split2(dw.x, dw.y, h.x, l.x); split2(dw.z, dw.w, h.y, l.y);
+  unsigned char* p = a_hi + (lane >> 1) * kLboA + row * 16 + (lane & 1) * 8;
+  *reinterpret_cast<uint2*>(p) = h;
+  *reinterpret_cast<uint2*>(p + kAHalf) = l;
+}
+// Sums of the receiver's q / k rows that a warp carries from one call of the edge loop to the next
+struct RevSums {
+  float4 gq, gk;
+  int i;
+  template <int F>
+  __device__ __forceinline__ void flush(int lane, float* __restrict__ g_qkv) const {
+    float* gi = g_qkv + (size_t)i * kProj + F * 3 * kF + 4 * lane;
+    if (f4_nonzero(gq)) red_add_v4(gi, gq);
+    if (f4_nonzero(gk)) red_add_v4(gi + kF, gk);
+  }
+  __device__ __forceinline__ void start(int receiver) { i = receiver; gq = f4_zero(); gk = f4_zero(); }
+};
 // Reverse edge loop of filter F over nu <= 4 tile rows [row0, row0 + nu) of one warp: logits of both directions of every edge,
 // cotangents of this receiver's q / k rows (added to g_qkv with vector reductions when the receiver changes), dw into the
 // A operand of the second MMA chain, the cutoff part of d/dr into the records.  The cotangents of the logits come from the
-// records (fields 36.. for the invariant filter, 12.. for the equivariant one); cutoff x logit goes back (44.. / 20.., 24..).
+// records (fields 24.. for the invariant filter, 16.. for the equivariant one); cutoff x logit takes their place.
 template <int F, bool FULL>
-__device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, const float* wt, int wrow0, int row0, int nu, unsigned char* a_hi,
-                                               int lane, const float* __restrict__ qkv, float* __restrict__ g_qkv, int n_scat) {
+__device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, float* rec, const float* wt, int wrow0, int row0, int nu,
+                                               unsigned char* a_hi, int lane, const float* __restrict__ qkv, float* __restrict__ g_qkv, int n_scat) {
+  constexpr int kField = F ? 16 : 24;
   const int col = 4 * lane, grp = lane >> 3, cg = lane & 7;
-  int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
   float4 qa = L.qa, ka = L.ka;
-  float4 gq = f4_zero(), gk = f4_zero();
-  if (FULL && cur_i == __float_as_int(rec[(row0 + 3) * kBwRec + 1])) {
+  const int first_i = __float_as_int(rec[row0 * kBwRec + 1]);
+  if (first_i != S.i) {
+    S.flush<F>(lane, g_qkv);
+    S.start(first_i);
+  }
+  if (FULL && first_i == __float_as_int(rec[(row0 + 3) * kBwRec + 1])) {
     // four pairs of one receiver (five runs of six): no branches between the rows, the eight logits summed together; lane cg of a head's
     // group then holds row cg / 2, direction cg & 1
     float v[8];
@@ -1049,37 +1159,29 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
     }
     float* mp = rec + (row0 + (cg >> 1)) * kBwRec;
     const int dir = cg & 1;
-    const float sc = mp[2], dcn = mp[3], da = mp[(F ? 12 : 36) + 4 * dir + grp];
+    const float sc = mp[2], dcn = mp[3], da = mp[kField + 4 * dir + grp];
     const float D = transpose_sum8(v, cg);
-    mp[(F ? 20 + 4 * dir : 48 - 4 * dir) + grp] = sc * D;
+    mp[kField + 4 * dir + grp] = sc * D;
     const float dD = sc * da;
     float gc = dcn * da * D;      // cutoff part of d/dr, summed over the directions and heads
     gc += __shfl_xor_sync(0xffffffffu, gc, 1);
     gc += __shfl_xor_sync(0xffffffffu, gc, 8);
     gc += __shfl_xor_sync(0xffffffffu, gc, 16);
-    if (grp == 0 && dir == 0) mp[32] += gc;
+    if (grp == 0 && dir == 0) mp[12] += gc;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const float dDA = __shfl_sync(0xffffffffu, dD, (lane & 24) + 2 * u), dDB = __shfl_sync(0xffffffffu, dD, (lane & 24) + 2 * u + 1);
       const float4 aw = f4_scale(dDA, w[u]), bw = f4_scale(dDB, w[u]);
-      gq = f4_mad(aw, L.kj[u], gq);
-      gk = f4_mad(bw, L.qj[u], gk);
+      S.gq = f4_mad(aw, L.kj[u], S.gq);
+      S.gk = f4_mad(bw, L.qj[u], S.gk);
       const int j = __float_as_int(rec[(row0 + u) * kBwRec]);
       if (j < n_scat) {
         float* gj = g_qkv + (size_t)j * kProj + F * 3 * kF + col;
         red_add_v4(gj, f4_mul(bw, ka));
         red_add_v4(gj + kF, f4_mul(aw, qa));
       }
-      const float4 dw = f4_fma(dDA, f4_mul(qa, L.kj[u]), f4_scale(dDB, f4_mul(L.qj[u], ka)));
-      uint2 h, l;
-      split2(dw.x, dw.y, h.x, l.x); split2(dw.z, dw.w, h.y, l.y);
-      unsigned char* p = a_hi + (lane >> 1) * kLboA + (row0 + u) * 16 + (lane & 1) * 8;
-      *reinterpret_cast<uint2*>(p) = h;
-      *reinterpret_cast<uint2*>(p + kAHalf) = l;
+      store_dw(a_hi, row0 + u, lane, f4_fma(dDA, f4_mul(qa, L.kj[u]), f4_scale(dDB, f4_mul(L.qj[u], ka))));
     }
-    float* gi = g_qkv + (size_t)cur_i * kProj + F * 3 * kF + col;
-    red_add_v4(gi, gq);
-    red_add_v4(gi + kF, gk);
     return;
   }
 #pragma unroll
@@ -1090,82 +1192,47 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, float* rec, co
     const float4 r0 = ld4(rp);
     const int j = __float_as_int(r0.x), i = __float_as_int(r0.y);
     const float sc = r0.z, dcn = r0.w;
-    if (i != cur_i) {      // rare: a run of four rows mostly stays with one receiver
-      {
-        float* gi = g_qkv + (size_t)cur_i * kProj + F * 3 * kF + col;
-        if (f4_nonzero(gq)) red_add_v4(gi, gq);
-        if (f4_nonzero(gk)) red_add_v4(gi + kF, gk);
-      }
-      cur_i = i;
-      gq = f4_zero(); gk = f4_zero();
+    if (i != S.i) {      // rare: a run of four rows mostly stays with one receiver
+      S.flush<F>(lane, g_qkv);
+      S.start(i);
       const float* pi = qkv + (size_t)i * kProj + F * 3 * kF;
       qa = ld4(pi + col); ka = ld4(pi + kF + col);
     }
     const float4 w = ld4(wt + (wrow0 + u) * kWStride + col);
-    const float4 qj = L.qj[u], kj = L.kj[u];
-    // packed FP32 arithmetic (fma.rn.f32x2) on the two halves of every float4: the products q_i k_j and q_j k_i serve both the
-    // logits and dw
-    const float2 w01 = make_float2(w.x, w.y), w23 = make_float2(w.z, w.w);
-    const float2 pA01 = __fmul2_rn(make_float2(qa.x, qa.y), make_float2(kj.x, kj.y)), pA23 = __fmul2_rn(make_float2(qa.z, qa.w), make_float2(kj.z, kj.w));
-    const float2 pB01 = __fmul2_rn(make_float2(qj.x, qj.y), make_float2(ka.x, ka.y)), pB23 = __fmul2_rn(make_float2(qj.z, qj.w), make_float2(ka.z, ka.w));
-    const float2 sA = __ffma2_rn(w23, pA23, __fmul2_rn(w01, pA01)), sB = __ffma2_rn(w23, pB23, __fmul2_rn(w01, pB01));
-    const float DA = group8_sum(sA.x + sA.y);
-    const float DB = group8_sum(sB.x + sB.y);
-    const float daA = rp[(F ? 12 : 36) + grp], daB = rp[(F ? 16 : 40) + grp];
-    if (cg == 0) {
-      if (F) { rp[20 + grp] = sc * DA; rp[24 + grp] = sc * DB; }
-      else { rp[44 + grp] = sc * DB; rp[48 + grp] = sc * DA; }
-    }
+    const float4 pA = f4_mul(qa, L.kj[u]), pB = f4_mul(L.qj[u], ka);      // serve both the logits and dw
+    const float DA = group8_sum(dot2(w, pA)), DB = group8_sum(dot2(w, pB));
+    const float daA = rp[kField + grp], daB = rp[kField + 4 + grp];
+    __syncwarp();      // the eight lanes of a head have read its cotangents: the logits take their place
+    if (cg == 0) { rp[kField + grp] = sc * DA; rp[kField + 4 + grp] = sc * DB; }
     const float dDA = sc * daA, dDB = sc * daB;
-    const float2 a2 = make_float2(dDA, dDA), b2 = make_float2(dDB, dDB);
-    {
-      const float2 g01 = __ffma2_rn(a2, __fmul2_rn(w01, make_float2(kj.x, kj.y)), make_float2(gq.x, gq.y));
-      const float2 g23 = __ffma2_rn(a2, __fmul2_rn(w23, make_float2(kj.z, kj.w)), make_float2(gq.z, gq.w));
-      gq = make_float4(g01.x, g01.y, g23.x, g23.y);
-      const float2 h01 = __ffma2_rn(b2, __fmul2_rn(w01, make_float2(qj.x, qj.y)), make_float2(gk.x, gk.y));
-      const float2 h23 = __ffma2_rn(b2, __fmul2_rn(w23, make_float2(qj.z, qj.w)), make_float2(gk.z, gk.w));
-      gk = make_float4(h01.x, h01.y, h23.x, h23.y);
-    }
+    const float4 aw = f4_scale(dDA, w), bw = f4_scale(dDB, w);
+    S.gq = f4_mad(aw, L.kj[u], S.gq);
+    S.gk = f4_mad(bw, L.qj[u], S.gk);
     if (j < n_scat && sc != 0.f) {      // the partner's shares: gq_j = dDB w k_i, gk_j = dDA w q_i
       float* gj = g_qkv + (size_t)j * kProj + F * 3 * kF + col;
-      const float2 m01 = __fmul2_rn(b2, w01), m23 = __fmul2_rn(b2, w23), n01 = __fmul2_rn(a2, w01), n23 = __fmul2_rn(a2, w23);
-      const float2 q01 = __fmul2_rn(m01, lo2(ka)), q23 = __fmul2_rn(m23, hi2(ka));
-      const float2 k01 = __fmul2_rn(n01, lo2(qa)), k23 = __fmul2_rn(n23, hi2(qa));
-      red_add_v4(gj, make_float4(q01.x, q01.y, q23.x, q23.y));
-      red_add_v4(gj + kF, make_float4(k01.x, k01.y, k23.x, k23.y));
+      red_add_v4(gj, f4_mul(bw, ka));
+      red_add_v4(gj + kF, f4_mul(aw, qa));
     }
-    const float2 d01 = __ffma2_rn(a2, pA01, __fmul2_rn(b2, pB01)), d23 = __ffma2_rn(a2, pA23, __fmul2_rn(b2, pB23));
-    const float dw0 = d01.x, dw1 = d01.y, dw2 = d23.x, dw3 = d23.y;
-    // dw as A operand of the second MMA chain: row = edge, columns 4 lane .. 4 lane + 3 of the hi and the lo matrix
-    {
-      uint2 h, l;
-      split2(dw0, dw1, h.x, l.x); split2(dw2, dw3, h.y, l.y);
-      unsigned char* p = a_hi + (lane >> 1) * kLboA + row * 16 + (lane & 1) * 8;
-      *reinterpret_cast<uint2*>(p) = h;
-      *reinterpret_cast<uint2*>(p + kAHalf) = l;
-    }
+    store_dw(a_hi, row, lane, f4_fma(dDA, pA, f4_scale(dDB, pB)));
     // cutoff part of d/dr, summed over the four heads
     float gc = dcn * fmaf(daA, DA, daB * DB);
     gc += __shfl_xor_sync(0xffffffffu, gc, 8);
     gc += __shfl_xor_sync(0xffffffffu, gc, 16);
-    if (lane == 0) rp[32] += gc;
+    if (lane == 0) rp[12] += gc;
   }
-  float* gi = g_qkv + (size_t)cur_i * kProj + F * 3 * kF + col;
-  if (f4_nonzero(gq)) red_add_v4(gi, gq);
-  if (f4_nonzero(gk)) red_add_v4(gi + kF, gk);
 }
 
-// record fields (floats): 0 j | 1 i | 2 cutoff / nbar | 3 its r-derivative | 4-7 invariants |
-// 12-15 dA, 16-19 dB: cotangents of the equivariant logits of edge (i<-j) and (j<-i) | 20-23, 24-27 those logits x cutoff |
-// 28-30 unit vector | 31 1/r | 32 d/dr (cutoff part) | 33 r | 34 1 for a list entry, 0 for a padding row |
-// 36-39, 40-43 cotangents of the invariant logits of edge (i<-j) and (j<-i) |
-// 44-47, 48-51 invariant logits of edges (j<-i) and (i<-j) x cutoff
+// record fields (floats): 0 j | 1 i | 2 cutoff / nbar | 3 its r-derivative | 4-7 invariants | 8-10 unit vector | 11 1/r |
+// 12 d/dr (cutoff part) | 13 r | 14 1 for a list entry, 0 for a padding row | 16-19, 20-23 cotangents of the equivariant logits of edge
+// (i<-j) and (j<-i), after that filter's loop the logits x cutoff | 24-27, 28-31 the same of the invariant logits |
+// 32-39, 40-47 transposed harmonics of both ends' cotangents of ev across the pair, two components per degree (angular_end)
 //
-// 16 warps.  Per tile: (1) four threads per edge prepare records and the A operand; (2) MMA chain w = Phi C + hs K2 (both filters);
-// (3) per filter, in two halves of 64 rows: tensor memory -> shared tile, reverse edge loop (4 rows per warp, sender rows
-// prefetched across the barriers), dw into the A operand, MMA chain [dPhi | dhs] = dw [C^T | K2^T]; (4) per edge the radial derivative
-// and the spherical hidden layer (the first filter's and the angular part of the force beneath the second filter's chain);
-// (5) force on the receiver, cotangent of ev.
+// 16 warps, the first four of which share the issue of the MMAs.  Per tile: (1) preparation of records and A operand: Chebyshev terms by two threads
+// per pair, the ev cotangents of the two ends by two others, then the hidden layers by four neighbouring threads per pair; (2) MMA chain
+// w = Phi C + hs K2 (both filters); (3) per filter, in two halves of 64 rows: tensor memory -> shared tile, reverse edge loop (4 rows per
+// warp, sender rows prefetched across the barriers), dw into the A operand, MMA chain [dPhi | dhs] = dw [C^T | K2^T]; (4) per pair the
+// radial derivative and the spherical hidden layer (the first filter's beneath the second filter's chain); (5) force on the receiver,
+// cotangent of ev.
 // PER_ENTRY (caller-supplied lists): `F` is the gradient with respect to the source list's displacement vectors (3 floats per
 // source entry, added to), `ve_orig` maps compacted entries to source entries, and the launch returns at once when *gate != 0.
 template <bool PER_ENTRY>
@@ -1181,21 +1248,23 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
                                                                     const int2* ve_orig, const int* gate,
                                                                     int n_own) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   float* rec = reinterpret_cast<float*>(smem + kOffBwRec);
   float* sph = reinterpret_cast<float*>(smem + kOffBwSph);
   float* wt = reinterpret_cast<float*>(smem + kOffBwW);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffBwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 16);
+  volatile int* failed = reinterpret_cast<volatile int*>(smem + kOffBwMisc + 20);
   for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kBwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
     const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
-    sph[k] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
+    sph[sph_at(f, c) + q] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
   }
   const uint32_t mbar = smem_u32(mbar_p);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(mbar));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *failed = 0;
   }
   grid_dep_sync();
   if (PER_ENTRY && gate && *gate != 0) return;
@@ -1208,12 +1277,22 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const int pad_i = ve_i[n_edges - 1];
   int* st_ij = reinterpret_cast<int*>(smem + kOffBwStIJ);
   float4* st_d = reinterpret_cast<float4*>(smem + kOffBwStD);
+  WarpRows R;
+  R.nu0 = rpw < 4 ? rpw : 4; R.nu1 = rpw - R.nu0;
+  R.row0 = R.nu0 * warp; R.row1 = 64 + R.nu1 * warp;
+  // list entry of a tile row within the tile, -1 for a padding row (see WarpRows)
+  auto entry_of = [&](int row) {
+    const int r = row & 63, nu = row < 64 ? R.nu0 : R.nu1;
+    if (r >= 16 * nu) return -1;
+    const int w = nu == 4 ? r >> 2 : (nu == 3 ? r / 3 : (nu == 2 ? r >> 1 : r));
+    return rpw * w + (r - nu * w) + (row < 64 ? 0 : R.nu0);
+  };
   // (i, j) and displacement of one tile's pairs into the staging buffers (threads 384..511): in flight beneath the tile before
   auto stage_tile = [&](long long t) {
     if (tid < 384 || t >= tile1) return;
-    const int row = tid - 384;
-    const long long e = t * tr + row;
-    if (row < tr && e < n_edges) {
+    const int row = tid - 384, k = entry_of(row);
+    const long long e = t * tr + k;
+    if (k >= 0 && e < n_edges) {
       cp_async4(st_ij + 2 * row, ve_i + e); cp_async4(st_ij + 2 * row + 1, ve_j + e);
       cp_async16(st_d + row, ve_d + e);
     } else {
@@ -1231,16 +1310,14 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_p;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_p, 0);
   const uint32_t a_hi = smem_u32(smem + kOffA), img = smem_u32(smem + kOffImg);
   unsigned char* a_ptr = smem + kOffA;
   const int deg = degree_of(lane < kMTot ? lane : 0);
   const int quad = warp & 3;                    // TMEM lane quadrant of this warp
   const int n_scat = n_recv;                    // partners below it own a row: they receive their share of a pair here
-  const int nu0 = rpw < 4 ? rpw : 4, nu1 = rpw - nu0;      // this warp's rows inside the two 64-row halves of the tile
-  const int wrow0 = nu0 * warp, wrow1 = nu1 * warp;
   uint32_t parity = 0;
-  bool failed = false;
+  const uint32_t on = elect_one();
 #ifdef SO3LR_TC_TIMING
   long long bph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   long long bc0 = clock64();
@@ -1248,62 +1325,66 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
 #else
 #define BW_MARK(k) do { } while (0)
 #endif
-  for (long long tile = tile0; tile < tile1 && !failed; ++tile) {
+  for (long long tile = tile0; tile < tile1; ++tile) {
     float dev8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // ---- per-edge preparation ----
     {
+      // a quarter of a pair's ev rows per thread (four neighbouring threads per pair): requested first, used last
+      const int hrow = 8 * warp + (lane >> 2), q = lane & 3;
+      const float* evi = ev_in + (size_t)st_ij[2 * hrow] * kMTot;
+      const float* evj = ev_in + (size_t)st_ij[2 * hrow + 1] * kMTot;
+      const float4 ei0 = ld4(evi + 4 * q), ej0 = ld4(evj + 4 * q);
+      float4 ei1 = f4_zero(), ej1 = f4_zero();
+      if (q < 2) { ei1 = ld4(evi + 16 + 4 * q); ej1 = ld4(evj + 16 + 4 * q); }
       const int row = tid & 127, role = tid >> 7;
-      const bool valid = row < tr && tile * tr + row < n_edges;
-      const int i = st_ij[2 * row], j = st_ij[2 * row + 1];
-      float* rp = rec + row * kBwRec;
+      const int k = entry_of(row);
+      const bool valid = k >= 0 && tile * tr + k < n_edges;
+      const float4 d = st_d[row];
+      const float r = d.w;
       if (role < 2) {
-        const float4 d = st_d[row];
-        const float r = d.w;
-        // the Chebyshev chunks first: once these 256 threads are through, the Chebyshev steps of both filters' MMA chains start
-        // beneath the rest of the preparation (the gathers of the other two threads of an entry above all)
+        // once these 256 threads are through, the Chebyshev steps of both filters' MMA chains start beneath the rest
         store_chebyshev_half(a_ptr, row, r, valid, role);
         fence_async_smem();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (tid == 0) {
+        if (warp < 4) {
+          asm volatile("bar.sync 1, 256;" ::: "memory");
           tc_fence_after();
-          issue_filter_mma(tmem, a_hi, img, 0, 0);
-          issue_filter_mma(tmem, a_hi, img, 1, 0);
+          issue_filter_mma(on, tmem, a_hi, img, warp >> 1, warp & 1, 0);
+        } else {
+          asm volatile("bar.arrive 1, 256;" ::: "memory");
         }
+      } else {
+        const int i = st_ij[2 * row], j = st_ij[2 * row + 1];
         const float ir = 1.f / r;
         const float ux = d.x * ir, uy = d.y * ir, uz = d.z * ir;
-        if (role == 0) {
+        float* rp = rec + row * kBwRec;
+        if (role == 2) {
           float cut, dcut;
           phys_cutoff(r, cut, dcut);
           st4(rp, make_float4(__int_as_float(j), __int_as_float(i), valid ? cut * kInvNbar : 0.f, valid ? dcut * kInvNbar : 0.f));
-          st4(rp + 20, f4_zero());
-          st4(rp + 24, f4_zero());
-          st4(rp + 28, make_float4(ux, uy, uz, ir));
-          st4(rp + 32, make_float4(0.f, r, valid ? 1.f : 0.f, 0.f));
-        } else {
-          float Y[kMTot];
-          sph_harm_24(ux, uy, uz, Y);
-          float dA[4] = {0.f, 0.f, 0.f, 0.f}, dB[4] = {0.f, 0.f, 0.f, 0.f};
-          const float* gevi = gev1 + (size_t)i * kMTot;
-          const float* gevj = gev1 + (size_t)j * kMTot;
-#pragma unroll
-          for (int c = 0; c < 6; ++c) {
-            const float4 a = ld4(gevi + 4 * c), b = ld4(gevj + 4 * c);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              dA[degree_of(4 * c + q)] = fmaf(av[q], Y[4 * c + q], dA[degree_of(4 * c + q)]);
-              dB[degree_of(4 * c + q)] = fmaf(bv[q], Y[4 * c + q], dB[degree_of(4 * c + q)]);
-            }
-          }
-          dB[0] = -dB[0]; dB[2] = -dB[2];   // Y_lm(-u) = (-1)^l Y_lm(u)
-          st4(rp + 12, make_float4(dA[0], dA[1], dA[2], dA[3]));
-          st4(rp + 16, make_float4(dB[0], dB[1], dB[2], dB[3]));
+          st4(rp + 8, make_float4(ux, uy, uz, ir));
+          st4(rp + 12, make_float4(0.f, r, valid ? 1.f : 0.f, 0.f));
         }
-      } else {
-        float s[4];
-        invariants(ev_in + (size_t)i * kMTot, ev_in + (size_t)j * kMTot, s);
-        if (role == 2) st4(rp + 4, make_float4(s[0], s[1], s[2], s[3]));
-        store_spherical_hidden_f(a_ptr, row, s, sph, role - 2);
+        angular_end(gev1 + (size_t)(role == 2 ? i : j) * kMTot, ux, uy, uz, role == 2 ? 1.f : -1.f, rp + 8 + 4 * role, rp + 16 + 8 * role);
+      }
+      {
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        const float dv[8] = {ej0.x - ei0.x, ej0.y - ei0.y, ej0.z - ei0.z, ej0.w - ei0.w, ej1.x - ei1.x, ej1.y - ei1.y, ej1.z - ei1.z, ej1.w - ei1.w};
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {      // components 4 q + c (degrees 1..3, and 15 of degree 4), then 16 + 4 q + (c - 4) of degree 4
+          const float x2 = dv[c] * dv[c];
+          if (c >= 4) { s[3] += x2; continue; }
+          const int l = degree_of(4 * q + c);
+#pragma unroll
+          for (int g = 0; g < 4; ++g) s[g] += l == g ? x2 : 0.f;
+        }
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          s[l] += __shfl_xor_sync(0xffffffffu, s[l], 1);
+          s[l] += __shfl_xor_sync(0xffffffffu, s[l], 2);
+          s[l] *= invw(l);
+        }
+        if (q == 0) st4(rec + hrow * kBwRec + 4, make_float4(s[0], s[1], s[2], s[3]));
+        store_spherical_hidden_quarter(a_ptr, hrow, s, sph, q);
       }
     }
     BW_MARK(0);
@@ -1312,22 +1393,18 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     __syncthreads();
     BW_MARK(1);
     stage_tile(tile + 1);
-    if (tid == 0) {
+    if (warp < 4) {
       tc_fence_after();
-      issue_filter_mma(tmem, a_hi, img, 0, 1);
-      issue_filter_mma(tmem, a_hi, img, 1, 1);
-      umma_commit(mbar);
+      issue_filter_mma(on, tmem, a_hi, img, warp >> 1, warp & 1, 1);
+      umma_commit_if(on, mbar);
     }
-    __syncwarp();
     // while the tensor cores run: the value path's logit cotangents (8 rows per warp), then the sender rows of the first edge run
-    edge_loops(rpw, [&](auto full) { value_logit_cotangents<full>(rec, rpw * warp, rpw, lane, qkv, g_xa); });
+    edge_loops(rpw, [&](auto full) { value_logit_cotangents<full>(rec, R, rpw, lane, qkv, g_xa); });
     RevLoads L;
-    reverse_prefetch<0>(L, rec, wrow0, lane, qkv);
-    bool done = true;
-    if (tid == 0) done = mbar_wait(mbar, parity);     // one thread polls; the others park at the barrier below
+    RevSums S;
+    reverse_prefetch<0>(L, rec, R.row0, lane, qkv);
+    wait_mma(mbar, parity, failed, err);
     parity ^= 1;
-    if (!__syncthreads_and(done)) { failed = true; break; }
-    tc_fence_after();
     BW_MARK(2);
     // this thread's shares of its row's cotangents of the invariants and of the radial derivative, both filters
     float ds0 = 0.f, ds1 = 0.f, ds2 = 0.f, ds3 = 0.f, drad = 0.f;
@@ -1344,14 +1421,14 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     // per pair, once the second MMA chain of filter f is through: radial derivative and spherical hidden layer (all four threads of a row)
     auto finish_filter = [&](int f) {
       const int row = tid & 127, role = tid >> 7;
-      float* rp = rec + row * kBwRec;
+      const float* rp = rec + row * kBwRec;
       const uint32_t lane_base = tmem + ((uint32_t)(32 * quad) << 16) + 128 * f;
       {
         // thread (odd, upper) takes the terms m = 2c + odd of c in [16 upper, 16 upper + 16): columns 32 odd + c.  T_m' = m U_{m-1}, and
         // U_{n+2} = 2 T_2 U_n - U_{n-2} from (U_{-2}, U_0) or (U_{-3}, U_{-1}), in the upper half from (U_30, U_32) or (U_29, U_31),
         // which follow from t by doubling: T_2n = 2 T_n^2 - 1, U_{2n-1} = 2 T_n U_{n-1}, U_n = t U_{n-1} + T_n, U_{n-2} = t U_{n-1} - T_n
         const int odd = role & 1, upper = role >> 1;
-        const float r = rp[33];
+        const float r = rp[13];
         const float x = expf(-kChebHalfGamma * r);
         const float t = fmaf(kChebA, x, kChebB), t2 = 2.f * t;
         const float dtdr = -kChebA * kChebHalfGamma * x;
@@ -1384,7 +1461,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
 #pragma unroll
         for (int c8 = 0; c8 < 8; ++c8) {
           const int c = 8 * role + c8;
-          const float* p = sph + (f * 32 + c) * 8;
+          const float* p = sph + sph_at(f, c);
           const float4 k = ld4(p);
           const float z = fmaf(s4.x, k.x, fmaf(s4.y, k.y, fmaf(s4.z, k.z, fmaf(s4.w, k.w, p[4]))));
           const float sg = __fdividef(1.f, 1.f + __expf(-z));
@@ -1398,87 +1475,72 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     BW_MARK(3);
-    edge_loops(nu0, [&](auto full) { reverse_edges4<0, full>(L, rec, wt, wrow0, wrow0, nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-    if (nu1) {
-      reverse_prefetch<0>(L, rec, 64 + wrow1, lane, qkv);
+    S.start(__float_as_int(rec[R.row0 * kBwRec + 1]));
+    edge_loops(R.nu0, [&](auto full) { reverse_edges4<0, full>(L, S, rec, wt, R.row0, R.row0, R.nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+    if (R.nu1) {
+      reverse_prefetch<0>(L, rec, R.row1, lane, qkv);
       BW_MARK(4);
       __syncthreads();
       copy_half(0, 1);
       tc_fence_before();
       __syncthreads();
       BW_MARK(3);
-      edge_loops(nu1, [&](auto full) { reverse_edges4<0, full>(L, rec, wt, wrow1, 64 + wrow1, nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+      edge_loops(R.nu1, [&](auto full) { reverse_edges4<0, full>(L, S, rec, wt, R.row1 - 64, R.row1, R.nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
     }
-    reverse_prefetch<1>(L, rec, wrow0, lane, qkv);
+    S.flush<0>(lane, g_qkv);
+    reverse_prefetch<1>(L, rec, R.row0, lane, qkv);
     BW_MARK(4);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp < 4) {
       tc_fence_after();
-      issue_reverse_mma(tmem, a_hi, img, 0);
-      umma_commit(mbar);
+      if (warp < 2) issue_reverse_mma(on, tmem, a_hi, img, 0, warp);
+      umma_commit_if(on, mbar);
     }
-    __syncwarp();
     // while the tensor cores run: the value path, and the first half of filter 1's accumulators (columns that this chain leaves alone).
     // What the chain yields is picked up beneath the next one.
-    edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, rpw * warp, rpw, lane, g_xa, g_qkv, n_scat); });
+    edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, R, rpw, lane, g_xa, g_qkv, n_scat); });
     copy_half(1, 0);
     tc_fence_before();
-    done = true;
-    if (tid == 0) done = mbar_wait(mbar, parity);
+    __syncthreads();
+    wait_mma(mbar, parity, failed, err);      // the next loop overwrites the operand that this chain reads
     parity ^= 1;
-    if (!__syncthreads_and(done)) { failed = true; break; }
-    tc_fence_after();
     BW_MARK(5);
     // ---- filter 1 ----
-    edge_loops(nu0, [&](auto full) { reverse_edges4<1, full>(L, rec, wt, wrow0, wrow0, nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-    if (nu1) {
-      reverse_prefetch<1>(L, rec, 64 + wrow1, lane, qkv);
+    S.start(__float_as_int(rec[R.row0 * kBwRec + 1]));
+    edge_loops(R.nu0, [&](auto full) { reverse_edges4<1, full>(L, S, rec, wt, R.row0, R.row0, R.nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+    if (R.nu1) {
+      reverse_prefetch<1>(L, rec, R.row1, lane, qkv);
       BW_MARK(4);
       __syncthreads();
       copy_half(1, 1);
       tc_fence_before();
       __syncthreads();
       BW_MARK(3);
-      edge_loops(nu1, [&](auto full) { reverse_edges4<1, full>(L, rec, wt, wrow1, 64 + wrow1, nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
+      edge_loops(R.nu1, [&](auto full) { reverse_edges4<1, full>(L, S, rec, wt, R.row1 - 64, R.row1, R.nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
     }
+    S.flush<1>(lane, g_qkv);
     BW_MARK(4);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp < 4) {
       tc_fence_after();
-      issue_reverse_mma(tmem, a_hi, img, 1);
-      umma_commit(mbar);
+      if (warp < 2) issue_reverse_mma(on, tmem, a_hi, img, 1, warp);
+      umma_commit_if(on, mbar);
     }
-    __syncwarp();
     if (lane < kMTot) {      // ev differences of this warp's rows of the final flush: requested now, used after the last MMA
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float* rp = rec + ((rpw * warp + k) & (TE - 1)) * kBwRec;
+        const float* rp = rec + (R.row(k) & (TE - 1)) * kBwRec;
         const int j = __float_as_int(rp[0]), i = __float_as_int(rp[1]);
         dev8[k] = ev_in[(size_t)j * kMTot + lane] - ev_in[(size_t)i * kMTot + lane];
       }
     }
-    {
-      // angular part of the force on the receiver (independent of the radial derivative that the running MMA yields): each of the four
-      // threads of a row takes one degree; the shares wait in the filter tile, above the ones of the last phase
-      const int row = tid & 127;
-      float4 ang = f4_zero();
-      const int l = tid >> 7;
-      if (l == 0) ang = angular_share<1>(rec + row * kBwRec, gev1);
-      else if (l == 1) ang = angular_share<2>(rec + row * kBwRec, gev1);
-      else if (l == 2) ang = angular_share<3>(rec + row * kBwRec, gev1);
-      else ang = angular_share<4>(rec + row * kBwRec, gev1);
-      st4(wt + kAngOff + (l * TE + row) * 4, ang);
-    }
     finish_filter(0);
-    done = true;
-    if (tid == 0) done = mbar_wait(mbar, parity);
+    wait_mma(mbar, parity, failed, err);
     parity ^= 1;
-    if (!__syncthreads_and(done)) { failed = true; break; }
-    tc_fence_after();
     BW_MARK(5);
     finish_filter(1);
     {
@@ -1490,22 +1552,28 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     BW_MARK(6);
-    if (failed) break;
-    // ---- force on the receiver (threads 0..127; the angular part was formed under the last MMA); cotangent of ev (8 rows per warp) ----
+    // ---- force on the receiver (threads 0..127); cotangent of ev (8 rows per warp) ----
     if (tid < 128) {
       const float* rp = rec + tid * kBwRec;
-      const bool on = rp[34] != 0.f;
+      const bool on = rp[14] != 0.f;
       const int i = on ? __float_as_int(rp[1]) : -1;
-      const float4 uu = ld4(rp + 28);
-      const float* ap = wt + kAngOff + tid * 4;
-      const float4 an0 = ld4(ap), an1 = ld4(ap + TE * 4), an2 = ld4(ap + 2 * TE * 4), an3 = ld4(ap + 3 * TE * 4);
-      const float4 ang = make_float4((an0.x + an1.x) + (an2.x + an3.x), (an0.y + an1.y) + (an2.y + an3.y), (an0.z + an1.z) + (an2.z + an3.z), 0.f);
+      const float4 uu = ld4(rp + 8);
+      float e1[3], e2[3], t1 = 0.f, t2 = 0.f;
+      tangent_frame(uu.x, uu.y, uu.z, e1, e2);
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        const float a = rp[16 + l], b = rp[20 + l];
+        t1 = fmaf(a, rp[32 + 2 * l], fmaf(b, rp[40 + 2 * l], t1));
+        t2 = fmaf(a, rp[33 + 2 * l], fmaf(b, rp[41 + 2 * l], t2));
+      }
+      t1 *= uu.w; t2 *= uu.w;
+      const float4 ang = make_float4(fmaf(t1, e1[0], t2 * e2[0]), fmaf(t1, e1[1], t2 * e2[1]), fmaf(t1, e1[2], t2 * e2[2]), 0.f);
       const float* dr = wt + 4 * 4 * TE + tid;
-      const float g_r = rp[32] + ((dr[0] + dr[TE]) + (dr[2 * TE] + dr[3 * TE]));
+      const float g_r = rp[12] + ((dr[0] + dr[TE]) + (dr[2 * TE] + dr[3 * TE]));
       float fsx = on ? fmaf(g_r, uu.x, ang.x) : 0.f, fsy = on ? fmaf(g_r, uu.y, ang.y) : 0.f, fsz = on ? fmaf(g_r, uu.z, ang.z) : 0.f;
       if (virial && on) {
         // both ends' halves on the receiver's row, unless the partner's is not summed here (rows below n_own are)
-        const float hr = (__float_as_int(rp[0]) < n_own ? 1.f : 0.5f) * rp[33];
+        const float hr = (__float_as_int(rp[0]) < n_own ? 1.f : 0.5f) * rp[13];
         const float wx = hr * uu.x, wy = hr * uu.y, wz = hr * uu.z;
         float* w = virial + 6 * (size_t)i;
         atomicAdd(w, wx * fsx); atomicAdd(w + 1, wy * fsy); atomicAdd(w + 2, wz * fsz);
@@ -1516,7 +1584,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         // half of the pair's force on the receiver goes to this entry of the source list, the other half with the opposite sign to the
         // reversed entry
         if (on) {
-          const int2 eo = ve_orig[tile * tr + tid];
+          const int2 eo = ve_orig[tile * tr + entry_of(tid)];
           float *g = F + 3 * (size_t)eo.x, *h = F + 3 * (size_t)eo.y;
           g[0] += 0.5f * fsx; g[1] += 0.5f * fsy; g[2] += 0.5f * fsz;
           h[0] -= 0.5f * fsx; h[1] -= 0.5f * fsy; h[2] -= 0.5f * fsz;
@@ -1542,19 +1610,18 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     }
     edge_loops(rpw, [&](auto full) {
       const float sc = -2.f * invw(deg);
-      const float* dp0 = wt + rpw * warp * 4 + deg;
+      auto row_of = [&](int k) { return full ? (k < 4 ? R.row0 + k : R.row1 + k - 4) : R.row(k); };
       auto share = [&](int k) {      // derivative with respect to the receiver's component; the partner's is its negative
-        const float* dp = dp0 + 4 * k;
+        const float* dp = wt + 4 * row_of(k) + deg;
         return sc * ((dp[0] + dp[TE * 4]) + (dp[2 * TE * 4] + dp[3 * TE * 4])) * dev8[k];
       };
-      const float* rp0 = rec + rpw * warp * kBwRec;
-      int cur_i = __float_as_int(rp0[1]);
+      int cur_i = __float_as_int(rec[row_of(0) * kBwRec + 1]);
       float acc = 0.f;
-      if (full && cur_i == __float_as_int(rp0[7 * kBwRec + 1])) {      // eight pairs of one receiver
+      if (full && cur_i == __float_as_int(rec[row_of(7) * kBwRec + 1])) {      // eight pairs of one receiver
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float t = share(k);
-          const int j = __float_as_int(rp0[k * kBwRec]);
+          const int j = __float_as_int(rec[row_of(k) * kBwRec]);
           acc += t;
           if (lane < kMTot && j < n_scat) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
         }
@@ -1562,7 +1629,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           if (!full && k >= rpw) break;
-          const float* rp = rp0 + k * kBwRec;
+          const float* rp = rec + row_of(k) * kBwRec;
           const int i = __float_as_int(rp[1]);
           if (i != cur_i) {
             if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
@@ -1571,7 +1638,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
           const float t = share(k);
           const int j = __float_as_int(rp[0]);
           acc += t;
-          if (lane < kMTot && j < n_scat && rp[34] != 0.f) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
+          if (lane < kMTot && j < n_scat && rp[14] != 0.f) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
         }
       }
       if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
@@ -1584,7 +1651,6 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[16 + q] = bph[q]; dbg[24] = tile1 - tile0; }
   if (dbg && (tid & 31) == 0 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[32 + 8 * warp + q] = bph[q]; }
 #endif
-  if (failed && tid == 0) atomicExch(err, 1);
   cp_async_wait_all();
   tc_fence_before();
   __syncthreads();
