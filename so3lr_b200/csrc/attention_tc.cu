@@ -169,6 +169,17 @@ __device__ __forceinline__ void umma_if(uint32_t on, uint32_t d_tmem, uint64_t a
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
 }
+// ... that writes the accumulator rows [64 half, 64 half + 64) only
+__device__ __forceinline__ void umma_half_if(uint32_t on, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, int half) {
+  const uint32_t off_lo = half ? 0xffffffffu : 0u, off_hi = ~off_lo;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%6, %6, %7, %7}, p;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on), "r"(off_lo), "r"(off_hi) : "memory");
+}
 __device__ __forceinline__ void umma_commit_if(uint32_t on, uint32_t mbar) {
   asm volatile(
       "{\n\t"
@@ -466,7 +477,7 @@ template <int PASS>
 __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_rows, int n, const int* __restrict__ row_ptr,
                                                                          const int* __restrict__ nbr_j, const float* dR,
                                                                          const int* partner, const int* asym,
-                                                                         int* __restrict__ total, int* blocks, int* __restrict__ ve_i,
+                                                                         int* total, int* blocks, int* __restrict__ ve_i,
                                                                          int* __restrict__ ve_j, float4* __restrict__ ve_d, int2* __restrict__ ve_orig) {
   grid_dep_sync();
   __shared__ int start[kCompactRows + 1];
@@ -485,6 +496,7 @@ __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_r
     if (partner && !all) { pe = partner[e]; return e < pe; }
     return true;
   };
+  if (PASS == kReserve && blockIdx.x == 0 && threadIdx.x == 0) total[1] = total[2] = 0;      // the tile queue
   int count = 0, j = -1, pe = -1;
   float4 d = f4_zero();
   for (int eb = e0; eb < e1; eb += 32) count += __popc(__ballot_sync(0xffffffffu, look(eb + lane, j, pe, d)));
@@ -513,7 +525,7 @@ __global__ void __launch_bounds__(32 * kCompactRows) compact_rows_kernel(int n_r
   }
 }
 // counts -> exclusive offsets, and their sum; one CTA (an eighth of a million atoms per 8 counts of a thread)
-__global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* blocks, int* __restrict__ total) {
+__global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* blocks, int* total) {
   grid_dep_sync();
   __shared__ int warp_sum_[32];
   const int tid = threadIdx.x, lane = tid & 31, per = (n + 1023) / 1024;
@@ -534,7 +546,7 @@ __global__ void __launch_bounds__(1024) scan_blocks_kernel(int n, int* blocks, i
   __syncthreads();
   int at = incl - sum + (tid >= 32 ? warp_sum_[(tid >> 5) - 1] : 0);
   for (int b = b0; b < b1; ++b) { const int c = blocks[b]; blocks[b] = at; at += c; }
-  if (tid == 1023) *total = at;
+  if (tid == 1023) { total[0] = at; total[1] = total[2] = 0; }      // the sum, the tile queue
 }
 // Every entry (i <- j, d) inside the cutoff of a caller-supplied list finds its reversed entry (j <- i, -d): the k-th of several equal
 // entries of a row takes the k-th match.  *asym is set when an entry has none or the numbers of equal entries differ.  One warp per row.
@@ -593,6 +605,32 @@ __device__ __forceinline__ int entries_per_warp(long long n_edges, int grid) {
   const long long rounds = (n_edges + (long long)TE * grid - 1) / ((long long)TE * grid);
   return (int)((n_edges + 16 * rounds * grid - 1) / (16 * rounds * grid));
 }
+// Which tiles a CTA takes.  Short lists: an equal share of consecutive tiles.  Long lists: runs of kTileRun tiles in the order in which CTAs
+// come free (CTA b starts with run b).  SMs differ by several per cent in the time of a tile (their distance from the L2 slices that hold its
+// rows), so equal shares end with the slowest; and all CTAs work in one stretch of the list at a time, whose rows stay in the L2.  The
+// next run is asked for during the first tile of a run.  `queue`: runs handed out beyond the first of every CTA | CTAs that are
+// through; both zero at the start of a launch: the build of the list clears them, and the last CTA to finish puts them back.
+constexpr int kTileRun = 2;
+constexpr int kQueuedTiles = 8;                // tiles per CTA from which on the queue is used
+struct TileWalk {
+  int tile, next, end;      // this tile, the one behind it; tiles from `end` on are not this CTA's
+  bool queued;
+  __device__ __forceinline__ explicit TileWalk(int n) {
+    const int grid = (int)gridDim.x, b = (int)blockIdx.x, share = n / grid, more = n - share * grid;
+    queued = share >= kQueuedTiles;
+    tile = queued ? kTileRun * b : b * share + min(b, more);
+    end = queued ? n : tile + share + (b < more);
+    next = tile;
+  }
+  __device__ __forceinline__ bool asks() const { return queued && tile % kTileRun == 0; }
+  __device__ __forceinline__ int ask(int* queue) const { return kTileRun * ((int)gridDim.x + atomicAdd(queue, 1)); }
+  // `run`: the first tile of the next run, asked for during the first tile of this one
+  __device__ __forceinline__ void look_ahead(const int* run) { next = queued && tile % kTileRun == kTileRun - 1 ? *run : tile + 1; }
+  // one thread per CTA, behind its last tile
+  __device__ __forceinline__ void finish(int* queue) const {
+    if (queued && atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) { atomicExch(queue, 0); atomicExch(queue + 1, 0); }
+  }
+};
 // `body(full)` with full = true_type where a warp's share is the whole run its loops are unrolled for (the run of a long list: branches
 // on the share inside the loops cost 4 % there), false_type where it is shorter
 template <class Body>
@@ -614,7 +652,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
                                                                     const int* ve_j, const float4* ve_d,
                                                                     const float* qkv, const float* ev_in,
                                                                     float* __restrict__ xa, float* __restrict__ ev1, int* __restrict__ err,
-                                                                    long long* __restrict__ dbg, const int* asym) {
+                                                                    long long* __restrict__ dbg, const int* asym, int* queue) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* rec = reinterpret_cast<float*>(smem + kOffFwRec);
@@ -625,6 +663,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   float* st_ev = reinterpret_cast<float*>(smem + kOffFwStEv);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffFwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffFwMisc + 16);
+  int* next_run = reinterpret_cast<int*>(smem + kOffFwMisc + 32);
   for (int k = tid; k < kTcImageBytes / 16; k += kFwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kFwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
     const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
@@ -639,17 +678,16 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
-  const long long n_tiles = (n_edges + tr - 1) / tr;
-  const long long tile0 = n_tiles * blockIdx.x / gridDim.x, tile1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
-  if (tile0 >= tile1) return;
+  TileWalk walk((int)((n_edges + tr - 1) / tr));
+  if (walk.tile >= walk.end) return;
   const int pad_i = ve_i[n_edges - 1];
   // partners below n_scat receive the pair's other direction (j <- i)
   const int n_scat = asym && *asym != 0 ? 0 : n_recv;
   // inputs of one tile into the staging buffers: receiver / sender, displacement, both atoms' ev rows (threads 256..383)
-  auto stage_tile = [&](long long tile) {
-    if (tid < 256 || tid >= 384 || tile >= tile1) return;
+  auto stage_tile = [&](int tile) {
+    if (tid < 256 || tid >= 384 || tile >= walk.end) return;
     const int row = tid - 256;
-    const long long e = tile * tr + row;
+    const long long e = (long long)tile * tr + row;
     int i = pad_i, j = pad_i;
     if (row < tr && e < n_edges) {
       i = ve_i[e]; j = ve_j[e];
@@ -671,7 +709,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  stage_tile(tile0);
+  stage_tile(walk.tile);
   cp_async_wait_all();
   fence_async_smem();
   tc_fence_before();
@@ -690,11 +728,13 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
 #else
 #define TC_MARK(k) do { } while (0)
 #endif
-  for (long long tile = tile0; tile < tile1; ++tile) {
+  for (; walk.tile < walk.end; walk.tile = walk.next) {
+    const long long entry0 = (long long)walk.tile * tr;
+    int run = 0;
     // ---- per-edge preparation from the staged inputs ----
     {
       const int row = tid & 127, role = tid >> 7;
-      const bool valid = row < tr && tile * tr + row < n_edges;
+      const bool valid = row < tr && entry0 + row < n_edges;
       if (role < 2) {
         const float4 d = st_d[row];
         const float r = d.w;
@@ -745,7 +785,9 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     TC_MARK(1);
-    stage_tile(tile + 1);
+    walk.look_ahead(next_run);
+    stage_tile(walk.next);
+    if (tid == kFwThreads - 1 && walk.asks()) run = walk.ask(queue);
     bool done = true;
     if (tid == kFwIssuer) {
       tc_fence_after();
@@ -911,13 +953,15 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
       if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
     });
     cp_async_wait_all();
+    if (tid == kFwThreads - 1 && walk.asks()) *next_run = run;
     __syncthreads();
     TC_MARK(7);
   }
 #ifdef SO3LR_TC_TIMING
-  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[q] = tph[q]; dbg[8] = tile1 - tile0; }
+  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[q] = tph[q]; dbg[8] = walk.end / gridDim.x; }
   if (dbg && (tid & 31) == 0 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[160 + 8 * warp + q] = tph[q]; }
 #endif
+  if (tid == kFwThreads - 1) walk.finish(queue);
   cp_async_wait_all();
   tc_fence_before();
   __syncthreads();
@@ -936,7 +980,7 @@ namespace {
 // 28-30 unit vector | 31 1/r | 32 d/dr | 33 r | 34 1 for a list entry, 0 for a padding row
 // [dPhi | dhs_f] = dw_f * [C_f^T | K2_f^T] (the same image read K-major: N = 96 rows, K = features): main accumulators in TMEM
 // columns [128 f, 128 f + 96), cross 256 columns above
-__device__ __forceinline__ void issue_reverse_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int cross) {
+__device__ __forceinline__ void issue_reverse_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int half, int cross) {
   const uint64_t da = desc_base(kLboA, 128) + (a_hi >> 4), dal = da + (kAHalf >> 4);
   const uint64_t db = desc_base(1536, 128) + ((img + f * kRevImgFilter) >> 4), dbl = db + (2 * kRevImgFilter >> 4);
   const uint32_t id96 = make_idesc(96, 0);
@@ -946,44 +990,55 @@ __device__ __forceinline__ void issue_reverse_mma(uint32_t on, uint32_t tmem, ui
     const uint64_t ah = da + ks * (2 * kLboA >> 4), al = dal + ks * (2 * kLboA >> 4);
     const uint64_t bh = db + ks * (2 * 1536 >> 4), bl = dbl + ks * (2 * 1536 >> 4);
     if (!cross) {
-      umma_if(on, d, ah, bh, id96, ks > 0);
+      umma_half_if(on, d, ah, bh, id96, ks > 0, half);
     } else {
-      umma_if(on, d, ah, bl, id96, ks > 0);
-      umma_if(on, d, al, bh, id96, 1);
+      umma_half_if(on, d, ah, bl, id96, ks > 0, half);
+      umma_half_if(on, d, al, bh, id96, 1, half);
     }
   }
 }
 
-// A warp owns up to eight consecutive pairs of a tile: the first nu0 <= 4 sit in rows [nu0 warp, nu0 warp + nu0), the others in rows
-// [64 + nu1 warp, 64 + nu1 warp + nu1): the filter tile holds 64 rows at a time.
-struct WarpRows {
-  int nu0, nu1, row0, row1;
-  __device__ __forceinline__ int row(int k) const { return k < nu0 ? row0 + k : row1 + (k - nu0); }
-};
 // Sender-side q / k rows of four consecutive tile rows for the reverse edge loop of filter F (lane = 4 features)
 // (for every row of the four: past a warp's share these are rows of other warps, whose values are not used)
 struct RevLoads {
-  float4 qj[4], kj[4], qa, ka;     // senders' rows; q / k of the first row's receiver
+  float4 qj[4], kj[4];
+  template <int F>
+  __device__ __forceinline__ void fetch(int u, const float* rec, int row, int lane, const float* __restrict__ qkv) {
+    const float* pj = qkv + (size_t)__float_as_int(rec[(row & (TE - 1)) * kBwRec]) * kProj + F * 3 * kF + 4 * lane;
+    qj[u] = ld4(pj);
+    kj[u] = ld4(pj + kF);
+  }
+};
+// A receiver's q / k rows and the sums of their cotangents, which a warp carries through its pairs
+struct Receiver {
+  float4 q, k, gq, gk;
+  int i;
+  template <int F>
+  __device__ __forceinline__ void start(int receiver, int lane, const float* __restrict__ qkv) {
+    i = receiver;
+    const float* pi = qkv + (size_t)i * kProj + F * 3 * kF + 4 * lane;
+    q = ld4(pi);
+    k = ld4(pi + kF);
+    gq = f4_zero(); gk = f4_zero();
+  }
+  template <int F>
+  __device__ __forceinline__ void flush(int lane, float* __restrict__ g_qkv) const {
+    float* gi = g_qkv + (size_t)i * kProj + F * 3 * kF + 4 * lane;
+    if (f4_nonzero(gq)) red_add_v4(gi, gq);
+    if (f4_nonzero(gk)) red_add_v4(gi + kF, gk);
+  }
 };
 template <int F>
 __device__ __forceinline__ void reverse_prefetch(RevLoads& L, const float* rec, int row0, int lane, const float* __restrict__ qkv) {
-  const int col = 4 * lane;
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const float* pj = qkv + (size_t)__float_as_int(rec[((row0 + u) & (TE - 1)) * kBwRec]) * kProj + F * 3 * kF;
-    L.qj[u] = ld4(pj + col);
-    L.kj[u] = ld4(pj + kF + col);
-  }
-  const float* pi = qkv + (size_t)__float_as_int(rec[row0 * kBwRec + 1]) * kProj + F * 3 * kF;
-  L.qa = ld4(pi + col);
-  L.ka = ld4(pi + kF + col);
+  for (int u = 0; u < 4; ++u) L.fetch<F>(u, rec, row0 + u, lane, qkv);
 }
 
 // Value path of the invariant filter, split off the edge loop so that it runs while the tensor cores are busy.
-// Before the loop (the nu = nu0 + nu1 pairs of one warp): cotangents of the invariant logits of both directions of every edge,
+// Before the loop (rows [row0, row0 + nu), nu <= 8, of one warp): cotangents of the invariant logits of both directions of every edge,
 // daA_h = <g_xa[i], v[j]>_h and daB_h = <g_xa[j], v[i]>_h, into record fields 24..27 and 28..31.
 template <bool FULL>
-__device__ __forceinline__ void value_logit_cotangents(float* rec, const WarpRows& R, int nu, int lane, const float* __restrict__ qkv,
+__device__ __forceinline__ void value_logit_cotangents(float* rec, int row0, int nu, int lane, const float* __restrict__ qkv,
                                                        const float* __restrict__ g_xa) {
   const int col = 4 * lane, grp = lane >> 3, cg = lane & 7;
   int cur_i = -1;
@@ -994,7 +1049,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, const WarpRow
     int ii[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const float* rp = rec + ((FULL ? (k0 ? R.row1 : R.row0) + u : R.row(k0 + u)) & (TE - 1)) * kBwRec;
+      const float* rp = rec + ((row0 + k0 + u) & (TE - 1)) * kBwRec;
       const int j = __float_as_int(rp[0]);
       ii[u] = __float_as_int(rp[1]);
       vj[u] = ld4(qkv + (size_t)j * kProj + 2 * kF + col);
@@ -1009,7 +1064,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, const WarpRow
       float v[8];
 #pragma unroll
       for (int u = 0; u < 4; ++u) { v[2 * u] = dot2(gx_i, vj[u]); v[2 * u + 1] = dot2(gxj[u], v_i); }
-      rec[((k0 ? R.row1 : R.row0) + (cg >> 1)) * kBwRec + 24 + 4 * (cg & 1) + grp] = transpose_sum8(v, cg);
+      rec[(row0 + k0 + (cg >> 1)) * kBwRec + 24 + 4 * (cg & 1) + grp] = transpose_sum8(v, cg);
       continue;
     }
 #pragma unroll
@@ -1022,7 +1077,7 @@ __device__ __forceinline__ void value_logit_cotangents(float* rec, const WarpRow
       }
       const float daA = group8_sum(dot2(gx_i, vj[u])), daB = group8_sum(dot2(gxj[u], v_i));
       if (cg == 0) {
-        float* rp = rec + R.row(k0 + u) * kBwRec;
+        float* rp = rec + (row0 + k0 + u) * kBwRec;
         rp[24 + grp] = daA;
         rp[28 + grp] = daB;
       }
@@ -1073,10 +1128,10 @@ __device__ __forceinline__ void angular_end(const float* __restrict__ gev, float
 // After the loop: cotangents of the value rows, gv_i = sum over its pairs (cutoff x logit of edge j<-i)_h g_xa[j] (fields 28..31) and,
 // pair by pair, gv_j += (cutoff x logit of edge i<-j)_h g_xa[i] (fields 24..27)
 template <bool FULL>
-__device__ __forceinline__ void value_cotangent(const float* rec, const WarpRows& R, int nu, int lane, const float* __restrict__ g_xa,
+__device__ __forceinline__ void value_cotangent(const float* rec, int row0, int nu, int lane, const float* __restrict__ g_xa,
                                                 float* __restrict__ g_qkv, int n_scat) {
   const int col = 4 * lane, grp = lane >> 3;
-  auto record = [&](int k) { return rec + ((FULL ? (k < 4 ? R.row0 + k : R.row1 + k - 4) : R.row(k)) & (TE - 1)) * kBwRec; };
+  auto record = [&](int k) { return rec + ((row0 + k) & (TE - 1)) * kBwRec; };
   float4 gxj[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) gxj[u] = ld4(g_xa + (size_t)__float_as_int(record(u)[0]) * kF + col);
@@ -1119,32 +1174,20 @@ __device__ __forceinline__ void store_dw(unsigned char* a_hi, int row, int lane,
   *reinterpret_cast<uint2*>(p) = h;
   *reinterpret_cast<uint2*>(p + kAHalf) = l;
 }
-// Sums of the receiver's q / k rows that a warp carries from one call of the edge loop to the next
-struct RevSums {
-  float4 gq, gk;
-  int i;
-  template <int F>
-  __device__ __forceinline__ void flush(int lane, float* __restrict__ g_qkv) const {
-    float* gi = g_qkv + (size_t)i * kProj + F * 3 * kF + 4 * lane;
-    if (f4_nonzero(gq)) red_add_v4(gi, gq);
-    if (f4_nonzero(gk)) red_add_v4(gi + kF, gk);
-  }
-  __device__ __forceinline__ void start(int receiver) { i = receiver; gq = f4_zero(); gk = f4_zero(); }
-};
 // Reverse edge loop of filter F over nu <= 4 tile rows [row0, row0 + nu) of one warp: logits of both directions of every edge,
 // cotangents of this receiver's q / k rows (added to g_qkv with vector reductions when the receiver changes), dw into the
 // A operand of the second MMA chain, the cutoff part of d/dr into the records.  The cotangents of the logits come from the
 // records (fields 24.. for the invariant filter, 16.. for the equivariant one); cutoff x logit takes their place.
-template <int F, bool FULL>
-__device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, float* rec, const float* wt, int wrow0, int row0, int nu,
+// NEXT: the rows of the four pairs that follow are requested as these come free.
+template <int F, bool FULL, bool NEXT>
+__device__ __forceinline__ void reverse_edges4(RevLoads& L, Receiver& S, float* rec, const float* wt, int wrow0, int row0, int nu,
                                                unsigned char* a_hi, int lane, const float* __restrict__ qkv, float* __restrict__ g_qkv, int n_scat) {
   constexpr int kField = F ? 16 : 24;
   const int col = 4 * lane, grp = lane >> 3, cg = lane & 7;
-  float4 qa = L.qa, ka = L.ka;
   const int first_i = __float_as_int(rec[row0 * kBwRec + 1]);
   if (first_i != S.i) {
     S.flush<F>(lane, g_qkv);
-    S.start(first_i);
+    S.start<F>(first_i, lane, qkv);
   }
   if (FULL && first_i == __float_as_int(rec[(row0 + 3) * kBwRec + 1])) {
     // four pairs of one receiver (five runs of six): no branches between the rows, the eight logits summed together; lane cg of a head's
@@ -1154,8 +1197,8 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, fl
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       w[u] = ld4(wt + (wrow0 + u) * kWStride + col);
-      v[2 * u] = dot3(qa, w[u], L.kj[u]);
-      v[2 * u + 1] = dot3(L.qj[u], w[u], ka);
+      v[2 * u] = dot3(S.q, w[u], L.kj[u]);
+      v[2 * u + 1] = dot3(L.qj[u], w[u], S.k);
     }
     float* mp = rec + (row0 + (cg >> 1)) * kBwRec;
     const int dir = cg & 1;
@@ -1177,10 +1220,11 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, fl
       const int j = __float_as_int(rec[(row0 + u) * kBwRec]);
       if (j < n_scat) {
         float* gj = g_qkv + (size_t)j * kProj + F * 3 * kF + col;
-        red_add_v4(gj, f4_mul(bw, ka));
-        red_add_v4(gj + kF, f4_mul(aw, qa));
+        red_add_v4(gj, f4_mul(bw, S.k));
+        red_add_v4(gj + kF, f4_mul(aw, S.q));
       }
-      store_dw(a_hi, row0 + u, lane, f4_fma(dDA, f4_mul(qa, L.kj[u]), f4_scale(dDB, f4_mul(L.qj[u], ka))));
+      store_dw(a_hi, row0 + u, lane, f4_fma(dDA, f4_mul(S.q, L.kj[u]), f4_scale(dDB, f4_mul(L.qj[u], S.k))));
+      if (NEXT) L.fetch<F>(u, rec, row0 + 4 + u, lane, qkv);
     }
     return;
   }
@@ -1194,12 +1238,10 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, fl
     const float sc = r0.z, dcn = r0.w;
     if (i != S.i) {      // rare: a run of four rows mostly stays with one receiver
       S.flush<F>(lane, g_qkv);
-      S.start(i);
-      const float* pi = qkv + (size_t)i * kProj + F * 3 * kF;
-      qa = ld4(pi + col); ka = ld4(pi + kF + col);
+      S.start<F>(i, lane, qkv);
     }
     const float4 w = ld4(wt + (wrow0 + u) * kWStride + col);
-    const float4 pA = f4_mul(qa, L.kj[u]), pB = f4_mul(L.qj[u], ka);      // serve both the logits and dw
+    const float4 pA = f4_mul(S.q, L.kj[u]), pB = f4_mul(L.qj[u], S.k);      // serve both the logits and dw
     const float DA = group8_sum(dot2(w, pA)), DB = group8_sum(dot2(w, pB));
     const float daA = rp[kField + grp], daB = rp[kField + 4 + grp];
     __syncwarp();      // the eight lanes of a head have read its cotangents: the logits take their place
@@ -1210,10 +1252,11 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, fl
     S.gk = f4_mad(bw, L.qj[u], S.gk);
     if (j < n_scat && sc != 0.f) {      // the partner's shares: gq_j = dDB w k_i, gk_j = dDA w q_i
       float* gj = g_qkv + (size_t)j * kProj + F * 3 * kF + col;
-      red_add_v4(gj, f4_mul(bw, ka));
-      red_add_v4(gj + kF, f4_mul(aw, qa));
+      red_add_v4(gj, f4_mul(bw, S.k));
+      red_add_v4(gj + kF, f4_mul(aw, S.q));
     }
     store_dw(a_hi, row, lane, f4_fma(dDA, pA, f4_scale(dDB, pB)));
+    if (NEXT) L.fetch<F>(u, rec, row0 + 4 + u, lane, qkv);
     // cutoff part of d/dr, summed over the four heads
     float gc = dcn * fmaf(daA, DA, daB * DB);
     gc += __shfl_xor_sync(0xffffffffu, gc, 8);
@@ -1221,18 +1264,35 @@ __device__ __forceinline__ void reverse_edges4(const RevLoads& L, RevSums& S, fl
     if (lane == 0) rp[12] += gc;
   }
 }
+// ... over a warp's nu <= 8 pairs
+template <int F>
+__device__ __forceinline__ void reverse_edges(RevLoads& L, float* rec, const float* wt, int wrow0, int row0, int nu, unsigned char* a_hi, int lane,
+                                              const float* __restrict__ qkv, float* __restrict__ g_qkv, int n_scat, Receiver& S) {
+  if (nu == 8) {
+    reverse_edges4<F, true, true>(L, S, rec, wt, wrow0, row0, 4, a_hi, lane, qkv, g_qkv, n_scat);
+    reverse_edges4<F, true, false>(L, S, rec, wt, wrow0 + 4, row0 + 4, 4, a_hi, lane, qkv, g_qkv, n_scat);
+  } else {
+    for (int k = 0; k < nu; k += 4) {
+      if (k) reverse_prefetch<F>(L, rec, row0 + k, lane, qkv);
+      reverse_edges4<F, false, false>(L, S, rec, wt, wrow0 + k, row0 + k, nu - k, a_hi, lane, qkv, g_qkv, n_scat);
+    }
+  }
+  S.flush<F>(lane, g_qkv);
+}
 
 // record fields (floats): 0 j | 1 i | 2 cutoff / nbar | 3 its r-derivative | 4-7 invariants | 8-10 unit vector | 11 1/r |
 // 12 d/dr (cutoff part) | 13 r | 14 1 for a list entry, 0 for a padding row | 16-19, 20-23 cotangents of the equivariant logits of edge
 // (i<-j) and (j<-i), after that filter's loop the logits x cutoff | 24-27, 28-31 the same of the invariant logits |
 // 32-39, 40-47 transposed harmonics of both ends' cotangents of ev across the pair, two components per degree (angular_end)
 //
-// 16 warps, the first four of which share the issue of the MMAs.  Per tile: (1) preparation of records and A operand: Chebyshev terms by two threads
-// per pair, the ev cotangents of the two ends by two others, then the hidden layers by four neighbouring threads per pair; (2) MMA chain
-// w = Phi C + hs K2 (both filters); (3) per filter, in two halves of 64 rows: tensor memory -> shared tile, reverse edge loop (4 rows per
-// warp, sender rows prefetched across the barriers), dw into the A operand, MMA chain [dPhi | dhs] = dw [C^T | K2^T]; (4) per pair the
-// radial derivative and the spherical hidden layer (the first filter's beneath the second filter's chain); (5) force on the receiver,
-// cotangent of ev.
+// 16 warps in two groups: the pairs of rows 0..63 belong to warps 0..7, those of rows 64..127 to warps 8..15.  Per tile: (1) all prepare the
+// records and the A operand: Chebyshev terms by two threads per pair, the ev cotangents of the two ends by two others, then the hidden layers
+// by four neighbouring threads per pair; (2) MMA chain w = Phi C + hs K2 (both filters, all rows), beneath it the value path's logit
+// cotangents; (3) per filter and group: tensor memory -> filter tile (64 rows), reverse edge loop, dw into the A operand, MMA chain
+// [dPhi | dhs] = dw [C^T | K2^T] of the group's rows (the other rows' results switched off).  The groups take turns with the filter tile:
+// the edge loops are bound by their row reductions (an SM sends 21 to 26 bytes per cycle), so while one group runs its loop the other goes
+// through the value path, the wait for its MMAs and the copy of its accumulators; (4) per pair the radial derivative and the spherical
+// hidden layer (the first filter's beneath the second filter's last chain); (5) force on the receiver, cotangent of ev.
 // PER_ENTRY (caller-supplied lists): `F` is the gradient with respect to the source list's displacement vectors (3 floats per
 // source entry, added to), `ve_orig` maps compacted entries to source entries, and the launch returns at once when *gate != 0.
 template <bool PER_ENTRY>
@@ -1245,7 +1305,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
                                                                     float* __restrict__ g_qkv, float* __restrict__ gev_in,
                                                                     float* F, float* __restrict__ virial,
                                                                     int* __restrict__ err, long long* __restrict__ dbg,
-                                                                    const int2* ve_orig, const int* gate,
+                                                                    const int2* ve_orig, const int* gate, int* queue,
                                                                     int n_own) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -1253,8 +1313,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   float* sph = reinterpret_cast<float*>(smem + kOffBwSph);
   float* wt = reinterpret_cast<float*>(smem + kOffBwW);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffBwMisc);
-  uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 16);
-  volatile int* failed = reinterpret_cast<volatile int*>(smem + kOffBwMisc + 20);
+  uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 48);
+  int* next_run = reinterpret_cast<int*>(smem + kOffBwMisc + 56);
+  volatile int* failed = reinterpret_cast<volatile int*>(smem + kOffBwMisc + 52);
   for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kBwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
     const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
@@ -1263,6 +1324,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const uint32_t mbar = smem_u32(mbar_p);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(mbar));
+    for (int k = 1; k < 5; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(mbar + 8 * k));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *failed = 0;
   }
@@ -1271,27 +1333,20 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
-  const long long n_tiles = (n_edges + tr - 1) / tr;
-  const long long tile0 = n_tiles * blockIdx.x / gridDim.x, tile1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
-  if (tile0 >= tile1) return;
+  TileWalk walk((int)((n_edges + tr - 1) / tr));
+  if (walk.tile >= walk.end) return;
   const int pad_i = ve_i[n_edges - 1];
   int* st_ij = reinterpret_cast<int*>(smem + kOffBwStIJ);
   float4* st_d = reinterpret_cast<float4*>(smem + kOffBwStD);
-  WarpRows R;
-  R.nu0 = rpw < 4 ? rpw : 4; R.nu1 = rpw - R.nu0;
-  R.row0 = R.nu0 * warp; R.row1 = 64 + R.nu1 * warp;
-  // list entry of a tile row within the tile, -1 for a padding row (see WarpRows)
-  auto entry_of = [&](int row) {
-    const int r = row & 63, nu = row < 64 ? R.nu0 : R.nu1;
-    if (r >= 16 * nu) return -1;
-    const int w = nu == 4 ? r >> 2 : (nu == 3 ? r / 3 : (nu == 2 ? r >> 1 : r));
-    return rpw * w + (r - nu * w) + (row < 64 ? 0 : R.nu0);
-  };
+  const int half = warp >> 3;                   // the rows of this warp's pairs: [64 half, 64 half + 8 rpw)
+  const int row0 = 64 * half + rpw * (warp & 7);
+  // list entry of a tile row within the tile, -1 for a padding row
+  auto entry_of = [&](int row) { return (row & 63) < 8 * rpw ? (row & 63) + (row >> 6) * 8 * rpw : -1; };
   // (i, j) and displacement of one tile's pairs into the staging buffers (threads 384..511): in flight beneath the tile before
-  auto stage_tile = [&](long long t) {
-    if (tid < 384 || t >= tile1) return;
+  auto stage_tile = [&](int t) {
+    if (tid < 384 || t >= walk.end) return;
     const int row = tid - 384, k = entry_of(row);
-    const long long e = t * tr + k;
+    const long long e = (long long)t * tr + k;
     if (k >= 0 && e < n_edges) {
       cp_async4(st_ij + 2 * row, ve_i + e); cp_async4(st_ij + 2 * row + 1, ve_j + e);
       cp_async16(st_d + row, ve_d + e);
@@ -1300,7 +1355,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       st_d[row] = make_float4(1.f, 0.f, 0.f, 1.f);
     }
   };
-  stage_tile(tile0);
+  stage_tile(walk.tile);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -1325,7 +1380,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
 #else
 #define BW_MARK(k) do { } while (0)
 #endif
-  for (long long tile = tile0; tile < tile1; ++tile) {
+  for (; walk.tile < walk.end; walk.tile = walk.next) {
+    const long long entry0 = (long long)walk.tile * tr;
+    int run = 0;
     float dev8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // ---- per-edge preparation ----
     {
@@ -1338,7 +1395,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       if (q < 2) { ei1 = ld4(evi + 16 + 4 * q); ej1 = ld4(evj + 16 + 4 * q); }
       const int row = tid & 127, role = tid >> 7;
       const int k = entry_of(row);
-      const bool valid = k >= 0 && tile * tr + k < n_edges;
+      const bool valid = k >= 0 && entry0 + k < n_edges;
       const float4 d = st_d[row];
       const float r = d.w;
       if (role < 2) {
@@ -1392,31 +1449,49 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     BW_MARK(1);
-    stage_tile(tile + 1);
+    walk.look_ahead(next_run);
+    stage_tile(walk.next);
+    if (tid == 256 && walk.asks()) run = walk.ask(queue);
     if (warp < 4) {
       tc_fence_after();
       issue_filter_mma(on, tmem, a_hi, img, warp >> 1, warp & 1, 1);
       umma_commit_if(on, mbar);
     }
     // while the tensor cores run: the value path's logit cotangents (8 rows per warp), then the sender rows of the first edge run
-    edge_loops(rpw, [&](auto full) { value_logit_cotangents<full>(rec, R, rpw, lane, qkv, g_xa); });
+    edge_loops(rpw, [&](auto full) { value_logit_cotangents<full>(rec, row0, rpw, lane, qkv, g_xa); });
     RevLoads L;
-    RevSums S;
-    reverse_prefetch<0>(L, rec, R.row0, lane, qkv);
+    Receiver S;
+    S.start<0>(__float_as_int(rec[row0 * kBwRec + 1]), lane, qkv);
+    reverse_prefetch<0>(L, rec, row0, lane, qkv);
     wait_mma(mbar, parity, failed, err);
-    parity ^= 1;
     BW_MARK(2);
     // this thread's shares of its row's cotangents of the invariants and of the radial derivative, both filters
     float ds0 = 0.f, ds1 = 0.f, ds2 = 0.f, ds3 = 0.f, drad = 0.f;
-    // accumulators of filter f, rows [64 hh, 64 hh + 64) -> filter tile: the 8 warps whose TMEM lanes hold them, 32 columns each
-    auto copy_half = [&](int f, int hh) {
-      if ((quad >> 1) != hh) return;
-      float v[32];
-      const int col = 32 * (warp >> 2);
-      tmem_ld32_combined(tmem + ((uint32_t)(32 * quad) << 16) + 128 * f + col, v);
+    // accumulators of filter f, rows of this group -> filter tile: the four warps of the group that can read them, 64 columns each
+    auto copy_half = [&](int f) {
+      if ((quad >> 1) != half) return;
+      const int col = 64 * ((warp >> 2) & 1);
       float* p = wt + (32 * (quad & 1) + lane) * kWStride + col;
 #pragma unroll
-      for (int k = 0; k < 32; k += 4) st4(p + k, make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+      for (int c = 0; c < 64; c += 16) {
+        float v[16];
+        tmem_ld16_combined(tmem + ((uint32_t)(32 * quad) << 16) + 128 * f + col + c, v);
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) st4(p + c + k, make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+      }
+    };
+    auto sync_group = [&] { asm volatile("bar.sync %0, 256;" ::"r"(4 + half) : "memory"); };
+    // dw of filter f stands in this group's rows: their chain of second MMAs, main and cross products by one warp each
+    auto second_chain = [&](int f) {
+      fence_async_smem();
+      tc_fence_before();
+      sync_group();
+      const int first = half ? 8 : 2;      // warps that do not copy accumulators
+      if (warp == first || warp == first + 1) {
+        tc_fence_after();
+        issue_reverse_mma(on, tmem, a_hi, img, f, half, warp - first);
+        umma_commit_if(on, mbar + 8 * (1 + 2 * f + half));
+      }
     };
     // per pair, once the second MMA chain of filter f is through: radial derivative and spherical hidden layer (all four threads of a row)
     auto finish_filter = [&](int f) {
@@ -1470,81 +1545,52 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         }
       }
     };
+    // The filter tile goes from the first group to the second and back, twice (named barriers 2: to the second group, 3: to the first).
     // ---- filter 0 ----
-    copy_half(0, 0);
+    if (half) asm volatile("bar.sync 2, 512;" ::: "memory");
+    copy_half(0);
     tc_fence_before();
-    __syncthreads();
+    sync_group();
     BW_MARK(3);
-    S.start(__float_as_int(rec[R.row0 * kBwRec + 1]));
-    edge_loops(R.nu0, [&](auto full) { reverse_edges4<0, full>(L, S, rec, wt, R.row0, R.row0, R.nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-    if (R.nu1) {
-      reverse_prefetch<0>(L, rec, R.row1, lane, qkv);
-      BW_MARK(4);
-      __syncthreads();
-      copy_half(0, 1);
-      tc_fence_before();
-      __syncthreads();
-      BW_MARK(3);
-      edge_loops(R.nu1, [&](auto full) { reverse_edges4<0, full>(L, S, rec, wt, R.row1 - 64, R.row1, R.nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-    }
-    S.flush<0>(lane, g_qkv);
-    reverse_prefetch<1>(L, rec, R.row0, lane, qkv);
+    reverse_edges<0>(L, rec, wt, row0 - 64 * half, row0, rpw, a_ptr, lane, qkv, g_qkv, n_scat, S);
     BW_MARK(4);
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (warp < 4) {
-      tc_fence_after();
-      if (warp < 2) issue_reverse_mma(on, tmem, a_hi, img, 0, warp);
-      umma_commit_if(on, mbar);
-    }
-    // while the tensor cores run: the value path, and the first half of filter 1's accumulators (columns that this chain leaves alone).
-    // What the chain yields is picked up beneath the next one.
-    edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, R, rpw, lane, g_xa, g_qkv, n_scat); });
-    copy_half(1, 0);
-    tc_fence_before();
-    __syncthreads();
-    wait_mma(mbar, parity, failed, err);      // the next loop overwrites the operand that this chain reads
-    parity ^= 1;
+    if (half) asm volatile("bar.arrive 3, 512;" ::: "memory");
+    else asm volatile("bar.arrive 2, 512;" ::: "memory");
+    second_chain(0);
+    edge_loops(rpw, [&](auto full) { value_cotangent<full>(rec, row0, rpw, lane, g_xa, g_qkv, n_scat); });
+    S.start<1>(__float_as_int(rec[row0 * kBwRec + 1]), lane, qkv);
+    reverse_prefetch<1>(L, rec, row0, lane, qkv);
+    wait_mma(mbar + 8 * (1 + half), parity, failed, err);      // the next loop overwrites the operand that this chain reads
     BW_MARK(5);
     // ---- filter 1 ----
-    S.start(__float_as_int(rec[R.row0 * kBwRec + 1]));
-    edge_loops(R.nu0, [&](auto full) { reverse_edges4<1, full>(L, S, rec, wt, R.row0, R.row0, R.nu0, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-    if (R.nu1) {
-      reverse_prefetch<1>(L, rec, R.row1, lane, qkv);
-      BW_MARK(4);
-      __syncthreads();
-      copy_half(1, 1);
-      tc_fence_before();
-      __syncthreads();
-      BW_MARK(3);
-      edge_loops(R.nu1, [&](auto full) { reverse_edges4<1, full>(L, S, rec, wt, R.row1 - 64, R.row1, R.nu1, a_ptr, lane, qkv, g_qkv, n_scat); }, 4);
-    }
-    S.flush<1>(lane, g_qkv);
-    BW_MARK(4);
-    fence_async_smem();
+    if (half) asm volatile("bar.sync 2, 512;" ::: "memory");
+    else asm volatile("bar.sync 3, 512;" ::: "memory");
+    copy_half(1);
     tc_fence_before();
-    __syncthreads();
-    if (warp < 4) {
-      tc_fence_after();
-      if (warp < 2) issue_reverse_mma(on, tmem, a_hi, img, 1, warp);
-      umma_commit_if(on, mbar);
-    }
+    sync_group();
+    BW_MARK(3);
+    reverse_edges<1>(L, rec, wt, row0 - 64 * half, row0, rpw, a_ptr, lane, qkv, g_qkv, n_scat, S);
+    BW_MARK(4);
+    if (!half) asm volatile("bar.arrive 2, 512;" ::: "memory");
+    second_chain(1);
     if (lane < kMTot) {      // ev differences of this warp's rows of the final flush: requested now, used after the last MMA
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float* rp = rec + (R.row(k) & (TE - 1)) * kBwRec;
+        const float* rp = rec + ((row0 + k) & (TE - 1)) * kBwRec;
         const int j = __float_as_int(rp[0]), i = __float_as_int(rp[1]);
         dev8[k] = ev_in[(size_t)j * kMTot + lane] - ev_in[(size_t)i * kMTot + lane];
       }
     }
+    wait_mma(mbar + 8, parity, failed, err);
+    wait_mma(mbar + 16, parity, failed, err);
     finish_filter(0);
-    wait_mma(mbar, parity, failed, err);
+    wait_mma(mbar + 24, parity, failed, err);
+    wait_mma(mbar + 32, parity, failed, err);
     parity ^= 1;
     BW_MARK(5);
     finish_filter(1);
     {
-      // the filter tile is free: it takes the four threads' shares
+      // the filter tile is free (both groups' last chains follow their loops): it takes the four threads' shares
       const int row = tid & 127, role = tid >> 7;
       st4(wt + (role * TE + row) * 4, make_float4(ds0, ds1, ds2, ds3));
       wt[(4 * 4 + role) * TE + row] = drad;
@@ -1584,7 +1630,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         // half of the pair's force on the receiver goes to this entry of the source list, the other half with the opposite sign to the
         // reversed entry
         if (on) {
-          const int2 eo = ve_orig[tile * tr + entry_of(tid)];
+          const int2 eo = ve_orig[entry0 + entry_of(tid)];
           float *g = F + 3 * (size_t)eo.x, *h = F + 3 * (size_t)eo.y;
           g[0] += 0.5f * fsx; g[1] += 0.5f * fsy; g[2] += 0.5f * fsz;
           h[0] -= 0.5f * fsx; h[1] -= 0.5f * fsy; h[2] -= 0.5f * fsz;
@@ -1610,18 +1656,17 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     }
     edge_loops(rpw, [&](auto full) {
       const float sc = -2.f * invw(deg);
-      auto row_of = [&](int k) { return full ? (k < 4 ? R.row0 + k : R.row1 + k - 4) : R.row(k); };
       auto share = [&](int k) {      // derivative with respect to the receiver's component; the partner's is its negative
-        const float* dp = wt + 4 * row_of(k) + deg;
+        const float* dp = wt + 4 * (row0 + k) + deg;
         return sc * ((dp[0] + dp[TE * 4]) + (dp[2 * TE * 4] + dp[3 * TE * 4])) * dev8[k];
       };
-      int cur_i = __float_as_int(rec[row_of(0) * kBwRec + 1]);
+      int cur_i = __float_as_int(rec[row0 * kBwRec + 1]);
       float acc = 0.f;
-      if (full && cur_i == __float_as_int(rec[row_of(7) * kBwRec + 1])) {      // eight pairs of one receiver
+      if (full && cur_i == __float_as_int(rec[(row0 + 7) * kBwRec + 1])) {      // eight pairs of one receiver
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float t = share(k);
-          const int j = __float_as_int(rec[row_of(k) * kBwRec]);
+          const int j = __float_as_int(rec[(row0 + k) * kBwRec]);
           acc += t;
           if (lane < kMTot && j < n_scat) atomicAdd(gev_in + (size_t)j * kMTot + lane, -t);
         }
@@ -1629,7 +1674,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           if (!full && k >= rpw) break;
-          const float* rp = rec + row_of(k) * kBwRec;
+          const float* rp = rec + (row0 + k) * kBwRec;
           const int i = __float_as_int(rp[1]);
           if (i != cur_i) {
             if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
@@ -1644,13 +1689,15 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
     });
     cp_async_wait_all();
+    if (tid == 256 && walk.asks()) *next_run = run;
     __syncthreads();
     BW_MARK(7);
   }
 #ifdef SO3LR_TC_TIMING
-  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[16 + q] = bph[q]; dbg[24] = tile1 - tile0; }
+  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[16 + q] = bph[q]; dbg[24] = walk.end / gridDim.x; }
   if (dbg && (tid & 31) == 0 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[32 + 8 * warp + q] = bph[q]; }
 #endif
+  if (tid == 256) walk.finish(queue);
   cp_async_wait_all();
   tc_fence_before();
   __syncthreads();
@@ -1670,7 +1717,7 @@ int configure_attention_tc_kernels() {
 }
 
 int valid_edges_reserve(ValidEdges* V, int n_rows, long long capacity) {
-  if (!V->total) SO3LR_CUDA_CHECK(dev_alloc(&V->total, 1));
+  if (!V->total) SO3LR_CUDA_CHECK(dev_alloc(&V->total, 3));      // and the tile queue
   const int n_blocks = (n_rows + kCompactRows - 1) / kCompactRows;
   if (n_blocks > V->block_cap) {
     dev_free(V->blocks);
@@ -1796,7 +1843,7 @@ int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, i
     SO3LR_CUDA_CHECK(cudaMemcpyAsync(xa, x_in, (size_t)n_recv * kF * sizeof(float), cudaMemcpyDeviceToDevice, s));
     SO3LR_CUDA_CHECK(cudaMemcpyAsync(ev1, ev_in, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
   }
-  { launch_chained(attn_fwd_tc_kernel, sm_count(), kFwThreads, kSmemFwd, s, L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym); count_launch(); }
+  { launch_chained(attn_fwd_tc_kernel, sm_count(), kFwThreads, kSmemFwd, s, L.tc_img_fwd, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, xa, ev1, err, tc_debug_buffer(), V.asym, V.total + 1); count_launch(); }
   return kOk;
 }
 
@@ -1809,7 +1856,7 @@ int launch_attn_bwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, i
   if (!gq_preset) SO3LR_CUDA_CHECK(cudaMemsetAsync(g_qkv, 0, (size_t)n_recv * kProj * sizeof(float), s));
   if (!gev_preset) SO3LR_CUDA_CHECK(cudaMemcpyAsync(gev_in, gev1, (size_t)n_recv * kMTot * sizeof(float), cudaMemcpyDeviceToDevice, s));
   { launch_chained(attn_bwd_tc_kernel<false>, sm_count(), kBwThreads, kSmemBwd, s, L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
-                                                              g_qkv, gev_in, F, virial, err, tc_debug_buffer(), nullptr, nullptr, n_own); count_launch(); }
+                                                              g_qkv, gev_in, F, virial, err, tc_debug_buffer(), nullptr, nullptr, V.total + 1, n_own); count_launch(); }
   return kOk;
 }
 
@@ -1818,7 +1865,7 @@ int launch_attn_bwd_tc_graph(cudaStream_t s, const LayerDev& L, const ValidEdges
   if (n_recv <= 0) return kOk;
   if (n_recv != V.n_rows || !V.orig) return kInvalidArgument;
   { launch_chained(attn_bwd_tc_kernel<true>, sm_count(), kBwThreads, kSmemBwd, s, L.tc_img, L.sph1_k, L.sph1_b, n_recv, V.total, V.i, V.j, V.d, qkv, ev_in, g_xa, gev1,
-                                                             g_qkv, gev_in, g_dR, nullptr, err, nullptr, V.orig, asym, 0); count_launch(); }
+                                                             g_qkv, gev_in, g_dR, nullptr, err, nullptr, V.orig, asym, V.total + 1, 0); count_launch(); }
   return kOk;
 }
 

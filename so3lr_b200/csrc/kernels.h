@@ -175,7 +175,7 @@ void launch_attn_bwd_mma(cudaStream_t s, const LayerDev& L, int n_recv, int n, c
 // Short-range pairs inside the cutoff, compacted once per evaluation, one entry per undirected pair: i[p] is its end with the smaller
 // index (the entries of one i are consecutive), j[p] the partner and d[p] = (dx, dy, dz, |dR|) from i to j, p < *total.  Caller-supplied lists whose entries do not come in reversed pairs (*asym != 0) keep every entry i <- j.
 struct ValidEdges {
-  int* total = nullptr;     // number of entries (on the device)
+  int* total = nullptr;     // number of entries | the two words of the tile queue (on the device)
   int* blocks = nullptr;    // scratch of the build
   int block_cap = 0;
   int* i = nullptr;
