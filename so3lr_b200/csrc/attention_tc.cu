@@ -47,7 +47,6 @@ constexpr int kAHalf = 16 * kLboA;            // one FP16 matrix of 128 rows x 1
 constexpr int kWStride = 132;                 // floats per row of the filter tile
 constexpr int kFwRec = 36;                    // floats per forward record: j | i | cutoff / nbar | - | Y[24] | padding (bank spread)
 constexpr int kFwThreads = 512;
-constexpr int kFwIssuer = 128;       // forward kernel: the thread that issues the MMAs (its own preparation is the shortest)
 constexpr int kBwRec = 52;                    // floats per reverse record (48 used; 52 spreads consecutive rows over the banks)
 constexpr int kBwThreads = 512;
 constexpr float kInvNbar = 1.0f / kAvgNumNeighbors;
@@ -62,19 +61,17 @@ constexpr int kOffA = kTcImageBytes;                         // A operand (hi | 
 constexpr int kARegion = TE * kWStride * 4;                  // 67584 >= 2 * kAHalf
 static_assert(kARegion >= 2 * kAHalf, "A region");
 constexpr int kOffFwRec = kOffA + kARegion;
+constexpr int kSphFloats = 4 * 136;           // first spherical layer: 8 floats per hidden unit, 8 more after every 16 units (banks)
 constexpr int kOffFwSph = kOffFwRec + TE * kFwRec * 4;
-constexpr int kOffFwMisc = kOffFwSph + 512 * 4;
-constexpr int kEvStride = 28;                                // floats per staged ev row (24 used; 112 B keeps 16-byte reads conflict-free)
-constexpr int kOffFwStIJ = kOffFwMisc + 64;                  // staged inputs of the next tile: (i, j) | displacement | ev rows of both atoms
+constexpr int kOffFwMisc = kOffFwSph + kSphFloats * 4;
+constexpr int kOffFwStIJ = kOffFwMisc + 64;                  // staged inputs of the next tile: (i, j) | displacement
 constexpr int kOffFwStD = kOffFwStIJ + TE * 8;
-constexpr int kOffFwStEv = kOffFwStD + TE * 16;
-constexpr int kSmemFwd = kOffFwStEv + TE * 2 * kEvStride * 4;
+constexpr int kSmemFwd = kOffFwStD + TE * 16;
 // reverse kernel: the filter tile holds 64 edges at a time
 constexpr int kOffBwW = kOffA + kARegion;
 constexpr int kOffBwRec = kOffBwW + 64 * kWStride * 4;
 constexpr int kOffBwSph = kOffBwRec + TE * kBwRec * 4;
-constexpr int kBwSphFloats = 4 * 136;         // reverse kernel: first spherical layer, 8 floats per hidden unit, 8 more after every 16 units (banks)
-constexpr int kOffBwMisc = kOffBwSph + kBwSphFloats * 4;
+constexpr int kOffBwMisc = kOffBwSph + kSphFloats * 4;
 constexpr int kOffBwStIJ = kOffBwMisc + 64;                  // staged inputs of the next tile: (i, j) | displacement
 constexpr int kOffBwStD = kOffBwStIJ + TE * 8;
 constexpr int kSmemBwd = kOffBwStD + TE * 16;
@@ -150,16 +147,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ uint32_t make_idesc(int n, int b_mn_major) {
   return (1u << 4) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TE >> 4) << 24);
 }
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The same for a whole warp that runs the issue code: `on` is set in one lane, which issues.  Descriptors then are the same in all lanes and
-// stay in uniform registers: 43 cycles from one MMA to the next instead of 53 where a single thread has branched off.
+// A whole warp runs the issue code; `on` is set in one lane, which issues.  Descriptors then are the same in all lanes and stay in uniform
+// registers: 43 cycles from one MMA to the next instead of 53 where a single thread has branched off.
 __device__ __forceinline__ void umma_if(uint32_t on, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
@@ -198,9 +187,6 @@ __device__ __forceinline__ uint32_t elect_one() {
       "}\n" : "=r"(on));
   return on;
 }
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
   for (int it = 0; it < kWaitSpins; ++it) {
     uint32_t ok;
@@ -235,29 +221,9 @@ __device__ __forceinline__ void wait_mma(uint32_t mbar, uint32_t parity, volatil
   tc_fence_after();
 }
 
-// main + cross / 2048 of 32 columns (cross accumulators sit 256 columns above the main ones)
-__device__ __forceinline__ void tmem_ld32_combined(uint32_t taddr, float* v) {
-  uint32_t a[32], b[32];      // both loads in flight before the one wait
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%65];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]), "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]), "=r"(a[16]), "=r"(a[17]), "=r"(a[18]), "=r"(a[19]), "=r"(a[20]), "=r"(a[21]), "=r"(a[22]), "=r"(a[23]), "=r"(a[24]), "=r"(a[25]), "=r"(a[26]), "=r"(a[27]), "=r"(a[28]), "=r"(a[29]), "=r"(a[30]), "=r"(a[31]),
-        "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]), "=r"(b[8]), "=r"(b[9]), "=r"(b[10]), "=r"(b[11]), "=r"(b[12]), "=r"(b[13]), "=r"(b[14]), "=r"(b[15]), "=r"(b[16]), "=r"(b[17]), "=r"(b[18]), "=r"(b[19]), "=r"(b[20]), "=r"(b[21]), "=r"(b[22]), "=r"(b[23]), "=r"(b[24]), "=r"(b[25]), "=r"(b[26]), "=r"(b[27]), "=r"(b[28]), "=r"(b[29]), "=r"(b[30]), "=r"(b[31])
-      : "r"(taddr), "r"(taddr + 256)
-      : "memory");
-  const float2 s2 = make_float2(kLoInv, kLoInv);
-#pragma unroll
-  for (int k = 0; k < 32; k += 2) {
-    const float2 r = __ffma2_rn(make_float2(__uint_as_float(b[k]), __uint_as_float(b[k + 1])), s2,
-                                make_float2(__uint_as_float(a[k]), __uint_as_float(a[k + 1])));
-    v[k] = r.x; v[k + 1] = r.y;
-  }
-}
-
-// the same for 16 columns (half the registers: for places with much else live)
+// main + cross / 2048 of 16 columns (cross accumulators sit 256 columns above the main ones)
 __device__ __forceinline__ void tmem_ld16_combined(uint32_t taddr, float* v) {
-  uint32_t a[16], b[16];
+  uint32_t a[16], b[16];      // both loads in flight before the one wait
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
@@ -288,19 +254,35 @@ __device__ __forceinline__ void tmem_ld8_combined(uint32_t taddr, float* v) {
   for (int k = 0; k < 8; ++k) v[k] = fmaf(__uint_as_float(b[k]), kLoInv, __uint_as_float(a[k]));
 }
 
-__device__ __forceinline__ void invariants(const float* __restrict__ evi, const float* __restrict__ evj, float* s) {
-  float d[kMTot];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    const float4 a = ld4(evj + 4 * c), b = ld4(evi + 4 * c);
-    d[4 * c] = a.x - b.x; d[4 * c + 1] = a.y - b.y; d[4 * c + 2] = a.z - b.z; d[4 * c + 3] = a.w - b.w;
+// A pair's ev rows, a quarter per thread of four neighbouring ones: request (`begin`), then the invariants of their difference in all four
+struct PairInvariants {
+  float4 i0, j0, i1, j1;
+  int q;
+  __device__ __forceinline__ void begin(const float* evi, const float* evj, int quarter) {
+    q = quarter;
+    i0 = ld4(evi + 4 * q); j0 = ld4(evj + 4 * q);
+    i1 = f4_zero(); j1 = f4_zero();
+    if (q < 2) { i1 = ld4(evi + 16 + 4 * q); j1 = ld4(evj + 16 + 4 * q); }
   }
-  s[0] = s[1] = s[2] = s[3] = 0.f;
+  __device__ __forceinline__ void finish(float (&s)[4]) const {
+    const float dv[8] = {j0.x - i0.x, j0.y - i0.y, j0.z - i0.z, j0.w - i0.w, j1.x - i1.x, j1.y - i1.y, j1.z - i1.z, j1.w - i1.w};
+    s[0] = s[1] = s[2] = s[3] = 0.f;
 #pragma unroll
-  for (int m = 0; m < kMTot; ++m) s[degree_of(m)] = fmaf(d[m], d[m], s[degree_of(m)]);
+    for (int c = 0; c < 8; ++c) {      // components 4 q + c (degrees 1..3, and 15 of degree 4), then 16 + 4 q + (c - 4) of degree 4
+      const float x2 = dv[c] * dv[c];
+      if (c >= 4) { s[3] += x2; continue; }
+      const int l = degree_of(4 * q + c);
 #pragma unroll
-  for (int l = 0; l < 4; ++l) s[l] *= invw(l);
-}
+      for (int g = 0; g < 4; ++g) s[g] += l == g ? x2 : 0.f;
+    }
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      s[l] += __shfl_xor_sync(0xffffffffu, s[l], 1);
+      s[l] += __shfl_xor_sync(0xffffffffu, s[l], 2);
+      s[l] *= invw(l);
+    }
+  }
+};
 
 // Column order of the Chebyshev block of the A operand: column k < 32 holds T_{2k}, column 32 + k holds T_{2k+1} (the rows of
 // the coefficient image are permuted to match).  Two threads share an edge: `odd` = 0 writes the even terms (chunks 0..3),
@@ -327,24 +309,7 @@ __device__ __forceinline__ void store_chebyshev_half(unsigned char* a_hi, int ro
     store_chunk(a_hi, 4 * odd + c, row, v);
   }
 }
-// hidden layer of spherical filter f into chunks 8 + 4 f .. 11 + 4 f
-__device__ __forceinline__ void store_spherical_hidden_f(unsigned char* a_hi, int row, const float* s, const float* sph8, int f) {
-  // sph8: per (filter, hidden unit) eight floats: the four first-layer weights, the bias, padding
-#pragma unroll
-  for (int c8 = 0; c8 < 4; ++c8) {
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float* p = sph8 + (f * 32 + 8 * c8 + q) * 8;
-      const float4 k = ld4(p);
-      const float z = fmaf(s[0], k.x, fmaf(s[1], k.y, fmaf(s[2], k.z, fmaf(s[3], k.w, p[4]))));
-      v[q] = __fdividef(z, 1.f + __expf(-z));
-    }
-    store_chunk(a_hi, 8 + 4 * f + c8, row, v);
-  }
-}
-
-// first-layer weights of hidden unit u of filter f in the reverse kernel's shared memory
+// first-layer weights of hidden unit u of filter f in shared memory: the four weights, the bias, padding
 __device__ __forceinline__ int sph_at(int f, int u) { return (f * 32 + u) * 8 + (2 * f + (u >> 4)) * 8; }
 // One of four neighbouring threads of a pair: two of the eight chunks of both hidden layers
 __device__ __forceinline__ void store_spherical_hidden_quarter(unsigned char* a_hi, int row, const float* s, const float* sph, int quarter) {
@@ -376,39 +341,31 @@ __device__ __forceinline__ uint64_t desc_base(uint32_t lbo, uint32_t sbo) {
 //   K2T_f hi | lo : [128 features][32 hidden], core (n/8, k/8) at (k/8) * 2048 + (n/8) * 128          (4 x 8 KB)
 // w = Phi * C + hs_f * K2_f: main accumulators in TMEM columns [0, 256), cross accumulators in [256, 512)
 // The Chebyshev steps (part 0) read chunks 0..7 of A only, the steps of the spherical hidden layers (part 1) chunks 8..15: part 0 is
-// issued as soon as the two threads per entry that write the Chebyshev terms are through, while the other two still gather `ev`
-// rows and evaluate the hidden layers.
-__device__ __noinline__ void issue_forward_mma(uint32_t tmem, uint32_t a_hi, uint32_t img, int part) {
+// issued as soon as the two threads per entry that write the Chebyshev terms are through, while the others still evaluate the hidden
+// layers.  Four warps share the work, one per filter and accumulator (`cross`: hi * lo + lo * hi): the issue of a chain waits behind the
+// load / store queue of its scheduler.
+__device__ __forceinline__ void issue_forward_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int cross, int part) {
   const uint64_t da = desc_base(kLboA, 128) + (a_hi >> 4), dal = da + (kAHalf >> 4);
-  const uint64_t dc = desc_base(4096, 128) + (img >> 4), dcl = dc + (32768 >> 4);
-  const uint64_t dk = desc_base(2048, 128) + ((img + 65536) >> 4), dkl = dk + (16384 >> 4);
-  const uint32_t id256 = make_idesc(256, 0), id128 = make_idesc(128, 0);
+  const uint64_t dc = desc_base(4096, 128) + ((img + f * 2048) >> 4), dcl = dc + (32768 >> 4);
+  const uint64_t dk = desc_base(2048, 128) + ((img + 65536 + f * 8192) >> 4), dkl = dk + (16384 >> 4);
+  const uint32_t id128 = make_idesc(128, 0), d = tmem + 128 * f + 256 * cross;
   // K steps 1 and 3 hold the Chebyshev terms of order 32..63 (even terms, then odd terms, 32 columns each).  Their coefficients
   // are below 2^-12 of the filter scale (the expansion converges geometrically), so their hi * lo cross terms are below 2^-23 of
   // it, like the lo * lo terms that are dropped everywhere: those steps issue the hi * hi product only.
-  if (part == 0) {
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      const uint64_t ah = da + ks * (2 * kLboA >> 4), al = dal + ks * (2 * kLboA >> 4);
-      const uint64_t bh = dc + ks * (2 * 4096 >> 4), bl = dcl + ks * (2 * 4096 >> 4);
-      umma(tmem, ah, bh, id256, ks > 0);
-      if (ks == 1 || ks == 3) continue;
-      umma(tmem + 256, ah, bl, id256, ks > 0);
-      umma(tmem + 256, al, bh, id256, 1);
+  for (int ks = 0; ks < 6; ++ks) {
+    if ((ks >= 4) != (part == 1)) continue;
+    const int chunk = ks < 4 ? 2 * ks : 8 + 4 * f + 2 * (ks - 4);
+    const uint64_t ah = da + chunk * (kLboA >> 4), al = dal + chunk * (kLboA >> 4);
+    const uint64_t bh = ks < 4 ? dc + ks * (2 * 4096 >> 4) : dk + (ks - 4) * (2 * 2048 >> 4);
+    const uint64_t bl = ks < 4 ? dcl + ks * (2 * 4096 >> 4) : dkl + (ks - 4) * (2 * 2048 >> 4);
+    if (!cross) {
+      umma_if(on, d, ah, bh, id128, ks > 0);
+    } else if (ks != 1 && ks != 3) {
+      umma_if(on, d, ah, bl, id128, ks > 0);
+      umma_if(on, d, al, bh, id128, 1);
     }
-    return;
   }
-#pragma unroll
-  for (int f = 0; f < 2; ++f)
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-      const int chunk = 8 + 4 * f + 2 * ks;
-      const uint64_t ah = da + chunk * (kLboA >> 4), al = dal + chunk * (kLboA >> 4);
-      const uint64_t bh = dk + (f * 8192 + ks * 2 * 2048 >> 4), bl = dkl + (f * 8192 + ks * 2 * 2048 >> 4);
-      umma(tmem + 128 * f, ah, bh, id128, 1);
-      umma(tmem + 256 + 128 * f, ah, bl, id128, 1);
-      umma(tmem + 256 + 128 * f, al, bh, id128, 1);
-    }
 }
 
 // Reverse kernel, one image for both directions, per filter f (24,576 bytes each; hi of f = 0, 1 then lo of f = 0, 1): the 96
@@ -417,8 +374,7 @@ __device__ __noinline__ void issue_forward_mma(uint32_t tmem, uint32_t a_hi, uin
 // Forward product (B read MN-major: N = features, K = rows): w_f = [Phi | hs_f] * [C_f ; K2_f], main accumulators in TMEM
 // columns [128 f, 128 f + 128), cross 256 columns above.
 constexpr int kRevImgFilter = 16 * 1536;
-// part 0: the four Chebyshev steps, part 1: the two steps of the filter's hidden layer (see issue_forward_mma).  Four warps share the work, one
-// per filter and accumulator (`cross`: hi * lo + lo * hi): the issue of a chain waits behind the load / store queue of its scheduler.
+// part 0: the four Chebyshev steps, part 1: the two steps of the filter's hidden layer (see issue_forward_mma)
 __device__ __forceinline__ void issue_filter_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int cross, int part) {
   const uint64_t da = desc_base(kLboA, 128) + (a_hi >> 4), dal = da + (kAHalf >> 4);
   const uint64_t db = desc_base(128, 1536) + ((img + f * kRevImgFilter) >> 4), dbl = db + (2 * kRevImgFilter >> 4);
@@ -642,10 +598,9 @@ __device__ __forceinline__ void edge_loops(int share, Body&& body, int run = 8) 
 // ------------------------------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------------------------------
-// 16 warps.  Per tile: (1) four threads per edge prepare the A operand (geometry + Chebyshev terms 0..31 | terms 32..63 | hidden
-// layer of filter 0 | of filter 1) from inputs that were staged in shared memory with cp.async during the previous tile;
-// (2) one thread issues the MMA chains of the two filters (one commit each) while every warp already has the sender rows of
-// its 8 edges in flight and 128 threads stage the next tile; (3) per filter: tensor memory -> shared tile, then the edge loop.
+// 16 warps.  Per tile: (1) preparation of the A operand and the records: Chebyshev terms by two threads per pair, geometry by a third (the
+// fourth's warps issue the MMAs), then the hidden layers by four neighbouring threads per pair; (2) the MMA chains of the two filters, while every warp already has the sender rows
+// of its 8 pairs in flight; (3) per filter: tensor memory -> shared tile, then the edge loop.
 __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsigned char* __restrict__ img_g, const float* __restrict__ sph1_k,
                                                                     const float* __restrict__ sph1_b, int n_recv,
                                                                     const int* n_listed, const int* ve_i,
@@ -654,25 +609,26 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
                                                                     float* __restrict__ xa, float* __restrict__ ev1, int* __restrict__ err,
                                                                     long long* __restrict__ dbg, const int* asym, int* queue) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   float* rec = reinterpret_cast<float*>(smem + kOffFwRec);
   float* sph = reinterpret_cast<float*>(smem + kOffFwSph);
   float* wt = reinterpret_cast<float*>(smem + kOffA);
   int* st_ij = reinterpret_cast<int*>(smem + kOffFwStIJ);
   float4* st_d = reinterpret_cast<float4*>(smem + kOffFwStD);
-  float* st_ev = reinterpret_cast<float*>(smem + kOffFwStEv);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffFwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffFwMisc + 16);
+  volatile int* failed = reinterpret_cast<volatile int*>(smem + kOffFwMisc + 20);
   int* next_run = reinterpret_cast<int*>(smem + kOffFwMisc + 32);
   for (int k = tid; k < kTcImageBytes / 16; k += kFwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kFwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
     const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
-    sph[k] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
+    sph[sph_at(f, c) + q] = q < 4 ? sph1_k[f * 128 + q * 32 + c] : (q == 4 ? sph1_b[f * 32 + c] : 0.f);
   }
   const uint32_t mbar0 = smem_u32(mbar_p);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(mbar0));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *failed = 0;
   }
   grid_dep_sync();
   const long long n_edges = *n_listed;
@@ -683,27 +639,18 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   const int pad_i = ve_i[n_edges - 1];
   // partners below n_scat receive the pair's other direction (j <- i)
   const int n_scat = asym && *asym != 0 ? 0 : n_recv;
-  // inputs of one tile into the staging buffers: receiver / sender, displacement, both atoms' ev rows (threads 256..383)
+  // (i, j) and displacement of one tile's pairs into the staging buffers (threads 256..383): in flight beneath the tile before
   auto stage_tile = [&](int tile) {
     if (tid < 256 || tid >= 384 || tile >= walk.end) return;
     const int row = tid - 256;
     const long long e = (long long)tile * tr + row;
-    int i = pad_i, j = pad_i;
     if (row < tr && e < n_edges) {
-      i = ve_i[e]; j = ve_j[e];
+      cp_async4(st_ij + 2 * row, ve_i + e); cp_async4(st_ij + 2 * row + 1, ve_j + e);
       cp_async16(st_d + row, ve_d + e);
     } else {
+      st_ij[2 * row] = pad_i; st_ij[2 * row + 1] = pad_i;
       st_d[row] = make_float4(1.f, 0.f, 0.f, 1.f);
     }
-    st_ij[2 * row] = i; st_ij[2 * row + 1] = j;
-    const float* gi = ev_in + (size_t)i * kMTot;
-    const float* gj = ev_in + (size_t)j * kMTot;
-    // receivers' rows in the first half of the buffer, senders' rows in the second: consecutive entries are 112 bytes apart in
-    // either half, which spreads the 16-byte accesses of eight threads over all banks (interleaved, 224 bytes apart, they collide
-    // in pairs)
-    float* d = st_ev + row * kEvStride;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) { cp_async16(d + 4 * c, gi + 4 * c); cp_async16(d + TE * kEvStride + 4 * c, gj + 4 * c); }
   };
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
@@ -715,7 +662,9 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_p;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_p, 0);
+  const uint32_t on = elect_one();
+  const bool issues = warp >= 12;      // one warp per scheduler, of those with the shortest preparation
   const uint32_t a_hi = smem_u32(smem + kOffA), img = smem_u32(smem + kOffImg);
   const int col = 4 * lane;
   const int deg = degree_of(lane < kMTot ? lane : 0);
@@ -731,84 +680,75 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   for (; walk.tile < walk.end; walk.tile = walk.next) {
     const long long entry0 = (long long)walk.tile * tr;
     int run = 0;
-    // ---- per-edge preparation from the staged inputs ----
+    // ---- per-edge preparation ----
     {
+      const int hrow = 8 * warp + (lane >> 2);
+      PairInvariants I;      // requested first, used last
+      I.begin(ev_in + (size_t)st_ij[2 * hrow] * kMTot, ev_in + (size_t)st_ij[2 * hrow + 1] * kMTot, lane & 3);
       const int row = tid & 127, role = tid >> 7;
       const bool valid = row < tr && entry0 + row < n_edges;
+      const float4 d = st_d[row];
+      const float r = d.w;
       if (role < 2) {
-        const float4 d = st_d[row];
-        const float r = d.w;
-        // the Chebyshev chunks first: once these 256 threads are through, their share of the MMA chain starts beneath the rest
-        // of the preparation
+        // once these 256 threads are through, their share of the MMA chains starts beneath the rest of the preparation
         store_chebyshev_half(smem + kOffA, row, r, valid, role);
         fence_async_smem();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (tid == kFwIssuer) {
-          tc_fence_after();
-          issue_forward_mma(tmem, a_hi, img, 0);
-        }
-        if (role == 0) {
-          const float ir = 1.f / r;
-          float cut, dcut;
-          phys_cutoff(r, cut, dcut);
-          float Y[kMTot];
-          sph_harm_24(d.x * ir, d.y * ir, d.z * ir, Y);
-          float* rp = rec + row * kFwRec;
-          st4(rp, make_float4(__int_as_float(st_ij[2 * row + 1]), __int_as_float(st_ij[2 * row]), valid ? cut * kInvNbar : 0.f, 0.f));
+        asm volatile("bar.arrive 1, 384;" ::: "memory");
+      } else if (role == 2) {
+        const float ir = 1.f / r;
+        float cut, dcut;
+        phys_cutoff(r, cut, dcut);
+        float Y[kMTot];
+        sph_harm_24(d.x * ir, d.y * ir, d.z * ir, Y);
+        float* rp = rec + row * kFwRec;
+        st4(rp, make_float4(__int_as_float(st_ij[2 * row + 1]), __int_as_float(st_ij[2 * row]), valid ? cut * kInvNbar : 0.f, 0.f));
 #pragma unroll
-          for (int c = 0; c < 6; ++c) st4(rp + 4 + 4 * c, make_float4(Y[4 * c], Y[4 * c + 1], Y[4 * c + 2], Y[4 * c + 3]));
-        }
-      } else {
-        float s[4];
-        invariants(st_ev + row * kEvStride, st_ev + (TE + row) * kEvStride, s);
-        store_spherical_hidden_f(smem + kOffA, row, s, sph, role - 2);
+        for (int c = 0; c < 6; ++c) st4(rp + 4 + 4 * c, make_float4(Y[4 * c], Y[4 * c + 1], Y[4 * c + 2], Y[4 * c + 3]));
+      }
+      float s[4];
+      I.finish(s);
+      store_spherical_hidden_quarter(smem + kOffA, hrow, s, sph, lane & 3);
+      if (issues) {
+        asm volatile("bar.sync 1, 384;" ::: "memory");
+        tc_fence_after();
+        issue_forward_mma(on, tmem, a_hi, img, (warp >> 1) & 1, warp & 1, 0);
       }
     }
     TC_MARK(0);
-    // the partners' q / k rows of filter 0 for this warp's pairs and the first receiver's rows, requested before the barrier (the
-    // indices are in the staging buffer since the previous tile): the warps with the shorter preparation start their gathers while
-    // the others still work, and all of them are in flight while the tensor cores run
+    // the partners' q / k rows of filter 0 for this warp's pairs and the first receiver's rows: in flight while the tensor cores run.  The
+    // indices are in the staging buffer since the previous tile, so the warps ask for them before the barrier; those that issue the MMAs do
+    // after it, because an MMA waits behind the loads in its scheduler's queue
     float4 qj[8], kj[8], qi, ki, vi;
-    int cur_i;
+    int cur_i, jr[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const float* pj = qkv + (size_t)st_ij[2 * ((k0 + u) & (TE - 1)) + 1] * kProj + col;      // past this warp's share: not used
-      qj[u] = ld4(pj);
-      kj[u] = ld4(pj + kF);
-    }
+    for (int u = 0; u < 8; ++u) jr[u] = st_ij[2 * ((k0 + u) & (TE - 1)) + 1];      // past this warp's share: not used
     cur_i = st_ij[2 * k0];
-    {
+    auto request_rows = [&] {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float* pj = qkv + (size_t)jr[u] * kProj + col;
+        qj[u] = ld4(pj);
+        kj[u] = ld4(pj + kF);
+      }
       const float* pi = qkv + (size_t)cur_i * kProj + col;
       qi = ld4(pi); ki = ld4(pi + kF); vi = ld4(pi + 2 * kF);
-    }
+    };
+    if (!issues) request_rows();
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     TC_MARK(1);
     walk.look_ahead(next_run);
+    if (issues) {
+      tc_fence_after();
+      issue_forward_mma(on, tmem, a_hi, img, (warp >> 1) & 1, warp & 1, 1);
+      umma_commit_if(on, mbar0);
+      request_rows();
+    }
     stage_tile(walk.next);
     if (tid == kFwThreads - 1 && walk.asks()) run = walk.ask(queue);
-    bool done = true;
-    if (tid == kFwIssuer) {
-      tc_fence_after();
-#ifdef SO3LR_TC_TIMING
-      const long long q0 = clock64();
-#endif
-      issue_forward_mma(tmem, a_hi, img, 1);
-      umma_commit(mbar0);
-#ifdef SO3LR_TC_TIMING
-      const long long q1 = clock64();
-#endif
-      done = mbar_wait(mbar0, parity);
-#ifdef SO3LR_TC_TIMING
-      if (dbg && blockIdx.x == 0) { dbg[9] += q1 - q0; dbg[10] += clock64() - q1; }
-#endif
-    }
-    if (!__syncthreads_and(done)) {
-      if (tid == 0) atomicExch(err, 1);
-      break;
-    }
-    tc_fence_after();
+    wait_mma(mbar0, parity, failed, err);
+    parity ^= 1;
     TC_MARK(2);
     // ---- filter 0: invariant logits, feature sums ----
     tmem_to_tile(tmem, 0, warp, lane, wt);
@@ -894,7 +834,6 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     qi = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
     ki = ld4(qkv + (size_t)cur_i * kProj + 4 * kF + col);
     TC_MARK(4);
-    parity ^= 1;
     __syncthreads();
     TC_MARK(5);
     // ---- filter 1: equivariant logits, spherical-harmonic sums ----
@@ -1386,13 +1325,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     float dev8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // ---- per-edge preparation ----
     {
-      // a quarter of a pair's ev rows per thread (four neighbouring threads per pair): requested first, used last
       const int hrow = 8 * warp + (lane >> 2), q = lane & 3;
-      const float* evi = ev_in + (size_t)st_ij[2 * hrow] * kMTot;
-      const float* evj = ev_in + (size_t)st_ij[2 * hrow + 1] * kMTot;
-      const float4 ei0 = ld4(evi + 4 * q), ej0 = ld4(evj + 4 * q);
-      float4 ei1 = f4_zero(), ej1 = f4_zero();
-      if (q < 2) { ei1 = ld4(evi + 16 + 4 * q); ej1 = ld4(evj + 16 + 4 * q); }
+      PairInvariants I;      // requested first, used last
+      I.begin(ev_in + (size_t)st_ij[2 * hrow] * kMTot, ev_in + (size_t)st_ij[2 * hrow + 1] * kMTot, q);
       const int row = tid & 127, role = tid >> 7;
       const int k = entry_of(row);
       const bool valid = k >= 0 && entry0 + k < n_edges;
@@ -1423,26 +1358,10 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         }
         angular_end(gev1 + (size_t)(role == 2 ? i : j) * kMTot, ux, uy, uz, role == 2 ? 1.f : -1.f, rp + 8 + 4 * role, rp + 16 + 8 * role);
       }
-      {
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-        const float dv[8] = {ej0.x - ei0.x, ej0.y - ei0.y, ej0.z - ei0.z, ej0.w - ei0.w, ej1.x - ei1.x, ej1.y - ei1.y, ej1.z - ei1.z, ej1.w - ei1.w};
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {      // components 4 q + c (degrees 1..3, and 15 of degree 4), then 16 + 4 q + (c - 4) of degree 4
-          const float x2 = dv[c] * dv[c];
-          if (c >= 4) { s[3] += x2; continue; }
-          const int l = degree_of(4 * q + c);
-#pragma unroll
-          for (int g = 0; g < 4; ++g) s[g] += l == g ? x2 : 0.f;
-        }
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          s[l] += __shfl_xor_sync(0xffffffffu, s[l], 1);
-          s[l] += __shfl_xor_sync(0xffffffffu, s[l], 2);
-          s[l] *= invw(l);
-        }
-        if (q == 0) st4(rec + hrow * kBwRec + 4, make_float4(s[0], s[1], s[2], s[3]));
-        store_spherical_hidden_quarter(a_ptr, hrow, s, sph, q);
-      }
+      float s[4];
+      I.finish(s);
+      if (q == 0) st4(rec + hrow * kBwRec + 4, make_float4(s[0], s[1], s[2], s[3]));
+      store_spherical_hidden_quarter(a_ptr, hrow, s, sph, q);
     }
     BW_MARK(0);
     fence_async_smem();
