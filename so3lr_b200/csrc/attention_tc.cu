@@ -395,12 +395,14 @@ __device__ __forceinline__ void issue_filter_mma(uint32_t on, uint32_t tmem, uin
   }
 }
 
-// 16-warp version: warps w, w + 4, w + 8, w + 12 share a quadrant and take 32 columns each; all 128 rows
+// accumulators of filter f, rows of a warp's group (warps 0..7 rows 0..63, warps 8..15 rows 64..127) -> filter tile: the four warps of the
+// group that can read them, 64 columns each
 __device__ __forceinline__ void tmem_to_tile(uint32_t tmem, int f, int warp, int lane, float* wt) {
-  const int q = warp & 3, col = 32 * (warp >> 2);
+  const int q = warp & 3, col = 64 * ((warp >> 2) & 1);
+  if ((q >> 1) != (warp >> 3)) return;
   float* p = wt + (32 * q + lane) * kWStride + col;
 #pragma unroll
-  for (int c = 0; c < 32; c += 16) {      // 16 columns at a time: the sender rows in flight hold most of the registers
+  for (int c = 0; c < 64; c += 16) {      // 16 columns at a time: the sender rows in flight hold most of the registers
     float v[16];
     tmem_ld16_combined(tmem + ((uint32_t)(32 * q) << 16) + 128 * f + col + c, v);
 #pragma unroll
@@ -639,12 +641,15 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   const int pad_i = ve_i[n_edges - 1];
   // partners below n_scat receive the pair's other direction (j <- i)
   const int n_scat = asym && *asym != 0 ? 0 : n_recv;
+  const int half = warp >> 3;            // the rows of this warp's pairs: [64 half, 64 half + 8 rpw)
+  // list entry of a tile row within the tile, -1 for a padding row
+  auto entry_of = [&](int row) { return (row & 63) < 8 * rpw ? (row & 63) + (row >> 6) * 8 * rpw : -1; };
   // (i, j) and displacement of one tile's pairs into the staging buffers (threads 256..383): in flight beneath the tile before
   auto stage_tile = [&](int tile) {
     if (tid < 256 || tid >= 384 || tile >= walk.end) return;
-    const int row = tid - 256;
-    const long long e = (long long)tile * tr + row;
-    if (row < tr && e < n_edges) {
+    const int row = tid - 256, k = entry_of(row);
+    const long long e = (long long)tile * tr + k;
+    if (k >= 0 && e < n_edges) {
       cp_async4(st_ij + 2 * row, ve_i + e); cp_async4(st_ij + 2 * row + 1, ve_j + e);
       cp_async16(st_d + row, ve_d + e);
     } else {
@@ -668,7 +673,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   const uint32_t a_hi = smem_u32(smem + kOffA), img = smem_u32(smem + kOffImg);
   const int col = 4 * lane;
   const int deg = degree_of(lane < kMTot ? lane : 0);
-  const int k0 = rpw * warp;             // this warp's rows of the tile in the edge loop
+  const int k0 = 64 * half + rpw * (warp & 7);      // this warp's rows of the tile in the edge loop
+  auto sync_group = [&] { asm volatile("bar.sync %0, 256;" ::"r"(2 + half) : "memory"); };
   uint32_t parity = 0;
 #ifdef SO3LR_TC_TIMING
   long long tph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -686,7 +692,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
       PairInvariants I;      // requested first, used last
       I.begin(ev_in + (size_t)st_ij[2 * hrow] * kMTot, ev_in + (size_t)st_ij[2 * hrow + 1] * kMTot, lane & 3);
       const int row = tid & 127, role = tid >> 7;
-      const bool valid = row < tr && entry0 + row < n_edges;
+      const int entry = entry_of(row);
+      const bool valid = entry >= 0 && entry0 + entry < n_edges;
       const float4 d = st_d[row];
       const float r = d.w;
       if (role < 2) {
@@ -753,7 +760,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     // ---- filter 0: invariant logits, feature sums ----
     tmem_to_tile(tmem, 0, warp, lane, wt);
     tc_fence_before();
-    __syncthreads();
+    sync_group();
     TC_MARK(3);
     edge_loops(rpw, [&](auto full) {
       // logits x cutoff of both directions: a of (i <- j), b of (j <- i); b's message goes out at once, a's are summed per receiver.
@@ -834,12 +841,12 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     qi = ld4(qkv + (size_t)cur_i * kProj + 3 * kF + col);
     ki = ld4(qkv + (size_t)cur_i * kProj + 4 * kF + col);
     TC_MARK(4);
-    __syncthreads();
+    sync_group();
     TC_MARK(5);
     // ---- filter 1: equivariant logits, spherical-harmonic sums ----
     tmem_to_tile(tmem, 1, warp, lane, wt);
     tc_fence_before();
-    __syncthreads();
+    sync_group();
     TC_MARK(6);
     edge_loops(rpw, [&](auto full) {
       float accev = 0.f;
