@@ -107,42 +107,42 @@ __device__ __forceinline__ void coulomb_chi_dev(const LrParams& p, float r, floa
   chi = (pot - p.v_rc) - (1.f - f) * (r - p.rc) * p.dv_rc;
   dchi = dpot - (1.f - f) * p.dv_rc + df * (r - p.rc) * p.dv_rc;
 }
-// ai = alpha_free h, ci = c6_free h^2 of both atoms come precomputed per atom
-__device__ __forceinline__ void dispersion_pair_dev(const LrParams& P, float r, float alf_i, float c6f_i, float hi, float alf_j, float c6f_j,
+// With a = alpha h and c = c6 h^2 the combination rule 2 c_i c_j a_i a_j / (a_i^2 c_j + a_j^2 c_i) is linear in both ratios,
+//   c6_ij = K h_i h_j,  K = 2 alpha_i alpha_j / (x_i + x_j),  x = alpha^2 / c6  of the free atom,
+// so its derivatives cost nothing.  The partials of T share the powers of R and p.
+__device__ __forceinline__ float dispersion_x(int Z) { return alpha_free(Z) * alpha_free(Z) / c6_free(Z); }
+__device__ __forceinline__ void dispersion_pair_dev(const LrParams& P, float r, float alf_i, float x_i, float hi, float alf_j, float x_j,
                                                     float hj, float& e, float& de_dr, float& de_dhi, float& de_dhj) {
-  const float ai = alf_i * hi, aj = alf_j * hj, ci = c6f_i * hi * hi, cj = c6f_j * hj * hj;
-  const float iden = rcp_fast(ai * ai * cj + aj * aj * ci);
-  const float c6 = 2.f * ci * cj * ai * aj * iden;
-  const float dlc6_dhi = (rcp_fast(ai) - 2.f * ai * cj * iden) * alf_i + (rcp_fast(ci) - aj * aj * iden) * 2.f * c6f_i * hi;
-  const float dlc6_dhj = (rcp_fast(aj) - 2.f * aj * ci * iden) * alf_j + (rcp_fast(cj) - ai * ai * iden) * 2.f * c6f_j * hj;
-  const float aij = 0.5f * (ai + aj);
+  const float aij = 0.5f * fmaf(alf_i, hi, alf_j * hj);
   const float a17 = exp2f(__log2f(aij) * (1.f / 7.f));
   const float fs = 2.5527961000248887f;
   const float rv = fs * a17;
-  const float sg = ((-0.00078893f * rv + 0.04125273f) * rv + 0.24428889f) * rv + (-0.00433008f);
-  const float dsg = ((3.f * -0.00078893f) * rv + 2.f * 0.04125273f) * rv + 0.24428889f;
+  const float sg = fmaf(fmaf(fmaf(-0.00078893f, rv, 0.04125273f), rv, 0.24428889f), rv, -0.00433008f);
+  const float dsg = fmaf(fmaf(3.f * -0.00078893f, rv, 2.f * 0.04125273f), rv, 0.24428889f);
   const float ig = 2.f * sg * sg;
   const float kp = kDispersionScale * 2.f * 2.54f;
   const float p = kp * a17;
   const float R = r * (1.f / kBohr);
   const float R2 = R * R, p2 = p * p;
   const float R4 = R2 * R2, p4 = p2 * p2;
-  const float R6 = R4 * R2, p6 = p4 * p2, R8 = R4 * R4, p8 = p4 * p4, R10 = R8 * R2, p10 = p8 * p2;
-  const float i6 = rcp_fast(R6 + p6), i8 = rcp_fast(R8 + p8), i10 = rcp_fast(R10 + p10);
-  const float t8 = 5.f * ig, t10 = 30.625f * ig * ig;
-  const float T = i6 + t8 * i8 + t10 * i10;
-  const float dT_dR = -(6.f * R4 * R * i6 * i6 + t8 * 8.f * R6 * R * i8 * i8 + t10 * 10.f * R8 * R * i10 * i10);
-  const float dT_dp = -(6.f * p4 * p * i6 * i6 + t8 * 8.f * p6 * p * i8 * i8 + t10 * 10.f * p8 * p * i10 * i10);
-  const float dT_dig = 5.f * i8 + 61.25f * ig * i10;
-  const float dT_da17 = dT_dp * kp + dT_dig * 4.f * sg * dsg * fs;
-  const float da17_dh = a17 * rcp_fast(7.f * aij) * 0.5f;
+  const float R6 = R4 * R2, p6 = p4 * p2;
+  const float i6 = rcp_fast(R6 + p6), i8 = rcp_fast(fmaf(R4, R4, p4 * p4)), i10 = rcp_fast(fmaf(R6, R4, p6 * p4));
+  const float t8 = 5.f * ig * i8, t10 = 30.625f * ig * ig * i10;
+  const float T = i6 + t8 + t10;
+  const float u6 = 6.f * i6 * i6, u8 = 8.f * t8 * i8, u10 = 10.f * t10 * i10;
+  const float dT_dR = -R4 * R * fmaf(R2, fmaf(R2, u10, u8), u6);
+  const float dT_dp = -p4 * p * fmaf(p2, fmaf(p2, u10, u8), u6);
+  const float dT_dig = fmaf(61.25f * ig, i10, 5.f * i8);
+  const float dT_da17 = fmaf(dT_dp, kp, dT_dig * (4.f * fs) * sg * dsg);
+  const float W = dT_da17 * a17 * rcp_fast(14.f * aij);          // dT / d(alpha_i h_i)
   float f = 1.f, df = 0.f;
   if (P.has_cutoff && P.has_damping) switching_dev(r, P.disp_on, P.rc, f, df);
-  const float pre = -kHartree * c6;
-  e = pre * T * f;
-  de_dr = pre * (dT_dR * (1.f / kBohr) * f + T * df);
-  de_dhi = pre * f * (T * dlc6_dhi + dT_da17 * da17_dh * alf_i);
-  de_dhj = pre * f * (T * dlc6_dhj + dT_da17 * da17_dh * alf_j);
+  const float pre = (-2.f * kHartree) * alf_i * alf_j * rcp_fast(x_i + x_j);
+  const float pf = pre * f, hh = hi * hj;
+  e = pf * hh * T;
+  de_dr = pre * hh * fmaf(dT_dR * (1.f / kBohr), f, T * df);
+  de_dhi = pf * hj * fmaf(hi * alf_i, W, T);
+  de_dhj = pf * hi * fmaf(hj * alf_j, W, T);
 }
 
 template <int MODE>
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
   const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
   if (e0 == e1) return;
   const float qi = q[i], hi = h[i];
-  const int Zi = Z[i];
+  const float alf_i = alpha_free(Z[i]), x_i = dispersion_x(Z[i]);
   const float gei = ge ? ge[i] : 1.f;
   float xi = 0.f, yi = 0.f, zi = 0.f;
   if (MODE == 0) { xi = R[3 * (size_t)i]; yi = R[3 * (size_t)i + 1]; zi = R[3 * (size_t)i + 2]; }
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
         const float e_c = kq * qi * qj * chi;
         float e_d, dd_dr, dd_dhi, dd_dhj;
         const int Zj = Z[j];
-        dispersion_pair_dev(P, r, alpha_free(Zi), c6_free(Zi), hi, alpha_free(Zj), c6_free(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
+        dispersion_pair_dev(P, r, alf_i, x_i, hi, alpha_free(Zj), dispersion_x(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
         e_d *= pf; dd_dr *= pf; dd_dhi *= pf; dd_dhj *= pf;
         ec += e_c; ed += e_d;
         gqi = fmaf(kq * qj, chi, gqi);
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
   if (MODE == 0 && virial) va.flush_warp(virial, (size_t)i, lane);
 }
 
-// The single-device long-range kernel with packed operands: per atom (x, y, z, q) and (h, alpha_free, c6_free, -) so that a pair costs two
+// The single-device long-range kernel with packed operands: per atom (x, y, z, q) and (h, alpha_free, alpha_free^2 / c6_free, -) so that a pair costs two
 // 16-byte gathers, and a packed accumulator (Fx, Fy, Fz, dE/dq) so that the sender's share of a pair is one
 // vector reduction (red.global.add.v4.f32) and one scalar one (dE/dh) instead of five scalar atomics.
 __global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* R, const float* q,
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) pair_pack_kernel(int n, const float* R, c
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   pq[i] = make_float4(R[3 * (size_t)i], R[3 * (size_t)i + 1], R[3 * (size_t)i + 2], q[i]);
-  hz[i] = make_float4(h[i], alpha_free(Z[i]), c6_free(Z[i]), 0.f);
+  hz[i] = make_float4(h[i], alpha_free(Z[i]), dispersion_x(Z[i]), 0.f);
   acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 // with e_atom also the per-atom energies: the sum of the network's, the repulsion's and the two pair terms' shares
@@ -248,14 +248,19 @@ __global__ void __launch_bounds__(256) pair_unpack_kernel(int n, const float4* a
 __device__ __forceinline__ void red_add_f4(float4* p, float x, float y, float z, float w) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
+// QUEUED (lists with a skin): the entries inside the cutoff (four of five at a 1 A skin) pass through a queue in shared memory, so that the
+// arithmetic of the pair terms runs with full warps.
+template <bool QUEUED>
 __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell cell, int n, const int* __restrict__ row_ptr,
                                                              const int* __restrict__ nbr_j, const float4* pq,
                                                              const float4* hz, float4* __restrict__ acc,
                                                              float* __restrict__ gh, float* e_coul,
                                                              float* e_disp, float* __restrict__ virial) {
+  __shared__ float4 queue_d[QUEUED ? 8 : 1][QUEUED ? 64 : 1];      // displacement and charge
+  __shared__ int queue_j[QUEUED ? 8 : 1][QUEUED ? 64 : 1];
   grid_dep_sync();
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 8 + warp;
   if (i >= n) return;
   VirialAcc va;
   const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
@@ -265,19 +270,12 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
   const float qi = pi.w, hi = hzi.x;
   const float pf = P.pair_factor, kq = pf * kKe, rc2 = P.rc * P.rc;
   float ec = 0.f, ed = 0.f, fx = 0.f, fy = 0.f, fz = 0.f, gqi = 0.f, ghi = 0.f;
-  for (int e = e0 + lane; e < e1; e += 32) {
-    const int j = nbr_j[e];
-    if (j < 0 || j >= n) continue;
-    const float4 pj = pq[j];
-    float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-    min_image(cell, dx, dy, dz);
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    if (!(r2 > 0.f) || (P.has_cutoff && r2 >= rc2)) continue;
+  auto pair = [&](int j, float dx, float dy, float dz, float qj) {
     const float4 hzj = hz[j];
+    const float r2 = dx * dx + dy * dy + dz * dz;
     const float rinv = rsqrtf(r2), r = r2 * rinv;
     float chi, dchi;
     coulomb_chi_dev(P, r, rinv, chi, dchi);
-    const float qj = pj.w;
     float e_d, dd_dr, dd_dhi, dd_dhj;
     dispersion_pair_dev(P, r, hzi.y, hzi.z, hi, hzj.y, hzj.z, hzj.x, e_d, dd_dr, dd_dhi, dd_dhj);
     ec = fmaf(kq * qi * qj, chi, ec);
@@ -290,7 +288,44 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
     fx += gx; fy += gy; fz += gz;
     red_add_f4(acc + j, -gx, -gy, -gz, kq * qi * chi);
     atomicAdd(gh + j, pf * dd_dhj);
+  };
+  int waiting = 0;
+  for (int eb = e0; eb < e1; eb += 32) {
+    const int e = eb + lane;
+    const int j = e < e1 ? nbr_j[e] : -1;
+    bool inside = j >= 0 && j < n;
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (inside) {
+      const float4 pj = pq[j];
+      d = make_float4(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z, pj.w);
+      min_image(cell, d.x, d.y, d.z);
+      const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+      inside = r2 > 0.f && !(P.has_cutoff && r2 >= rc2);
+    }
+    if (!QUEUED) {
+      if (inside) pair(j, d.x, d.y, d.z, d.w);
+      continue;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, inside);
+    if (inside) {
+      const int at = waiting + __popc(m & ((1u << lane) - 1u));
+      queue_d[warp][at] = d;
+      queue_j[warp][at] = j;
+    }
+    waiting += __popc(m);
+    __syncwarp();
+    if (waiting >= 32) {
+      waiting -= 32;
+      const float4 w = queue_d[warp][waiting + lane];
+      pair(queue_j[warp][waiting + lane], w.x, w.y, w.z, w.w);
+      __syncwarp();
+    }
   }
+  if (QUEUED && lane < waiting) {
+    const float4 w = queue_d[warp][lane];
+    pair(queue_j[warp][lane], w.x, w.y, w.z, w.w);
+  }
+  __syncwarp();
   ec = warp_sum(ec); ed = warp_sum(ed); gqi = warp_sum(gqi); ghi = warp_sum(ghi);
   fx = warp_sum(fx); fy = warp_sum(fy); fz = warp_sum(fz);
   if (lane == 0) {
@@ -318,7 +353,7 @@ __global__ void __launch_bounds__(256) pair_lr_owned_kernel(LrParams P, Cell cel
   if (i >= n_owned) return;
   const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
   const float qi = q[i], hi = h[i];
-  const float alf_i = alpha_free(Z[i]), c6f_i = c6_free(Z[i]);
+  const float alf_i = alpha_free(Z[i]), x_i = dispersion_x(Z[i]);
   const float xi = R[3 * (size_t)i], yi = R[3 * (size_t)i + 1], zi = R[3 * (size_t)i + 2];
   float ec = 0.f, ed = 0.f, fx = 0.f, fy = 0.f, fz = 0.f, gqi = 0.f, ghi = 0.f;
   VirialAcc va;
@@ -335,7 +370,7 @@ __global__ void __launch_bounds__(256) pair_lr_owned_kernel(LrParams P, Cell cel
     const float qj = q[j], hj = h[j];
     const int Zj = Z[j];
     float e_d, dd_dr, dd_dhi, dd_dhj;
-    dispersion_pair_dev(P, r, alf_i, c6f_i, hi, alpha_free(Zj), c6_free(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
+    dispersion_pair_dev(P, r, alf_i, x_i, hi, alpha_free(Zj), dispersion_x(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
     const bool both = j < n_owned;
     const float w = both ? 1.f : 0.5f;                             // share of the pair energy booked on this row
     ec = fmaf(w * kKe * qi * qj, chi, ec);
@@ -556,13 +591,14 @@ void launch_pair_lr(cudaStream_t s, const LrParams& P, const Cell& cell, int n, 
 
 void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, int n, const int* row_ptr, const int* nbr_j, const int* Z,
                            const float* R, const float* q, const float* h, float* pack /* 12 n floats */, float* F, float* gq, float* gh,
-                           float* e_coul, float* e_disp, float* virial, const float* e_nn, const float* e_zbl, float* e_atom) {
+                           float* e_coul, float* e_disp, float* virial, const float* e_nn, const float* e_zbl, float* e_atom, bool skin) {
   if (n <= 0) return;
   float4* pq = reinterpret_cast<float4*>(pack);
   float4* acc = pq + n;
   float4* hz = acc + n;
   launch_chained(pair_pack_kernel, (n + 255) / 256, 256, 0, s, n, R, q, h, Z, pq, hz, acc);
-  launch_chained(pair_lr_packed_kernel, (n + 7) / 8, 256, 0, s, P, cell, n, row_ptr, nbr_j, pq, hz, acc, gh, e_coul, e_disp, virial);
+  launch_chained(skin ? pair_lr_packed_kernel<true> : pair_lr_packed_kernel<false>, (n + 7) / 8, 256, 0, s, P, cell, n, row_ptr, nbr_j, pq, hz, acc,
+                 gh, e_coul, e_disp, virial);
   launch_chained(pair_unpack_kernel, (n + 255) / 256, 256, 0, s, n, acc, F, gq, e_nn, e_zbl, e_coul, e_disp, e_atom);
   count_launch(3);
 }
