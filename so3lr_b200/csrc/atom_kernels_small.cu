@@ -228,13 +228,18 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
   if (proj) load_w<32>(w, proj + (size_t)((tid >> 7) * 4 + ((tid >> 5) & 3)) * 1024 + lane, 32);      // thread (projection, column): 32 outputs of its head
   else load_w128(w, L.ex_xxT);
   grid_dep_sync();
+  // this thread's shares of the CTA's g_qkv rows (16-byte pieces, NTHR apart): all requested at once, and cleared for the next attention
+  // layer behind the barrier.  A load and the clearing store of its piece in turn serialise: 8 us a launch at 1,536 atoms
+  constexpr int kPieces = (AT * (kProj / 4) + NTHR - 1) / NTHR;
+  auto piece = [&](int u) { return tid + u * NTHR; };
+  auto listed = [&](int u) { return piece(u) < AT * (kProj / 4) && row0 + piece(u) / (kProj / 4) < n; };
   if (proj) {
-    for (int k = tid; k < AT * (kProj / 4); k += NTHR) {
-      const int a = k / (kProj / 4);
-      float* p = g_qkv_up + (size_t)row0 * kProj + 4 * k;
-      st4(gq + 4 * k, row0 + a < n ? ld4(p) : zero4());
-      if (row0 + a < n) st4(p, zero4());      // the next attention layer adds into zeros
-    }
+    float4 v[kPieces];
+#pragma unroll
+    for (int u = 0; u < kPieces; ++u) v[u] = listed(u) ? ld4(g_qkv_up + (size_t)row0 * kProj + 4 * piece(u)) : zero4();
+#pragma unroll
+    for (int u = 0; u < kPieces; ++u)
+      if (piece(u) < AT * (kProj / 4)) st4(gq + 4 * piece(u), v[u]);
   }
   if (own) {
     g3 = ld4((proj ? g_xa : g4) + ra);
@@ -247,6 +252,9 @@ __global__ void __launch_bounds__(NTHR, 1) post_bwd_small_kernel(LayerDev L, int
   }
   if (proj) {
     __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPieces; ++u)
+      if (listed(u)) st4(g_qkv_up + (size_t)row0 * kProj + 4 * piece(u), zero4());
     float2 acc[AT];
     zero_acc<AT>(acc);
     dot_rows<AT, 32>(acc, w, gq + 32 * warp, kProj);
