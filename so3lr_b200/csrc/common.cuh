@@ -104,11 +104,15 @@ struct VirialAcc {
     xz = fmaf(0.5f * wx, fz, fmaf(0.5f * wz, fx, xz));
     xy = fmaf(0.5f * wx, fy, fmaf(0.5f * wy, fx, xy));
   }
-  // all lanes of the warp that owns atom i call this; lane 0 adds the warp's total to the atom's row
-  SO3LR_D void flush_warp(float* __restrict__ W, size_t i, int lane) {
+  // all lanes of the warp that owns atom i call this; lane 0 adds the warp's total to the atom's row (`shared`: one of several warps)
+  SO3LR_D void flush_warp(float* __restrict__ W, size_t i, int lane, bool shared = false) {
     const float a = warp_sum(xx), b = warp_sum(yy), c = warp_sum(zz), d = warp_sum(yz), e = warp_sum(xz), f = warp_sum(xy);
     if (lane == 0) {
       float* w = W + 6 * i;
+      if (shared) {
+        atomicAdd(w, a); atomicAdd(w + 1, b); atomicAdd(w + 2, c); atomicAdd(w + 3, d); atomicAdd(w + 4, e); atomicAdd(w + 5, f);
+        return;
+      }
       w[0] += a; w[1] += b; w[2] += c; w[3] += d; w[4] += e; w[5] += f;
     }
   }

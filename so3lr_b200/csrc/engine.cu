@@ -887,7 +887,7 @@ int evaluate_fused(so3lr_b200_system* S, cudaStream_t st, const float* R, float*
   launch_charge_conserve(st, S->n_graphs, S->d_graph_start, S->q_raw, S->d_total_charge, S->hv, S->q, S->h, S->n, S->red_scratch);
   S->prof.begin(kPPairLr, st);
   launch_pair_lr_packed(st, S->lr, S->cell, n, S->lrl.row_ptr, S->lrl.nbr_j, S->d_Z, R, S->q, S->h, S->pair_pack, F, S->gq, S->gh, S->e_coul,
-                        S->e_disp, S->vir(), S->e_nn, S->e_zbl, S->ks.mode ? nullptr : S->e_atom, S->opt.skin > 0.f);
+                        S->e_disp, S->vir(), S->e_nn, S->e_zbl, S->ks.mode ? nullptr : S->e_atom, S->opt.skin > 0.f, S->lrl.count);
   S->prof.end(st);
   if (S->ks.mode) {
     S->prof.begin(kPKspace, st);

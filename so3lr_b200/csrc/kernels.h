@@ -265,7 +265,8 @@ void launch_pair_lr(cudaStream_t s, const LrParams& P, const Cell& cell, int n, 
 void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, int n, const int* row_ptr, const int* nbr_j, const int* Z,
                            const float* R, const float* q, const float* h, float* pack, float* F, float* gq, float* gh, float* e_coul,
                            float* e_disp, float* virial,
-                           const float* e_nn, const float* e_zbl, float* e_atom, bool skin /* the list reaches beyond the cutoff */);
+                           const float* e_nn, const float* e_zbl, float* e_atom, bool skin /* the list reaches beyond the cutoff */,
+                           long long pairs /* entries of the list */);
 // Domain-decomposed variant: rows 0 .. n_owned-1 of an ordered list (j > i) over owned atoms and ghosts, ghosts carrying
 // the larger indices.  Pairs of two owned atoms are evaluated once and scatter the partner's derivatives (atomics); pairs
 // with a ghost end book half of the energy and the row atom's derivatives.  gq, gh are zeroed here and accumulated, F_add is

@@ -249,9 +249,9 @@ __device__ __forceinline__ void red_add_f4(float4* p, float x, float y, float z,
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 // QUEUED (lists with a skin): the entries inside the cutoff (four of five at a 1 A skin) pass through a queue in shared memory, so that the
-// arithmetic of the pair terms runs with full warps.
+// arithmetic of the pair terms runs with full warps.  `split` warps share a row (see pair_row_split).
 template <bool QUEUED>
-__global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell cell, int n, const int* __restrict__ row_ptr,
+__global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell cell, int n, int split, const int* __restrict__ row_ptr,
                                                              const int* __restrict__ nbr_j, const float4* pq,
                                                              const float4* hz, float4* __restrict__ acc,
                                                              float* __restrict__ gh, float* e_coul,
@@ -260,11 +260,11 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
   __shared__ int queue_j[QUEUED ? 8 : 1][QUEUED ? 64 : 1];
   grid_dep_sync();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = blockIdx.x * 8 + warp;
+  const int i = (blockIdx.x * 8 + warp) / split, part = (blockIdx.x * 8 + warp) % split;
   if (i >= n) return;
   VirialAcc va;
-  const int e0 = row_ptr[i], e1 = row_ptr[i + 1];
-  if (e0 == e1) return;
+  const int e0 = row_ptr[i] + 32 * part, e1 = row_ptr[i + 1];
+  if (e0 >= e1) return;
   const float4 pi = pq[i];
   const float4 hzi = hz[i];
   const float qi = pi.w, hi = hzi.x;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
     atomicAdd(gh + j, pf * dd_dhj);
   };
   int waiting = 0;
-  for (int eb = e0; eb < e1; eb += 32) {
+  for (int eb = e0; eb < e1; eb += 32 * split) {
     const int e = eb + lane;
     const int j = e < e1 ? nbr_j[e] : -1;
     bool inside = j >= 0 && j < n;
@@ -329,12 +329,19 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
   ec = warp_sum(ec); ed = warp_sum(ed); gqi = warp_sum(gqi); ghi = warp_sum(ghi);
   fx = warp_sum(fx); fy = warp_sum(fy); fz = warp_sum(fz);
   if (lane == 0) {
-    e_coul[i] += ec;     // only this warp writes the energies of row i
-    e_disp[i] += ed;
+    if (split == 1) { e_coul[i] += ec; e_disp[i] += ed; }      // only this warp writes the energies of row i
+    else { atomicAdd(e_coul + i, ec); atomicAdd(e_disp + i, ed); }
     red_add_f4(acc + i, fx, fy, fz, gqi);
     atomicAdd(gh + i, ghi);
   }
-  if (virial) va.flush_warp(virial, (size_t)i, lane);
+  if (virial) va.flush_warp(virial, (size_t)i, lane, split > 1);
+}
+// Warps per row.  A short list leaves most of the chip idle with one: 1,536 atoms are 10 warps per SM, and a row of the ordered list holds up to
+// 12 rounds of 32 pairs, each a chain of gathers and some 400 instructions (2 us).  As many warps as 32 per SM allow and the average row has rounds.
+int pair_row_split(int n, long long pairs) {
+  const long long rounds = (pairs / n + 31) / 32, room = 32LL * sm_count() / n;
+  const long long s = rounds < room ? rounds : room;
+  return s < 1 ? 1 : (s > 16 ? 16 : (int)s);
 }
 
 // Owned rows of an ordered list over owned atoms and ghosts (decomposed runs; ghosts carry the larger indices, so the list
@@ -591,13 +598,15 @@ void launch_pair_lr(cudaStream_t s, const LrParams& P, const Cell& cell, int n, 
 
 void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, int n, const int* row_ptr, const int* nbr_j, const int* Z,
                            const float* R, const float* q, const float* h, float* pack /* 12 n floats */, float* F, float* gq, float* gh,
-                           float* e_coul, float* e_disp, float* virial, const float* e_nn, const float* e_zbl, float* e_atom, bool skin) {
+                           float* e_coul, float* e_disp, float* virial, const float* e_nn, const float* e_zbl, float* e_atom, bool skin,
+                           long long pairs) {
   if (n <= 0) return;
   float4* pq = reinterpret_cast<float4*>(pack);
   float4* acc = pq + n;
   float4* hz = acc + n;
   launch_chained(pair_pack_kernel, (n + 255) / 256, 256, 0, s, n, R, q, h, Z, pq, hz, acc);
-  launch_chained(skin ? pair_lr_packed_kernel<true> : pair_lr_packed_kernel<false>, (n + 7) / 8, 256, 0, s, P, cell, n, row_ptr, nbr_j, pq, hz, acc,
+  const int split = pair_row_split(n, pairs);
+  launch_chained(skin ? pair_lr_packed_kernel<true> : pair_lr_packed_kernel<false>, (unsigned)(((long long)n * split + 7) / 8), 256, 0, s, P, cell, n, split, row_ptr, nbr_j, pq, hz, acc,
                  gh, e_coul, e_disp, virial);
   launch_chained(pair_unpack_kernel, (n + 255) / 256, 256, 0, s, n, acc, F, gq, e_nn, e_zbl, e_coul, e_disp, e_atom);
   count_launch(3);
