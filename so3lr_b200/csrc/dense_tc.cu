@@ -89,16 +89,33 @@ __device__ __forceinline__ uint64_t desc_base(uint32_t lbo, uint32_t sbo) {
 }
 // instruction descriptor, kind::f16: FP16 operands, FP32 accumulator, both operands K-major, M = 128
 __device__ __forceinline__ uint32_t make_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TM >> 4) << 24); }
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// A whole warp runs the issue code; `on` is set in one lane, which issues: descriptors stay in uniform registers
+__device__ __forceinline__ void umma_if(uint32_t on, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t on, uint32_t mbar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(mbar), "r"(on) : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t on;
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n" : "=r"(on));
+  return on;
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
   for (int it = 0; it < kWaitSpins; ++it) {
@@ -185,9 +202,12 @@ __device__ __forceinline__ float dsilu_fast(float x) {
 }
 
 // D[128 x n] (+)= A[:, chunks] * B: A from chunk `a_chunk0` on (2 chunks per K step of 16), B image at w_smem (hi matrix, lo
-// matrix w_lo bytes above, core-matrix stride along K = 16 n bytes).  Issued by one thread; three MMAs per K step.
-__device__ __noinline__ void issue_gemm(uint32_t tmem, int d_col, uint32_t a_smem, int a_chunk0, uint32_t w_smem, uint32_t w_lo, int n, int ksteps,
-                                        uint32_t accumulate) {
+// matrix w_lo bytes above, core-matrix stride along K = 16 n bytes): the hi*hi products (cross = 0) or the hi*lo and lo*hi products.
+// The first four warps share the issue of a contraction: main and cross products by one warp each, or a head per warp.  One
+// thread takes about 100 cycles an MMA: 2.5 to 3 k cycles for the 24 of a 128 x 128 contraction, 18 k for the 120 small ones of the
+// block-diagonal projections' reverse, which the tensor cores are through with in 1.6 and 2 k.
+__device__ __forceinline__ void issue_gemm(uint32_t on, int cross, uint32_t tmem, int d_col, uint32_t a_smem, int a_chunk0, uint32_t w_smem,
+                                           uint32_t w_lo, int n, int ksteps, uint32_t accumulate) {
   const uint64_t da = desc_base(2048, 128) + ((a_smem + a_chunk0 * 2048) >> 4), dal = da + (kALo >> 4);
   const uint64_t db = desc_base(16 * n, 128) + (w_smem >> 4), dbl = db + (w_lo >> 4);
   const uint32_t idesc = make_idesc(n);
@@ -196,9 +216,12 @@ __device__ __noinline__ void issue_gemm(uint32_t tmem, int d_col, uint32_t a_sme
   for (int ks = 0; ks < ksteps; ++ks) {
     const uint64_t ah = da + ks * a_step, al = dal + ks * a_step, bh = db + ks * b_step, bl = dbl + ks * b_step;
     const uint32_t acc = (ks > 0) ? 1u : accumulate;
-    umma(tmem + d_col, ah, bh, idesc, acc);
-    umma(tmem + kColCross + d_col, ah, bl, idesc, acc);
-    umma(tmem + kColCross + d_col, al, bh, idesc, 1u);
+    if (!cross) {
+      umma_if(on, tmem + d_col, ah, bh, idesc, acc);
+    } else {
+      umma_if(on, tmem + kColCross + d_col, ah, bl, idesc, acc);
+      umma_if(on, tmem + kColCross + d_col, al, bh, idesc, 1u);
+    }
   }
 }
 
@@ -223,7 +246,8 @@ struct Tile {
   float4* red;
   float* redf;
   uint32_t mbar, mbar2, wbar, tmem, tlane;
-  uint32_t mph, mph2, wph;      // phases of the two barriers (wph is only followed by thread 0)
+  uint32_t mph, mph2, wph;      // phases of the barriers (wph is only followed by the warps that issue)
+  uint32_t on;                  // set in the lane that issues its warp's MMAs
   int tid, warp, lane, row, quarter, c0;
   bool failed;
 
@@ -235,15 +259,15 @@ struct Tile {
     inv = reinterpret_cast<float4*>(sm + kOffInv);
     red = reinterpret_cast<float4*>(sm + kOffRed);
     redf = reinterpret_cast<float*>(sm + kOffRed2);
-    tid = threadIdx.x; warp = tid >> 5; lane = tid & 31; row = tid & 127; quarter = tid >> 7; c0 = 32 * quarter;
+    tid = threadIdx.x; warp = __shfl_sync(0xffffffffu, tid >> 5, 0); lane = tid & 31; on = elect_one(); row = tid & 127; quarter = tid >> 7; c0 = 32 * quarter;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kOffMisc);
     uint32_t* tmem_p = reinterpret_cast<uint32_t*>(sm + kOffMisc + 32);
     mbar = smem_u32(bars); wbar = smem_u32(bars + 1); mbar2 = smem_u32(bars + 2);
     mph = 0; mph2 = 0; wph = 0; failed = false;
     if (tid == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(mbar));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar2));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(mbar2));
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -254,7 +278,7 @@ struct Tile {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    tmem = *tmem_p;
+    tmem = __shfl_sync(0xffffffffu, *tmem_p, 0);
     tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
   }
   __device__ __forceinline__ void finish(int* err) {
@@ -272,7 +296,7 @@ struct Tile {
     if (!mbar_wait(wbar, wph)) failed = true;
     wph ^= 1;
   }
-  // operands written: make them visible to the tensor core, then thread 0 issues (inside `issue`) and commits
+  // operands written: make them visible to the tensor core, then the first four warps issue and commit (each of them once per phase)
   __device__ __forceinline__ void operands_ready() {
     fence_async_smem();
     tc_fence_before();
@@ -399,12 +423,12 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
     }
     T.operands_ready();
     DN_MARK(1);
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       DN_MARK(2);
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     T.wait_mma();
     DN_MARK(3);
@@ -425,12 +449,12 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
     }
     T.operands_ready();
     DN_MARK(4);
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       DN_MARK(5);
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     T.flush_rows(z1_out, kF, row0, n, kF);
     T.wait_mma();
@@ -458,12 +482,12 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
     }
     T.operands_ready();
     DN_MARK(7);
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       DN_MARK(8);
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     // gates and ev2 while the exchange contraction runs
     if (quarter == 3) {
@@ -543,14 +567,15 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
         const int set = r & 1;
         if (r == 3) {
 #pragma unroll 1
-          for (int h = 0; h < 4; ++h) issue_gemm(T.tmem, 128 * set + 32 * h, a_smem, 4 * h, w_smem + 3 * kProjBlockBytes + h * 4096, 2048, 32, 2, 0);
-        } else {
+          for (int x = 0; x < 2; ++x)
+            issue_gemm(T.on, x, T.tmem, 128 * set + 32 * warp, a_smem, 4 * warp, w_smem + 3 * kProjBlockBytes + warp * 4096, 2048, 32, 2, 0);
+        } else if (warp < 2) {
           const int h = r < 3 ? r : 3;
-          issue_gemm(T.tmem, 128 * set, a_smem, 4 * h, w_smem + (r < 3 ? r : 0) * kProjBlockBytes, kProjBlockBytes / 2, 128, 2, 0);
+          issue_gemm(T.on, warp, T.tmem, 128 * set, a_smem, 4 * h, w_smem + (r < 3 ? r : 0) * kProjBlockBytes, kProjBlockBytes / 2, 128, 2, 0);
         }
-        umma_commit(set ? T.mbar2 : T.mbar);
+        umma_commit_if(T.on, set ? T.mbar2 : T.mbar);
       };
-      if (tid == 0) {
+      if (warp < 4) {
         T.wait_weights();
         tc_fence_after();
         issue_round(0);
@@ -576,7 +601,7 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_fwd_tc_kernel(LayerDev L, i
         tc_fence_before();
         __syncthreads();
         DN_MARK(18);
-        if (tid == 0 && r + 2 < 5) {
+        if (warp < 4 && r + 2 < 5) {
           if (r + 2 == 4) T.wait_weights();
           tc_fence_after();
           issue_round(r + 2);
@@ -691,14 +716,14 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
         DN_MARK(42);
         T.operands_ready();
         DN_MARK(43);
-        if (tid == 0) {
+        if (warp < 4) {
           if (w == 0 || w == 4) T.wait_weights();
           DN_MARK(44);
           tc_fence_after();
 #pragma unroll 1
-          for (int h = 0; h < 4; ++h)
-            issue_gemm(T.tmem, 32 * h, smem_u32(Aw), 4 * h, w_smem + (w < 4 ? w : 0) * kProjBlockBytes + h * 4096, 2048, 32, 2, w > 0);
-          umma_commit((w & 1) ? T.mbar2 : T.mbar);
+          for (int x = 0; x < 2; ++x)      // a head per warp
+            issue_gemm(T.on, x, T.tmem, 32 * warp, smem_u32(Aw), 4 * warp, w_smem + (w < 4 ? w : 0) * kProjBlockBytes + warp * 4096, 2048, 32, 2, w > 0);
+          umma_commit_if(T.on, (w & 1) ? T.mbar2 : T.mbar);
           DN_MARK(45);
         }
       }
@@ -820,11 +845,11 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
     }
     T.operands_ready();
     DN_MARK(33);
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     T.wait_mma();
     DN_MARK(34);
@@ -849,11 +874,11 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
     }
     T.operands_ready();
     DN_MARK(35);
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     T.load_rows(z1, kF, row0, n);
     T.wait_mma();
@@ -873,11 +898,11 @@ __global__ void __launch_bounds__(NTHR, 1) atom_post_bwd_tc_kernel(LayerDev L, i
     }
     T.operands_ready();
     DN_MARK(37);
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     // normalised xa -> staging tile, 1 / std -> stat (warp-local) while the contraction runs
     {
@@ -1013,11 +1038,11 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n
     // energy and charge heads share the structure Dense(128) -> silu -> dot
 #pragma unroll 1
     for (int head = 0; head < 2; ++head) {
-      if (tid == 0) {
+      if (warp < 4) {
         T.wait_weights();
         tc_fence_after();
-        issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
-        umma_commit(T.mbar);
+        if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 0);
+        umma_commit_if(T.on, T.mbar);
       }
       if (head == 1) T.flush_rows(ze, kF, row0, n, kF);      // the first head's pre-activations leave beneath the second contraction
       T.wait_mma();
@@ -1063,11 +1088,11 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n
       }
     }
     // Hirshfeld: 128 -> 64 -> 64, then the dot product with the element's query
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 16384, 64, 8, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 16384, 64, 8, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     T.flush_rows(zq, kF, row0, n, kF);
     T.wait_mma();
@@ -1086,10 +1111,10 @@ __global__ void __launch_bounds__(NTHR, 1) heads_fwd_tc_kernel(ModelDev M, int n
       a_store32(T.A, c0, row, v);
     }
     T.operands_ready();
-    if (tid == 0) {
+    if (warp < 4) {
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem + 32768, 8192, 64, 4, 0);
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem + 32768, 8192, 64, 4, 0);
+      umma_commit_if(T.on, T.mbar);
     }
     flush_rows64(T, zh, row0, n);
     T.wait_mma();
@@ -1174,11 +1199,11 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n
     }
     load_rows64(T, zh, row0, n);
     T.operands_ready();
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 128, a_smem, 0, w_smem, 8192, 64, 4, 0);      // g_sh = g_k H_fin^T into columns [128, 192)
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 128, a_smem, 0, w_smem, 8192, 64, 4, 0);      // g_sh = g_k H_fin^T into columns [128, 192)
+      umma_commit_if(T.on, T.mbar);
     }
     T.wait_mma();
     if (quarter < 2) {      // g_zh = g_sh * silu'(zh) -> A
@@ -1192,10 +1217,10 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n
       a_store32(T.A, c0, row, v);
     }
     T.operands_ready();      // also: every thread is done with the staging tile, which now becomes the second operand buffer
-    if (tid == 0) {
+    if (warp < 4) {
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem + 16384, 16384, 128, 4, 0);      // gx = g_zh H_reg^T
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem + 16384, 16384, 128, 4, 0);      // gx = g_zh H_reg^T
+      umma_commit_if(T.on, T.mbar);
     }
     // energy branch operand (warp-local): c_e fin_e silu'(ze) -> second buffer
 #pragma unroll
@@ -1230,19 +1255,19 @@ __global__ void __launch_bounds__(NTHR, 1) heads_bwd_tc_kernel(ModelDev M, int n
       a_store8(T.A, 4 * i + ch, wr, v);
     }
     T.operands_ready();
-    if (tid == 0) {
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 0, smem_u32(A1), 0, w_smem, 32768, 128, 8, 1);      // gx += g_ze E_reg^T
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, smem_u32(A1), 0, w_smem, 32768, 128, 8, 1);      // gx += g_ze E_reg^T
+      umma_commit_if(T.on, T.mbar);
     }
     T.wait_mma();
-    if (tid == 0) {
-      T.load_weights(M.q_regT_u, 65536);
+    if (tid == 0) T.load_weights(M.q_regT_u, 65536);
+    if (warp < 4) {
       T.wait_weights();
       tc_fence_after();
-      issue_gemm(T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 1);      // gx += g_zq Q_reg^T
-      umma_commit(T.mbar);
+      if (warp < 2) issue_gemm(T.on, warp, T.tmem, 0, a_smem, 0, w_smem, 32768, 128, 8, 1);      // gx += g_zq Q_reg^T
+      umma_commit_if(T.on, T.mbar);
     }
     T.wait_mma();
     {
