@@ -111,32 +111,36 @@ __device__ __forceinline__ double exp_near_0(double x) {
   return fma(x8, p89, fma(x4, fma(x2, p67, p45), fma(x2, p23, p01)));
 }
 // One factor of the chain propagator over `delta`; returns the momentum scale.  xi, p: chain positions and momenta, iQ: reciprocal
-// masses (one thread walks a chain of dependent operations: a division costs it as much as an exponential).
-__device__ double nhc_substep(int L, double* xi, double* p, const double* iQ, double& ke, double delta, double kT, double dof) {
-  const int M = L - 1;
+// masses (one thread walks a chain of dependent operations: a division costs it as much as an exponential).  LT: the chain's length where
+// it is known at compile time, which keeps the chain in registers (a runtime length indexes local memory: every access is a store
+// and a load in that chain of operations); 0 otherwise.
+template <int LT>
+__device__ __forceinline__ double nhc_substep(int length, double* xi, double* p, const double* iQ, double& ke, double delta, double kT, double dof) {
+  const int L = LT ? LT : length, M = L - 1;
   const double d2 = 0.5 * delta, d4 = 0.25 * delta, d8 = 0.125 * delta;
+  double s[LT ? LT : kNhcMaxChain];      // exp(-d8 p[m + 1] / Q[m + 1]): p[m + 1] is the same in both sweeps
   if (L == 1) {
     p[0] += d4 * (2.0 * ke - dof * kT);
   } else {
     p[M] += d4 * (p[M - 1] * p[M - 1] * iQ[M - 1] - kT);
-    for (int m = M - 1; m > 0; --m) {
-      double G = p[m - 1] * p[m - 1] * iQ[m - 1] - kT;
-      double s = exp_near_0(-d8 * p[m + 1] * iQ[m + 1]);
-      p[m] = s * (s * p[m] + d4 * G);
+#pragma unroll
+    for (int m = M - 1; m >= 0; --m) {
+      const double G = m > 0 ? p[m - 1] * p[m - 1] * iQ[m - 1] - kT : 2.0 * ke - dof * kT;
+      s[m] = exp_near_0(-d8 * p[m + 1] * iQ[m + 1]);
+      p[m] = s[m] * (s[m] * p[m] + d4 * G);
     }
-    double s = exp_near_0(-d8 * p[1] * iQ[1]);
-    p[0] = s * (s * p[0] + d4 * (2.0 * ke - dof * kT));
   }
   const double scale = exp_near_0(-d2 * p[0] * iQ[0]);
   ke *= scale * scale;
+#pragma unroll
   for (int m = 0; m < L; ++m) xi[m] += d2 * p[m] * iQ[m];
   double G = 2.0 * ke - dof * kT;
   if (L == 1) {
     p[0] += d4 * G;
   } else {
+#pragma unroll
     for (int m = 0; m < M; ++m) {
-      double s = exp_near_0(-d8 * p[m + 1] * iQ[m + 1]);
-      p[m] = s * (s * p[m] + d4 * G);
+      p[m] = s[m] * (s[m] * p[m] + d4 * G);
       G = p[m] * p[m] * iQ[m] - kT;
     }
     p[M] += d4 * G;
@@ -144,11 +148,13 @@ __device__ double nhc_substep(int L, double* xi, double* p, const double* iQ, do
   return scale;
 }
 
-// Advances the chain stored at `chain` by n_half half steps (one thread); returns the product of the momentum scales.
-// chain[0] (kinetic energy) follows the scaling; chain[1] is left to the caller.
-__device__ double nhc_advance(double* chain, int L, int chain_steps, int sy_steps, double dt, double tau, double kT, double dof,
-                              int n_half) {
-  double xi[kNhcMaxChain], p[kNhcMaxChain], iQ[kNhcMaxChain];
+template <int LT>
+__device__ __forceinline__ double nhc_walk(double* chain, int length, int chain_steps, int sy_steps, double dt, double tau, double kT, double dof,
+                                           int n_half) {
+  constexpr int kRoom = LT ? LT : kNhcMaxChain;
+  const int L = LT ? LT : length;
+  double xi[kRoom], p[kRoom], iQ[kRoom];
+#pragma unroll
   for (int m = 0; m < L; ++m) {
     xi[m] = chain[2 + m];
     p[m] = chain[2 + kNhcMaxChain + m];
@@ -157,14 +163,30 @@ __device__ double nhc_advance(double* chain, int L, int chain_steps, int sy_step
   double ke = chain[0], total = 1.0;
   const double* w = kSyWeights[sy_steps / 2];
   const double delta = dt / chain_steps;
+#pragma unroll 1
   for (int h = 0; h < n_half; ++h)
-    for (int i = 0; i < chain_steps * sy_steps; ++i) total *= nhc_substep(L, xi, p, iQ, ke, delta * w[i % sy_steps], kT, dof);
+#pragma unroll 1
+    for (int i = 0; i < chain_steps * sy_steps; ++i) total *= nhc_substep<LT>(L, xi, p, iQ, ke, delta * w[i % sy_steps], kT, dof);
+#pragma unroll
   for (int m = 0; m < L; ++m) {
     chain[2 + m] = xi[m];
     chain[2 + kNhcMaxChain + m] = p[m];
   }
   chain[0] = ke;
   return total;
+}
+// Advances the chain stored at `chain` by n_half half steps (one thread); returns the product of the momentum scales.
+// chain[0] (kinetic energy) follows the scaling; chain[1] is left to the caller.
+__device__ double nhc_advance(double* chain, int L, int chain_steps, int sy_steps, double dt, double tau, double kT, double dof,
+                              int n_half) {
+  switch (L) {
+    case 1: return nhc_walk<1>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half);
+    case 2: return nhc_walk<2>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half);
+    case 3: return nhc_walk<3>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half);
+    case 4: return nhc_walk<4>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half);
+    case 5: return nhc_walk<5>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half);
+    default: return nhc_walk<0>(chain, L, chain_steps, sy_steps, dt, tau, kT, dof, n_half);
+  }
 }
 
 __device__ double sum_partials_256(const double* __restrict__ partials, int n_partials, double* sh) {
