@@ -459,14 +459,14 @@ int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bo
   if (which != 0) {
     if (!S->nws_lr && !(S->nws_lr = nlist_workspace_create())) return kCudaError;
     rc = nlist_begin(S->nws_lr, st, S->cell, S->n, R, r_lr, S->opt.lr_both_directions ? 0 : 1, seg ? seg : (gs_lr ? S->d_seg : nullptr),
-                     gs_lr, &S->lrl, 1, nullptr, -1, allow_sort);
+                     gs_lr, &S->lrl, 1, nullptr, -1, allow_sort, which == -1 && nlist_counts_in_one_kernel(S->n));
     if (rc) return rc;
   }
   SO3LR_CUDA_CHECK(cudaStreamSynchronize(st));
   if (which != 1) rc = nlist_end(S->nws, st, S->cell, &S->sr);
   if (rc) return rc;
   if (which != 0) {
-    rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
+    rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl, which == -1);
     // the first list is filled: its votes have served (dev_free waits for the device)
     if (rc == kCudaError && which != 1 && nlist_drop_votes(S->nws)) rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
   }

@@ -11,11 +11,10 @@ cudaError_t host_alloc_bytes(void** p, size_t bytes);
 void host_free(void* p);
 void devmem_flush(int device);     // gives the idle blocks back
 long long devmem_fail(long long nth, bool on);      // tests: see so3lr_b200_host_fail_allocation
-// Launch whose kernel starts with grid_dep_sync(): its CTAs may be placed while the kernel before it in the stream still runs, so that the
-// launch itself (1.5 to 2 us between two dependent kernels) and the kernel's own preparations overlap with that one's end.  Like that of
-// <<<>>>, a failure stays with the runtime: every entry point asks for it with cudaGetLastError after its last launch.
+// Launch of a kernel that may start once every CTA of the kernel before it in the stream has let it (griddepcontrol.launch_dependents) or is
+// through
 template <typename... P, typename... A>
-void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -23,6 +22,13 @@ void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cu
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = s;
   c.attrs = attr; c.numAttrs = 1;
   cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+// Launch whose kernel starts with grid_dep_sync(): its CTAs may be placed while the kernel before it in the stream still runs, so that the
+// launch itself (1.5 to 2 us between two dependent kernels) and the kernel's own preparations overlap with that one's end.  Like that of
+// <<<>>>, a failure stays with the runtime: every entry point asks for it with cudaGetLastError after its last launch.
+template <typename... P, typename... A>
+void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  launch_early(kernel, grid, block, smem, s, args...);
 }
 template <typename T>
 cudaError_t dev_alloc(T** p, size_t n) { return dev_alloc_bytes(reinterpret_cast<void**>(p), (n ? n : 1) * sizeof(T)); }
@@ -309,9 +315,11 @@ int nlist_row_total(cudaStream_t s, int n, const int* row_count_dev, long long* 
 // nlist_build in two halves with a wait for the stream between them: several lists (a workspace each) share one wait.  `any_order`: the
 // entries of a row may come in any order.
 int nlist_begin(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered, const int* seg,
-                const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order);
+                const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order,
+                bool beside = false);
+bool nlist_counts_in_one_kernel(int n);         // the count kernel of n rows is the last thing that nlist_begin enqueues
 bool nlist_drop_votes(NlistWorkspace* ws);      // short of memory: the workspace gives up what it can do without
-int nlist_end(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, NeighborListDev* out);
+int nlist_end(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, NeighborListDev* out, bool beside = false);
 int nlist_build(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
                 const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows = -1);
 

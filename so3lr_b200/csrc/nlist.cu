@@ -276,6 +276,11 @@ __device__ __forceinline__ void build_row(const Cell& cell, const Grid& G, int n
   if (!FILL && lane == 0) row_count[i] = count;
 }
 
+// The row kernels of the short- and the long-range list of a rebuild do not depend on each other: the second may run beside the first (see
+// `beside` in nlist_begin).  It then has no wait at its start, but ends no earlier than the first: what follows waits for it alone.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void end_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <bool FILL>
 __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int n, const float* __restrict__ R, float r_list, float r2max,
                                                          int ordered, const int* __restrict__ seg,
@@ -283,6 +288,7 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
                                                          int* __restrict__ row_count, const int* __restrict__ row_ptr,
                                                          int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
                                                          unsigned* __restrict__ masks, int mask_stride, TailScan tail) {
+  let_next_start();
   build_row<FILL>(cell, G, n, R, r_list, r2max, ordered, seg, pos_sorted, cell_start, row_count, row_ptr, nbr_j, edge_i, capacity, masks, mask_stride);
   if (!FILL) {
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -292,6 +298,7 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
     }
     tail_scan(tail, n, row_count);
   }
+  end_after_previous();
 }
 
 // batched free-space graphs: the candidates of atom i are the atoms of its own graph
@@ -301,6 +308,7 @@ __global__ void __launch_bounds__(256) build_rows_graph_kernel(int n, const floa
                                                                int* __restrict__ row_count, const int* __restrict__ row_ptr,
                                                                int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
                                                                TailScan tail) {
+  let_next_start();
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i < n) {
@@ -326,6 +334,7 @@ __global__ void __launch_bounds__(256) build_rows_graph_kernel(int n, const floa
   if (!FILL && lane == 0) row_count[i] = count;
   }
   if (!FILL) tail_scan(tail, n, row_count);
+  end_after_previous();
 }
 
 // 64-bit sum of the per-row counts.  The exclusive scan that follows runs in 32 bits (CSR offsets are int): this total, not
@@ -396,6 +405,12 @@ int ensure_atoms(NlistWorkspace* w, int n) {
   w->n_cap = n;
   return kOk;
 }
+template <class... P, class... A>
+void launch_rows(bool beside, void (*kernel)(P...), int blocks, cudaStream_t s, A&&... args) {
+  if (beside) launch_early(kernel, blocks, 256, 0, s, args...);
+  else kernel<<<blocks, 256, 0, s>>>(static_cast<P>(args)...);
+  count_launch();
+}
 int ensure_bytes(void** p, size_t* have, size_t need) {
   if (need <= *have) return kOk;
   if (*p) dev_free(*p);
@@ -458,8 +473,12 @@ int spatial_order(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, co
 // cells costs the read-back of all positions.  The line lies below the crossing: the tests grow with the square of the atoms.
 constexpr int kOneCellAtoms = 1024;
 
+bool nlist_counts_in_one_kernel(int n) { return n <= kTailScanRows; }
+// `beside`: the kernel enqueued last is another list's count (or, in nlist_end, fill), beside which this one's may run.  Short lists are bound
+// by latency: the four row kernels of 1,536 atoms take 23, 26, 16 and 13 us one behind the other, the last CTA's scan of each among them.
 int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
-                const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order) {
+                const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order,
+                bool beside) {
   w->n_rows = 0;
   if (n <= 0) { out->count = 0; return kOk; }
   if (n_rows < 0 || n_rows > n) n_rows = n;
@@ -467,6 +486,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   if (!w->ticket) {
     SO3LR_CUDA_CHECK(dev_alloc(&w->ticket, 2));
     SO3LR_CUDA_CHECK(cudaMemsetAsync(w->ticket, 0, 2 * sizeof(int), s));
+    beside = false;
   }
   if (!w->d_total) SO3LR_CUDA_CHECK(dev_alloc(&w->d_total, 1));
   if (!w->h_total) SO3LR_CUDA_CHECK(host_alloc(&w->h_total, 1));
@@ -499,6 +519,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     } else {
       // bounding box on the host side would need a reduction; use a coarse device-free approach: the caller
       // passes free-space systems of moderate size, so read the positions back once per build.
+      beside = false;
       std::vector<float> h((size_t)n * 3);
       SO3LR_CUDA_CHECK(cudaMemcpyAsync(h.data(), R, h.size() * sizeof(float), cudaMemcpyDeviceToHost, s));
       SO3LR_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -518,6 +539,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     n_cells = G.nc[0] * G.nc[1] * G.nc[2];
     binned = n_cells > 1;      // the atoms of a single cell come in their own order either way
     if (binned) {
+      beside = false;      // its own cells come first
       if (n_cells + 1 > w->cell_cap) {
         w->cell_cap = 0;
         if (int rcc = ensure(&w->cell_start, (size_t)n_cells + 1)) return rcc;
@@ -569,10 +591,10 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
   if (n_rows <= kTailScanRows && allow_grow) { tail.ticket = w->ticket; tail.row_ptr = out->row_ptr; tail.total_host = w->h_total; }
   tail.check_finite = tail.ticket && !by_graph && !cell.periodic && !binned;      // in place of the bounding box's test of the extent
   if (by_graph)
-    { build_rows_graph_kernel<false><<<blocks, 256, 0, s>>>(n_rows, R, r2max, ordered, seg, graph_start, w->row_count, nullptr, nullptr, nullptr, 0, tail); count_launch(); }
+    launch_rows(beside, build_rows_graph_kernel<false>, blocks, s, n_rows, R, r2max, ordered, seg, graph_start, w->row_count, nullptr, nullptr, nullptr, 0, tail);
   else
-    { build_rows_kernel<false><<<blocks, 256, 0, s>>>(cell, G, n_rows, R, r_list, r2max, ordered, seg, binned ? w->pos_sorted : nullptr,
-                                                    w->cell_start, w->row_count, nullptr, nullptr, nullptr, 0, masks, mask_stride, tail); count_launch(); }
+    launch_rows(beside, build_rows_kernel<false>, blocks, s, cell, G, n_rows, R, r_list, r2max, ordered, seg, binned ? w->pos_sorted : nullptr,
+                w->cell_start, w->row_count, nullptr, nullptr, nullptr, 0, masks, mask_stride, tail);
   if (!tail.ticket) {
     SO3LR_CUDA_CHECK(cudaMemsetAsync(w->d_total, 0, sizeof(long long), s));
     { int tb = (n_rows + 255) / 256; if (tb > 1024) tb = 1024;
@@ -590,7 +612,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
 }
 
 // the second half, once the stream has been waited for
-int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListDev* out) {
+int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListDev* out, bool beside) {
   const int n_rows = w->n_rows;
   if (n_rows <= 0) return kOk;
   const int blocks = (n_rows + 7) / 8, allow_grow = w->allow_grow;
@@ -619,12 +641,12 @@ int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListD
   if (total <= out->capacity) out->count = total;
   const bool truncated = total > out->capacity;
   if (w->by_graph)
-    { build_rows_graph_kernel<true><<<blocks, 256, 0, s>>>(n_rows, w->R, r2max, w->ordered, w->seg, w->graph_start, nullptr, out->row_ptr,
-                                                         out->nbr_j, out->edge_i, out->capacity, TailScan{}); count_launch(); }
+    launch_rows(beside, build_rows_graph_kernel<true>, blocks, s, n_rows, w->R, r2max, w->ordered, w->seg, w->graph_start, nullptr, out->row_ptr,
+                out->nbr_j, out->edge_i, out->capacity, TailScan{});
   else
-    { build_rows_kernel<true><<<blocks, 256, 0, s>>>(cell, w->G, n_rows, w->R, w->r_list, r2max, w->ordered, w->seg, w->binned ? w->pos_sorted : nullptr,
-                                                   w->cell_start, nullptr, out->row_ptr, out->nbr_j, out->edge_i, out->capacity, w->masks,
-                                                   w->mask_stride, TailScan{}); count_launch(); }
+    launch_rows(beside, build_rows_kernel<true>, blocks, s, cell, w->G, n_rows, w->R, w->r_list, r2max, w->ordered, w->seg,
+                w->binned ? w->pos_sorted : nullptr, w->cell_start, nullptr, out->row_ptr, out->nbr_j, out->edge_i, out->capacity, w->masks,
+                w->mask_stride, TailScan{});
   if (truncated) { clamp_rows_kernel<<<(n_rows + 1 + 255) / 256, 256, 0, s>>>(n_rows, out->row_ptr, out->capacity); count_launch(); }
   SO3LR_CUDA_CHECK(cudaGetLastError());
   return truncated ? kOverflow : kOk;

@@ -606,8 +606,9 @@ void launch_pair_lr_packed(cudaStream_t s, const LrParams& P, const Cell& cell, 
   float4* hz = acc + n;
   launch_chained(pair_pack_kernel, (n + 255) / 256, 256, 0, s, n, R, q, h, Z, pq, hz, acc);
   const int split = pair_row_split(n, pairs);
-  launch_chained(skin ? pair_lr_packed_kernel<true> : pair_lr_packed_kernel<false>, (unsigned)(((long long)n * split + 7) / 8), 256, 0, s, P, cell, n, split, row_ptr, nbr_j, pq, hz, acc,
-                 gh, e_coul, e_disp, virial);
+  const unsigned blocks = (unsigned)(((long long)n * split + 7) / 8);
+  if (skin) launch_chained(pair_lr_packed_kernel<true>, blocks, 256, 0, s, P, cell, n, split, row_ptr, nbr_j, pq, hz, acc, gh, e_coul, e_disp, virial);
+  else launch_chained(pair_lr_packed_kernel<false>, blocks, 256, 0, s, P, cell, n, split, row_ptr, nbr_j, pq, hz, acc, gh, e_coul, e_disp, virial);
   launch_chained(pair_unpack_kernel, (n + 255) / 256, 256, 0, s, n, acc, F, gq, e_nn, e_zbl, e_coul, e_disp, e_atom);
   count_launch(3);
 }
