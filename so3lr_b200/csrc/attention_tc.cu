@@ -12,18 +12,23 @@
 // from a table (4 KB per edge and layer through L2 before); hs_f is the hidden layer of the spherical filter.  FP32 accuracy
 // comes from the two-term FP16 split used throughout the library (x = hi + lo / 2048; products hi*hi into one accumulator,
 // hi*lo + lo*hi into a second one).  Operands sit in shared memory in the 8 x 8 core-matrix order without swizzle; the
-// 96 KB weight image is resident for the whole kernel.  One thread issues the MMAs; completion arrives on an mbarrier
-// (tcgen05.commit); every wait is bounded and reports through an error word instead of hanging.
+// 96 KB weight image is resident for the whole kernel.  Four warps issue the MMAs, one per scheduler and accumulator; completion arrives on
+// an mbarrier (tcgen05.commit) on which every thread waits for itself; every wait is bounded and reports through an error word
+// instead of hanging.
 //
 // After the MMA the filter tile is moved from tensor memory to shared memory (row = edge) and the edge loop runs in the
 // "lane = 4 features" layout of the other attention kernels: sender rows are read with coalesced 512-byte loads, logits are
 // 8-lane reductions.  A warp owns a run of consecutive pairs and adds its partial sums to the receiver's row with vector
 // reductions in global memory (a receiver's pairs can span warps, tiles and CTAs); the partner's share of a pair goes out as one
 // reduction per row.  Those cost less than the second evaluation they replace: the L2 takes 5.4 TB/s of 512-byte row reductions
-// (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.  With every pair evaluated at
-// both ends instead, 98,304 atoms took 1.99 / 5.12 ms a launch (forward / reverse), with one evaluation 1.23 / 3.12 ms, and with the
-// logits of four pairs of a receiver summed together, no branches between them, and the first filter finished beneath the second
-// filter's chain, 1.16 / 2.79 ms.
+// (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.
+//
+// What binds the kernels: the latency of four warps per scheduler (their 128 registers fill the register file).  Per 128 pairs the reverse
+// kernel issues 64 k warp instructions (16 k cycles of the 44 k a tile takes), moves 23 k wavefronts through the load / store pipe, 4 k
+// through the tensor cores' and keeps the way to the L2 busy for 18 k cycles (a row reduction leaves an SM at 21 to 26 bytes per cycle);
+// none is near its limit, and forms with more warps, fewer registers or two independent tiles per SM ended within 15 % of it or above.
+// 98,304 atoms (1.97 M pairs), forward / reverse, ms per launch: 1.99 / 5.12 with every pair evaluated at both ends, 1.16 / 2.85 with one
+// evaluation per pair, entry loops that sum four pairs' logits together and one thread that issues, 1.01 / 2.50 as it stands.
 //
 // The reverse kernel forms dw in the same loop, writes it straight into shared memory as the (FP16-split) A operand of a
 // second MMA chain against the SAME weight image read with the other major-ness,
