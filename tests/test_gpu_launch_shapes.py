@@ -69,16 +69,26 @@ def test_rows_shared_by_warps_and_queued_pairs(molecules):
     assert np.abs(W0 - W1).max() <= 2e-4 * np.abs(W0).max()
 
 
-@pytest.mark.parametrize("molecules,periodic", [(3, False), (64, True), (300, False), (512, True), (2048, True), (11000, True)])
-def test_lists_built_side_by_side(molecules, periodic):
-    """Both lists of an evaluation, whose row kernels may overlap, against each of them exported alone."""
+@pytest.mark.parametrize("molecules,form,cutoff", [(3, "free", 9.0), (64, "box", 9.0), (300, "free", 9.0), (512, "box", 9.0), (2048, "box", 9.0),
+                                                   (11000, "box", 9.0), (1200, "box", 12.0), (2048, "box", 12.0), (2048, "sheared", 12.0),
+                                                   (4100, "long", 12.0)])
+def test_lists_built_for_an_evaluation(molecules, form, cutoff):
+    """Both lists of an evaluation, whose row kernels may overlap, against each of them exported alone: the numbers of entries exactly, in two
+    positions of the cells."""
     from so3lr_b200.engine import System
     Z, R, cell = _box(molecules, 90)
-    s = System(Z, cell if periodic else None, cutoff_lr=9.0, damping=2.0)
-    for shift in (0.0, 0.37):
+    if form == "free":
+        cell = None
+    elif form == "sheared":      # a skewed cell of the same volume: another packing, whose overlaps do not matter to a list
+        cell = np.asarray(cell, dtype=np.float64) + np.array([[0, 0, 0], [0.3, 0, 0], [-0.2, 0.25, 0]]) * float(cell[0][0])
+    elif form == "long":
+        cell = np.asarray(cell, dtype=np.float64) * np.array([[2.0], [1.0], [0.8]])
+        R = R * torch.tensor([2.0, 1.0, 0.8], device="cuda")
+    s = System(Z, cell, cutoff_lr=cutoff, damping=2.0)
+    alone = System(Z, cell, cutoff_lr=cutoff, damping=2.0)
+    for shift in (0.0, 3.37):
         s.compute(R + shift)
         both = s.stats()
-        alone = System(Z, cell if periodic else None, cutoff_lr=9.0, damping=2.0)
         for which, key in ((0, "edges"), (1, "pairs")):
             _, count, overflow = alone.neighbor_list(R + shift, which, both[key] + 8)
             assert count == both[key] and not overflow, (which, count, both[key])
