@@ -2136,7 +2136,8 @@ SO3LR_B200_API void so3lr_b200_host_dispersion_fast(float r, int zi, int zj, flo
   LrParams P{};
   P.has_cutoff = cutoff_lr > 0.f; P.rc = cutoff_lr; P.cuton = kCutonFraction * cutoff_lr; P.has_damping = damping > 0.f;
   P.disp_on = cutoff_lr - damping; P.pair_factor = 1.f;
-  dispersion_pair_fast(P, r, zi, zj, hi, hj, out4[0], out4[1], out4[2], out4[3]);
+  if (P.has_cutoff && r >= P.rc) { for (int k = 0; k < 4; ++k) out4[k] = 0.f; return; }      // the kernels leave such pairs out
+  dispersion_pair_fast(P, r, alpha_free(zi), dispersion_x(zi), hi, alpha_free(zj), dispersion_x(zj), hj, out4[0], out4[1], out4[2], out4[3]);
 }
 SO3LR_B200_API void so3lr_b200_host_zbl(const float* blob, float r, int zi, int zj, float* out2) {
   BlobOffsets O = blob_offsets();

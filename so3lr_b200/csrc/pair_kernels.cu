@@ -69,27 +69,7 @@ __global__ void force_scatter_kernel(int n, long long n_edges, const int* __rest
   atomicAdd(F + 3 * (size_t)j, -gx); atomicAdd(F + 3 * (size_t)j + 1, -gy); atomicAdd(F + 3 * (size_t)j + 2, -gz);
 }
 
-// one warp per row i; lanes stride over the row's pairs
-// Device forms of the pair terms for the long-range kernels: the same functions as coulomb_chi / dispersion_pair_fast / switching
-// of pair_terms.cuh with approximate reciprocals and exponentials (rcp.approx, ex2.approx, lg2.approx: 1-2 ulp each) in place
-// of IEEE divisions and libm calls, and the switch written with one exponential:
-//   s(1-c) / (s(1-c) + s(c)),  s(a) = exp(-1/a)   ==   1 / (1 + E),  E = exp(1/(1-c) - 1/c)
-__device__ __forceinline__ float rcp_fast(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ void switching_dev(float x, float on, float off, float& f, float& df) {
-  const float iw = rcp_fast(off - on);
-  const float c = (x - on) * iw;
-  if (c <= 0.f) { f = 1.f; df = 0.f; return; }
-  if (c >= 1.f) { f = 0.f; df = 0.f; return; }
-  const float ia = rcp_fast(1.f - c), ib = rcp_fast(c);
-  const float t = fminf(fmaxf(ia - ib, -80.f), 80.f);
-  const float E = __expf(t);
-  f = rcp_fast(1.f + E);
-  df = -(E * f) * (f * (ia * ia + ib * ib)) * iw;   // in this order no intermediate leaves the float range
-}
+// coulomb_chi of pair_terms.cuh with the approximate operations
 __device__ __forceinline__ void coulomb_chi_dev(const LrParams& p, float r, float rinv, float& chi, float& dchi) {
   const float inv_sig = 1.f / kSigmaCoulomb;
   const float x = r * inv_sig;
@@ -103,48 +83,12 @@ __device__ __forceinline__ void coulomb_chi_dev(const LrParams& p, float r, floa
   }
   if (!p.has_cutoff) { chi = pot; dchi = dpot; return; }
   float f, df;
-  switching_dev(r, p.cuton, p.rc, f, df);
+  switching_fast(r, p.cuton, p.rc, f, df);
   chi = (pot - p.v_rc) - (1.f - f) * (r - p.rc) * p.dv_rc;
   dchi = dpot - (1.f - f) * p.dv_rc + df * (r - p.rc) * p.dv_rc;
 }
-// With a = alpha h and c = c6 h^2 the combination rule 2 c_i c_j a_i a_j / (a_i^2 c_j + a_j^2 c_i) is linear in both ratios,
-//   c6_ij = K h_i h_j,  K = 2 alpha_i alpha_j / (x_i + x_j),  x = alpha^2 / c6  of the free atom,
-// so its derivatives cost nothing.  The partials of T share the powers of R and p.
-__device__ __forceinline__ float dispersion_x(int Z) { return alpha_free(Z) * alpha_free(Z) / c6_free(Z); }
-__device__ __forceinline__ void dispersion_pair_dev(const LrParams& P, float r, float alf_i, float x_i, float hi, float alf_j, float x_j,
-                                                    float hj, float& e, float& de_dr, float& de_dhi, float& de_dhj) {
-  const float aij = 0.5f * fmaf(alf_i, hi, alf_j * hj);
-  const float a17 = exp2f(__log2f(aij) * (1.f / 7.f));
-  const float fs = 2.5527961000248887f;
-  const float rv = fs * a17;
-  const float sg = fmaf(fmaf(fmaf(-0.00078893f, rv, 0.04125273f), rv, 0.24428889f), rv, -0.00433008f);
-  const float dsg = fmaf(fmaf(3.f * -0.00078893f, rv, 2.f * 0.04125273f), rv, 0.24428889f);
-  const float ig = 2.f * sg * sg;
-  const float kp = kDispersionScale * 2.f * 2.54f;
-  const float p = kp * a17;
-  const float R = r * (1.f / kBohr);
-  const float R2 = R * R, p2 = p * p;
-  const float R4 = R2 * R2, p4 = p2 * p2;
-  const float R6 = R4 * R2, p6 = p4 * p2;
-  const float i6 = rcp_fast(R6 + p6), i8 = rcp_fast(fmaf(R4, R4, p4 * p4)), i10 = rcp_fast(fmaf(R6, R4, p6 * p4));
-  const float t8 = 5.f * ig * i8, t10 = 30.625f * ig * ig * i10;
-  const float T = i6 + t8 + t10;
-  const float u6 = 6.f * i6 * i6, u8 = 8.f * t8 * i8, u10 = 10.f * t10 * i10;
-  const float dT_dR = -R4 * R * fmaf(R2, fmaf(R2, u10, u8), u6);
-  const float dT_dp = -p4 * p * fmaf(p2, fmaf(p2, u10, u8), u6);
-  const float dT_dig = fmaf(61.25f * ig, i10, 5.f * i8);
-  const float dT_da17 = fmaf(dT_dp, kp, dT_dig * (4.f * fs) * sg * dsg);
-  const float W = dT_da17 * a17 * rcp_fast(14.f * aij);          // dT / d(alpha_i h_i)
-  float f = 1.f, df = 0.f;
-  if (P.has_cutoff && P.has_damping) switching_dev(r, P.disp_on, P.rc, f, df);
-  const float pre = (-2.f * kHartree) * alf_i * alf_j * rcp_fast(x_i + x_j);
-  const float pf = pre * f, hh = hi * hj;
-  e = pf * hh * T;
-  de_dr = pre * hh * fmaf(dT_dR * (1.f / kBohr), f, T * df);
-  de_dhi = pf * hj * fmaf(hi * alf_i, W, T);
-  de_dhj = pf * hi * fmaf(hj * alf_j, W, T);
-}
 
+// one warp per row i; lanes stride over the row's pairs
 template <int MODE>
 __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int n, const int* __restrict__ row_ptr,
                                                       const int* __restrict__ nbr_j, const int* __restrict__ Z,
@@ -188,7 +132,7 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
         const float e_c = kq * qi * qj * chi;
         float e_d, dd_dr, dd_dhi, dd_dhj;
         const int Zj = Z[j];
-        dispersion_pair_dev(P, r, alf_i, x_i, hi, alpha_free(Zj), dispersion_x(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
+        dispersion_pair_fast(P, r, alf_i, x_i, hi, alpha_free(Zj), dispersion_x(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
         e_d *= pf; dd_dr *= pf; dd_dhi *= pf; dd_dhj *= pf;
         ec += e_c; ed += e_d;
         gqi = fmaf(kq * qj, chi, gqi);
@@ -277,7 +221,7 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
     float chi, dchi;
     coulomb_chi_dev(P, r, rinv, chi, dchi);
     float e_d, dd_dr, dd_dhi, dd_dhj;
-    dispersion_pair_dev(P, r, hzi.y, hzi.z, hi, hzj.y, hzj.z, hzj.x, e_d, dd_dr, dd_dhi, dd_dhj);
+    dispersion_pair_fast(P, r, hzi.y, hzi.z, hi, hzj.y, hzj.z, hzj.x, e_d, dd_dr, dd_dhi, dd_dhj);
     ec = fmaf(kq * qi * qj, chi, ec);
     ed = fmaf(pf, e_d, ed);
     gqi = fmaf(kq * qj, chi, gqi);
@@ -377,7 +321,7 @@ __global__ void __launch_bounds__(256) pair_lr_owned_kernel(LrParams P, Cell cel
     const float qj = q[j], hj = h[j];
     const int Zj = Z[j];
     float e_d, dd_dr, dd_dhi, dd_dhj;
-    dispersion_pair_dev(P, r, alf_i, x_i, hi, alpha_free(Zj), dispersion_x(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
+    dispersion_pair_fast(P, r, alf_i, x_i, hi, alpha_free(Zj), dispersion_x(Zj), hj, e_d, dd_dr, dd_dhi, dd_dhj);
     const bool both = j < n_owned;
     const float w = both ? 1.f : 0.5f;                             // share of the pair energy booked on this row
     ec = fmaf(w * kKe * qi * qj, chi, ec);

@@ -109,55 +109,85 @@ SO3LR_HD void dispersion_pair(const LrParams& p, float r, int Zi, int Zj, float 
   e = E.v; de_dr = E.d0; de_dhi = E.d1; de_dhj = E.d2;
 }
 
-// The same dispersion energy and derivatives with hand-derived partials instead of forward-mode dual numbers (about a
-// quarter of the arithmetic; used by the long-range pair kernels, checked against dispersion_pair on the host).
+// Approximate operations of the long-range pair kernels (rcp.approx, ex2.approx, lg2.approx: 1-2 ulp each) in place of IEEE divisions and
+// libm calls, which stand in for them on the host.
+SO3LR_HD float rcp_fast(float x) {
+#ifdef __CUDA_ARCH__
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+#else
+  return 1.f / x;
+#endif
+}
+SO3LR_HD float exp_fast(float x) {
+#ifdef __CUDA_ARCH__
+  return __expf(x);
+#else
+  return expf(x);
+#endif
+}
+SO3LR_HD float seventh_root(float x) {
+#ifdef __CUDA_ARCH__
+  return exp2f(__log2f(x) * (1.f / 7.f));
+#else
+  return powf(x, 1.f / 7.f);
+#endif
+}
+// `switching` with one exponential: s(1-c) / (s(1-c) + s(c)),  s(a) = exp(-1/a)   ==   1 / (1 + E),  E = exp(1/(1-c) - 1/c)
+SO3LR_HD void switching_fast(float x, float on, float off, float& f, float& df) {
+  const float iw = rcp_fast(off - on);
+  const float c = (x - on) * iw;
+  if (c <= 0.f) { f = 1.f; df = 0.f; return; }
+  if (c >= 1.f) { f = 0.f; df = 0.f; return; }
+  const float ia = rcp_fast(1.f - c), ib = rcp_fast(c);
+  const float t = fminf(fmaxf(ia - ib, -80.f), 80.f);
+  const float E = exp_fast(t);
+  f = rcp_fast(1.f + E);
+  df = -(E * f) * (f * (ia * ia + ib * ib)) * iw;   // in this order no intermediate leaves the float range
+}
+
+// The dispersion term of the long-range pair kernels, with hand-derived partials (checked against float64 on the host); the caller keeps
+// to pairs inside the cutoff.
 //   E = -Hartree * c6 * T * f(r),  T = 1/(R^6+p^6) + 5 ig/(R^8+p^8) + 30.625 ig^2/(R^10+p^10),  R = r / Bohr,
 //   p = 6.096 a17, ig = 2 sg^2, sg = cubic(fs * a17), a17 = ((a_i + a_j)/2)^(1/7), a = alpha_free * h, c = c6_free * h^2,
 //   c6 = 2 c_i c_j a_i a_j / (a_i^2 c_j + a_j^2 c_i)
-SO3LR_HD void dispersion_pair_fast(const LrParams& P, float r, int Zi, int Zj, float hi, float hj, float& e, float& de_dr,
-                                   float& de_dhi, float& de_dhj) {
-  if (P.has_cutoff && r >= P.rc) { e = de_dr = de_dhi = de_dhj = 0.f; return; }
-  const float alf_i = alpha_free(Zi), alf_j = alpha_free(Zj), c6f_i = c6_free(Zi), c6f_j = c6_free(Zj);
-  const float ai = alf_i * hi, aj = alf_j * hj, ci = c6f_i * hi * hi, cj = c6f_j * hj * hj;
-  const float den = ai * ai * cj + aj * aj * ci, iden = 1.f / den;
-  const float c6 = 2.f * ci * cj * ai * aj * iden;
-  // d ln c6 / d h = (d ln c6/d a) alpha + (d ln c6/d c) 2 c6free h
-  const float dlc6_dhi = (1.f / ai - 2.f * ai * cj * iden) * alf_i + (1.f / ci - aj * aj * iden) * 2.f * c6f_i * hi;
-  const float dlc6_dhj = (1.f / aj - 2.f * aj * ci * iden) * alf_j + (1.f / cj - ai * ai * iden) * 2.f * c6f_j * hj;
-  const float aij = 0.5f * (ai + aj);
-#ifdef __CUDA_ARCH__
-  const float a17 = exp2f(log2f(aij) * (1.f / 7.f));
-#else
-  const float a17 = powf(aij, 1.f / 7.f);
-#endif
+// With a = alpha h and c = c6 h^2 that combination rule is linear in both ratios,
+//   c6_ij = K h_i h_j,  K = 2 alpha_i alpha_j / (x_i + x_j),  x = alpha^2 / c6  of the free atom,
+// so its derivatives cost nothing.  The partials of T share the powers of R and p.
+SO3LR_HD float dispersion_x(int Z) { return alpha_free(Z) * alpha_free(Z) / c6_free(Z); }
+SO3LR_HD void dispersion_pair_fast(const LrParams& P, float r, float alf_i, float x_i, float hi, float alf_j, float x_j,
+                                   float hj, float& e, float& de_dr, float& de_dhi, float& de_dhj) {
+  const float aij = 0.5f * fmaf(alf_i, hi, alf_j * hj);
+  const float a17 = seventh_root(aij);
   const float fs = 2.5527961000248887f;
   const float rv = fs * a17;
-  const float sg = ((-0.00078893f * rv + 0.04125273f) * rv + 0.24428889f) * rv + (-0.00433008f);
-  const float dsg = ((3.f * -0.00078893f) * rv + 2.f * 0.04125273f) * rv + 0.24428889f;
+  const float sg = fmaf(fmaf(fmaf(-0.00078893f, rv, 0.04125273f), rv, 0.24428889f), rv, -0.00433008f);
+  const float dsg = fmaf(fmaf(3.f * -0.00078893f, rv, 2.f * 0.04125273f), rv, 0.24428889f);
   const float ig = 2.f * sg * sg;
   const float kp = kDispersionScale * 2.f * 2.54f;
   const float p = kp * a17;
   const float R = r * (1.f / kBohr);
   const float R2 = R * R, p2 = p * p;
   const float R4 = R2 * R2, p4 = p2 * p2;
-  const float R6 = R4 * R2, p6 = p4 * p2, R8 = R4 * R4, p8 = p4 * p4, R10 = R8 * R2, p10 = p8 * p2;
-  const float i6 = 1.f / (R6 + p6), i8 = 1.f / (R8 + p8), i10 = 1.f / (R10 + p10);
-  const float t8 = 5.f * ig, t10 = 30.625f * ig * ig;
-  const float T = i6 + t8 * i8 + t10 * i10;
-  // partials of T
-  const float dT_dR = -(6.f * R4 * R * i6 * i6 + t8 * 8.f * R6 * R * i8 * i8 + t10 * 10.f * R8 * R * i10 * i10);
-  const float dT_dp = -(6.f * p4 * p * i6 * i6 + t8 * 8.f * p6 * p * i8 * i8 + t10 * 10.f * p8 * p * i10 * i10);
-  const float dT_dig = 5.f * i8 + 61.25f * ig * i10;
-  // a17 enters through p (= kp a17) and through sg(rv = fs a17)
-  const float dT_da17 = dT_dp * kp + dT_dig * 4.f * sg * dsg * fs;
-  const float da17_dh = a17 / (7.f * aij) * 0.5f;          // times alpha_free of the atom
+  const float R6 = R4 * R2, p6 = p4 * p2;
+  const float i6 = rcp_fast(R6 + p6), i8 = rcp_fast(fmaf(R4, R4, p4 * p4)), i10 = rcp_fast(fmaf(R6, R4, p6 * p4));
+  const float t8 = 5.f * ig * i8, t10 = 30.625f * ig * ig * i10;
+  const float T = i6 + t8 + t10;
+  const float u6 = 6.f * i6 * i6, u8 = 8.f * t8 * i8, u10 = 10.f * t10 * i10;
+  const float dT_dR = -R4 * R * fmaf(R2, fmaf(R2, u10, u8), u6);
+  const float dT_dp = -p4 * p * fmaf(p2, fmaf(p2, u10, u8), u6);
+  const float dT_dig = fmaf(61.25f * ig, i10, 5.f * i8);
+  const float dT_da17 = fmaf(dT_dp, kp, dT_dig * (4.f * fs) * sg * dsg);
+  const float W = dT_da17 * a17 * rcp_fast(14.f * aij);          // dT / d(alpha_i h_i)
   float f = 1.f, df = 0.f;
-  if (P.has_cutoff && P.has_damping) switching(r, P.disp_on, P.rc, f, df);
-  const float pre = -kHartree * c6;
-  e = pre * T * f;
-  de_dr = pre * (dT_dR * (1.f / kBohr) * f + T * df);
-  de_dhi = pre * f * (T * dlc6_dhi + dT_da17 * da17_dh * alf_i);
-  de_dhj = pre * f * (T * dlc6_dhj + dT_da17 * da17_dh * alf_j);
+  if (P.has_cutoff && P.has_damping) switching_fast(r, P.disp_on, P.rc, f, df);
+  const float pre = (-2.f * kHartree) * alf_i * alf_j * rcp_fast(x_i + x_j);
+  const float pf = pre * f, hh = hi * hj;
+  e = pf * hh * T;
+  de_dr = pre * hh * fmaf(dT_dR * (1.f / kBohr), f, T * df);
+  de_dhi = pf * hj * fmaf(hi * alf_i, W, T);
+  de_dhj = pf * hi * fmaf(hj * alf_j, W, T);
 }
 
 struct ZblParams {

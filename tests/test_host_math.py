@@ -1,6 +1,8 @@
 """Host-callable pieces of the device math (same source as the kernels) against the CPU oracle. No GPU needed."""
 import ctypes as C
 import math
+import os
+import re
 
 import numpy as np
 import pytest
@@ -17,7 +19,6 @@ def _p(a):
 
 
 def test_library_exports_every_declared_symbol():
-    import os, re
     hdr = open(os.path.join(os.path.dirname(__file__), "..", "include", "so3lr_b200.h")).read()
     declared = set(re.findall(r"\b(so3lr_b200_[a-z0-9_]+)\s*\(", hdr))
     declared -= {"so3lr_b200_model", "so3lr_b200_system", "so3lr_b200_options"}
@@ -69,12 +70,21 @@ def test_pair_terms_match_oracle(cutoff, damping):
         np.testing.assert_allclose(out[3], ed.item(), rtol=5e-5, atol=1e-7)
         np.testing.assert_allclose(out[4], ded_r.item(), rtol=2e-4, atol=1e-7)
         np.testing.assert_allclose(out[5:7], ded_h.numpy(), rtol=2e-4, atol=1e-7)
-        # the hand-derived form the pair kernels use
+        # the function that the pair kernels evaluate (test_pair_kernels_evaluate_the_checked_dispersion_term), its approximate operations
+        # replaced by libm's
         o4 = np.zeros(4, np.float32)
         lib.so3lr_b200_host_dispersion_fast(r, zi, zj, hi, hj, cutoff, damping, _p(o4))
         np.testing.assert_allclose(o4[0], ed.item(), rtol=5e-5, atol=1e-7)
         np.testing.assert_allclose(o4[1], ded_r.item(), rtol=2e-4, atol=1e-7)
         np.testing.assert_allclose(o4[2:4], ded_h.numpy(), rtol=2e-4, atol=1e-7)
+
+
+def test_pair_kernels_evaluate_the_checked_dispersion_term():
+    """What the host check above covers is what the kernels call: they hold no dispersion term of their own."""
+    src = open(os.path.join(os.path.dirname(__file__), "..", "so3lr_b200", "csrc", "pair_kernels.cu")).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    assert len(re.findall(r"(?<!void )\bdispersion_pair_fast\(", src)) >= 3
+    assert not re.findall(r"\bvoid dispersion\w*\(", src)
 
 
 def test_zbl_matches_oracle(oracle_params):
