@@ -174,18 +174,21 @@ SO3LR_HD void dispersion_pair_fast(const LrParams& P, float r, float alf_i, floa
   const float i6 = rcp_fast(R6 + p6), i8 = rcp_fast(fmaf(R4, R4, p4 * p4)), i10 = rcp_fast(fmaf(R6, R4, p6 * p4));
   const float t8 = 5.f * ig * i8, t10 = 30.625f * ig * ig * i10;
   const float T = i6 + t8 + t10;
-  const float u6 = 6.f * i6 * i6, u8 = 8.f * t8 * i8, u10 = 10.f * t10 * i10;
+  // R^-12 and R^-20 leave the float range long before the slope R^-7 does (digits go from 900 A on, everything at 4,000 A): scaled by 2^40,
+  // which the constants of both partials take back
+  constexpr float kUp = 1099511627776.f, kDown = 1.f / kUp;
+  const float u6 = (6.f * kUp) * i6 * i6, u8 = (8.f * kUp) * t8 * i8, u10 = (10.f * kUp) * t10 * i10;
   const float dT_dR = -R4 * R * fmaf(R2, fmaf(R2, u10, u8), u6);
   const float dT_dp = -p4 * p * fmaf(p2, fmaf(p2, u10, u8), u6);
   const float dT_dig = fmaf(61.25f * ig, i10, 5.f * i8);
-  const float dT_da17 = fmaf(dT_dp, kp, dT_dig * (4.f * fs) * sg * dsg);
+  const float dT_da17 = fmaf(dT_dp, kp * kDown, dT_dig * (4.f * fs) * sg * dsg);
   const float W = dT_da17 * a17 * rcp_fast(14.f * aij);          // dT / d(alpha_i h_i)
   float f = 1.f, df = 0.f;
   if (P.has_cutoff && P.has_damping) switching_fast(r, P.disp_on, P.rc, f, df);
   const float pre = (-2.f * kHartree) * alf_i * alf_j * rcp_fast(x_i + x_j);
   const float pf = pre * f, hh = hi * hj;
   e = pf * hh * T;
-  de_dr = pre * hh * fmaf(dT_dR * (1.f / kBohr), f, T * df);
+  de_dr = pre * hh * fmaf(dT_dR * (kDown / kBohr), f, T * df);
   de_dhi = pf * hj * fmaf(hi * alf_i, W, T);
   de_dhj = pf * hi * fmaf(hj * alf_j, W, T);
 }

@@ -87,6 +87,21 @@ def test_pair_kernels_evaluate_the_checked_dispersion_term():
     assert not re.findall(r"\bvoid dispersion\w*\(", src)
 
 
+@pytest.mark.parametrize("zi,zj,hi,hj", [(18, 18, 1.0, 1.0), (1, 1, 0.6, 0.7), (8, 1, 0.9, 0.65), (11, 17, 0.55, 1.1), (2, 10, 1.0, 1.0)])
+def test_dispersion_term_of_far_pairs(zi, zj, hi, hj):
+    """Without a cutoff nothing bounds the distance: energy and slope keep their digits where the products behind the slope (R^-12, R^-20) are
+    far below the float range.  Some forty roundings of 2^-24 = 6e-8, those of R counted up to ten times, and rounded constants: 4e-6 at
+    most, 2e-5 allowed."""
+    for r in (30.0, 100.0, 300.0, 900.0, 1500.0, 2500.0, 3300.0, 5000.0, 8000.0):
+        o4 = np.zeros(4, np.float32)
+        lib.so3lr_b200_host_dispersion_fast(r, zi, zj, hi, hj, -1.0, -1.0, _p(o4))
+        rt = torch.tensor([r], dtype=torch.float64, requires_grad=True)
+        ht = torch.tensor([hi, hj], dtype=torch.float64, requires_grad=True)
+        e = O.dispersion_pair(rt, torch.tensor([zi]), torch.tensor([zj]), ht[0:1], ht[1:2], None, None)[0]
+        er, eh = torch.autograd.grad(e, [rt, ht])
+        np.testing.assert_allclose(o4, [e.item(), er.item(), *eh.numpy()], rtol=2e-5, atol=0, err_msg=str(r))
+
+
 def test_zbl_matches_oracle(oracle_params):
     blob = np.load(O.DEFAULT_BLOB)["blob"].astype(np.float32)
     a, c, p, dd = O.zbl_energy(oracle_params, None, None, None, None, None)
