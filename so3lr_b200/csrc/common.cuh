@@ -80,6 +80,8 @@ SO3LR_D float dsilu_f(float x) {
 // while the kernel runs, which lets the compiler take the non-coherent path, or move a load above the wait (whose "memory"
 // clobber holds back only loads of memory that somebody else may change).  __ldg is for weights.  Write-only outputs, lists and other
 // arrays that are complete before the first chained kernel starts may keep the qualifier; device functions called after the wait too.
+// Lists are: an operation launched the ordinary way stands between the kernels that write them and the first chained kernel that reads
+// them (the copy of the reference positions at the end of rebuild_lists, the clearing at the start of so3lr_b200_dd_begin).
 SO3LR_D void grid_dep_sync() {
 #ifdef __CUDA_ARCH__
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -454,23 +454,26 @@ int rebuild_lists(so3lr_b200_system* S, cudaStream_t st, const float* R_user, bo
   }
   // both lists are counted, the host reads both totals in one wait, then both are filled
   int rc = kOk;
-  if (which != 1) rc = nlist_begin(S->nws, st, S->cell, S->n, R, r_sr, 0, seg, gs, &S->sr, 1, nullptr, -1, allow_sort);
+  const bool both = which == -1, both_counts = both && nlist_counts_in_one_kernel(S->n);
+  if (which != 1) rc = nlist_begin(S->nws, st, S->cell, S->n, R, r_sr, 0, seg, gs, &S->sr, 1, nullptr, -1, allow_sort,
+                                   both_counts ? RowsBeside::kFirst : RowsBeside::kNo);
   if (rc) return rc;
   if (which != 0) {
     if (!S->nws_lr && !(S->nws_lr = nlist_workspace_create())) return kCudaError;
     rc = nlist_begin(S->nws_lr, st, S->cell, S->n, R, r_lr, S->opt.lr_both_directions ? 0 : 1, seg ? seg : (gs_lr ? S->d_seg : nullptr),
-                     gs_lr, &S->lrl, 1, nullptr, -1, allow_sort, which == -1 && nlist_counts_in_one_kernel(S->n));
+                     gs_lr, &S->lrl, 1, nullptr, -1, allow_sort, both_counts ? RowsBeside::kSecond : RowsBeside::kNo);
     if (rc) return rc;
   }
   SO3LR_CUDA_CHECK(cudaStreamSynchronize(st));
-  if (which != 1) rc = nlist_end(S->nws, st, S->cell, &S->sr);
+  if (which != 1) rc = nlist_end(S->nws, st, S->cell, &S->sr, both ? RowsBeside::kFirst : RowsBeside::kNo);
   if (rc) return rc;
   if (which != 0) {
-    rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl, which == -1);
+    rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl, both ? RowsBeside::kSecond : RowsBeside::kNo);
     // the first list is filled: its votes have served (dev_free waits for the device)
     if (rc == kCudaError && which != 1 && nlist_drop_votes(S->nws)) rc = nlist_end(S->nws_lr, st, S->cell, &S->lrl);
   }
   if (rc) return rc;
+  // also keeps the chained kernels of the evaluation from starting before the lists are complete (see grid_dep_sync)
   SO3LR_CUDA_CHECK(cudaMemcpyAsync(S->d_Rref, R_user, (size_t)S->n * 3 * sizeof(float), cudaMemcpyDeviceToDevice, st));
   rc = ensure_edge_buffers(S, S->sr.count);
   if (rc) {
@@ -1846,6 +1849,7 @@ SO3LR_B200_API int so3lr_b200_dd_begin(so3lr_b200_system* S, void* stream, const
     S->n_rebuilds++;
   }
   const ModelDev& M = S->mctx;
+  // ordinary operations: the chained kernels behind them find the lists complete (see grid_dep_sync)
   fill(st, S->e_zbl, n0, 0.f);
   fill(st, S->F_s, (size_t)n0 * 3, 0.f);
   if (S->vir()) fill(st, S->virial, (size_t)n0 * 6, 0.f);

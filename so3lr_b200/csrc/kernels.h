@@ -313,13 +313,15 @@ int spatial_order(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, c
 // leave the int range (the builder returns the same status before it fills a single row)
 int nlist_row_total(cudaStream_t s, int n, const int* row_count_dev, long long* total_host);
 // nlist_build in two halves with a wait for the stream between them: several lists (a workspace each) share one wait.  `any_order`: the
-// entries of a row may come in any order.
+// entries of a row may come in any order.  Of two lists that are begun (ended) one right behind the other the first may say kFirst, which lets
+// the next kernel of the stream start early, and the second kSecond, whose kernel runs beside it.
+enum class RowsBeside { kNo, kFirst, kSecond };
 int nlist_begin(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered, const int* seg,
                 const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order,
-                bool beside = false);
+                RowsBeside beside = RowsBeside::kNo);
 bool nlist_counts_in_one_kernel(int n);         // the count kernel of n rows is the last thing that nlist_begin enqueues
 bool nlist_drop_votes(NlistWorkspace* ws);      // short of memory: the workspace gives up what it can do without
-int nlist_end(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, NeighborListDev* out, bool beside = false);
+int nlist_end(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, NeighborListDev* out, RowsBeside beside = RowsBeside::kNo);
 int nlist_build(NlistWorkspace* ws, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
                 const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows = -1);
 

@@ -277,7 +277,8 @@ __device__ __forceinline__ void build_row(const Cell& cell, const Grid& G, int n
 }
 
 // The row kernels of the short- and the long-range list of a rebuild do not depend on each other: the second may run beside the first (see
-// `beside` in nlist_begin).  It then has no wait at its start, but ends no earlier than the first: what follows waits for it alone.
+// RowsBeside).  It then has no wait at its start, but ends no earlier than the first: what follows waits for it alone.  Only the first
+// of two lets its successor start: no kernel but the second takes its place while a list is being written.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void end_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -287,8 +288,8 @@ __global__ void __launch_bounds__(256) build_rows_kernel(Cell cell, Grid G, int 
                                                          const float4* __restrict__ pos_sorted, const int* __restrict__ cell_start,
                                                          int* __restrict__ row_count, const int* __restrict__ row_ptr,
                                                          int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
-                                                         unsigned* __restrict__ masks, int mask_stride, TailScan tail) {
-  let_next_start();
+                                                         unsigned* __restrict__ masks, int mask_stride, TailScan tail, bool first_of_two) {
+  if (first_of_two) let_next_start();
   build_row<FILL>(cell, G, n, R, r_list, r2max, ordered, seg, pos_sorted, cell_start, row_count, row_ptr, nbr_j, edge_i, capacity, masks, mask_stride);
   if (!FILL) {
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(256) build_rows_graph_kernel(int n, const floa
                                                                const int* __restrict__ seg, const int* __restrict__ graph_start,
                                                                int* __restrict__ row_count, const int* __restrict__ row_ptr,
                                                                int* __restrict__ nbr_j, int* __restrict__ edge_i, long long capacity,
-                                                               TailScan tail) {
-  let_next_start();
+                                                               TailScan tail, bool first_of_two) {
+  if (first_of_two) let_next_start();
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i < n) {
@@ -406,9 +407,10 @@ int ensure_atoms(NlistWorkspace* w, int n) {
   return kOk;
 }
 template <class... P, class... A>
-void launch_rows(bool beside, void (*kernel)(P...), int blocks, cudaStream_t s, A&&... args) {
-  if (beside) launch_early(kernel, blocks, 256, 0, s, args...);
-  else kernel<<<blocks, 256, 0, s>>>(static_cast<P>(args)...);
+void launch_rows(RowsBeside beside, void (*kernel)(P...), int blocks, cudaStream_t s, A&&... args) {
+  const bool first = beside == RowsBeside::kFirst;
+  if (beside == RowsBeside::kSecond) launch_early(kernel, blocks, 256, 0, s, args..., first);
+  else kernel<<<blocks, 256, 0, s>>>(args..., first);
   count_launch();
 }
 int ensure_bytes(void** p, size_t* have, size_t need) {
@@ -474,19 +476,22 @@ int spatial_order(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, co
 constexpr int kOneCellAtoms = 1024;
 
 bool nlist_counts_in_one_kernel(int n) { return n <= kTailScanRows; }
-// `beside`: the kernel enqueued last is another list's count (or, in nlist_end, fill), beside which this one's may run.  Short lists are bound
-// by latency: the four row kernels of 1,536 atoms take 23, 26, 16 and 13 us one behind the other, the last CTA's scan of each among them.
+// `beside` kSecond: the kernel enqueued last is another list's count (or, in nlist_end, fill), launched as kFirst, beside which this one's may
+// run.  Short lists are bound by latency: the four row kernels of 1,536 atoms take 23, 26, 16 and 13 us one behind the other, the last
+// CTA's scan of each among them.
 int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, const float* R, float r_list, int ordered,
                 const int* seg, const int* graph_start, NeighborListDev* out, int allow_grow, int* d_overflow, int n_rows, bool any_order,
-                bool beside) {
+                RowsBeside beside) {
   w->n_rows = 0;
   if (n <= 0) { out->count = 0; return kOk; }
   if (n_rows < 0 || n_rows > n) n_rows = n;
+  // work of this list's own comes in between
+  auto not_second = [&] { if (beside == RowsBeside::kSecond) beside = RowsBeside::kNo; };
   if (int rca = ensure_atoms(w, n)) return rca;
   if (!w->ticket) {
     SO3LR_CUDA_CHECK(dev_alloc(&w->ticket, 2));
     SO3LR_CUDA_CHECK(cudaMemsetAsync(w->ticket, 0, 2 * sizeof(int), s));
-    beside = false;
+    not_second();
   }
   if (!w->d_total) SO3LR_CUDA_CHECK(dev_alloc(&w->d_total, 1));
   if (!w->h_total) SO3LR_CUDA_CHECK(host_alloc(&w->h_total, 1));
@@ -519,7 +524,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     } else {
       // bounding box on the host side would need a reduction; use a coarse device-free approach: the caller
       // passes free-space systems of moderate size, so read the positions back once per build.
-      beside = false;
+      not_second();
       std::vector<float> h((size_t)n * 3);
       SO3LR_CUDA_CHECK(cudaMemcpyAsync(h.data(), R, h.size() * sizeof(float), cudaMemcpyDeviceToHost, s));
       SO3LR_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -539,7 +544,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
     n_cells = G.nc[0] * G.nc[1] * G.nc[2];
     binned = n_cells > 1;      // the atoms of a single cell come in their own order either way
     if (binned) {
-      beside = false;      // its own cells come first
+      not_second();
       if (n_cells + 1 > w->cell_cap) {
         w->cell_cap = 0;
         if (int rcc = ensure(&w->cell_start, (size_t)n_cells + 1)) return rcc;
@@ -612,7 +617,7 @@ int nlist_begin(NlistWorkspace* w, cudaStream_t s, const Cell& cell, int n, cons
 }
 
 // the second half, once the stream has been waited for
-int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListDev* out, bool beside) {
+int nlist_end(NlistWorkspace* w, cudaStream_t s, const Cell& cell, NeighborListDev* out, RowsBeside beside) {
   const int n_rows = w->n_rows;
   if (n_rows <= 0) return kOk;
   const int blocks = (n_rows + 7) / 8, allow_grow = w->allow_grow;

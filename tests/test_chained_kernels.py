@@ -43,6 +43,41 @@ def test_non_coherent_loads_are_of_weights(source):
         assert arg.startswith(("L.", "M.")) or arg in {"const", "W", "p", "bias", "fin"}, arg
 
 
+def _function(source, name):
+    m = re.search(r"\b%s\([^;{]*\)\s*\{" % name, SOURCES[source])
+    return SOURCES[source][m.end():SOURCES[source].index("\n}\n", m.end())]
+
+
+def test_only_the_second_of_two_lists_starts_beside_the_kernel_before_it():
+    """Kernels that launch_early starts without a wait at their start: the row kernels of a second list, beside the first list's.  Nothing else may
+    take its place while a list is being written, and each of them ends behind its predecessor."""
+    everything = SOURCES | {os.path.basename(f): re.sub(r"//[^\n]*", "", open(f).read()) for p in ("*.h", "*.cuh") for f in glob.glob(os.path.join(CSRC, p))}
+    assert {f for f, s in everything.items() if "griddepcontrol" in s} == {"common.cuh", "nlist.cu"}
+    assert {f: len(re.findall(r"(?<!void )launch_early\(", s)) for f, s in everything.items() if "launch_early(" in s} == {"kernels.h": 1, "nlist.cu": 1}
+    s = SOURCES["nlist.cu"]
+    rows = set(re.findall(r"launch_rows\(beside, (\w+)", s))
+    assert rows == {"build_rows_kernel", "build_rows_graph_kernel"}
+    assert len(re.findall(r"let_next_start\(\)", s)) == 1 + len(rows) == 1 + len(re.findall(r"if \(first_of_two\) let_next_start\(\);", s))
+    for k in rows:
+        assert re.search(r"void (?:__launch_bounds__\(256\) )?%s\([^{]*bool first_of_two\) \{\s*if \(first_of_two\) let_next_start" % k, s)
+        body = _function("nlist.cu", k)
+        assert body.rstrip().endswith("end_after_previous();") and "return" not in body
+    assert "if (beside == RowsBeside::kSecond) launch_early(" in _function("nlist.cu", "launch_rows")
+    assert set(re.findall(r"(\w+) \? RowsBeside::k(?:First|Second) : RowsBeside::kNo", SOURCES["engine.cu"])) == {"both", "both_counts"}
+    assert len(re.findall(r"RowsBeside::k(?:First|Second)", SOURCES["engine.cu"])) == 4
+
+
+def test_lists_are_complete_ahead_of_the_first_chained_kernel():
+    """An operation launched the ordinary way between the kernels that write a list and the chained kernels that take it as constant."""
+    body = _function("engine.cu", "rebuild_lists")
+    behind = body[body.rindex("nlist_end("):]
+    assert "launch_chained" not in body[body.index("nlist_begin("):] and "cudaMemcpyAsync(S->d_Rref" in behind
+    assert "return kOk" not in behind[:behind.index("cudaMemcpyAsync(S->d_Rref")]
+    body = _function("engine.cu", "so3lr_b200_dd_begin")
+    behind = body[body.rindex("nlist_build("):]
+    assert behind.index("fill(st, S->e_zbl, n0, 0.f);") < behind.index("launch_sr_geometry_zbl(")
+
+
 def test_one_clearing_launch_holds_all_its_arrays():
     """The arrays travel in an object of fixed size that is passed by value: one too many must not be written behind its end."""
     s = SOURCES["engine.cu"]
