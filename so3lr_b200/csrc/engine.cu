@@ -139,7 +139,7 @@ __global__ void export_list_kernel(int n, long long count, long long capacity, c
   idx[capacity + e] = e < count ? nbr_j[e] : n;
 }
 // atoms are evaluated in a spatially sorted order: slot k holds atom perm[k]
-__global__ void gather_positions_kernel(int n, const int* __restrict__ perm, const float* R, float* __restrict__ Rs) {
+__global__ void gather_positions_kernel(int n, const int* perm /* the sort right ahead writes it */, const float* R, float* __restrict__ Rs) {
   grid_dep_sync();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;

@@ -33,7 +33,8 @@ def test_inputs_of_chained_kernels_are_not_promised_constant(kernel):
         if k == kernel:
             assert "grid_dep_sync();" in body
             promised = set(re.findall(r"const [\w ]+\* __restrict__ (\w+)", params))
-            assert promised <= CONSTANT, promised - CONSTANT
+            constant = CONSTANT - {"perm"} if k == "gather_positions_kernel" else CONSTANT      # it stands right behind the sort that makes the order
+            assert promised <= constant, promised - constant
 
 
 @pytest.mark.parametrize("source", sorted({f for f, *_ in _kernels()}))
