@@ -684,9 +684,12 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
 #ifdef SO3LR_TC_TIMING
   long long tph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   long long tc0 = clock64();
+  if (dbg && tid == 32 && blockIdx.x == 0) dbg[8] = 0;
 #define TC_MARK(k) do { if (dbg && (tid & 31) == 0) { const long long c = clock64(); tph[k] += c - tc0; tc0 = c; } } while (0)
+#define TC_TILE(slot) do { if (dbg && tid == 32 && blockIdx.x == 0) ++dbg[slot]; } while (0)
 #else
 #define TC_MARK(k) do { } while (0)
+#define TC_TILE(slot) do { } while (0)
 #endif
   for (; walk.tile < walk.end; walk.tile = walk.next) {
     const long long entry0 = (long long)walk.tile * tr;
@@ -907,9 +910,10 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     if (tid == kFwThreads - 1 && walk.asks()) *next_run = run;
     __syncthreads();
     TC_MARK(7);
+    TC_TILE(8);
   }
 #ifdef SO3LR_TC_TIMING
-  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[q] = tph[q]; dbg[8] = walk.end / gridDim.x; }
+  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[q] = tph[q]; }
   if (dbg && (tid & 31) == 0 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[160 + 8 * warp + q] = tph[q]; }
 #endif
   if (tid == kFwThreads - 1) walk.finish(queue);
@@ -1327,6 +1331,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
 #ifdef SO3LR_TC_TIMING
   long long bph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   long long bc0 = clock64();
+  if (dbg && tid == 32 && blockIdx.x == 0) dbg[24] = 0;
 #define BW_MARK(k) do { if (dbg && (tid & 31) == 0) { const long long c = clock64(); bph[k] += c - bc0; bc0 = c; } } while (0)
 #else
 #define BW_MARK(k) do { } while (0)
@@ -1623,9 +1628,10 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     if (tid == 256 && walk.asks()) *next_run = run;
     __syncthreads();
     BW_MARK(7);
+    TC_TILE(24);
   }
 #ifdef SO3LR_TC_TIMING
-  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[16 + q] = bph[q]; dbg[24] = walk.end / gridDim.x; }
+  if (dbg && tid == 32 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[16 + q] = bph[q]; }
   if (dbg && (tid & 31) == 0 && blockIdx.x == 0) { for (int q = 0; q < 8; ++q) dbg[32 + 8 * warp + q] = bph[q]; }
 #endif
   if (tid == 256) walk.finish(queue);
@@ -1729,7 +1735,8 @@ int valid_edges_count_directed(const ValidEdges& V, long long* n_host) {
   return kOk;
 }
 
-// development aid: SO3LR_B200_TC_DEBUG=1 makes the forward kernel record the cycles its first CTA spends in each phase
+// development aid of builds with -DSO3LR_TC_TIMING: SO3LR_B200_TC_DEBUG=1 makes the first CTA of both kernels record the cycles of each phase and
+// the number of its tiles
 static long long* tc_debug_buffer() {
   static long long* buf = [] {
     long long* p = nullptr;
@@ -1760,10 +1767,8 @@ void tc_debug_print() {
       for (int q = 0; q < 8; ++q) std::fprintf(stderr, " %6lld", h[160 + 8 * w + q] / h[8]);
       std::fprintf(stderr, "\n");
     }
-  std::fprintf(stderr, "tc fwd mma issue %lld wait %lld cycles per tile\n", h[9] / (h[8] ? h[8] : 1), h[10] / (h[8] ? h[8] : 1));
-  std::fprintf(stderr, "tc fwd phases (cycles per tile, %lld tiles): prep %lld | sync %lld | mma+wait %lld | tmem0 %lld | loop0 %lld | sync %lld | tmem1 %lld | loop1 %lld\n",
-               h[8], h[0] / (h[8] ? h[8] : 1), h[1] / (h[8] ? h[8] : 1), h[2] / (h[8] ? h[8] : 1), h[3] / (h[8] ? h[8] : 1), h[4] / (h[8] ? h[8] : 1),
-               h[5] / (h[8] ? h[8] : 1), h[6] / (h[8] ? h[8] : 1), h[7] / (h[8] ? h[8] : 1));
+  if (h[8]) std::fprintf(stderr, "tc fwd phases (cycles per tile, %lld tiles): prep %lld | sync %lld | mma+wait %lld | tmem0 %lld | loop0 %lld | sync %lld | tmem1 %lld | loop1 %lld\n",
+               h[8], h[0] / h[8], h[1] / h[8], h[2] / h[8], h[3] / h[8], h[4] / h[8], h[5] / h[8], h[6] / h[8], h[7] / h[8]);
 }
 int launch_attn_fwd_tc(cudaStream_t s, const LayerDev& L, const ValidEdges& V, int n_recv, const float* qkv, const float* x_in,
                        const float* ev_in, float* xa, float* ev1, int* err, bool preset) {

@@ -88,6 +88,22 @@ def test_one_clearing_launch_holds_all_its_arrays():
     assert len(uses) == len(re.findall(r"ClearArgs A;", s)) and all(0 < u.count("A.add(") <= room for u in uses)
 
 
+def test_cycle_counts_are_divided_by_the_tiles_that_were_walked():
+    """Timing builds of the attention kernels: every slot that is printed is written, and the divisors are counted tile by tile."""
+    s = SOURCES["attention_tc.cu"]
+    printed = _function("attention_tc.cu", "tc_debug_print")
+    phases, tiles = {}, {}
+    for name in ("attn_fwd_tc_kernel", "attn_bwd_tc_kernel"):
+        m = re.search(r"__global__ void (?:__launch_bounds__\([^)]*\) )?%s\(" % name, s)
+        body = s[m.end():s.index("tcgen05.dealloc", m.end())]
+        (slot,) = re.findall(r"TC_TILE\((\d+)\);", body)
+        assert f"dbg[{slot}] = 0" in body and "gridDim.x;" not in "".join(re.findall(r"if \(dbg[^\n]*", body))
+        (at,) = re.findall(r"dbg\[(?:(\d+) \+ )?q\] = [tb]ph\[q\]", body)
+        tiles[name], phases[name] = int(slot), range(int(at or 0), int(at or 0) + 8)
+    for slot in map(int, re.findall(r"(?<!long long )\bh\[(\d+)\]", printed)):
+        assert slot in tiles.values() or any(slot in r for r in phases.values()), slot
+
+
 def test_statuses_of_the_attention_launches_are_looked_at():
     """They refuse a list that was compacted for other rows; an evaluation that went on would hold no attention sums."""
     calls = re.findall(r"([^;{}]*?)\b((?:launch_attn_\w+_tc\w*|attn_\w+_dispatch)\()", SOURCES["engine.cu"])
