@@ -392,6 +392,8 @@ SO3LR_B200_API void so3lr_b200_host_pair_terms(float r, int zi, int zj, float qi
 SO3LR_B200_API int so3lr_b200_host_kspace_tiles(int n1, int n2, int n3, int64_t* counts4, double* weight_sum);
 /* out2 = chi(r), d chi / d r of the Coulomb pair function; smearing > 0 takes the reciprocal-space part out of it */
 SO3LR_B200_API void so3lr_b200_host_coulomb_chi(float r, float cutoff_lr, float smearing, float* out2);
+/* tiles of the block that walks most of n_tiles equal tiles in the tiled attention kernels, -1 if a tile is missed or walked twice */
+SO3LR_B200_API int64_t so3lr_b200_host_tile_walk(int n_tiles, int grid);
 SO3LR_B200_API void so3lr_b200_host_dispersion_fast(float r, int zi, int zj, float hi, float hj, float cutoff_lr, float damping,
                                                     float* out4);
 SO3LR_B200_API void so3lr_b200_host_zbl(const float* blob_host, float r, int zi, int zj, float* out2);

@@ -39,6 +39,7 @@
 #include <cuda_fp16.h>
 #include <cstdlib>
 #include <type_traits>
+#include <vector>
 
 #include "kernels.h"
 
@@ -568,27 +569,32 @@ __device__ __forceinline__ int entries_per_warp(long long n_edges, int grid) {
   const long long rounds = (n_edges + (long long)TE * grid - 1) / ((long long)TE * grid);
   return (int)((n_edges + 16 * rounds * grid - 1) / (16 * rounds * grid));
 }
-// Which tiles a CTA takes.  Short lists: an equal share of consecutive tiles.  Long lists: runs of kTileRun tiles in the order in which CTAs
-// come free (CTA b starts with run b).  SMs differ by several per cent in the time of a tile (their distance from the L2 slices that hold its
-// rows), so equal shares end with the slowest; and all CTAs work in one stretch of the list at a time, whose rows stay in the L2.  The
-// next run is asked for during the first tile of a run.  `queue`: runs handed out beyond the first of every CTA | CTAs that are
-// through; both zero at the start of a launch: the build of the list clears them, and the last CTA to finish puts them back.
-constexpr int kTileRun = 2;
+// Which tiles a CTA takes.  Short lists: an equal share of consecutive tiles.  Long lists: the tiles in the order in which CTAs come free (CTA b
+// starts with tiles b and grid + b).  SMs differ by several per cent in the time of a tile (their distance from the L2 slices that hold its
+// rows), so equal shares end with the slowest; and all CTAs work in one stretch of the list at a time, whose rows stay in the L2.  A
+// tile's inputs are staged beneath the tile before it, so during each tile the one behind the next is asked for.  `queue`: tiles handed
+// out beyond the first two of every CTA | CTAs that are through; both zero at the start of a launch: the build of the list clears them,
+// and the last CTA to finish puts them back.
+// Forward / reverse, us a launch, tiles per CTA: queue | equal shares | a queue of runs of two tiles, which ends with a whole tile too many where
+// the share is odd.  2.2: 43.3 / 80.5 | 41.8 / 79.9 | 52.3 / 101.7, 5.2: 76.2 / 155.1 | 75.0 / 154.6 | -, 7.3: 89.5 / 206.1 | 90.0 / 207.1 | -,
+// 8.3: 99.4 / 230.4 | 99.9 / 232.6 | 108.5 / 252.6, 14.4: 156 / 374 | 158 / 376 | 166 / 397, 25.8: 264 / 638 | 264 / 681 | 263 / 641,
+// 104: 1,003 / 2,474 | 1,028 / 2,698 | 1,003 / 2,501.  The line stands behind the crossing (6): below it the queue's first question costs.
 constexpr int kQueuedTiles = 8;                // tiles per CTA from which on the queue is used
 struct TileWalk {
   int tile, next, end;      // this tile, the one behind it; tiles from `end` on are not this CTA's
   bool queued;
-  __device__ __forceinline__ explicit TileWalk(int n) {
-    const int grid = (int)gridDim.x, b = (int)blockIdx.x, share = n / grid, more = n - share * grid;
+  SO3LR_HD TileWalk(int n, int grid, int b) {
+    const int share = n / grid, more = n - share * grid;
     queued = share >= kQueuedTiles;
-    tile = queued ? kTileRun * b : b * share + min(b, more);
+    tile = queued ? b : b * share + (b < more ? b : more);
     end = queued ? n : tile + share + (b < more);
     next = tile;
   }
-  __device__ __forceinline__ bool asks() const { return queued && tile % kTileRun == 0; }
-  __device__ __forceinline__ int ask(int* queue) const { return kTileRun * ((int)gridDim.x + atomicAdd(queue, 1)); }
-  // `run`: the first tile of the next run, asked for during the first tile of this one
-  __device__ __forceinline__ void look_ahead(const int* run) { next = queued && tile % kTileRun == kTileRun - 1 ? *run : tile + 1; }
+  SO3LR_HD int second(int grid) const { return grid + tile; }
+  SO3LR_HD static int handed(int grid, int ticket) { return 2 * grid + ticket; }
+  // `handed_out`: two words in shared memory, taken in turns (`turn`): a warp may still look up the next tile when another one is at the end of
+  // this one and writes the tile that follows
+  SO3LR_HD void look_ahead(const int* handed_out, uint32_t turn) { next = queued ? handed_out[turn] : tile + 1; }
   // one thread per CTA, behind its last tile
   __device__ __forceinline__ void finish(int* queue) const {
     if (queued && atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) { atomicExch(queue, 0); atomicExch(queue + 1, 0); }
@@ -625,7 +631,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffFwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffFwMisc + 16);
   volatile int* failed = reinterpret_cast<volatile int*>(smem + kOffFwMisc + 20);
-  int* next_run = reinterpret_cast<int*>(smem + kOffFwMisc + 32);
+  int* handed_out = reinterpret_cast<int*>(smem + kOffFwMisc + 32);
   for (int k = tid; k < kTcImageBytes / 16; k += kFwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kFwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
     const int q = k & 7, c = (k >> 3) & 31, f = k >> 8;
@@ -641,7 +647,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
   const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
-  TileWalk walk((int)((n_edges + tr - 1) / tr));
+  TileWalk walk((int)((n_edges + tr - 1) / tr), (int)gridDim.x, (int)blockIdx.x);
   if (walk.tile >= walk.end) return;
   const int pad_i = ve_i[n_edges - 1];
   // partners below n_scat receive the pair's other direction (j <- i)
@@ -667,6 +673,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   stage_tile(walk.tile);
+  if (tid == 0) handed_out[0] = walk.second((int)gridDim.x);
   cp_async_wait_all();
   fence_async_smem();
   tc_fence_before();
@@ -753,7 +760,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     TC_MARK(1);
-    walk.look_ahead(next_run);
+    walk.look_ahead(handed_out, parity);
     if (issues) {
       tc_fence_after();
       issue_forward_mma(on, tmem, a_hi, img, (warp >> 1) & 1, warp & 1, 1);
@@ -761,7 +768,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
       request_rows();
     }
     stage_tile(walk.next);
-    if (tid == kFwThreads - 1 && walk.asks()) run = walk.ask(queue);
+    if (tid == kFwThreads - 1 && walk.queued) run = TileWalk::handed((int)gridDim.x, atomicAdd(queue, 1));
     wait_mma(mbar0, parity, failed, err);
     parity ^= 1;
     TC_MARK(2);
@@ -907,7 +914,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsign
       if (lane < kMTot && accev != 0.f) atomicAdd(ev1 + (size_t)cur_i * kMTot + lane, accev);
     });
     cp_async_wait_all();
-    if (tid == kFwThreads - 1 && walk.asks()) *next_run = run;
+    if (tid == kFwThreads - 1 && walk.queued) handed_out[parity] = run;
     __syncthreads();
     TC_MARK(7);
     TC_TILE(8);
@@ -1269,7 +1276,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   float* wt = reinterpret_cast<float*>(smem + kOffBwW);
   unsigned long long* mbar_p = reinterpret_cast<unsigned long long*>(smem + kOffBwMisc);
   uint32_t* tmem_p = reinterpret_cast<uint32_t*>(smem + kOffBwMisc + 48);
-  int* next_run = reinterpret_cast<int*>(smem + kOffBwMisc + 56);
+  int* handed_out = reinterpret_cast<int*>(smem + kOffBwMisc + 56);
   volatile int* failed = reinterpret_cast<volatile int*>(smem + kOffBwMisc + 52);
   for (int k = tid; k < kTcImageBytes / 16; k += kBwThreads) reinterpret_cast<uint4*>(smem + kOffImg)[k] = reinterpret_cast<const uint4*>(img_g)[k];
   for (int k = tid; k < 512; k += kBwThreads) {      // [filter][hidden unit][w0 w1 w2 w3 b - - -]
@@ -1288,7 +1295,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
   const long long n_edges = *n_listed;
   if (n_edges <= 0) return;
   const int rpw = entries_per_warp(n_edges, gridDim.x), tr = 16 * rpw;      // entries per warp / per tile
-  TileWalk walk((int)((n_edges + tr - 1) / tr));
+  TileWalk walk((int)((n_edges + tr - 1) / tr), (int)gridDim.x, (int)blockIdx.x);
   if (walk.tile >= walk.end) return;
   const int pad_i = ve_i[n_edges - 1];
   int* st_ij = reinterpret_cast<int*>(smem + kOffBwStIJ);
@@ -1311,6 +1318,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     }
   };
   stage_tile(walk.tile);
+  if (tid == 0) handed_out[0] = walk.second((int)gridDim.x);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_p)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -1385,9 +1393,9 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     tc_fence_before();
     __syncthreads();
     BW_MARK(1);
-    walk.look_ahead(next_run);
+    walk.look_ahead(handed_out, parity);
     stage_tile(walk.next);
-    if (tid == 256 && walk.asks()) run = walk.ask(queue);
+    if (tid == 256 && walk.queued) run = TileWalk::handed((int)gridDim.x, atomicAdd(queue, 1));
     if (warp < 4) {
       tc_fence_after();
       issue_filter_mma(on, tmem, a_hi, img, warp >> 1, warp & 1, 1);
@@ -1625,7 +1633,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       if (lane < kMTot && acc != 0.f) atomicAdd(gev_in + (size_t)cur_i * kMTot + lane, acc);
     });
     cp_async_wait_all();
-    if (tid == 256 && walk.asks()) *next_run = run;
+    if (tid == 256 && walk.queued) handed_out[parity] = run;
     __syncthreads();
     BW_MARK(7);
     TC_TILE(24);
@@ -1733,6 +1741,35 @@ int valid_edges_count_directed(const ValidEdges& V, long long* n_host) {
   SO3LR_CUDA_CHECK(e);
   *n_host = (long long)h;
   return kOk;
+}
+
+// The walks of all CTAs over n tiles whose times are all alike, CTAs coming free in the order of their numbers
+long long tile_walk_longest(int n, int grid) {
+  struct Cta { TileWalk walk; int handed_out[2]; int tiles; };
+  std::vector<Cta> ctas;
+  for (int b = 0; b < grid; ++b) {
+    Cta c{TileWalk(n, grid, b), {0, 0}, 0};
+    c.handed_out[0] = c.walk.second(grid);
+    ctas.push_back(c);
+  }
+  std::vector<char> seen(n > 0 ? n : 0, 0);
+  long long walked = 0;
+  int tickets = 0, longest = 0;
+  for (bool any = true; any;) {
+    any = false;
+    for (Cta& c : ctas) {
+      if (c.walk.tile >= c.walk.end) continue;
+      any = true;
+      if (c.walk.tile < 0 || c.walk.tile >= n || seen[c.walk.tile]++) return -1;
+      const uint32_t turn = c.tiles & 1;
+      c.walk.look_ahead(c.handed_out, turn);
+      if (c.walk.queued) c.handed_out[turn ^ 1] = TileWalk::handed(grid, tickets++);
+      c.walk.tile = c.walk.next;
+      if (++c.tiles > longest) longest = c.tiles;
+      ++walked;
+    }
+  }
+  return walked == n ? longest : -1;
 }
 
 // development aid of builds with -DSO3LR_TC_TIMING: SO3LR_B200_TC_DEBUG=1 makes the first CTA of both kernels record the cycles of each phase and

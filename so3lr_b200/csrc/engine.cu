@@ -2136,6 +2136,7 @@ SO3LR_B200_API void so3lr_b200_host_coulomb_chi(float r, float cutoff_lr, float 
   set_coulomb_shift(P);
   coulomb_chi(P, r, out2[0], out2[1]);
 }
+SO3LR_B200_API int64_t so3lr_b200_host_tile_walk(int n_tiles, int grid) { return n_tiles < 0 || grid < 1 ? -1 : tile_walk_longest(n_tiles, grid); }
 SO3LR_B200_API void so3lr_b200_host_dispersion_fast(float r, int zi, int zj, float hi, float hj, float cutoff_lr, float damping, float* out4) {
   LrParams P{};
   P.has_cutoff = cutoff_lr > 0.f; P.rc = cutoff_lr; P.cuton = kCutonFraction * cutoff_lr; P.has_damping = damping > 0.f;

@@ -205,6 +205,8 @@ void valid_edges_free(ValidEdges* V);
 int valid_edges_build(ValidEdges* V, cudaStream_t s, int n_rows, int n, const int* row_ptr, const int* nbr_j, const float* dR,
                       int* asym = nullptr, long long n_source = 0, bool total_cleared = false);
 // entries i <- j of the latest build counted per direction (synchronises)
+// host check of how the attention kernels hand out their tiles: tiles of the CTA that has most, -1 where a tile is left out or taken twice
+long long tile_walk_longest(int n_tiles, int grid);
 int valid_edges_count_directed(const ValidEdges& V, long long* n_host);
 // The reverse kernel for caller-supplied lists: runs only while *asym == 0 and, instead of summing forces, adds to every source
 // entry e (V.orig) half of the force that the pair exerts on its receiver, g[e] += (dE/d dR_e - dE/d dR_e') / 2 with e' the

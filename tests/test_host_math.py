@@ -184,3 +184,11 @@ def test_ewald_tiles_count_every_index_once(shape):
     assert wsum.value == n1 * n2 * n3 - 1
     assert counts[3] == 0 and 1 <= counts[2] <= 4 and counts[1] <= counts[0]
     assert counts[0] * 256 >= (n1 * n2 * n3 - 1) / 2
+
+
+@pytest.mark.parametrize("grid", [1, 2, 7, 132, 148])
+def test_tiles_are_handed_out_once_and_evenly(grid):
+    """Tiles of one list over the blocks of an attention kernel: each once, and no block has more than its share rounded up."""
+    for n in sorted({0, 1, grid - 1, *(k * grid + d for k in (1, 2, 7, 8, 9, 10, 11, 12, 25, 104) for d in (-1, 0, 1, grid // 3, grid // 2))}):
+        if n >= 0:
+            assert lib.so3lr_b200_host_tile_walk(n, grid) == -(-n // grid), (n, grid)
