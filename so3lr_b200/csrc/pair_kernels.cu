@@ -1,5 +1,7 @@
 // Edge geometry + ZBL repulsion on the short-range graph, the fused long-range pair kernel (damped Coulomb +
 // dispersion with analytic gradients) and the small per-graph reductions around them.
+#include <algorithm>
+
 #include "kernels.h"
 
 namespace so3lr {
@@ -281,11 +283,14 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
   if (virial) va.flush_warp(virial, (size_t)i, lane, split > 1);
 }
 // Warps per row.  A short list leaves most of the chip idle with one: 1,536 atoms are 10 warps per SM, and a row of the ordered list holds up to
-// 12 rounds of 32 pairs, each a chain of gathers and some 400 instructions (2 us).  As many warps as 32 per SM allow and the average row has rounds.
+// 12 rounds of 32 pairs, each a chain of gathers and some 400 instructions (2 us).  As many warps as the average row has rounds and as 32
+// per SM allow (what 62 registers a thread keep resident); never more than 12 (390 atoms in a list with both directions).
+// The three launches of the pair terms without / with a 1 A skin, us, one warp a row -> this rule: 192 atoms 17.5 / 18.9 -> 13.3 / 13.4 (3 warps),
+// 390: 24.7 / 27.6 -> 15.0 / 15.5 (6, 7), 600: 29.9 / 33.9 -> 17.6 / 18.1 (7), 1,536: 36.5 / 48.0 -> 24.1 / 25.8 (3); one warp from 2,369 atoms
+// on: 38.0 / 50.0 at 2,400 (two warps there, two waves of blocks: 35.6 / 36.0).
 int pair_row_split(int n, long long pairs) {
   const long long rounds = (pairs / n + 31) / 32, room = 32LL * sm_count() / n;
-  const long long s = rounds < room ? rounds : room;
-  return s < 1 ? 1 : (s > 16 ? 16 : (int)s);
+  return (int)std::max(1LL, std::min(rounds, room));
 }
 
 // Owned rows of an ordered list over owned atoms and ghosts (decomposed runs; ghosts carry the larger indices, so the list
