@@ -172,7 +172,7 @@ def algorithmic_bytes(group, N, E, P):
 # box (attn_bwd_tc_kernel, attn_fwd_tc_kernel; atom_post_*_tc_kernel: the launch with the fused projections).  A full-size
 # capture is not taken (ncu replays each launch about 40 times); lists and per-atom arrays grow with the atom count at fixed
 # density, so the figure is scaled by N / 98304 and the line says so in `traffic_source`.
-NCU_TRAFFIC_98K = {"attn_bwd": 2524.0e6, "attn_fwd": 851.4e6, "atom_post_fwd": 487.2e6, "atom_post_bwd": 559.4e6}
+NCU_TRAFFIC_98K = {"attn_bwd": 1095.2e6, "attn_fwd": 506.2e6, "atom_post_fwd": 483.4e6, "atom_post_bwd": 558.7e6}
 
 
 def ncu_traffic(group, n_atoms):

@@ -24,11 +24,12 @@
 // (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.
 //
 // What binds the kernels: the latency of four warps per scheduler (their 128 registers fill the register file).  Per 128 pairs the reverse
-// kernel issues 64 k warp instructions (16 k cycles of the 44 k a tile takes), moves 23 k wavefronts through the load / store pipe, 4 k
-// through the tensor cores' and keeps the way to the L2 busy for 18 k cycles (a row reduction leaves an SM at 21 to 26 bytes per cycle);
-// none is near its limit, and forms with more warps, fewer registers or two independent tiles per SM ended within 15 % of it or above.
+// kernel issues 64 k warp instructions (16 k cycles of the 43 k a tile takes), moves 24 k wavefronts through the load / store pipe, 7 k
+// through the tensor cores' and keeps the way to the L2 busy for 18 k cycles (407 KB of reductions, which leave an SM at 21 to 26 bytes
+// per cycle); the forward kernel 28 k instructions (7 k cycles of 17.6 k), 12 k and 2 k wavefronts (counters at 98,304 atoms).  None is
+// near its limit, and forms with more warps, fewer registers or two independent tiles per SM ended within 15 % of it or above.
 // 98,304 atoms (1.97 M pairs), forward / reverse, ms per launch: 1.99 / 5.12 with every pair evaluated at both ends, 1.16 / 2.85 with one
-// evaluation per pair, entry loops that sum four pairs' logits together and one thread that issues, 1.01 / 2.50 as it stands.
+// evaluation per pair, entry loops that sum four pairs' logits together and one thread that issues, 1.00 / 2.47 as it stands.
 //
 // The reverse kernel forms dw in the same loop, writes it straight into shared memory as the (FP16-split) A operand of a
 // second MMA chain against the SAME weight image read with the other major-ness,
@@ -612,8 +613,8 @@ __device__ __forceinline__ void edge_loops(int share, Body&& body, int run = 8) 
 // forward
 // ------------------------------------------------------------------------------------------------------------------
 // 16 warps.  Per tile: (1) preparation of the A operand and the records: Chebyshev terms by two threads per pair, geometry by a third (the
-// fourth's warps issue the MMAs), then the hidden layers by four neighbouring threads per pair; (2) the MMA chains of the two filters, while every warp already has the sender rows
-// of its 8 pairs in flight; (3) per filter: tensor memory -> shared tile, then the edge loop.
+// fourth's warps issue the MMAs), then the hidden layers by four neighbouring threads per pair; (2) the MMA chains of the two filters, while
+// every warp already has the sender rows of its 8 pairs in flight; (3) per filter: tensor memory -> shared tile, then the edge loop.
 __global__ void __launch_bounds__(kFwThreads, 1) attn_fwd_tc_kernel(const unsigned char* __restrict__ img_g, const float* __restrict__ sph1_k,
                                                                     const float* __restrict__ sph1_b, int n_recv,
                                                                     const int* n_listed, const int* ve_i,
@@ -937,9 +938,6 @@ namespace {
 // ------------------------------------------------------------------------------------------------------------------
 // reverse
 // ------------------------------------------------------------------------------------------------------------------
-// record fields (floats): 0 j | 1 i | 2 cutoff / nbar | 3 its r-derivative | 4-7 invariants | 8-11 their cotangents |
-// 12-15 dA, 16-19 dB: cotangents of the equivariant logits of edge (i<-j) and (j<-i) | 20-23, 24-27 those logits x cutoff |
-// 28-30 unit vector | 31 1/r | 32 d/dr | 33 r | 34 1 for a list entry, 0 for a padding row
 // [dPhi | dhs_f] = dw_f * [C_f^T | K2_f^T] (the same image read K-major: N = 96 rows, K = features): main accumulators in TMEM
 // columns [128 f, 128 f + 96), cross 256 columns above
 __device__ __forceinline__ void issue_reverse_mma(uint32_t on, uint32_t tmem, uint32_t a_hi, uint32_t img, int f, int half, int cross) {
@@ -1545,8 +1543,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
     // ---- force on the receiver (threads 0..127); cotangent of ev (8 rows per warp) ----
     if (tid < 128) {
       const float* rp = rec + tid * kBwRec;
-      const bool on = rp[14] != 0.f;
-      const int i = on ? __float_as_int(rp[1]) : -1;
+      const bool listed = rp[14] != 0.f;
+      const int i = listed ? __float_as_int(rp[1]) : -1;
       const float4 uu = ld4(rp + 8);
       float e1[3], e2[3], t1 = 0.f, t2 = 0.f;
       tangent_frame(uu.x, uu.y, uu.z, e1, e2);
@@ -1560,8 +1558,8 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       const float4 ang = make_float4(fmaf(t1, e1[0], t2 * e2[0]), fmaf(t1, e1[1], t2 * e2[1]), fmaf(t1, e1[2], t2 * e2[2]), 0.f);
       const float* dr = wt + 4 * 4 * TE + tid;
       const float g_r = rp[12] + ((dr[0] + dr[TE]) + (dr[2 * TE] + dr[3 * TE]));
-      float fsx = on ? fmaf(g_r, uu.x, ang.x) : 0.f, fsy = on ? fmaf(g_r, uu.y, ang.y) : 0.f, fsz = on ? fmaf(g_r, uu.z, ang.z) : 0.f;
-      if (virial && on) {
+      float fsx = listed ? fmaf(g_r, uu.x, ang.x) : 0.f, fsy = listed ? fmaf(g_r, uu.y, ang.y) : 0.f, fsz = listed ? fmaf(g_r, uu.z, ang.z) : 0.f;
+      if (virial && listed) {
         // both ends' halves on the receiver's row, unless the partner's is not summed here (rows below n_own are)
         const float hr = (__float_as_int(rp[0]) < n_own ? 1.f : 0.5f) * rp[13];
         const float wx = hr * uu.x, wy = hr * uu.y, wz = hr * uu.z;
@@ -1573,7 +1571,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       if (PER_ENTRY) {
         // half of the pair's force on the receiver goes to this entry of the source list, the other half with the opposite sign to the
         // reversed entry
-        if (on) {
+        if (listed) {
           const int2 eo = ve_orig[entry0 + entry_of(tid)];
           float *g = F + 3 * (size_t)eo.x, *h = F + 3 * (size_t)eo.y;
           g[0] += 0.5f * fsx; g[1] += 0.5f * fsy; g[2] += 0.5f * fsz;
@@ -1583,7 +1581,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
       // the rows of a tile are sorted by receiver: sum each run of equal receivers inside the warp (segmented scan) and let its
       // last lane add the total, instead of up to 32 additions to one address; the partners differ and get theirs one by one
       const int jp = __float_as_int(rp[0]);
-      if (on && jp < n_scat) {
+      if (listed && jp < n_scat) {
         atomicAdd(F + 3 * (size_t)jp, -fsx); atomicAdd(F + 3 * (size_t)jp + 1, -fsy); atomicAdd(F + 3 * (size_t)jp + 2, -fsz);
       }
 #pragma unroll
@@ -1593,7 +1591,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) attn_bwd_tc_kernel(const unsign
         if (lane >= o && ti == i) { fsx += tx; fsy += ty; fsz += tz; }
       }
       const int inext = __shfl_down_sync(0xffffffffu, i, 1);
-      if (on && (lane == 31 || inext != i)) {
+      if (listed && (lane == 31 || inext != i)) {
         atomicAdd(F + 3 * (size_t)i, fsx); atomicAdd(F + 3 * (size_t)i + 1, fsy); atomicAdd(F + 3 * (size_t)i + 2, fsz);
       }
       }

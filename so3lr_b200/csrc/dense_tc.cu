@@ -204,7 +204,7 @@ __device__ __forceinline__ float dsilu_fast(float x) {
 // D[128 x n] (+)= A[:, chunks] * B: A from chunk `a_chunk0` on (2 chunks per K step of 16), B image at w_smem (hi matrix, lo
 // matrix w_lo bytes above, core-matrix stride along K = 16 n bytes): the hi*hi products (cross = 0) or the hi*lo and lo*hi products.
 // The first four warps share the issue of a contraction: main and cross products by one warp each, or a head per warp.  One
-// thread takes about 100 cycles an MMA: 2.5 to 3 k cycles for the 24 of a 128 x 128 contraction, 18 k for the 120 small ones of the
+// thread takes 100 to 150 cycles an MMA: 2.5 to 3 k cycles for the 24 of a 128 x 128 contraction, 18 k for the 120 small ones of the
 // block-diagonal projections' reverse, which the tensor cores are through with in 1.6 and 2 k.
 __device__ __forceinline__ void issue_gemm(uint32_t on, int cross, uint32_t tmem, int d_col, uint32_t a_smem, int a_chunk0, uint32_t w_smem,
                                            uint32_t w_lo, int n, int ksteps, uint32_t accumulate) {
@@ -259,7 +259,8 @@ struct Tile {
     inv = reinterpret_cast<float4*>(sm + kOffInv);
     red = reinterpret_cast<float4*>(sm + kOffRed);
     redf = reinterpret_cast<float*>(sm + kOffRed2);
-    tid = threadIdx.x; warp = __shfl_sync(0xffffffffu, tid >> 5, 0); lane = tid & 31; on = elect_one(); row = tid & 127; quarter = tid >> 7; c0 = 32 * quarter;
+    tid = threadIdx.x; warp = __shfl_sync(0xffffffffu, tid >> 5, 0); lane = tid & 31; on = elect_one();
+    row = tid & 127; quarter = tid >> 7; c0 = 32 * quarter;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kOffMisc);
     uint32_t* tmem_p = reinterpret_cast<uint32_t*>(sm + kOffMisc + 32);
     mbar = smem_u32(bars); wbar = smem_u32(bars + 1); mbar2 = smem_u32(bars + 2);
