@@ -24,8 +24,8 @@
 // (3.2 TB/s once the target exceeds it), and a pair sends 0.6 KB forward and 2.7 KB in reverse.
 //
 // What binds the kernels: the latency of four warps per scheduler (their 128 registers fill the register file).  Per 128 pairs the reverse
-// kernel issues 64 k warp instructions (16 k cycles of the 43 k a tile takes), moves 24 k wavefronts through the load / store pipe, 7 k
-// through the tensor cores' and keeps the way to the L2 busy for 18 k cycles (407 KB of reductions, which leave an SM at 21 to 26 bytes
+// kernel issues 65 k warp instructions (16 k cycles of the 43 k a tile takes), moves 24 k wavefronts through the load / store pipe, 7 k
+// through the tensor cores' and keeps the way to the L2 busy for 18 k cycles (410 KB of reductions, which leave an SM at 21 to 26 bytes
 // per cycle); the forward kernel 28 k instructions (7 k cycles of 17.6 k), 12 k and 2 k wavefronts (counters at 98,304 atoms).  None is
 // near its limit, and forms with more warps, fewer registers or two independent tiles per SM ended within 15 % of it or above.
 // 98,304 atoms (1.97 M pairs), forward / reverse, ms per launch: 1.99 / 5.12 with every pair evaluated at both ends, 1.16 / 2.85 with one
