@@ -2083,6 +2083,10 @@ void so3lr_b200_host_sph_harm(float x, float y, float z, float* y24) { sph_harm_
 SO3LR_B200_API void so3lr_b200_host_sph_harm_vjp(float x, float y, float z, const float* g24, float* g3) {
   sph_harm_24_vjp(x, y, z, g24, g3[0], g3[1], g3[2]);
 }
+static void host_coulomb_chi(const LrParams& P, float r, float& chi, float& dchi) {
+  if (P.has_cutoff && r >= P.rc) { chi = dchi = 0.f; return; }      // the kernels leave such pairs out
+  coulomb_chi(P, r, 1.f / r, chi, dchi);
+}
 SO3LR_B200_API void so3lr_b200_host_pair_terms(float r, int zi, int zj, float qi, float qj, float hi, float hj, float cutoff_lr, float damping,
                                 float* out8) {
   LrParams P{};
@@ -2090,7 +2094,7 @@ SO3LR_B200_API void so3lr_b200_host_pair_terms(float r, int zi, int zj, float qi
   P.disp_on = cutoff_lr - damping; P.pair_factor = 1.f;
   set_coulomb_shift(P);
   float chi, dchi;
-  coulomb_chi(P, r, chi, dchi);
+  host_coulomb_chi(P, r, chi, dchi);
   out8[0] = kKe * qi * qj * chi; out8[1] = kKe * qi * qj * dchi; out8[2] = kKe * qj * chi;
   dispersion_pair(P, r, zi, zj, hi, hj, out8[3], out8[4], out8[5], out8[6]);
   out8[7] = 0.f;
@@ -2134,7 +2138,7 @@ SO3LR_B200_API void so3lr_b200_host_coulomb_chi(float r, float cutoff_lr, float 
   P.has_cutoff = cutoff_lr > 0.f; P.rc = cutoff_lr; P.cuton = kCutonFraction * cutoff_lr; P.pair_factor = 1.f;
   P.k_alpha = smearing > 0.f ? (float)(1.0 / (std::sqrt(2.0) * (double)smearing)) : 0.f;
   set_coulomb_shift(P);
-  coulomb_chi(P, r, out2[0], out2[1]);
+  host_coulomb_chi(P, r, out2[0], out2[1]);
 }
 SO3LR_B200_API int64_t so3lr_b200_host_tile_walk(int n_tiles, int grid) { return n_tiles < 0 || grid < 1 ? -1 : tile_walk_longest(n_tiles, grid); }
 SO3LR_B200_API void so3lr_b200_host_dispersion_fast(float r, int zi, int zj, float hi, float hj, float cutoff_lr, float damping, float* out4) {

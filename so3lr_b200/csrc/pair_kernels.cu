@@ -71,25 +71,6 @@ __global__ void force_scatter_kernel(int n, long long n_edges, const int* __rest
   atomicAdd(F + 3 * (size_t)j, -gx); atomicAdd(F + 3 * (size_t)j + 1, -gy); atomicAdd(F + 3 * (size_t)j + 2, -gz);
 }
 
-// coulomb_chi of pair_terms.cuh with the approximate operations
-__device__ __forceinline__ void coulomb_chi_dev(const LrParams& p, float r, float rinv, float& chi, float& dchi) {
-  const float inv_sig = 1.f / kSigmaCoulomb;
-  const float x = r * inv_sig;
-  float pot = erff(x) * rinv;
-  float dpot = (1.1283791670955126f * inv_sig * __expf(-x * x) - pot) * rinv;
-  if (p.k_alpha > 0.f) {     // the reciprocal-space sum holds erf(r k_alpha) / r
-    const float y = r * p.k_alpha;
-    const float potk = erff(y) * rinv;
-    pot -= potk;
-    dpot -= (1.1283791670955126f * p.k_alpha * __expf(-y * y) - potk) * rinv;
-  }
-  if (!p.has_cutoff) { chi = pot; dchi = dpot; return; }
-  float f, df;
-  switching_fast(r, p.cuton, p.rc, f, df);
-  chi = (pot - p.v_rc) - (1.f - f) * (r - p.rc) * p.dv_rc;
-  dchi = dpot - (1.f - f) * p.dv_rc + df * (r - p.rc) * p.dv_rc;
-}
-
 // one warp per row i; lanes stride over the row's pairs
 template <int MODE>
 __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int n, const int* __restrict__ row_ptr,
@@ -127,7 +108,7 @@ __global__ void __launch_bounds__(256) pair_lr_kernel(LrParams P, Cell cell, int
       if (r2 > 0.f && (!P.has_cutoff || r2 < P.rc * P.rc)) {
         const float rinv = rsqrtf(r2), r = r2 * rinv;
         float chi, dchi;
-        coulomb_chi_dev(P, r, rinv, chi, dchi);
+        coulomb_chi(P, r, rinv, chi, dchi);
         const float qj = q[j], hj = h[j];
         const float pf = P.pair_factor;
         const float kq = pf * kKe;
@@ -221,7 +202,7 @@ __global__ void __launch_bounds__(256) pair_lr_packed_kernel(LrParams P, Cell ce
     const float r2 = dx * dx + dy * dy + dz * dz;
     const float rinv = rsqrtf(r2), r = r2 * rinv;
     float chi, dchi;
-    coulomb_chi_dev(P, r, rinv, chi, dchi);
+    coulomb_chi(P, r, rinv, chi, dchi);
     float e_d, dd_dr, dd_dhi, dd_dhj;
     dispersion_pair_fast(P, r, hzi.y, hzi.z, hi, hzj.y, hzj.z, hzj.x, e_d, dd_dr, dd_dhi, dd_dhj);
     ec = fmaf(kq * qi * qj, chi, ec);
@@ -322,7 +303,7 @@ __global__ void __launch_bounds__(256) pair_lr_owned_kernel(LrParams P, Cell cel
     if (!(r2 > 0.f) || (P.has_cutoff && r2 >= P.rc * P.rc)) continue;
     const float rinv = rsqrtf(r2), r = r2 * rinv;
     float chi, dchi;
-    coulomb_chi_dev(P, r, rinv, chi, dchi);
+    coulomb_chi(P, r, rinv, chi, dchi);
     const float qj = q[j], hj = h[j];
     const int Zj = Z[j];
     float e_d, dd_dr, dd_dhi, dd_dhj;

@@ -56,27 +56,6 @@ struct LrParams {
   float k_alpha;        // 1 / (sqrt(2) s) when the reciprocal-space sum holds erf(r / (sqrt(2) s)) / r of every pair; 0: off
 };
 
-// erf-damped Coulomb kernel chi(r) (energy = ke q_i q_j chi) and d chi / d r
-SO3LR_HD void coulomb_chi(const LrParams& p, float r, float& chi, float& dchi) {
-  const float inv_sig = 1.f / kSigmaCoulomb;
-  float x = r * inv_sig;
-  float er = erff(x);
-  float pot = er / r;
-  float dpot = (1.1283791670955126f * inv_sig * expf(-x * x) - pot) / r;
-  if (p.k_alpha > 0.f) {
-    const float y = r * p.k_alpha;
-    const float potk = erff(y) / r;
-    pot -= potk;
-    dpot -= (1.1283791670955126f * p.k_alpha * expf(-y * y) - potk) / r;
-  }
-  if (!p.has_cutoff) { chi = pot; dchi = dpot; return; }
-  if (r >= p.rc) { chi = 0.f; dchi = 0.f; return; }
-  float f, df;
-  switching(r, p.cuton, p.rc, f, df);
-  chi = (pot - p.v_rc) - (1.f - f) * (r - p.rc) * p.dv_rc;
-  dchi = dpot - (1.f - f) * p.dv_rc + df * (r - p.rc) * p.dv_rc;
-}
-
 // Dispersion energy (eV) of one pair and its derivatives w.r.t. r (Angstrom), h_i and h_j.
 SO3LR_HD void dispersion_pair(const LrParams& p, float r, int Zi, int Zj, float hi, float hj, float& e, float& de_dr,
                               float& de_dhi, float& de_dhj) {
@@ -145,6 +124,25 @@ SO3LR_HD void switching_fast(float x, float on, float off, float& f, float& df) 
   const float E = exp_fast(t);
   f = rcp_fast(1.f + E);
   df = -(E * f) * (f * (ia * ia + ib * ib)) * iw;   // in this order no intermediate leaves the float range
+}
+
+// erf-damped Coulomb kernel chi(r) (energy = ke q_i q_j chi) and d chi / d r of a pair inside the cutoff; rinv = 1 / r
+SO3LR_HD void coulomb_chi(const LrParams& p, float r, float rinv, float& chi, float& dchi) {
+  const float inv_sig = 1.f / kSigmaCoulomb;
+  const float x = r * inv_sig;
+  float pot = erff(x) * rinv;
+  float dpot = (1.1283791670955126f * inv_sig * exp_fast(-x * x) - pot) * rinv;
+  if (p.k_alpha > 0.f) {     // the reciprocal-space sum holds erf(r k_alpha) / r
+    const float y = r * p.k_alpha;
+    const float potk = erff(y) * rinv;
+    pot -= potk;
+    dpot -= (1.1283791670955126f * p.k_alpha * exp_fast(-y * y) - potk) * rinv;
+  }
+  if (!p.has_cutoff) { chi = pot; dchi = dpot; return; }
+  float f, df;
+  switching_fast(r, p.cuton, p.rc, f, df);
+  chi = (pot - p.v_rc) - (1.f - f) * (r - p.rc) * p.dv_rc;
+  dchi = dpot - (1.f - f) * p.dv_rc + df * (r - p.rc) * p.dv_rc;
 }
 
 // The dispersion term of the long-range pair kernels, with hand-derived partials (checked against float64 on the host); the caller keeps

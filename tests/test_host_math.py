@@ -70,7 +70,7 @@ def test_pair_terms_match_oracle(cutoff, damping):
         np.testing.assert_allclose(out[3], ed.item(), rtol=5e-5, atol=1e-7)
         np.testing.assert_allclose(out[4], ded_r.item(), rtol=2e-4, atol=1e-7)
         np.testing.assert_allclose(out[5:7], ded_h.numpy(), rtol=2e-4, atol=1e-7)
-        # the function that the pair kernels evaluate (test_pair_kernels_evaluate_the_checked_dispersion_term), its approximate operations
+        # the function that the pair kernels evaluate (test_pair_kernels_evaluate_the_checked_pair_terms), its approximate operations
         # replaced by libm's
         o4 = np.zeros(4, np.float32)
         lib.so3lr_b200_host_dispersion_fast(r, zi, zj, hi, hj, cutoff, damping, _p(o4))
@@ -79,12 +79,13 @@ def test_pair_terms_match_oracle(cutoff, damping):
         np.testing.assert_allclose(o4[2:4], ded_h.numpy(), rtol=2e-4, atol=1e-7)
 
 
-def test_pair_kernels_evaluate_the_checked_dispersion_term():
-    """What the host check above covers is what the kernels call: they hold no dispersion term of their own."""
+def test_pair_kernels_evaluate_the_checked_pair_terms():
+    """What the host checks of this file cover is what the kernels call: they hold no pair terms of their own."""
     src = open(os.path.join(os.path.dirname(__file__), "..", "so3lr_b200", "csrc", "pair_kernels.cu")).read()
     src = re.sub(r"//[^\n]*", "", src)
-    assert len(re.findall(r"(?<!void )\bdispersion_pair_fast\(", src)) >= 3
-    assert not re.findall(r"\bvoid dispersion\w*\(", src)
+    for name in ("dispersion_pair_fast", "coulomb_chi"):
+        assert len(re.findall(r"(?<!void )\b%s\(" % name, src)) >= 3
+    assert not re.findall(r"\bvoid (?:dispersion|coulomb|switching)\w*\(", src)
 
 
 @pytest.mark.parametrize("zi,zj,hi,hj", [(18, 18, 1.0, 1.0), (1, 1, 0.6, 0.7), (8, 1, 0.9, 0.65), (11, 17, 0.55, 1.1), (2, 10, 1.0, 1.0)])
